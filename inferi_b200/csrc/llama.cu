@@ -133,8 +133,7 @@ struct ib_llama {
     // sampling beyond greedy (ib_llama_set_sampler): parameters, scratch, and the graph that carries the sampler node
     float temperature = 0.f, topp = 0.f;
     uint64_t sample_seed = 0;
-    float *sample_probs = nullptr;
-    unsigned long long *sample_keys = nullptr;
+    float *sample_probs = nullptr;   // only for vocabularies that the sampler cannot hold in shared memory
     cudaGraphExec_t graph_exec_sample = nullptr;
     uint64_t launches_per_token_sample = 0;
     // prompt prefill (ib_llama_prefill): buffers for up to PREFILL_MAX_TOKENS tokens at a time, allocated at the first call
@@ -285,7 +284,7 @@ static int32_t record_token(ib_llama *m, cudaStream_t s, uint32_t pdl) {
     if (m->temperature > 0.f) {
         // temperature / top-p sampling replaces the greedy token (models/sampler.rs:32-52); the coin is a function of
         // (seed, position)
-        if ((rc = launch_sample(ctx, s, m->logits, c.vocab_size, m->temperature, m->topp, m->sample_seed, &m->ctl->pos, 0.f, m->sample_probs, m->sample_keys,
+        if ((rc = launch_sample(ctx, s, m->logits, c.vocab_size, m->temperature, m->topp, m->sample_seed, &m->ctl->pos, 0.f, m->sample_probs,
                                 &m->ctl->next, nullptr, pdl)))
             return rc;
     }
@@ -401,7 +400,6 @@ int32_t ib_llama_destroy(ib_llama *m) {
     if (m->graph_exec_short) cudaGraphExecDestroy(m->graph_exec_short);
     if (m->graph_exec_sample_short) cudaGraphExecDestroy(m->graph_exec_sample_short);
     if (m->sample_probs) cudaFree(m->sample_probs);
-    if (m->sample_keys) cudaFree(m->sample_keys);
     if (m->own_stream) cudaStreamDestroy(m->own_stream);
     if (m->staged) cudaEventDestroy(m->staged);
     for (int r = 0; r < m->tp_size && r < IB_MAX_TP; r++)
@@ -637,10 +635,7 @@ int32_t ib_llama_set_sampler(ib_llama *m, float temperature, float topp, uint64_
     if (m->graph_exec_sample_short) { cudaGraphExecDestroy(m->graph_exec_sample_short); m->graph_exec_sample_short = nullptr; }
     m->temperature = temperature; m->topp = topp; m->sample_seed = seed;
     if (temperature == 0.f) return IB_OK;   // greedy: the graph recorded at creation
-    if (!m->sample_probs) {
-        IB_CHECK_CUDA(cudaMalloc(&m->sample_probs, sizeof(float) * m->cfg.vocab_size));
-        IB_CHECK_CUDA(cudaMalloc(&m->sample_keys, sizeof(unsigned long long) * sample_keys_capacity(m->cfg.vocab_size)));
-    }
+    if (!m->sample_probs && sample_scratch_bytes(m->cfg.vocab_size)) IB_CHECK_CUDA(cudaMalloc(&m->sample_probs, sample_scratch_bytes(m->cfg.vocab_size)));
     int32_t rc = capture_graph(m, &m->graph_exec_sample, &m->launches_per_token_sample);
     if (rc == IB_OK && m->short_positions) {
         if (m->graph_exec_sample_short) { cudaGraphExecDestroy(m->graph_exec_sample_short); m->graph_exec_sample_short = nullptr; }

@@ -5,22 +5,54 @@
 // host with an unseeded `rand::random()`; here the logits stay on the device and the coin of a position is a pure
 // function of (seed, position), so a sequence can be reproduced.
 //
-// One CTA of 1024 threads (the work is a few passes over <= a few hundred thousand floats in L2):
 //   x_i = logit_i / temperature;  p_i = exp(x_i - max x) / sum          (softmax.rs:134-142)
 //   multinomial: first i with coin < p_0 + ... + p_i, else n - 1         (sampler.rs:62-77)
 //   top-p: candidates p_i >= (1 - topp) / (n - 1), sorted by descending p (stable: ascending index on ties), cut after
 //          the first prefix whose sum exceeds topp, then first i with coin * prefix_sum < running sum (sampler.rs:84-129)
-// Sums run in a fixed order (per-thread chunks, then a block scan): results are deterministic; they can differ from a
-// sequential f32 sum by rounding (of the order of sqrt(n) * 2^-24 in the running sum), which changes the sampled token only when
-// the coin falls that close to a boundary between two tokens.
+//
+// The launch is ONE thread-block cluster of 16 CTAs (8 where the device cannot place 16).  Every CTA holds a contiguous
+// slice of the vocabulary in shared memory; what the CTAs have to tell one another (maximum, sum, histograms) goes
+// through distributed shared memory and the cluster barrier, so the whole of it is one launch without a round trip to
+// L2.  The work is a few passes over some hundred KB: with one CTA those passes alone took 100 us, and the sort of the
+// candidates (thousands for a language model's distribution) several hundred.
+//
+// Nothing is sorted here.  Both steps of top-p ask for the element at which the running sum of the sorted candidates
+// crosses a bound, and that is a selection: a histogram of probability mass over the top bits of p (2048 bins, sixteen
+// per factor of two) finds the bin of the crossing, and only the few elements of that bin are listed and ordered.  A bin
+// that holds more elements than the list (flat distributions) is cut into finer bins first; when all bits are used up
+// its elements are equal and are taken in index order.
+//
+// Masses are added as integers in units of 2^-52 (p's f32 mantissa fits), so the sums are exact, independent of the
+// order in which the atomics happen, and at least as close to the real sums as the sequential f32 ones.
+//
+// What bounds it: latency (ten cluster barriers and the passes between them), not bytes: 513 KB of logits.  128256 tokens
+// of a language model's distribution, top-p 0.95: 27 us per launch; the version with one CTA and a sort 515 us.  Multinomial
+// 12 us; a flat distribution (everything in one bin) 114 us.
 #include "common.cuh"
 
+#include <cooperative_groups.h>
 #include <math.h>
 
 namespace ib {
 
-constexpr int SAMPLE_THREADS = 1024;
-constexpr uint32_t SAMPLE_SMEM_KEYS = 4096;   // candidates that are sorted in shared memory; more go through global memory
+namespace cg = cooperative_groups;
+
+constexpr int SAMPLE_THREADS = 1024, SAMPLE_WARPS = SAMPLE_THREADS / 32;
+constexpr uint32_t SAMPLE_MAX_CLUSTER = 16;
+constexpr uint32_t SAMPLE_BINS = 2048, SAMPLE_TOP_SHIFT = 19;   // p <= 1: bits(p) >> 19 <= 0x7F0
+constexpr uint32_t SAMPLE_LIST = 4096;                          // elements of a bin that are ordered in shared memory
+constexpr uint32_t SAMPLE_SLICE_MAX = 32768;                    // floats of a slice that fit shared memory beside the rest; longer slices live in global memory
+
+struct SampleShared {
+    uint32_t lo[SAMPLE_BINS], hi[SAMPLE_BINS];      // this CTA's histogram of mass: 64-bit sums as two words (see mass_add)
+    unsigned long long tot[SAMPLE_BINS];            // first CTA: the cluster's histogram
+    unsigned long long list[SAMPLE_LIST];           // first CTA: the elements of one bin, key = (~bits(p), index)
+    float xf[2][SAMPLE_MAX_CLUSTER];                // one word from every CTA of the cluster
+    unsigned long long xu[2][SAMPLE_MAX_CLUSTER];
+    unsigned long long red[SAMPLE_WARPS];
+    unsigned long long base, answer, cum;           // first CTA: mass ahead of the bin; the crossing element's key and running sum
+    uint32_t count, prefix, found, slot;
+};
 
 // coin of a position: splitmix64 of (seed, position), top 24 bits -> [0, 1)
 __host__ __device__ inline float sample_coin(uint64_t seed, uint32_t pos) {
@@ -31,220 +63,395 @@ __host__ __device__ inline float sample_coin(uint64_t seed, uint32_t pos) {
     return (float)(uint32_t)(z >> 40) * (1.0f / 16777216.0f);
 }
 
-__device__ __forceinline__ float block_reduce_max(float v, float *sm) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (lane == 0) sm[warp] = v;
-    __syncthreads();
-    float r = sm[0];
-    for (int w = 1; w < SAMPLE_THREADS / 32; w++) r = fmaxf(r, sm[w]);
-    __syncthreads();
-    return r;
+// p in units of 2^-52 (p in [0, 1]; exact for p >= 2^-29, rounded down below)
+__device__ __forceinline__ unsigned long long mass_of(float p) {
+    const uint32_t b = __float_as_uint(p), e = b >> 23;
+    if (e == 0) return 0ull;
+    const unsigned long long m = (b & 0x7FFFFFu) | 0x800000u;
+    const int s = (int)e - 98;   // value = m * 2^(e - 150)
+    return s >= 0 ? m << s : (s > -24 ? m >> -s : 0ull);
+}
+// 64-bit shared-memory sum out of two native 32-bit atomics: whoever makes the low word wrap carries the one
+__device__ __forceinline__ void mass_add(SampleShared &S, uint32_t bin, unsigned long long q) {
+    const uint32_t l = (uint32_t)q;
+    const uint32_t old = atomicAdd(&S.lo[bin], l);
+    const uint32_t h = (uint32_t)(q >> 32) + ((uint32_t)(old + l) < old ? 1u : 0u);
+    if (h) atomicAdd(&S.hi[bin], h);
 }
 
-// Exclusive scan of one value per thread in thread order; returns the prefix of this thread, *total gets the sum.
-__device__ __forceinline__ float block_scan(float v, float *sm, float *total) {
+template <typename T> __device__ __forceinline__ T shfl_down_t(T v, int o) { return __shfl_down_sync(0xffffffffu, v, o); }
+
+// Inclusive scan over the block in thread order; *total gets the sum.  Ends with a barrier.
+__device__ __forceinline__ unsigned long long block_scan(unsigned long long v, SampleShared &S, unsigned long long *total) {
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    float inc = v;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const float t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
+        const unsigned long long t = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v += t;
     }
-    if (lane == 31) sm[warp] = inc;
+    if (lane == 31) S.red[warp] = v;
     __syncthreads();
-    float base = 0.f, tot = 0.f;
-    for (int w = 0; w < SAMPLE_THREADS / 32; w++) {
-        if (w == warp) base = tot;
-        tot += sm[w];
-    }
-    __syncthreads();
-    *total = tot;
-    return base + inc - v;
-}
-__device__ __forceinline__ uint32_t block_scan_u32(uint32_t v, uint32_t *sm, uint32_t *total) {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint32_t inc = v;
+    unsigned long long w = S.red[lane];   // SAMPLE_WARPS == 32
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
-        const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += t;
+        const unsigned long long t = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += t;
     }
-    if (lane == 31) sm[warp] = inc;
+    *total = __shfl_sync(0xffffffffu, w, 31);
+    const unsigned long long ahead = __shfl_sync(0xffffffffu, w, warp ? warp - 1 : 0);
     __syncthreads();
-    uint32_t base = 0, tot = 0;
-    for (int w = 0; w < SAMPLE_THREADS / 32; w++) {
-        if (w == warp) base = tot;
-        tot += sm[w];
-    }
-    __syncthreads();
-    *total = tot;
-    return base + inc - v;
+    return v + (warp ? ahead : 0ull);
 }
 
-// First index i in [0, count) with limit < value(0) + ... + value(i) (running sum in index order), or `none`.
-// `running_at` receives the running sum at that index (or the total).  Values come from `get(i)`.
-template <typename Get>
-__device__ __forceinline__ uint32_t first_crossing(uint32_t count, float limit, Get get, float *smf, uint32_t *smu, uint32_t none, float *running_at) {
-    const uint32_t chunk = (count + SAMPLE_THREADS - 1) / SAMPLE_THREADS;
-    const uint32_t i0 = min(count, threadIdx.x * chunk), i1 = min(count, i0 + chunk);
-    float s = 0.f;
-    for (uint32_t i = i0; i < i1; i++) s += get(i);
-    float total;
-    const float base = block_scan(s, smf, &total);
-    uint32_t found = 0xFFFFFFFFu;
-    float at = 0.f, run = base;
-    for (uint32_t i = i0; i < i1; i++) {
-        run += get(i);
-        if (limit < run) { found = i; at = run; break; }
+// Ascending bitonic sort of list[0 .. cap) (cap a power of two <= SAMPLE_LIST).  Up to 1024 keys a thread holds one and the
+// exchanges inside a warp are shuffles.
+__device__ __forceinline__ void sort_list(unsigned long long *list, uint32_t cap) {
+    const uint32_t tid = threadIdx.x;
+    if (cap <= SAMPLE_THREADS) {
+        unsigned long long v = tid < cap ? list[tid] : ~0ull;
+        for (uint32_t k = 2; k <= cap; k <<= 1)
+            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+                unsigned long long o;
+                if (j >= 32) {
+                    __syncthreads();
+                    if (tid < cap) list[tid] = v;
+                    __syncthreads();
+                    o = tid < cap ? list[tid ^ j] : ~0ull;
+                } else o = __shfl_xor_sync(0xffffffffu, v, j);
+                const bool keep_min = ((tid & k) == 0) == ((tid & j) == 0);
+                v = keep_min ? (v < o ? v : o) : (v < o ? o : v);
+            }
+        __syncthreads();
+        if (tid < cap) list[tid] = v;
+        __syncthreads();
+        return;
     }
-    // the lowest index over the block, with its running sum
-    __shared__ unsigned long long best;
-    if (threadIdx.x == 0) best = ~0ull;
-    __syncthreads();
-    if (found != 0xFFFFFFFFu) atomicMin(&best, ((unsigned long long)found << 32) | __float_as_uint(at));
-    __syncthreads();
-    const unsigned long long b = best;
-    __syncthreads();
-    (void)smu;
-    if (b == ~0ull) { *running_at = total; return none; }
-    *running_at = __uint_as_float((uint32_t)b);
-    return (uint32_t)(b >> 32);
+    for (uint32_t k = 2; k <= cap; k <<= 1)
+        for (uint32_t j = k >> 1; j > 0; j >>= 1) {
+            for (uint32_t t = tid; t < cap / 2; t += SAMPLE_THREADS) {
+                const uint32_t a = ((t & ~(j - 1)) << 1) | (t & (j - 1)), b = a | j;
+                const unsigned long long x = list[a], y = list[b];
+                if ((x > y) == ((a & k) == 0)) { list[a] = y; list[b] = x; }
+            }
+            __syncthreads();
+        }
 }
 
-__device__ __forceinline__ void cmp_swap(unsigned long long &a, unsigned long long &b, bool up) {
-    if ((a > b) == up) { const unsigned long long t = a; a = b; b = t; }
-}
+// `probs` [n]: scratch for slices that do not fit shared memory (null otherwise).  `pos_ptr` / `seed`: the coin
+// (sample_coin); with pos_ptr == null `coin_in` is used.  Writes the token to *out (and to *out2 if non-null).
+__global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const float *__restrict__ logits, uint32_t n, uint32_t slice, float temperature, float topp,
+                                                                uint64_t seed, const uint32_t *pos_ptr, float coin_in, float *probs, uint32_t *out,
+                                                                uint32_t *out2, uint32_t pdl) {
+    extern __shared__ __align__(16) uint8_t smem[];
+    SampleShared &S = *reinterpret_cast<SampleShared *>(smem);
+    cg::cluster_group cluster = cg::this_cluster();
+    const uint32_t C = cluster.num_blocks(), rank = cluster.block_rank(), tid = threadIdx.x;
+    const int lane = tid & 31, warp = tid >> 5;
+    SampleShared &first = *cluster.map_shared_rank(&S, 0);
+    auto barrier = [&]() { cluster.sync(); };
 
-// `probs` [n] and `keys` [next power of two >= n] are scratch.  `pos_ptr` / `seed`: the coin (sample_coin); with
-// pos_ptr == null `coin_in` is used.  Writes the token to *out (and to *out2 if non-null).
-__global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const float *__restrict__ logits, uint32_t n, float temperature, float topp, uint64_t seed,
-                                                                const uint32_t *pos_ptr, float coin_in, float *probs, unsigned long long *keys,
-                                                                uint32_t *out, uint32_t *out2, uint32_t pdl) {
-    extern __shared__ unsigned long long sm_keys[];   // SAMPLE_SMEM_KEYS
-    __shared__ float smf[SAMPLE_THREADS / 32];
-    __shared__ uint32_t smu[SAMPLE_THREADS / 32];
+    cluster.barrier_arrive();   // every CTA of the cluster runs: needed before its shared memory is written from outside
+    for (uint32_t b = tid; b < SAMPLE_BINS; b += SAMPLE_THREADS) { S.lo[b] = 0u; S.hi[b] = 0u; }
+    if (tid == 0) { S.count = 0u; S.found = 0u; }
     if (pdl) {
         asm volatile("griddepcontrol.launch_dependents;");
         asm volatile("griddepcontrol.wait;" ::: "memory");
     }
     const float coin = pos_ptr ? sample_coin(seed, *pos_ptr) : coin_in;
-    const uint32_t tid = threadIdx.x;
+    const uint32_t i0 = min(n, rank * slice), len = min(n, i0 + slice) - i0;
+    float *P = probs ? probs + i0 : reinterpret_cast<float *>(smem + sizeof(SampleShared));
 
     // x = logits / temperature, softmax (softmax.rs:134-142)
     float mx = -INFINITY;
-    for (uint32_t i = tid; i < n; i += SAMPLE_THREADS) {
-        const float x = __fdiv_rn(__ldcg(logits + i), temperature);
-        probs[i] = x;
+    for (uint32_t i = tid; i < len; i += SAMPLE_THREADS) {
+        const float x = __fdiv_rn(__ldcg(logits + i0 + i), temperature);
+        P[i] = x;
         mx = fmaxf(mx, x);
     }
-    mx = block_reduce_max(mx, smf);
-    const uint32_t chunk = (n + SAMPLE_THREADS - 1) / SAMPLE_THREADS;
-    const uint32_t i0 = min(n, tid * chunk), i1 = min(n, i0 + chunk);
-    __syncthreads();   // probs written with a strided pattern, read back in chunks
+    // one f32 per CTA -> every CTA; `op` folds warps, then CTAs, in a fixed order
+    auto exchange = [&](float v, int which, auto op) {
+        float *red = reinterpret_cast<float *>(S.red);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
+        if (lane == 0) red[warp] = v;
+        __syncthreads();
+        if (warp == 0) {
+            v = red[lane];
+#pragma unroll
+            for (int o = 16; o; o >>= 1) v = op(v, __shfl_xor_sync(0xffffffffu, v, o));
+            if ((uint32_t)lane < C) *cluster.map_shared_rank(&S.xf[which][rank], lane) = v;
+        }
+        barrier();
+        v = S.xf[which][0];
+        for (uint32_t r = 1; r < C; r++) v = op(v, S.xf[which][r]);
+        return v;
+    };
+    cluster.barrier_wait();
+    mx = exchange(mx, 0, [](float a, float b) { return fmaxf(a, b); });
     float s = 0.f;
-    for (uint32_t i = i0; i < i1; i++) {
-        const float e = expf(probs[i] - mx);
-        probs[i] = e;
+    for (uint32_t i = tid; i < len; i += SAMPLE_THREADS) {
+        const float e = expf(P[i] - mx);
+        P[i] = e;
         s += e;
     }
-    float sum;
-    block_scan(s, smf, &sum);
-    for (uint32_t i = i0; i < i1; i++) probs[i] = __fdiv_rn(probs[i], sum);
-    __syncthreads();
-
-    uint32_t token;
-    float run;
-    if (topp <= 0.f || topp >= 1.f) {
-        // sampler.rs:62-77
-        token = first_crossing(n, coin, [&](uint32_t i) { return probs[i]; }, smf, smu, n - 1, &run);
-    } else {
-        // sampler.rs:84-129.  Candidates in index order (stable), key = descending probability then ascending index.
-        const float cutoff = __fdiv_rn(1.0f - topp, (float)n - 1.0f);
-        uint32_t cnt = 0;
-        for (uint32_t i = i0; i < i1; i++) cnt += probs[i] >= cutoff;
-        uint32_t n0;
-        uint32_t at = block_scan_u32(cnt, smu, &n0);
-        if (n0 == 0) {
-            // No probability reaches the cut-off ((1 - topp) / (n - 1) can exceed the largest one, e.g. n = 2 with a small
-            // topp).  The reference subtracts 1 from an unsigned zero there (sampler.rs:108); defined here as the arg-max,
-            // lowest index on ties.
-            __shared__ unsigned long long amax;
-            if (tid == 0) amax = 0ull;
-            __syncthreads();
-            unsigned long long b = 0ull;
-            for (uint32_t i = i0; i < i1; i++) {
-                const unsigned long long k = ((unsigned long long)__float_as_uint(probs[i]) << 32) | (0xFFFFFFFFu - i);   // p >= 0: bits order like values
-                b = k > b ? k : b;
-            }
-            if (i0 < i1) atomicMax(&amax, b);
-            __syncthreads();
-            if (tid == 0) {
-                const uint32_t t = 0xFFFFFFFFu - (uint32_t)(amax & 0xFFFFFFFFull);
-                *out = t;
-                if (out2) *out2 = t;
-            }
-            return;
-        }
-        uint32_t cap = 1;
-        while (cap < n0) cap <<= 1;
-        unsigned long long *K = cap <= SAMPLE_SMEM_KEYS ? sm_keys : keys;
-        for (uint32_t i = i0; i < i1; i++)
-            if (probs[i] >= cutoff) K[at++] = ((unsigned long long)(~__float_as_uint(probs[i])) << 32) | i;
-        for (uint32_t i = n0 + tid; i < cap; i += SAMPLE_THREADS) K[i] = ~0ull;
-        __syncthreads();
-        // bitonic sort, ascending keys
-        for (uint32_t k = 2; k <= cap; k <<= 1)
-            for (uint32_t j = k >> 1; j > 0; j >>= 1) {
-                for (uint32_t t = tid; t < cap / 2; t += SAMPLE_THREADS) {
-                    const uint32_t lo = ((t & ~(j - 1)) << 1) | (t & (j - 1)), hi = lo | j;
-                    unsigned long long a = K[lo], b = K[hi];
-                    cmp_swap(a, b, (lo & k) == 0);
-                    K[lo] = a; K[hi] = b;
-                }
-                __syncthreads();
-            }
-        auto prob_at = [&](uint32_t i) { return __uint_as_float(~(uint32_t)(K[i] >> 32)); };
-        float cumulative;
-        uint32_t last = first_crossing(n0, topp, prob_at, smf, smu, n0 - 1, &cumulative);   // first prefix whose sum exceeds topp
-        const float r = coin * cumulative;
-        const uint32_t pick = first_crossing(last + 1, r, prob_at, smf, smu, last, &run);
-        token = (uint32_t)(K[pick] & 0xFFFFFFFFull);
-    }
-    if (tid == 0) {
+    const float sum = exchange(s, 1, [](float a, float b) { return a + b; });
+    auto done = [&](uint32_t token) {
         *out = token;
         if (out2) *out2 = token;
+    };
+
+    if (topp <= 0.f || topp >= 1.f) {
+        // sampler.rs:62-77: the slices' masses, then the slice that holds the crossing looks for it
+        const uint32_t per = (len + SAMPLE_THREADS - 1) / SAMPLE_THREADS, a = min(len, tid * per), b = min(len, a + per);
+        unsigned long long mine = 0ull, total, ahead = 0ull;
+        for (uint32_t i = a; i < b; i++) {
+            const float p = __fdiv_rn(P[i], sum);
+            P[i] = p;
+            mine += mass_of(p);
+        }
+        const unsigned long long upto = block_scan(mine, S, &total);
+        if (tid < C) *cluster.map_shared_rank(&S.xu[0][rank], tid) = total;
+        barrier();
+        const unsigned long long X = (unsigned long long)((double)coin * 4503599627370496.0);
+        for (uint32_t r = 0; r < rank; r++) ahead += S.xu[0][r];
+        unsigned long long run = ahead + upto - mine;
+        if (X >= run && X < run + mine) {
+            for (uint32_t i = a; i < b; i++) {
+                run += mass_of(P[i]);
+                if (X < run) { done(i0 + i); break; }
+            }
+        }
+        if (rank == C - 1 && tid == 0 && X >= ahead + total) done(n - 1);
+        return;
     }
+
+    // sampler.rs:84-129
+    const float cutoff = __fdiv_rn(1.0f - topp, (float)n - 1.0f);
+    for (uint32_t base = 0; base < len; base += SAMPLE_THREADS) {
+        const uint32_t i = base + tid;
+        const float p = i < len ? __fdiv_rn(P[i], sum) : -1.f;
+        if (i < len) P[i] = p;
+        const bool cand = p >= cutoff;
+        const uint32_t bin = min(__float_as_uint(p) >> SAMPLE_TOP_SHIFT, SAMPLE_BINS - 1), act = __ballot_sync(0xffffffffu, cand);
+        if (act == 0u) continue;
+        // flat distributions: a warp whose 32 candidates share a bin adds them up first
+        int same = 0;
+        if (act == 0xffffffffu) __match_all_sync(0xffffffffu, bin, &same);
+        unsigned long long q = cand ? mass_of(p) : 0ull;
+        if (same) {
+#pragma unroll
+            for (int o = 16; o; o >>= 1) q += __shfl_xor_sync(0xffffffffu, q, o);
+            if (lane == 0) mass_add(S, bin, q);
+        } else if (cand) mass_add(S, bin, q);
+    }
+
+    // the cluster's histogram in the first CTA: every CTA adds up its share of the bins over the CTAs
+    auto gather_bins = [&]() {
+        barrier();
+        const uint32_t lanes = C / 2, share = SAMPLE_BINS / C, bin = rank * share + tid / lanes, r0 = tid % lanes;   // share * lanes == SAMPLE_THREADS
+        unsigned long long v = 0ull;
+#pragma unroll
+        for (uint32_t k = 0; k < 2; k++) {
+            SampleShared &o = *cluster.map_shared_rank(&S, r0 + k * lanes);
+            v += ((unsigned long long)o.hi[bin] << 32) + o.lo[bin];
+        }
+        for (uint32_t o = lanes / 2; o; o >>= 1) v += shfl_down_t(v, o);
+        if (r0 == 0) first.tot[bin] = v;
+        barrier();
+    };
+    // first CTA: the bin, counted from the largest, at which base + running mass exceeds X -> S.prefix, S.base, S.found
+    auto find_bin = [&](unsigned long long base, unsigned long long X, uint32_t prefix_above, unsigned long long *total) {
+        const unsigned long long a = S.tot[SAMPLE_BINS - 1 - 2 * tid], b = S.tot[SAMPLE_BINS - 2 - 2 * tid];
+        const unsigned long long upto = base + block_scan(a + b, S, total), before = upto - a - b;
+        if (tid == 0) S.count = 0u;
+        if (X >= before && X < upto) {
+            const bool second = X >= before + a;
+            S.prefix = prefix_above | (SAMPLE_BINS - 1 - 2 * tid - (second ? 1u : 0u));
+            S.base = second ? before + a : before;
+            S.found = 1u;
+        }
+        __syncthreads();
+    };
+
+    gather_bins();
+    unsigned long long X = (unsigned long long)((double)topp * 4503599627370496.0), total = 0ull;
+    uint32_t listed = 0xFFFFFFFFu, listed_m = 0;   // the top-level bin whose elements are in the list, ordered, and their number
+    // Query 0: where the running sum exceeds topp (only that running sum matters: `cum`); query 1: where it exceeds coin * cum.
+    for (int query = 0; query < 2; query++) {
+        if (rank == 0) {
+            find_bin(0ull, X, 0u, &total);
+            if (!S.found && tid == 0) S.cum = total;   // query 0 only: the candidates do not reach topp, all of them are in
+        }
+        barrier();
+        const uint32_t found = first.found;
+        if (query == 0 && !found) {
+            // (no candidate at all - (1 - topp) / (n - 1) above the largest probability, e.g. n = 2 with a small topp: the reference
+            // subtracts 1 from an unsigned zero there (sampler.rs:108); defined here as the arg-max, lowest index on ties)
+            if (first.cum == 0ull) {
+                unsigned long long b = 0ull;
+                for (uint32_t i = tid; i < len; i += SAMPLE_THREADS) {
+                    const unsigned long long k = ((unsigned long long)__float_as_uint(P[i]) << 32) | (0xFFFFFFFFu - (i0 + i));   // p >= 0: bits order like values
+                    b = k > b ? k : b;
+                }
+#pragma unroll
+                for (int o = 16; o; o >>= 1) { const unsigned long long t = __shfl_xor_sync(0xffffffffu, b, o); b = t > b ? t : b; }
+                if (lane == 0) S.red[warp] = b;
+                __syncthreads();
+                if (tid == 0) {
+                    for (int w = 1; w < SAMPLE_WARPS; w++) b = S.red[w] > b ? S.red[w] : b;
+                    first.xu[1][rank] = b;
+                }
+                barrier();
+                if (rank == 0 && tid == 0) {
+                    for (uint32_t r = 0; r < C; r++) b = S.xu[1][r] > b ? S.xu[1][r] : b;
+                    done(0xFFFFFFFFu - (uint32_t)b);
+                }
+                return;
+            }
+        } else {
+            uint32_t shift = SAMPLE_TOP_SHIFT;
+            for (;;) {
+                const uint32_t prefix = first.prefix;
+                const bool have = shift == SAMPLE_TOP_SHIFT && prefix == listed;
+                if (!have) {
+                    // the bin's elements into the first CTA's list
+                    auto in_bin = [&](uint32_t i) {
+                        const float p = P[i];
+                        const uint32_t bits = __float_as_uint(p);
+                        return p >= cutoff && (shift == SAMPLE_TOP_SHIFT ? min(bits >> shift, SAMPLE_BINS - 1) : bits >> shift) == prefix;
+                    };
+                    uint32_t c = 0;
+                    for (uint32_t i = tid; i < len; i += SAMPLE_THREADS) c += in_bin(i);
+                    unsigned long long mine;
+                    const uint32_t at0 = (uint32_t)block_scan(c, S, &mine) - c;
+                    if (tid == 0 && mine) S.slot = atomicAdd(&first.count, (uint32_t)mine);
+                    __syncthreads();
+                    if (c) {
+                        uint32_t at = S.slot + at0;
+                        for (uint32_t i = tid; i < len; i += SAMPLE_THREADS)
+                            if (in_bin(i)) {
+                                if (at < SAMPLE_LIST) first.list[at] = ((unsigned long long)(~__float_as_uint(P[i])) << 32) | (i0 + i);
+                                at++;
+                            }
+                    }
+                    if (tid < C) *cluster.map_shared_rank(&S.xu[1][rank], tid) = mine;
+                    barrier();
+                }
+                const uint32_t m = have ? listed_m : first.count;
+                if (m <= SAMPLE_LIST) {
+                    if (rank == 0) {
+                        uint32_t cap = 1;
+                        while (cap < m) cap <<= 1;
+                        if (!have) {
+                            for (uint32_t i = m + tid; i < cap; i += SAMPLE_THREADS) S.list[i] = ~0ull;
+                            __syncthreads();
+                            sort_list(S.list, cap);
+                        }
+                        const uint32_t per = (m + SAMPLE_THREADS - 1) / SAMPLE_THREADS, a = min(m, tid * per), b = min(m, a + per);
+                        auto q_at = [&](uint32_t i) { return mass_of(__uint_as_float(~(uint32_t)(S.list[i] >> 32))); };
+                        unsigned long long mine = 0ull, all;
+                        for (uint32_t i = a; i < b; i++) mine += q_at(i);
+                        unsigned long long run = S.base + block_scan(mine, S, &all) - mine;
+                        if (X >= run && X < run + mine) {
+                            for (uint32_t i = a; i < b; i++) {
+                                run += q_at(i);
+                                if (X < run) { S.cum = run; S.answer = S.list[i]; break; }
+                            }
+                        }
+                        __syncthreads();
+                        if (query == 1 && tid == 0) done((uint32_t)S.answer);
+                    }
+                    listed = shift == SAMPLE_TOP_SHIFT ? prefix : 0xFFFFFFFFu;
+                    listed_m = m;
+                    break;
+                }
+                if (shift == 0) {
+                    // more equal elements than the list holds: number k of them in index order
+                    const unsigned long long q = mass_of(__uint_as_float(prefix)), b0 = first.base, k = (X - b0) / q;
+                    if (query == 0) {
+                        if (rank == 0 && tid == 0) S.cum = b0 + (k + 1) * q;
+                        barrier();   // (everyone has read the first CTA's words)
+                    } else {
+                        unsigned long long ahead = 0ull, mine;
+                        for (uint32_t r = 0; r < rank; r++) ahead += S.xu[1][r];
+                        const uint32_t per = (len + SAMPLE_THREADS - 1) / SAMPLE_THREADS, a = min(len, tid * per), b = min(len, a + per);
+                        uint32_t c = 0;
+                        for (uint32_t i = a; i < b; i++) c += __float_as_uint(P[i]) == prefix;
+                        unsigned long long at = ahead + block_scan(c, S, &mine) - c;
+                        for (uint32_t i = a; i < b; i++)
+                            if (__float_as_uint(P[i]) == prefix && at++ == k) done(i0 + i);
+                    }
+                    listed = 0xFFFFFFFFu;
+                    break;
+                }
+                // finer bins inside this one
+                const uint32_t next = shift > 11 ? shift - 11 : 0, width = shift - next;
+                for (uint32_t b = tid; b < SAMPLE_BINS; b += SAMPLE_THREADS) { S.lo[b] = 0u; S.hi[b] = 0u; }
+                __syncthreads();
+                for (uint32_t i = tid; i < len; i += SAMPLE_THREADS) {
+                    const float p = P[i];
+                    const uint32_t bits = __float_as_uint(p);
+                    if (p >= cutoff && bits >> shift == prefix) mass_add(S, (bits >> next) & ((1u << width) - 1u), mass_of(p));
+                }
+                gather_bins();
+                if (rank == 0) find_bin(S.base, X, prefix << width, &total);
+                shift = next;
+                barrier();
+            }
+        }
+        if (query == 0) {
+            // the second bound, known to the first CTA; the top-level histogram is needed again if finer ones took its place
+            barrier();
+            X = (unsigned long long)((double)coin * (double)first.cum);
+            if (listed == 0xFFFFFFFFu && found) {
+                for (uint32_t b = tid; b < SAMPLE_BINS; b += SAMPLE_THREADS) { S.lo[b] = 0u; S.hi[b] = 0u; }
+                __syncthreads();
+                for (uint32_t i = tid; i < len; i += SAMPLE_THREADS)
+                    if (P[i] >= cutoff) mass_add(S, min(__float_as_uint(P[i]) >> SAMPLE_TOP_SHIFT, SAMPLE_BINS - 1), mass_of(P[i]));
+                gather_bins();
+            }
+        }
+    }
+    barrier();   // no CTA leaves while another may still read its shared memory
 }
+
+// Scratch a launch needs in global memory (0 for vocabularies whose slices fit shared memory: up to 262144 tokens on clusters of 8)
+size_t sample_scratch_bytes(uint32_t n) { return (n + 7) / 8 <= SAMPLE_SLICE_MAX ? 0 : sizeof(float) * (size_t)n; }
 
 int32_t launch_sample(ib_ctx *ctx, cudaStream_t s, const float *logits, uint32_t n, float temperature, float topp, uint64_t seed, const uint32_t *pos_ptr,
-                      float coin, float *probs, unsigned long long *keys, uint32_t *out, uint32_t *out2, uint32_t pdl) {
-    static bool attr_set[16] = {false};
-    const size_t smem = SAMPLE_SMEM_KEYS * sizeof(unsigned long long);
-    if (!attr_set[ctx->device & 15]) {
-        IB_CHECK_CUDA(cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        attr_set[ctx->device & 15] = true;
-    }
+                      float coin, float *probs, uint32_t *out, uint32_t *out2, uint32_t pdl) {
+    static uint32_t cluster_size[16] = {0};
+    const size_t smem_max = sizeof(SampleShared) + SAMPLE_SLICE_MAX * sizeof(float);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(1);
+    cudaLaunchAttribute attr[2];
     cfg.blockDim = dim3(SAMPLE_THREADS);
-    cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl ? 1 : 0;
-    IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, sample_kernel, logits, n, temperature, topp, seed, pos_ptr, coin, probs, keys, out, out2, pdl));
+    uint32_t &C = cluster_size[ctx->device & 15];
+    if (!C) {
+        IB_CHECK_CUDA(cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_max));
+        IB_CHECK_CUDA(cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        // 16 CTAs of one cluster have to fit one graphics-processing cluster of the device
+        int fit = 0;
+        attr[0].val.clusterDim.x = SAMPLE_MAX_CLUSTER;
+        cfg.gridDim = dim3(SAMPLE_MAX_CLUSTER);
+        cfg.numAttrs = 1;
+        cfg.dynamicSmemBytes = smem_max;
+        C = (cudaOccupancyMaxActiveClusters(&fit, sample_kernel, &cfg) == cudaSuccess && fit > 0) ? SAMPLE_MAX_CLUSTER : 8u;
+        cudaGetLastError();
+    }
+    const uint32_t slice = (n + C - 1) / C;
+    attr[0].val.clusterDim.x = C;
+    cfg.gridDim = dim3(C);
+    cfg.dynamicSmemBytes = sizeof(SampleShared) + (probs ? 0 : slice * sizeof(float));
+    cfg.numAttrs = pdl ? 2 : 1;
+    IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, sample_kernel, logits, n, slice, temperature, topp, seed, pos_ptr, coin, probs, out, out2, pdl));
     ctx->launches++;
     return IB_OK;
-}
-
-size_t sample_keys_capacity(uint32_t n) {
-    size_t cap = 1;
-    while (cap < n) cap <<= 1;
-    return cap;
 }
 
 }  // namespace ib
@@ -257,12 +464,11 @@ extern "C" int32_t ib_sample(ib_ctx *ctx, void *stream, const float *logits_dev,
     IB_REQUIRE(coin >= 0.f && coin < 1.f, "ib_sample: coin=%f outside [0, 1)", (double)coin);
     IB_REQUIRE(temperature >= 0.f, "ib_sample: negative temperature");
     if (temperature == 0.f) return launch_argmax(ctx, (cudaStream_t)stream, logits_dev, n, out_dev);   // sampler.rs:33-35
-    // one stream-ordered allocation for both scratch arrays (probabilities, then the sort keys, 8-byte aligned)
-    const size_t probs_bytes = (sizeof(float) * n + 7) & ~(size_t)7;
-    uint8_t *scratch = nullptr;
-    IB_CHECK_CUDA(cudaMallocAsync((void **)&scratch, probs_bytes + sizeof(unsigned long long) * sample_keys_capacity(n), (cudaStream_t)stream));
-    const int32_t rc = launch_sample(ctx, (cudaStream_t)stream, logits_dev, n, temperature, topp, 0, nullptr, coin, reinterpret_cast<float *>(scratch),
-                                     reinterpret_cast<unsigned long long *>(scratch + probs_bytes), out_dev, nullptr, 0);
-    cudaFreeAsync(scratch, (cudaStream_t)stream);
+    // stream-ordered scratch for the vocabularies that need it
+    float *scratch = nullptr;
+    const size_t bytes = sample_scratch_bytes(n);
+    if (bytes) IB_CHECK_CUDA(cudaMallocAsync((void **)&scratch, bytes, (cudaStream_t)stream));
+    const int32_t rc = launch_sample(ctx, (cudaStream_t)stream, logits_dev, n, temperature, topp, 0, nullptr, coin, scratch, out_dev, nullptr, 0);
+    if (scratch) cudaFreeAsync(scratch, (cudaStream_t)stream);
     return rc;
 }

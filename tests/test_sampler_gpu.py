@@ -87,6 +87,14 @@ def test_flat_and_tied_distributions(backend):
         assert gpu_sample(backend, tied, 1.0, 0.9, coin) == oracle.sample(tied, 1.0, 0.9, coin)[0]
 
 
+@pytest.mark.parametrize("n,step", [(4097, 0.0), (40000, 0.0), (128256, 1e-6), (262145, 0.0)])
+def test_bins_with_more_elements_than_the_list(backend, n, step):
+    """All (or all but rounding) probabilities equal: the crossing's bin overflows the list at every level and its elements are taken in index
+    order; 262145 tokens no longer fit shared memory."""
+    logits = (np.arange(n, dtype=np.float32) % 7) * np.float32(step)
+    check_many(backend, logits, 1.0, 0.9, np.float32([0.0, 0.37, 0.999999]))
+
+
 def test_temperature_zero_is_argmax_and_contract(backend):
     x = np.float32([0.1, 3.0, -1.0, 3.0, 2.0])
     assert gpu_sample(backend, x, 0.0, 0.9, 0.5) == 1                   # greedy, lowest index on ties
