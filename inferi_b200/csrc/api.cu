@@ -244,6 +244,7 @@ int32_t ib_gemv_quant(ib_ctx *ctx, void *stream, float *out_dev, const ib_qtenso
     GemvParams p = {};
     fill_seg(p.seg[0], m, out_dev);
     p.nseg = 1; p.cols = (uint32_t)m->cols; p.epi = EPI_STORE; p.x = v_dev;
+    p.pdl = 1;   // ahead of its wait for the stream's previous kernel the GEMV reads only the matrix, which no kernel of a stream writes
     return launch_gemv(ctx, (cudaStream_t)stream, p);
 }
 
@@ -258,6 +259,7 @@ int32_t ib_ffn_gate_up(ib_ctx *ctx, void *stream, float *out_dev, const ib_qtens
     fill_seg(p.seg[0], gate, out_dev);
     fill_seg(p.seg[1], up, nullptr);
     p.nseg = 2; p.cols = (uint32_t)gate->cols; p.epi = EPI_SWIGLU; p.x = x_dev; p.norm_w = norm_w_dev; p.eps = eps;
+    p.pdl = norm_w_dev == nullptr;   // the norm weights are read ahead of the wait: only where they cannot be the previous kernel's output
     return launch_gemv(ctx, (cudaStream_t)stream, p);
 }
 
@@ -340,6 +342,7 @@ int32_t ib_attention(ib_ctx *ctx, void *stream, const ib_attn_params *params, co
     IB_REQUIRE(params->n_heads / params->kv_mul <= 1024, "ib_attention: too many kv heads");
     a.q = q_dev; a.k_cache = k_cache_dev; a.v_cache = v_cache_dev; a.kv_dtype = kv_dtype; a.out = out_dev;
     a.scratch = ctx->attn_scratch; a.counters = ctx->attn_counters;
+    a.pdl = 2;
     return launch_attention(ctx, (cudaStream_t)stream, a);
 }
 

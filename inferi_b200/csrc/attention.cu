@@ -21,6 +21,7 @@ template <int HS, int KVM, typename T>
 __global__ void __launch_bounds__(ATTN_THREADS) attn_kernel(const AttnArgs a) {
     __shared__ float sm[attn_block_smem_floats(HS, KVM)];
     if (a.pdl) asm volatile("griddepcontrol.launch_dependents;");
+    if (a.pdl == 2) asm volatile("griddepcontrol.wait;" ::: "memory");
     // The position was written by the end of the previous token, many kernels ago, and not by the predecessor (which
     // only waits for its own predecessor after it has let this kernel start): it can be read before the wait.
     const uint32_t kvh = blockIdx.x, split = blockIdx.y;
@@ -28,7 +29,7 @@ __global__ void __launch_bounds__(ATTN_THREADS) attn_kernel(const AttnArgs a) {
     uint32_t nsplit, per;
     attn_split_plan(pos + 1, a.max_splits, nsplit, per);
     if (split >= nsplit) return;
-    attn_block<HS, KVM, T, ATTN_STEPS>(a, a.kc, a.vc, kvh, split, nsplit, per, pos + 1, (int)threadIdx.x, 1, sm, a.pdl != 0);
+    attn_block<HS, KVM, T, ATTN_STEPS>(a, a.kc, a.vc, kvh, split, nsplit, per, pos + 1, (int)threadIdx.x, 1, sm, a.pdl == 1);
 }
 
 size_t attn_scratch_bytes(const ib_attn_params &p, uint32_t max_splits) {
@@ -206,5 +207,6 @@ extern "C" int32_t ib_attention_static(void *stream, const ib_attn_params *param
     a.scratch = g_static_scratch_addr[dev];
     a.counters = g_static_counters_addr[dev];   // zero when the library is loaded; the kernel puts every counter back to zero
     a.max_splits = splits;
+    a.pdl = 2;
     return launch_attention(&local, (cudaStream_t)stream, a);
 }

@@ -101,6 +101,8 @@ __global__ void __launch_bounds__(ATTN_THREADS, 3) attn_gqa4_kernel(const AttnAr
     __shared__ __align__(16) float sm_cl[GQA4_CLUSTER_MAX * KVM * (HS + 2)];   // cluster mode: the slices' partials, in the first CTA
 
     if (a.pdl) asm volatile("griddepcontrol.launch_dependents;");
+    const bool early = a.pdl == 1;   // rows may be requested ahead of the wait
+    if (a.pdl == 2) asm volatile("griddepcontrol.wait;" ::: "memory");
     // The position was written at the end of the previous token, not by the predecessor: it can be read before the wait.
     const uint32_t kvh = blockIdx.x, split = blockIdx.y;
     const uint32_t total = (a.pos_ptr ? *a.pos_ptr : a.p.pos) + 1;
@@ -131,13 +133,13 @@ __global__ void __launch_bounds__(ATTN_THREADS, 3) attn_gqa4_kernel(const AttnAr
 #pragma unroll
         for (int s = 0; s < STEPS; s++) {
             const uint32_t t = base0 + s * RPW + g, tc = t < t1 ? t : t1 - 1;
-            if (tc + 1 != total || !a.pdl) {
+            if (tc + 1 != total || !early) {
                 kraw[s] = __ldcg(reinterpret_cast<const uint4 *>(kc + (size_t)tc * kv_dim));
                 vraw[s] = __ldcg(reinterpret_cast<const uint4 *>(vc + (size_t)tc * kv_dim));
             }
         }
     }
-    if (a.pdl) {
+    if (early) {
         asm volatile("griddepcontrol.wait;" ::: "memory");
         if (base0 < t1) {
 #pragma unroll

@@ -207,7 +207,8 @@ struct AttnLaunch {
     float *scratch;            // [n_kv_heads][max_splits][kv_mul][head_size + 2]
     unsigned int *counters;    // [n_kv_heads], zero before the first launch; the kernel re-zeroes them
     uint32_t max_splits;
-    uint32_t pdl;
+    uint32_t pdl;              // 0: plain launch; 1: programmatic dependent launch inside the token graph, where the predecessor writes only q and the
+                               // newest cache row; 2: programmatic dependent launch behind any kernel
     // With pos_ptr (a graph node that serves many positions): the caller promises that the position stays below
     // attn_cluster_positions(); the launch then groups a kv head's slices into a thread-block cluster and merges them there.
     // Such a launch is slower at long contexts (clusters constrain the placement of the grid's one wave of CTAs), so a graph

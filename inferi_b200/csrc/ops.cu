@@ -1,42 +1,74 @@
 // Stand-alone element-wise ops of the token loop (RMSNorm, RoPE, SwiGLU, residual add, arg-max).
 // Inside the model these are fused into GEMV prologues/epilogues; the stand-alone kernels serve the
 // op-level API that mirrors crates/inferi/src/ops/{rms_norm,rope,silu}.rs and context.rs:516-530.
+//
+// All of them are launched with programmatic dependent launch: each lets its successor start at once and waits for its
+// predecessor before it touches an operand, so that in a chain of op calls the next kernel's launch and set-up overlap the
+// previous kernel's tail (worth 1-2 us per launch where a kernel itself takes 2 us).
 #include "common.cuh"
 
 #include <math.h>
 
 namespace ib {
 
+__device__ __forceinline__ void pdl_enter() {
+    asm volatile("griddepcontrol.launch_dependents;");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename... KArgs, typename... Args>
+static int32_t launch_op(ib_ctx *ctx, cudaStream_t s, void (*kernel)(KArgs...), uint32_t grid, uint32_t block, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.stream = s;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, (KArgs)args...));
+    ctx->launches++;
+    return IB_OK;
+}
+
 // ---- RMSNorm: crates/inferi-shaders/src/rms_norm.rs:78-121 ----
-__global__ void __launch_bounds__(1024) rms_norm_kernel(float *__restrict__ out, const float *__restrict__ x, const float *__restrict__ w, uint32_t n,
-                                                        float eps) {
-    __shared__ float red[33];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5;
-    float ss = 0.f;
-    for (uint32_t i = tid; i < n; i += blockDim.x) {
-        const float v = x[i];
-        ss += v * v;
+// One CTA; latency bound (one load, a block reduction, one store).  The first RMS_KEEP values of a thread stay in registers,
+// so the vector is read once and the loads of x and w are all in flight together.
+constexpr uint32_t RMS_KEEP = 4;
+__global__ void __launch_bounds__(1024) rms_norm_kernel(float *out, const float *x, const float *w, uint32_t n, float eps) {
+    __shared__ float red[32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nwarps = blockDim.x >> 5, step = blockDim.x;
+    pdl_enter();
+    float v[RMS_KEEP], g[RMS_KEEP];
+#pragma unroll
+    for (uint32_t k = 0; k < RMS_KEEP; k++) {
+        const uint32_t i = tid + k * step;
+        v[k] = i < n ? x[i] : 0.f;
+        g[k] = i < n ? w[i] : 0.f;
     }
+    float ss = 0.f;
+#pragma unroll
+    for (uint32_t k = 0; k < RMS_KEEP; k++) ss += v[k] * v[k];
+    for (uint32_t i = tid + RMS_KEEP * step; i < n; i += step) ss += x[i] * x[i];
 #pragma unroll
     for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
     if (lane == 0) red[warp] = ss;
     __syncthreads();
-    if (tid == 0) {
-        float t = 0.f;
-        for (int i = 0; i < nwarps; i++) t += red[i];
-        red[32] = 1.0f / sqrtf(t / (float)n + eps);
+    float t = lane < nwarps ? red[lane] : 0.f;
+#pragma unroll
+    for (int o = 16; o; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    const float rms = 1.0f / sqrtf(t / (float)n + eps);
+#pragma unroll
+    for (uint32_t k = 0; k < RMS_KEEP; k++) {
+        const uint32_t i = tid + k * step;
+        if (i < n) out[i] = (v[k] * rms) * g[k];
     }
-    __syncthreads();
-    const float rms = red[32];
-    for (uint32_t i = tid; i < n; i += blockDim.x) out[i] = (x[i] * rms) * w[i];
+    for (uint32_t i = tid + RMS_KEEP * step; i < n; i += step) out[i] = (x[i] * rms) * w[i];
 }
 
 int32_t launch_rms_norm(ib_ctx *ctx, cudaStream_t s, float *out, const float *x, const float *w, uint32_t n, float eps) {
-    const int threads = n >= 4096 ? 1024 : (n >= 1024 ? 512 : 128);
-    rms_norm_kernel<<<1, threads, 0, s>>>(out, x, w, n, eps);
-    ctx->launches++;
-    IB_CHECK_CUDA(cudaGetLastError());
-    return IB_OK;
+    return launch_op(ctx, s, rms_norm_kernel, 1, n >= 2048 ? 1024 : (n >= 1024 ? 512 : 128), out, x, w, n, eps);
 }
 
 // ---- RoPE: crates/inferi-shaders/src/rope.rs:51-92 (Original), :97-141 (NeoX) ----
@@ -44,9 +76,10 @@ int32_t launch_rms_norm(ib_ctx *ctx, cudaStream_t s, float *out, const float *x,
 // powf and passed by value, so that device and host agree on them bit for bit.
 struct RopeTheta { float t[128]; };
 
-__global__ void rope_kernel(int variant, float *__restrict__ q, uint32_t q_len, float *__restrict__ k, uint32_t kv_dim, uint32_t head_size, uint32_t pos,
+__global__ void rope_kernel(int variant, float *q, uint32_t q_len, float *k, uint32_t kv_dim, uint32_t head_size, uint32_t pos,
                             const RopeTheta th) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_enter();
     if (i >= q_len / 2) return;
     const uint32_t half = head_size / 2;
     uint32_t i0, i1, j;
@@ -69,37 +102,30 @@ int32_t launch_rope(ib_ctx *ctx, cudaStream_t s, int variant, float *q, uint32_t
     RopeTheta th;
     for (uint32_t j = 0; j < head_size / 2; j++) th.t[j] = powf(base_freq, -(float)(2 * j) / (float)head_size);
     const uint32_t n = q_len / 2;
-    rope_kernel<<<(n + 127) / 128, 128, 0, s>>>(variant, q, q_len, k, kv_dim, head_size, pos, th);
-    ctx->launches++;
-    IB_CHECK_CUDA(cudaGetLastError());
-    return IB_OK;
+    return launch_op(ctx, s, rope_kernel, (n + 127) / 128, 128, variant, q, q_len, k, kv_dim, head_size, pos, th);
 }
 
 // ---- SwiGLU: crates/inferi-shaders/src/silu.rs:24-53 ----
-__global__ void silu_mul_kernel(float *__restrict__ h1, const float *__restrict__ h2, uint32_t n) {
+__global__ void silu_mul_kernel(float *h1, const float *h2, uint32_t n) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_enter();
     if (i < n) {
         const float a = h1[i];
         h1[i] = h2[i] * (a / (1.0f + expf(-a)));
     }
 }
 int32_t launch_silu_mul(ib_ctx *ctx, cudaStream_t s, float *h1, const float *h2, uint32_t n) {
-    silu_mul_kernel<<<(n + 255) / 256, 256, 0, s>>>(h1, h2, n);
-    ctx->launches++;
-    IB_CHECK_CUDA(cudaGetLastError());
-    return IB_OK;
+    return launch_op(ctx, s, silu_mul_kernel, (n + 255) / 256, 256, h1, h2, n);
 }
 
 // ---- residual add: crates/inferi/src/context.rs:516-530 ----
-__global__ void add_assign_kernel(float *__restrict__ a, const float *__restrict__ b, uint32_t n) {
+__global__ void add_assign_kernel(float *a, const float *b, uint32_t n) {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    pdl_enter();
     if (i < n) a[i] += b[i];
 }
 int32_t launch_add_assign(ib_ctx *ctx, cudaStream_t s, float *a, const float *b, uint32_t n) {
-    add_assign_kernel<<<(n + 255) / 256, 256, 0, s>>>(a, b, n);
-    ctx->launches++;
-    IB_CHECK_CUDA(cudaGetLastError());
-    return IB_OK;
+    return launch_op(ctx, s, add_assign_kernel, (n + 255) / 256, 256, a, b, n);
 }
 
 // ---- greedy arg-max: crates/inferi/src/models/sampler.rs:54-56; lowest index on ties ----
@@ -111,11 +137,12 @@ __device__ __forceinline__ unsigned long long amax_key(float v, uint32_t idx) {
 
 constexpr int ARGMAX_MAX_CTAS = 1024;
 
-__global__ void __launch_bounds__(256) argmax_kernel(const float *__restrict__ x, uint32_t n, unsigned long long *slots, unsigned int *counter, uint32_t *out) {
+__global__ void __launch_bounds__(256) argmax_kernel(const float *x, uint32_t n, unsigned long long *slots, unsigned int *counter, uint32_t *out) {
     __shared__ unsigned long long sm[8];
     __shared__ bool is_last;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     unsigned long long best = 0ull;
+    pdl_enter();
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) best = max(best, amax_key(x[i], i));
 #pragma unroll
     for (int o = 16; o; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
@@ -160,10 +187,7 @@ int32_t launch_argmax(ib_ctx *ctx, cudaStream_t s, const float *x, uint32_t n, u
     int grid = (int)((n + 1023) / 1024);
     if (grid > ctx->sm_count * 2) grid = ctx->sm_count * 2;
     if (grid < 1) grid = 1;
-    argmax_kernel<<<grid, 256, 0, s>>>(x, n, ctx->argmax_scratch, ctx->argmax_counter, out);
-    ctx->launches++;
-    IB_CHECK_CUDA(cudaGetLastError());
-    return IB_OK;
+    return launch_op(ctx, s, argmax_kernel, (uint32_t)grid, 256, x, n, ctx->argmax_scratch, ctx->argmax_counter, out);
 }
 
 }  // namespace ib

@@ -18,14 +18,21 @@ from ._lib import AttnParams, InferiError, KV_F16, KV_F32, ROPE_NEOX, ROPE_ORIGI
 from .quant import BLOCK_BYTES, BLOCK_ELEMS, F32, NAMES, Q4_K, Q5_K, Q6_K, Q8_0, row_bytes  # noqa: F401
 
 
+_f32, _tensor = torch.float32, torch.Tensor
+_current_device, _raw_stream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+
+
 def _stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+    """The current device's current stream as an integer, without building a `torch.cuda.Stream` object per call (3.2 us against 0.15)."""
+    if not torch.cuda.is_initialized():
+        return torch.cuda.current_stream().cuda_stream
+    return _raw_stream(_current_device())
 
 
 def _f32_dev(t: torch.Tensor, name: str) -> int:
-    if not (isinstance(t, torch.Tensor) and t.is_cuda and t.dtype == torch.float32 and t.is_contiguous()):
-        raise InferiError(1, f"{name}: expected a contiguous float32 CUDA tensor")
-    return t.data_ptr()
+    if isinstance(t, _tensor) and t.dtype is _f32 and t.is_cuda and t.is_contiguous():
+        return t.data_ptr()
+    raise InferiError(1, f"{name}: expected a contiguous float32 CUDA tensor")
 
 
 class Backend:
