@@ -136,15 +136,17 @@ struct ib_llama {
     float *sample_probs = nullptr;   // only for vocabularies that the sampler cannot hold in shared memory
     cudaGraphExec_t graph_exec_sample = nullptr;
     uint64_t launches_per_token_sample = 0;
-    // prompt prefill (ib_llama_prefill): buffers for up to PREFILL_MAX_TOKENS tokens at a time, allocated at the first call
+    // prompt prefill (ib_llama_prefill): one allocation for passes of up to `chunks` chunks of PF_CHUNK tokens, made at the
+    // first call and again by a call with a longer prompt
     struct PrefillBuffers {
-        float *X = nullptr, *q = nullptr, *att = nullptr, *planes = nullptr, *planes2 = nullptr, *attn_scratch = nullptr;
+        uint8_t *arena = nullptr;
+        uint32_t chunks = 0;
+        float *X = nullptr, *q = nullptr, *att = nullptr, *planes = nullptr, *attn_scratch = nullptr;
         __half *hi = nullptr, *lo = nullptr;
         uint32_t *tokens = nullptr;
         unsigned int *attn_counters = nullptr;
         uint32_t attn_splits = 0;
         size_t attn_scratch_step = 0;
-        bool ready = false;
     } pf;
     // tensors and device vectors the model owns (a model loaded from a GGUF file frees its weights with itself)
     std::vector<ib_qtensor *> owned_tensors;
@@ -404,9 +406,7 @@ int32_t ib_llama_destroy(ib_llama *m) {
     if (m->staged) cudaEventDestroy(m->staged);
     for (int r = 0; r < m->tp_size && r < IB_MAX_TP; r++)
         if (m->peers_mapped_by_ipc && m->comm_peer[r] && m->comm_peer[r] != m->comm) cudaIpcCloseMemHandle(m->comm_peer[r]);
-    void *pbufs[] = {m->pf.X, m->pf.q, m->pf.att, m->pf.planes, m->pf.planes2, m->pf.attn_scratch, m->pf.hi, m->pf.lo, m->pf.tokens, m->pf.attn_counters};
-    for (void *b : pbufs)
-        if (b) cudaFree(b);
+    if (m->pf.arena) cudaFree(m->pf.arena);
     void *bufs[] = {m->x, m->xb, m->q, m->hb, m->logits, m->theta, m->rope_cs, m->ctl, m->seq, m->attn_scratch, m->attn_counters, m->argmax_slots,
                     m->argmax_counter, m->x2, m->comm, m->epoch, m->reduce_done};
     for (void *b : bufs)
@@ -741,33 +741,67 @@ int32_t ib_llama_forward(ib_llama *m, void *stream, uint32_t token, uint32_t pos
 }
 
 // ---- prompt prefill on the tensor cores ----
-static int32_t prefill_prepare(ib_llama *m) {
-    if (m->pf.ready) return IB_OK;
+// The GEMM launches of a layer: matrices that follow one another, read the same inputs and have the same type share one.
+struct PrefillGroup {
+    const ib_qtensor *mats[PF_MAX_SEGS];
+    uint32_t n_mats, rows, cols;
+};
+static uint32_t prefill_groups(const ib_qtensor *const *mats, uint32_t n, PrefillGroup *out) {
+    uint32_t g = 0;
+    for (uint32_t i = 0; i < n; i++) {
+        if (i == 0 || mats[i]->qtype != mats[i - 1]->qtype) out[g++] = PrefillGroup{{nullptr}, 0, 0, (uint32_t)mats[i]->cols};
+        PrefillGroup &p = out[g - 1];
+        p.mats[p.n_mats++] = mats[i];
+        p.rows += (uint32_t)mats[i]->rows;
+    }
+    return g;
+}
+// floats of a launch's planes for a pass of n tokens
+static size_t prefill_plane_floats(const ib_ctx *ctx, const PrefillGroup &g, uint32_t n) {
+    return (size_t)prefill_max_pieces(prefill_streamk(ctx, g.rows, g.cols, n)) * n * g.rows;
+}
+
+static int32_t prefill_prepare(ib_llama *m, uint32_t n) {
+    const uint32_t chunks = ((n < PREFILL_MAX_TOKENS ? n : PREFILL_MAX_TOKENS) + PF_CHUNK - 1) / PF_CHUNK;
+    auto &B = m->pf;
+    if (chunks <= B.chunks) return IB_OK;
     const ib_llama_config &c = m->cfg;
-    const uint32_t H = c.hidden_size, F = m->ffn_l, Q = m->q_dim_l, KV = m->kv_dim_l, N = PREFILL_MAX_TOKENS;
+    const uint32_t H = c.hidden_size, F = m->ffn_l, Q = m->q_dim_l, KV = m->kv_dim_l, N = chunks * PF_CHUNK;
     const uint32_t widest = F > H ? (F > Q ? F : Q) : (H > Q ? H : Q);
-    size_t plane_elems = 0;   // largest planes * rows over the matrices (per token)
-    const ib_llama_layer_weights &w = m->layers[0];
-    const ib_qtensor *mats[] = {w.attn_q, w.attn_k, w.attn_v, w.attn_output, w.ffn_gate, w.ffn_up, w.ffn_down};
-    for (const ib_qtensor *t : mats) {
-        const size_t e = (size_t)prefill_max_pieces(prefill_streamk(m->ctx, (uint32_t)t->rows, (uint32_t)t->cols), (uint32_t)t->rows) * t->rows;
-        if (e > plane_elems) plane_elems = e;
+    size_t planes = 0;   // the largest result that is alive at once, over the layers and over the passes' lengths
+    for (const ib_llama_layer_weights &w : m->layers) {
+        const ib_qtensor *sets[4][3] = {{w.attn_q, w.attn_k, w.attn_v}, {w.attn_output}, {w.ffn_gate, w.ffn_up}, {w.ffn_down}};
+        const uint32_t counts[4] = {3, 1, 2, 1};
+        for (int k = 0; k < 4; k++)
+            for (uint32_t ch = 1; ch <= chunks; ch++) {
+                PrefillGroup g[3];
+                size_t sum = 0;
+                for (uint32_t i = 0, ng = prefill_groups(sets[k], counts[k], g); i < ng; i++) sum += prefill_plane_floats(m->ctx, g[i], ch * PF_CHUNK);
+                planes = sum > planes ? sum : planes;
+            }
     }
     ib_attn_params ap{c.max_position_embeddings, KV, c.num_attention_heads / c.num_key_value_heads, m->n_heads_l, m->head_size, 0};
-    m->pf.attn_splits = 16;   // per query; the queries of a prompt fill the GPU between them
-    m->pf.attn_scratch_step = attn_scratch_bytes(ap, m->pf.attn_splits) / sizeof(float);
-    IB_CHECK_CUDA(cudaMalloc(&m->pf.X, sizeof(float) * N * H));
-    IB_CHECK_CUDA(cudaMalloc(&m->pf.q, sizeof(float) * N * Q));
-    IB_CHECK_CUDA(cudaMalloc(&m->pf.att, sizeof(float) * N * Q));
-    IB_CHECK_CUDA(cudaMalloc(&m->pf.hi, sizeof(__half) * (N + 8) * widest));   // the inputs' tiles + the tiles of their sub-block sums
-    IB_CHECK_CUDA(cudaMalloc(&m->pf.lo, sizeof(__half) * (N + 8) * widest));
-    IB_CHECK_CUDA(cudaMalloc(&m->pf.planes, sizeof(float) * N * plane_elems));
-    IB_CHECK_CUDA(cudaMalloc(&m->pf.planes2, sizeof(float) * N * plane_elems));
-    IB_CHECK_CUDA(cudaMalloc(&m->pf.tokens, sizeof(uint32_t) * N));
-    IB_CHECK_CUDA(cudaMalloc(&m->pf.attn_scratch, sizeof(float) * N * m->pf.attn_scratch_step));
-    IB_CHECK_CUDA(cudaMalloc(&m->pf.attn_counters, sizeof(unsigned int) * N * m->n_kv_l));
-    IB_CHECK_CUDA(cudaMemset(m->pf.attn_counters, 0, sizeof(unsigned int) * N * m->n_kv_l));
-    m->pf.ready = true;
+    B.attn_splits = 16;   // per query; the queries of a prompt fill the GPU between them
+    B.attn_scratch_step = attn_scratch_bytes(ap, B.attn_splits) / sizeof(float);
+    if (B.arena) {   // growing: wait for work that may still use the old one
+        IB_CHECK_CUDA(cudaDeviceSynchronize());
+        IB_CHECK_CUDA(cudaFree(B.arena));
+        B.arena = nullptr;
+        B.chunks = 0;
+    }
+    size_t total = 0;
+    auto place = [&](size_t bytes) { const size_t at = total; total += (bytes + 255) & ~(size_t)255; return at; };
+    const size_t oX = place(sizeof(float) * N * H), oq = place(sizeof(float) * N * Q), oatt = place(sizeof(float) * N * Q);
+    const size_t ohi = place(sizeof(__half) * chunks * pf_x_halves(widest)), olo = place(sizeof(__half) * chunks * pf_x_halves(widest));
+    const size_t opl = place(sizeof(float) * planes), otok = place(sizeof(uint32_t) * N), osc = place(sizeof(float) * PF_CHUNK * B.attn_scratch_step);
+    const size_t octr = place(sizeof(unsigned int) * PF_CHUNK * m->n_kv_l);
+    IB_CHECK_CUDA(cudaMalloc(&B.arena, total));
+    B.X = (float *)(B.arena + oX); B.q = (float *)(B.arena + oq); B.att = (float *)(B.arena + oatt);
+    B.hi = (__half *)(B.arena + ohi); B.lo = (__half *)(B.arena + olo); B.planes = (float *)(B.arena + opl); B.tokens = (uint32_t *)(B.arena + otok);
+    B.attn_scratch = (float *)(B.arena + osc); B.attn_counters = (unsigned int *)(B.arena + octr);
+    IB_CHECK_CUDA(cudaMemset(B.attn_counters, 0, sizeof(unsigned int) * PF_CHUNK * m->n_kv_l));
+    IB_CHECK_CUDA(cudaDeviceSynchronize());
+    B.chunks = chunks;
     return IB_OK;
 }
 
@@ -791,60 +825,67 @@ int32_t ib_llama_prefill(ib_llama *m, void *stream, const uint32_t *tokens_host,
                 return set_error(IB_ERR_UNSUPPORTED, "ib_llama_prefill: a %llux%llu matrix of type %d is outside the tensor-core path; use ib_llama_generate",
                                  (unsigned long long)t->rows, (unsigned long long)t->cols, t->qtype);
     }
-    int32_t rc = prefill_prepare(m);
+    int32_t rc = prefill_prepare(m, n);
     if (rc) return rc;
     cudaStream_t s = (cudaStream_t)stream;
-    const uint32_t H = c.hidden_size, F = m->ffn_l, Q = m->q_dim_l, KV = m->kv_dim_l;
+    const uint32_t H = c.hidden_size, Q = m->q_dim_l, KV = m->kv_dim_l;
     auto &B = m->pf;
-    auto gemm = [&](const ib_qtensor *w, uint32_t nc, float *planes, StreamK &ks) -> int32_t {
-        ks = prefill_streamk(ctx, (uint32_t)w->rows, (uint32_t)w->cols);
-        return launch_prefill_gemm(ctx, s, w, B.hi, B.lo, nc, planes, ks);
+    // the GEMMs of `mats` (same inputs) into planes that follow one another; g / row0: where each matrix's rows are
+    auto gemm = [&](const ib_qtensor *const *mats, uint32_t count, uint32_t nc, PfPlanes *g, uint32_t *row0) -> int32_t {
+        PrefillGroup groups[3];
+        const uint32_t ng = prefill_groups(mats, count, groups);
+        float *at = B.planes;
+        for (uint32_t i = 0, k = 0; i < ng; i++) {
+            const PrefillGroup &p = groups[i];
+            const StreamK sk = prefill_streamk(ctx, p.rows, p.cols, nc);
+            const PfPlanes pl{at, at + (size_t)nc * p.rows, sk, p.rows, (nc + PF_CHUNK - 1) / PF_CHUNK, nc};
+            const int32_t r = launch_prefill_gemm(ctx, s, p.mats, p.n_mats, B.hi, B.lo, nc, at, at + (size_t)nc * p.rows, sk);
+            if (r) return r;
+            for (uint32_t j = 0, row = 0; j < p.n_mats; row += (uint32_t)p.mats[j]->rows, j++, k++) { g[k] = pl; row0[k] = row; }
+            at += prefill_plane_floats(ctx, p, nc);
+        }
+        return IB_OK;
     };
 #define PF(expr) do { if ((rc = (expr)) != IB_OK) return rc; } while (0)
     for (uint32_t t0 = 0; t0 < n; t0 += PREFILL_MAX_TOKENS) {
         const uint32_t nc = n - t0 < PREFILL_MAX_TOKENS ? n - t0 : PREFILL_MAX_TOKENS, pos0 = start_pos + t0;
         IB_CHECK_CUDA(cudaMemcpyAsync(B.tokens, tokens_host + t0, sizeof(uint32_t) * nc, cudaMemcpyHostToDevice, s));
         PF(launch_prefill_embed(ctx, s, m->token_embd, B.tokens, nc, c.vocab_size, B.X));
+        PfPlanes g[3];
+        uint32_t row0[3];
         for (uint32_t l = 0; l < c.num_hidden_layers; l++) {
             const ib_llama_layer_weights &w = m->layers[l];
-            StreamK ks = {};
-            PrefillEpiParams e = {};
-            e.n = nc; e.theta = m->theta; e.head_size = m->head_size; e.pos0 = pos0; e.kv_dim = KV; e.kv_dtype = (uint32_t)m->kv_dtype;
-            // q, k, v: RMSNorm, GEMM, bias, RoPE, cache append (transformer.rs:420-445)
-            PF(launch_prefill_norm_split(ctx, s, B.X, w.attn_norm_dev, c.rms_norm_eps, nc, H, B.hi, B.lo));
-            PF(gemm(w.attn_q, nc, B.planes, ks));
-            e.planes = B.planes; e.sk = ks; e.rows = Q; e.mode = PE_Q; e.bias = w.attn_q_bias_dev; e.out = B.q;
-            PF(launch_prefill_epilogue(ctx, s, e));
-            PF(gemm(w.attn_k, nc, B.planes, ks));
-            e.sk = ks; e.rows = KV; e.mode = PE_K; e.bias = w.attn_k_bias_dev; e.cache = m->k_cache[l];
-            PF(launch_prefill_epilogue(ctx, s, e));
-            PF(gemm(w.attn_v, nc, B.planes, ks));
-            e.sk = ks; e.mode = PE_V; e.bias = w.attn_v_bias_dev; e.cache = m->v_cache[l];
-            PF(launch_prefill_epilogue(ctx, s, e));
-            // causal attention: query t over positions 0 .. pos0 + t (transformer.rs:448), all queries in one launch
-            AttnLaunch a = {};
-            a.p = ib_attn_params{c.max_position_embeddings, KV, kv_mul, m->n_heads_l, m->head_size, pos0};
-            a.q = B.q; a.k_cache = m->k_cache[l]; a.v_cache = m->v_cache[l]; a.kv_dtype = m->kv_dtype; a.out = B.att;
-            a.scratch = B.attn_scratch; a.counters = B.attn_counters; a.max_splits = B.attn_splits;
-            a.n_queries = nc; a.q_step = Q; a.out_step = Q; a.counter_step = m->n_kv_l; a.scratch_step = B.attn_scratch_step;
-            if (nc > 1 && !attn_gqa4_eligible(a)) return set_error(IB_ERR_UNSUPPORTED, "ib_llama_prefill: head size %u is outside the batched attention kernel; use ib_llama_generate", m->head_size);
-            PF(launch_attention(ctx, s, a));
-            // o_proj + residual (transformer.rs:450-453)
-            PF(launch_prefill_norm_split(ctx, s, B.att, nullptr, 0.f, nc, Q, B.hi, B.lo));
-            PF(gemm(w.attn_output, nc, B.planes, ks));
-            e.sk = ks; e.rows = H; e.mode = PE_RESIDUAL; e.bias = nullptr; e.out = B.X;
-            PF(launch_prefill_epilogue(ctx, s, e));
+            // q, k, v: (the previous layer's residual,) RMSNorm, GEMM, bias, RoPE, cache append (transformer.rs:420-445)
+            PF(launch_prefill_norm_split(ctx, s, B.X, l ? &g[0] : nullptr, w.attn_norm_dev, c.rms_norm_eps, nc, H, B.hi, B.lo));
+            const ib_qtensor *qkv[3] = {w.attn_q, w.attn_k, w.attn_v}, *gu[2] = {w.ffn_gate, w.ffn_up};
+            PF(gemm(qkv, 3, nc, g, row0));
+            PfQkv e = {};
+            for (int i = 0; i < 3; i++) { e.g[i] = g[i]; e.row0[i] = row0[i]; }
+            e.bias[0] = w.attn_q_bias_dev; e.bias[1] = w.attn_k_bias_dev; e.bias[2] = w.attn_v_bias_dev;
+            e.n = nc; e.q_dim = Q; e.kv_dim = KV; e.head_size = m->head_size; e.pos0 = pos0; e.kv_dtype = (uint32_t)m->kv_dtype; e.theta = m->theta;
+            e.q = B.q; e.k_cache = m->k_cache[l]; e.v_cache = m->v_cache[l];
+            PF(launch_prefill_qkv(ctx, s, e));
+            // causal attention: query t over positions 0 .. pos0 + t (transformer.rs:448)
+            for (uint32_t q0 = 0; q0 < nc; q0 += PF_CHUNK) {
+                AttnLaunch a = {};
+                a.p = ib_attn_params{c.max_position_embeddings, KV, kv_mul, m->n_heads_l, m->head_size, pos0 + q0};
+                a.q = B.q + (size_t)q0 * Q; a.k_cache = m->k_cache[l]; a.v_cache = m->v_cache[l]; a.kv_dtype = m->kv_dtype; a.out = B.att + (size_t)q0 * Q;
+                a.scratch = B.attn_scratch; a.counters = B.attn_counters; a.max_splits = B.attn_splits; a.pdl = 2;
+                a.n_queries = nc - q0 < PF_CHUNK ? nc - q0 : PF_CHUNK; a.q_step = Q; a.out_step = Q; a.counter_step = m->n_kv_l; a.scratch_step = B.attn_scratch_step;
+                if (a.n_queries > 1 && !attn_gqa4_eligible(a)) return set_error(IB_ERR_UNSUPPORTED, "ib_llama_prefill: head size %u is outside the batched attention kernel; use ib_llama_generate", m->head_size);
+                PF(launch_attention(ctx, s, a));
+            }
+            // o_proj + residual (transformer.rs:450-453); the residual add is part of the next norm kernel
+            PF(launch_prefill_norm_split(ctx, s, B.att, nullptr, nullptr, 0.f, nc, Q, B.hi, B.lo));
+            PF(gemm(&w.attn_output, 1, nc, g, row0));
             // gate, up, SwiGLU (transformer.rs:454-464)
-            PF(launch_prefill_norm_split(ctx, s, B.X, w.ffn_norm_dev, c.rms_norm_eps, nc, H, B.hi, B.lo));
-            PF(gemm(w.ffn_gate, nc, B.planes, ks));
-            PF(gemm(w.ffn_up, nc, B.planes2, ks));
-            e.planes2 = B.planes2; e.sk = ks; e.rows = F; e.mode = PE_SWIGLU; e.hi = B.hi; e.lo = B.lo;
-            PF(launch_prefill_epilogue(ctx, s, e));
+            PF(launch_prefill_norm_split(ctx, s, B.X, &g[0], w.ffn_norm_dev, c.rms_norm_eps, nc, H, B.hi, B.lo));
+            PF(gemm(gu, 2, nc, g, row0));
+            PF(launch_prefill_swiglu(ctx, s, g[0], B.hi, B.lo));
             // down + residual (transformer.rs:465-468)
-            PF(gemm(w.ffn_down, nc, B.planes, ks));
-            e.sk = ks; e.rows = H; e.mode = PE_RESIDUAL; e.out = B.X;
-            PF(launch_prefill_epilogue(ctx, s, e));
+            PF(gemm(&w.ffn_down, 1, nc, g, row0));
         }
+        PF(launch_prefill_residual(ctx, s, B.X, g[0]));
         if (t0 + nc == n) IB_CHECK_CUDA(cudaMemcpyAsync(m->x, B.X + (size_t)(nc - 1) * H, sizeof(float) * H, cudaMemcpyDeviceToDevice, s));
     }
 #undef PF

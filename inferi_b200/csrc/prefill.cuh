@@ -1,46 +1,91 @@
-// Prompt prefill on the tensor cores: what the model code (llama.cu) uses of prefill.cu.
+// Prompt prefill on the tensor cores: what the model code (llama.cu), the GEMM (prefill_gemm.cu) and the element-wise kernels
+// around it (prefill.cu) share.
 #pragma once
 
 #include "token.cuh"
 
 namespace ib {
 
-constexpr uint32_t PREFILL_MAX_TOKENS = 128;   // tokens per GEMM (the N of the MMA); longer prompts go in chunks
+constexpr uint32_t PF_CHUNK = 128;             // tokens per GEMM tile (the N of the MMA)
+constexpr uint32_t PREFILL_MAX_TOKENS = 1024;  // tokens that go through the layers together; longer prompts go in passes
+constexpr uint32_t PF_MAX_SEGS = 3;            // matrices of one GEMM launch
 
-// How a prefill GEMM's work is handed out: the (128-row tile, 256-column block) units, tile-major, are cut into `ctas`
-// contiguous, equally long ranges - one per CTA of a grid that fills the GPU exactly once, whatever the matrix's shape
-// (a grid of tiles x K slices was 1.5 waves for the FFN matrices).  A tile's K range can then fall to several CTAs; each
-// writes its partial sums to the plane numbered by its position among the tile's CTAs, and the element-wise kernel behind
-// the GEMM adds a tile's planes in that order.
+// How a prefill GEMM's work is handed out: the units (128-row tile, chunk of 128 tokens, 256-column block), in that order, are
+// cut into `ctas` contiguous, equally long ranges - one per CTA of a grid that fills the GPU exactly once, whatever the
+// matrix's shape (a grid of tiles x K slices was 1.5 waves for the FFN matrices).  The K range of a tile (= row tile and
+// chunk) can then fall to several CTAs; each writes its partial sums to the plane numbered by its position among the tile's
+// CTAs, and the element-wise kernel behind the GEMM adds a tile's planes in that order.
 struct StreamK {
     uint32_t ctas, nb, total;   // CTAs, 256-column blocks per row, units = tiles * nb
-    __host__ __device__ uint32_t first_unit(uint32_t c) const { return (uint32_t)(((uint64_t)c * total) / ctas); }
-    __host__ __device__ uint32_t cta_of(uint32_t u) const { return (uint32_t)((((uint64_t)u + 1) * ctas - 1) / total); }
+    // 32-bit arithmetic: the launcher keeps total below 2^24
+    __host__ __device__ uint32_t first_unit(uint32_t c) const { return c * total / ctas; }
+    __host__ __device__ uint32_t cta_of(uint32_t u) const { return ((u + 1) * ctas - 1) / total; }
     __host__ __device__ uint32_t pieces(uint32_t tile) const { return cta_of(tile * nb + nb - 1) - cta_of(tile * nb) + 1; }
 };
-StreamK prefill_streamk(const ib_ctx *ctx, uint32_t rows, uint32_t cols);
-uint32_t prefill_max_pieces(const StreamK &sk, uint32_t rows);   // most planes any tile of the matrix needs
+StreamK prefill_streamk(const ib_ctx *ctx, uint32_t rows, uint32_t cols, uint32_t n);
+uint32_t prefill_max_pieces(const StreamK &sk);   // bound of the planes that any tile needs
 
-enum PrefillEpilogue : uint32_t { PE_Q = 0, PE_K = 1, PE_V = 2, PE_RESIDUAL = 3, PE_SWIGLU = 4, PE_STORE = 5 };
-struct PrefillEpiParams {
-    const float *planes, *planes2;   // [piece][n][rows] partial sums (planes2: the up matrix of PE_SWIGLU)
-    StreamK sk;                      // the hand-out of the GEMM that wrote them: rows of tile t have sk.pieces(t) planes
-    uint32_t n, rows, mode;
-    const float *bias;               // PE_Q / PE_K / PE_V, or null
-    const float *theta;              // [head_size / 2]
-    uint32_t head_size, pos0, kv_dim, kv_dtype;
-    float *out;                      // PE_Q: q [n][rows]; PE_RESIDUAL: X [n][rows] (added to); PE_STORE: [n][rows]
-    void *cache;                     // PE_K / PE_V: this layer's cache [max_pos][kv_dim]
-    __half *hi, *lo;                 // PE_SWIGLU: the product, split, [n_pad][rows]
+struct PgParams {
+    uint32_t tile0[PF_MAX_SEGS];   // first row tile of each matrix (0xFFFFFFFF: not there)
+    uint32_t rows, n, chunks;      // rows of all matrices together, tokens, chunks of 128 tokens
+    const __half *x_hi, *x_lo;     // the tokens' inputs split into two f16, tiled (pf_x_index); per chunk x_chunk halves
+    size_t x_chunk;
+    float *plane0, *planes;        // [n][rows] the first CTA's sums of every tile; [piece - 1][n][rows] the others'
+    uint32_t x_stages, x_tile;     // ring of the inputs: stages, bytes of a stage's hi (= lo) tile (set by the launcher)
+    StreamK sk;
+    uint32_t *err;
+    unsigned long long wait_ns;
 };
 
+// ---- the tokens' inputs in global memory, laid out the way the tensor core reads them from shared memory ----
+// Per chunk of 128 tokens: one tile of 128 token rows per 64 columns in the K-major core-matrix layout (8 rows x 16 bytes;
+// 16 KiB), so that a stage's tile is one bulk copy.  Four consecutive columns are stored in the order 0, 2, 1, 3, the order in
+// which the producers unpack the weights.
+__host__ __device__ inline uint32_t pf_x_index(uint32_t t, uint32_t c) {   // halves inside the chunk; t: token inside the chunk
+    const uint32_t k = (c & 4u) | ((c & 1u) << 1) | ((c >> 1) & 1u);
+    return (c >> 6) * (PF_CHUNK * 64) + (t >> 3) * 512 + ((c & 63) >> 3) * 64 + (t & 7) * 8 + k;
+}
+// Behind the input tiles of a chunk sit the tiles of its sub-block sums: per 256 columns one tile of 128 token rows x 16 halves
+// in the same core-matrix layout (the sums of the block's eight 32-column sub-blocks, then eight zeros), hi and lo halves
+// like the inputs.  The k-quant GEMM multiplies them with the sub-blocks' minimums.
+__host__ __device__ inline uint32_t pf_s_index(uint32_t t, uint32_t sb, uint32_t cols) {
+    return PF_CHUNK * cols + (sb >> 3) * (PF_CHUNK * 16) + (t >> 3) * 128 + (t & 7) * 8 + (sb & 7);
+}
+__host__ __device__ inline size_t pf_x_halves(uint32_t cols) { return (size_t)(PF_CHUNK + 8) * cols; }   // halves per chunk (hi or lo)
 
 bool prefill_gemm_eligible(const ib_qtensor *m);
-// planes[piece][n][rows] = partial sums of W . x_t over the K ranges of the tile's CTAs; x_hi / x_lo: 128 x cols halves in the tiled layout that
-// launch_prefill_norm_split and the PE_SWIGLU epilogue write (one 16 KiB tile per 64 columns), rows n .. (n rounded up to 16) - 1 zero
-int32_t launch_prefill_gemm(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *m, const __half *x_hi, const __half *x_lo, uint32_t n, float *planes, const StreamK &sk);
+// plane0 / planes = partial sums of W x_t over the K ranges of the tile's CTAs; x_hi / x_lo: the layout above, token rows n .. (n rounded
+// up to 16) - 1 of the last chunk zero.  The matrices of a launch have the same type and width; their rows follow one another.
+int32_t launch_prefill_gemm(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *const *mats, uint32_t n_mats, const __half *x_hi, const __half *x_lo, uint32_t n, float *plane0,
+                            float *planes, const StreamK &sk);
+
+// One GEMM launch's result, as the element-wise kernels read it
+struct PfPlanes {
+    const float *plane0, *planes;
+    StreamK sk;
+    uint32_t rows, chunks, n;
+};
+
 int32_t launch_prefill_embed(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *embd, const uint32_t *tokens_dev, uint32_t n, uint32_t vocab, float *X);
-int32_t launch_prefill_norm_split(ib_ctx *ctx, cudaStream_t s, const float *X, const float *w, float eps, uint32_t n, uint32_t cols, __half *hi, __half *lo);
-int32_t launch_prefill_epilogue(ib_ctx *ctx, cudaStream_t s, const PrefillEpiParams &p);
+// X += the planes (if any); y = RMSNorm(X) with weights w (null: y = X), split and tiled into hi / lo
+int32_t launch_prefill_norm_split(ib_ctx *ctx, cudaStream_t s, float *X, const PfPlanes *add, const float *w, float eps, uint32_t n, uint32_t cols, __half *hi, __half *lo);
+// X += the planes
+int32_t launch_prefill_residual(ib_ctx *ctx, cudaStream_t s, float *X, const PfPlanes &add);
+// out += the planes behind plane 0 (= out): completes a GEMM whose plane 0 was its output
+int32_t launch_prefill_finish(ib_ctx *ctx, cudaStream_t s, float *out, const PfPlanes &add);
+// y = up * silu(gate), split and tiled: gate = rows 0 .. F-1, up = rows F .. 2F-1 of one launch
+int32_t launch_prefill_swiglu(ib_ctx *ctx, cudaStream_t s, const PfPlanes &gu, __half *hi, __half *lo);
+
+struct PfQkv {
+    PfPlanes g[3];                   // the launches that q, k and v came from (two or three may be the same launch) ...
+    uint32_t row0[3];                // ... and the row of the launch at which each starts
+    const float *bias[3];
+    uint32_t n, q_dim, kv_dim, head_size, pos0, kv_dtype;
+    const float *theta;              // [head_size / 2]
+    float *q;                        // [n][q_dim]
+    void *k_cache, *v_cache;         // this layer's cache [max_pos][kv_dim]
+};
+// bias, rotation, q out and cache append
+int32_t launch_prefill_qkv(ib_ctx *ctx, cudaStream_t s, const PfQkv &p);
 
 }  // namespace ib

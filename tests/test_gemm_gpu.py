@@ -34,6 +34,25 @@ def test_gemm_matches_row_by_row_gemv(backend, qt, rows, cols, n):
     m.close()
 
 
+@pytest.mark.parametrize("qt,rows,cols,n", [
+    (quant.Q4_K, 128, 256, 129), (quant.Q5_K, 256, 512, 255), (quant.Q6_K, 128, 2048, 130), (quant.Q8_0, 384, 256, 257),   # edges of the 128-token chunks
+    (quant.Q8_0, 128, 1024, 15), (quant.Q5_K, 128, 768, 17), (quant.Q6_K, 640, 4096, 1029),                                # ... of the 16-token padding, two passes
+])
+def test_gemm_across_chunks_of_tokens(backend, qt, rows, cols, n):
+    """Every row of the result: the tokens of all chunks, and the tiles whose K range is split between CTAs."""
+    blocks = quant.random_blocks(qt, rows, cols, seed=rows + cols + n, scale=0.05)
+    x = np.random.default_rng(n).standard_normal((n, cols)).astype(np.float32)
+    m = GpuQuantTensor(backend, qt, rows, cols, blocks)
+    out = torch.full((n, rows), float("nan"), device="cuda")
+    GemmQuant(backend).launch(out, m, torch.from_numpy(x).cuda())
+    w = torch.from_numpy(np.stack([oracle.dequantize(qt, blocks[r], cols) for r in range(rows)])).cuda().double()
+    want = torch.from_numpy(x).cuda().double() @ w.T
+    err = float((out.double() - want).norm() / want.norm())
+    assert err < 1e-5      # operands carry >= 21 bits: 2^-21 per product, averaged over the sum
+    assert float((out.double() - want).abs().max()) < 1e-4 * float(want.abs().max())
+    m.close()
+
+
 def test_gemm_rejects_shapes_outside_the_tensor_core_path(backend):
     blocks = quant.random_blocks(quant.Q4_K, 64, 256, seed=1)
     m = GpuQuantTensor(backend, quant.Q4_K, 64, 256, blocks)     # 64 rows: not a multiple of 128
