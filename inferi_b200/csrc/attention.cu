@@ -93,30 +93,28 @@ int32_t launch_attention(ib_ctx *ctx, cudaStream_t s, const AttnLaunch &a) {
     IB_REQUIRE(a.pos_ptr || p.pos < p.seq_len, "attention: pos=%u outside the cache of %u rows", p.pos, p.seq_len);
     IB_REQUIRE(a.max_splits >= 1 && a.max_splits <= 2 * p.head_size && a.max_splits <= 256, "attention: %u position slices exceed what the merge step holds (%u)",
                a.max_splits, 2 * p.head_size < 256 ? 2 * p.head_size : 256);
-    AttnArgs args{p, a.pos_ptr, a.q, a.k_cache, a.v_cache, a.out, a.scratch, a.counters, a.max_splits, a.pdl, 0u, a.q_step, a.out_step, a.counter_step, a.scratch_step};
+    AttnArgs args{p, a.pos_ptr, a.q, a.k_cache, a.v_cache, a.out, a.scratch, a.counters, a.max_splits, a.pdl, 0u};
     const bool f16 = a.kv_dtype == IB_KV_F16;
     const bool gqa4 = attn_gqa4_eligible(a);
-    const uint32_t nq = a.n_queries > 1 ? a.n_queries : 1;
-    IB_REQUIRE(nq == 1 || (gqa4 && !a.pos_ptr && p.pos + nq <= p.seq_len), "attention: a batched launch needs the f16 / 4-heads-per-kv-head kernel and host-known positions inside the cache");
     // with a host-known position only the splits that will do work are launched
     uint32_t splits = a.max_splits;
     if (!a.pos_ptr) {
         uint32_t need, per;
-        if (gqa4) attn_split_plan(p.pos + nq, a.max_splits, need, per, GQA4_MIN_PER_SPLIT, GQA4_KNEE, GQA4_KNEE_PER);
-        else attn_split_plan(p.pos + nq, a.max_splits, need, per);
+        if (gqa4) attn_split_plan(p.pos + 1, a.max_splits, need, per, GQA4_MIN_PER_SPLIT, GQA4_KNEE, GQA4_KNEE_PER);
+        else attn_split_plan(p.pos + 1, a.max_splits, need, per);
         if (need < splits) splits = need;
     }
     if (gqa4) {
         // short contexts merge inside a thread-block cluster (the first one of the kv head)
         if (a.pos_ptr) {
             args.cluster = a.short_context ? gqa4_cluster_size(splits) : 0u;
-        } else if (p.pos + nq <= GQA4_CLUSTER_MAX * GQA4_CLUSTER_PER) {
-            const uint32_t want = (p.pos + nq + GQA4_MIN_PER_SPLIT - 1) / GQA4_MIN_PER_SPLIT;
+        } else if (p.pos + 1 <= GQA4_CLUSTER_MAX * GQA4_CLUSTER_PER) {
+            const uint32_t want = (p.pos + 1 + GQA4_MIN_PER_SPLIT - 1) / GQA4_MIN_PER_SPLIT;
             const uint32_t cs = want < GQA4_CLUSTER_MAX ? want : GQA4_CLUSTER_MAX;
             if (cs >= 2 && cs <= a.max_splits) { splits = cs; args.cluster = cs; }
         }
     }
-    const dim3 grid(n_kv, splits, nq);
+    const dim3 grid(n_kv, splits);
     if (gqa4) {
         cudaLaunchConfig_t cfg = {};
         cfg.gridDim = grid;

@@ -26,10 +26,6 @@ struct AttnArgs {
     uint32_t max_splits;
     uint32_t pdl;       // programmatic dependent launch: 0 no, 1 the predecessor writes only q and the newest cache row, 2 it may write anything
     uint32_t cluster;   // CTAs per thread-block cluster along the slices of a kv head (attn_gqa4_kernel only); 0: no clusters
-    // Several queries in one launch (prompt prefill; gridDim.z = number of queries, only in the kernel for the Llama-3
-    // shape): query z sits at position p.pos + z, its vectors, scratch and counters `*_step` elements after query 0's.
-    uint32_t q_step, out_step, counter_step;
-    size_t scratch_step;
 };
 
 template <typename T> struct KvVec;

@@ -214,10 +214,6 @@ struct AttnLaunch {
     // Such a launch is slower at long contexts (clusters constrain the placement of the grid's one wave of CTAs), so a graph
     // for longer contexts is recorded without it.  With a host-known position the launch decides by itself.
     uint32_t short_context;
-    // batched launch (prompt prefill): n_queries > 1 queries at positions p.pos, p.pos + 1, ...; steps in elements between
-    // consecutive queries' q / out / scratch / counters.  Only the kernel for the Llama-3 shape takes it.
-    uint32_t n_queries, q_step, out_step, counter_step;
-    size_t scratch_step;
 };
 bool attn_gqa4_eligible(const AttnLaunch &a);
 size_t attn_scratch_bytes(const ib_attn_params &p, uint32_t max_splits);

@@ -141,12 +141,9 @@ struct ib_llama {
     struct PrefillBuffers {
         uint8_t *arena = nullptr;
         uint32_t chunks = 0;
-        float *X = nullptr, *q = nullptr, *att = nullptr, *planes = nullptr, *attn_scratch = nullptr;
+        float *X = nullptr, *q = nullptr, *planes = nullptr;
         __half *hi = nullptr, *lo = nullptr;
         uint32_t *tokens = nullptr;
-        unsigned int *attn_counters = nullptr;
-        uint32_t attn_splits = 0;
-        size_t attn_scratch_step = 0;
     } pf;
     // tensors and device vectors the model owns (a model loaded from a GGUF file frees its weights with itself)
     std::vector<ib_qtensor *> owned_tensors;
@@ -766,7 +763,7 @@ static int32_t prefill_prepare(ib_llama *m, uint32_t n) {
     auto &B = m->pf;
     if (chunks <= B.chunks) return IB_OK;
     const ib_llama_config &c = m->cfg;
-    const uint32_t H = c.hidden_size, F = m->ffn_l, Q = m->q_dim_l, KV = m->kv_dim_l, N = chunks * PF_CHUNK;
+    const uint32_t H = c.hidden_size, F = m->ffn_l, Q = m->q_dim_l, N = chunks * PF_CHUNK;
     const uint32_t widest = F > H ? (F > Q ? F : Q) : (H > Q ? H : Q);
     size_t planes = 0;   // the largest result that is alive at once, over the layers and over the passes' lengths
     for (const ib_llama_layer_weights &w : m->layers) {
@@ -780,9 +777,6 @@ static int32_t prefill_prepare(ib_llama *m, uint32_t n) {
                 planes = sum > planes ? sum : planes;
             }
     }
-    ib_attn_params ap{c.max_position_embeddings, KV, c.num_attention_heads / c.num_key_value_heads, m->n_heads_l, m->head_size, 0};
-    B.attn_splits = 16;   // per query; the queries of a prompt fill the GPU between them
-    B.attn_scratch_step = attn_scratch_bytes(ap, B.attn_splits) / sizeof(float);
     if (B.arena) {   // growing: wait for work that may still use the old one
         IB_CHECK_CUDA(cudaDeviceSynchronize());
         IB_CHECK_CUDA(cudaFree(B.arena));
@@ -791,16 +785,12 @@ static int32_t prefill_prepare(ib_llama *m, uint32_t n) {
     }
     size_t total = 0;
     auto place = [&](size_t bytes) { const size_t at = total; total += (bytes + 255) & ~(size_t)255; return at; };
-    const size_t oX = place(sizeof(float) * N * H), oq = place(sizeof(float) * N * Q), oatt = place(sizeof(float) * N * Q);
+    const size_t oX = place(sizeof(float) * N * H), oq = place(sizeof(float) * N * Q);
     const size_t ohi = place(sizeof(__half) * chunks * pf_x_halves(widest)), olo = place(sizeof(__half) * chunks * pf_x_halves(widest));
-    const size_t opl = place(sizeof(float) * planes), otok = place(sizeof(uint32_t) * N), osc = place(sizeof(float) * PF_CHUNK * B.attn_scratch_step);
-    const size_t octr = place(sizeof(unsigned int) * PF_CHUNK * m->n_kv_l);
+    const size_t opl = place(sizeof(float) * planes), otok = place(sizeof(uint32_t) * N);
     IB_CHECK_CUDA(cudaMalloc(&B.arena, total));
-    B.X = (float *)(B.arena + oX); B.q = (float *)(B.arena + oq); B.att = (float *)(B.arena + oatt);
+    B.X = (float *)(B.arena + oX); B.q = (float *)(B.arena + oq);
     B.hi = (__half *)(B.arena + ohi); B.lo = (__half *)(B.arena + olo); B.planes = (float *)(B.arena + opl); B.tokens = (uint32_t *)(B.arena + otok);
-    B.attn_scratch = (float *)(B.arena + osc); B.attn_counters = (unsigned int *)(B.arena + octr);
-    IB_CHECK_CUDA(cudaMemset(B.attn_counters, 0, sizeof(unsigned int) * PF_CHUNK * m->n_kv_l));
-    IB_CHECK_CUDA(cudaDeviceSynchronize());
     B.chunks = chunks;
     return IB_OK;
 }
@@ -866,17 +856,8 @@ int32_t ib_llama_prefill(ib_llama *m, void *stream, const uint32_t *tokens_host,
             e.q = B.q; e.k_cache = m->k_cache[l]; e.v_cache = m->v_cache[l];
             PF(launch_prefill_qkv(ctx, s, e));
             // causal attention: query t over positions 0 .. pos0 + t (transformer.rs:448)
-            for (uint32_t q0 = 0; q0 < nc; q0 += PF_CHUNK) {
-                AttnLaunch a = {};
-                a.p = ib_attn_params{c.max_position_embeddings, KV, kv_mul, m->n_heads_l, m->head_size, pos0 + q0};
-                a.q = B.q + (size_t)q0 * Q; a.k_cache = m->k_cache[l]; a.v_cache = m->v_cache[l]; a.kv_dtype = m->kv_dtype; a.out = B.att + (size_t)q0 * Q;
-                a.scratch = B.attn_scratch; a.counters = B.attn_counters; a.max_splits = B.attn_splits; a.pdl = 2;
-                a.n_queries = nc - q0 < PF_CHUNK ? nc - q0 : PF_CHUNK; a.q_step = Q; a.out_step = Q; a.counter_step = m->n_kv_l; a.scratch_step = B.attn_scratch_step;
-                if (a.n_queries > 1 && !attn_gqa4_eligible(a)) return set_error(IB_ERR_UNSUPPORTED, "ib_llama_prefill: head size %u is outside the batched attention kernel; use ib_llama_generate", m->head_size);
-                PF(launch_attention(ctx, s, a));
-            }
+            PF(launch_prefill_attention(ctx, s, B.q, m->k_cache[l], m->v_cache[l], nc, pos0, m->n_kv_l, m->head_size, B.hi, B.lo));
             // o_proj + residual (transformer.rs:450-453); the residual add is part of the next norm kernel
-            PF(launch_prefill_norm_split(ctx, s, B.att, nullptr, nullptr, 0.f, nc, Q, B.hi, B.lo));
             PF(gemm(&w.attn_output, 1, nc, g, row0));
             // gate, up, SwiGLU (transformer.rs:454-464)
             PF(launch_prefill_norm_split(ctx, s, B.X, &g[0], w.ffn_norm_dev, c.rms_norm_eps, nc, H, B.hi, B.lo));

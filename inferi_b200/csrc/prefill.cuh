@@ -85,6 +85,10 @@ struct PfQkv {
     float *q;                        // [n][q_dim]
     void *k_cache, *v_cache;         // this layer's cache [max_pos][kv_dim]
 };
+// causal attention of n queries at positions pos0 .. pos0 + n - 1 (four query heads per kv head, f16 cache that already holds their
+// rows); the result as the next GEMM's inputs
+int32_t launch_prefill_attention(ib_ctx *ctx, cudaStream_t s, const float *q, const void *k_cache, const void *v_cache, uint32_t n, uint32_t pos0, uint32_t n_kv, uint32_t head_size,
+                                 __half *hi, __half *lo);
 // bias, rotation, q out and cache append
 int32_t launch_prefill_qkv(ib_ctx *ctx, cudaStream_t s, const PfQkv &p);
 

@@ -74,6 +74,28 @@ def test_long_prompt_goes_in_chunks_and_matches_the_oracle(backend):
     dev_w.close()
 
 
+@pytest.mark.parametrize("hidden,heads,n,start", [(512, 8, 17, 0), (512, 8, 1, 300), (512, 4, 65, 0), (512, 4, 15, 470), (512, 8, 200, 130)])
+def test_prompt_attention_at_the_edges_of_its_tiles(backend, hidden, heads, n, start):
+    """16-token and 64-position tiles with remainders, positions divided between the CTAs of a cluster (few tokens far into the
+    context), both head sizes: against the decode loop's attention, whose cache rows are the same f16 values."""
+    cfg = Llama2Config(hidden, 1024, 1, heads, heads // 4, 512, 512, 500000.0, 1e-5)
+    recipe = dict(Q4_K_M, token_embd=quant.Q4_K, attn_v=quant.Q5_K, ffn_down=quant.Q8_0, output=quant.Q4_K)
+    w = synth_weights(cfg, seed=31, recipe=recipe, std=0.06)      # sharper scores than 0.02 gives
+    dev_w = Llama2Weights(backend, cfg, w)
+    toks = np.random.default_rng(32 + n).integers(0, cfg.vocab_size, start + n).tolist()
+    loop, fast = Llama2(backend, cfg, dev_w, kv_f16=True), Llama2(backend, cfg, dev_w, kv_f16=True)
+    loop.generate(toks, 0)
+    if start:
+        fast.prefill(toks[:start])
+    fast.prefill(toks[start:], start_pos=start)
+    a, b = loop.hidden_state(), fast.hidden_state()
+    # the loop's activations are 16-bit block fixed point (2^-15 of a group's largest value per GEMV, seven GEMVs deep)
+    assert np.abs(a - b).max() <= 2e-3 * np.abs(a).max()
+    loop.close()
+    fast.close()
+    dev_w.close()
+
+
 def test_prefill_refuses_what_the_tensor_core_path_does_not_take(backend):
     cfg = Llama2Config(256, 2048, 2, 4, 2, 512, 64, 500000.0, 1e-5)     # 2 query heads per kv head, 256-row matrices... kv_mul = 2
     w = synth_weights(cfg, seed=5, recipe=dict(Q4_K_M, token_embd=quant.Q4_K, attn_v=quant.Q4_K, ffn_down=quant.Q4_K, output=quant.Q4_K))
