@@ -10,7 +10,7 @@ constexpr int PACK_THREADS = 512;        // threads that take part in the activa
 constexpr uint32_t GEMV_MAX_COLS = 32768;
 
 // Activation form in shared memory, for `cols` columns (a multiple of 32):
-//   ACT_LIMBS int8 limbs a0, a1 [cols] each;  f32 scale s/127 per 32 columns;  f32 sum of the quantized x per 16 columns
+//   ACT_LIMBS int8 limbs a0, a1 [cols] each;  f32 scale s/(127 * 254) per 32 columns;  f32 sum of the quantized x per 16 columns
 //   x ~= (s/127) * (a0 + a1/254)      (resolution 1.6e-5 * max|x| of the 32-group: 16-bit block fixed point)
 //   (+ 192 bytes: in the group-major chunk order each limb array carries one 16-byte skew per group, see act_chunk_pos)
 // The 16-column sums (used for the k-quants' minimums and the Q6_K -32 terms) are sums of the QUANTIZED values, so that
@@ -38,12 +38,11 @@ __device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c) {
     asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
     return d;
 }
-// the integer dot products of the limbs -> the dot product in units of the group's scale; d[0 .. ACT_LIMBS-1]
-__device__ __forceinline__ float limb_combine(const int *d) {
-    float v = (float)d[0] + (float)d[1] * (1.0f / 254.0f);
-    if (ACT_LIMBS > 2) v += (float)d[ACT_LIMBS - 1] * (1.0f / 64516.0f);
-    return v;
-}
+// The integer dot products of the two limbs -> the dot product in units of the group's scale.  254 d0 + d1 is formed as an
+// integer (at most 2^28 for every format's longest chain) and converted once: one multiply-add and one conversion instead of
+// two conversions and a float multiply-add, and exact up to the conversion's rounding.
+static_assert(ACT_LIMBS == 2, "the dot products combine two limbs");
+__device__ __forceinline__ float limb_combine(const int *d) { return (float)(d[0] * 254 + d[1]); }
 __device__ __forceinline__ float h2f(uint32_t bits16) { return __half2float(__ushort_as_half((unsigned short)bits16)); }
 
 __device__ __forceinline__ void named_barrier(int id, int nthreads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory"); }
@@ -86,6 +85,29 @@ __device__ __forceinline__ void pack_prefetch_norm(const float *__restrict__ nor
 // and the one-chunk skew between groups keeps the four chunks that neighbouring threads store apart as well.
 __device__ __forceinline__ uint32_t act_chunk_pos(uint32_t run, uint32_t nq) { return nq ? (run & 3u) * (nq + 1) + (run >> 2) : run; }
 
+constexpr float ACT_UNIT = 1.0f / (127.0f * 254.0f);   // times a group's largest |x|: the unit of 254 a0 + a1
+
+// Four columns -> their bytes of the two limbs; `inv` = 127 / largest |x| of the group; `sum` += the quantized values in units of
+// the first limb.  Round-to-nearest-even by adding 1.5 * 2^23: the sum's low mantissa byte is the rounded value in two's
+// complement (|t| <= 127), and subtracting the constant again gives it back as a float - no conversion instructions.
+__device__ __forceinline__ void pack_four(const float (&e)[4], float inv, uint32_t &w0, uint32_t &w1, float &sum) {
+    constexpr float MAGIC = 12582912.0f;
+    uint32_t b0[4], b1[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+        const float t = e[k] * inv;
+        const float r0 = t + MAGIC, q0 = r0 - MAGIC;            // the limbs as floats: q0, q1
+        const float t1 = (t - q0) * 254.0f;
+        const float r1 = t1 + MAGIC, q1 = r1 - MAGIC;
+        b0[k] = __float_as_uint(r0);
+        b1[k] = __float_as_uint(r1);
+        sum += q0 + q1 * (1.0f / 254.0f);
+    }
+    // low bytes of four words -> one word
+    w0 = __byte_perm(__byte_perm(b0[0], b0[1], 0x0040), __byte_perm(b0[2], b0[3], 0x0040), 0x5410);
+    w1 = __byte_perm(__byte_perm(b1[0], b1[1], 0x0040), __byte_perm(b1[2], b1[3], 0x0040), 0x5410);
+}
+
 __device__ __forceinline__ void pack_run(const float4 (&v)[4], uint32_t run, uint32_t cols, uint8_t *smem, bool store, uint32_t nq = 0) {
     const int lane = threadIdx.x & 31;
     float amax = 0.f, sum = 0.f;   // sum: of the quantized values, in units of the group's scale
@@ -93,39 +115,20 @@ __device__ __forceinline__ void pack_run(const float4 (&v)[4], uint32_t run, uin
     for (int j = 0; j < 4; j++) amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));   // the other half of the 32-column group
     const float inv = amax > 0.f ? __fdividef(127.0f, amax) : 0.f;   // 2 ulp: the limbs absorb it (|t| stays within 127 + 1e-5)
-    // round-to-nearest-even by adding 1.5 * 2^23: the sum's low mantissa byte is the rounded value in two's complement
-    // (|t| <= 127), and subtracting the constant again gives it back as a float - no conversion instructions
-    constexpr float MAGIC = 12582912.0f;
-    uint32_t w0[4], w1[4], w2[4];
+    uint32_t w0[4], w1[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         const float e[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
-        uint32_t b0[4], b1[4], b2[4];
-#pragma unroll
-        for (int k = 0; k < 4; k++) {
-            const float t = e[k] * inv;
-            const float r0 = t + MAGIC, q0 = r0 - MAGIC;            // the limbs as floats: q0, q1, q2
-            const float t1 = (t - q0) * 254.0f;
-            const float r1 = t1 + MAGIC, q1 = r1 - MAGIC;
-            const float t2 = (t1 - q1) * 254.0f;
-            const float r2 = t2 + MAGIC;
-            b0[k] = __float_as_uint(r0); b1[k] = __float_as_uint(r1); b2[k] = __float_as_uint(r2);
-            sum += q0 + q1 * (1.0f / 254.0f) + (ACT_LIMBS > 2 ? (r2 - MAGIC) * (1.0f / 64516.0f) : 0.f);
-        }
-        // low bytes of four words -> one word
-        w0[j] = __byte_perm(__byte_perm(b0[0], b0[1], 0x0040), __byte_perm(b0[2], b0[3], 0x0040), 0x5410);
-        w1[j] = __byte_perm(__byte_perm(b1[0], b1[1], 0x0040), __byte_perm(b1[2], b1[3], 0x0040), 0x5410);
-        w2[j] = __byte_perm(__byte_perm(b2[0], b2[1], 0x0040), __byte_perm(b2[2], b2[3], 0x0040), 0x5410);
+        pack_four(e, inv, w0[j], w1[j], sum);
     }
     if (store) {
         const size_t ls = cols + (nq ? 64u : 0u);   // = Act::lstride()
-        uint4 *l0 = reinterpret_cast<uint4 *>(smem), *l1 = reinterpret_cast<uint4 *>(smem + ls), *l2 = reinterpret_cast<uint4 *>(smem + 2 * ls);
+        uint4 *l0 = reinterpret_cast<uint4 *>(smem), *l1 = reinterpret_cast<uint4 *>(smem + ls);
         float *sc = reinterpret_cast<float *>(smem + ACT_LIMBS * ls), *sx16 = sc + cols / 32;
         const uint32_t at = act_chunk_pos(run, nq);
         l0[at] = make_uint4(w0[0], w0[1], w0[2], w0[3]);
         l1[at] = make_uint4(w1[0], w1[1], w1[2], w1[3]);
-        if (ACT_LIMBS > 2) l2[at] = make_uint4(w2[0], w2[1], w2[2], w2[3]);
-        if ((lane & 1) == 0) sc[run >> 1] = amax * (1.0f / 127.0f);
+        if ((lane & 1) == 0) sc[run >> 1] = amax * ACT_UNIT;
         sx16[run] = sum * (amax * (1.0f / 127.0f));
     }
 }

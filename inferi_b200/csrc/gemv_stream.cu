@@ -23,7 +23,7 @@ namespace ib {
 
 
 struct StreamGeom {
-    uint32_t stages, stage_bytes, act_off, part_off, bar_off;
+    uint32_t stages, stage_bytes, act_off, part_off, bar_off, b_off;   // b_off: gate/up - where the up rows start inside a stage
     // the launch's tiles in hand-out order: per segment the pairs, the pairs per tile and the tiles; bytes per pair
     uint32_t seg_pairs[3], seg_pt[3], seg_tiles[3], seg_cost[3], total_tiles, meta_off;
     uint32_t dynamic;   // 1: tiles are claimed from a counter; 0: every CTA streams its own byte-balanced range of pairs
@@ -47,8 +47,8 @@ struct Consumer {
     uint32_t ring;        // shared address of the ring
     uint32_t part;        // shared address of the per-stage partial sums [stages][2][CW][PT_MAX]
     uint32_t meta;        // shared address of [stages] (segment, first pair, pairs, -) descriptors written by the producer
-    uint32_t bar0, S, stage_bytes;
-    uint32_t CG, RG, cg, rg, u;
+    uint32_t bar0, S, stage_bytes, b_off;
+    uint32_t RG, cg, rg, u;
     bool has_unit;
     int lane;
 };
@@ -62,58 +62,72 @@ constexpr uint32_t PART_STAGE_FLOATS = 2 * CW * PT_MAX;
 // two partial sums per pair (its columns of the two rows) in the stage's partial block and arrives on the stage's "done"
 // barrier.  It never waits for another consumer warp: adding up the column groups and everything that follows is the
 // epilogue warp's work.
+// What bounds the short launches is this loop's instruction stream, so whatever does not change from tile to tile is carried in
+// registers by additions and whatever only changes with the segment is set when the segment does.  (With that, one conversion per
+// pair of limb sums and the eight-column packing, a token's launches of an 8B Q4_K_M model went from 1632 to 1550 us.)
 template <uint32_t QT>
 __device__ __forceinline__ void consume_tiles(const GemvParams &p, const Consumer &c, const Act &A) {
     const int lane = c.lane;
     UnitAct ua;
     LaneConst lc;
-    uint32_t cur_type = 0xFFFFFFFFu;
-    const uint32_t S = c.S, RG = c.RG;
-    uint32_t st = 0, par = 0;
     constexpr bool ONE_TYPE = (QT != QT_MIXED && QT != QT_Q4_Q6);
-    const uint32_t rb0 = (uint32_t)p.seg[0].row_bytes, rb1 = (uint32_t)p.seg[1].row_bytes, rb2 = (uint32_t)p.seg[2].row_bytes;
     const bool swiglu = p.epi == EPI_SWIGLU;   // gate rows, then up rows, in one tile: a "pair" is gate row r + up row r
-    {
-        // The lane's activations go into registers in the layout of the first segment's format before the first tile is
-        // waited for: the copy of that tile and this load overlap.
-        const uint32_t q0 = ONE_TYPE ? QT : p.seg[0].qtype;
-        unit_init<QT>(q0, c.u, lc);
-        if (c.has_unit) load_unit_act(q0, c.u, A, ua);
-        cur_type = q0;
-    }
+    const uint32_t rb0 = (uint32_t)p.seg[0].row_bytes, rb1 = (uint32_t)p.seg[1].row_bytes, rb2 = (uint32_t)p.seg[2].row_bytes, RG = c.RG, rg = c.rg;
+    uint32_t cur_type = ONE_TYPE ? QT : p.seg[0].qtype, cur_s = 0, stride = swiglu ? rb0 : 2 * rb0, step = RG * stride, to_b = swiglu ? c.b_off : rb0;
+    uint32_t row_off = rg * stride;
+    // The lane's activations go into registers in the layout of the first segment's format before the first tile is
+    // waited for: the copy of that tile and this load overlap.
+    unit_init<QT>(cur_type, c.u, lc);
+    if (c.has_unit) load_unit_act(cur_type, c.u, A, ua);
+    uint32_t full = c.bar0, tile = c.ring, meta = c.meta, par = 0;
+    uint32_t pt = c.part + 4 * part_index(lane >> 4, c.cg, rg);
+    const uint32_t full_end = c.bar0 + 8 * c.S, to_done = 16 * c.S;
+    const bool up = lane & 16, writer = (lane & 15) == 0;
 #pragma unroll 1
-    for (;; st = (st + 1 == S) ? 0 : st + 1, par ^= (st == 0) ? 1u : 0u) {
-        if (!mbar_wait(c.bar0 + 8 * st, par, p.err, 1, p.wait_ns)) return;   // the error word is raised; give up on this CTA's rows
-        const uint4 tm = lds128(c.meta + 16 * st);
-        const uint32_t s = tm.x, n = tm.z;
+    for (;;) {
+        if (!mbar_wait(full, par, p.err, 1, p.wait_ns)) return;   // the error word is raised; give up on this CTA's rows
+        const uint4 tm = lds128(meta);
+        const uint32_t n = tm.z;
         if (n == 0) break;   // no tiles left
-        const uint32_t qtype = ONE_TYPE ? QT : (s == 0 ? p.seg[0].qtype : (s == 1 ? p.seg[1].qtype : p.seg[2].qtype));
-        if (qtype != cur_type) {   // (re)load this lane's activations in the layout of the segment's format
-            unit_init<QT>(qtype, c.u, lc);
-            if (c.has_unit) load_unit_act(qtype, c.u, A, ua);
-            cur_type = qtype;
-        }
-        const uint32_t tile = c.ring + st * c.stage_bytes;
-        const uint32_t rbA = (swiglu || s == 0) ? rb0 : (s == 1 ? rb1 : rb2);
-        const uint32_t strideA = swiglu ? rbA : 2 * rbA;
-        const uint32_t offB = swiglu ? n * rbA : rbA, strideB = swiglu ? rb1 : strideA;
-        const uint32_t pt = c.part + 4 * (st * PART_STAGE_FLOATS);
-        for (uint32_t pr = c.rg; pr < n; pr += RG) {
-            float va = 0.f, vb = 0.f;
-            if (c.has_unit) {
-                va = unit_dot<QT>(qtype, tile + pr * strideA, lc, ua);
-                vb = unit_dot<QT>(qtype, tile + offB + pr * strideB, lc, ua);
+        if (tm.x != cur_s) {
+            cur_s = tm.x;
+            const uint32_t rb = cur_s == 1 ? rb1 : rb2;
+            stride = 2 * rb;
+            step = RG * stride;
+            to_b = rb;
+            row_off = rg * stride;
+            if (!ONE_TYPE) {
+                const uint32_t qtype = cur_s == 1 ? p.seg[1].qtype : p.seg[2].qtype;
+                if (qtype != cur_type) {   // (re)load this lane's activations in the layout of the segment's format
+                    cur_type = qtype;
+                    unit_init<QT>(qtype, c.u, lc);
+                    if (c.has_unit) load_unit_act(qtype, c.u, A, ua);
+                }
             }
+        }
+        uint32_t at = tile + row_off, out = pt;
+        for (uint32_t pr = rg; pr < n; pr += RG, at += step, out += 4 * RG) {
+            float va = 0.f, vb = 0.f;
+            if (c.has_unit) unit_dot2<QT>(cur_type, at, at + to_b, lc, ua, va, vb);
             // one shuffle tree for both rows: after the first exchange the upper half-warp carries row B
-            const bool up = lane & 16;
             float v = (up ? vb : va) + __shfl_xor_sync(0xffffffffu, up ? va : vb, 16);
 #pragma unroll
             for (int o = 8; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if ((lane & 15) == 0)   // lane 0 holds row A's sum, lane 16 row B's
-                asm volatile("st.shared.f32 [%0], %1;" ::"r"(pt + 4 * part_index(lane >> 4, c.cg, pr)), "f"(v) : "memory");
+            if (writer) asm volatile("st.shared.f32 [%0], %1;" ::"r"(out), "f"(v) : "memory");   // lane 0 holds row A's sum, lane 16 row B's
         }
         __syncwarp();   // lane 16's partials are ordered before lane 0's arrival (a release)
-        if (lane == 0) mbar_arrive(c.bar0 + 8 * (2 * S + st));   // this warp is done with the stage: weights read, partials left
+        if (lane == 0) mbar_arrive(full + to_done);   // this warp is done with the stage: weights read, partials left
+        full += 8;
+        tile += c.stage_bytes;
+        meta += 16;
+        pt += 4 * PART_STAGE_FLOATS;
+        if (full == full_end) {
+            full = c.bar0;
+            tile = c.ring;
+            meta = c.meta;
+            pt -= 4 * PART_STAGE_FLOATS * c.S;
+            par ^= 1u;
+        }
     }
 }
 
@@ -247,7 +261,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const Ge
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the consumers' reads of the slot come first
                 mbar_expect_tx(full, ba + bb);
                 bulk_g2s(dst, srcA, ba, full);
-                if (swiglu) bulk_g2s(dst + ba, srcB, bb, full);
+                if (swiglu) bulk_g2s(dst + geo.b_off, srcB, bb, full);
             }
             if (!dyn) tc.advance(sh);
             else if (held > 1) { t++; held--; }
@@ -324,11 +338,11 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const Ge
 
     // ================= consumer warps =================
     Consumer c;
-    c.ring = smem_u32(ring); c.part = part; c.meta = smem_u32(smem + geo.meta_off); c.bar0 = bar0; c.S = S; c.stage_bytes = geo.stage_bytes;
-    c.CG = CG; c.RG = RG; c.cg = warp % CG; c.rg = warp / CG; c.u = c.cg * 32 + lane; c.has_unit = c.u < units; c.lane = lane;
+    c.ring = smem_u32(ring); c.part = part; c.meta = smem_u32(smem + geo.meta_off); c.bar0 = bar0; c.S = S; c.stage_bytes = geo.stage_bytes; c.b_off = geo.b_off;
+    c.RG = RG; c.cg = warp % CG; c.rg = warp / CG; c.u = c.cg * 32 + lane; c.has_unit = c.u < units; c.lane = lane;
     const Act A{act_sm, p.cols, p.cols / 64};
-    float4 norm_g[4];
-    pack_prefetch_norm(p.norm_w, p.cols, norm_g);   // weights: fetched while the previous kernel is still running
+    float4 norm_g[2];
+    pack_prefetch_norm8(p.norm_w, p.cols, norm_g);   // weights: fetched while the previous kernel is still running
     {
         // The launch parameters the tile loop reads, touched while the previous kernel is still running: their first read
         // misses the constant cache, and that round trip would otherwise sit between the activations and the first tile.
@@ -479,6 +493,7 @@ int32_t launch_gemv_stream(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p
         geo.seg_tiles[s] = (geo.seg_pairs[s] + pt - 1) / pt;
         geo.total_tiles += geo.seg_tiles[s];
     }
+    geo.b_off = geo.seg_pt[0] * (uint32_t)p.seg[0].row_bytes;
     int grid = ctx->sm_count;       // one persistent CTA per SM
     if ((uint32_t)grid > pairs) grid = (int)pairs;
     if (grid < 1) grid = 1;

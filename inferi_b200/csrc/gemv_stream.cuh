@@ -36,7 +36,8 @@ __device__ __forceinline__ unsigned long long global_ns() {
     return t;
 }
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t *err, uint32_t code, unsigned long long limit_ns) {
-    if (mbar_try_wait(bar, parity)) return true;
+    for (int i = 0; i < 16; i++)   // a read of the clock stalls the warp for about a microsecond: not before the wait is a long one
+        if (mbar_try_wait(bar, parity)) return true;
     const unsigned long long t0 = global_ns();
     for (;;) {
         for (int i = 0; i < 256; i++)
@@ -452,6 +453,18 @@ __device__ __forceinline__ float unit_dot(uint32_t qtype, uint32_t row, const La
     }
 }
 
+// Two rows at shared addresses `a` and `b`; one format switch for both.
+template <uint32_t QT>
+__device__ __forceinline__ void unit_dot2(uint32_t qtype, uint32_t a, uint32_t b, const LaneConst &lc, const UnitAct &ua, float &va, float &vb) {
+    if (QT == QT_Q4_Q6) {
+        if (qtype == IB_Q4_K) { va = Unit<IB_Q4_K>::dot(a, lc, ua); vb = Unit<IB_Q4_K>::dot(b, lc, ua); }
+        else { va = Unit<IB_Q6_K>::dot(a, lc, ua); vb = Unit<IB_Q6_K>::dot(b, lc, ua); }
+        return;
+    }
+    va = unit_dot<QT>(qtype, a, lc, ua);
+    vb = unit_dot<QT>(qtype, b, lc, ua);
+}
+
 // -------------------------------------------------------------------------------------------------
 // Prologue of the streaming kernel, run by the 16 consumer warps: y = x * w -> limb form in
 // shared memory.  The RMS factor is NOT applied here: it is one scalar for the whole vector, the GEMV is linear, so the
@@ -459,27 +472,36 @@ __device__ __forceinline__ float unit_dot(uint32_t qtype, uint32_t row, const La
 // critical path: every warp leaves its part of the sum in red[warp], arrives on `ss_bar` and carries on; only the
 // epilogue warp waits there.
 // -------------------------------------------------------------------------------------------------
+// A thread converts 8 consecutive columns at a time (a 32-column group is four lanes, a 16-column sum two): with 4096 columns
+// all 512 threads take part - with 16 columns per thread half of them did, for twice as long.  `g`: the norm weights of
+// the thread's first group, fetched ahead of the wait for the previous kernel.
+constexpr uint32_t PACK_GROUPS = 4;   // groups in flight per thread: 16384 columns
+__device__ __forceinline__ void pack_prefetch_norm8(const float *__restrict__ norm_w, uint32_t cols, float4 (&g)[2]) {
+    const uint32_t grp = threadIdx.x;
+    if (norm_w && grp < cols / 8) {
+        g[0] = __ldg(reinterpret_cast<const float4 *>(norm_w) + 2 * grp);
+        g[1] = __ldg(reinterpret_cast<const float4 *>(norm_w) + 2 * grp + 1);
+    } else g[0] = g[1] = make_float4(1.f, 1.f, 1.f, 1.f);
+}
 __device__ __forceinline__ void pack_stream(uint8_t *smem, uint32_t cols, const float *__restrict__ x, const float *__restrict__ norm_w, float *red,
-                                            uint32_t ss_bar, const float4 (&g)[4], uint32_t nq) {
-    constexpr int NT = PACK_THREADS;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const uint32_t nruns = cols / 16;    // cols is a multiple of 64: runs pair up inside a warp; at most 2 * NT of them (cols <= 16384)
-    const float4 *x4 = reinterpret_cast<const float4 *>(x);
-    const float4 *w4 = reinterpret_cast<const float4 *>(norm_w);
-    PackRegs r;
+                                            uint32_t ss_bar, const float4 (&g)[2], uint32_t nq) {
+    constexpr uint32_t NT = PACK_THREADS;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, groups = cols / 8;   // cols is a multiple of 64: whole four-lane groups
+    const float4 *x4 = reinterpret_cast<const float4 *>(x), *w4 = reinterpret_cast<const float4 *>(norm_w);
+    float4 r[PACK_GROUPS][2];
 #pragma unroll
-    for (int i = 0; i < PACK_RUNS; i++) {
-        const uint32_t run = tid + NT * i;
-#pragma unroll
-        for (int j = 0; j < 4; j++) r.x[i][j] = run < nruns ? __ldcg(x4 + 4 * run + j) : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t i = 0; i < PACK_GROUPS; i++) {
+        const uint32_t grp = tid + NT * i;
+        r[i][0] = grp < groups ? __ldcg(x4 + 2 * grp) : make_float4(0.f, 0.f, 0.f, 0.f);
+        r[i][1] = grp < groups ? __ldcg(x4 + 2 * grp + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
     if (norm_w) {
         // crates/inferi-shaders/src/rms_norm.rs:112-120: the sum of squares; the factor itself is applied by the epilogue warp
         float ss = 0.f;
 #pragma unroll
-        for (int i = 0; i < PACK_RUNS; i++)
+        for (uint32_t i = 0; i < PACK_GROUPS; i++)
 #pragma unroll
-            for (int j = 0; j < 4; j++) ss += (r.x[i][j].x * r.x[i][j].x + r.x[i][j].y * r.x[i][j].y) + (r.x[i][j].z * r.x[i][j].z + r.x[i][j].w * r.x[i][j].w);
+            for (int j = 0; j < 2; j++) ss += (r[i][j].x * r[i][j].x + r[i][j].y * r[i][j].y) + (r[i][j].z * r[i][j].z + r[i][j].w * r[i][j].w);
 #pragma unroll
         for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
         if (lane == 0) {
@@ -487,23 +509,44 @@ __device__ __forceinline__ void pack_stream(uint8_t *smem, uint32_t cols, const 
             mbar_arrive(ss_bar);   // a release: the epilogue warp's wait sees red[warp]
         }
     }
+    const uint32_t ls = cols + (nq ? 64u : 0u);   // = Act::lstride()
+    float *sc = reinterpret_cast<float *>(smem + ACT_LIMBS * ls), *sx16 = sc + cols / 32;
 #pragma unroll
-    for (int i = 0; i < PACK_RUNS; i++) {
-        const uint32_t run = tid + NT * i;
-        if ((uint32_t)(warp * 32 + NT * i) < nruns) {   // warp-uniform: both lanes of a 32-column group are present
-            const bool ok = run < nruns;
-            if (norm_w && ok) {
+    for (uint32_t i = 0; i < PACK_GROUPS; i++) {
+        const uint32_t grp = tid + NT * i;
+        if (warp * 32 + NT * i >= groups) continue;   // warp-uniform
+        const bool ok = grp < groups;
+        float4 (&v)[2] = r[i];
+        if (norm_w && ok) {
 #pragma unroll
-                for (int j = 0; j < 4; j++) {
-                    const float4 w = (i == 0) ? g[j] : __ldg(w4 + 4 * run + j);
-                    float4 &v = r.x[i][j];
-                    v.x *= w.x; v.y *= w.y; v.z *= w.z; v.w *= w.w;
-                }
+            for (int j = 0; j < 2; j++) {
+                const float4 w = i == 0 ? g[j] : __ldg(w4 + 2 * grp + j);
+                v[j].x *= w.x; v[j].y *= w.y; v[j].z *= w.z; v[j].w *= w.w;
             }
-            pack_run(r.x[i], run, cols, smem, ok, nq);
+        }
+        float amax = fmaxf(fmaxf(fmaxf(fabsf(v[0].x), fabsf(v[0].y)), fmaxf(fabsf(v[0].z), fabsf(v[0].w))),
+                           fmaxf(fmaxf(fabsf(v[1].x), fabsf(v[1].y)), fmaxf(fabsf(v[1].z), fabsf(v[1].w))));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+        const float inv = amax > 0.f ? __fdividef(127.0f, amax) : 0.f;   // 2 ulp: the limbs absorb it (|t| stays within 127 + 1e-5)
+        uint32_t w0[2], w1[2];
+        float sum = 0.f;
+#pragma unroll
+        for (int j = 0; j < 2; j++) {
+            const float e[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+            pack_four(e, inv, w0[j], w1[j], sum);
+        }
+        sum += __shfl_xor_sync(0xffffffffu, sum, 1);
+        if (ok) {
+            const uint32_t run = grp >> 1;
+            uint8_t *l0 = smem + 16 * act_chunk_pos(run, nq) + 8 * (grp & 1);
+            *reinterpret_cast<uint2 *>(l0) = make_uint2(w0[0], w0[1]);
+            *reinterpret_cast<uint2 *>(l0 + ls) = make_uint2(w1[0], w1[1]);
+            if ((grp & 3) == 0) sc[grp >> 2] = amax * ACT_UNIT;
+            if ((grp & 1) == 0) sx16[run] = sum * (amax * (1.0f / 127.0f));
         }
     }
-    named_barrier(1, NT);
+    named_barrier(1, PACK_THREADS);
 }
 
 __device__ __forceinline__ float2 residual_prefetch(const float *resid, uint32_t pair) { return __ldcg(reinterpret_cast<const float2 *>(resid + 2 * pair)); }
