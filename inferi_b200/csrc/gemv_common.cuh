@@ -10,25 +10,21 @@ constexpr int PACK_THREADS = 512;        // threads that take part in the activa
 constexpr uint32_t GEMV_MAX_COLS = 32768;
 
 // Activation form in shared memory, for `cols` columns (a multiple of 32):
-//   ACT_LIMBS int8 limbs a0, a1 [cols] each;  f32 scale s/(127 * 254) per 32 columns;  f32 sum of the quantized x per 16 columns
-//   x ~= (s/127) * (a0 + a1/254)      (resolution 1.6e-5 * max|x| of the 32-group: 16-bit block fixed point)
-//   (+ 192 bytes: in the group-major chunk order each limb array carries one 16-byte skew per group, see act_chunk_pos)
+//   ACT_LIMBS int8 limbs a0, a1 [cols] each;  f32 scale s/32512 per 32 columns;  f32 sum of the quantized x per 16 columns
+//   x ~= (s/32512) * (256 a0 + a1)     (resolution 1.5e-5 * max|x| of the 32-group: 16-bit block fixed point)
 // The 16-column sums (used for the k-quants' minimums and the Q6_K -32 terms) are sums of the QUANTIZED values, so that
 // sum_k w_k a_k is evaluated exactly for the a_k the dot products see; the only error of a GEMV is sum_k w_k (a_k - x_k),
 // 2e-5 .. 1e-4 relative.  (A third limb - 24-bit fixed point - costs a third more dp4a and 16 more registers per lane: 583
 // against 619 tok/s on the 8B architecture; the logits of the 1B architecture then differ from the f32 oracle's by 7e-4
 // instead of 2.7e-3 max-abs, at a tolerance of 2e-2.)
 constexpr int ACT_LIMBS = 2;
-__host__ __device__ inline size_t act_smem_bytes(uint32_t cols) { return (size_t)cols * ACT_LIMBS + cols / 32 * 4 + cols / 16 * 4 + 192; }
+__host__ __device__ inline size_t act_smem_bytes(uint32_t cols) { return (size_t)cols * ACT_LIMBS + cols / 32 * 4 + cols / 16 * 4; }
 
 struct Act {
     const uint8_t *base;
     uint32_t cols;
-    uint32_t nq = 0;   // 0: 16-column chunks in column order; else cols / 64: group-major order, see act_chunk_pos
-    __device__ __forceinline__ uint32_t pos(uint32_t e16) const { return nq ? (e16 & 3u) * (nq + 1) + (e16 >> 2) : e16; }
-    __device__ __forceinline__ uint32_t lstride() const { return cols + (nq ? 64u : 0u); }
-    __device__ __forceinline__ const uint4 *limb(int k) const { return reinterpret_cast<const uint4 *>(base + (size_t)k * lstride()); }
-    __device__ __forceinline__ const float *sc() const { return reinterpret_cast<const float *>(base + (size_t)ACT_LIMBS * lstride()); }
+    __device__ __forceinline__ const uint4 *limb(int k) const { return reinterpret_cast<const uint4 *>(base + (size_t)k * cols); }
+    __device__ __forceinline__ const float *sc() const { return reinterpret_cast<const float *>(base + (size_t)ACT_LIMBS * cols); }
     __device__ __forceinline__ const float *sx16() const { return sc() + cols / 32; }
 };
 
@@ -38,11 +34,11 @@ __device__ __forceinline__ int dp4a_us(uint32_t a, uint32_t b, int c) {
     asm("dp4a.u32.s32 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
     return d;
 }
-// The integer dot products of the two limbs -> the dot product in units of the group's scale.  254 d0 + d1 is formed as an
-// integer (at most 2^28 for every format's longest chain) and converted once: one multiply-add and one conversion instead of
-// two conversions and a float multiply-add, and exact up to the conversion's rounding.
+// The integer dot products of the two limbs -> the dot product in units of the group's scale.  256 d0 + d1 is formed as an
+// integer (at most 2^28 for every format's longest chain) and converted once: exact up to the conversion's rounding.
 static_assert(ACT_LIMBS == 2, "the dot products combine two limbs");
-__device__ __forceinline__ float limb_combine(const int *d) { return (float)(d[0] * 254 + d[1]); }
+__device__ __forceinline__ int limb_sum(int d0, int d1) { return d0 * 256 + d1; }
+__device__ __forceinline__ float limb_combine(const int *d) { return (float)limb_sum(d[0], d[1]); }
 __device__ __forceinline__ float h2f(uint32_t bits16) { return __half2float(__ushort_as_half((unsigned short)bits16)); }
 
 __device__ __forceinline__ void named_barrier(int id, int nthreads) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(nthreads) : "memory"); }
@@ -79,57 +75,43 @@ __device__ __forceinline__ void pack_prefetch_norm(const float *__restrict__ nor
     }
 }
 
-// Position of the 16-column chunk `run` inside a limb array.  With nq = cols / 64 the chunks are stored "group-major":
-// chunk 4u + g sits at g * (nq + 1) + u.  The lanes of a warp, each reading chunk 4u + g of its unit u, then touch
-// consecutive 16-byte words (in column order they would be 64 bytes apart: a 4-way bank conflict on every 128-bit load),
-// and the one-chunk skew between groups keeps the four chunks that neighbouring threads store apart as well.
-__device__ __forceinline__ uint32_t act_chunk_pos(uint32_t run, uint32_t nq) { return nq ? (run & 3u) * (nq + 1) + (run >> 2) : run; }
+constexpr float ACT_STEPS = 32512.0f;   // = 127 * 256: the largest |x| of a group is so many units, a0 = +-127, a1 = 0
 
-constexpr float ACT_UNIT = 1.0f / (127.0f * 254.0f);   // times a group's largest |x|: the unit of 254 a0 + a1
-
-// Four columns -> their bytes of the two limbs; `inv` = 127 / largest |x| of the group; `sum` += the quantized values in units of
-// the first limb.  Round-to-nearest-even by adding 1.5 * 2^23: the sum's low mantissa byte is the rounded value in two's
-// complement (|t| <= 127), and subtracting the constant again gives it back as a float - no conversion instructions.
-__device__ __forceinline__ void pack_four(const float (&e)[4], float inv, uint32_t &w0, uint32_t &w1, float &sum) {
-    constexpr float MAGIC = 12582912.0f;
-    uint32_t b0[4], b1[4];
+// Four columns -> their bytes of the two limbs; `inv` = ACT_STEPS / largest |x| of the group; `s0`, `s1` += the limbs.
+// One multiply-add rounds to an integer: added to 1.5 * 2^23 the value sits in the low bits of the float, in two's complement.
+// It is formed 128 too high, so that its bits 8-15 are a0 rounded to nearest and its low byte is a1 + 128.
+__device__ __forceinline__ void pack_four(const float (&e)[4], float inv, uint32_t &w0, uint32_t &w1, int &s0, int &s1) {
+    constexpr float MAGIC = 12582912.0f + 128.0f;
+    uint32_t b[4];
 #pragma unroll
-    for (int k = 0; k < 4; k++) {
-        const float t = e[k] * inv;
-        const float r0 = t + MAGIC, q0 = r0 - MAGIC;            // the limbs as floats: q0, q1
-        const float t1 = (t - q0) * 254.0f;
-        const float r1 = t1 + MAGIC, q1 = r1 - MAGIC;
-        b0[k] = __float_as_uint(r0);
-        b1[k] = __float_as_uint(r1);
-        sum += q0 + q1 * (1.0f / 254.0f);
-    }
-    // low bytes of four words -> one word
-    w0 = __byte_perm(__byte_perm(b0[0], b0[1], 0x0040), __byte_perm(b0[2], b0[3], 0x0040), 0x5410);
-    w1 = __byte_perm(__byte_perm(b1[0], b1[1], 0x0040), __byte_perm(b1[2], b1[3], 0x0040), 0x5410);
+    for (int k = 0; k < 4; k++) b[k] = __float_as_uint(fmaf(e[k], inv, MAGIC));
+    w0 = __byte_perm(__byte_perm(b[0], b[1], 0x0051), __byte_perm(b[2], b[3], 0x0051), 0x5410);
+    w1 = __byte_perm(__byte_perm(b[0], b[1], 0x0040), __byte_perm(b[2], b[3], 0x0040), 0x5410) ^ 0x80808080u;
+    s0 = dp4a_ss(w0, 0x01010101u, s0);
+    s1 = dp4a_ss(w1, 0x01010101u, s1);
 }
 
-__device__ __forceinline__ void pack_run(const float4 (&v)[4], uint32_t run, uint32_t cols, uint8_t *smem, bool store, uint32_t nq = 0) {
+__device__ __forceinline__ void pack_run(const float4 (&v)[4], uint32_t run, uint32_t cols, uint8_t *smem, bool store) {
     const int lane = threadIdx.x & 31;
-    float amax = 0.f, sum = 0.f;   // sum: of the quantized values, in units of the group's scale
+    float amax = 0.f;
+    int s0 = 0, s1 = 0;
 #pragma unroll
     for (int j = 0; j < 4; j++) amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
     amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));   // the other half of the 32-column group
-    const float inv = amax > 0.f ? __fdividef(127.0f, amax) : 0.f;   // 2 ulp: the limbs absorb it (|t| stays within 127 + 1e-5)
+    const float inv = amax > 0.f ? __fdividef(ACT_STEPS, amax) : 0.f;   // 2 ulp: the limbs absorb it (the largest |x| still rounds to 32512)
     uint32_t w0[4], w1[4];
 #pragma unroll
     for (int j = 0; j < 4; j++) {
         const float e[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
-        pack_four(e, inv, w0[j], w1[j], sum);
+        pack_four(e, inv, w0[j], w1[j], s0, s1);
     }
     if (store) {
-        const size_t ls = cols + (nq ? 64u : 0u);   // = Act::lstride()
-        uint4 *l0 = reinterpret_cast<uint4 *>(smem), *l1 = reinterpret_cast<uint4 *>(smem + ls);
-        float *sc = reinterpret_cast<float *>(smem + ACT_LIMBS * ls), *sx16 = sc + cols / 32;
-        const uint32_t at = act_chunk_pos(run, nq);
-        l0[at] = make_uint4(w0[0], w0[1], w0[2], w0[3]);
-        l1[at] = make_uint4(w1[0], w1[1], w1[2], w1[3]);
-        if ((lane & 1) == 0) sc[run >> 1] = amax * ACT_UNIT;
-        sx16[run] = sum * (amax * (1.0f / 127.0f));
+        uint4 *l0 = reinterpret_cast<uint4 *>(smem), *l1 = reinterpret_cast<uint4 *>(smem + cols);
+        float *sc = reinterpret_cast<float *>(smem + ACT_LIMBS * cols), *sx16 = sc + cols / 32;
+        l0[run] = make_uint4(w0[0], w0[1], w0[2], w0[3]);
+        l1[run] = make_uint4(w1[0], w1[1], w1[2], w1[3]);
+        if ((lane & 1) == 0) sc[run >> 1] = amax * (1.0f / ACT_STEPS);
+        sx16[run] = (float)limb_sum(s0, s1) * (amax * (1.0f / ACT_STEPS));
     }
 }
 
@@ -144,8 +126,7 @@ struct PackReduce {
 // `g` holds the norm weights of the thread's first run (from pack_prefetch_norm).
 template <int NT = PACK_THREADS>
 __device__ __forceinline__ void pack_activation(uint8_t *smem, uint32_t cols, const float *__restrict__ x, const float *__restrict__ norm_w, float eps,
-                                                float *red /* [NT/32 + 1] */, const float4 (&g)[4], const PackReduce rd = PackReduce{nullptr, 0, nullptr},
-                                                uint32_t nq = 0) {
+                                                float *red /* [NT/32 + 1] */, const float4 (&g)[4], const PackReduce rd = PackReduce{nullptr, 0, nullptr}) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const uint32_t nruns = cols / 16;    // cols is a multiple of 32, so runs pair up inside a warp
     const float4 *x4 = reinterpret_cast<const float4 *>(x);
@@ -212,7 +193,7 @@ __device__ __forceinline__ void pack_activation(uint8_t *smem, uint32_t cols, co
                     v.x = (v.x * rms) * w.x; v.y = (v.y * rms) * w.y; v.z = (v.z * rms) * w.z; v.w = (v.w * rms) * w.w;
                 }
             }
-            pack_run(r.x[i], run, cols, smem, ok, nq);
+            pack_run(r.x[i], run, cols, smem, ok);
         }
     }
     for (uint32_t base = warp * 32 + NT * PACK_RUNS; base < nruns; base += NT) {   // rows wider than the registers hold
@@ -227,7 +208,7 @@ __device__ __forceinline__ void pack_activation(uint8_t *smem, uint32_t cols, co
                 v[j].x = (v[j].x * rms) * w.x; v[j].y = (v[j].y * rms) * w.y; v[j].z = (v[j].z * rms) * w.z; v[j].w = (v[j].w * rms) * w.w;
             }
         }
-        pack_run(v, run, cols, smem, ok, nq);
+        pack_run(v, run, cols, smem, ok);
     }
     named_barrier(1, NT);
 }

@@ -3,17 +3,21 @@
 // Replaces the reference shaders crates/inferi-shaders/src/gemv_quant_{q8_0x2,q4_k,q5_k,q6_kx2}.rs (one 32-thread
 // workgroup per 4 rows, 4-byte scattered loads) and their launcher crates/inferi/src/ops/gemv_quant.rs:183-341.
 //
-// One persistent CTA per SM owns a contiguous, byte-balanced range of row pairs.
-//  * A producer warp streams the CTA's rows from HBM into a shared-memory ring with bulk asynchronous copies
-//    (cp.async.bulk, one copy per tile of up to 8 contiguous row pairs, completion on an mbarrier).  It starts
-//    before the kernel waits for its predecessor (programmatic dependent launch): weights never depend on the
-//    previous kernel, so the ring fills while that kernel is still finishing.
-//  * Sixteen consumer warps split a row's columns: every lane owns one 64-weight unit of the row and keeps that
-//    unit's activations — two int8 limbs per column, see gemv_common.cuh — in registers for the whole kernel, so
-//    the inner loop touches shared memory only for weights.  Per weight the work is a byte mask and dp4a.
-//  * Per row the lane partials are shuffled down, per-warp partials meet in shared memory, and the last warp of a
-//    row group to arrive adds them in a fixed order and runs the epilogue (store / residual add / SwiGLU /
-//    RoPE + KV append / arg-max).  No warp ever waits for another one except through the ring.
+// One persistent CTA per SM, as two pipelines (one where all warps are needed for one row).  Each has:
+//  * A producer warp that streams rows from HBM into its part of a shared-memory ring with bulk asynchronous copies
+//    (cp.async.bulk, one copy per tile of contiguous row pairs, completion on an mbarrier).  It starts before the kernel
+//    waits for its predecessor (programmatic dependent launch): weights never depend on the previous kernel, so the ring
+//    fills while that kernel is still finishing.
+//  * Sixteen consumer warps split a row's columns in blocks of 256 and work on eight rows at a time.  A warp's activations - two
+//    int8 limbs per column, see gemv_common.cuh - stay in registers for the whole kernel as operands of integer mma, so
+//    the inner loop touches shared memory for weights and scales only (gemv_stream.cuh).
+//  * Per-warp partial row sums meet in shared memory; the epilogue warp adds them in a fixed order and runs the epilogue
+//    (store / residual add / SwiGLU / RoPE + KV append / arg-max).  No warp ever waits for another one except through the ring.
+// What bounds it: a launch that streams, HBM (gate/up of an 8B model, 66 MB: 12.7 us, 5.2 TB/s with the fixed part); every launch
+// carries 3-4 us that no byte moves in - the input vector from L2, its packing, the B operands, the first tile's products and the
+// last tile's epilogue, one after the other - which is most of a short one (4096 x 4096 Q4_K, 9.4 MB: 4.7 us).  Byte dot products on
+// lanes that each own 64 columns, one producer and one epilogue warp: 15.5 and 5.8 us; there a tile took about 0.9 us whatever its size
+// (a producer's or an epilogue's latency per tile), and the dot products as long as HBM.
 // Every wait on an mbarrier is bounded; a wait that gives up raises the context's error word and carries on.
 #include "gemv_stream.cuh"
 
@@ -23,21 +27,20 @@ namespace ib {
 
 
 struct StreamGeom {
-    uint32_t stages, stage_bytes, act_off, part_off, bar_off, b_off;   // b_off: gate/up - where the up rows start inside a stage
+    uint32_t stages, stage_bytes, act_off, part_off, bar_off;
     // the launch's tiles in hand-out order: per segment the pairs, the pairs per tile and the tiles; bytes per pair
     uint32_t seg_pairs[3], seg_pt[3], seg_tiles[3], seg_cost[3], total_tiles, meta_off;
-    uint32_t dynamic;   // 1: tiles are claimed from a counter; 0: every CTA streams its own byte-balanced range of pairs
-    uint32_t head_per_cta, head_tiles, tail_pt;   // counter hand-out: see tile_of
+    uint32_t NB, CG, RG, mode;   // see Split
+    uint32_t P;            // pipelines
+    uint32_t ahead;        // stages: how far the first round of copies runs ahead of their arrival
+    uint32_t slices;       // lanes of the epilogue warp that share the addition of a pair's partial sums
+    uint32_t unit;   // tiles are claimed from a counter, so many at a time; 0: every CTA streams its own byte-balanced range of pairs
+    uint32_t head;   // counter hand-out: so many tiles of every pipeline are its own by position
 };
 
 // Counter hand-out (one segment only): tile number -> (segment 0, first pair, pairs); pairs == 0 past the last tile.
-// The first `head_tiles` tiles hold `seg_pt[0]` pairs each and belong to the CTAs by position (CTA b: tiles b * head_per_cta
-// ...); the rest of the pairs follow as smaller tiles of `tail_pt` pairs, claimed from the counter.
 __device__ __forceinline__ uint4 tile_of(const StreamGeom &g, uint32_t t) {
-    const uint32_t np = g.seg_pairs[0];
-    uint32_t first, pt;
-    if (t < g.head_tiles) { pt = g.seg_pt[0]; first = t * pt; }
-    else { pt = g.tail_pt; first = g.head_tiles * g.seg_pt[0] + (t - g.head_tiles) * pt; }
+    const uint32_t np = g.seg_pairs[0], pt = g.seg_pt[0], first = t * pt;
     if (first >= np) return make_uint4(0, 0, 0, 0);
     return make_uint4(0, first, (np - first) < pt ? (np - first) : pt, 0);
 }
@@ -45,87 +48,126 @@ __device__ __forceinline__ uint4 tile_of(const StreamGeom &g, uint32_t t) {
 // ---- consumer side ----
 struct Consumer {
     uint32_t ring;        // shared address of the ring
-    uint32_t part;        // shared address of the per-stage partial sums [stages][2][CW][PT_MAX]
+    uint32_t part;        // shared address of this column group's partial sums of the first stage
     uint32_t meta;        // shared address of [stages] (segment, first pair, pairs, -) descriptors written by the producer
-    uint32_t bar0, S, stage_bytes, b_off;
-    uint32_t RG, cg, rg, u;
-    bool has_unit;
+    uint32_t bar0, S, stage_bytes;
+    uint32_t zeros;            // shared address of 16 zero bytes
+    uint32_t stream, RG, pt;   // the stream's stages: stream, stream + RG, ... < S; pairs per tile
+    uint32_t blk, nb;          // the warp's first block of 256 columns, blocks
     int lane;
 };
 
-// Offset (in floats) of the partial of (row of the pair, column-group warp, pair of the tile) inside a stage's block:
-// pairs are the fastest index, so that the lanes of the epilogue warp (one pair each) read consecutive words.
-__device__ __forceinline__ uint32_t part_index(uint32_t row, uint32_t cg, uint32_t pr) { return (row * CW + cg) * PT_MAX + pr; }
+// Partial sums of a stage: [column group][2 * pair + row of the pair], so that the epilogue warp's lanes (one pair each) read
+// consecutive pairs of words.
 constexpr uint32_t PART_STAGE_FLOATS = 2 * CW * PT_MAX;
 
-// A consumer warp: its lanes' 64-column units of every row pair of every tile.  Per tile it waits for the weights, leaves
-// two partial sums per pair (its columns of the two rows) in the stage's partial block and arrives on the stage's "done"
-// barrier.  It never waits for another consumer warp: adding up the column groups and everything that follows is the
-// epilogue warp's work.
-// What bounds the short launches is this loop's instruction stream, so whatever does not change from tile to tile is carried in
-// registers by additions and whatever only changes with the segment is set when the segment does.  (With that, one conversion per
-// pair of limb sums and the eight-column packing, a token's launches of an 8B Q4_K_M model went from 1632 to 1550 us.)
-template <uint32_t QT>
+// A consumer warp.  The tiles of a CTA go round-robin to RG streams of CG warps each, so that the streams' waits, loads and
+// reductions overlap.  Per tile a warp waits for the weights, leaves its columns' part of every row sum in the stage's partial
+// block, 8 rows at a time, and arrives on the stage's "done" barrier.  It never waits for another consumer warp: adding up the
+// column groups and everything that follows is the epilogue warp's work.
+template <uint32_t QT, uint32_t MODE>
 __device__ __forceinline__ void consume_tiles(const GemvParams &p, const Consumer &c, const Act &A) {
-    const int lane = c.lane;
-    UnitAct ua;
+    const uint32_t g = c.lane >> 2, t = c.lane & 3;
     LaneConst lc;
+    constexpr bool FOUR = MODE == ROWS4;
+    constexpr uint32_t NB = MODE == ROWS8 ? 2 : NB_MAX;
+    uint32_t B[NB][8];
+    UnitAct ua[2];
     constexpr bool ONE_TYPE = (QT != QT_MIXED && QT != QT_Q4_Q6);
-    const bool swiglu = p.epi == EPI_SWIGLU;   // gate rows, then up rows, in one tile: a "pair" is gate row r + up row r
-    const uint32_t rb0 = (uint32_t)p.seg[0].row_bytes, rb1 = (uint32_t)p.seg[1].row_bytes, rb2 = (uint32_t)p.seg[2].row_bytes, RG = c.RG, rg = c.rg;
-    uint32_t cur_type = ONE_TYPE ? QT : p.seg[0].qtype, cur_s = 0, stride = swiglu ? rb0 : 2 * rb0, step = RG * stride, to_b = swiglu ? c.b_off : rb0;
-    uint32_t row_off = rg * stride;
-    // The lane's activations go into registers in the layout of the first segment's format before the first tile is
-    // waited for: the copy of that tile and this load overlap.
-    unit_init<QT>(cur_type, c.u, lc);
-    if (c.has_unit) load_unit_act(cur_type, c.u, A, ua);
-    uint32_t full = c.bar0, tile = c.ring, meta = c.meta, par = 0;
-    uint32_t pt = c.part + 4 * part_index(lane >> 4, c.cg, rg);
-    const uint32_t full_end = c.bar0 + 8 * c.S, to_done = 16 * c.S;
-    const bool up = lane & 16, writer = (lane & 15) == 0;
+    const bool swiglu = p.epi == EPI_SWIGLU;   // a "pair" is gate row r + up row r: 4 gate rows, then their 4 up rows, at a time
+    const uint32_t act = smem_u32(A.base), sc0 = act + ACT_LIMBS * A.cols, sx0 = sc0 + A.cols / 8;
+    // The lane's activations go into registers in the order of a format's B operand: for the first segment before the first tile
+    // is waited for (the copy of that tile and this load overlap), again when a segment of another format begins.
+    auto enter = [&](uint32_t qtype, uint32_t stride) {
+        with_format<QT>(qtype, [&](auto f) {
+            lc.sc = sc0;
+            lc.sx = sx0;
+            f.template init<FOUR>(g, t, stride, c.blk, lc);
+#pragma unroll
+            for (uint32_t i = 0; i < NB; i++) {
+                if (i < c.nb) f.operand(FOUR && (i & 1) ? g ^ 4 : g, t, act + (g & 1) * A.cols, c.zeros, c.blk + i, B[i]);
+                else
+                    for (int k = 0; k < 8; k++) B[i][k] = 0;
+            }
+            if (MODE == ROWS8) {
+                f.template unit<FOUR>(lc, 0, ua[0]);
+                if (c.nb == 2) f.template unit<FOUR>(lc, 1, ua[1]);
+            }
+        });
+    };
+    uint32_t cur_type = ONE_TYPE ? QT : p.seg[0].qtype, cur_s = 0, stride = (uint32_t)p.seg[0].row_bytes;
+    enter(cur_type, stride);
+    const uint32_t together = FOUR ? 4 : 8, half = together / 2;   // rows at a time; gate/up: gate rows, then their up rows
+    const uint32_t add = swiglu ? half : together, row_of = g & (add - 1), b_off = swiglu && (g & half) ? c.pt * stride : 0;   // the up rows follow a full tile's gate rows
+    const uint32_t part0 = c.part + 4 * (swiglu ? 2 * row_of + ((g & half) ? 1 : 0) : row_of), out_step = 4 * together;
+    const bool writer = t == 0 && g < together;
+    const bool lone = FOUR && !lc.first;   // 4 rows: this lane's units are in the second block of a step, which the last step may lack
+    uint32_t st = c.stream, par = 0, ring = c.ring;   // ring: address of stage st
 #pragma unroll 1
     for (;;) {
-        if (!mbar_wait(full, par, p.err, 1, p.wait_ns)) return;   // the error word is raised; give up on this CTA's rows
-        const uint4 tm = lds128(meta);
+        if (!mbar_wait(c.bar0 + 8 * st, par, p.err, 1, p.wait_ns)) return;   // the error word is raised; give up on this CTA's rows
+        const uint4 tm = lds128(c.meta + 16 * st);
         const uint32_t n = tm.z;
-        if (n == 0) break;   // no tiles left
+        if (n == 0) {   // no tiles left
+            if (c.lane == 0) mbar_arrive(c.bar0 + 8 * (2 * c.S + st));
+            break;
+        }
         if (tm.x != cur_s) {
             cur_s = tm.x;
-            const uint32_t rb = cur_s == 1 ? rb1 : rb2;
-            stride = 2 * rb;
-            step = RG * stride;
-            to_b = rb;
-            row_off = rg * stride;
-            if (!ONE_TYPE) {
-                const uint32_t qtype = cur_s == 1 ? p.seg[1].qtype : p.seg[2].qtype;
-                if (qtype != cur_type) {   // (re)load this lane's activations in the layout of the segment's format
-                    cur_type = qtype;
-                    unit_init<QT>(qtype, c.u, lc);
-                    if (c.has_unit) load_unit_act(qtype, c.u, A, ua);
-                }
-            }
+            const uint32_t qtype = ONE_TYPE ? QT : (cur_s == 1 ? p.seg[1].qtype : p.seg[2].qtype);
+            const uint32_t rb = (uint32_t)(cur_s == 1 ? p.seg[1].row_bytes : p.seg[2].row_bytes);
+            if (qtype != cur_type || rb != stride) enter(qtype, rb);
+            cur_type = qtype;
+            stride = rb;
         }
-        uint32_t at = tile + row_off, out = pt;
-        for (uint32_t pr = rg; pr < n; pr += RG, at += step, out += 4 * RG) {
-            float va = 0.f, vb = 0.f;
-            if (c.has_unit) unit_dot2<QT>(cur_type, at, at + to_b, lc, ua, va, vb);
-            // one shuffle tree for both rows: after the first exchange the upper half-warp carries row B
-            float v = (up ? vb : va) + __shfl_xor_sync(0xffffffffu, up ? va : vb, 16);
+        const uint32_t base = ring + b_off, rows = swiglu ? n : 2 * n;
+        uint32_t out = part0 + st * (4 * PART_STAGE_FLOATS);
+        for (uint32_t r = row_of, first = 0; first < rows; first += add, r += add, out += out_step) {
+            // rows past the tile's last one repeat it: what they give is not used
+            const uint32_t row = base + (r < rows ? r : rows - 1) * stride;
+            float v = 0.f;
+            with_format<QT>(cur_type, [&](auto f) {   // straight-line code: the steps' loads and products overlap
+                if constexpr (FOUR) {
+                    f.template unit<true>(lc, 0, ua[0]);
+                    v = f.template dot<true>(row, lc, 0, B[0], B[1], ua[0]);
+                    if (c.nb == 1 && lone) v = 0.f;
+                    if (c.nb > 2) {
+                        f.template unit<true>(lc, 1, ua[1]);
+                        const float y = f.template dot<true>(row, lc, 1, B[2], B[3], ua[1]);
+                        v += c.nb == 3 && lone ? 0.f : y;
+                    }
+                } else if constexpr (MODE == ROWS8_LONG) {
+                    if (c.nb == NB_MAX) {
 #pragma unroll
-            for (int o = 8; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-            if (writer) asm volatile("st.shared.f32 [%0], %1;" ::"r"(out), "f"(v) : "memory");   // lane 0 holds row A's sum, lane 16 row B's
+                        for (uint32_t i = 0; i < NB_MAX; i++) {
+                            f.template unit<false>(lc, i, ua[i & 1]);
+                            v += f.template dot<false>(row, lc, i, B[i], B[i], ua[i & 1]);
+                        }
+                    } else {
+#pragma unroll
+                        for (uint32_t i = 0; i < NB_MAX - 1; i++)
+                            if (i < c.nb) {
+                                f.template unit<false>(lc, i, ua[0]);
+                                v += f.template dot<false>(row, lc, i, B[i], B[i], ua[0]);
+                            }
+                    }
+                } else {
+                    v = f.template dot<false>(row, lc, 0, B[0], B[0], ua[0]);
+                    if (c.nb == 2) v += f.template dot<false>(row, lc, 1, B[1], B[1], ua[1]);
+                }
+            });
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            if (FOUR) v += __shfl_xor_sync(0xffffffffu, v, 16);
+            if (writer) asm volatile("st.shared.f32 [%0], %1;" ::"r"(out), "f"(v) : "memory");
         }
-        __syncwarp();   // lane 16's partials are ordered before lane 0's arrival (a release)
-        if (lane == 0) mbar_arrive(full + to_done);   // this warp is done with the stage: weights read, partials left
-        full += 8;
-        tile += c.stage_bytes;
-        meta += 16;
-        pt += 4 * PART_STAGE_FLOATS;
-        if (full == full_end) {
-            full = c.bar0;
-            tile = c.ring;
-            meta = c.meta;
-            pt -= 4 * PART_STAGE_FLOATS * c.S;
+        __syncwarp();   // the lanes' partials are ordered before lane 0's arrival (a release)
+        if (c.lane == 0) mbar_arrive(c.bar0 + 8 * (2 * c.S + st));   // this warp is done with the stage: weights read, partials left
+        st += c.RG;
+        ring += c.stage_bytes;
+        if (st >= c.S) {
+            st = c.stream;
+            ring = c.ring;
             par ^= 1u;
         }
     }
@@ -134,155 +176,175 @@ __device__ __forceinline__ void consume_tiles(const GemvParams &p, const Consume
 // The epilogue warp: per tile it waits until every consumer warp has left its partials, adds up the column groups in a
 // fixed order (bitwise deterministic results), hands the stage back to the producer and runs the epilogue of the tile's
 // row pairs, one pair per lane.
-__device__ __forceinline__ void finish_tiles(const GemvParams &p, uint32_t part, uint32_t meta, uint32_t bar0, uint32_t S, uint32_t CG, int lane,
-                                             const float *red, unsigned long long &best) {
-    uint32_t st = 0, par = 0;
+__device__ __forceinline__ void finish_tiles(const GemvParams &p, const StreamGeom &geo, uint32_t part, uint32_t meta, uint32_t bar0, uint32_t pipe,
+                                             uint32_t lane, const float *red, unsigned long long &best) {
+    const uint32_t S = geo.stages, CG = geo.CG, slices = geo.slices, width = 32 / slices;   // lanes: `slices` groups of `width` pairs
+    const uint32_t pr = lane % width, slice = lane / width;
+    uint32_t st = pipe, par = 0;
     float rms = 1.0f;
-    bool rms_known = p.norm_w == nullptr;
+    if (p.norm_w) {
+        // RMSNorm factor of the input vector (crates/inferi-shaders/src/rms_norm.rs:112-120): the consumer warps left
+        // their parts of the sum of squares in `red`; added in a fixed order
+        if (!mbar_wait(bar0 + 8 * (3 * S), 0, p.err, 6, p.wait_ns)) return;
+        float t = 0.f;
+#pragma unroll
+        for (int w = 0; w < PACK_THREADS / 32; w++) t += red[w];
+        rms = 1.0f / sqrtf(t / (float)p.cols + p.eps);
+    }
     const bool residual = p.epi == EPI_RESIDUAL;
 #pragma unroll 1
-    for (;; st = (st + 1 == S) ? 0 : st + 1, par ^= (st == 0) ? 1u : 0u) {
-        if (!mbar_wait(bar0 + 8 * st, par, p.err, 1, p.wait_ns)) return;
+    for (;;) {
+        // the pairs' residual values are requested before the wait for the dot products: the L2 round trip overlaps it
+        float2 rpre = make_float2(0.f, 0.f);
+        if (residual) {
+            if (!mbar_wait(bar0 + 8 * st, par, p.err, 1, p.wait_ns)) return;
+            const uint4 tm = lds128(meta + 16 * st);
+            if (lane < tm.z) rpre = residual_prefetch(p.resid, tm.y + lane);
+        }
+        if (!mbar_wait(bar0 + 8 * (2 * S + st), par, p.err, 5, p.wait_ns)) return;   // (implies the tile's announcement)
         const uint4 tm = lds128(meta + 16 * st);
         const uint32_t s = tm.x, first_pair = tm.y, n = tm.z;
         if (n == 0) break;
-        const bool mine = (uint32_t)lane < n;
-        // the pair's residual values are requested before the wait for the dot products: the L2 round trip overlaps it
-        float2 rpre = make_float2(0.f, 0.f);
-        if (residual && mine) rpre = residual_prefetch(p.resid, first_pair + lane);
-        if (!rms_known) {
-            // RMSNorm factor of the input vector (crates/inferi-shaders/src/rms_norm.rs:112-120): the consumer warps left
-            // their parts of the sum of squares in `red`; added in a fixed order
-            if (!mbar_wait(bar0 + 8 * (3 * S), 0, p.err, 6, p.wait_ns)) return;
-            float t = 0.f;
-#pragma unroll
-            for (int w = 0; w < PACK_THREADS / 32; w++) t += red[w];
-            rms = 1.0f / sqrtf(t / (float)p.cols + p.eps);
-            rms_known = true;
-        }
-        if (!mbar_wait(bar0 + 8 * (2 * S + st), par, p.err, 5, p.wait_ns)) return;
+        const bool mine = lane < n;
         float va = 0.f, vb = 0.f;
-        if (mine) {
-            const uint32_t pt = part + 4 * (st * PART_STAGE_FLOATS);
-            for (uint32_t g = 0; g < CG; g++) {
-                va += __uint_as_float(lds32(pt + 4 * part_index(0, g, lane)));
-                vb += __uint_as_float(lds32(pt + 4 * part_index(1, g, lane)));
-            }
+        const uint32_t at = part + 4 * (st * PART_STAGE_FLOATS + 2 * pr);
+#pragma unroll 2
+        for (uint32_t g = slice; g < CG; g += slices) {
+            const uint2 v = lds64(at + 4 * (g * 2 * PT_MAX));
+            va += __uint_as_float(v.x);
+            vb += __uint_as_float(v.y);
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(bar0 + 8 * (S + st));   // partials read: the producer may refill the stage
+#pragma unroll
+        for (uint32_t o = 16; o; o >>= 1)
+            if (o >= width) {
+                va += __shfl_xor_sync(0xffffffffu, va, o);
+                vb += __shfl_xor_sync(0xffffffffu, vb, o);
+            }
         if (mine) epilogue(p, s, first_pair + lane, va * rms, vb * rms, best, rpre);
+        st += geo.P;
+        if (st >= S) {
+            st = pipe;
+            par ^= 1u;
+        }
     }
 }
 
 // ---- the kernel ----
 // Shared-memory barriers: full[S] (the producer's expect_tx arrival + the copy's bytes), empty[S] (one arrival: the
 // epilogue warp has read the stage's partials, which implies that every consumer warp is done with its weights),
-// done[S] (one arrival per working consumer warp), ss (one arrival per consumer warp: its part of the input's sum of squares).
+// done[S] (one arrival per consumer warp of the tile's stream), ss (one arrival per consumer warp: its part of the input's sum of squares).
 // One instance per weight format (or format pair); what the launch does with the row sums is a run-time switch in the
 // epilogue warp, so that the launches of a token graph share their code.
-template <uint32_t QT>
+template <uint32_t QT, uint32_t MODE>
 __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const GemvParams p, const StreamGeom geo) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ float red[PACK_THREADS / 32 + 1];
+    __shared__ uint4 zeros;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    if (threadIdx.x == 0) zeros = make_uint4(0, 0, 0, 0);
 
-    uint8_t *ring = smem;
     uint8_t *act_sm = smem + geo.act_off;
-    const uint32_t part = smem_u32(smem + geo.part_off);                        // [stages][2][CW][PT_MAX] floats
+    const uint32_t part = smem_u32(smem + geo.part_off);                        // [stages][CW][2 * PT_MAX] floats
     const uint32_t bar0 = smem_u32(smem + geo.bar_off);                         // full[stages], empty[stages], done[stages]
     const uint32_t S = geo.stages;
 
-    const uint32_t units = p.cols / 64;
-    const uint32_t CG = (units + 31) / 32;       // warps that split one row's columns
-    const uint32_t RG = CW / CG;                 // row groups working side by side
-    const uint32_t active = CG * RG;             // consumer warps with work
+    const uint32_t CG = geo.CG, RG = geo.RG, active = CG * RG;   // consumer warps with work
 
     if (threadIdx.x <= 3 * S) {
         const uint32_t which = threadIdx.x / S;
-        mbar_init(bar0 + 8 * threadIdx.x, which == 2 ? active : (which == 3 ? (uint32_t)CW : 1u));
+        mbar_init(bar0 + 8 * threadIdx.x, which == 2 ? CG : (which == 3 ? (uint32_t)CW : 1u));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
     if (p.pdl) asm volatile("griddepcontrol.launch_dependents;");
 
-    if (warp == W_PRODUCER) {
+    if (warp >= W_PRODUCER && warp < W_EPILOGUE) {
         // ================= producer warp: picks tiles and streams them =================
         // With many tiles per CTA they are handed out through a counter in global memory, so that a CTA which starts late
         // (its SM was the last to be freed by the previous kernel) or runs slowly takes fewer of them.  With few tiles per
-        // CTA a tile is too coarse a unit for that: every CTA then streams its own byte-balanced range of row pairs, cut
-        // into tiles.  Either way the slot's descriptor tells the other warps what the tile is.  Lane 0 picks, waits for
+        // CTA a tile is too coarse a unit for that: every pipeline then streams its own byte-balanced range of row pairs, cut
+        // into tiles.  Either way the slot's descriptor tells the other warps what the tile is.  One lane picks, waits for
         // the slot, announces the tile and issues its bulk copies.
+        // A tile costs this lane 0.4-0.7 us, most of it between issuing a copy and being able to prepare the next one, and a
+        // claim another 0.6: with one producer per SM that, not HBM, was the pace of the launches that stream.  Hence two pipelines.
+        const uint32_t pipe = warp - W_PRODUCER;
+        if (pipe >= geo.P || lane != 0) return;
         uint4 *meta = reinterpret_cast<uint4 *>(smem + geo.meta_off);
-        const bool dyn = geo.dynamic != 0;
+        const bool dyn = geo.unit != 0, swiglu = p.epi == EPI_SWIGLU;
+        const uint32_t pipes = gridDim.x * geo.P, me = blockIdx.x * geo.P + pipe;
         Share sh;
         TileCursor tc;
-        const bool swiglu = p.epi == EPI_SWIGLU;
-        if (!dyn) {
-            make_share(p, geo.stage_bytes, RG, sh);
+        // counter hand-out: a pipeline's first tiles are its own by position (no round trip before the first copy), every
+        // later unit of tiles is claimed
+        uint32_t held = 0, t = 0;
+        if (dyn) {
+            held = geo.head;
+            t = me * held;
+        } else {
+            make_share(p, geo.seg_pt, pipes, me, sh);
             tc.init(sh);
         }
-        uint32_t st = 0, par = 1;   // parity of the slot's previous use ("1" before the first one: nothing to wait for)
+        uint32_t cost = swiglu ? (uint32_t)p.seg[0].row_bytes : geo.seg_cost[0], cost_b = (uint32_t)p.seg[1].row_bytes, cur = 0;
+        const uint8_t *w = p.seg[0].w, *wb = p.seg[1].w;
+        uint32_t st = pipe, ring = smem_u32(smem), par = 1, ends = 0;   // par: parity of the slot's previous use ("1" before the first one); ends: end markers, one per stream
         bool first_round = true;
-        // counter hand-out: the CTA's first tiles are its own by position (no round trip before the first copy), every
-        // later one is claimed
-        uint32_t t = blockIdx.x * geo.head_per_cta, held = geo.head_per_cta;
-        for (uint32_t k = 0;; k++, st = (st + 1 == S) ? 0 : st + 1) {
-            if (st == 0 && k > 0) { par ^= 1u; first_round = false; }
-            // the tile after this one is claimed now: the counter's round trip overlaps the wait for the slot
-            const uint4 tm = dyn ? tile_of(geo, t) : (tc.valid(sh) ? make_uint4(tc.seg, tc.next, tc.count(sh), 0) : make_uint4(0, 0, 0, 0));
-            uint32_t tn = 0;
-            if (dyn && held == 1 && tm.z != 0 && lane == 0) tn = geo.head_tiles + atomicAdd(p.tile_claim, 1u);
-            uint32_t ok = 1;
-            if (!first_round && lane == 0) ok = mbar_wait(bar0 + 8 * (S + st), par, p.err, 2, p.wait_ns) ? 1u : 0u;
-            ok = __shfl_sync(0xffffffffu, ok, 0);
-            if (!ok) break;
-            const uint32_t s = tm.x, first_pair = tm.y, n = tm.z;
-            const uint32_t full = bar0 + 8 * st;
-            if (lane == 0) meta[st] = tm;
-            if (n == 0) {
-                // no tiles left: tell the others, and let the last CTA to get here clear the counters for their next use
-                if (lane == 0) {
-                    mbar_arrive(full);
-                    if (dyn && atomicAdd(p.tile_claim + 1, 1u) == gridDim.x - 1) {
-                        p.tile_claim[0] = 0u;
-                        p.tile_claim[1] = 0u;
-                    }
+        for (;;) {
+            uint4 tm = make_uint4(0, 0, 0, 0);
+            if (dyn) {
+                if (held == 0) {
+                    t = geo.head * pipes + geo.unit * atomicAdd(p.tile_claim, 1u);
+                    held = geo.unit;
                 }
-                break;
-            }
-            const uint32_t cost = s == 0 ? geo.seg_cost[0] : (s == 1 ? geo.seg_cost[1] : geo.seg_cost[2]);
-            const uint32_t dst = smem_u32(ring + (size_t)st * geo.stage_bytes);
-            const uint32_t ba = swiglu ? n * (uint32_t)p.seg[0].row_bytes : n * cost;
-            const uint32_t bb = swiglu ? n * (uint32_t)p.seg[1].row_bytes : 0u;
-            const uint8_t *srcA = swiglu ? p.seg[0].w + (size_t)first_pair * p.seg[0].row_bytes : p.seg[s].w + (size_t)first_pair * cost;
-            const uint8_t *srcB = swiglu ? p.seg[1].w + (size_t)first_pair * p.seg[1].row_bytes : nullptr;
-            if (lane == 0) {
+                tm = tile_of(geo, t);
+            } else if (tc.valid(sh)) tm = make_uint4(tc.seg, tc.next, tc.count(sh), 0);
+            const uint32_t n = tm.z, full = bar0 + 8 * st;
+            // Slot free?  In the first round every slot is; there the copies in flight are kept to what the memory system's latency
+            // needs: a ring-full of them would only queue up, and the input vector's few kilobytes behind them.
+            if (!first_round ? !mbar_wait(bar0 + 8 * (S + st), par, p.err, 2, p.wait_ns)
+                             : (st >= geo.ahead && !mbar_wait(bar0 + 8 * (st - geo.ahead), 0, p.err, 1, p.wait_ns)))
+                return;
+            meta[st] = tm;
+            if (n == 0) {
+                // no tiles left: tell the others, and let the last pipeline to get here clear the counters for their next use
+                mbar_arrive(full);
+                if (++ends == geo.RG / geo.P) break;
+            } else {
+                if (tm.x != cur) {
+                    cur = tm.x;
+                    cost = cur == 1 ? geo.seg_cost[1] : geo.seg_cost[2];
+                    w = cur == 1 ? p.seg[1].w : p.seg[2].w;
+                }
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the consumers' reads of the slot come first
+                const uint32_t ba = n * cost, bb = swiglu ? n * cost_b : 0u, dst = ring + st * geo.stage_bytes;
                 mbar_expect_tx(full, ba + bb);
-                bulk_g2s(dst, srcA, ba, full);
-                if (swiglu) bulk_g2s(dst + geo.b_off, srcB, bb, full);
+                bulk_g2s(dst, w + (size_t)tm.y * cost, ba, full);
+                if (swiglu) bulk_g2s(dst + geo.seg_pt[0] * cost, wb + (size_t)tm.y * cost_b, bb, full);
+                if (!dyn) tc.advance(sh);
+                else { t++; held--; }
             }
-            if (!dyn) tc.advance(sh);
-            else if (held > 1) { t++; held--; }
-            else t = __shfl_sync(0xffffffffu, tn, 0);
-            // The CTA's first tile travels alone: with a ring-full of copies in flight at once the copy engine interleaves
-            // them and all of them - the first one too - arrive when the last byte does, which is later than the consumers
-            // are ready for the first tile.  The others follow as soon as the first has landed.
-            if (k == 0) {
-                uint32_t ok0 = 1;
-                if (lane == 0) ok0 = mbar_wait(bar0, 0, p.err, 1, p.wait_ns) ? 1u : 0u;
-                if (!__shfl_sync(0xffffffffu, ok0, 0)) break;
+            st += geo.P;
+            if (st >= S) {
+                st = pipe;
+                par ^= 1u;
+                first_round = false;
             }
+        }
+        if (dyn && atomicAdd(p.tile_claim + 1, 1u) == pipes - 1) {
+            p.tile_claim[0] = 0u;
+            p.tile_claim[1] = 0u;
         }
         return;
     }
 
-    if (warp == W_EPILOGUE) {
+    if (warp >= W_EPILOGUE) {
         // ================= epilogue warp =================
+        const uint32_t pipe = warp - W_EPILOGUE;
+        if (pipe >= geo.P) return;
         // outputs (and the residual it reads) are touched by the previous kernels of the stream: wait for them like the consumers do
         if (p.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
-        if (p.reduce_src) {
+        if (p.reduce_src && pipe == 0) {
             // Tensor parallel: the previous row-split GEMV of every rank leaves its partial sums in this rank's slots.  The sum
             // (x + the partials in rank order, so every rank gets the same bits) is formed once per rank: this warp adds up
             // the groups of 32 columns that fall to its CTA and stores them as the new residual stream; the consumer warps of
@@ -302,23 +364,24 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const Ge
             __syncwarp();
             if (lane == 0 && cnt) asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p.reduce_done), "r"(cnt) : "memory");
         }
+        const uint32_t epis = geo.P;   // epilogue warps at work
         unsigned long long best = 0ull;
-        finish_tiles(p, part, smem_u32(smem + geo.meta_off), bar0, S, CG, lane, red, best);
+        finish_tiles(p, geo, part, smem_u32(smem + geo.meta_off), bar0, pipe, lane, red, best);
         if (p.epi == EPI_ARGMAX) {
 #pragma unroll
             for (int o = 16; o; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
             uint32_t last = 0;
             if (lane == 0) {
-                p.argmax_slots[blockIdx.x] = best;
+                p.argmax_slots[blockIdx.x * epis + pipe] = best;
                 __threadfence();
-                last = (atomicAdd(p.argmax_counter, 1u) == gridDim.x - 1) ? 1u : 0u;
+                last = (atomicAdd(p.argmax_counter, 1u) == gridDim.x * epis - 1) ? 1u : 0u;
             }
             last = __shfl_sync(0xffffffffu, last, 0);
             if (last) {
-                // the last CTA to arrive folds every CTA's candidate; no CTA waits for another
+                // the last pipeline to arrive folds all candidates; no CTA waits for another
                 __threadfence();
                 unsigned long long b = 0ull;
-                for (uint32_t i = lane; i < gridDim.x; i += 32) b = max(b, __ldcg(p.argmax_slots + i));
+                for (uint32_t i = lane; i < gridDim.x * epis; i += 32) b = max(b, __ldcg(p.argmax_slots + i));
 #pragma unroll
                 for (int o = 16; o; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
                 if (lane == 0) {
@@ -338,9 +401,15 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const Ge
 
     // ================= consumer warps =================
     Consumer c;
-    c.ring = smem_u32(ring); c.part = part; c.meta = smem_u32(smem + geo.meta_off); c.bar0 = bar0; c.S = S; c.stage_bytes = geo.stage_bytes; c.b_off = geo.b_off;
-    c.RG = RG; c.cg = warp % CG; c.rg = warp / CG; c.u = c.cg * 32 + lane; c.has_unit = c.u < units; c.lane = lane;
-    const Act A{act_sm, p.cols, p.cols / 64};
+    const uint32_t cg = warp % CG, stream = warp / CG, blocks = p.cols / 256;
+    c.zeros = smem_u32(&zeros); c.meta = smem_u32(smem + geo.meta_off); c.bar0 = bar0; c.S = S; c.lane = lane;
+    c.part = part + 4 * (cg * 2 * PT_MAX);
+    c.stream = stream; c.RG = RG; c.pt = geo.seg_pt[0];
+    c.ring = smem_u32(smem) + stream * geo.stage_bytes;
+    c.stage_bytes = geo.stage_bytes * RG;   // from one of the stream's stages to the next
+    c.blk = cg * geo.NB;
+    c.nb = blocks - c.blk < geo.NB ? blocks - c.blk : geo.NB;
+    const Act A{act_sm, p.cols};
     float4 norm_g[2];
     pack_prefetch_norm8(p.norm_w, p.cols, norm_g);   // weights: fetched while the previous kernel is still running
     {
@@ -356,17 +425,22 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const Ge
         if (threadIdx.x == 0) wait_counter_gpu(p.reduce_done, ((*p.epoch_ptr) * p.xchg_per_epoch + p.reduce_use) * (p.cols / 32), p.err, 7, p.wait_ns);
         named_barrier(1, PACK_THREADS);
     }
-    pack_stream(act_sm, p.cols, p.reduce_src ? p.x_out : p.x, p.norm_w, red, bar0 + 8 * (3 * S), norm_g, p.cols / 64);
-    if ((uint32_t)warp < active) consume_tiles<QT>(p, c, A);
+    pack_stream(act_sm, p.cols, p.reduce_src ? p.x_out : p.x, p.norm_w, red, bar0 + 8 * (3 * S), norm_g);
+    if ((uint32_t)warp < active) consume_tiles<QT, MODE>(p, c, A);
 }
 
 // -------------------------------------------------------------------------------------------------
 // host side
 // -------------------------------------------------------------------------------------------------
-constexpr size_t STREAM_SMEM_BUDGET = 194 * 1024;   // one CTA per SM; stays under the 196 KB shared-memory configuration, which leaves 60 KB of L1 (register spills live there)
+// AHEAD_BYTES: about HBM's latency times an SM's share of its rate; with the ring-full in flight a Q8_0 4096 x 4096 launch takes 5.7 us
+// instead of 5.3.  TILE_BYTES: a tile's fixed costs (waits, operands' latency, epilogue) spread over so much; gate/up of a 1B model
+// 6.6 us at half of it.
+constexpr uint32_t AHEAD_BYTES = 73728;
+constexpr uint32_t TILE_BYTES = 40960, UNIT_BYTES = 40960, MIN_STAGES = 3, MAX_STAGES = 12;
+constexpr size_t STREAM_SMEM_BUDGET = 226 * 1024;   // one CTA per SM
 
 bool gemv_stream_eligible(const GemvParams &p) {
-    if (p.cols % 64 || p.cols > 16384) return false;
+    if (p.cols % 256 || p.cols > 256 * NB_MAX * CW) return false;
     for (uint32_t s = 0; s < p.nseg; s++) {
         const uint32_t q = p.seg[s].qtype;
         if (q != IB_Q4_K && q != IB_Q5_K && q != IB_Q6_K && q != IB_Q8_0) return false;
@@ -375,11 +449,11 @@ bool gemv_stream_eligible(const GemvParams &p) {
     return true;
 }
 
-template <uint32_t QT>
-static int32_t launch_stream_inst(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p, int grid, const StreamGeom &geo, size_t smem) {
+template <uint32_t QT, uint32_t MODE>
+static int32_t launch_stream_rows(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p, int grid, const StreamGeom &geo, size_t smem) {
     static bool attr_set[16] = {false};
     if (!attr_set[ctx->device & 15]) {
-        IB_CHECK_CUDA(cudaFuncSetAttribute(gemv_stream_kernel<QT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STREAM_SMEM_BUDGET));
+        IB_CHECK_CUDA(cudaFuncSetAttribute(gemv_stream_kernel<QT, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)STREAM_SMEM_BUDGET));
         attr_set[ctx->device & 15] = true;
     }
     cudaLaunchConfig_t cfg = {};
@@ -392,13 +466,23 @@ static int32_t launch_stream_inst(ib_ctx *ctx, cudaStream_t stream, const GemvPa
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = p.pdl ? 1 : 0;
-    IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemv_stream_kernel<QT>, p, geo));
+    IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, gemv_stream_kernel<QT, MODE>, p, geo));
     ctx->launches++;
     return IB_OK;
 }
 
-// Which instance serves a launch: the one of its format; launches that mix Q4_K and Q6_K segments - or that ask for it
-// (`pair_instance`: the launches of a Q4_K_M token graph, so that all of them run the same code) - the two-format one.
+template <uint32_t QT>
+static int32_t launch_stream_inst(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p, int grid, const StreamGeom &geo, size_t smem) {
+    switch (geo.mode) {
+    case ROWS4: return launch_stream_rows<QT, ROWS4>(ctx, stream, p, grid, geo, smem);
+    case ROWS8_LONG: return launch_stream_rows<QT, ROWS8_LONG>(ctx, stream, p, grid, geo, smem);
+    default: return launch_stream_rows<QT, ROWS8>(ctx, stream, p, grid, geo, smem);
+    }
+}
+
+// Which instance serves a launch: the one of its format; launches that mix Q4_K and Q6_K segments the two-format one.  (One
+// two-format instance for all launches of a Q4_K_M token keeps one copy of the code in the instruction caches, but each launch then
+// runs through twice the code: 1584 against 1454 us per token of an 8B model.)
 static int32_t launch_stream_format(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p, int grid, const StreamGeom &geo, size_t smem) {
     uint32_t qt = p.seg[0].qtype;
     bool only_q4_q6 = true;
@@ -406,7 +490,7 @@ static int32_t launch_stream_format(ib_ctx *ctx, cudaStream_t stream, const Gemv
         if (p.seg[s].qtype != qt) qt = QT_MIXED;
         only_q4_q6 = only_q4_q6 && (p.seg[s].qtype == IB_Q4_K || p.seg[s].qtype == IB_Q6_K);
     }
-    if (only_q4_q6 && (qt == QT_MIXED || p.pair_instance)) return launch_stream_inst<QT_Q4_Q6>(ctx, stream, p, grid, geo, smem);
+    if (only_q4_q6 && qt == QT_MIXED) return launch_stream_inst<QT_Q4_Q6>(ctx, stream, p, grid, geo, smem);
     switch (qt) {
     case IB_Q4_K: return launch_stream_inst<IB_Q4_K>(ctx, stream, p, grid, geo, smem);
     case IB_Q6_K: return launch_stream_inst<IB_Q6_K>(ctx, stream, p, grid, geo, smem);
@@ -428,55 +512,26 @@ int32_t launch_gemv_stream(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p
             pairs += p.seg[s].rows / 2;
         }
     }
-    // tile = whole "rounds" of the row groups (RG pairs each, one pair per consumer warp) of up to ~56 KB, in as many stages
-    // as fit beside the activations (at most 4): several copies in flight per SM keep HBM busy while one tile is consumed
-    const uint32_t units = p.cols / 64, CG = (units + 31) / 32, RG = CW / CG;
+    // Tile = whole groups of 8 (4) rows, as many as fit TILE_BYTES and leave every stream a tile, and no more than a third of the ring.  As many stages as fit beside the activations.
+    int grid = ctx->sm_count;       // one persistent CTA per SM
+    if ((uint32_t)grid > pairs) grid = (int)pairs;
+    if (grid < 1) grid = 1;
     const size_t act = (act_smem_bytes(p.cols) + 127) & ~(size_t)127;
-    auto part_bytes = [](uint32_t S) { return (size_t)S * PART_STAGE_FLOATS * 4; };
-    auto bar_bytes = [](uint32_t S) { return ((size_t)(3 * S + 1) * 8 + 15) & ~(size_t)15; };
-    // returns 0 if the layout does not fit, 1 if it fits, 2 if it fits and every segment's tile is whole rounds
-    auto layout = [&](uint32_t max_tile_bytes, uint32_t &stage, uint32_t &S, size_t &total) {
-        bool whole = true;
-        auto pairs_per_tile = [&](uint32_t cost) {
-            uint32_t pt = RG;
-            while (pt * 2 <= PT_MAX && pt * 2 * cost <= max_tile_bytes) pt *= 2;
-            while (pt > 1 && pt * cost > max_tile_bytes) pt--;
-            if (pt % RG) whole = false;
-            return pt;
-        };
-        stage = 0;
-        if (p.epi == EPI_SWIGLU) stage = pairs_per_tile(max_cost) * max_cost;
-        else
-            for (uint32_t s = 0; s < p.nseg; s++) {
-                const uint32_t c = (uint32_t)(2 * p.seg[s].row_bytes);
-                const uint32_t b = pairs_per_tile(c) * c;
-                if (b > stage) stage = b;
-            }
-        stage = (stage + 127) & ~127u;
-        for (S = 4;; S--) {
-            total = (size_t)S * stage + act + part_bytes(S) + bar_bytes(S) + S * 16;   // + partials + barriers + tile descriptors
-            if (total <= STREAM_SMEM_BUDGET || S == 2) break;
-        }
-        return total <= STREAM_SMEM_BUDGET ? (whole ? 2 : 1) : 0;
-    };
-    uint32_t stage = 0, S = 0;
-    size_t total = 0;
-    const uint32_t tries[5] = {57344, 75776, 49152, 32768, max_cost};
-    int chosen = -1;
-    for (int pass = 2; pass >= 1 && chosen < 0; pass--)
-        for (int i = 0; i < 5 && chosen < 0; i++)
-            if (layout(tries[i], stage, S, total) >= pass) chosen = i;
-    if (chosen < 0)
+    const size_t per_stage = PART_STAGE_FLOATS * 4 + 3 * 8 + 16;   // partials, barriers, tile descriptor
+    const size_t room = STREAM_SMEM_BUDGET - act - 256;
+    const uint32_t max_stage = (uint32_t)(room / MIN_STAGES - per_stage) & ~127u;
+    Split split = split_of(p.cols, 4 * max_cost <= max_stage);
+    if (max_cost > max_stage)
         return set_error(IB_ERR_UNSUPPORTED, "gemv: a row pair of %u bytes with %u columns does not fit the streaming kernel's ring", max_cost, p.cols);
+    auto pairs_per_tile = [&](uint32_t cost) {
+        uint32_t pt = split.mode == ROWS4 ? 2 : 4;
+        while (pt * 2 <= PT_MAX && pt * 2 * cost <= TILE_BYTES && pairs / ((uint32_t)grid * pt * 2) >= split.RG) pt *= 2;
+        while (pt > 1 && pt * cost > max_stage) pt--;
+        return pt;
+    };
     StreamGeom geo;
-    geo.stages = S;
-    geo.stage_bytes = stage;
-    geo.act_off = S * stage;
-    geo.part_off = (uint32_t)(geo.act_off + act);
-    geo.bar_off = (uint32_t)(geo.part_off + part_bytes(S));
-    geo.meta_off = (uint32_t)(geo.bar_off + bar_bytes(S));
-    // the tiles in hand-out order: per segment whole rounds of the row groups, as many as fit a stage
     geo.total_tiles = 0;
+    uint32_t stage_data = 0;
     for (uint32_t s = 0; s < 3; s++) {
         geo.seg_pairs[s] = geo.seg_tiles[s] = 0;
         geo.seg_pt[s] = 1;
@@ -484,38 +539,48 @@ int32_t launch_gemv_stream(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p
         const bool swiglu = p.epi == EPI_SWIGLU;
         if (s >= (swiglu ? 1u : p.nseg)) continue;
         const uint32_t cost = swiglu ? max_cost : (uint32_t)(2 * p.seg[s].row_bytes);
-        uint32_t pt = stage / cost;
-        pt = pt < 1 ? 1 : (pt > (uint32_t)PT_MAX ? (uint32_t)PT_MAX : pt);
-        if (pt > RG) pt = pt / RG * RG;
+        const uint32_t pt = pairs_per_tile(cost);
         geo.seg_cost[s] = cost;
         geo.seg_pt[s] = pt;
         geo.seg_pairs[s] = swiglu ? p.seg[0].rows : p.seg[s].rows / 2;
         geo.seg_tiles[s] = (geo.seg_pairs[s] + pt - 1) / pt;
         geo.total_tiles += geo.seg_tiles[s];
+        if (pt * cost > stage_data) stage_data = pt * cost;
     }
-    geo.b_off = geo.seg_pt[0] * (uint32_t)p.seg[0].row_bytes;
-    int grid = ctx->sm_count;       // one persistent CTA per SM
-    if ((uint32_t)grid > pairs) grid = (int)pairs;
-    if (grid < 1) grid = 1;
-    // Hand-out: launches of one segment with enough tiles per CTA give every CTA its first tiles by position and let the
-    // CTAs claim the rest from a counter - whole tiles when there are many (>= 6 per CTA), one-round tiles for the last
-    // third or so when there are few (>= 2.5 per CTA, e.g. gate/up with 3.0), where a whole tile would be too coarse a
-    // unit to even out the CTAs' end times.  Everything else: static byte-balanced ranges.
-    geo.dynamic = 0;
-    geo.head_per_cta = geo.head_tiles = 0;
-    geo.tail_pt = geo.seg_pt[0];
+    geo.stage_bytes = (stage_data + 127) & ~127u;
+    uint32_t S = (uint32_t)(room / (geo.stage_bytes + per_stage));
+    if (S > MAX_STAGES) S = MAX_STAGES;
+    // A stage always serves the same stream: the barriers' parities only order uses that one and the same warp waits for.
+    while (split.RG > S) split.RG /= 2;
+    S -= S % split.RG;
+    geo.NB = split.NB;
+    geo.mode = split.mode;
+    geo.CG = split.CG;
+    geo.RG = split.RG;
+    geo.P = split.RG < (uint32_t)PIPES ? 1u : (uint32_t)PIPES;
+    uint32_t most = geo.seg_pt[0] > geo.seg_pt[1] ? geo.seg_pt[0] : geo.seg_pt[1], width = 1;
+    most = geo.seg_pt[2] > most ? geo.seg_pt[2] : most;
+    while (width < most) width *= 2;
+    geo.slices = 32 / width;
+    geo.ahead = (AHEAD_BYTES / geo.stage_bytes) / geo.P * geo.P;
+    if (geo.ahead < geo.P) geo.ahead = geo.P;
+    geo.stages = S;
+    geo.act_off = S * geo.stage_bytes;
+    geo.part_off = (uint32_t)(geo.act_off + act);
+    geo.bar_off = geo.part_off + S * PART_STAGE_FLOATS * 4;
+    geo.meta_off = (geo.bar_off + (3 * S + 1) * 8 + 15) & ~15u;
+    const size_t total = geo.meta_off + S * 16;
+    // Hand-out: launches of one segment with enough tiles per CTA give every CTA its first ring of tiles by position and let the
+    // CTAs claim the rest from a counter, in units of about UNIT_BYTES (a claim takes about as long as such a unit's copy).
+    // Everything else: static byte-balanced ranges.
+    geo.unit = geo.head = 0;
     const bool single = p.epi == EPI_SWIGLU || p.nseg == 1;
-    const uint32_t tiles_x2_per_cta = 2u * geo.total_tiles / (uint32_t)grid;
-    if (single && tiles_x2_per_cta >= 12u) {
-        geo.dynamic = 1;
-        geo.head_per_cta = S;
-    } else if (single && tiles_x2_per_cta >= 5u && geo.seg_pt[0] >= 2 * RG) {
-        geo.dynamic = 1;
-        const uint32_t whole = geo.total_tiles / (uint32_t)grid;
-        geo.head_per_cta = whole - 1 < S ? whole - 1 : S;
-        geo.tail_pt = RG;
+    uint32_t unit = UNIT_BYTES / geo.stage_bytes;
+    if (unit < 1) unit = 1;
+    if (single && geo.total_tiles >= 6 * unit * (uint32_t)grid) {
+        geo.unit = unit;
+        geo.head = geo.total_tiles / ((uint32_t)grid * geo.P) * 3 / 4;
     }
-    geo.head_tiles = (uint32_t)grid * geo.head_per_cta;
     // the counters through which this launch's CTAs share out the tiles: consecutive launches overlap (programmatic
     // dependent launch), so they take different pairs of a small ring; the last CTA of a launch clears its pair
     GemvParams q = p;

@@ -9,8 +9,9 @@ namespace ib {
 
 
 constexpr int CW = 16;                          // consumer warps
-constexpr int W_PRODUCER = CW, W_EPILOGUE = CW + 1;
-constexpr int STREAM_THREADS = (CW + 2) * 32;   // + 1 producer warp + 1 epilogue warp
+constexpr int PIPES = 2;                        // pipelines: a producer warp, part of the ring and of the consumers, an epilogue warp
+constexpr int W_PRODUCER = CW, W_EPILOGUE = CW + PIPES;
+constexpr int STREAM_THREADS = (CW + 2 * PIPES) * 32;   // 20 warps: 5 per scheduler at 96 registers fill its register file
 constexpr int PT_MAX = 16;                      // row pairs per tile
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -19,13 +20,12 @@ __device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
 }
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-constexpr uint32_t TRY_WAIT_HINT_NS = 2000u;   // suspend-time hint of mbarrier.try_wait
 __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
     uint32_t ok;
     asm volatile(
-        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+        "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
         : "=r"(ok)
-        : "r"(bar), "r"(parity), "r"(TRY_WAIT_HINT_NS)   // suspend-time hint in ns: a waiting warp sleeps instead of spinning through issue slots
+        : "r"(bar), "r"(parity)   // a waiting warp sleeps for a while instead of spinning through issue slots
         : "memory");
     return ok != 0;
 }
@@ -35,9 +35,9 @@ __device__ __forceinline__ unsigned long long global_ns() {
     asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
     return t;
 }
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t *err, uint32_t code, unsigned long long limit_ns) {
-    for (int i = 0; i < 16; i++)   // a read of the clock stalls the warp for about a microsecond: not before the wait is a long one
-        if (mbar_try_wait(bar, parity)) return true;
+// The clock is read (about a microsecond) and the limit applied only after many tries, out of line: what the loops of the kernel
+// carry is the few instructions of the first ones.
+__device__ __noinline__ bool mbar_wait_long(uint32_t bar, uint32_t parity, uint32_t *err, uint32_t code, unsigned long long limit_ns) {
     const unsigned long long t0 = global_ns();
     for (;;) {
         for (int i = 0; i < 256; i++)
@@ -49,6 +49,12 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
         __threadfence_system();
     }
     return false;
+}
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_t *err, uint32_t code, unsigned long long limit_ns) {
+#pragma unroll 1
+    for (int i = 0; i < 64; i++)
+        if (mbar_try_wait(bar, parity)) return true;
+    return mbar_wait_long(bar, parity, err, code, limit_ns);
 }
 // ---- waits on words that another GPU (or another CTA) writes.  Counters only grow; a reader waits until the counter has
 // reached the value that the current use implies.  Bounded like every other wait here. ----
@@ -163,17 +169,10 @@ __device__ __forceinline__ void share_range(uint32_t lo, uint32_t hi, uint32_t s
     b = y > pairs ? pairs : y;
 }
 
-__device__ __forceinline__ uint32_t tile_pairs(uint32_t stage_bytes, uint32_t cost, uint32_t RG) {
-    uint32_t pt = stage_bytes / cost;
-    pt = pt < 1 ? 1 : (pt > PT_MAX ? PT_MAX : pt);
-    if (pt > RG) pt = pt / RG * RG;   // whole rounds of the row groups
-    return pt;
-}
-
 // `swiglu`: gate and up rows travel together (one "pair" = gate row r + up row r).  `sources`/`me`: the CTAs sharing the
 // work and this CTA's index among them.
 __device__ __forceinline__ void make_share_rt(bool swiglu, uint32_t nseg, uint32_t rows0, uint32_t rows1, uint32_t rows2, uint32_t rb0, uint32_t rb1,
-                                              uint32_t rb2, uint32_t stage_bytes, uint32_t RG, uint32_t G, uint32_t me, Share &sh) {
+                                              uint32_t rb2, const uint32_t (&pt)[3], uint32_t G, uint32_t me, Share &sh) {
     uint32_t n0, n1 = 0, n2 = 0;
     sh.nseg = swiglu ? 1u : nseg;
     sh.c1 = sh.c2 = 16;
@@ -190,14 +189,14 @@ __device__ __forceinline__ void make_share_rt(bool swiglu, uint32_t nseg, uint32
     share_range(lo, hi, 0, k0, n0, sh.a0, sh.b0);
     share_range(lo, hi, s1, k1, n1, sh.a1, sh.b1);
     share_range(lo, hi, s2, k2, n2, sh.a2, sh.b2);
-    sh.t0 = tile_pairs(stage_bytes, sh.c0, RG);
-    sh.t1 = tile_pairs(stage_bytes, sh.c1, RG);
-    sh.t2 = tile_pairs(stage_bytes, sh.c2, RG);
+    sh.t0 = pt[0];
+    sh.t1 = pt[1];
+    sh.t2 = pt[2];
 }
 
-__device__ __forceinline__ void make_share(const GemvParams &p, uint32_t stage_bytes, uint32_t RG, Share &sh) {
+__device__ __forceinline__ void make_share(const GemvParams &p, const uint32_t (&pt)[3], uint32_t G, uint32_t me, Share &sh) {
     make_share_rt(p.epi == EPI_SWIGLU, p.nseg, p.seg[0].rows, p.seg[1].rows, p.seg[2].rows, (uint32_t)p.seg[0].row_bytes, (uint32_t)p.seg[1].row_bytes,
-                  (uint32_t)p.seg[2].row_bytes, stage_bytes, RG, gridDim.x, blockIdx.x, sh);
+                  (uint32_t)p.seg[2].row_bytes, pt, G, me, sh);
 }
 
 struct TileCursor {
@@ -218,251 +217,353 @@ struct TileCursor {
     }
 };
 
-// ---- per-lane activation registers of one 64-weight unit ----
-struct UnitAct {
-    uint4 l[ACT_LIMBS][4];   // limbs x 4 groups of 16 columns
-    float s[4];      // per-group scale (already divided where the format needs it)
-    float x[4];      // per-group sum of x
+// -------------------------------------------------------------------------------------------------
+// The dot products, on the integer tensor path (mma.sync m16n8k32, 8-bit operands, 32-bit accumulators).
+//
+// A warp works on 8 rows x 256 columns (a "block") at a time: lane (g, t) = (lane >> 2, lane & 3) reads 64 weights of row g
+// and ends up with the integer dot products of unit t of that row: 64 columns with their sub-block scales, both activation
+// limbs.  Four mma per block and format:
+//  * the 16 rows of the A operand are two stretches, X and Y, of the same 8 weight rows (X in rows 0-7, Y in rows 8-15), so a
+//    lane's A registers are simply what it read from row g;
+//  * a sub-block must not be summed with its neighbours, so every sub-block gets its own pair of B columns (limb 0, limb 1) and
+//    a column holds activations only in the k slots of its sub-block, zeros elsewhere.  The four column pairs serve two
+//    sub-blocks of X and two of Y; the accumulators where a row meets the other stretch's columns are not used;
+//  * accumulator columns 2t, 2t+1 land in lane t: a select between the X and the Y rows leaves every lane with one unit.
+// The order of the k slots is free as long as A and B agree; it is chosen so that a lane's bytes are consecutive in memory.
+// Rows of more than 16 blocks are so long that 8 of them are a third to a half of the ring; they are worked on 4 rows x 512 columns
+// at a time.  The A rows are then stretch X of the 4 rows, stretch Y of the 4 rows - both of one block - and the same of the next
+// block, which has B columns of its own: 8 mma with half of the results used, and everything else as before (with 8-row tiles HBM
+// waited for the consumers: two tiles fill the ring and land together; with 8-row products of 4-row tiles the consumers became the
+// limit).
+// Per 64 weights this issues 4 mma and 16 masks where byte dot products took 32 dp4a, and the row sum needs 2 shuffles per
+// 8 rows instead of 5 per 2 rows.  HBM delivers 64 Q4_K weights per lane and scheduler every ~195 clocks; the dot products took
+// about 250, these take about 100.
+// -------------------------------------------------------------------------------------------------
+constexpr int NB_MAX = 4;   // blocks of 256 columns per consumer warp
+
+// c = a . b, or c += a . b
+#define IB_MMA(NAME, TYPE)                                                                                                               \
+    __device__ __forceinline__ void NAME(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {     \
+        asm("mma.sync.aligned.m16n8k32.row.col.s32." TYPE ".s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"            \
+            : "=r"(c[0]), "=r"(c[1]), "=r"(c[2]), "=r"(c[3])                                                                             \
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));                                                             \
+    }                                                                                                                                    \
+    __device__ __forceinline__ void NAME##_add(int (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) { \
+        asm("mma.sync.aligned.m16n8k32.row.col.s32." TYPE ".s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"                \
+            : "+r"(c[0]), "+r"(c[1]), "+r"(c[2]), "+r"(c[3])                                                                             \
+            : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));                                                                     \
+    }
+IB_MMA(mma_u8, "u8")
+IB_MMA(mma_s8, "s8")
+#undef IB_MMA
+
+// Everything that depends only on the lane and the warp's first block: byte offsets inside a row, shifts, masks.
+struct LaneConst {
+    uint32_t o0, o1, o2, o3;   // byte offsets inside a row
+    uint32_t sh, ma, mb, mc;   // scale extraction
+    uint32_t h0, h1;           // Q5_K: shifts of the fifth bits
+    uint32_t sc, sx;           // shared addresses of the unit's activation scales and 16-column sums
+    bool first;                // this lane's unit is in accumulator rows 0-7
 };
 
-// Unit u of a row, by format:
-//   Q4_K / Q5_K: block u>>2, 64-column chunk c = u&3: columns 256b + 64c .. +63; groups 0,1 = low nibbles, 2,3 = high nibbles
-//   Q6_K       : block u>>2, half i = (u>>1)&1, 16-byte half h = u&1: groups g = 0..3 at 256b + 128i + 32g + 16h
-//   Q8_0       : blocks 2u, 2u+1: columns 64u .. +63
-__device__ __forceinline__ void load_unit_act(uint32_t qtype, uint32_t u, const Act &A, UnitAct &ua) {
-    uint32_t e16[4];
-    if (qtype == IB_Q6_K) {
-        const uint32_t b = u >> 2, i = (u >> 1) & 1, h = u & 1, base = 16 * b + 8 * i + h;
-#pragma unroll
-        for (int g = 0; g < 4; g++) e16[g] = base + 2 * g;
-    } else {
-#pragma unroll
-        for (int g = 0; g < 4; g++) e16[g] = 4 * u + g;
-    }
-    // 32-bit shared addresses, computed once; volatile loads: they must stay where they are (as ordinary loads they are
-    // loop-invariant and would be hoisted to one place where every format's copies stay live at once)
-    const uint32_t base = smem_u32(A.base), ls = A.lstride();
-    const uint32_t sc0 = base + ACT_LIMBS * ls, sx0 = sc0 + A.cols / 8;   // f32 scale per 32 columns, then f32 sum per 16 columns
-#pragma unroll
-    for (int g = 0; g < 4; g++) {
-        const uint32_t at = base + 16 * A.pos(e16[g]);
-#pragma unroll
-        for (int k = 0; k < ACT_LIMBS; k++) ua.l[k][g] = lds128(at + k * ls);
-        ua.s[g] = __uint_as_float(lds32(sc0 + 4 * (e16[g] >> 1)));
-        ua.x[g] = __uint_as_float(lds32(sx0 + 4 * e16[g]));
-    }
-    if (qtype == IB_Q4_K) { ua.s[2] *= (1.0f / 16.0f); ua.s[3] *= (1.0f / 16.0f); }  // high nibbles are used in place (16 q)
-    if (qtype == IB_Q4_K || qtype == IB_Q5_K) {   // groups 0,1 (and 2,3) form one 32-column sub-block: one sum each
-        ua.x[0] += ua.x[1];
-        ua.x[2] += ua.x[3];
-    }
-}
+// The lane's unit of a step: activation scales and sums, ready for the format's formula.  At most two steps per warp: kept in
+// registers (8 rows at a time); longer rows read them from shared memory for every dot product.
+struct UnitAct { float s[4], x[4]; };
 
-// One row (in shared memory, 32-bit shared address) x one unit -> the lane's partial dot product.  Everything that
-// depends only on the lane (byte offsets inside a row, shift amounts, masks) is computed once in init().
-struct LaneConst { uint32_t o0, o1, o2, o3, k, ma, mb, mc; };
-// component w of a 128-bit register group; w is a compile-time constant wherever this is used (unrolled loops)
-__device__ __forceinline__ uint32_t comp(const uint4 &v, int w) { return w == 0 ? v.x : (w == 1 ? v.y : (w == 2 ? v.z : v.w)); }
-template <uint32_t QT> struct Unit;
-
-// 6-bit (scale, min) pairs of sub-blocks 2c and 2c+1 of a Q4_K / Q5_K header without a branch on c (the lanes of a warp
-// differ in c): lanes with c < 2 carry masks (0x3F3F, 0, 0), the others (0, 0x3030, 0x0F0F), and both read the same three
+// 6-bit (scale, min) pairs of sub-blocks 2t and 2t+1 of a Q4_K / Q5_K header without a branch on t (the lanes of a warp
+// differ in t): lanes with t < 2 carry masks (0x3F3F, 0, 0), the others (0, 0x3030, 0x0F0F), and both read the same three
 // half-words (crates/inferi/src/quantization.rs:394-402).
 __device__ __forceinline__ void kquant_scales_lane(const uint4 &hdr, const LaneConst &lc, uint32_t &sc2, uint32_t &m2) {
-    const uint32_t y2 = hdr.y >> lc.o2, z2 = hdr.z >> lc.o2, w2 = hdr.w >> lc.o2;   // o2 = 16 * (c & 1); the masks drop the upper half
+    const uint32_t y2 = hdr.y >> lc.sh, z2 = hdr.z >> lc.sh, w2 = hdr.w >> lc.sh;   // sh = 16 * (t & 1); the masks drop the upper half
     sc2 = (y2 & lc.ma) | ((y2 >> 2) & lc.mb) | (w2 & lc.mc);
     m2 = (z2 & lc.ma) | ((z2 >> 2) & lc.mb) | ((w2 >> 4) & lc.mc);
 }
-__device__ __forceinline__ void kquant_lane_init(uint32_t c, LaneConst &lc) {
-    lc.k = c;
-    lc.o2 = 16 * (c & 1);
-    lc.ma = c < 2 ? 0x3F3Fu : 0u;
-    lc.mb = c < 2 ? 0u : 0x3030u;
-    lc.mc = c < 2 ? 0u : 0x0F0Fu;
-}
-// d * (sc_lo * lo + sc_hi * hi) - dmin * (m_lo * x_lo + m_hi * x_hi) for one 64-column chunk of a Q4_K / Q5_K block
-__device__ __forceinline__ float kquant_finish(const uint4 &hdr, uint32_t sc2, uint32_t m2, float lo, float hi, float x_lo, float x_hi) {
+// d * (sc_lo * lo + sc_hi * hi) - dmin * (m_lo * x_lo + m_hi * x_hi) for the 64 columns of a unit of a Q4_K / Q5_K block;
+// `lo`, `hi`: the integer dot products, a.s their units, a.x the sums of the columns
+__device__ __forceinline__ float kquant_finish(const uint4 &hdr, const LaneConst &lc, float lo, float hi, const float s0, const float s1, const float x0, const float x1) {
+    uint32_t sc2, m2;
+    kquant_scales_lane(hdr, lc, sc2, m2);
     const float2 dm = __half22float2(*reinterpret_cast<const __half2 *>(&hdr.x));
-    const float a = (float)(sc2 & 0xFFu) * lo + (float)(sc2 >> 8) * hi;
-    const float b = (float)(m2 & 0xFFu) * x_lo + (float)(m2 >> 8) * x_hi;
+    const float a = (float)(sc2 & 0xFFu) * (s0 * lo) + (float)(sc2 >> 8) * (s1 * hi);
+    const float b = (float)(m2 & 0xFFu) * x0 + (float)(m2 >> 8) * x1;
     return dm.x * a - dm.y * b;
 }
+// scales of columns 64u .. +31 and +32 .. +63 of the block and the sums of the same columns; `hi_unit`: what a high dot product counts
+template <bool FOUR>
+__device__ __forceinline__ void kquant_unit(const LaneConst &lc, uint32_t i, float hi_unit, UnitAct &a) {
+    const uint2 s = lds64(lc.sc + (FOUR ? 64 : 32) * i);
+    const uint4 x = lds128(lc.sx + (FOUR ? 128 : 64) * i);
+    a.s[0] = __uint_as_float(s.x);
+    a.s[1] = __uint_as_float(s.y) * hi_unit;
+    a.x[0] = __uint_as_float(x.x) + __uint_as_float(x.y);
+    a.x[1] = __uint_as_float(x.z) + __uint_as_float(x.w);
+}
+// this lane's unit out of the accumulators (4 rows: `e` has the products with the second block's operand)
+template <bool FOUR>
+__device__ __forceinline__ float unit_of(const int (&c)[4], const int (&e)[4], bool first) {
+    const int lower = limb_sum(c[0], c[1]), upper = FOUR ? limb_sum(e[2], e[3]) : limb_sum(c[2], c[3]);
+    return (float)(first ? lower : upper);
+}
+// Which rows and units a lane works on.  `sx`: the stretch in its lower A row (the upper one holds the other stretch, or the same
+// stretch of the next block); `own`: its unit is in the lower A rows; `u`: the unit, of block `next` (0, 1) of the step.
+struct LaneUnit { uint32_t sx, u, next; bool own; };
+template <bool FOUR>
+__device__ __forceinline__ LaneUnit lane_unit(uint32_t g, uint32_t t, bool swap) {
+    LaneUnit l;
+    l.sx = (FOUR ? g >> 2 : 0u) ^ (swap ? 1u : 0u);
+    l.own = (t >> 1) == l.sx;
+    l.next = FOUR && !l.own ? 1u : 0u;
+    l.u = l.next ? t ^ 2u : t;
+    return l;
+}
 
-template <> struct Unit<IB_Q4_K> {
-    static __device__ __forceinline__ void init(uint32_t u, LaneConst &lc) {
-        kquant_lane_init(u & 3, lc);
-        lc.o0 = (u >> 2) * 144;
-        lc.o1 = lc.o0 + 16 + 32 * lc.k;
-    }
-    static __device__ __forceinline__ float dot(uint32_t row, const LaneConst &lc, const UnitAct &ua) {
-        const uint4 hdr = lds128(row + lc.o0), q0 = lds128(row + lc.o1), q1 = lds128(row + lc.o1 + 16);
-        const uint32_t qa[4] = {q0.x, q0.y, q0.z, q0.w}, qb[4] = {q1.x, q1.y, q1.z, q1.w};
-        int L[3] = {0, 0, 0}, H[3] = {0, 0, 0};   // low nibbles = sub-block 2c (groups 0,1), high nibbles = sub-block 2c+1 (groups 2,3)
-#pragma unroll
-        for (int w = 0; w < 4; w++) {
-            const uint32_t lo = qa[w] & 0x0F0F0F0Fu, hi = qa[w] & 0xF0F0F0F0u;
-#pragma unroll
-            for (int k = 0; k < ACT_LIMBS; k++) {
-                L[k] = dp4a_ss(lo, comp(ua.l[k][0], w), L[k]);
-                H[k] = dp4a_us(hi, comp(ua.l[k][2], w), H[k]);
-            }
-        }
-#pragma unroll
-        for (int w = 0; w < 4; w++) {
-            const uint32_t lo = qb[w] & 0x0F0F0F0Fu, hi = qb[w] & 0xF0F0F0F0u;
-#pragma unroll
-            for (int k = 0; k < ACT_LIMBS; k++) {
-                L[k] = dp4a_ss(lo, comp(ua.l[k][1], w), L[k]);
-                H[k] = dp4a_us(hi, comp(ua.l[k][3], w), H[k]);
-            }
-        }
-        uint32_t sc2, m2;
-        kquant_scales_lane(hdr, lc, sc2, m2);
-        return kquant_finish(hdr, sc2, m2, ua.s[0] * limb_combine(L), ua.s[2] * limb_combine(H), ua.x[0], ua.x[2]);
+// Per format:  init: the lane's constants for the warp's first block `blk` (rows `stride` bytes apart);  operand: the B registers
+// of block `blk` (`limb`: shared address of limb (g & 1) of the activations: B column g belongs to unit g >> 1, limb g & 1; the
+// second block of a 4-row step has the units of X and Y exchanged: pass g ^ 4);  dot: step `i` (a block, or two) of the row at
+// shared address `row`, operands `b`, `b2` -> the lane's unit of that row;  unit: the activations' side of step i.
+template <uint32_t QT> struct Frag;
+
+// Rows whose stride is close to a multiple of the 128 bytes of a shared-memory wavefront all start at the same bank: every other
+// row then reads its stretch Y first, so that the two rows a wavefront serves use both halves of the banks.
+__device__ __forceinline__ bool swap_stretches(uint32_t g, uint32_t stride) { return (g & 1) && ((stride + 32) & 127) < 64; }
+
+// Q4_K and Q5_K: X = the 64 quant bytes of units 0 and 1 (each 32 bytes: low nibbles sub-block 2t, high nibbles 2t+1), Y = units
+// 2 and 3; lane t holds 16 bytes of unit (t >> 1) of either.
+template <bool FOUR>
+__device__ __forceinline__ void kquant_init(uint32_t g, uint32_t t, uint32_t stride, uint32_t block_bytes, uint32_t quants_at, uint32_t blk, LaneConst &lc) {
+    const LaneUnit l = lane_unit<FOUR>(g, t, swap_stretches(g, stride));
+    const uint32_t at = blk * block_bytes;
+    lc.o0 = at + l.next * block_bytes;
+    lc.o1 = at + quants_at + 16 * t + 64 * l.sx;
+    lc.o2 = FOUR ? lc.o1 + block_bytes : at + quants_at + 16 * t + 64 * (1 - l.sx);
+    lc.first = l.own;
+    lc.sh = 16 * (l.u & 1);
+    lc.ma = l.u < 2 ? 0x3F3Fu : 0u;
+    lc.mb = l.u < 2 ? 0u : 0x3030u;
+    lc.mc = l.u < 2 ? 0u : 0x0F0Fu;
+    lc.o3 = at + 16 + 16 * (t & 1);   // Q5_K: the fifth bits of this lane's 16 columns, bit 2u / 2u+1 of a byte for unit u
+    lc.h0 = 2 * (t >> 1) + 4 * l.sx;
+    lc.h1 = FOUR ? lc.h0 : 2 * (t >> 1) + 4 * (1 - l.sx);
+    lc.sc += 4 * (8 * (blk + l.next) + 2 * l.u);
+    lc.sx += 4 * (16 * (blk + l.next) + 4 * l.u);
+}
+__device__ __forceinline__ void load_operand(uint32_t lo_at, uint32_t hi_at, uint32_t (&b)[8]) {
+    const uint4 lo = lds128(lo_at), hi = lds128(hi_at);
+    b[0] = lo.x; b[1] = lo.y; b[2] = lo.z; b[3] = lo.w;
+    b[4] = hi.x; b[5] = hi.y; b[6] = hi.z; b[7] = hi.w;
+}
+// `zeros`: shared address of 16 bytes of zeros, what a lane's slots outside its column's sub-block hold
+__device__ __forceinline__ void kquant_operand(uint32_t g, uint32_t t, uint32_t limb, uint32_t zeros, uint32_t blk, uint32_t (&b)[8]) {
+    const uint32_t q = g >> 1, at = limb + 256 * blk + 64 * q + 16 * (t & 1);
+    const bool has = (t >> 1) == (q & 1);
+    load_operand(has ? at : zeros, has ? at + 32 : zeros, b);
+}
+
+template <> struct Frag<IB_Q4_K> {
+    template <bool FOUR>
+    static __device__ __forceinline__ void unit(const LaneConst &lc, uint32_t i, UnitAct &a) { kquant_unit<FOUR>(lc, i, 1.0f / 16.0f, a); }
+    template <bool FOUR>
+    static __device__ __forceinline__ void init(uint32_t g, uint32_t t, uint32_t stride, uint32_t blk, LaneConst &lc) { kquant_init<FOUR>(g, t, stride, 144, 16, blk, lc); }
+    static __device__ __forceinline__ void operand(uint32_t g, uint32_t t, uint32_t limb, uint32_t zeros, uint32_t blk, uint32_t (&b)[8]) { kquant_operand(g, t, limb, zeros, blk, b); }
+    template <bool FOUR>
+    static __device__ __forceinline__ float dot(uint32_t row, const LaneConst &lc, uint32_t i, const uint32_t (&b)[8], const uint32_t (&b2)[8], const UnitAct &a) {
+        constexpr uint32_t LO = 0x0F0F0F0Fu, HI = 0xF0F0F0F0u, STEP = FOUR ? 2 * 144 : 144;   // high nibbles are used in place: 16 q
+        const uint4 v = lds128(row + lc.o1 + STEP * i), w = lds128(row + lc.o2 + STEP * i), hdr = lds128(row + lc.o0 + STEP * i);
+        int L[4], H[4], L2[4], H2[4];
+        mma_u8(L, v.x & LO, w.x & LO, v.y & LO, w.y & LO, b[0], b[1]);
+        mma_u8(H, v.x & HI, w.x & HI, v.y & HI, w.y & HI, b[4], b[5]);
+        if (FOUR) mma_u8(L2, v.x & LO, w.x & LO, v.y & LO, w.y & LO, b2[0], b2[1]);
+        if (FOUR) mma_u8(H2, v.x & HI, w.x & HI, v.y & HI, w.y & HI, b2[4], b2[5]);
+        mma_u8_add(L, v.z & LO, w.z & LO, v.w & LO, w.w & LO, b[2], b[3]);
+        mma_u8_add(H, v.z & HI, w.z & HI, v.w & HI, w.w & HI, b[6], b[7]);
+        if (FOUR) mma_u8_add(L2, v.z & LO, w.z & LO, v.w & LO, w.w & LO, b2[2], b2[3]);
+        if (FOUR) mma_u8_add(H2, v.z & HI, w.z & HI, v.w & HI, w.w & HI, b2[6], b2[7]);
+        return kquant_finish(hdr, lc, unit_of<FOUR>(L, L2, lc.first), unit_of<FOUR>(H, H2, lc.first), a.s[0], a.s[1], a.x[0], a.x[1]);
     }
 };
 
-template <> struct Unit<IB_Q5_K> {
-    static __device__ __forceinline__ void init(uint32_t u, LaneConst &lc) {
-        kquant_lane_init(u & 3, lc);
-        lc.o0 = (u >> 2) * 176;
-        lc.o1 = lc.o0 + 48 + 32 * lc.k;
-        lc.o3 = 2 * lc.k;
-    }
-    static __device__ __forceinline__ float dot(uint32_t row, const LaneConst &lc, const UnitAct &ua) {
-        const uint4 hdr = lds128(row + lc.o0), hA = lds128(row + lc.o0 + 16), hB = lds128(row + lc.o0 + 32);
-        const uint4 q0 = lds128(row + lc.o1), q1 = lds128(row + lc.o1 + 16);
-        const uint32_t qw[8] = {q0.x, q0.y, q0.z, q0.w, q1.x, q1.y, q1.z, q1.w};
-        const uint32_t hw[8] = {hA.x, hA.y, hA.z, hA.w, hB.x, hB.y, hB.z, hB.w};
-        int L[3] = {0, 0, 0}, H[3] = {0, 0, 0};
+template <> struct Frag<IB_Q5_K> {
+    template <bool FOUR>
+    static __device__ __forceinline__ void unit(const LaneConst &lc, uint32_t i, UnitAct &a) { kquant_unit<FOUR>(lc, i, 1.0f, a); }
+    template <bool FOUR>
+    static __device__ __forceinline__ void init(uint32_t g, uint32_t t, uint32_t stride, uint32_t blk, LaneConst &lc) { kquant_init<FOUR>(g, t, stride, 176, 48, blk, lc); }
+    static __device__ __forceinline__ void operand(uint32_t g, uint32_t t, uint32_t limb, uint32_t zeros, uint32_t blk, uint32_t (&b)[8]) { kquant_operand(g, t, limb, zeros, blk, b); }
+    static __device__ __forceinline__ uint32_t lo5(uint32_t q, uint32_t h) { return (q & 0x0F0F0F0Fu) | ((h << 4) & 0x10101010u); }
+    static __device__ __forceinline__ uint32_t hi5(uint32_t q, uint32_t h) { return ((q >> 4) & 0x0F0F0F0Fu) | ((h << 3) & 0x10101010u); }
+    template <bool FOUR>
+    static __device__ __forceinline__ float dot(uint32_t row, const LaneConst &lc, uint32_t i, const uint32_t (&b)[8], const uint32_t (&b2)[8], const UnitAct &a) {
+        constexpr uint32_t STEP = FOUR ? 2 * 176 : 176;
+        const uint4 v = lds128(row + lc.o1 + STEP * i), w = lds128(row + lc.o2 + STEP * i), h = lds128(row + lc.o3 + STEP * i);
+        const uint4 k = FOUR ? lds128(row + lc.o3 + STEP * i + 176) : h, hdr = lds128(row + lc.o0 + STEP * i);
+        const uint32_t hv[4] = {h.x >> lc.h0, h.y >> lc.h0, h.z >> lc.h0, h.w >> lc.h0}, hw[4] = {k.x >> lc.h1, k.y >> lc.h1, k.z >> lc.h1, k.w >> lc.h1};
+        int L[4], H[4], L2[4], H2[4];
+        const uint32_t vv[4] = {v.x, v.y, v.z, v.w}, ww[4] = {w.x, w.y, w.z, w.w};
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-            const uint32_t t = hw[i] >> lc.o3;  // bit 0 of each byte: fifth bit of the low-nibble element, bit 1: of the high-nibble element
-            const uint32_t lo = (qw[i] & 0x0F0F0F0Fu) | ((t << 4) & 0x10101010u);
-            const uint32_t hi = ((qw[i] >> 4) & 0x0F0F0F0Fu) | ((t << 3) & 0x10101010u);
-#pragma unroll
-            for (int k = 0; k < ACT_LIMBS; k++) {
-                L[k] = dp4a_ss(lo, comp(ua.l[k][i >> 2], i & 3), L[k]);
-                H[k] = dp4a_ss(hi, comp(ua.l[k][2 + (i >> 2)], i & 3), H[k]);
+        for (int j = 0; j < 4; j += 2) {
+            const uint32_t l0 = lo5(vv[j], hv[j]), l1 = lo5(ww[j], hw[j]), l2 = lo5(vv[j + 1], hv[j + 1]), l3 = lo5(ww[j + 1], hw[j + 1]);
+            const uint32_t h0 = hi5(vv[j], hv[j]), h1 = hi5(ww[j], hw[j]), h2 = hi5(vv[j + 1], hv[j + 1]), h3 = hi5(ww[j + 1], hw[j + 1]);
+            if (j == 0) {
+                mma_u8(L, l0, l1, l2, l3, b[0], b[1]);
+                mma_u8(H, h0, h1, h2, h3, b[4], b[5]);
+                if (FOUR) mma_u8(L2, l0, l1, l2, l3, b2[0], b2[1]);
+                if (FOUR) mma_u8(H2, h0, h1, h2, h3, b2[4], b2[5]);
+            } else {
+                mma_u8_add(L, l0, l1, l2, l3, b[2], b[3]);
+                mma_u8_add(H, h0, h1, h2, h3, b[6], b[7]);
+                if (FOUR) mma_u8_add(L2, l0, l1, l2, l3, b2[2], b2[3]);
+                if (FOUR) mma_u8_add(H2, h0, h1, h2, h3, b2[6], b2[7]);
             }
         }
-        uint32_t sc2, m2;
-        kquant_scales_lane(hdr, lc, sc2, m2);
-        return kquant_finish(hdr, sc2, m2, ua.s[0] * limb_combine(L), ua.s[2] * limb_combine(H), ua.x[0], ua.x[2]);
+        return kquant_finish(hdr, lc, unit_of<FOUR>(L, L2, lc.first), unit_of<FOUR>(H, H2, lc.first), a.s[0], a.s[1], a.x[0], a.x[1]);
     }
 };
 
 // Q6_K rows are stored as groups of 8 blocks: [8 x 128 ql][8 x 64 qh][8 x 16 scales][8 x 2 d] = 1680 bytes per 2048 columns.
-template <> struct Unit<IB_Q6_K> {
-    static __device__ __forceinline__ void init(uint32_t u, LaneConst &lc) {
-        const uint32_t b = u >> 2, i = (u >> 1) & 1, h = u & 1, grp = (b >> 3) * 1680, bb = b & 7;
-        lc.o0 = grp + 128 * bb + 64 * i + 16 * h;
-        lc.o1 = grp + 1024 + 64 * bb + 32 * i + 16 * h;
-        lc.o2 = grp + 1536 + 16 * bb + 8 * i;
-        lc.o3 = grp + 1664 + 2 * bb;
-        lc.k = 8 * h;
-        lc.ma = lc.mb = lc.mc = 0;
+// X / Y = halves 0 / 1 of a block (128 columns; their 32-byte ql segments hold columns +0 and +64, and +32 and +96).  A scale
+// covers 16 columns, so each of the four 32-column stretches of a half is a product of its own; lane t holds 8 of its columns.
+// Unit t: half i = t >> 1, 16-column half h = t & 1 of all four stretches.
+template <> struct Frag<IB_Q6_K> {
+    template <bool FOUR>
+    static __device__ __forceinline__ void init(uint32_t g, uint32_t t, uint32_t, uint32_t blk, LaneConst &lc) {
+        const LaneUnit l = lane_unit<FOUR>(g, t, false);
+        const uint32_t grp = (blk >> 3) * 1680, bb = blk & 7;   // a warp's blocks never straddle a group: their number divides 8
+        lc.o0 = grp + 128 * bb + 8 * t + (FOUR ? 64 * l.sx : 0);
+        lc.o1 = grp + 1024 + 64 * bb + 8 * t + (FOUR ? 32 * l.sx : 0);
+        lc.o2 = grp + 1536 + 16 * (bb + l.next) + 8 * (l.u >> 1);
+        lc.o3 = grp + 1664 + 2 * (bb + l.next);
+        lc.sh = 8 * (l.u & 1);
+        lc.ma = lc.mb = lc.mc = lc.h0 = lc.h1 = 0;
+        lc.first = l.own;
+        lc.sc += 4 * (8 * (blk + l.next) + 4 * (l.u >> 1));
+        lc.sx += 4 * (16 * (blk + l.next) + 8 * (l.u >> 1) + (l.u & 1));
     }
-    static __device__ __forceinline__ float dot(uint32_t row, const LaneConst &lc, const UnitAct &ua) {
-        const uint4 qa = lds128(row + lc.o0), qb = lds128(row + lc.o0 + 32), qh = lds128(row + lc.o1);
-        const uint2 scw = lds64(row + lc.o2);   // scales[8i .. 8i+7]
-        const float d = h2f(lds16(row + lc.o3));
-        const uint32_t la[4] = {qa.x, qa.y, qa.z, qa.w}, lb[4] = {qb.x, qb.y, qb.z, qb.w}, hh[4] = {qh.x, qh.y, qh.z, qh.w};
-        int D[4][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+    static __device__ __forceinline__ void operand(uint32_t g, uint32_t t, uint32_t limb, uint32_t zeros, uint32_t blk, uint32_t (&b)[8]) {
+        const uint32_t i = g >> 2, h = (g >> 1) & 1;
+        const uint32_t at = limb + 256 * blk + 128 * i + 16 * h + 8 * (t & 1);
 #pragma unroll
-        for (int w = 0; w < 4; w++) {
-            // crates/inferi/src/quantization.rs:237-246: 4 low bits from ql, 2 high bits from qh
-            const uint32_t g0 = (la[w] & 0x0F0F0F0Fu) | ((hh[w] << 4) & 0x30303030u);
-            const uint32_t g1 = (lb[w] & 0x0F0F0F0Fu) | ((hh[w] << 2) & 0x30303030u);
-            const uint32_t g2 = ((la[w] >> 4) & 0x0F0F0F0Fu) | (hh[w] & 0x30303030u);
-            const uint32_t g3 = ((lb[w] >> 4) & 0x0F0F0F0Fu) | ((hh[w] >> 2) & 0x30303030u);
-#pragma unroll
-            for (int k = 0; k < ACT_LIMBS; k++) {
-                D[0][k] = dp4a_ss(g0, comp(ua.l[k][0], w), D[0][k]);
-                D[1][k] = dp4a_ss(g1, comp(ua.l[k][1], w), D[1][k]);
-                D[2][k] = dp4a_ss(g2, comp(ua.l[k][2], w), D[2][k]);
-                D[3][k] = dp4a_ss(g3, comp(ua.l[k][3], w), D[3][k]);
-            }
+        for (int s = 0; s < 4; s++) {
+            const uint2 v = lds64((t >> 1) == h ? at + 32 * s : zeros);
+            b[2 * s] = v.x;
+            b[2 * s + 1] = v.y;
         }
-        // scale of group g is byte 2g + h of the 8 loaded: bytes {h, 2+h} of word x, {h, 2+h} of word y
-        const uint32_t sx = scw.x >> lc.k, sy = scw.y >> lc.k;
-        const float s0 = (float)(int)(int8_t)(sx & 0xFF), s1 = (float)(int)(int8_t)((sx >> 16) & 0xFF);
-        const float s2 = (float)(int)(int8_t)(sy & 0xFF), s3 = (float)(int)(int8_t)((sy >> 16) & 0xFF);
-        float v = s0 * (ua.s[0] * limb_combine(D[0]) - 32.0f * ua.x[0]);
-        v += s1 * (ua.s[1] * limb_combine(D[1]) - 32.0f * ua.x[1]);
-        v += s2 * (ua.s[2] * limb_combine(D[2]) - 32.0f * ua.x[2]);
-        v += s3 * (ua.s[3] * limb_combine(D[3]) - 32.0f * ua.x[3]);
+    }
+    template <bool FOUR>
+    static __device__ __forceinline__ void unit(const LaneConst &lc, uint32_t i, UnitAct &a) {
+        constexpr uint32_t K = FOUR ? 2 : 1;
+        const uint4 s = lds128(lc.sc + 32 * K * i);
+        a.s[0] = __uint_as_float(s.x); a.s[1] = __uint_as_float(s.y); a.s[2] = __uint_as_float(s.z); a.s[3] = __uint_as_float(s.w);
+#pragma unroll
+        for (int k = 0; k < 4; k++) a.x[k] = -32.0f * __uint_as_float(lds32(lc.sx + 64 * K * i + 8 * k));
+    }
+    // crates/inferi/src/quantization.rs:237-246: 4 low bits from ql, 2 high bits from qh.  `h`: the two bits in bits 4-5 of each
+    // byte, bits 6-7 clear; bits 0-3 are dropped
+    static __device__ __forceinline__ uint32_t join(uint32_t q, uint32_t h) { return (q & 0x0F0F0F0Fu) | (h & 0xF0F0F0F0u); }
+    template <bool FOUR>
+    static __device__ __forceinline__ float dot(uint32_t row, const LaneConst &lc, uint32_t i, const uint32_t (&b)[8], const uint32_t (&b2)[8], const UnitAct &a) {
+        constexpr uint32_t K = FOUR ? 2 : 1;   // the upper A rows: the other half, 64 (32) bytes on, or the next block, 128 (64) bytes on
+        const uint32_t q0 = row + lc.o0 + 128 * K * i, h0 = row + lc.o1 + 64 * K * i;
+        const uint2 hx = lds64(h0), hy = lds64(h0 + 32 * K);
+        const uint2 ax = lds64(q0), ay = lds64(q0 + 64 * K), bx = lds64(q0 + 32), by = lds64(q0 + 32 + 64 * K);
+        constexpr uint32_t M = 0x33333333u;
+        int D[4][4], E[4][4];
+#pragma unroll
+        for (int s = 0; s < 2; s++) {   // the two 32-byte segments: columns +0, +64 and +32, +96 of a half
+            const uint2 x = s ? bx : ax, y = s ? by : ay;
+            const uint32_t e0 = (s ? hx.x >> 2 : hx.x) & M, e1 = (s ? hy.x >> 2 : hy.x) & M, e2 = (s ? hx.y >> 2 : hx.y) & M, e3 = (s ? hy.y >> 2 : hy.y) & M;
+            const uint32_t l0 = join(x.x, e0 << 4), l1 = join(y.x, e1 << 4), l2 = join(x.y, e2 << 4), l3 = join(y.y, e3 << 4);
+            const uint32_t u0 = join(x.x >> 4, e0), u1 = join(y.x >> 4, e1), u2 = join(x.y >> 4, e2), u3 = join(y.y >> 4, e3);
+            mma_u8(D[s], l0, l1, l2, l3, b[2 * s], b[2 * s + 1]);
+            mma_u8(D[s + 2], u0, u1, u2, u3, b[2 * s + 4], b[2 * s + 5]);
+            if (FOUR) mma_u8(E[s], l0, l1, l2, l3, b2[2 * s], b2[2 * s + 1]);
+            if (FOUR) mma_u8(E[s + 2], u0, u1, u2, u3, b2[2 * s + 4], b2[2 * s + 5]);
+        }
+        const uint2 scw = lds64(row + lc.o2 + 16 * K * i);   // scales[8 half .. +7]: stretch s is byte 2s + h
+        const float d = h2f(lds16(row + lc.o3 + 2 * K * i));
+        const uint32_t sa = scw.x >> lc.sh, sb = scw.y >> lc.sh;
+        const float w[4] = {(float)(int)(int8_t)(sa & 0xFF), (float)(int)(int8_t)((sa >> 16) & 0xFF), (float)(int)(int8_t)(sb & 0xFF),
+                            (float)(int)(int8_t)((sb >> 16) & 0xFF)};
+        float v = 0.f;
+#pragma unroll
+        for (int k = 0; k < 4; k++) v += w[k] * (a.s[k] * unit_of<FOUR>(D[k], E[k], lc.first) + a.x[k]);
         return d * v;
     }
 };
 
-// Q8_0 rows are stored as groups of 8 blocks: [8 x 32 quants][8 x 2 scale] = 272 bytes per 256 columns.
-template <> struct Unit<IB_Q8_0> {
-    static __device__ __forceinline__ void init(uint32_t u, LaneConst &lc) {
-        const uint32_t b0 = 2 * u, grp = (b0 >> 3) * 272, bb = b0 & 7;
-        lc.o0 = grp + 32 * bb;
-        lc.o1 = grp + 256 + 2 * bb;
-        lc.o2 = lc.o3 = lc.k = lc.ma = lc.mb = lc.mc = 0;
+// Q8_0 rows are stored as groups of 8 blocks: [8 x 32 quants][8 x 2 scale] = 272 bytes per 256 columns.  Two products: X, Y =
+// blocks 0-1, 2-3 of the group and 4-5, 6-7; unit t is blocks t and 4 + t.
+template <> struct Frag<IB_Q8_0> {
+    template <bool FOUR>
+    static __device__ __forceinline__ void unit(const LaneConst &lc, uint32_t i, UnitAct &a) {
+        a.s[0] = __uint_as_float(lds32(lc.sc + (FOUR ? 64 : 32) * i));
+        a.s[1] = __uint_as_float(lds32(lc.sc + (FOUR ? 64 : 32) * i + 16));
     }
-    static __device__ __forceinline__ float dot(uint32_t row, const LaneConst &lc, const UnitAct &ua) {
-        const uint4 q[4] = {lds128(row + lc.o0), lds128(row + lc.o0 + 16), lds128(row + lc.o0 + 32), lds128(row + lc.o0 + 48)};
-        const uint32_t dbits = lds32(row + lc.o1);   // f16 scales of the two blocks
-        const float2 dd = __half22float2(*reinterpret_cast<const __half2 *>(&dbits));
-        int A[3] = {0, 0, 0}, B[3] = {0, 0, 0};   // block 2u (groups 0,1), block 2u+1 (groups 2,3)
-#pragma unroll
-        for (int g = 0; g < 4; g++)
-#pragma unroll
-            for (int w = 0; w < 4; w++)
-#pragma unroll
-                for (int k = 0; k < ACT_LIMBS; k++) {
-                    if (g < 2) A[k] = dp4a_ss(comp(q[g], w), comp(ua.l[k][g], w), A[k]);
-                    else B[k] = dp4a_ss(comp(q[g], w), comp(ua.l[k][g], w), B[k]);
-                }
-        return dd.x * (ua.s[0] * limb_combine(A)) + dd.y * (ua.s[2] * limb_combine(B));
+    template <bool FOUR>
+    static __device__ __forceinline__ void init(uint32_t g, uint32_t t, uint32_t stride, uint32_t blk, LaneConst &lc) {
+        const LaneUnit l = lane_unit<FOUR>(g, t, swap_stretches(g, stride));
+        lc.o0 = 272 * (blk + l.next) + 256 + 2 * l.u;
+        lc.o1 = 272 * blk + 16 * t + 64 * l.sx;
+        lc.o2 = FOUR ? lc.o1 + 272 : 272 * blk + 16 * t + 64 * (1 - l.sx);
+        lc.o3 = lc.sh = lc.ma = lc.mb = lc.mc = lc.h0 = lc.h1 = 0;
+        lc.first = l.own;
+        lc.sc += 4 * (8 * (blk + l.next) + l.u);
+    }
+    static __device__ __forceinline__ void operand(uint32_t g, uint32_t t, uint32_t limb, uint32_t zeros, uint32_t blk, uint32_t (&b)[8]) {
+        const uint32_t q = g >> 1, at = limb + 256 * blk + 32 * q + 16 * (t & 1);
+        const bool has = (t >> 1) == (q & 1);
+        load_operand(has ? at : zeros, has ? at + 128 : zeros, b);
+    }
+    template <bool FOUR>
+    static __device__ __forceinline__ float dot(uint32_t row, const LaneConst &lc, uint32_t i, const uint32_t (&b)[8], const uint32_t (&b2)[8], const UnitAct &a) {
+        constexpr uint32_t K = FOUR ? 2 : 1;
+        const uint32_t p = row + lc.o1 + 272 * K * i, c = row + lc.o2 + 272 * K * i;
+        const uint4 v = lds128(p), w = lds128(c), y = lds128(p + 128), z = lds128(c + 128);
+        const float d0 = h2f(lds16(row + lc.o0 + 272 * K * i)), d1 = h2f(lds16(row + lc.o0 + 272 * K * i + 8));
+        int P[4], Q[4], P2[4], Q2[4];
+        mma_s8(P, v.x, w.x, v.y, w.y, b[0], b[1]);
+        mma_s8(Q, y.x, z.x, y.y, z.y, b[4], b[5]);
+        if (FOUR) mma_s8(P2, v.x, w.x, v.y, w.y, b2[0], b2[1]);
+        if (FOUR) mma_s8(Q2, y.x, z.x, y.y, z.y, b2[4], b2[5]);
+        mma_s8_add(P, v.z, w.z, v.w, w.w, b[2], b[3]);
+        mma_s8_add(Q, y.z, z.z, y.w, z.w, b[6], b[7]);
+        if (FOUR) mma_s8_add(P2, v.z, w.z, v.w, w.w, b2[2], b2[3]);
+        if (FOUR) mma_s8_add(Q2, y.z, z.z, y.w, z.w, b2[6], b2[7]);
+        return d0 * (a.s[0] * unit_of<FOUR>(P, P2, lc.first)) + d1 * (a.s[1] * unit_of<FOUR>(Q, Q2, lc.first));
     }
 };
 
 constexpr uint32_t QT_MIXED = 0xFFu;   // kernel instance for launches whose segments differ in format
 constexpr uint32_t QT_Q4_Q6 = 0xFEu;   // ... and hold only Q4_K and Q6_K (q, k, v of the Q4_K_M recipe): two formats to switch between, not four
 
-template <uint32_t QT>
-__device__ __forceinline__ void unit_init(uint32_t qtype, uint32_t u, LaneConst &lc) {
-    lc.o0 = lc.o1 = lc.o2 = lc.o3 = lc.k = lc.ma = lc.mb = lc.mc = 0;
-    if (QT == QT_Q4_Q6) {
-        if (qtype == IB_Q4_K) Unit<IB_Q4_K>::init(u, lc);
-        else Unit<IB_Q6_K>::init(u, lc);
-        return;
-    }
-    if (QT != QT_MIXED) { Unit<(QT == QT_MIXED || QT == QT_Q4_Q6) ? IB_Q4_K : QT>::init(u, lc); return; }
-    switch (qtype) {
-    case IB_Q4_K: Unit<IB_Q4_K>::init(u, lc); break;
-    case IB_Q6_K: Unit<IB_Q6_K>::init(u, lc); break;
-    case IB_Q5_K: Unit<IB_Q5_K>::init(u, lc); break;
-    default: Unit<IB_Q8_0>::init(u, lc); break;
-    }
-}
-template <uint32_t QT>
-__device__ __forceinline__ float unit_dot(uint32_t qtype, uint32_t row, const LaneConst &lc, const UnitAct &ua) {
-    if (QT == QT_Q4_Q6) return qtype == IB_Q4_K ? Unit<IB_Q4_K>::dot(row, lc, ua) : Unit<IB_Q6_K>::dot(row, lc, ua);
-    if (QT != QT_MIXED) return Unit<(QT == QT_MIXED || QT == QT_Q4_Q6) ? IB_Q4_K : QT>::dot(row, lc, ua);
-    switch (qtype) {
-    case IB_Q4_K: return Unit<IB_Q4_K>::dot(row, lc, ua);
-    case IB_Q6_K: return Unit<IB_Q6_K>::dot(row, lc, ua);
-    case IB_Q5_K: return Unit<IB_Q5_K>::dot(row, lc, ua);
-    default: return Unit<IB_Q8_0>::dot(row, lc, ua);
-    }
+// f(Frag<format>) for the format of a launch's instance, or of its segment where the instance serves several
+template <uint32_t QT, class F>
+__device__ __forceinline__ void with_format(uint32_t qtype, F &&f) {
+    if constexpr (QT == QT_Q4_Q6) {
+        if (qtype == IB_Q4_K) f(Frag<IB_Q4_K>{});
+        else f(Frag<IB_Q6_K>{});
+    } else if constexpr (QT == QT_MIXED) {
+        switch (qtype) {
+        case IB_Q4_K: f(Frag<IB_Q4_K>{}); break;
+        case IB_Q6_K: f(Frag<IB_Q6_K>{}); break;
+        case IB_Q5_K: f(Frag<IB_Q5_K>{}); break;
+        default: f(Frag<IB_Q8_0>{}); break;
+        }
+    } else f(Frag<QT>{});
 }
 
-// Two rows at shared addresses `a` and `b`; one format switch for both.
-template <uint32_t QT>
-__device__ __forceinline__ void unit_dot2(uint32_t qtype, uint32_t a, uint32_t b, const LaneConst &lc, const UnitAct &ua, float &va, float &vb) {
-    if (QT == QT_Q4_Q6) {
-        if (qtype == IB_Q4_K) { va = Unit<IB_Q4_K>::dot(a, lc, ua); vb = Unit<IB_Q4_K>::dot(b, lc, ua); }
-        else { va = Unit<IB_Q6_K>::dot(a, lc, ua); vb = Unit<IB_Q6_K>::dot(b, lc, ua); }
-        return;
-    }
-    va = unit_dot<QT>(qtype, a, lc, ua);
-    vb = unit_dot<QT>(qtype, b, lc, ua);
+// How a launch's rows are split over the consumer warps: NB blocks of 256 columns per warp, CG warps side by side cover a row and
+// form a stream, RG such streams share the tiles.  One or two blocks per warp where half of the warps then cover a row (one stream
+// per pipeline; short rows leave room for two), four for longer rows - 8 rows at a time as long as three such tiles fit the ring
+// (`long8`), else 4 rows at a time.
+constexpr uint32_t ROWS8 = 0, ROWS8_LONG = 1, ROWS4 = 2;   // 8 rows of one or two blocks per warp, of up to four, 4 rows of up to four
+struct Split { uint32_t NB, CG, RG, mode; };
+inline Split split_of(uint32_t cols, bool long8) {
+    const uint32_t blocks = cols / 256;
+    Split s;
+    s.NB = blocks <= 8 ? 1 : (blocks <= 16 ? 2 : NB_MAX);
+    s.mode = s.NB < NB_MAX ? ROWS8 : (long8 ? ROWS8_LONG : ROWS4);
+    s.CG = (blocks + s.NB - 1) / s.NB;
+    s.RG = s.CG <= 4 ? 4 : (s.CG <= 8 ? 2 : 1);   // 1, or a multiple of the pipelines
+    return s;
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -483,17 +584,31 @@ __device__ __forceinline__ void pack_prefetch_norm8(const float *__restrict__ no
         g[1] = __ldg(reinterpret_cast<const float4 *>(norm_w) + 2 * grp + 1);
     } else g[0] = g[1] = make_float4(1.f, 1.f, 1.f, 1.f);
 }
+// Eight floats past L1 (the previous kernel has just written them).  As two 16-byte loads a warp fetches every 32-byte sector
+// twice, and all SMs want the same sectors at once.  `whole`: 32-byte aligned.
+__device__ __forceinline__ void load_8(const float4 *p, bool whole, float4 &a, float4 &b) {
+    if (whole)
+        asm volatile("ld.global.cg.v8.f32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                     : "=f"(a.x), "=f"(a.y), "=f"(a.z), "=f"(a.w), "=f"(b.x), "=f"(b.y), "=f"(b.z), "=f"(b.w)
+                     : "l"(p)
+                     : "memory");
+    else {
+        a = __ldcg(p);
+        b = __ldcg(p + 1);
+    }
+}
 __device__ __forceinline__ void pack_stream(uint8_t *smem, uint32_t cols, const float *__restrict__ x, const float *__restrict__ norm_w, float *red,
-                                            uint32_t ss_bar, const float4 (&g)[2], uint32_t nq) {
+                                            uint32_t ss_bar, const float4 (&g)[2]) {
     constexpr uint32_t NT = PACK_THREADS;
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, groups = cols / 8;   // cols is a multiple of 64: whole four-lane groups
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, groups = cols / 8;   // cols is a multiple of 256: whole warps
     const float4 *x4 = reinterpret_cast<const float4 *>(x), *w4 = reinterpret_cast<const float4 *>(norm_w);
+    const bool whole = ((uintptr_t)x & 31) == 0;
     float4 r[PACK_GROUPS][2];
 #pragma unroll
     for (uint32_t i = 0; i < PACK_GROUPS; i++) {
         const uint32_t grp = tid + NT * i;
-        r[i][0] = grp < groups ? __ldcg(x4 + 2 * grp) : make_float4(0.f, 0.f, 0.f, 0.f);
-        r[i][1] = grp < groups ? __ldcg(x4 + 2 * grp + 1) : make_float4(0.f, 0.f, 0.f, 0.f);
+        r[i][0] = r[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (grp < groups) load_8(x4 + 2 * grp, whole, r[i][0], r[i][1]);
     }
     if (norm_w) {
         // crates/inferi-shaders/src/rms_norm.rs:112-120: the sum of squares; the factor itself is applied by the epilogue warp
@@ -509,8 +624,7 @@ __device__ __forceinline__ void pack_stream(uint8_t *smem, uint32_t cols, const 
             mbar_arrive(ss_bar);   // a release: the epilogue warp's wait sees red[warp]
         }
     }
-    const uint32_t ls = cols + (nq ? 64u : 0u);   // = Act::lstride()
-    float *sc = reinterpret_cast<float *>(smem + ACT_LIMBS * ls), *sx16 = sc + cols / 32;
+    float *sc = reinterpret_cast<float *>(smem + ACT_LIMBS * cols), *sx16 = sc + cols / 32;
 #pragma unroll
     for (uint32_t i = 0; i < PACK_GROUPS; i++) {
         const uint32_t grp = tid + NT * i;
@@ -528,22 +642,22 @@ __device__ __forceinline__ void pack_stream(uint8_t *smem, uint32_t cols, const 
                            fmaxf(fmaxf(fabsf(v[1].x), fabsf(v[1].y)), fmaxf(fabsf(v[1].z), fabsf(v[1].w))));
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
         amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        const float inv = amax > 0.f ? __fdividef(127.0f, amax) : 0.f;   // 2 ulp: the limbs absorb it (|t| stays within 127 + 1e-5)
+        const float inv = amax > 0.f ? __fdividef(ACT_STEPS, amax) : 0.f;   // 2 ulp: the limbs absorb it (the largest |x| still rounds to 32512)
         uint32_t w0[2], w1[2];
-        float sum = 0.f;
+        int s0 = 0, s1 = 0;
 #pragma unroll
         for (int j = 0; j < 2; j++) {
             const float e[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
-            pack_four(e, inv, w0[j], w1[j], sum);
+            pack_four(e, inv, w0[j], w1[j], s0, s1);
         }
+        int sum = limb_sum(s0, s1);
         sum += __shfl_xor_sync(0xffffffffu, sum, 1);
         if (ok) {
             const uint32_t run = grp >> 1;
-            uint8_t *l0 = smem + 16 * act_chunk_pos(run, nq) + 8 * (grp & 1);
-            *reinterpret_cast<uint2 *>(l0) = make_uint2(w0[0], w0[1]);
-            *reinterpret_cast<uint2 *>(l0 + ls) = make_uint2(w1[0], w1[1]);
-            if ((grp & 3) == 0) sc[grp >> 2] = amax * ACT_UNIT;
-            if ((grp & 1) == 0) sx16[run] = sum * (amax * (1.0f / 127.0f));
+            *reinterpret_cast<uint2 *>(smem + 8 * grp) = make_uint2(w0[0], w0[1]);
+            *reinterpret_cast<uint2 *>(smem + cols + 8 * grp) = make_uint2(w1[0], w1[1]);
+            if ((grp & 3) == 0) sc[grp >> 2] = amax * (1.0f / ACT_STEPS);
+            if ((grp & 1) == 0) sx16[run] = (float)sum * (amax * (1.0f / ACT_STEPS));
         }
     }
     named_barrier(1, PACK_THREADS);

@@ -184,11 +184,7 @@ static int32_t record_token(ib_llama *m, cudaStream_t s, uint32_t pdl) {
     const uint32_t H = c.hidden_size, L = c.num_hidden_layers;
     const CommLayout cl(H, tp);
     int32_t rc;
-    // every launch of the graph asks for the shared two-format instance where its formats allow (Q4_K_M models: all of them)
-    auto emit_gemv = [&](GemvParams p) -> int32_t {
-        p.pair_instance = 1;
-        return launch_gemv(ctx, s, p);
-    };
+    auto emit_gemv = [&](const GemvParams &p) -> int32_t { return launch_gemv(ctx, s, p); };
     auto emit_attn = [&](const AttnLaunch &a) -> int32_t { return launch_attention(ctx, s, a); };
     {
         QDesc e{m->token_embd->dev, m->token_embd->row_bytes, (uint32_t)m->token_embd->qtype, m->token_embd->layout, m->token_embd->nb};
@@ -874,7 +870,7 @@ int32_t ib_llama_prefill(ib_llama *m, void *stream, const uint32_t *tokens_host,
     GemvParams p = {};
     fill_seg(p.seg[0], m->output, m->logits);
     p.nseg = 1; p.cols = H; p.epi = EPI_ARGMAX; p.x = m->x; p.norm_w = m->output_norm; p.eps = c.rms_norm_eps;
-    p.argmax_slots = m->argmax_slots; p.argmax_counter = m->argmax_counter; p.argmax_out = &m->ctl->next; p.pair_instance = 1;
+    p.argmax_slots = m->argmax_slots; p.argmax_counter = m->argmax_counter; p.argmax_out = &m->ctl->next;
     if ((rc = launch_gemv(ctx, s, p))) return rc;
     m->x_final = m->x;
     if (next_token_host) IB_CHECK_CUDA(cudaMemcpyAsync(next_token_host, &m->ctl->next, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));

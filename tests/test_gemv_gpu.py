@@ -8,7 +8,7 @@ import torch
 import oracle
 from helpers import OP_RTOL, assert_close
 from inferi_b200 import quant
-from inferi_b200.ops import GemvQuant, GpuQuantTensor, InferiError
+from inferi_b200.ops import FfnGateUp, GemvQuant, GpuQuantTensor, InferiError
 
 pytestmark = pytest.mark.gpu
 GOLDEN = np.load(os.path.join(os.path.dirname(__file__), "golden", "blocks.npz"))
@@ -75,6 +75,28 @@ def test_benchmark_shapes(backend, qt, rows, cols, seed):
     # linearity in v (a size-independent property): W(2v) == 2 W v exactly in binary floating point
     got2 = run_gemv(backend, qt, rows, cols, blocks, 2 * v)
     assert np.array_equal(got2, 2 * got)
+
+
+# where the streaming kernel's split changes: 1, 5, 9, 17, 32, 33 blocks of 256 columns (blocks per warp, warps per row, a last
+# warp with fewer blocks), rows so long that it works on 4 instead of 8 of them (with 1, 2, 3 and 4 blocks in the last warp), and
+# row counts that leave every SM a few rows more or less than whole tiles
+@pytest.mark.parametrize("qt,rows,cols", [
+    (quant.Q4_K, 1484, 256), (quant.Q4_K, 1484, 1280), (quant.Q5_K, 2372, 2304), (quant.Q8_0, 1484, 2304), (quant.Q5_K, 1484, 4352),
+    (quant.Q4_K, 1484, 8192), (quant.Q6_K, 596, 8192), (quant.Q4_K, 1484, 8448), (quant.Q8_0, 1484, 8448), (quant.Q8_0, 300, 9728),
+    (quant.Q8_0, 300, 9984), (quant.Q6_K, 1484, 10240), (quant.Q5_K, 300, 14336), (quant.Q4_K, 300, 16128),
+])
+def test_streaming_splits(backend, qt, rows, cols):
+    _shape_case(backend, qt, rows, cols)
+    # the fused gate/up launch: gate and up rows of a tile are worked on together
+    g = quant.random_blocks(qt, rows, cols, seed=rows + cols)
+    u = quant.random_blocks(qt, rows, cols, seed=rows + cols + 1)
+    v = np.random.default_rng(cols + 1).standard_normal(cols).astype(np.float32)
+    gm, um = (GpuQuantTensor(backend, qt, rows, cols, m) for m in (g, u))
+    out = torch.empty(rows, device="cuda")
+    FfnGateUp(backend).launch(out, gm, um, torch.from_numpy(v).cuda())
+    a, b = (np.asarray(oracle.gemv_ref(qt, rows, cols, m, v), np.float64) for m in (g, u))
+    # the product of two dot products, each within OP_RTOL
+    assert_close(out.cpu().numpy(), b * a / (1 + np.exp(-np.maximum(a, -700.0))), rtol=2 * OP_RTOL, what=f"gate/up {quant.NAMES[qt]} {rows}x{cols}")
 
 
 def test_f32_matrix_and_special_vectors(backend):
