@@ -191,15 +191,16 @@ __device__ __forceinline__ void finish_tiles(const GemvParams &p, const StreamGe
         for (int w = 0; w < PACK_THREADS / 32; w++) t += red[w];
         rms = 1.0f / sqrtf(t / (float)p.cols + p.eps);
     }
-    const bool residual = p.epi == EPI_RESIDUAL;
+    const bool reads = p.epi == EPI_RESIDUAL || p.epi == EPI_QKV;
+    const uint32_t pos = p.epi == EPI_QKV ? __ldcg(p.pos_ptr) : 0u;
 #pragma unroll 1
     for (;;) {
-        // the pairs' residual values are requested before the wait for the dot products: the L2 round trip overlaps it
-        float2 rpre = make_float2(0.f, 0.f);
-        if (residual) {
+        // what the epilogue reads is requested before the wait for the dot products: the L2 round trip overlaps it
+        float2 pre = make_float2(0.f, 0.f);
+        if (reads) {
             if (!mbar_wait(bar0 + 8 * st, par, p.err, 1, p.wait_ns)) return;
             const uint4 tm = lds128(meta + 16 * st);
-            if (lane < tm.z) rpre = residual_prefetch(p.resid, tm.y + lane);
+            if (lane < tm.z) pre = epilogue_prefetch(p, tm.x, tm.y + lane);
         }
         if (!mbar_wait(bar0 + 8 * (2 * S + st), par, p.err, 5, p.wait_ns)) return;   // (implies the tile's announcement)
         const uint4 tm = lds128(meta + 16 * st);
@@ -222,7 +223,7 @@ __device__ __forceinline__ void finish_tiles(const GemvParams &p, const StreamGe
                 va += __shfl_xor_sync(0xffffffffu, va, o);
                 vb += __shfl_xor_sync(0xffffffffu, vb, o);
             }
-        if (mine) epilogue(p, s, first_pair + lane, va * rms, vb * rms, best, rpre);
+        if (mine) epilogue(p, s, first_pair + lane, va * rms, vb * rms, best, pre, pos);
         st += geo.P;
         if (st >= S) {
             st = pipe;
@@ -288,6 +289,10 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const Ge
         }
         uint32_t cost = swiglu ? (uint32_t)p.seg[0].row_bytes : geo.seg_cost[0], cost_b = (uint32_t)p.seg[1].row_bytes, cur = 0;
         const uint8_t *w = p.seg[0].w, *wb = p.seg[1].w;
+        // The weights of a token pass through L2 once; as the first to be evicted they leave the rest of it - the code of the token's
+        // other kernels, the cache, the activations - in place (attention in the first layer of a token, after the classifier's
+        // hundreds of megabytes: 13.5 us instead of 5).
+        const uint64_t policy = evict_first_policy();
         uint32_t st = pipe, ring = smem_u32(smem), par = 1, ends = 0;   // par: parity of the slot's previous use ("1" before the first one); ends: end markers, one per stream
         bool first_round = true;
         for (;;) {
@@ -319,8 +324,8 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const Ge
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the consumers' reads of the slot come first
                 const uint32_t ba = n * cost, bb = swiglu ? n * cost_b : 0u, dst = ring + st * geo.stage_bytes;
                 mbar_expect_tx(full, ba + bb);
-                bulk_g2s(dst, w + (size_t)tm.y * cost, ba, full);
-                if (swiglu) bulk_g2s(dst + geo.seg_pt[0] * cost, wb + (size_t)tm.y * cost_b, bb, full);
+                bulk_g2s(dst, w + (size_t)tm.y * cost, ba, full, policy);
+                if (swiglu) bulk_g2s(dst + geo.seg_pt[0] * cost, wb + (size_t)tm.y * cost_b, bb, full, policy);
                 if (!dyn) tc.advance(sh);
                 else { t++; held--; }
             }

@@ -120,9 +120,16 @@ __device__ __forceinline__ bool wait_counter_gpu(const uint32_t *flag, uint32_t 
     return false;
 }
 
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar) {
-    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+// `policy`: an L2 eviction policy from evict_first_policy()
+__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void *src, uint32_t bytes, uint32_t bar, uint64_t policy) {
+    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1], %2, [%3], %4;" ::"r"(dst), "l"(src), "r"(bytes),
+                 "r"(bar), "l"(policy)
                  : "memory");
+}
+__device__ __forceinline__ uint64_t evict_first_policy() {
+    uint64_t p;
+    asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));
+    return p;
 }
 
 // Shared-memory loads by 32-bit shared address (no generic-address arithmetic in the inner loop).  volatile: they stay
@@ -663,12 +670,18 @@ __device__ __forceinline__ void pack_stream(uint8_t *smem, uint32_t cols, const 
     named_barrier(1, PACK_THREADS);
 }
 
-__device__ __forceinline__ float2 residual_prefetch(const float *resid, uint32_t pair) { return __ldcg(reinterpret_cast<const float2 *>(resid + 2 * pair)); }
+// What the epilogue of a pair reads from memory: the residual, or the rotation of a q / k pair.  Requested ahead of the wait for
+// the dot products.
+__device__ __forceinline__ float2 epilogue_prefetch(const GemvParams &p, uint32_t s, uint32_t pair) {
+    if (p.epi == EPI_RESIDUAL) return __ldcg(reinterpret_cast<const float2 *>(p.resid + 2 * pair));
+    if (p.epi == EPI_QKV && s < 2) return __ldcg(p.rope_cs + (((2 * pair) % p.head_size) >> 1));
+    return make_float2(0.f, 0.f);
+}
 
-// ---- epilogue of one row pair (run by the epilogue warp only, so the kind of epilogue is a run-time switch: one kernel
+// ---- epilogue of one row pair (run by an epilogue warp only, so the kind of epilogue is a run-time switch: one kernel
 // instance per weight format serves every role in the token graph and stays in the instruction cache) ----
-// `resid_pre`: the pair's residual values (EPI_RESIDUAL), fetched by the caller ahead of the wait for the dot products.
-__device__ __forceinline__ void epilogue(const GemvParams &p, uint32_t s, uint32_t pair, float a, float b, unsigned long long &best, float2 resid_pre) {
+// `pre`: from epilogue_prefetch;  `pos`: the token's position (EPI_QKV).
+__device__ __forceinline__ void epilogue(const GemvParams &p, uint32_t s, uint32_t pair, float a, float b, unsigned long long &best, float2 pre, uint32_t pos) {
     const uint32_t epi = p.epi;
     if (epi == EPI_SWIGLU) {
         // crates/inferi-shaders/src/silu.rs:16-19,46-52: a = gate row, b = up row
@@ -679,7 +692,7 @@ __device__ __forceinline__ void epilogue(const GemvParams &p, uint32_t s, uint32
     if (epi == EPI_STORE) {
         *reinterpret_cast<float2 *>(p.seg[s].out + r0) = make_float2(a, b);
     } else if (epi == EPI_RESIDUAL) {
-        *reinterpret_cast<float2 *>(p.seg[s].out + r0) = make_float2(resid_pre.x + a, resid_pre.y + b);
+        *reinterpret_cast<float2 *>(p.seg[s].out + r0) = make_float2(pre.x + a, pre.y + b);
     } else if (epi == EPI_QKV) {
         if (p.bias[s]) {
             const float2 bv = __ldg(reinterpret_cast<const float2 *>(p.bias[s] + r0));
@@ -688,16 +701,15 @@ __device__ __forceinline__ void epilogue(const GemvParams &p, uint32_t s, uint32
         }
         if (s < 2) {
             // crates/inferi-shaders/src/rope.rs:75-91 (adjacent pairs)
-            const float2 cs = __ldcg(p.rope_cs + ((r0 % p.head_size) >> 1));
             const float x = a, y = b;
-            a = cs.x * x - cs.y * y;
-            b = cs.y * x + cs.x * y;
+            a = pre.x * x - pre.y * y;
+            b = pre.y * x + pre.x * y;
         }
         if (s == 0) {
             *reinterpret_cast<float2 *>(p.seg[0].out + r0) = make_float2(a, b);
         } else {
             void *cache = (s == 1) ? p.k_cache : p.v_cache;
-            const size_t off = (size_t)(*p.pos_ptr) * p.kv_dim + r0;
+            const size_t off = (size_t)pos * p.kv_dim + r0;
             if (p.kv_dtype == IB_KV_F16) reinterpret_cast<__half2 *>(cache)[off >> 1] = __floats2half2_rn(a, b);
             else reinterpret_cast<float2 *>(cache)[off >> 1] = make_float2(a, b);
         }
