@@ -81,8 +81,48 @@ bool attn_gqa4_eligible(const AttnLaunch &a) {
            ((uintptr_t)a.k_cache % 16) == 0 && ((uintptr_t)a.v_cache % 16) == 0 && ((uintptr_t)a.out % 16) == 0 && ((uintptr_t)a.scratch % 16) == 0;
 }
 
-uint32_t attn_cluster_positions(const AttnLaunch &a) {
-    return attn_gqa4_eligible(a) ? gqa4_cluster_size(a.max_splits) * GQA4_CLUSTER_PER : 0u;
+// CTAs per cluster: as many as fit the GPU with one cluster per kv head
+static uint32_t gqa4_cluster_ctas(const ib_ctx *ctx, const ib_attn_params &p) {
+    const uint32_t n_kv = p.n_heads / p.kv_mul;
+    uint32_t c = GQA4_CLUSTER_MAX;
+    while (c > 1 && c * n_kv > (uint32_t)ctx->sm_count) c /= 2;
+    return c;
+}
+
+// The middle regime ends where the long one's bytes in flight (three CTAs on every SM against one on less than half of them) outweigh
+// its slower merge: measured us per launch, 8 kv heads, middle / long - head size 64: 6.9 / 8.7 at 2048 positions, 12.8 / 16.1 at
+// 8192, 20.1 / 20.8 at 16384; head size 128: 8.7 / 9.7 at 2048, 12.4 / 12.0 at 4096.  Its CTAs need an SM each and their clusters a GPC
+// with so many free ones: with clusters on more than half of the SMs some wait for others (16 kv heads: twice the time).
+constexpr uint32_t GQA4_MIDDLE_PER_64 = 2048, GQA4_MIDDLE_PER_128 = 384;
+uint32_t attn_regime_positions(const ib_ctx *ctx, const AttnLaunch &a, uint32_t regime) {
+    if (!attn_gqa4_eligible(a) || ctx->sm_count == 0) return 0u;   // (ib_attention_static knows no device)
+    const uint32_t c = gqa4_cluster_ctas(ctx, a.p), n_kv = a.p.n_heads / a.p.kv_mul;
+    if (regime == ATTN_SHORT) return c * GQA4_SHORT_PER;
+    if (2 * c * n_kv > (uint32_t)ctx->sm_count) return 0u;
+    return c * (a.p.head_size == 128 ? GQA4_MIDDLE_PER_128 : GQA4_MIDDLE_PER_64);
+}
+
+template <int HS, uint32_t REGIME>
+static int32_t launch_gqa4(ib_ctx *ctx, cudaStream_t s, const AttnArgs &args, dim3 grid) {
+    const uint32_t smem = gqa4_smem_floats(HS, REGIME) * sizeof(float);   // at most 48 KB: no attribute needed
+    static_assert(gqa4_smem_floats(HS, REGIME) * sizeof(float) + 4096 <= 49152, "dynamic and static shared memory without opting in");
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(gqa4_warps(HS, REGIME) * 32);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 1;
+    attr[0].val.clusterDim.y = REGIME != ATTN_LONG ? grid.y : 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = args.pdl ? 2 : 1;
+    IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, attn_gqa4_kernel<HS, REGIME>, args));
+    ctx->launches++;
+    return IB_OK;
 }
 
 int32_t launch_attention(ib_ctx *ctx, cudaStream_t s, const AttnLaunch &a) {
@@ -96,44 +136,35 @@ int32_t launch_attention(ib_ctx *ctx, cudaStream_t s, const AttnLaunch &a) {
     AttnArgs args{p, a.pos_ptr, a.q, a.k_cache, a.v_cache, a.out, a.scratch, a.counters, a.max_splits, a.pdl, 0u};
     const bool f16 = a.kv_dtype == IB_KV_F16;
     const bool gqa4 = attn_gqa4_eligible(a);
-    // with a host-known position only the splits that will do work are launched
+    if (gqa4) {
+        // a launch that serves many positions (a graph node) is told the regime they are in
+        uint32_t regime = a.regime;
+        if (!a.pos_ptr) {
+            regime = ATTN_LONG;
+            for (uint32_t r : {ATTN_MIDDLE, ATTN_SHORT})
+                if (p.pos < attn_regime_positions(ctx, a, r)) regime = r;
+        }
+        uint32_t splits = a.max_splits, per;
+        if (regime != ATTN_LONG) args.cluster = splits = gqa4_cluster_ctas(ctx, p);
+        if (!a.pos_ptr) {   // with a host-known position only the slices that will do work are launched
+            gqa4_plan(p.pos + 1, a.max_splits, args.cluster, gqa4_warps(p.head_size, regime), splits, per);
+            if (regime != ATTN_LONG) args.cluster = splits;
+        }
+        const dim3 grid(n_kv, splits);
+        const bool wide = p.head_size == 128;
+        switch (regime) {
+        case ATTN_SHORT: return wide ? launch_gqa4<128, ATTN_SHORT>(ctx, s, args, grid) : launch_gqa4<64, ATTN_SHORT>(ctx, s, args, grid);
+        case ATTN_MIDDLE: return wide ? launch_gqa4<128, ATTN_MIDDLE>(ctx, s, args, grid) : launch_gqa4<64, ATTN_MIDDLE>(ctx, s, args, grid);
+        default: return wide ? launch_gqa4<128, ATTN_LONG>(ctx, s, args, grid) : launch_gqa4<64, ATTN_LONG>(ctx, s, args, grid);
+        }
+    }
     uint32_t splits = a.max_splits;
     if (!a.pos_ptr) {
         uint32_t need, per;
-        if (gqa4) attn_split_plan(p.pos + 1, a.max_splits, need, per, GQA4_MIN_PER_SPLIT, GQA4_KNEE, GQA4_KNEE_PER);
-        else attn_split_plan(p.pos + 1, a.max_splits, need, per);
+        attn_split_plan(p.pos + 1, a.max_splits, need, per);
         if (need < splits) splits = need;
     }
-    if (gqa4) {
-        // short contexts merge inside a thread-block cluster (the first one of the kv head)
-        if (a.pos_ptr) {
-            args.cluster = a.short_context ? gqa4_cluster_size(splits) : 0u;
-        } else if (p.pos + 1 <= GQA4_CLUSTER_MAX * GQA4_CLUSTER_PER) {
-            const uint32_t want = (p.pos + 1 + GQA4_MIN_PER_SPLIT - 1) / GQA4_MIN_PER_SPLIT;
-            const uint32_t cs = want < GQA4_CLUSTER_MAX ? want : GQA4_CLUSTER_MAX;
-            if (cs >= 2 && cs <= a.max_splits) { splits = cs; args.cluster = cs; }
-        }
-    }
     const dim3 grid(n_kv, splits);
-    if (gqa4) {
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = grid;
-        cfg.blockDim = dim3(ATTN_THREADS);
-        cfg.stream = s;
-        cudaLaunchAttribute attr[2];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 1;
-        attr[0].val.clusterDim.y = args.cluster ? args.cluster : 1;
-        attr[0].val.clusterDim.z = 1;
-        attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-        attr[1].val.programmaticStreamSerializationAllowed = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = args.pdl ? 2 : 1;
-        if (p.head_size == 128) IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, attn_gqa4_kernel<128>, args));
-        else IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, attn_gqa4_kernel<64>, args));
-        ctx->launches++;
-        return IB_OK;
-    }
     if (p.head_size == 128) return f16 ? launch_kvm<128, __half>(ctx, s, args, grid) : launch_kvm<128, float>(ctx, s, args, grid);
     if (p.head_size == 64) return f16 ? launch_kvm<64, __half>(ctx, s, args, grid) : launch_kvm<64, float>(ctx, s, args, grid);
     return set_error(IB_ERR_UNSUPPORTED, "attention: head_size=%u (supported: 64, 128)", p.head_size);

@@ -22,29 +22,23 @@
 namespace ib {
 
 constexpr uint32_t GQA4_ROWS_PER_WARP_STEP = 8;
-// Slices: one warp step of every warp (32 positions) each while there are at most 16 of them, then 16 slices that grow to
-// 128 positions, then slices of 128 positions up to the launch's maximum, then longer ones.  Measured on a B200 (us per
-// launch at 128 / 512 / 2048 / 8192 positions): 32 per slice throughout 4.6 / 6.1 / 12.6 / 17.1; 128 per slice 5.4 / 7.6 /
-// 9.1 / 17.1; 256 per slice 5.4 / 10.6 / 11.3 / 16.1.
+// Three ways to split a kv head's positions, by context length:
+//  * short: the slices are the CTAs of one thread-block cluster, 4 warps each.  They leave their partials in the shared memory of the
+//    cluster's first CTA (distributed shared memory) and meet at the cluster barrier; the first CTA merges from its own shared
+//    memory.  Publishing the partials through global memory, counting arrivals with an atomic and reading them back are three L2
+//    round trips (~2.6 us of a ~6 us kernel at these lengths); the cluster barrier is one hardware barrier.  Up to two row-loop
+//    iterations per slice.
+//  * middle: the same with 8 or 16 warps per CTA, which hold the row loop at a few iterations.
+//  * long: many CTAs of 4 warps (one wave of 3 per SM), merged through global memory.  Slices: one warp step of every warp (32
+//    positions) each while there are at most 16 of them, then 16 slices that grow to 128 positions, then slices of 128
+//    positions up to the launch's maximum, then longer ones.
+// Clusters have at most 8 CTAs: eight clusters of 16 - one per kv head of the Llama-3 models - do not all fit the GPU at once.
+constexpr uint32_t GQA4_CLUSTER_MAX = 8, GQA4_SHORT_PER = 64;   // positions per slice up to which `short` is used
+__host__ __device__ constexpr int gqa4_warps(uint32_t hs, uint32_t regime) { return regime != ATTN_MIDDLE ? ATTN_WARPS : (hs == 128 ? 8 : 16); }   // (head size 128 needs 142 registers)
 constexpr uint32_t GQA4_MIN_PER_SPLIT = ATTN_WARPS * GQA4_ROWS_PER_WARP_STEP, GQA4_KNEE = 16, GQA4_KNEE_PER = 128;
-// Short contexts: the slices of a kv head (at most 8) are the CTAs of one thread-block cluster.  They leave their partials in
-// the shared memory of the cluster's first CTA (distributed shared memory) and meet at the cluster barrier; the first CTA
-// merges from its own shared memory.  Publishing the partials through global memory, counting arrivals with an atomic and
-// reading them back are three L2 round trips (~2.6 us of a ~6 us kernel at these lengths); the cluster barrier is one
-// hardware barrier.  Longer contexts use more slices than a cluster has CTAs and keep the global-memory merge.
-// The cluster size is a divisor of the launch's slice count (so that no CTA is launched for the clusters' sake: with 55
-// slices x 8 kv heads = 440 CTAs the grid is exactly one wave of 148 SMs x 3, and rounding 55 up to 56 made a second wave
-// that cost 40 % at long contexts); `cluster` = 0: no clusters.
-constexpr uint32_t GQA4_CLUSTER_MAX = 8, GQA4_CLUSTER_PER = 64;   // beyond two row-loop iterations per slice the sixteen slices of the global merge are faster
-__host__ __device__ __forceinline__ uint32_t gqa4_cluster_size(uint32_t splits) {
-    for (uint32_t c = GQA4_CLUSTER_MAX; c >= 2; c--)
-        if (splits % c == 0) return c;
-    return 0;
-}
-__host__ __device__ __forceinline__ void gqa4_plan(uint32_t total, uint32_t max_splits, uint32_t cluster, uint32_t &nsplit, uint32_t &per, bool &in_cluster) {
-    in_cluster = cluster != 0 && total <= cluster * GQA4_CLUSTER_PER;
-    if (in_cluster) {
-        nsplit = (total + GQA4_MIN_PER_SPLIT - 1) / GQA4_MIN_PER_SPLIT;
+__host__ __device__ __forceinline__ void gqa4_plan(uint32_t total, uint32_t max_splits, uint32_t cluster, uint32_t warps, uint32_t &nsplit, uint32_t &per) {
+    if (cluster) {
+        nsplit = (total + warps * GQA4_ROWS_PER_WARP_STEP - 1) / (warps * GQA4_ROWS_PER_WARP_STEP);
         if (nsplit > cluster) nsplit = cluster;
         per = (total + nsplit - 1) / nsplit;
         nsplit = (total + per - 1) / per;
@@ -78,20 +72,53 @@ __device__ __forceinline__ void halve_exchange(float (&v)[N], int lane, int o) {
     }
 }
 
-template <int HS>
-__global__ void __launch_bounds__(ATTN_THREADS, 3) attn_gqa4_kernel(const AttnArgs a) {
+// o += w * p[0 .. N-1];  p[0 .. N-1] = w * o: in pairs where there are any (p is 8-byte aligned then)
+template <int N>
+__device__ __forceinline__ void add_scaled(float (&o)[N], float w, const float *p) {
+    if constexpr (N % 2 == 0) {
+#pragma unroll
+        for (int e = 0; e < N; e += 2) {
+            const float2 v = *reinterpret_cast<const float2 *>(p + e);
+            o[e] += w * v.x;
+            o[e + 1] += w * v.y;
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < N; e++) o[e] += w * p[e];
+    }
+}
+template <int N>
+__device__ __forceinline__ void store_scaled(float *p, const float (&o)[N], float w) {
+    if constexpr (N % 2 == 0) {
+#pragma unroll
+        for (int e = 0; e < N; e += 2) *reinterpret_cast<float2 *>(p + e) = make_float2(o[e] * w, o[e + 1] * w);
+    } else {
+#pragma unroll
+        for (int e = 0; e < N; e++) p[e] = o[e] * w;
+    }
+}
+
+// floats of dynamic shared memory: the warps' accumulators, and with clusters the slices' partials (in the first CTA)
+__host__ __device__ constexpr uint32_t gqa4_smem_floats(uint32_t hs, uint32_t regime) {
+    return gqa4_warps(hs, regime) * 4 * hs + (regime != ATTN_LONG ? GQA4_CLUSTER_MAX * 4 * (hs + 2) : 0);
+}
+
+template <int HS, uint32_t REGIME>
+__global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MIDDLE ? 1 : 3) attn_gqa4_kernel(const AttnArgs a) {
     constexpr int KVM = 4, EPL = 8;
+    constexpr bool CLUSTER = REGIME != ATTN_LONG;
+    constexpr int W = gqa4_warps(HS, REGIME), T = W * 32;
     constexpr int L = HS / EPL;          // lanes per cache row
     constexpr int RPW = 32 / L;          // rows per warp step
     constexpr int STEPS = L / KVM;       // steps per warp iteration: STEPS * KVM partial scores per lane = L
     constexpr int ROWS = STEPS * RPW;    // = 8
     static_assert(ROWS == (int)GQA4_ROWS_PER_WARP_STEP && STEPS * KVM == L, "lane layout");
-    __shared__ __align__(16) float sm_acc[ATTN_WARPS * KVM * HS];
-    __shared__ float sm_m[ATTN_WARPS * KVM], sm_l[ATTN_WARPS * KVM];
-    __shared__ __align__(16) float sm_p[ATTN_WARPS][32];
-    __shared__ __align__(16) float sm_alpha[ATTN_WARPS][4];
+    extern __shared__ __align__(16) float sm_acc[];   // [W][KVM][HS]
+    float *sm_cl = sm_acc + W * KVM * HS;             // clusters: [slices][KVM][HS + 2]
+    __shared__ float sm_m[W * KVM], sm_l[W * KVM];
+    __shared__ __align__(16) float sm_p[W][32];
+    __shared__ __align__(16) float sm_alpha[W][4];
     __shared__ uint32_t sm_last;
-    __shared__ __align__(16) float sm_cl[GQA4_CLUSTER_MAX * KVM * (HS + 2)];   // cluster mode: the slices' partials, in the first CTA
 
     if (a.pdl) asm volatile("griddepcontrol.launch_dependents;");
     const bool early = a.pdl == 1;   // rows may be requested ahead of the wait
@@ -100,13 +127,9 @@ __global__ void __launch_bounds__(ATTN_THREADS, 3) attn_gqa4_kernel(const AttnAr
     const uint32_t kvh = blockIdx.x, split = blockIdx.y;
     const uint32_t total = (a.pos_ptr ? *a.pos_ptr : a.p.pos) + 1;
     uint32_t nsplit, per;
-    bool in_cluster;
-    gqa4_plan(total, a.max_splits, a.cluster, nsplit, per, in_cluster);
-    // cluster mode: the first cluster of a kv head (slices 0 .. a.cluster - 1) does the work, all of its CTAs meet at the barrier below
-    // (the ones without a slice bring nothing); the other clusters leave as a whole
-    if (in_cluster ? split >= a.cluster : split >= nsplit) return;
-    if (in_cluster && split >= nsplit) {
-        if (nsplit > 1) cooperative_groups::this_cluster().sync();   // the barrier of the working CTAs below
+    gqa4_plan(total, a.max_splits, CLUSTER ? a.cluster : 0u, W, nsplit, per);
+    if (split >= nsplit) {
+        if (CLUSTER && nsplit > 1) cooperative_groups::this_cluster().sync();   // the barrier of the working CTAs below
         return;
     }
     const uint32_t t0 = split * per, t1 = min(total, t0 + per);
@@ -167,8 +190,8 @@ __global__ void __launch_bounds__(ATTN_THREADS, 3) attn_gqa4_kernel(const AttnAr
     // trip plus arithmetic, however many iterations it has, and twice the bytes are in flight per warp.
     uint4 knext[STEPS], vnext[STEPS];
 #pragma unroll 1
-    for (uint32_t base = base0; base < t1; base += ATTN_WARPS * ROWS) {
-        const uint32_t nbase = base + ATTN_WARPS * ROWS;
+    for (uint32_t base = base0; base < t1; base += W * ROWS) {
+        const uint32_t nbase = base + W * ROWS;
         if (nbase < t1) {
 #pragma unroll
             for (int s = 0; s < STEPS; s++) {
@@ -264,47 +287,41 @@ __global__ void __launch_bounds__(ATTN_THREADS, 3) attn_gqa4_kernel(const AttnAr
     if (lane < KVM) { sm_m[warp * KVM + lane] = M; sm_l[warp * KVM + lane] = l; }
     __syncthreads();
 
-    // every thread owns PER consecutive outputs of one head; all of them are in flight together
+    // every thread owns PER consecutive outputs of one head (16 warps at head size 64: half of the threads one each)
     constexpr uint32_t slot = HS + 2;
-    constexpr int PER = KVM * HS / ATTN_THREADS;   // 4 (head size 128) or 2 (64)
-    static_assert(PER == 2 || PER == 4, "outputs per thread");
-    const int m_out = (tid * PER) / HS, d_out = (tid * PER) % HS;
+    constexpr int PER = KVM * HS >= T ? KVM * HS / T : 1;
+    const bool has = tid * PER < KVM * HS;
+    const int at = has ? tid * PER : 0, m_out = at / HS, d_out = at % HS;
     float *part = a.scratch + ((size_t)kvh * a.max_splits + split) * KVM * slot;
+    float *out = a.out + (size_t)(kvh * KVM + m_out) * HS + d_out;
     {
         float mx = sm_m[m_out];
 #pragma unroll
-        for (int w = 1; w < ATTN_WARPS; w++) mx = fmaxf(mx, sm_m[w * KVM + m_out]);
+        for (int w = 1; w < W; w++) mx = fmaxf(mx, sm_m[w * KVM + m_out]);
         float o[PER], ls = 0.f;
 #pragma unroll
         for (int e = 0; e < PER; e++) o[e] = 0.f;
 #pragma unroll
-        for (int w = 0; w < ATTN_WARPS; w++) {
+        for (int w = 0; w < W; w++) {
             const float wt = merge_weight(sm_m[w * KVM + m_out], mx);
             ls += wt * sm_l[w * KVM + m_out];
-#pragma unroll
-            for (int e = 0; e < PER; e += 2) {
-                const float2 t = *reinterpret_cast<const float2 *>(&sm_acc[(w * KVM + m_out) * HS + d_out + e]);
-                o[e] += wt * t.x;
-                o[e + 1] += wt * t.y;
-            }
+            add_scaled(o, wt, &sm_acc[(w * KVM + m_out) * HS + d_out]);
         }
         if (nsplit == 1) {
-            const float inv = 1.0f / ls;
-#pragma unroll
-            for (int e = 0; e < PER; e += 2)
-                *reinterpret_cast<float2 *>(a.out + (size_t)(kvh * KVM + m_out) * HS + d_out + e) = make_float2(o[e] * inv, o[e + 1] * inv);
+            if (has) store_scaled(out, o, 1.0f / ls);
             return;
         }
-        if (in_cluster) {
+        if constexpr (CLUSTER) {
             // the partial goes into the first CTA's shared memory; after the cluster barrier that CTA merges the slices
             namespace cg = cooperative_groups;
             cg::cluster_group cluster = cg::this_cluster();
-            float *dst = cluster.map_shared_rank(sm_cl, 0) + ((size_t)split * KVM + m_out) * slot;
-#pragma unroll
-            for (int e = 0; e < PER; e += 2) *reinterpret_cast<float2 *>(dst + d_out + e) = make_float2(o[e], o[e + 1]);
-            if (d_out == 0) *reinterpret_cast<float2 *>(dst + HS) = make_float2(mx, ls);
+            if (has) {
+                float *dst = cluster.map_shared_rank(sm_cl, 0) + ((size_t)split * KVM + m_out) * slot;
+                store_scaled(dst + d_out, o, 1.0f);
+                if (d_out == 0) *reinterpret_cast<float2 *>(dst + HS) = make_float2(mx, ls);
+            }
             cluster.sync();
-            if (split != 0) return;
+            if (split != 0 || !has) return;
             float cm = -INFINITY;
             for (uint32_t s = 0; s < nsplit; s++) cm = fmaxf(cm, sm_cl[(s * KVM + m_out) * slot + HS]);
             float lsum = 0.f, acc[PER];
@@ -314,19 +331,16 @@ __global__ void __launch_bounds__(ATTN_THREADS, 3) attn_gqa4_kernel(const AttnAr
                 const float *ps = sm_cl + (s * KVM + m_out) * slot;
                 const float wt = merge_weight(ps[HS], cm);
                 lsum += wt * ps[HS + 1];
-#pragma unroll
-                for (int e = 0; e < PER; e++) acc[e] += wt * ps[d_out + e];
+                add_scaled(acc, wt, ps + d_out);
             }
-            const float inv = 1.0f / lsum;
-#pragma unroll
-            for (int e = 0; e < PER; e += 2)
-                *reinterpret_cast<float2 *>(a.out + (size_t)(kvh * KVM + m_out) * HS + d_out + e) = make_float2(acc[e] * inv, acc[e + 1] * inv);
+            store_scaled(out, acc, 1.0f / lsum);
             return;
+        } else {
+            store_scaled(part + m_out * slot + d_out, o, 1.0f);
+            if (d_out == 0) *reinterpret_cast<float2 *>(part + m_out * slot + HS) = make_float2(mx, ls);
         }
-#pragma unroll
-        for (int e = 0; e < PER; e += 2) *reinterpret_cast<float2 *>(part + m_out * slot + d_out + e) = make_float2(o[e], o[e + 1]);
-        if (d_out == 0) *reinterpret_cast<float2 *>(part + m_out * slot + HS) = make_float2(mx, ls);
     }
+    if constexpr (!CLUSTER) {
 
     // The block's partial is published by one release/acquire arrival of thread 0: the barrier before it orders the other
     // threads' stores ahead of the release, the barrier after it orders their reads of the other blocks' partials (from
@@ -382,6 +396,7 @@ __global__ void __launch_bounds__(ATTN_THREADS, 3) attn_gqa4_kernel(const AttnAr
     for (int e = 0; e < PER; e += 2)
         *reinterpret_cast<float2 *>(a.out + (size_t)(kvh * KVM + m_out) * HS + d_out + e) = make_float2(o[e] * inv, o[e + 1] * inv);
     if (tid == 0) a.counters[kvh] = 0u;
+    }
 }
 
 }  // namespace ib

@@ -208,16 +208,16 @@ struct AttnLaunch {
     uint32_t max_splits;
     uint32_t pdl;              // 0: plain launch; 1: programmatic dependent launch inside the token graph, where the predecessor writes only q and the
                                // newest cache row; 2: programmatic dependent launch behind any kernel
-    // With pos_ptr (a graph node that serves many positions): the caller promises that the position stays below
-    // attn_cluster_positions(); the launch then groups a kv head's slices into a thread-block cluster and merges them there.
-    // Such a launch is slower at long contexts (clusters constrain the placement of the grid's one wave of CTAs), so a graph
-    // for longer contexts is recorded without it.  With a host-known position the launch decides by itself.
-    uint32_t short_context;
+    // With pos_ptr (a graph node that serves many positions): the caller promises that the position stays within
+    // attn_regime_positions(); a launch's shape depends on the regime, so a graph is recorded for each.  With a host-known position
+    // the launch decides by itself.
+    uint32_t regime;
 };
+constexpr uint32_t ATTN_LONG = 0, ATTN_SHORT = 1, ATTN_MIDDLE = 2;
 bool attn_gqa4_eligible(const AttnLaunch &a);
 size_t attn_scratch_bytes(const ib_attn_params &p, uint32_t max_splits);
 uint32_t attn_max_splits(const ib_ctx *ctx, const ib_attn_params &p);
 int32_t launch_attention(ib_ctx *ctx, cudaStream_t s, const AttnLaunch &a);
-uint32_t attn_cluster_positions(const AttnLaunch &a);   // positions (pos + 1) up to which `short_context` may be set; 0: never
+uint32_t attn_regime_positions(const ib_ctx *ctx, const AttnLaunch &a, uint32_t regime);   // positions (pos + 1) up to which `regime` may be set; 0: never
 
 }  // namespace ib

@@ -123,18 +123,17 @@ struct ib_llama {
     uint32_t *epoch = nullptr;
     uint32_t *h_pinned = nullptr;  // [4 + seq_cap] staging for control block and token ids
     cudaEvent_t staged = nullptr;  // the last copy out of h_pinned has been issued and finished
-    cudaGraphExec_t graph_exec = nullptr;
-    // the same token for positions below `short_positions`: its attention nodes merge their slices inside thread-block clusters
-    cudaGraphExec_t graph_exec_short = nullptr, graph_exec_sample_short = nullptr;
-    uint32_t short_positions = 0;
-    bool recording_short = false;
+    // [ATTN_LONG], and for the contexts where the attention nodes have another shape [ATTN_SHORT], [ATTN_MIDDLE]: the positions that
+    // `regime_positions` says (0: no such graph)
+    cudaGraphExec_t graph_exec[3] = {}, graph_exec_sample[3] = {};
+    uint32_t regime_positions[3] = {};
+    uint32_t recording_regime = ATTN_LONG;
     cudaStream_t own_stream = nullptr;
     uint64_t launches_per_token = 0;
     // sampling beyond greedy (ib_llama_set_sampler): parameters, scratch, and the graph that carries the sampler node
     float temperature = 0.f, topp = 0.f;
     uint64_t sample_seed = 0;
     float *sample_probs = nullptr;   // only for vocabularies that the sampler cannot hold in shared memory
-    cudaGraphExec_t graph_exec_sample = nullptr;
     uint64_t launches_per_token_sample = 0;
     // prompt prefill (ib_llama_prefill): one allocation for passes of up to `chunks` chunks of PF_CHUNK tokens, made at the
     // first call and again by a call with a longer prompt
@@ -239,8 +238,9 @@ static int32_t record_token(ib_llama *m, cudaStream_t s, uint32_t pdl) {
         AttnLaunch a = {};
         a.p = ap; a.pos_ptr = &m->ctl->pos; a.q = m->q; a.k_cache = m->k_cache[l]; a.v_cache = m->v_cache[l]; a.kv_dtype = m->kv_dtype;
         a.out = m->xb; a.scratch = m->attn_scratch; a.counters = m->attn_counters; a.max_splits = m->attn_splits; a.pdl = pdl;
-        a.short_context = m->recording_short ? 1u : 0u;
-        if (l == 0) m->short_positions = attn_cluster_positions(a);
+        a.regime = m->recording_regime;
+        if (l == 0)
+            for (uint32_t r : {ATTN_SHORT, ATTN_MIDDLE}) m->regime_positions[r] = attn_regime_positions(ctx, a, r);
         if ((rc = emit_attn(a))) return rc;
         // o_proj + residual (transformer.rs:450-453)
         p = GemvParams{};
@@ -384,16 +384,16 @@ void llama_adopt(ib_llama *m, std::vector<ib_qtensor *> &&tensors, std::vector<v
 extern "C" {
 
 static int32_t finish_graph(ib_llama *m);
+static void drop_graphs(cudaGraphExec_t (&exec)[3]);
+static int32_t capture_graphs(ib_llama *m, cudaGraphExec_t (&exec)[3], uint64_t *launches_per_token);
 static int32_t capture_graph(ib_llama *m, cudaGraphExec_t *exec, uint64_t *launches_per_token);
 
 int32_t ib_llama_destroy(ib_llama *m) {
     if (!m) return IB_OK;
     cudaSetDevice(m->ctx->device);
     cudaDeviceSynchronize();
-    if (m->graph_exec) cudaGraphExecDestroy(m->graph_exec);
-    if (m->graph_exec_sample) cudaGraphExecDestroy(m->graph_exec_sample);
-    if (m->graph_exec_short) cudaGraphExecDestroy(m->graph_exec_short);
-    if (m->graph_exec_sample_short) cudaGraphExecDestroy(m->graph_exec_sample_short);
+    drop_graphs(m->graph_exec);
+    drop_graphs(m->graph_exec_sample);
     if (m->sample_probs) cudaFree(m->sample_probs);
     if (m->own_stream) cudaStreamDestroy(m->own_stream);
     if (m->staged) cudaEventDestroy(m->staged);
@@ -580,16 +580,30 @@ int32_t ib_llama_create(ib_ctx *ctx, const ib_llama_config *config, const ib_lla
 // Records the token graph (once every pointer it needs is known) and instantiates it.
 static int32_t finish_graph(ib_llama *m) {
     IB_CHECK_CUDA(cudaDeviceSynchronize());
-    int32_t rc = capture_graph(m, &m->graph_exec, &m->launches_per_token);
-    if (rc != IB_OK || m->short_positions == 0) return rc;
-    // the variant for short contexts (record_token noted up to which position the attention kernel offers it)
-    if (m->graph_exec_short) { cudaGraphExecDestroy(m->graph_exec_short); m->graph_exec_short = nullptr; }
-    uint64_t same = 0;
-    m->recording_short = true;
-    rc = capture_graph(m, &m->graph_exec_short, &same);
-    return rc;
+    return capture_graphs(m, m->graph_exec, &m->launches_per_token);
 }
 
+static void drop_graphs(cudaGraphExec_t (&exec)[3]) {
+    for (cudaGraphExec_t &e : exec) {
+        if (e) cudaGraphExecDestroy(e);
+        e = nullptr;
+    }
+}
+
+// The token's graphs: for long contexts, and for the shorter ones whose attention nodes have another shape (record_token notes up to
+// which position).  All have the same number of nodes.
+static int32_t capture_graphs(ib_llama *m, cudaGraphExec_t (&exec)[3], uint64_t *launches_per_token) {
+    drop_graphs(exec);
+    static_assert(ATTN_LONG == 0, "recorded first: the others' positions are noted then");
+    int32_t rc = IB_OK;
+    for (uint32_t r = 0; r < 3 && rc == IB_OK; r++) {
+        if (r != ATTN_LONG && m->regime_positions[r] == 0) continue;
+        m->recording_regime = r;
+        rc = capture_graph(m, &exec[r], launches_per_token);
+    }
+    m->recording_regime = ATTN_LONG;
+    return rc;
+}
 
 // Records the token's kernels (with the sampler node when a temperature is set) into a graph and instantiates it.
 static int32_t capture_graph(ib_llama *m, cudaGraphExec_t *exec, uint64_t *launches_per_token) {
@@ -599,7 +613,6 @@ static int32_t capture_graph(ib_llama *m, cudaGraphExec_t *exec, uint64_t *launc
     const int32_t rc = record_token(m, m->own_stream, 1);
     cudaGraph_t graph = nullptr;
     cudaError_t ce = cudaStreamEndCapture(m->own_stream, &graph);
-    m->recording_short = false;
     *launches_per_token = ctx->launches - before;
     ctx->launches = before;  // recording is not launching
     if (rc != IB_OK) {
@@ -624,18 +637,11 @@ int32_t ib_llama_set_sampler(ib_llama *m, float temperature, float topp, uint64_
         if (m->tp_size > 1) return set_error(IB_ERR_UNSUPPORTED, "ib_llama_set_sampler: sampling needs the whole vocabulary on one GPU (tensor-parallel models are greedy)");
     }
     IB_CHECK_CUDA(cudaDeviceSynchronize());
-    if (m->graph_exec_sample) { cudaGraphExecDestroy(m->graph_exec_sample); m->graph_exec_sample = nullptr; }
-    if (m->graph_exec_sample_short) { cudaGraphExecDestroy(m->graph_exec_sample_short); m->graph_exec_sample_short = nullptr; }
+    drop_graphs(m->graph_exec_sample);
     m->temperature = temperature; m->topp = topp; m->sample_seed = seed;
     if (temperature == 0.f) return IB_OK;   // greedy: the graph recorded at creation
     if (!m->sample_probs && sample_scratch_bytes(m->cfg.vocab_size)) IB_CHECK_CUDA(cudaMalloc(&m->sample_probs, sample_scratch_bytes(m->cfg.vocab_size)));
-    int32_t rc = capture_graph(m, &m->graph_exec_sample, &m->launches_per_token_sample);
-    if (rc == IB_OK && m->short_positions) {
-        if (m->graph_exec_sample_short) { cudaGraphExecDestroy(m->graph_exec_sample_short); m->graph_exec_sample_short = nullptr; }
-        uint64_t same = 0;
-        m->recording_short = true;
-        rc = capture_graph(m, &m->graph_exec_sample_short, &same);
-    }
+    const int32_t rc = capture_graphs(m, m->graph_exec_sample, &m->launches_per_token_sample);
     if (rc != IB_OK) { m->temperature = 0.f; return rc; }
     return IB_OK;
 }
@@ -695,7 +701,7 @@ int32_t ib_llama_tp_connect_ptrs(ib_llama *m, void *const *areas) {
 }
 
 static int32_t run_tokens(ib_llama *m, cudaStream_t s, const uint32_t *tokens, uint32_t n_prompt, uint32_t start_pos, uint32_t n_steps) {
-    if (!m->graph_exec) return set_error(IB_ERR_COMM, "the tensor-parallel model is not connected yet: call ib_llama_tp_connect on every rank first");
+    if (!m->graph_exec[ATTN_LONG]) return set_error(IB_ERR_COMM, "the tensor-parallel model is not connected yet: call ib_llama_tp_connect on every rank first");
     // control block + given tokens in one pinned staging buffer -> two small async copies
     uint32_t *h = m->h_pinned;
     IB_CHECK_CUDA(cudaEventSynchronize(m->staged));  // an earlier call's copies out of the staging buffer are done
@@ -704,12 +710,12 @@ static int32_t run_tokens(ib_llama *m, cudaStream_t s, const uint32_t *tokens, u
     IB_CHECK_CUDA(cudaMemcpyAsync(m->ctl, h, sizeof(TokenCtl), cudaMemcpyHostToDevice, s));
     IB_CHECK_CUDA(cudaMemcpyAsync(m->seq, h + 4, sizeof(uint32_t) * n_prompt, cudaMemcpyHostToDevice, s));
     IB_CHECK_CUDA(cudaEventRecord(m->staged, s));
-    const bool sampled = m->temperature > 0.f && m->graph_exec_sample;
+    const bool sampled = m->temperature > 0.f && m->graph_exec_sample[ATTN_LONG];
     for (uint32_t i = 0; i < n_steps; i++) {
-        // positions below short_positions replay the graph whose attention nodes merge inside thread-block clusters
-        const bool shrt = (uint64_t)start_pos + i + 1 <= m->short_positions;
-        cudaGraphExec_t exec = sampled ? (shrt && m->graph_exec_sample_short ? m->graph_exec_sample_short : m->graph_exec_sample)
-                                       : (shrt && m->graph_exec_short ? m->graph_exec_short : m->graph_exec);
+        // the graph whose attention nodes have the shape for this many positions
+        const uint64_t positions = (uint64_t)start_pos + i + 1;
+        const uint32_t regime = positions <= m->regime_positions[ATTN_SHORT] ? ATTN_SHORT : (positions <= m->regime_positions[ATTN_MIDDLE] ? ATTN_MIDDLE : ATTN_LONG);
+        cudaGraphExec_t exec = sampled ? m->graph_exec_sample[regime] : m->graph_exec[regime];
         IB_CHECK_CUDA(cudaGraphLaunch(exec, s));
         m->ctx->launches += sampled ? m->launches_per_token_sample : m->launches_per_token;
     }

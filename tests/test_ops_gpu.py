@@ -104,6 +104,16 @@ def test_attention(backend, kv_dtype, hs, n_heads, kv_mul, pos, seq):
         assert_close(out.cpu().numpy(), ref, what=f"attention hs={hs} pos={pos}")
 
 
+# both sides of the context lengths where a kv head's slices change shape (8 CTAs of 64 positions; 2048 or 384 each), the first one with
+# a single row in the last slice; and few and many kv heads
+@pytest.mark.parametrize("hs,n_kv,total", [
+    (64, 8, 512), (64, 8, 513), (64, 8, 1025), (64, 8, 16384), (64, 8, 16385), (64, 1, 900), (64, 3, 5000), (64, 20, 600),
+    (128, 8, 512), (128, 8, 513), (128, 8, 3072), (128, 8, 3073), (128, 2, 1000), (128, 12, 700),
+])
+def test_attention_slice_shapes(backend, hs, n_kv, total):
+    test_attention(backend, np.float16, hs, 4 * n_kv, 4, total - 1, total + 3)
+
+
 @pytest.mark.parametrize("ctx_len", [8192, 16384, 32768])
 def test_long_context_attention(backend, ctx_len):
     """Long-context stress: 32 query / 8 kv heads of 128, f16 cache from N(0,1), RoPE on q and on every k row."""
