@@ -479,7 +479,7 @@ def main():
                    "frac_of_bf16_sustained_peak": round(flops / (p_ms * 1e-3) / 1e12 / 1385.0, 4),
                    "weight_stream_bound_ms": round(cfg.weight_bytes() / (peak_hbm() * 1e9) * 1e3, 3),
                    "decode_path_ms_for_the_same_prompt": round(128 * ms / K, 1), "next_token_matches_decode_path": bool(nxt_p == loop_first),
-                   "note": "Q4_K / Q5_K: exact integer weights (scale x quant) in f16 x inputs split hi / lo, 2 tcgen05.mma per 16 columns, per-block f32 scaling from tensor memory; Q6_K: weights and inputs split hi / lo, 3 tcgen05.mma per 16 columns; flops counted once (2 x matrix parameters x tokens, classifier excluded)"}
+                   "note": "exact integer weights (scale x quant) in f16 x inputs split hi / lo, 2 tcgen05.mma per 16 columns, per-block f32 scaling from tensor memory; flops counted once (2 x matrix parameters x tokens, classifier excluded)"}
 
     # ---- roofline --------------------------------------------------------------------------------------------
     peak1, peak_src = measured_peaks()
@@ -508,7 +508,7 @@ def main():
 
     line = {
         "metric": METRIC, "value": tok_s, "unit": UNIT, "n_gpus": world, "steps": K, "warmup": W, "ms_per_step": ms / K,
-        "higher_is_better": True, "scaling": "strong", "vs_baseline": None, "dtype": "int8 dp4a weights x 2-limb int8 activations (16-bit block fixed point), f32 accumulate",
+        "higher_is_better": True, "scaling": "strong", "vs_baseline": None, "dtype": "integer mma: quantized weights x 2-limb int8 activations (16-bit block fixed point), f32 accumulate",
         "data": "synthetic",
         "config": {"workload": workload_name(cfg), "parallelism": f"tp{world}" if world > 1 else "single GPU", "prompt_tokens": W, "decode_tokens": K, "l2": "weights per token (4.9 GB) exceed L2 (126 MB)",
                    "prefill": "prompt fed through the decode path (as the reference does), untimed"},
