@@ -18,7 +18,7 @@ from ._lib import AttnParams, InferiError, KV_F16, KV_F32, ROPE_NEOX, ROPE_ORIGI
 from .quant import BLOCK_BYTES, BLOCK_ELEMS, F32, NAMES, Q4_K, Q5_K, Q6_K, Q8_0, row_bytes  # noqa: F401
 
 
-_f32, _tensor = torch.float32, torch.Tensor
+_f16, _f32, _tensor = torch.float16, torch.float32, torch.Tensor
 _current_device, _raw_stream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
 
 
@@ -33,6 +33,10 @@ def _f32_dev(t: torch.Tensor, name: str) -> int:
     if isinstance(t, _tensor) and t.dtype is _f32 and t.is_cuda and t.is_contiguous():
         return t.data_ptr()
     raise InferiError(1, f"{name}: expected a contiguous float32 CUDA tensor")
+
+
+# The launches below take their tensors' addresses first: with a CUDA tensor among them CUDA is initialised, and the stream can be
+# read without asking (these calls are a few microseconds each, most of it the launch itself).
 
 
 class Backend:
@@ -118,7 +122,10 @@ class GemvQuant:
         """out[rows] = m . v[cols] on the current stream (asynchronous, like recording into a pass)."""
         if v.numel() != m.cols or out.numel() != m.rows:
             raise InferiError(1, f"gemv: matrix is {m.rows}x{m.cols} but v has {v.numel()} and out {out.numel()} elements")
-        check(self.backend.lib.ib_gemv_quant(self.backend.handle, _stream_ptr(), _f32_dev(out, "out"), m.handle, _f32_dev(v, "v")))
+        b, out_ptr, v_ptr = self.backend, _f32_dev(out, "out"), _f32_dev(v, "v")
+        rc = b.lib.ib_gemv_quant(b.handle, _raw_stream(_current_device()), out_ptr, m.handle, v_ptr)
+        if rc:
+            check(rc)
 
     def launch_host(self, m: GpuQuantTensor, v: np.ndarray) -> np.ndarray:
         """The same op for host buffers: copy in, run, copy out, synchronise."""
@@ -177,8 +184,10 @@ class RmsNorm:
         n = value.numel()
         if result.numel() != n or weight.numel() != n:
             raise InferiError(1, "rms_norm: result, value and weight must have the same length")
-        check(self.backend.lib.ib_rms_norm(self.backend.handle, _stream_ptr(), _f32_dev(result, "result"), _f32_dev(value, "value"),
-                                           _f32_dev(weight, "weight"), n, config.nudge_factor))
+        b, r, v, w = self.backend, _f32_dev(result, "result"), _f32_dev(value, "value"), _f32_dev(weight, "weight")
+        rc = b.lib.ib_rms_norm(b.handle, _raw_stream(_current_device()), r, v, w, n, config.nudge_factor)
+        if rc:
+            check(rc)
 
 
 @dataclass
@@ -201,8 +210,10 @@ class RoPE:
     def launch(self, variant: int, config: RoPEConfig, in_out_q: torch.Tensor, in_out_k: torch.Tensor) -> None:
         if in_out_k.numel() < config.kv_dim:
             raise InferiError(1, "rope: k is shorter than kv_dim")
-        check(self.backend.lib.ib_rope(self.backend.handle, _stream_ptr(), variant, _f32_dev(in_out_q, "q"), in_out_q.numel(),
-                                       _f32_dev(in_out_k, "k"), config.kv_dim, config.head_size, config.pos, config.base_freq))
+        b, q, k = self.backend, _f32_dev(in_out_q, "q"), _f32_dev(in_out_k, "k")
+        rc = b.lib.ib_rope(b.handle, _raw_stream(_current_device()), variant, q, in_out_q.numel(), k, config.kv_dim, config.head_size, config.pos, config.base_freq)
+        if rc:
+            check(rc)
 
 
 class Silu:
@@ -214,9 +225,13 @@ class Silu:
     from_backend = classmethod(lambda cls, backend: cls(backend))
 
     def launch(self, in_out_h1: torch.Tensor, in_h2: torch.Tensor) -> None:
-        if in_out_h1.numel() != in_h2.numel():
+        n = in_out_h1.numel()
+        if n != in_h2.numel():
             raise InferiError(1, "silu: h1 and h2 must have the same length")
-        check(self.backend.lib.ib_silu_mul(self.backend.handle, _stream_ptr(), _f32_dev(in_out_h1, "h1"), _f32_dev(in_h2, "h2"), in_out_h1.numel()))
+        b, h1, h2 = self.backend, _f32_dev(in_out_h1, "h1"), _f32_dev(in_h2, "h2")
+        rc = b.lib.ib_silu_mul(b.handle, _raw_stream(_current_device()), h1, h2, n)
+        if rc:
+            check(rc)
 
 
 class FusedAttention:
@@ -229,23 +244,32 @@ class FusedAttention:
 
     def launch(self, params: AttnParams, q: torch.Tensor, key_cache: torch.Tensor, value_cache: torch.Tensor, xb: torch.Tensor) -> None:
         """key_cache / value_cache: [seq_len, kv_dim] float32 or float16 CUDA tensors."""
-        if key_cache.dtype != value_cache.dtype or key_cache.dtype not in (torch.float16, torch.float32):
+        dtype = key_cache.dtype
+        if dtype is not value_cache.dtype or (dtype is not _f16 and dtype is not _f32):
             raise InferiError(1, "attention: the caches must both be float16 or both float32")
+        need = params.seq_len * params.kv_dim
         for t, name in ((key_cache, "key_cache"), (value_cache, "value_cache")):
-            if not (t.is_cuda and t.is_contiguous() and t.numel() >= params.seq_len * params.kv_dim):
+            if not (t.is_cuda and t.is_contiguous() and t.numel() >= need):
                 raise InferiError(1, f"attention: {name} must be a contiguous CUDA tensor of at least seq_len*kv_dim elements")
-        if q.numel() != params.n_heads * params.head_size or xb.numel() != q.numel():
+        n = params.n_heads * params.head_size
+        if q.numel() != n or xb.numel() != n:
             raise InferiError(1, "attention: q and xb must hold n_heads*head_size elements")
-        kv = KV_F16 if key_cache.dtype == torch.float16 else KV_F32
-        check(self.backend.lib.ib_attention(self.backend.handle, _stream_ptr(), C.byref(params), _f32_dev(q, "q"), key_cache.data_ptr(),
-                                            value_cache.data_ptr(), kv, _f32_dev(xb, "xb")))
+        b, q_ptr, xb_ptr = self.backend, _f32_dev(q, "q"), _f32_dev(xb, "xb")
+        rc = b.lib.ib_attention(b.handle, _raw_stream(_current_device()), C.byref(params), q_ptr, key_cache.data_ptr(), value_cache.data_ptr(),
+                                KV_F16 if dtype is _f16 else KV_F32, xb_ptr)
+        if rc:
+            check(rc)
 
 
 def add_assign(backend: Backend, a: torch.Tensor, b: torch.Tensor) -> None:
     """≙ `LlmContext::add_assign` (crates/inferi/src/context.rs:516-530): a += b."""
-    if a.numel() != b.numel():
+    n = a.numel()
+    if n != b.numel():
         raise InferiError(1, "add_assign: length mismatch")
-    check(backend.lib.ib_add_assign(backend.handle, _stream_ptr(), _f32_dev(a, "a"), _f32_dev(b, "b"), a.numel()))
+    a_ptr, b_ptr = _f32_dev(a, "a"), _f32_dev(b, "b")
+    rc = backend.lib.ib_add_assign(backend.handle, _raw_stream(_current_device()), a_ptr, b_ptr, n)
+    if rc:
+        check(rc)
 
 
 def argmax(backend: Backend, logits: torch.Tensor, out: torch.Tensor) -> None:
