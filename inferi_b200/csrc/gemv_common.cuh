@@ -91,13 +91,20 @@ __device__ __forceinline__ void pack_four(const float (&e)[4], float inv, uint32
     s1 = dp4a_ss(w1, 0x01010101u, s1);
 }
 
+// The larger of two, or NaN where one of them is: a NaN among a group's columns has to reach the group's scale, because the limbs
+// cannot carry one (fmaxf drops it, and a row's sum then comes out finite).
+__device__ __forceinline__ float max_nan(float a, float b) {
+    float r;
+    asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float abs_max(const float4 &v) { return max_nan(max_nan(fabsf(v.x), fabsf(v.y)), max_nan(fabsf(v.z), fabsf(v.w))); }
+
 __device__ __forceinline__ void pack_run(const float4 (&v)[4], uint32_t run, uint32_t cols, uint8_t *smem, bool store) {
     const int lane = threadIdx.x & 31;
-    float amax = 0.f;
     int s0 = 0, s1 = 0;
-#pragma unroll
-    for (int j = 0; j < 4; j++) amax = fmaxf(amax, fmaxf(fmaxf(fabsf(v[j].x), fabsf(v[j].y)), fmaxf(fabsf(v[j].z), fabsf(v[j].w))));
-    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));   // the other half of the 32-column group
+    float amax = max_nan(max_nan(abs_max(v[0]), abs_max(v[1])), max_nan(abs_max(v[2]), abs_max(v[3])));
+    amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 1));   // the other half of the 32-column group
     const float inv = amax > 0.f ? __fdividef(ACT_STEPS, amax) : 0.f;   // 2 ulp: the limbs absorb it (the largest |x| still rounds to 32512)
     uint32_t w0[4], w1[4];
 #pragma unroll

@@ -645,10 +645,9 @@ __device__ __forceinline__ void pack_stream(uint8_t *smem, uint32_t cols, const 
                 v[j].x *= w.x; v[j].y *= w.y; v[j].z *= w.z; v[j].w *= w.w;
             }
         }
-        float amax = fmaxf(fmaxf(fmaxf(fabsf(v[0].x), fabsf(v[0].y)), fmaxf(fabsf(v[0].z), fabsf(v[0].w))),
-                           fmaxf(fmaxf(fabsf(v[1].x), fabsf(v[1].y)), fmaxf(fabsf(v[1].z), fabsf(v[1].w))));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-        amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+        float amax = max_nan(abs_max(v[0]), abs_max(v[1]));
+        amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
+        amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
         const float inv = amax > 0.f ? __fdividef(ACT_STEPS, amax) : 0.f;   // 2 ulp: the limbs absorb it (the largest |x| still rounds to 32512)
         uint32_t w0[2], w1[2];
         int s0 = 0, s1 = 0;

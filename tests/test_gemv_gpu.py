@@ -134,3 +134,24 @@ def test_contract_violations_are_errors(backend):
         GemvQuant(backend).launch(torch.zeros(8, device="cuda"), m, torch.zeros(128, device="cuda"))
     with pytest.raises(InferiError):           # host tensor where a device tensor is required
         GemvQuant(backend).launch(torch.zeros(8), m, torch.zeros(256, device="cuda"))
+
+
+@pytest.mark.parametrize("bad", [float("nan"), float("inf"), float("-inf")])
+@pytest.mark.parametrize("qt,rows,cols", [(quant.Q8_0, 64, 2048), (quant.Q4_K, 64, 2304), (quant.Q5_K, 64, 8448), (quant.Q6_K, 64, 2048), (quant.Q4_K, 8, 16640)])
+def test_a_column_that_is_no_number_reaches_every_row(backend, qt, rows, cols, bad):
+    """Every row of an f32 product with such a column is NaN or infinite; so is the fixed-point one (streaming kernel, and the
+    wider rows' kernel).  The gate/up launch, which multiplies two such products, too."""
+    blocks = quant.random_blocks(qt, rows, cols, seed=cols + qt)
+    for at in (0, 37, cols - 1):
+        v = np.random.default_rng(at).standard_normal(cols).astype(np.float32)
+        v[at] = bad
+        got = run_gemv(backend, qt, rows, cols, blocks, v)
+        assert not np.isfinite(got).any()
+        if np.isnan(bad):
+            assert np.isnan(got).all()
+    m = GpuQuantTensor(backend, qt, rows, cols, blocks)
+    out = torch.zeros(rows, device="cuda")
+    v[cols - 1] = float("nan")
+    FfnGateUp(backend).launch(out, m, m, torch.from_numpy(v).cuda())
+    assert torch.isnan(out).all()
+    m.close()
