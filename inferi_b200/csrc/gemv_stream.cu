@@ -294,7 +294,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const Ge
         // hundreds of megabytes: 13.5 us instead of 5).
         const uint64_t policy = evict_first_policy();
         uint32_t st = pipe, ring = smem_u32(smem), par = 1, ends = 0;   // par: parity of the slot's previous use ("1" before the first one); ends: end markers, one per stream
-        bool first_round = true;
+        bool first_round = true, gave_up = false;
         for (;;) {
             uint4 tm = make_uint4(0, 0, 0, 0);
             if (dyn) {
@@ -308,8 +308,10 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const Ge
             // Slot free?  In the first round every slot is; there the copies in flight are kept to what the memory system's latency
             // needs: a ring-full of them would only queue up, and the input vector's few kilobytes behind them.
             if (!first_round ? !mbar_wait(bar0 + 8 * (S + st), par, p.err, 2, p.wait_ns)
-                             : (st >= geo.ahead && !mbar_wait(bar0 + 8 * (st - geo.ahead), 0, p.err, 1, p.wait_ns)))
-                return;
+                             : (st >= geo.ahead && !mbar_wait(bar0 + 8 * (st - geo.ahead), 0, p.err, 1, p.wait_ns))) {
+                gave_up = true;
+                break;
+            }
             meta[st] = tm;
             if (n == 0) {
                 // no tiles left: tell the others, and let the last pipeline to get here clear the counters for their next use
@@ -336,6 +338,13 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const Ge
                 first_round = false;
             }
         }
+        if (gave_up) {
+            // The copies in flight write into this CTA's shared memory: let them land (bounded, like every wait) before the CTA can end.
+            // A stage's last announcement is this round's up to `st` and the previous round's from there on.
+            for (uint32_t s = pipe; s < S && (s < st || !first_round); s += geo.P) mbar_wait(bar0 + 8 * s, s < st ? par ^ 1u : par, nullptr, 1, p.wait_ns);
+        }
+        // Every pipeline gets here, one that gave up too: a launch that ended early must not leave counts behind for the next one that
+        // is given these counters.
         if (dyn && atomicAdd(p.tile_claim + 1, 1u) == pipes - 1) {
             p.tile_claim[0] = 0u;
             p.tile_claim[1] = 0u;

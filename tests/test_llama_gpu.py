@@ -207,6 +207,43 @@ def test_bounded_wait_expires_when_a_rank_never_arrives(backend):
     be.close()   # every tensor and model of this context is gone by now
 
 
+def test_a_wait_that_gave_up_leaves_no_counts_for_later_launches():
+    """The same missing peer, with a classifier whose tiles are handed out through a counter (1024 tiles of 36 KB): its launch ends
+    early, in the middle of the hand-out.  Launches of that kind take one of sixteen counter pairs in turn, so the pair of the launch
+    that gave up comes up again within sixteen: every row of every one of them has to be there."""
+    from inferi_b200 import tp
+    from inferi_b200.ops import Backend, GemvQuant
+    be = Backend(0)
+    be.set_wait_limit(3_000_000)
+    cfg = Llama2Config(2048, 2048, 1, 32, 8, 65536, 32, 500000.0, 1e-5)
+    recipe = {k: quant.Q4_K for k in ("attn_q", "attn_k", "attn_v", "attn_output", "ffn_gate", "ffn_up", "ffn_down", "token_embd", "output")}
+    mine = tp.shard_weights(cfg, synth_weights(cfg, seed=12, recipe=recipe, device="cuda"), 0, 2)
+    dev_w = Llama2Weights(be, cfg, mine, shapes=tp.shard_shapes(cfg, 2, quant.Q4_K))
+    model = Llama2(be, cfg, dev_w, kv_f16=True, tp_rank=0, tp_size=2, connect=False)
+    ghost = torch.zeros(model.tp_area()[1], dtype=torch.uint8, device="cuda")
+    model.connect_areas([None, ghost.data_ptr()])
+    for _ in range(2):
+        with pytest.raises(InferiError) as e:
+            model.forward(5, 0)
+        assert e.value.code == 5
+    torch.cuda.synchronize()
+    model.close()
+    dev_w.close()
+    be.set_wait_limit(2_000_000_000)
+    rows, cols = 32768, 2048
+    blocks = mine["output"][1].cpu().numpy()
+    v = np.random.default_rng(13).standard_normal(cols).astype(np.float32)
+    m = GpuQuantTensor(be, quant.Q4_K, rows, cols, blocks)
+    outs = torch.full((40, rows), float("nan"), device="cuda")
+    for out in outs:
+        GemvQuant(be).launch(out, m, torch.from_numpy(v).cuda())
+    torch.cuda.synchronize()
+    ref = torch.from_numpy(np.asarray(oracle.gemv_ref(quant.Q4_K, rows, cols, blocks, v))).cuda()
+    assert (outs - ref).abs().max() <= 1e-3 * ref.abs().max()
+    m.close()
+    be.close()
+
+
 def test_logits_across_the_position_where_the_token_graph_changes(backend):
     """Below position 320 the model replays a token graph whose attention nodes merge their slices inside thread-block
     clusters, from there on the one that merges through global memory: the logits on both sides of the change must agree
