@@ -225,7 +225,16 @@ extern "C" int32_t ib_gemm_quant(ib_ctx *ctx, void *stream, float *out_dev, cons
     IB_REQUIRE(ctx && m && out_dev && x_dev, "ib_gemm_quant: null argument");
     IB_REQUIRE(m->ctx->device == ctx->device, "ib_gemm_quant: tensor lives on device %d, context on %d", m->ctx->device, ctx->device);
     IB_REQUIRE(n >= 1, "ib_gemm_quant: no rows");
-    if (!prefill_gemm_eligible(m))
+    // Q6_K and Q8_0 matrices whose rows are not in the re-tiled layout (Q6_K rows that are no multiple of 8 blocks, rows wider than the
+    // GEMV takes): re-tiled into the scratch by every call, one read and one write of the matrix ahead of a GEMM that reads it at least once more
+    ib_qtensor tiled = *m;
+    const bool retile = m->layout == LAYOUT_GGUF && (m->qtype == IB_Q6_K || m->qtype == IB_Q8_0) && m->cols % 256 == 0;
+    if (retile) {
+        tiled.layout = LAYOUT_SOA;
+        tiled.row_bytes = soa_row_bytes(m->qtype, m->nb);
+        tiled.dev = nullptr;
+    }
+    if (!prefill_gemm_eligible(&tiled))
         return set_error(IB_ERR_UNSUPPORTED, "ib_gemm_quant: %llux%llu of type %d (the tensor-core path takes Q8_0/Q4_K/Q5_K/Q6_K with rows %% 128 == 0 and cols %% 256 == 0)",
                          (unsigned long long)m->rows, (unsigned long long)m->cols, m->qtype);
     int prev = -1;
@@ -238,7 +247,7 @@ extern "C" int32_t ib_gemm_quant(ib_ctx *ctx, void *stream, float *out_dev, cons
     auto bytes_of = [&](uint32_t nc, size_t &half_bytes) {
         const StreamK sk = prefill_streamk(ctx, rows, cols, nc);
         half_bytes = (nc + PF_CHUNK - 1) / PF_CHUNK * pf_x_halves(cols) * sizeof(__half);
-        return 2 * half_bytes + (size_t)(prefill_max_pieces(sk) - 1) * nc * rows * sizeof(float);
+        return 2 * half_bytes + (((size_t)(prefill_max_pieces(sk) - 1) * nc * rows * sizeof(float) + 255) & ~(size_t)255);
     };
     size_t half_bytes = 0, need = bytes_of(pass, half_bytes);
     while (pass > PF_CHUNK && need > ((size_t)512 << 20)) {
@@ -250,6 +259,8 @@ extern "C" int32_t ib_gemm_quant(ib_ctx *ctx, void *stream, float *out_dev, cons
         const size_t last = bytes_of(n % pass, hb) - 2 * hb + 2 * half_bytes;
         if (last > need) need = last;
     }
+    const size_t tiled_at = need;
+    if (retile) need += m->rows * tiled.row_bytes;
     int32_t rc = IB_OK;
     if (need > ctx->tc_scratch_bytes) {
         // growing the scratch: wait for work that may still use the old one
@@ -263,12 +274,17 @@ extern "C" int32_t ib_gemm_quant(ib_ctx *ctx, void *stream, float *out_dev, cons
     }
     __half *hi = reinterpret_cast<__half *>(ctx->tc_scratch), *lo = reinterpret_cast<__half *>((uint8_t *)ctx->tc_scratch + half_bytes);
     float *planes = reinterpret_cast<float *>((uint8_t *)ctx->tc_scratch + 2 * half_bytes);
+    if (retile && rc == IB_OK) {
+        tiled.dev = (uint8_t *)ctx->tc_scratch + tiled_at;
+        rc = retile_to_soa(ctx, s, m->qtype, m->dev, tiled.dev, m->rows, m->nb);
+    }
+    const ib_qtensor *w = &tiled;
     for (uint32_t t0 = 0; rc == IB_OK && t0 < n; t0 += pass) {
         const uint32_t nc = n - t0 < pass ? n - t0 : pass;
         const StreamK sk = prefill_streamk(ctx, rows, cols, nc);
         float *out = out_dev + (size_t)t0 * rows;   // plane 0 of every tile
         rc = launch_prefill_norm_split(ctx, s, const_cast<float *>(x_dev) + (size_t)t0 * cols, nullptr, nullptr, 0.f, nc, cols, hi, lo);
-        if (rc == IB_OK) rc = launch_prefill_gemm(ctx, s, &m, 1, hi, lo, nc, out, planes, sk);
+        if (rc == IB_OK) rc = launch_prefill_gemm(ctx, s, &w, 1, hi, lo, nc, out, planes, sk, !retile);
         if (rc == IB_OK && prefill_max_pieces(sk) > 1) rc = launch_prefill_finish(ctx, s, out, PfPlanes{out, planes, sk, rows, (nc + PF_CHUNK - 1) / PF_CHUNK, nc});
     }
     if (prev >= 0 && prev != ctx->device) cudaSetDevice(prev);

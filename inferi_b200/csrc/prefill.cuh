@@ -55,9 +55,9 @@ __host__ __device__ inline size_t pf_x_halves(uint32_t cols) { return (size_t)(P
 
 bool prefill_gemm_eligible(const ib_qtensor *m);
 // plane0 / planes = partial sums of W x_t over the K ranges of the tile's CTAs; x_hi / x_lo: the layout above, token rows n .. (n rounded
-// up to 16) - 1 of the last chunk zero.  The matrices of a launch have the same type and width; their rows follow one another.
+// up to 16) - 1 of the last chunk zero; early: the weights may be read before the stream's previous kernels are done.  The matrices of a launch have the same type and width; their rows follow one another.
 int32_t launch_prefill_gemm(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *const *mats, uint32_t n_mats, const __half *x_hi, const __half *x_lo, uint32_t n, float *plane0,
-                            float *planes, const StreamK &sk);
+                            float *planes, const StreamK &sk, bool early = true);
 
 // One GEMM launch's result, as the element-wise kernels read it
 struct PfPlanes {

@@ -688,7 +688,7 @@ static int32_t pg_encode(const ib_qtensor *m, int fmt, CUtensorMap *maps) {
 }
 
 template <int FMT>
-static int32_t pg_launch(ib_ctx *ctx, cudaStream_t s, PgParams &p, const PgMaps &maps) {
+static int32_t pg_launch(ib_ctx *ctx, cudaStream_t s, PgParams &p, const PgMaps &maps, bool early) {
     static bool attr_set[16] = {};
     constexpr uint32_t room = PG_SMEM_LIMIT - pg_fixed_smem(FMT);
     static_assert(room >= 3 * 2 * PF_CHUNK * 128, "shared memory");
@@ -708,14 +708,14 @@ static int32_t pg_launch(ib_ctx *ctx, cudaStream_t s, PgParams &p, const PgMaps 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = early ? 1 : 0;
     IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, prefill_gemm_kernel<FMT>, p, maps));
     ctx->launches++;
     return IB_OK;
 }
 
 int32_t launch_prefill_gemm(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *const *mats, uint32_t n_mats, const __half *x_hi, const __half *x_lo, uint32_t n, float *plane0,
-                            float *planes, const StreamK &sk) {
+                            float *planes, const StreamK &sk, bool early) {
     IB_REQUIRE(n_mats >= 1 && n_mats <= PF_MAX_SEGS, "prefill GEMM: %u matrices", n_mats);
     IB_REQUIRE(sk.total < (1u << 24), "prefill GEMM: %u units of work are too many for one launch", sk.total);
     IB_REQUIRE(((uintptr_t)x_hi % 16) == 0 && ((uintptr_t)x_lo % 16) == 0, "prefill GEMM: the input tiles must be 16-byte aligned for the bulk copies");
@@ -736,10 +736,10 @@ int32_t launch_prefill_gemm(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *const
     p.n = n; p.chunks = (n + PF_CHUNK - 1) / PF_CHUNK; p.x_hi = x_hi; p.x_lo = x_lo; p.x_chunk = pf_x_halves((uint32_t)mats[0]->cols);
     p.plane0 = plane0; p.planes = planes; p.sk = sk; p.err = ctx->err_dev; p.wait_ns = ctx->wait_limit_ns;
     switch (fmt) {
-    case PG_Q4K: return pg_launch<PG_Q4K>(ctx, s, p, maps);
-    case PG_Q5K: return pg_launch<PG_Q5K>(ctx, s, p, maps);
-    case PG_Q6K: return pg_launch<PG_Q6K>(ctx, s, p, maps);
-    case PG_Q80: return pg_launch<PG_Q80>(ctx, s, p, maps);
+    case PG_Q4K: return pg_launch<PG_Q4K>(ctx, s, p, maps, early);
+    case PG_Q5K: return pg_launch<PG_Q5K>(ctx, s, p, maps, early);
+    case PG_Q6K: return pg_launch<PG_Q6K>(ctx, s, p, maps, early);
+    case PG_Q80: return pg_launch<PG_Q80>(ctx, s, p, maps, early);
     default: return set_error(IB_ERR_UNSUPPORTED, "prefill GEMM: a matrix of type %d", mats[0]->qtype);
     }
 }

@@ -53,6 +53,25 @@ def test_gemm_across_chunks_of_tokens(backend, qt, rows, cols, n):
     m.close()
 
 
+@pytest.mark.parametrize("qt,rows,cols,n", [
+    (quant.Q6_K, 128, 256, 3), (quant.Q6_K, 256, 768, 130), (quant.Q6_K, 1280, 3072, 17), (quant.Q6_K, 128, 11008, 5), (quant.Q6_K, 128, 34816, 2),
+    (quant.Q8_0, 128, 33024, 9),
+])
+def test_gemm_takes_rows_that_no_gemv_layout_holds(backend, qt, rows, cols, n):
+    """Q6_K rows that are no multiple of 8 blocks, and rows wider than the GEMV takes: twice, as the second call finds the first one's
+    scratch, with another matrix in between."""
+    x = torch.from_numpy(np.random.default_rng(n).standard_normal((n, cols)).astype(np.float32)).cuda()
+    for seed in (1, 2, 1):
+        blocks = quant.random_blocks(qt, rows, cols, seed=rows + cols + seed, scale=0.05)
+        m = GpuQuantTensor(backend, qt, rows, cols, blocks)
+        out = torch.full((n, rows), float("nan"), device="cuda")
+        GemmQuant(backend).launch(out, m, x)
+        w = torch.from_numpy(np.stack([oracle.dequantize(qt, blocks[r], cols) for r in range(rows)])).cuda().double()
+        want = x.double() @ w.T
+        assert float((out.double() - want).norm() / want.norm()) < 1e-5      # as above
+        m.close()
+
+
 def test_gemm_rejects_shapes_outside_the_tensor_core_path(backend):
     blocks = quant.random_blocks(quant.Q4_K, 64, 256, seed=1)
     m = GpuQuantTensor(backend, quant.Q4_K, 64, 256, blocks)     # 64 rows: not a multiple of 128
