@@ -120,6 +120,11 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
     __shared__ __align__(16) float sm_alpha[W][4];
     __shared__ uint32_t sm_last;
 
+    namespace cg = cooperative_groups;
+    cg::cluster_group cluster = cg::this_cluster();
+    // Another CTA's shared memory may be written only once that CTA has started: everyone arrives here, and waits ahead of the first
+    // remote store (or of leaving), behind the rows.
+    if constexpr (CLUSTER) cluster.barrier_arrive();
     if (a.pdl) asm volatile("griddepcontrol.launch_dependents;");
     const bool early = a.pdl == 1;   // rows may be requested ahead of the wait
     if (a.pdl == 2) asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -129,7 +134,10 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
     uint32_t nsplit, per;
     gqa4_plan(total, a.max_splits, CLUSTER ? a.cluster : 0u, W, nsplit, per);
     if (split >= nsplit) {
-        if (CLUSTER && nsplit > 1) cooperative_groups::this_cluster().sync();   // the barrier of the working CTAs below
+        if constexpr (CLUSTER) {
+            cluster.barrier_wait();
+            if (nsplit > 1) cluster.sync();   // the barrier of the working CTAs below
+        }
         return;
     }
     const uint32_t t0 = split * per, t1 = min(total, t0 + per);
@@ -309,12 +317,12 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
         }
         if (nsplit == 1) {
             if (has) store_scaled(out, o, 1.0f / ls);
+            if constexpr (CLUSTER) cluster.barrier_wait();
             return;
         }
         if constexpr (CLUSTER) {
             // the partial goes into the first CTA's shared memory; after the cluster barrier that CTA merges the slices
-            namespace cg = cooperative_groups;
-            cg::cluster_group cluster = cg::this_cluster();
+            cluster.barrier_wait();
             if (has) {
                 float *dst = cluster.map_shared_rank(sm_cl, 0) + ((size_t)split * KVM + m_out) * slot;
                 store_scaled(dst + d_out, o, 1.0f);

@@ -114,6 +114,31 @@ def test_attention_slice_shapes(backend, hs, n_kv, total):
     test_attention(backend, np.float16, hs, 4 * n_kv, 4, total - 1, total + 3)
 
 
+@pytest.mark.parametrize("hs,n_kv,total", [(64, 8, 33), (64, 8, 500), (64, 3, 1500), (128, 8, 70), (128, 8, 400), (128, 4, 2000)])
+def test_attention_clusters_whose_ctas_start_apart(backend, hs, n_kv, total):
+    """A kv head's slices merge in the shared memory of their cluster's first CTA.  Products on another stream take SMs away at
+    changing moments, so that the CTAs of a cluster start at different times: every launch gives the same bits."""
+    g = torch.Generator(device="cuda")
+    g.manual_seed(total)
+    kc, vc = (torch.randn(total, n_kv * hs, device="cuda", generator=g).half() for _ in range(2))
+    q = torch.randn(4 * n_kv * hs, device="cuda", generator=g)
+    outs = torch.zeros(60, 4 * n_kv * hs, device="cuda")
+    p, op = AttnParams(total, n_kv * hs, 4, 4 * n_kv, hs, total - 1), FusedAttention(backend)
+    op.launch(p, q, kc, vc, outs[0])
+    a = torch.randn(1024, 1024, device="cuda", generator=g)
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    for i in range(1, 60):
+        with torch.cuda.stream(side):
+            torch.mm(a[: 64 + 16 * i], a)
+        op.launch(p, q, kc, vc, outs[i])
+    torch.cuda.synchronize()
+    assert torch.equal(outs, outs[0].expand_as(outs))
+    Q, K, V = q.double().view(n_kv, 4, hs), kc.double().view(total, n_kv, hs), vc.double().view(total, n_kv, hs)
+    want = torch.einsum("gmt,tgh->gmh", torch.softmax(torch.einsum("gmh,tgh->gmt", Q, K) / hs**0.5, -1), V).reshape(-1)
+    assert_close(outs[0].cpu().numpy(), want.cpu().numpy(), what=f"attention hs={hs} n_kv={n_kv} total={total}")
+
+
 @pytest.mark.parametrize("ctx_len", [8192, 16384, 32768])
 def test_long_context_attention(backend, ctx_len):
     """Long-context stress: 32 query / 8 kv heads of 128, f16 cache from N(0,1), RoPE on q and on every k row."""
