@@ -88,7 +88,9 @@ IB_API int32_t ib_qtensor_info(const ib_qtensor *qt, int32_t *qtype, uint64_t *r
 
 /* Replaces `GemvQuant::launch` (crates/inferi/src/ops/gemv_quant.rs:183-341): out[rows] = W . v[cols].  The streaming kernels
  * take v as 16-bit block fixed point (per 32 columns a scale and two int8 limbs): the result differs from an f32 evaluation by
- * 2e-5 to 1e-4 relative (the reference's shaders accumulate in f32; the tolerance of the parity tests is 1e-3). */
+ * 2e-5 to 1e-4 relative (the reference's shaders accumulate in f32; the tolerance of the parity tests is 1e-3).
+ * v must be 16-byte aligned and out 8-byte aligned for the types and widths that the streaming kernels take (IB_ERR_INVALID otherwise);
+ * the generic kernel takes any float pointer. */
 IB_API int32_t ib_gemv_quant(ib_ctx *ctx, void *stream, float *out_dev, const ib_qtensor *m, const float *v_dev);
 /* The same call for host buffers: copies v in, runs the kernel, copies out back, synchronises. */
 IB_API int32_t ib_gemv_quant_host(ib_ctx *ctx, float *out_host, const ib_qtensor *m, const float *v_host);

@@ -133,6 +133,7 @@ int32_t launch_attention(ib_ctx *ctx, cudaStream_t s, const AttnLaunch &a) {
     IB_REQUIRE(a.pos_ptr || p.pos < p.seq_len, "attention: pos=%u outside the cache of %u rows", p.pos, p.seq_len);
     IB_REQUIRE(a.max_splits >= 1 && a.max_splits <= 2 * p.head_size && a.max_splits <= 256, "attention: %u position slices exceed what the merge step holds (%u)",
                a.max_splits, 2 * p.head_size < 256 ? 2 * p.head_size : 256);
+    IB_REQUIRE(((uintptr_t)a.k_cache % 16) == 0 && ((uintptr_t)a.v_cache % 16) == 0, "attention: the caches must be 16-byte aligned");
     AttnArgs args{p, a.pos_ptr, a.q, a.k_cache, a.v_cache, a.out, a.scratch, a.counters, a.max_splits, a.pdl, 0u};
     const bool f16 = a.kv_dtype == IB_KV_F16;
     const bool gqa4 = attn_gqa4_eligible(a);

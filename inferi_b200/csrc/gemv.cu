@@ -552,7 +552,13 @@ int32_t launch_gemv(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p_in) {
     p.err = ctx->err_dev;
     p.wait_ns = ctx->wait_limit_ns;
     IB_REQUIRE(p.nseg >= 1 && p.nseg <= 3, "gemv: bad segment count %u", p.nseg);
-    if (gemv_stream_eligible(p)) return launch_gemv_stream(ctx, stream, p);
+    // what the kernels read and write in vectors; a pointer off these boundaries would fault the GPU
+    IB_REQUIRE(((uintptr_t)p.x % 16) == 0 && ((uintptr_t)p.norm_w % 16) == 0, "gemv: the input vector and the norm weights must be 16-byte aligned");
+    if (gemv_stream_eligible(p)) {
+        for (uint32_t s = 0; s < p.nseg; s++)
+            IB_REQUIRE((p.epi == EPI_SWIGLU || ((uintptr_t)p.seg[s].out % 8) == 0) && ((uintptr_t)p.bias[s] % 8) == 0, "gemv: the output and the bias must be 8-byte aligned");
+        return launch_gemv_stream(ctx, stream, p);
+    }
     if (p.tp > 1 || p.epi == EPI_PUSH)   // the cross-GPU exchange exists only in the streaming kernel
         return set_error(IB_ERR_UNSUPPORTED, "gemv: a tensor-parallel shard (cols=%u) does not meet the streaming kernel's shape rules", p.cols);
     IB_REQUIRE(p.cols % 32 == 0 && p.cols <= GEMV_MAX_COLS, "gemv: cols=%u unsupported by the fast kernels", p.cols);

@@ -155,3 +155,31 @@ def test_a_column_that_is_no_number_reaches_every_row(backend, qt, rows, cols, b
     FfnGateUp(backend).launch(out, m, m, torch.from_numpy(v).cuda())
     assert torch.isnan(out).all()
     m.close()
+
+
+@pytest.mark.parametrize("qt,rows,cols", [(quant.Q8_0, 64, 2048), (quant.Q4_K, 64, 2304), (quant.Q6_K, 64, 2048), (quant.Q4_K, 8, 16640)])
+def test_views_off_the_vector_boundaries_are_refused(backend, qt, rows, cols):
+    """The kernels read the input in 16-byte pieces and write pairs of rows: a contiguous view that starts in between is an error from the
+    host, not a fault; one that starts on a boundary is taken."""
+    blocks = quant.random_blocks(qt, rows, cols, seed=cols + qt)
+    v = np.random.default_rng(qt).standard_normal(cols).astype(np.float32)
+    ref = oracle.gemv_ref(qt, rows, cols, blocks, v)
+    m = GpuQuantTensor(backend, qt, rows, cols, blocks)
+    x, out = torch.zeros(cols + 4, device="cuda"), torch.zeros(rows + 2, device="cuda")
+    wide = cols == 16640      # a row wider than the streaming kernel takes: its kernel writes single rows
+    for at in (0, 1, 2, 3, 4):
+        for to in (0, 1, 2):
+            xv, ov = x[at:at + cols], out[to:to + rows]
+            xv.copy_(torch.from_numpy(v))
+            if at % 4 or (to % 2 and not wide):
+                with pytest.raises(InferiError) as e:
+                    GemvQuant(backend).launch(ov, m, xv)
+                assert e.value.code == 1 and "aligned" in e.value.message
+            else:
+                GemvQuant(backend).launch(ov, m, xv)
+                assert_close(ov.cpu().numpy(), ref, what=f"views at {at}, {to}")
+    with pytest.raises(InferiError):
+        FfnGateUp(backend).launch(out[:rows], m, m, x[:cols], norm_w=torch.ones(cols + 1, device="cuda")[1:])
+    FfnGateUp(backend).launch(out[1:1 + rows], m, m, x[4:], norm_w=torch.ones(cols, device="cuda"))
+    torch.cuda.synchronize()
+    m.close()

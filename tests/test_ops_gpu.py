@@ -114,6 +114,19 @@ def test_attention_slice_shapes(backend, hs, n_kv, total):
     test_attention(backend, np.float16, hs, 4 * n_kv, 4, total - 1, total + 3)
 
 
+@pytest.mark.parametrize("dtype,mul", [(torch.float16, 4), (torch.float16, 2), (torch.float32, 4)])
+def test_caches_off_the_vector_boundary_are_refused(backend, dtype, mul):
+    p, op = AttnParams(8, 128, mul, 2 * mul, 64, 5), FusedAttention(backend)
+    q, o = torch.ones(2 * mul * 64, device="cuda"), torch.zeros(2 * mul * 64, device="cuda")
+    c = torch.ones(8 * 128 + 8, device="cuda", dtype=dtype)
+    for k, v in ((c[1:], c), (c, c[1:])):
+        with pytest.raises(InferiError) as e:
+            op.launch(p, q, k[:1024], v[:1024], o)
+        assert e.value.code == 1 and "aligned" in e.value.message
+    op.launch(p, q, c[8:], c[:1024], o)
+    assert torch.allclose(o, torch.ones_like(o))
+
+
 @pytest.mark.parametrize("hs,n_kv,total", [(64, 8, 33), (64, 8, 500), (64, 3, 1500), (128, 8, 70), (128, 8, 400), (128, 4, 2000)])
 def test_attention_clusters_whose_ctas_start_apart(backend, hs, n_kv, total):
     """A kv head's slices merge in the shared memory of their cluster's first CTA.  Products on another stream take SMs away at
