@@ -89,6 +89,7 @@ struct ib_ctx {
     // scratch of the tensor-core GEMM entry point (input halves + partial planes), grown on demand
     void *tc_scratch = nullptr;
     size_t tc_scratch_bytes = 0;
+    uint32_t tc_pass = 0xFFFFFFFFu;   // the longest pass (tokens) that the device has had room for
     // limit of every wait inside a kernel (on a shared-memory barrier, on another rank's arrival); ib_ctx_set_wait_limit
     uint64_t wait_limit_ns = 2000000000ull;
 };

@@ -135,11 +135,11 @@ struct ib_llama {
     uint64_t sample_seed = 0;
     float *sample_probs = nullptr;   // only for vocabularies that the sampler cannot hold in shared memory
     uint64_t launches_per_token_sample = 0;
-    // prompt prefill (ib_llama_prefill): one allocation for passes of up to `chunks` chunks of PF_CHUNK tokens, made at the
-    // first call and again by a call with a longer prompt
+    // prompt prefill (ib_llama_prefill): one allocation for passes of up to `chunks` chunks of PF_CHUNK tokens (a power of two),
+    // made at the first call and again by a call with a longer prompt; where the device has no room for it, for shorter passes
     struct PrefillBuffers {
         uint8_t *arena = nullptr;
-        uint32_t chunks = 0;
+        uint32_t chunks = 0, most = PREFILL_MAX_TOKENS / PF_CHUNK;   // most: what the device has had room for
         float *X = nullptr, *q = nullptr, *planes = nullptr;
         __half *hi = nullptr, *lo = nullptr;
         uint32_t *tokens = nullptr;
@@ -761,40 +761,55 @@ static size_t prefill_plane_floats(const ib_ctx *ctx, const PrefillGroup &g, uin
 }
 
 static int32_t prefill_prepare(ib_llama *m, uint32_t n) {
-    const uint32_t chunks = ((n < PREFILL_MAX_TOKENS ? n : PREFILL_MAX_TOKENS) + PF_CHUNK - 1) / PF_CHUNK;
     auto &B = m->pf;
+    uint32_t chunks = 1;   // grown in powers of two: prompts that get longer and longer allocate four times at most
+    while (chunks < B.most && chunks * PF_CHUNK < n) chunks *= 2;
     if (chunks <= B.chunks) return IB_OK;
     const ib_llama_config &c = m->cfg;
-    const uint32_t H = c.hidden_size, F = m->ffn_l, Q = m->q_dim_l, N = chunks * PF_CHUNK;
+    const uint32_t H = c.hidden_size, F = m->ffn_l, Q = m->q_dim_l;
     const uint32_t widest = F > H ? (F > Q ? F : Q) : (H > Q ? H : Q);
-    size_t planes = 0;   // the largest result that is alive at once, over the layers and over the passes' lengths
-    for (const ib_llama_layer_weights &w : m->layers) {
-        const ib_qtensor *sets[4][3] = {{w.attn_q, w.attn_k, w.attn_v}, {w.attn_output}, {w.ffn_gate, w.ffn_up}, {w.ffn_down}};
-        const uint32_t counts[4] = {3, 1, 2, 1};
-        for (int k = 0; k < 4; k++)
-            for (uint32_t ch = 1; ch <= chunks; ch++) {
-                PrefillGroup g[3];
-                size_t sum = 0;
-                for (uint32_t i = 0, ng = prefill_groups(sets[k], counts[k], g); i < ng; i++) sum += prefill_plane_floats(m->ctx, g[i], ch * PF_CHUNK);
-                planes = sum > planes ? sum : planes;
-            }
-    }
     if (B.arena) {   // growing: wait for work that may still use the old one
         IB_CHECK_CUDA(cudaDeviceSynchronize());
         IB_CHECK_CUDA(cudaFree(B.arena));
         B.arena = nullptr;
         B.chunks = 0;
     }
-    size_t total = 0;
-    auto place = [&](size_t bytes) { const size_t at = total; total += (bytes + 255) & ~(size_t)255; return at; };
-    const size_t oX = place(sizeof(float) * N * H), oq = place(sizeof(float) * N * Q);
-    const size_t ohi = place(sizeof(__half) * chunks * pf_x_halves(widest)), olo = place(sizeof(__half) * chunks * pf_x_halves(widest));
-    const size_t opl = place(sizeof(float) * planes), otok = place(sizeof(uint32_t) * N);
-    IB_CHECK_CUDA(cudaMalloc(&B.arena, total));
-    B.X = (float *)(B.arena + oX); B.q = (float *)(B.arena + oq);
-    B.hi = (__half *)(B.arena + ohi); B.lo = (__half *)(B.arena + olo); B.planes = (float *)(B.arena + opl); B.tokens = (uint32_t *)(B.arena + otok);
-    B.chunks = chunks;
-    return IB_OK;
+    for (;; chunks /= 2) {
+        const uint32_t N = chunks * PF_CHUNK;
+        size_t planes = 0;   // the largest result that is alive at once, over the layers and over the passes' lengths
+        for (const ib_llama_layer_weights &w : m->layers) {
+            const ib_qtensor *sets[4][3] = {{w.attn_q, w.attn_k, w.attn_v}, {w.attn_output}, {w.ffn_gate, w.ffn_up}, {w.ffn_down}};
+            const uint32_t counts[4] = {3, 1, 2, 1};
+            for (int k = 0; k < 4; k++)
+                for (uint32_t ch = 1; ch <= chunks; ch++) {
+                    PrefillGroup g[3];
+                    size_t sum = 0;
+                    for (uint32_t i = 0, ng = prefill_groups(sets[k], counts[k], g); i < ng; i++) sum += prefill_plane_floats(m->ctx, g[i], ch * PF_CHUNK);
+                    planes = sum > planes ? sum : planes;
+                }
+        }
+        size_t total = 0;
+        auto place = [&](size_t bytes) { const size_t at = total; total += (bytes + 255) & ~(size_t)255; return at; };
+        const size_t oX = place(sizeof(float) * N * H), oq = place(sizeof(float) * N * Q);
+        const size_t ohi = place(sizeof(__half) * chunks * pf_x_halves(widest)), olo = place(sizeof(__half) * chunks * pf_x_halves(widest));
+        const size_t opl = place(sizeof(float) * planes), otok = place(sizeof(uint32_t) * N);
+        const cudaError_t e = cudaMalloc(&B.arena, total);
+        if (e == cudaErrorMemoryAllocation && chunks > 1) {   // a prompt goes through in shorter passes rather than not at all
+            cudaGetLastError();
+            B.arena = nullptr;
+            B.most = chunks / 2;
+            continue;
+        }
+        if (e != cudaSuccess) {
+            cudaGetLastError();
+            B.arena = nullptr;
+            return set_error(e == cudaErrorMemoryAllocation ? IB_ERR_OOM : IB_ERR_CUDA, "ib_llama_prefill: buffers of %llu bytes: %s", (unsigned long long)total, cudaGetErrorString(e));
+        }
+        B.X = (float *)(B.arena + oX); B.q = (float *)(B.arena + oq);
+        B.hi = (__half *)(B.arena + ohi); B.lo = (__half *)(B.arena + olo); B.planes = (float *)(B.arena + opl); B.tokens = (uint32_t *)(B.arena + otok);
+        B.chunks = chunks;
+        return IB_OK;
+    }
 }
 
 int32_t ib_llama_prefill(ib_llama *m, void *stream, const uint32_t *tokens_host, uint32_t n, uint32_t start_pos, uint32_t *next_token_host) {
@@ -839,8 +854,9 @@ int32_t ib_llama_prefill(ib_llama *m, void *stream, const uint32_t *tokens_host,
         return IB_OK;
     };
 #define PF(expr) do { if ((rc = (expr)) != IB_OK) return rc; } while (0)
-    for (uint32_t t0 = 0; t0 < n; t0 += PREFILL_MAX_TOKENS) {
-        const uint32_t nc = n - t0 < PREFILL_MAX_TOKENS ? n - t0 : PREFILL_MAX_TOKENS, pos0 = start_pos + t0;
+    const uint32_t pass = B.chunks * PF_CHUNK;
+    for (uint32_t t0 = 0; t0 < n; t0 += pass) {
+        const uint32_t nc = n - t0 < pass ? n - t0 : pass, pos0 = start_pos + t0;
         IB_CHECK_CUDA(cudaMemcpyAsync(B.tokens, tokens_host + t0, sizeof(uint32_t) * nc, cudaMemcpyHostToDevice, s));
         PF(launch_prefill_embed(ctx, s, m->token_embd, B.tokens, nc, c.vocab_size, B.X));
         PfPlanes g[3];

@@ -244,33 +244,45 @@ extern "C" int32_t ib_gemm_quant(ib_ctx *ctx, void *stream, float *out_dev, cons
     const uint32_t rows = (uint32_t)m->rows, cols = (uint32_t)m->cols;
     // a pass: what the layers of a prompt take, and less where the split planes of a tall matrix would grow beyond 512 MiB
     uint32_t pass = n < PREFILL_MAX_TOKENS ? n : PREFILL_MAX_TOKENS;
+    if (pass > ctx->tc_pass) pass = ctx->tc_pass;
     auto bytes_of = [&](uint32_t nc, size_t &half_bytes) {
         const StreamK sk = prefill_streamk(ctx, rows, cols, nc);
         half_bytes = (nc + PF_CHUNK - 1) / PF_CHUNK * pf_x_halves(cols) * sizeof(__half);
         return 2 * half_bytes + (((size_t)(prefill_max_pieces(sk) - 1) * nc * rows * sizeof(float) + 255) & ~(size_t)255);
     };
-    size_t half_bytes = 0, need = bytes_of(pass, half_bytes);
-    while (pass > PF_CHUNK && need > ((size_t)512 << 20)) {
-        pass = (pass / 2 + PF_CHUNK - 1) / PF_CHUNK * PF_CHUNK;
-        need = bytes_of(pass, half_bytes);
-    }
-    if (n % pass) {   // the last, shorter pass may split its tiles further
-        size_t hb = 0;
-        const size_t last = bytes_of(n % pass, hb) - 2 * hb + 2 * half_bytes;
-        if (last > need) need = last;
-    }
-    const size_t tiled_at = need;
-    if (retile) need += m->rows * tiled.row_bytes;
+    auto shorter = [](uint32_t p) { return (p / 2 + PF_CHUNK - 1) / PF_CHUNK * PF_CHUNK; };
+    size_t half_bytes = 0;
+    while (pass > PF_CHUNK && bytes_of(pass, half_bytes) > ((size_t)512 << 20)) pass = shorter(pass);
+    size_t need, tiled_at;
     int32_t rc = IB_OK;
-    if (need > ctx->tc_scratch_bytes) {
+    for (;; pass = shorter(pass)) {
+        need = bytes_of(pass, half_bytes);
+        if (n % pass) {   // the last, shorter pass may split its tiles further
+            size_t hb = 0;
+            const size_t last = bytes_of(n % pass, hb) - 2 * hb + 2 * half_bytes;
+            if (last > need) need = last;
+        }
+        tiled_at = need;
+        if (retile) need += m->rows * tiled.row_bytes;
+        if (need <= ctx->tc_scratch_bytes) break;
         // growing the scratch: wait for work that may still use the old one
         cudaError_t e = cudaDeviceSynchronize();
         if (e == cudaSuccess && ctx->tc_scratch) e = cudaFree(ctx->tc_scratch);
         ctx->tc_scratch = nullptr;
         ctx->tc_scratch_bytes = 0;
         if (e == cudaSuccess) e = cudaMalloc(&ctx->tc_scratch, need);
-        if (e != cudaSuccess) rc = set_error(e == cudaErrorMemoryAllocation ? IB_ERR_OOM : IB_ERR_CUDA, "ib_gemm_quant: scratch of %llu bytes: %s", (unsigned long long)need, cudaGetErrorString(e));
-        else ctx->tc_scratch_bytes = need;
+        if (e == cudaSuccess) {
+            ctx->tc_scratch_bytes = need;
+            break;
+        }
+        cudaGetLastError();
+        ctx->tc_scratch = nullptr;
+        if (e == cudaErrorMemoryAllocation && pass > PF_CHUNK) {   // shorter passes rather than none
+            ctx->tc_pass = shorter(pass);
+            continue;
+        }
+        rc = set_error(e == cudaErrorMemoryAllocation ? IB_ERR_OOM : IB_ERR_CUDA, "ib_gemm_quant: scratch of %llu bytes: %s", (unsigned long long)need, cudaGetErrorString(e));
+        break;
     }
     __half *hi = reinterpret_cast<__half *>(ctx->tc_scratch), *lo = reinterpret_cast<__half *>((uint8_t *)ctx->tc_scratch + half_bytes);
     float *planes = reinterpret_cast<float *>((uint8_t *)ctx->tc_scratch + 2 * half_bytes);

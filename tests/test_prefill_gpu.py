@@ -96,6 +96,43 @@ def test_prompt_attention_at_the_edges_of_its_tiles(backend, hidden, heads, n, s
     dev_w.close()
 
 
+def test_prompts_and_gemms_go_in_shorter_passes_where_memory_is_short(backend):
+    """1024 tokens through layers of the 8B architecture take 330 MB of buffers at once, 128 tokens 45 MB: with 150 MB free on the device the
+    prompt goes through in shorter passes, to the same result, and so do 1024 rows through one matrix.  (Sums of f32
+    that are split differently: 1e-6; where that rounds a cache value the other way, 2^-11 of one of the 1500 rows that are averaged.)"""
+    from inferi_b200.ops import Backend, GemmQuant
+    cfg = Llama2Config(4096, 14336, 1, 32, 8, 512, 2048, 500000.0, 1e-5)
+    w = synth_weights(cfg, seed=51, device="cuda", recipe=dict(Q4_K_M, token_embd=quant.Q4_K, output=quant.Q4_K))
+    toks = np.random.default_rng(52).integers(0, 512, 1500).tolist()
+    x = torch.randn(1024, 4096, device="cuda")
+
+    def results(free):
+        be = Backend(0)
+        dev_w = Llama2Weights(be, cfg, w)
+        model = Llama2(be, cfg, dev_w, kv_f16=True)
+        out = torch.zeros(1024, 14336, device="cuda")
+        torch.cuda.synchronize()
+        torch.cuda.empty_cache()
+        hog = torch.empty(torch.cuda.mem_get_info()[0] - free, dtype=torch.uint8, device="cuda") if free else None
+        model.prefill(toks)
+        hidden = model.hidden_state()
+        model.prefill(toks[:9])
+        model.prefill(toks)          # the buffers that a long prompt got are kept
+        assert np.array_equal(hidden, model.hidden_state())
+        GemmQuant(be).launch(out, dev_w.layers[0]["ffn_gate"], x)
+        torch.cuda.synchronize()
+        del hog
+        torch.cuda.empty_cache()
+        model.close()
+        dev_w.close()
+        be.close()
+        return hidden, out
+
+    (h0, g0), (h1, g1) = results(0), results(150 << 20)
+    assert np.abs(h0 - h1).max() <= 1e-4 * np.abs(h0).max()
+    assert float((g0 - g1).abs().max()) <= 1e-5 * float(g0.abs().max())
+
+
 def test_prefill_refuses_what_the_tensor_core_path_does_not_take(backend):
     cfg = Llama2Config(256, 2048, 2, 4, 2, 512, 64, 500000.0, 1e-5)     # 2 query heads per kv head, 256-row matrices... kv_mul = 2
     w = synth_weights(cfg, seed=5, recipe=dict(Q4_K_M, token_embd=quant.Q4_K, attn_v=quant.Q4_K, ffn_down=quant.Q4_K, output=quant.Q4_K))
