@@ -19,7 +19,8 @@ from .quant import BLOCK_BYTES, BLOCK_ELEMS, F32, NAMES, Q4_K, Q5_K, Q6_K, Q8_0,
 
 
 _f16, _f32, _tensor = torch.float16, torch.float32, torch.Tensor
-_current_device, _raw_stream = torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream
+# (a torch without CUDA has neither: it can import this module, make quantized data and read files; no launch gets as far as these)
+_current_device, _raw_stream = getattr(torch._C, "_cuda_getDevice", None), getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def _stream_ptr() -> int:

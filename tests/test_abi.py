@@ -3,6 +3,8 @@ work without a GPU instead of falling back to anything."""
 import ctypes as C
 import os
 import re
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -85,3 +87,15 @@ def test_quantizer_round_trip(qt, bound):
     # zero rows stay zero and finite
     z = oracle.dequantize(qt, quant.quantize(qt, torch.zeros(4, 256)).numpy(), 1024)
     assert np.array_equal(z, np.zeros(1024, np.float32))
+
+
+def test_the_package_imports_with_a_torch_that_has_no_cuda():
+    """Without these two functions of torch's CUDA build the modules import, and a context is refused with the library's own message."""
+    code = ("import torch\n"
+            "for n in ('_cuda_getDevice', '_cuda_getCurrentRawStream'):\n    delattr(torch._C, n)\n"
+            "from inferi_b200 import ops\n"
+            "try:\n    ops.RmsNorm(None).launch(ops.RmsNormConfig(1e-5), torch.zeros(4), torch.zeros(4), torch.zeros(4))\n"
+            "except ops.InferiError as e:\n    assert 'float32 CUDA tensor' in str(e)\n"
+            "print('imported')\n")
+    out = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, cwd=ROOT, timeout=300)
+    assert out.returncode == 0 and "imported" in out.stdout, out.stderr[-2000:]
