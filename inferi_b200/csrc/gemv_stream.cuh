@@ -648,7 +648,7 @@ __device__ __forceinline__ void pack_stream(uint8_t *smem, uint32_t cols, const 
         float amax = max_nan(abs_max(v[0]), abs_max(v[1]));
         amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
         amax = max_nan(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
-        const float inv = amax > 0.f ? __fdividef(ACT_STEPS, amax) : 0.f;   // 2 ulp: the limbs absorb it (the largest |x| still rounds to 32512)
+        const float inv = pack_units(v, amax);
         uint32_t w0[2], w1[2];
         int s0 = 0, s1 = 0;
 #pragma unroll

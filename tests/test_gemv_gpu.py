@@ -183,3 +183,14 @@ def test_views_off_the_vector_boundaries_are_refused(backend, qt, rows, cols):
     FfnGateUp(backend).launch(out[1:1 + rows], m, m, x[4:], norm_w=torch.ones(cols, device="cuda"))
     torch.cuda.synchronize()
     m.close()
+
+
+@pytest.mark.parametrize("power", [-121, -115, -112, -100, 100, 108])
+@pytest.mark.parametrize("qt,rows,cols", [(quant.Q8_0, 64, 2048), (quant.Q4_K, 64, 2304), (quant.Q5_K, 64, 8448), (quant.Q6_K, 64, 2048), (quant.Q4_K, 8, 16640)])
+def test_vectors_far_from_one(backend, qt, rows, cols, power):
+    """A vector times a power of two gives the product times it.  What is lost at the lower end is the group's scale, largest |x| / 32512,
+    which f32 holds to a multiple of 2^-149: half of one of 2^(power + 1) / 32512 is 2^(-136 - power) of it, 3e-5 at 2^-121."""
+    blocks = quant.random_blocks(qt, rows, cols, seed=cols + qt, scale=1e-3)
+    v = np.clip(np.random.default_rng(power + 200).standard_normal(cols), -1.9, 1.9).astype(np.float32)
+    got = np.ldexp(run_gemv(backend, qt, rows, cols, blocks, np.ldexp(v, power)).astype(np.float64), -power)
+    assert_close(got, oracle.gemv_ref(qt, rows, cols, blocks, v), what=f"{quant.NAMES[qt]} {rows}x{cols} at 2^{power}")
