@@ -81,25 +81,33 @@ bool attn_gqa4_eligible(const AttnLaunch &a) {
            ((uintptr_t)a.k_cache % 16) == 0 && ((uintptr_t)a.v_cache % 16) == 0 && ((uintptr_t)a.out % 16) == 0 && ((uintptr_t)a.scratch % 16) == 0;
 }
 
-// CTAs per cluster: as many as fit the GPU with one cluster per kv head
-static uint32_t gqa4_cluster_ctas(const ib_ctx *ctx, const ib_attn_params &p) {
-    const uint32_t n_kv = p.n_heads / p.kv_mul;
+// CTAs per cluster, one cluster per kv head.  Short: as many as the GPU holds.  Middle: its CTAs need an SM each and their clusters a GPC
+// with so many free ones; on more than two thirds of the SMs some clusters wait for others (12 kv heads x 8 CTAs fit; 16 x 8 take twice
+// the time: 13.4 us against 8.9 as 16 x 4 at 2048 positions).  Fewer than 4 CTAs per kv head: no middle regime.
+static uint32_t gqa4_cluster_ctas(const ib_ctx *ctx, const ib_attn_params &p, uint32_t regime) {
+    const uint32_t n_kv = p.n_heads / p.kv_mul, room = (uint32_t)ctx->sm_count * 2 / (regime == ATTN_MIDDLE ? 3 : 2);
     uint32_t c = GQA4_CLUSTER_MAX;
-    while (c > 1 && c * n_kv > (uint32_t)ctx->sm_count) c /= 2;
-    return c;
+    while (c > 1 && c * n_kv > room) c /= 2;
+    return regime == ATTN_MIDDLE && (c < 4 || c * n_kv > room) ? 0u : c;
 }
 
-// The middle regime ends where the long one's bytes in flight (three CTAs on every SM against one on less than half of them) outweigh
-// its slower merge: measured us per launch, 8 kv heads, middle / long - head size 64: 6.9 / 8.7 at 2048 positions, 12.8 / 16.1 at
-// 8192, 20.1 / 20.8 at 16384; head size 128: 8.7 / 9.7 at 2048, 12.4 / 12.0 at 4096.  Its CTAs need an SM each and their clusters a GPC
-// with so many free ones: with clusters on more than half of the SMs some wait for others (16 kv heads: twice the time).
-constexpr uint32_t GQA4_MIDDLE_PER_64 = 2048, GQA4_MIDDLE_PER_128 = 384;
+// Up to how many positions per CTA of a kv head's cluster a regime is the fastest.  A cluster regime's time hardly depends on the number
+// of kv heads, the long one's does: with few heads it has more CTAs per head.  Measured us per launch, short / middle / long:
+//   head size 64:   4 kv heads  5.3 / 6.2 / 6.5 at 1536 positions, 6.1 / 6.6 / 7.0 at 2048;  8 heads  4.4 / 5.7 / 6.6 at 640, 4.9 / 5.9 / 6.8 at
+//                   1024, 6.7 / 6.3 / 7.6 at 1536;  16 (middle in clusters of 4)  5.0 / 6.0 / 7.0 at 768, 6.8 / 6.8 / 7.9 at 1024.
+//                   Middle against long: 18.9 / 22.4 at 16384 with 4 heads (26.0 / 24.6 at 24576), 20.2 / 21.0 with 8 (27.4 / 25.2), 20.5 / 23.1
+//                   with 12;  16 heads  8.9 / 9.9 at 2048, 12.4 / 12.6 at 4096 (11.7 / 11.1
+//                   from a cache that is still in L2), 16.2 / 15.6 at 6144.
+//   head size 128:  8 kv heads  3.6 / 4.1 / 4.2 at 128, 4.0 / 4.2 / 4.5 at 192, 4.2 / 4.1 / 4.4 at 224, 5.0 / 4.5 / 6.2 at 512.
+//                   Middle against long: 7.9 / 7.9 at 2560 with 2 heads (8.7 / 8.1 at 3072), 9.1 / 9.3 with 4 (10.1 / 9.5), 10.3 / 10.6 at 3072
+//                   with 8 (12.1 / 11.7 at 4096), 10.4 / 11.5 at 3072 with 12;  16 heads  7.9 / 8.1 at 1024, 9.9 / 9.2 at 1536.
 uint32_t attn_regime_positions(const ib_ctx *ctx, const AttnLaunch &a, uint32_t regime) {
-    if (!attn_gqa4_eligible(a) || ctx->sm_count == 0) return 0u;   // (ib_attention_static knows no device)
-    const uint32_t c = gqa4_cluster_ctas(ctx, a.p), n_kv = a.p.n_heads / a.p.kv_mul;
-    if (regime == ATTN_SHORT) return c * GQA4_SHORT_PER;
-    if (2 * c * n_kv > (uint32_t)ctx->sm_count) return 0u;
-    return c * (a.p.head_size == 128 ? GQA4_MIDDLE_PER_128 : GQA4_MIDDLE_PER_64);
+    if (!attn_gqa4_eligible(a) || ctx->sm_count == 0) return 0u;
+    const uint32_t n_kv = a.p.n_heads / a.p.kv_mul, middle = gqa4_cluster_ctas(ctx, a.p, ATTN_MIDDLE), c = gqa4_cluster_ctas(ctx, a.p, regime);
+    const bool wide = a.p.head_size == 128;
+    if (regime == ATTN_MIDDLE) return c * (wide ? (c < 8 ? 256 : (n_kv <= 4 ? 320 : 384)) : (c < 8 ? 512 : 2048));
+    if (middle == 0 || c < 8) return c * (wide && middle ? 24 : 64);
+    return c * (wide ? 24 : (middle < 8 ? 96 : (n_kv <= 4 ? 256 : 128)));
 }
 
 template <int HS, uint32_t REGIME>
@@ -146,7 +154,7 @@ int32_t launch_attention(ib_ctx *ctx, cudaStream_t s, const AttnLaunch &a) {
                 if (p.pos < attn_regime_positions(ctx, a, r)) regime = r;
         }
         uint32_t splits = a.max_splits, per;
-        if (regime != ATTN_LONG) args.cluster = splits = gqa4_cluster_ctas(ctx, p);
+        if (regime != ATTN_LONG) args.cluster = splits = gqa4_cluster_ctas(ctx, p, regime);
         if (!a.pos_ptr) {   // with a host-known position only the slices that will do work are launched
             gqa4_plan(p.pos + 1, a.max_splits, args.cluster, gqa4_warps(p.head_size, regime), splits, per);
             if (regime != ATTN_LONG) args.cluster = splits;

@@ -26,14 +26,13 @@ constexpr uint32_t GQA4_ROWS_PER_WARP_STEP = 8;
 //  * short: the slices are the CTAs of one thread-block cluster, 4 warps each.  They leave their partials in the shared memory of the
 //    cluster's first CTA (distributed shared memory) and meet at the cluster barrier; the first CTA merges from its own shared
 //    memory.  Publishing the partials through global memory, counting arrivals with an atomic and reading them back are three L2
-//    round trips (~2.6 us of a ~6 us kernel at these lengths); the cluster barrier is one hardware barrier.  Up to two row-loop
-//    iterations per slice.
+//    round trips (~2.6 us of a ~6 us kernel at these lengths); the cluster barrier is one hardware barrier.
 //  * middle: the same with 8 or 16 warps per CTA, which hold the row loop at a few iterations.
 //  * long: many CTAs of 4 warps (one wave of 3 per SM), merged through global memory.  Slices: one warp step of every warp (32
 //    positions) each while there are at most 16 of them, then 16 slices that grow to 128 positions, then slices of 128
 //    positions up to the launch's maximum, then longer ones.
 // Clusters have at most 8 CTAs: eight clusters of 16 - one per kv head of the Llama-3 models - do not all fit the GPU at once.
-constexpr uint32_t GQA4_CLUSTER_MAX = 8, GQA4_SHORT_PER = 64;   // positions per slice up to which `short` is used
+constexpr uint32_t GQA4_CLUSTER_MAX = 8;
 __host__ __device__ constexpr int gqa4_warps(uint32_t hs, uint32_t regime) { return regime != ATTN_MIDDLE ? ATTN_WARPS : (hs == 128 ? 8 : 16); }   // (head size 128 needs 142 registers)
 constexpr uint32_t GQA4_MIN_PER_SPLIT = ATTN_WARPS * GQA4_ROWS_PER_WARP_STEP, GQA4_KNEE = 16, GQA4_KNEE_PER = 128;
 __host__ __device__ __forceinline__ void gqa4_plan(uint32_t total, uint32_t max_splits, uint32_t cluster, uint32_t warps, uint32_t &nsplit, uint32_t &per) {
@@ -125,7 +124,11 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
     // Another CTA's shared memory may be written only once that CTA has started: everyone arrives here, and waits ahead of the first
     // remote store (or of leaving), behind the rows.
     if constexpr (CLUSTER) cluster.barrier_arrive();
-    if (a.pdl) asm volatile("griddepcontrol.launch_dependents;");
+    // Behind any kernel (pdl 2), the long regime lets its successor start with the last of its own rows: an attention launch that
+    // starts earlier takes the SMs' free slots unevenly and itself ends later (4 kv heads of 128, 4096 positions, back to back: 10.2 us
+    // against 11.4).  In a token graph the successor fills a whole SM and cannot.
+    const bool late = !CLUSTER && a.pdl == 2;
+    if (a.pdl && !late) asm volatile("griddepcontrol.launch_dependents;");
     const bool early = a.pdl == 1;   // rows may be requested ahead of the wait
     if (a.pdl == 2) asm volatile("griddepcontrol.wait;" ::: "memory");
     // The position was written at the end of the previous token, not by the predecessor: it can be read before the wait.
@@ -200,6 +203,7 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
 #pragma unroll 1
     for (uint32_t base = base0; base < t1; base += W * ROWS) {
         const uint32_t nbase = base + W * ROWS;
+        if (late && nbase >= t1) asm volatile("griddepcontrol.launch_dependents;");
         if (nbase < t1) {
 #pragma unroll
             for (int s = 0; s < STEPS; s++) {

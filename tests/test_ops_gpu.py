@@ -104,11 +104,14 @@ def test_attention(backend, kv_dtype, hs, n_heads, kv_mul, pos, seq):
         assert_close(out.cpu().numpy(), ref, what=f"attention hs={hs} pos={pos}")
 
 
-# both sides of the context lengths where a kv head's slices change shape (8 CTAs of 64 positions; 2048 or 384 each), the first one with
-# a single row in the last slice; and few and many kv heads
+# both sides of the context lengths where a kv head's slices change shape (clusters of 8 CTAs of 64 to 256 positions each, of wider CTAs, and of
+# 4 with many kv heads; no clusters), the first one with a single row in the last slice; and few and many kv heads
 @pytest.mark.parametrize("hs,n_kv,total", [
     (64, 8, 512), (64, 8, 513), (64, 8, 1025), (64, 8, 16384), (64, 8, 16385), (64, 1, 900), (64, 3, 5000), (64, 20, 600),
     (128, 8, 512), (128, 8, 513), (128, 8, 3072), (128, 8, 3073), (128, 2, 1000), (128, 12, 700),
+    (64, 4, 2048), (64, 4, 2049), (64, 12, 1024), (64, 12, 1025), (64, 12, 16385), (64, 16, 768), (64, 16, 769), (64, 16, 2048), (64, 16, 2049), (64, 26, 257),
+    (128, 8, 192), (128, 8, 193), (128, 1, 2560), (128, 1, 2561), (128, 12, 3072), (128, 12, 3073), (128, 16, 192), (128, 16, 1024), (128, 16, 1025),
+    (128, 20, 97), (128, 26, 257),
 ])
 def test_attention_slice_shapes(backend, hs, n_kv, total):
     test_attention(backend, np.float16, hs, 4 * n_kv, 4, total - 1, total + 3)
