@@ -245,17 +245,17 @@ def test_a_wait_that_gave_up_leaves_no_counts_for_later_launches():
 
 
 def test_logits_across_the_position_where_the_token_graph_changes(backend):
-    """Below position 320 the model replays a token graph whose attention nodes merge their slices inside thread-block
-    clusters, from there on the one that merges through global memory: the logits on both sides of the change must agree
-    with the oracle fed the same tokens (teacher forcing, so that a near-tie cannot send the two down different branches)."""
-    # 32 query / 8 kv heads of 64 (the 1B layer shapes): 8 kv heads make 55 slices, clusters of 5, and the change at 5 x 64 positions
-    cfg = Llama2Config(2048, 8192, 2, 32, 8, 1024, 512, 500000.0, 1e-5)
+    """Up to 1024 positions the model replays a token graph whose attention nodes are clusters of narrow CTAs, from there on one with
+    wider CTAs: the logits on both sides of the change must agree with the oracle fed the same tokens (teacher forcing, so that a
+    near-tie cannot send the two down different branches)."""
+    # 32 query / 8 kv heads of 64 (the 1B layer shapes): clusters of 8 CTAs, and the change behind 8 x 128 positions
+    cfg = Llama2Config(2048, 8192, 2, 32, 8, 1024, 1152, 500000.0, 1e-5)
     w = synth_weights(cfg, seed=4242)
     dev_w = Llama2Weights(backend, cfg, w)
     model = Llama2(backend, cfg, dev_w, kv_f16=True)
-    seq = [7, 300, 41, 9] + model.generate([7, 300, 41, 9], 330).tolist()      # the device loop crosses the change by itself
+    seq = [7, 300, 41, 9] + model.generate([7, 300, 41, 9], 1034).tolist()     # the device loop crosses the change by itself
     ref = oracle.Llama(oracle_cfg(cfg), weights_to_host(w), kv_f16=True)
-    first, last = 312, 328
+    first, last = 1016, 1032
     probe = Llama2(backend, cfg, dev_w, kv_f16=True)
     probe.generate(seq[:first], 0)                                               # cache rows 0 .. first - 1
     worst = 0.0
@@ -267,7 +267,76 @@ def test_logits_across_the_position_where_the_token_graph_changes(backend):
         worst = max(worst, float(np.abs(logits - want).max()))
         assert nxt == seq[pos + 1], f"the per-token path and the device loop disagree at position {pos}"
     assert worst <= LOGITS_MAX_ABS, f"logits differ by {worst} around the change of graphs"
-    print(f"logits around position 320 agree with the oracle to {worst:.3e}")
+    print(f"logits around position 1024 agree with the oracle to {worst:.3e}")
     model.close()
     probe.close()
+    dev_w.close()
+
+
+def one_layer_logits_f64(cfg, w, seq, positions):
+    """Logits of a one-layer model at `positions` in 64 bits, the cache rounded to f16: keys and values depend on nothing but the tokens."""
+    def mat(t, rows, cols):
+        return torch.from_numpy(oracle.dequantize(t[0], t[1].cpu().numpy(), rows * cols).reshape(rows, cols)).cuda().double()
+
+    def norm(x, g):
+        return x / torch.sqrt((x * x).mean(-1, keepdim=True) + cfg.rms_norm_eps) * g.cuda().double()
+
+    sh, lw, H, hs, nkv = cfg.shapes(), w["layers"][0], cfg.hidden_size, cfg.head_size, cfg.num_key_value_heads
+    W = {n: mat(lw[n], *sh[n]) for n in sh if n in lw}
+    theta = torch.tensor(cfg.rope_theta, dtype=torch.float32).pow(-torch.arange(0, hs, 2, dtype=torch.float32) / hs)
+
+    def rope(x, pos):       # [n, heads, hs], adjacent pairs; the angle is an f32 product, as in the kernels
+        a = (pos.float()[:, None] * theta).double().cuda()[:, None, :]
+        re, im = x[..., 0::2], x[..., 1::2]
+        return torch.stack((a.cos() * re - a.sin() * im, a.sin() * re + a.cos() * im), -1).flatten(-2)
+
+    x = mat(w["token_embd"], cfg.vocab_size, H)[torch.as_tensor(seq).long()]
+    h = norm(x, lw["attn_norm"])
+    at = torch.arange(len(seq))
+    K = rope((h @ W["attn_k"].T).view(-1, nkv, hs), at).half().double()
+    V = (h @ W["attn_v"].T).view(-1, nkv, hs).half().double()
+    out = []
+    for p in positions:
+        q = rope((h[p] @ W["attn_q"].T).view(1, -1, hs), at[p:p + 1]).view(nkv, -1, hs)
+        pr = torch.softmax(torch.einsum("gmh,tgh->gmt", q, K[:p + 1]) / hs ** 0.5, -1)
+        y = x[p] + W["attn_output"] @ torch.einsum("gmt,tgh->gmh", pr, V[:p + 1]).reshape(-1)
+        f = norm(y, lw["ffn_norm"])
+        y = y + W["ffn_down"] @ (torch.nn.functional.silu(W["ffn_gate"] @ f) * (W["ffn_up"] @ f))
+        out.append((mat(w["output"], cfg.vocab_size, H) @ norm(y, w["output_norm"])).cpu().numpy())
+    return out
+
+
+def test_logits_across_both_changes_of_the_token_graph(backend):
+    """8 kv heads of 128: the attention nodes' shape changes behind 192 positions and again behind 3072.  Rows of earlier tokens come from
+    `prefill`; around each change the logits of single steps, of the greedy device loop and of the sampling one are those of the f64
+    model (weights of this spread make the scores' deviation 1.6, so that a slice that is left out moves the logits by a tenth)."""
+    cfg = Llama2Config(4096, 2048, 1, 32, 8, 1024, 3104, 500000.0, 1e-5)
+    w = synth_weights(cfg, seed=77, device="cuda", recipe=dict(Q4_K_M, token_embd=quant.Q4_K, output=quant.Q6_K))
+    dev_w = Llama2Weights(backend, cfg, w)
+    model = Llama2(backend, cfg, dev_w, kv_f16=True)
+    seq = np.random.default_rng(78).integers(0, 1024, 3084).tolist()
+    done, worst = 0, 0.0
+    for change in (192, 3072):
+        first, end = change - 6, change + 6
+        want = one_layer_logits_f64(cfg, w, seq, range(first, end))
+        model.prefill(seq[done:first], start_pos=done)
+        singles = [model.forward(seq[p], p, want_logits=True)[1] for p in range(first, end)]
+        worst = max([worst] + [float(np.abs(a - b).max()) for a, b in zip(singles, want)])
+        for temperature in (0.0, 0.8):
+            model.set_sampler(temperature, 0.9, seed=5)
+            for stop in (change, change + 1, end):          # the step before the change, the one behind it, and the last one
+                model.generate(seq[first:stop], 0, start_pos=first)
+                assert np.array_equal(model.last_logits(), singles[stop - 1 - first]), f"temperature {temperature}, up to position {stop}"
+            # tokens of its own across the change: the same as step by step
+            own = model.generate([seq[first]], 10, start_pos=first).tolist()
+            tok = seq[first]
+            for i, o in enumerate(own):
+                tok, _ = model.forward(tok, first + i)
+                assert tok == o
+        model.set_sampler(0.0)
+        model.generate(seq[first:end], 0, start_pos=first)   # the cache rows of `seq` again
+        done = end
+    assert worst <= LOGITS_MAX_ABS, f"logits differ by {worst} around the changes of graphs"
+    print(f"logits around positions 192 and 3072 agree with the f64 model to {worst:.3e}")
+    model.close()
     dev_w.close()
