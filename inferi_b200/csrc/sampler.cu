@@ -63,13 +63,14 @@ __host__ __device__ inline float sample_coin(uint64_t seed, uint32_t pos) {
     return (float)(uint32_t)(z >> 40) * (1.0f / 16777216.0f);
 }
 
-// p in units of 2^-52 (p in [0, 1]; exact for p >= 2^-29, rounded down below)
+// p in units of 2^-52 (p in [0, 1]; exact for p >= 2^-29, rounded down below, but never to nothing: a coin of 0 falls to the first token
+// whose p is above 0, however small).  A p that is no number - the logits held one, or an infinity - has no mass.
 __device__ __forceinline__ unsigned long long mass_of(float p) {
     const uint32_t b = __float_as_uint(p), e = b >> 23;
-    if (e == 0) return 0ull;
+    if (!(p > 0.f)) return 0ull;
     const unsigned long long m = (b & 0x7FFFFFu) | 0x800000u;
     const int s = (int)e - 98;   // value = m * 2^(e - 150)
-    return s >= 0 ? m << s : (s > -24 ? m >> -s : 0ull);
+    return s >= 0 ? m << s : (s > -24 ? m >> -s : 1ull);
 }
 // 64-bit shared-memory sum out of two native 32-bit atomics: whoever makes the low word wrap carries the one
 __device__ __forceinline__ void mass_add(SampleShared &S, uint32_t bin, unsigned long long q) {

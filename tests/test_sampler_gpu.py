@@ -95,6 +95,32 @@ def test_bins_with_more_elements_than_the_list(backend, n, step):
     check_many(backend, logits, 1.0, 0.9, np.float32([0.0, 0.37, 0.999999]))
 
 
+@pytest.mark.parametrize("n", [2, 100, 40000, 300000])
+@pytest.mark.parametrize("depth", [30.0, 37.0, 85.0])
+def test_a_coin_of_zero_falls_to_the_first_token_that_can_come(backend, n, depth):
+    """Its probability may be far below the coins' resolution (e^-37 = 2^-53, e^-85 over 300000 tokens is no normal f32); one of 0 cannot come."""
+    logits = np.zeros(n, dtype=np.float32)
+    logits[0], logits[n // 2] = -depth, -200.0
+    assert oracle.sample(logits, 1.0, 0.0, 0.0)[0] == 0
+    for topp in (0.0, 1.0):
+        assert gpu_sample(backend, logits, 1.0, topp, 0.0) == 0
+    logits[0] = -200.0
+    if n > 2:
+        assert gpu_sample(backend, logits, 1.0, 0.0, 0.0) == oracle.sample(logits, 1.0, 0.0, 0.0)[0] == 1
+
+
+@pytest.mark.parametrize("n", [2, 100, 40000, 300000])
+@pytest.mark.parametrize("value", [float("nan"), -float("nan"), float("inf")])
+def test_logits_that_are_no_numbers_still_give_a_token(backend, n, value):
+    """Every probability is NaN: no running sum exceeds the coin (multinomial: the last token) and there is no candidate (top-p: the
+    arg-max of equal keys, the first token)."""
+    logits = np.random.default_rng(n).standard_normal(n).astype(np.float32)
+    logits[n // 2] = value
+    for coin in (0.0, 0.5, 0.999999):
+        assert gpu_sample(backend, logits, 0.8, 0.0, coin) == n - 1
+        assert gpu_sample(backend, logits, 0.8, 0.9, coin) == 0
+
+
 def test_temperature_zero_is_argmax_and_contract(backend):
     x = np.float32([0.1, 3.0, -1.0, 3.0, 2.0])
     assert gpu_sample(backend, x, 0.0, 0.9, 0.5) == 1                   # greedy, lowest index on ties
