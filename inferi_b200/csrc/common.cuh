@@ -179,7 +179,6 @@ int32_t launch_gemv_stream(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p
 // IB_OK, or IB_ERR_TIMEOUT when a kernel raised the context's error word (call after a synchronisation)
 int32_t check_device_error(ib_ctx *ctx);
 int32_t launch_gemv_generic(ib_ctx *ctx, cudaStream_t stream, const ib_qtensor *m, const float *v, float *out);
-uint64_t soa_row_bytes(int qtype, uint32_t nb);   // of a row of nb Q8_0 or Q6_K blocks
 int32_t retile_to_soa(ib_ctx *ctx, cudaStream_t stream, int qtype, const uint8_t *src, uint8_t *dst, uint64_t rows, uint32_t nb);
 bool gemv_fast_eligible(int qtype, uint64_t rows, uint64_t cols);
 void fill_seg(GemvSeg &s, const ib_qtensor *m, float *out);

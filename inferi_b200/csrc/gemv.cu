@@ -472,23 +472,22 @@ __global__ void __launch_bounds__(256) gemv_generic_kernel(const uint8_t *__rest
 }
 
 // -------------------------------------------------------------------------------------------------
-// re-tiling into the SOA row layout (the same bytes per row, or more where the last group of 8 blocks is not full)
+// upload-time re-tiling into the SOA row layout (same bytes per row)
 // -------------------------------------------------------------------------------------------------
-__global__ void retile_kernel(int qtype, const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, uint64_t rows, uint32_t nb,
-                              uint64_t dst_row) {
+__global__ void retile_kernel(int qtype, const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, uint64_t rows, uint32_t nb) {
     const uint64_t total = rows * nb;
     for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total; t += (uint64_t)gridDim.x * blockDim.x) {
         const uint64_t r = t / nb;
         const uint32_t b = (uint32_t)(t % nb), bb = b & 7;
         if (qtype == IB_Q8_0) {
             const uint8_t *s = src + (r * nb + b) * 34;
-            uint8_t *d = dst + r * dst_row + (size_t)(b >> 3) * 272;
+            uint8_t *d = dst + r * nb * 34 + (size_t)(b >> 3) * 272;
             for (int i = 0; i < 32; i++) d[32 * bb + i] = s[2 + i];
             d[256 + 2 * bb] = s[0];
             d[256 + 2 * bb + 1] = s[1];
         } else {  // Q6_K
             const uint8_t *s = src + (r * nb + b) * 210;
-            uint8_t *d = dst + r * dst_row + (size_t)(b >> 3) * 1680;
+            uint8_t *d = dst + r * nb * 210 + (size_t)(b >> 3) * 1680;
             for (int i = 0; i < 128; i++) d[128 * bb + i] = s[i];
             for (int i = 0; i < 64; i++) d[1024 + 64 * bb + i] = s[128 + i];
             for (int i = 0; i < 16; i++) d[1536 + 16 * bb + i] = s[192 + i];
@@ -498,13 +497,11 @@ __global__ void retile_kernel(int qtype, const uint8_t *__restrict__ src, uint8_
     }
 }
 
-uint64_t soa_row_bytes(int qtype, uint32_t nb) { return (uint64_t)((nb + 7) / 8) * (qtype == IB_Q8_0 ? 272 : 1680); }
-
 int32_t retile_to_soa(ib_ctx *ctx, cudaStream_t stream, int qtype, const uint8_t *src, uint8_t *dst, uint64_t rows, uint32_t nb) {
     const uint64_t total = rows * nb;
     const int threads = 256;
     const int blocks = (int)((total + threads - 1) / threads < 65535 ? (total + threads - 1) / threads : 65535);
-    retile_kernel<<<blocks, threads, 0, stream>>>(qtype, src, dst, rows, nb, soa_row_bytes(qtype, nb));
+    retile_kernel<<<blocks, threads, 0, stream>>>(qtype, src, dst, rows, nb);
     ctx->launches++;
     IB_CHECK_CUDA(cudaGetLastError());
     return IB_OK;

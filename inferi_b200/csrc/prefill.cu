@@ -225,13 +225,13 @@ extern "C" int32_t ib_gemm_quant(ib_ctx *ctx, void *stream, float *out_dev, cons
     IB_REQUIRE(ctx && m && out_dev && x_dev, "ib_gemm_quant: null argument");
     IB_REQUIRE(m->ctx->device == ctx->device, "ib_gemm_quant: tensor lives on device %d, context on %d", m->ctx->device, ctx->device);
     IB_REQUIRE(n >= 1, "ib_gemm_quant: no rows");
-    // Q6_K and Q8_0 matrices whose rows are not in the re-tiled layout (Q6_K rows that are no multiple of 8 blocks, rows wider than the
-    // GEMV takes): re-tiled into the scratch by every call, one read and one write of the matrix ahead of a GEMM that reads it at least once more
+    // Q6_K and Q8_0 matrices whose rows are wider than the GEMV takes are not in the re-tiled layout: re-tiled into the scratch by every
+    // call, one read and one write of the matrix ahead of a GEMM that reads it at least once more.  (Rows that the layout cannot hold, Q6_K of
+    // no multiple of 8 blocks, are refused.)
     ib_qtensor tiled = *m;
-    const bool retile = m->layout == LAYOUT_GGUF && (m->qtype == IB_Q6_K || m->qtype == IB_Q8_0) && m->cols % 256 == 0;
+    const bool retile = m->layout == LAYOUT_GGUF && (m->qtype == IB_Q6_K || m->qtype == IB_Q8_0) && m->nb % 8 == 0;
     if (retile) {
         tiled.layout = LAYOUT_SOA;
-        tiled.row_bytes = soa_row_bytes(m->qtype, m->nb);
         tiled.dev = nullptr;
     }
     if (!prefill_gemm_eligible(&tiled))

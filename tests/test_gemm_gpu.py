@@ -54,12 +54,10 @@ def test_gemm_across_chunks_of_tokens(backend, qt, rows, cols, n):
 
 
 @pytest.mark.parametrize("qt,rows,cols,n", [
-    (quant.Q6_K, 128, 256, 3), (quant.Q6_K, 256, 768, 130), (quant.Q6_K, 1280, 3072, 17), (quant.Q6_K, 128, 11008, 5), (quant.Q6_K, 128, 34816, 2),
-    (quant.Q8_0, 128, 33024, 9),
+    (quant.Q6_K, 128, 34816, 2), (quant.Q6_K, 256, 34816, 130), (quant.Q8_0, 128, 33024, 9),
 ])
 def test_gemm_takes_rows_that_no_gemv_layout_holds(backend, qt, rows, cols, n):
-    """Q6_K rows that are no multiple of 8 blocks, and rows wider than the GEMV takes: twice, as the second call finds the first one's
-    scratch, with another matrix in between."""
+    """Rows wider than the GEMV takes: twice, as the second call finds the first one's scratch, with another matrix in between."""
     x = torch.from_numpy(np.random.default_rng(n).standard_normal((n, cols)).astype(np.float32)).cuda()
     for seed in (1, 2, 1):
         blocks = quant.random_blocks(qt, rows, cols, seed=rows + cols + seed, scale=0.05)
@@ -70,6 +68,15 @@ def test_gemm_takes_rows_that_no_gemv_layout_holds(backend, qt, rows, cols, n):
         want = x.double() @ w.T
         assert float((out.double() - want).norm() / want.norm()) < 1e-5      # as above
         m.close()
+
+
+@pytest.mark.parametrize("cols", [256, 768, 3072, 33024])
+def test_gemm_rejects_rows_that_the_copies_cannot_take(backend, cols):
+    m = GpuQuantTensor(backend, quant.Q6_K, 128, cols, quant.random_blocks(quant.Q6_K, 128, cols, seed=2))     # no multiple of 8 blocks
+    with pytest.raises(InferiError) as e:
+        GemmQuant(backend).launch(torch.empty(2, 128, device="cuda"), m, torch.zeros(2, cols, device="cuda"))
+    assert e.value.code == 4
+    m.close()
 
 
 def test_gemm_rejects_shapes_outside_the_tensor_core_path(backend):
