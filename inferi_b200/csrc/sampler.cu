@@ -10,7 +10,7 @@
 //   top-p: candidates p_i >= (1 - topp) / (n - 1), sorted by descending p (stable: ascending index on ties), cut after
 //          the first prefix whose sum exceeds topp, then first i with coin * prefix_sum < running sum (sampler.rs:84-129)
 //
-// The launch is ONE thread-block cluster of 16 CTAs (8 where the device cannot place 16).  Every CTA holds a contiguous
+// The launch is ONE thread-block cluster of 16 CTAs (8 where the device cannot place 16; one CTA for small vocabularies).  Every CTA holds a contiguous
 // slice of the vocabulary in shared memory; what the CTAs have to tell one another (maximum, sum, histograms) goes
 // through distributed shared memory and the cluster barrier, so the whole of it is one launch without a round trip to
 // L2.  The work is a few passes over some hundred KB: with one CTA those passes alone took 100 us, and the sort of the
@@ -39,6 +39,9 @@ namespace cg = cooperative_groups;
 
 constexpr int SAMPLE_THREADS = 1024, SAMPLE_WARPS = SAMPLE_THREADS / 32;
 constexpr uint32_t SAMPLE_MAX_CLUSTER = 16;
+// Vocabularies up to this size are one CTA's work: its barriers are a third of a cluster's, and a pass over them is four elements a thread.
+// us per call, 1 / 16 CTAs: 512 tokens 12.4 / 20.5 (flat 20.6 / 28.7), 4096 16.4 / 20.5 (39.6 / 43.1), 8192 18.8 / 20.5, 32000 39.0 / 22.6.
+constexpr uint32_t SAMPLE_ONE_CTA = 4096;
 constexpr uint32_t SAMPLE_BINS = 2048, SAMPLE_TOP_SHIFT = 19;   // p <= 1: bits(p) >> 19 <= 0x7F0
 constexpr uint32_t SAMPLE_LIST = 4096;                          // elements of a bin that are ordered in shared memory
 constexpr uint32_t SAMPLE_SLICE_MAX = 32768;                    // floats of a slice that fit shared memory beside the rest; longer slices live in global memory
@@ -149,7 +152,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const float *__r
     const uint32_t C = cluster.num_blocks(), rank = cluster.block_rank(), tid = threadIdx.x;
     const int lane = tid & 31, warp = tid >> 5;
     SampleShared &first = *cluster.map_shared_rank(&S, 0);
-    auto barrier = [&]() { cluster.sync(); };
+    auto barrier = [&]() { if (C > 1) cluster.sync(); else __syncthreads(); };
 
     cluster.barrier_arrive();   // every CTA of the cluster runs: needed before its shared memory is written from outside
     for (uint32_t b = tid; b < SAMPLE_BINS; b += SAMPLE_THREADS) { S.lo[b] = 0u; S.hi[b] = 0u; }
@@ -249,6 +252,11 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const float *__r
     // the cluster's histogram in the first CTA: every CTA adds up its share of the bins over the CTAs
     auto gather_bins = [&]() {
         barrier();
+        if (C == 1) {
+            for (uint32_t b = tid; b < SAMPLE_BINS; b += SAMPLE_THREADS) S.tot[b] = ((unsigned long long)S.hi[b] << 32) + S.lo[b];
+            __syncthreads();
+            return;
+        }
         const uint32_t lanes = C / 2, share = SAMPLE_BINS / C, bin = rank * share + tid / lanes, r0 = tid % lanes;   // share * lanes == SAMPLE_THREADS
         unsigned long long v = 0ull;
 #pragma unroll
@@ -445,9 +453,9 @@ int32_t launch_sample(ib_ctx *ctx, cudaStream_t s, const float *logits, uint32_t
         C = (cudaOccupancyMaxActiveClusters(&fit, sample_kernel, &cfg) == cudaSuccess && fit > 0) ? SAMPLE_MAX_CLUSTER : 8u;
         cudaGetLastError();
     }
-    const uint32_t slice = (n + C - 1) / C;
-    attr[0].val.clusterDim.x = C;
-    cfg.gridDim = dim3(C);
+    const uint32_t ctas = n <= SAMPLE_ONE_CTA ? 1u : C, slice = (n + ctas - 1) / ctas;
+    attr[0].val.clusterDim.x = ctas;
+    cfg.gridDim = dim3(ctas);
     cfg.dynamicSmemBytes = sizeof(SampleShared) + (probs ? 0 : slice * sizeof(float));
     cfg.numAttrs = pdl ? 2 : 1;
     IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, sample_kernel, logits, n, slice, temperature, topp, seed, pos_ptr, coin, probs, out, out2, pdl));

@@ -75,7 +75,7 @@ def test_sampler_matches_the_reference_algorithm(backend, n, temperature, topp):
 
 
 def test_flat_and_tied_distributions(backend):
-    """Near-uniform logits put the whole vocabulary into the nucleus (the global-memory sort path); equal probabilities
+    """Near-uniform logits put the whole vocabulary into the nucleus (one bin holds it all and is cut into finer ones); equal probabilities
     must be taken in index order (the reference's stable sort)."""
     rng = np.random.default_rng(5)
     n = 40000
@@ -87,10 +87,10 @@ def test_flat_and_tied_distributions(backend):
         assert gpu_sample(backend, tied, 1.0, 0.9, coin) == oracle.sample(tied, 1.0, 0.9, coin)[0]
 
 
-@pytest.mark.parametrize("n,step", [(4097, 0.0), (40000, 0.0), (128256, 1e-6), (262145, 0.0)])
+@pytest.mark.parametrize("n,step", [(4096, 0.0), (4096, 1e-6), (4097, 0.0), (40000, 0.0), (128256, 1e-6), (262145, 0.0)])
 def test_bins_with_more_elements_than_the_list(backend, n, step):
     """All (or all but rounding) probabilities equal: the crossing's bin overflows the list at every level and its elements are taken in index
-    order; 262145 tokens no longer fit shared memory."""
+    order; 4096 tokens are the most that one CTA takes, 262145 no longer fit shared memory."""
     logits = (np.arange(n, dtype=np.float32) % 7) * np.float32(step)
     check_many(backend, logits, 1.0, 0.9, np.float32([0.0, 0.37, 0.999999]))
 
