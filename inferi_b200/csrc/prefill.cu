@@ -124,6 +124,28 @@ __global__ void __launch_bounds__(256) prefill_finish_kernel(float *out, const P
     for (int k = 0; k < 8; k++) o[k] = v.v[k];
 }
 
+// The same, one column per thread and eight planes requested at a time: for results of few columns and dozens of planes
+__global__ void __launch_bounds__(256) prefill_finish_narrow_kernel(float *out, const PfPlanes add) {
+    pf_enter();
+    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= add.n * add.rows) return;
+    const uint32_t t = i / add.rows, r = i - t * add.rows, np = add.sk.pieces((r >> 7) * add.chunks + t / PF_CHUNK);
+    if (np == 1) return;
+    const size_t plane = (size_t)add.n * add.rows;
+    const float *p = add.planes + i;
+    float v = __ldcg(out + i);
+    uint32_t s = 1;
+    for (; s + 8 <= np; s += 8) {
+        float a[8];
+#pragma unroll
+        for (int k = 0; k < 8; k++) a[k] = __ldcg(p + (s - 1 + k) * plane);
+#pragma unroll
+        for (int k = 0; k < 8; k++) v += a[k];
+    }
+    for (; s < np; s++) v += __ldcg(p + (s - 1) * plane);
+    out[i] = v;
+}
+
 __global__ void __launch_bounds__(256) prefill_swiglu_kernel(const PfPlanes gu, __half *hi, __half *lo) {
     pf_enter();
     const uint32_t F = gu.rows / 2, per = F / 8, i = blockIdx.x * blockDim.x + threadIdx.x, t = i / per, c = (i - t * per) * 8;   // whole warps: F % 256 == 0
@@ -208,7 +230,12 @@ int32_t launch_prefill_residual(ib_ctx *ctx, cudaStream_t s, float *X, const PfP
     return pf_launch(ctx, s, prefill_residual_kernel, pf_grid((size_t)add.n * add.rows / 8), 256, X, add);
 }
 int32_t launch_prefill_finish(ib_ctx *ctx, cudaStream_t s, float *out, const PfPlanes &add) {
-    return pf_launch(ctx, s, prefill_finish_kernel, pf_grid((size_t)add.n * add.rows / 8), 256, out, add);
+    // A matrix of few rows is cut into dozens of pieces, and threads of eight columns each are then too few to bring the planes in
+    // (Q4_K 512 x 14336, 38 planes, the whole GEMM, eight columns / one: 64 tokens 42.9 / 22.8 us, 128 tokens 44.3 / 24.7,
+    // 300 tokens 43.1 / 34.3).  Where eight columns each are a CTA per SM they do as well.
+    const size_t columns = (size_t)add.n * add.rows;
+    if (prefill_max_pieces(add.sk) > 8 && columns < (size_t)8 * 256 * (uint32_t)ctx->sm_count) return pf_launch(ctx, s, prefill_finish_narrow_kernel, pf_grid(columns), 256, out, add);
+    return pf_launch(ctx, s, prefill_finish_kernel, pf_grid(columns / 8), 256, out, add);
 }
 int32_t launch_prefill_swiglu(ib_ctx *ctx, cudaStream_t s, const PfPlanes &gu, __half *hi, __half *lo) {
     return pf_launch(ctx, s, prefill_swiglu_kernel, pf_grid((size_t)((gu.n + 15) & ~15u) * gu.rows / 16), 256, gu, hi, lo);

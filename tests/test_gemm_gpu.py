@@ -37,6 +37,7 @@ def test_gemm_matches_row_by_row_gemv(backend, qt, rows, cols, n):
 @pytest.mark.parametrize("qt,rows,cols,n", [
     (quant.Q4_K, 128, 256, 129), (quant.Q5_K, 256, 512, 255), (quant.Q6_K, 128, 2048, 130), (quant.Q8_0, 384, 256, 257),   # edges of the 128-token chunks
     (quant.Q8_0, 128, 1024, 15), (quant.Q5_K, 128, 768, 17), (quant.Q6_K, 640, 4096, 1029),                                # ... of the 16-token padding, two passes
+    (quant.Q4_K, 512, 14336, 130), (quant.Q5_K, 256, 2304, 1), (quant.Q8_0, 1024, 4096, 290), (quant.Q8_0, 1024, 4096, 300),   # dozens of planes, one column per thread; the result too large for that
 ])
 def test_gemm_across_chunks_of_tokens(backend, qt, rows, cols, n):
     """Every row of the result: the tokens of all chunks, and the tiles whose K range is split between CTAs."""
