@@ -154,6 +154,7 @@ __device__ __forceinline__ void attn_block(const AttnArgs &a, const void *k_cach
     }
 
     for (uint32_t base = base0; base < t1; base += ATTN_WARPS * TILE) {
+        if (a.pdl == 2 && base + ATTN_WARPS * TILE >= t1) asm volatile("griddepcontrol.launch_dependents;");
         if (!(wait_inside && base == base0)) {
 #pragma unroll
             for (int s = 0; s < STEPS; s++) {
