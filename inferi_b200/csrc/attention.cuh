@@ -1,6 +1,5 @@
-// Device side of the grouped-query decode attention: one 4-warp block of threads handles one (kv head, position slice)
-// pair.  Used by the stand-alone attention kernel (one CTA per pair) and by the whole-token kernel (four such blocks
-// per CTA, synchronised with named barriers).
+// Device side of the grouped-query decode attention: one 4-warp CTA handles one (kv head, position slice) pair.  What the general
+// kernel (attention.cu) and the one for the Llama-3 shape (attention_gqa4.cuh) share, and the general one's body.
 //
 // Semantics follow `run_cpu` of crates/inferi-shaders/src/fused_attention.rs:191-245: score = q.k / sqrt(head_size),
 // softmax over positions 0..=pos, weighted sum of V.  Cache rows are [position, kv_dim] (fused_attention.rs:107-108).
@@ -72,13 +71,11 @@ __host__ __device__ __forceinline__ void attn_split_plan(uint32_t total, uint32_
     nsplit = (total + per - 1) / per;  // every remaining split is non-empty
 }
 
-// QS = the group's query vectors are staged in shared memory (KVM * HS more floats after the block's other arrays) and
-// read per use instead of being held in registers: for callers that are short of registers.
 // One block (ATTN_THREADS threads, `tid` = 0..127, synchronised on named barrier `bar`) computes slice `split` of kv head
 // `kvh` for all KVM query heads of the group; K and V rows are read once for the group.  With more than one slice every
 // block leaves an un-normalised partial (max, sum, accumulator) and the last block of the kv head to arrive merges them:
 // no block ever waits for another.  STEPS = cache-row steps per tile kept in registers.
-template <int HS, int KVM, typename T, int STEPS, bool QS = false>
+template <int HS, int KVM, typename T, int STEPS>
 __device__ __forceinline__ void attn_block(const AttnArgs &a, const void *k_cache, const void *v_cache, uint32_t kvh, uint32_t split, uint32_t nsplit,
                                            uint32_t per, uint32_t total, int tid, int bar, float *sm, bool wait_inside = false) {
     constexpr int EPL = KvVec<T>::EPL;   // elements per 16-byte lane load
@@ -132,17 +129,11 @@ __device__ __forceinline__ void attn_block(const AttnArgs &a, const void *k_cach
         }
     }
 
-    float qr[QS ? 1 : KVM][QS ? 1 : EPL];
-    float *sm_q = reinterpret_cast<float *>(sm_last + 4);   // [KVM][HS], only with QS
-    if (QS) {
-        for (int i = tid; i < KVM * HS; i += ATTN_THREADS) sm_q[i] = __ldcg(a.q + (size_t)kvh * KVM * HS + i);
-        attn_bar(bar);
-    } else {
+    float qr[KVM][EPL];
 #pragma unroll
-        for (int m = 0; m < KVM; m++)
+    for (int m = 0; m < KVM; m++)
 #pragma unroll
-            for (int e = 0; e < EPL; e++) qr[QS ? 0 : m][QS ? 0 : e] = __ldcg(a.q + (size_t)(kvh * KVM + m) * HS + li * EPL + e);
-    }
+        for (int e = 0; e < EPL; e++) qr[m][e] = __ldcg(a.q + (size_t)(kvh * KVM + m) * HS + li * EPL + e);
 
     float M[KVM], l[KVM], acc[KVM][EPL];
 #pragma unroll
@@ -154,7 +145,6 @@ __device__ __forceinline__ void attn_block(const AttnArgs &a, const void *k_cach
     }
 
     for (uint32_t base = base0; base < t1; base += ATTN_WARPS * TILE) {
-        if (a.pdl == 2 && base + ATTN_WARPS * TILE >= t1) asm volatile("griddepcontrol.launch_dependents;");
         if (!(wait_inside && base == base0)) {
 #pragma unroll
             for (int s = 0; s < STEPS; s++) {
@@ -164,6 +154,7 @@ __device__ __forceinline__ void attn_block(const AttnArgs &a, const void *k_cach
                 vraw[s] = __ldcg(reinterpret_cast<const uint4 *>(vc + (size_t)tc * kv_dim));
             }
         }
+        if (a.pdl == 2 && base + ATTN_WARPS * TILE >= t1) asm volatile("griddepcontrol.launch_dependents;");
         float sc[STEPS][KVM];
 #pragma unroll
         for (int s = 0; s < STEPS; s++) {
@@ -174,7 +165,7 @@ __device__ __forceinline__ void attn_block(const AttnArgs &a, const void *k_cach
             for (int m = 0; m < KVM; m++) {
                 float d = 0.f;
 #pragma unroll
-                for (int e = 0; e < EPL; e++) d = fmaf(QS ? sm_q[m * HS + li * EPL + e] : qr[QS ? 0 : m][QS ? 0 : e], kf[e], d);
+                for (int e = 0; e < EPL; e++) d = fmaf(qr[m][e], kf[e], d);
 #pragma unroll
                 for (int o = LPR / 2; o; o >>= 1) d += __shfl_xor_sync(0xffffffffu, d, o);
                 sc[s][m] = valid ? d * scale : -INFINITY;

@@ -3,12 +3,12 @@
 // Replaces the reference shaders crates/inferi-shaders/src/gemv_quant_{q8_0x2,q4_k,q5_k,q6_kx2}.rs (one 32-thread
 // workgroup per 4 rows, 4-byte scattered loads) and their launcher crates/inferi/src/ops/gemv_quant.rs:183-341.
 //
-// One persistent CTA per SM, as two pipelines (one where all warps are needed for one row).  Each has:
+// One persistent CTA per SM of sixteen consumer warps, as two pipelines (one where all warps are needed for one row).  Each has:
 //  * A producer warp that streams rows from HBM into its part of a shared-memory ring with bulk asynchronous copies
 //    (cp.async.bulk, one copy per tile of contiguous row pairs, completion on an mbarrier).  It starts before the kernel
 //    waits for its predecessor (programmatic dependent launch): weights never depend on the previous kernel, so the ring
 //    fills while that kernel is still finishing.
-//  * Sixteen consumer warps split a row's columns in blocks of 256 and work on eight rows at a time.  A warp's activations - two
+//  * Its consumer warps split a row's columns in blocks of 256 and work on eight rows at a time.  A warp's activations - two
 //    int8 limbs per column, see gemv_common.cuh - stay in registers for the whole kernel as operands of integer mma, so
 //    the inner loop touches shared memory for weights and scales only (gemv_stream.cuh).
 //  * Per-warp partial row sums meet in shared memory; the epilogue warp adds them in a fixed order and runs the epilogue
@@ -28,8 +28,8 @@ namespace ib {
 
 struct StreamGeom {
     uint32_t stages, stage_bytes, act_off, part_off, bar_off;
-    // the launch's tiles in hand-out order: per segment the pairs, the pairs per tile and the tiles; bytes per pair
-    uint32_t seg_pairs[3], seg_pt[3], seg_tiles[3], seg_cost[3], total_tiles, meta_off;
+    // the launch's tiles in hand-out order: per segment the pairs, the pairs per tile and the bytes per pair
+    uint32_t seg_pairs[3], seg_pt[3], seg_cost[3], meta_off;
     uint32_t NB, CG, RG, mode;   // see Split
     uint32_t P;            // pipelines
     uint32_t ahead;        // stages: how far the first round of copies runs ahead of their arrival
@@ -545,10 +545,9 @@ int32_t launch_gemv_stream(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p
         return pt;
     };
     StreamGeom geo;
-    geo.total_tiles = 0;
-    uint32_t stage_data = 0;
+    uint32_t stage_data = 0, tiles = 0;
     for (uint32_t s = 0; s < 3; s++) {
-        geo.seg_pairs[s] = geo.seg_tiles[s] = 0;
+        geo.seg_pairs[s] = 0;
         geo.seg_pt[s] = 1;
         geo.seg_cost[s] = 16;
         const bool swiglu = p.epi == EPI_SWIGLU;
@@ -558,8 +557,7 @@ int32_t launch_gemv_stream(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p
         geo.seg_cost[s] = cost;
         geo.seg_pt[s] = pt;
         geo.seg_pairs[s] = swiglu ? p.seg[0].rows : p.seg[s].rows / 2;
-        geo.seg_tiles[s] = (geo.seg_pairs[s] + pt - 1) / pt;
-        geo.total_tiles += geo.seg_tiles[s];
+        tiles += (geo.seg_pairs[s] + pt - 1) / pt;
         if (pt * cost > stage_data) stage_data = pt * cost;
     }
     geo.stage_bytes = (stage_data + 127) & ~127u;
@@ -585,16 +583,16 @@ int32_t launch_gemv_stream(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p
     geo.bar_off = geo.part_off + S * PART_STAGE_FLOATS * 4;
     geo.meta_off = (geo.bar_off + (3 * S + 1) * 8 + 15) & ~15u;
     const size_t total = geo.meta_off + S * 16;
-    // Hand-out: launches of one segment with enough tiles per CTA give every CTA its first ring of tiles by position and let the
-    // CTAs claim the rest from a counter, in units of about UNIT_BYTES (a claim takes about as long as such a unit's copy).
+    // Hand-out: launches of one segment with enough tiles per CTA give every pipeline three quarters of its share by position and let
+    // the pipelines claim the rest from a counter, in units of about UNIT_BYTES (a claim takes about as long as such a unit's copy).
     // Everything else: static byte-balanced ranges.
     geo.unit = geo.head = 0;
     const bool single = p.epi == EPI_SWIGLU || p.nseg == 1;
     uint32_t unit = UNIT_BYTES / geo.stage_bytes;
     if (unit < 1) unit = 1;
-    if (single && geo.total_tiles >= 6 * unit * (uint32_t)grid) {
+    if (single && tiles >= 6 * unit * (uint32_t)grid) {
         geo.unit = unit;
-        geo.head = geo.total_tiles / ((uint32_t)grid * geo.P) * 3 / 4;
+        geo.head = tiles / ((uint32_t)grid * geo.P) * 3 / 4;
     }
     // the counters through which this launch's CTAs share out the tiles: consecutive launches overlap (programmatic
     // dependent launch), so they take different pairs of a small ring; the last CTA of a launch clears its pair

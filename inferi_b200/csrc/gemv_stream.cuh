@@ -1,6 +1,5 @@
-// Device-side building blocks of the streaming quantized GEMV (shared by the stand-alone GEMV kernel and the
-// whole-token kernel): mbarrier / bulk-copy wrappers with bounded waits, the byte-balanced row split, the per-format
-// 64-weight unit dot products and the row-pair epilogues.
+// Device-side building blocks of the streaming quantized GEMV (gemv_stream.cu): mbarrier / bulk-copy wrappers with bounded
+// waits, the byte-balanced row split, the per-format 64-weight unit dot products and the row-pair epilogues.
 #pragma once
 
 #include "gemv_common.cuh"
@@ -164,7 +163,6 @@ struct Share {
     uint32_t nseg;
     __device__ __forceinline__ uint32_t a(uint32_t s) const { return s == 0 ? a0 : (s == 1 ? a1 : a2); }
     __device__ __forceinline__ uint32_t b(uint32_t s) const { return s == 0 ? b0 : (s == 1 ? b1 : b2); }
-    __device__ __forceinline__ uint32_t cost(uint32_t s) const { return s == 0 ? c0 : (s == 1 ? c1 : c2); }
     __device__ __forceinline__ uint32_t pt(uint32_t s) const { return s == 0 ? t0 : (s == 1 ? t1 : t2); }
 };
 

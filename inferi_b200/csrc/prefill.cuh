@@ -7,7 +7,9 @@
 namespace ib {
 
 constexpr uint32_t PF_CHUNK = 128;             // tokens per GEMM tile (the N of the MMA)
-constexpr uint32_t PREFILL_MAX_TOKENS = 1024;  // tokens that go through the layers together; longer prompts go in passes
+// Tokens that go through the layers together; longer prompts go in passes.  Two passes cost hardly more than a pass of twice the length would
+// (two layers of the 8B shapes: 1024 tokens 2.45 ms, 2000 tokens 5.28), and the buffers grow by 41 MB per 128 tokens of these shapes.
+constexpr uint32_t PREFILL_MAX_TOKENS = 1024;
 constexpr uint32_t PF_MAX_SEGS = 3;            // matrices of one GEMM launch
 
 // How a prefill GEMM's work is handed out: the units (128-row tile, chunk of 128 tokens, 256-column block), in that order, are
