@@ -20,7 +20,7 @@ constexpr int ATTN_STEPS = 8;              // row steps per tile kept in registe
 template <int HS, int KVM, typename T>
 __global__ void __launch_bounds__(ATTN_THREADS) attn_kernel(const AttnArgs a) {
     __shared__ float sm[attn_block_smem_floats(HS, KVM)];
-    if (a.pdl == 1) asm volatile("griddepcontrol.launch_dependents;");   // (2: behind the rows, see attn_overlaps)
+    if (a.pdl == 1) asm volatile("griddepcontrol.launch_dependents;");   // (2: with the last rows, attn_block)
     if (a.pdl == 2) asm volatile("griddepcontrol.wait;" ::: "memory");
     // The position was written by the end of the previous token, many kernels ago, and not by the predecessor (which
     // only waits for its own predecessor after it has let this kernel start): it can be read before the wait.
@@ -48,15 +48,6 @@ uint32_t attn_max_splits(const ib_ctx *ctx, const ib_attn_params &p) {
     return s;
 }
 
-// Whether a launch may start before its predecessor has ended.  In the token graph always (its predecessor holds whole SMs).  Behind
-// any kernel (pdl 2) only where its CTAs need no more than one slot per SM: a grid of one wave that is placed while another kernel still holds some of the slots ends up unevenly spread and takes longer than the start it saved (us per
-// launch back to back, early against not: 32 kv heads of 128, f32, 3000 positions 22.5 / 17.2; 8 of 64 with 2 query heads, 16384 positions
-// 20.5 / 18.1; 1 of 128 with 4, 8192 positions 23.8 / 21.6).  Its successor is let in with the last of the rows, and not ahead of them, for the same
-// reason: between an add and a 4096 x 4096 product of the op API the sequence is 1.02 times as fast as with both early.
-static bool attn_overlaps(const ib_ctx *ctx, const AttnArgs &args, dim3 grid) {
-    return args.pdl == 1 || (args.pdl == 2 && grid.x * grid.y <= (uint32_t)ctx->sm_count);
-}
-
 template <int HS, int KVM, typename T>
 static int32_t launch_t(ib_ctx *ctx, cudaStream_t s, const AttnArgs &args, dim3 grid) {
     cudaLaunchConfig_t cfg = {};
@@ -67,7 +58,7 @@ static int32_t launch_t(ib_ctx *ctx, cudaStream_t s, const AttnArgs &args, dim3 
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = attn_overlaps(ctx, args, grid) ? 1 : 0;
+    cfg.numAttrs = args.pdl ? 1 : 0;
     IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, attn_kernel<HS, KVM, T>, args));
     ctx->launches++;
     return IB_OK;
@@ -138,7 +129,7 @@ static int32_t launch_gqa4(ib_ctx *ctx, cudaStream_t s, const AttnArgs &args, di
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = attn_overlaps(ctx, args, grid) ? 2 : 1;
+    cfg.numAttrs = args.pdl ? 2 : 1;
     IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, attn_gqa4_kernel<HS, REGIME>, args));
     ctx->launches++;
     return IB_OK;
