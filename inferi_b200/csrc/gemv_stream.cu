@@ -19,6 +19,11 @@
 // last tile's epilogue, one after the other - which is most of a short one (4096 x 4096 Q4_K, 9.4 MB: 4.7 us).  Byte dot products on
 // lanes that each own 64 columns, one producer and one epilogue warp: 15.5 and 5.8 us; there a tile took about 0.9 us whatever its size
 // (a producer's or an epilogue's latency per tile), and the dot products as long as HBM.
+// A launch starts with its code and its parameters in no near cache, so what it runs first is kept short: the split is multiplications by
+// constants of the host, the producers make their own barriers ready and copy without meeting the other warps, every line of the
+// parameters is touched by another warp at once, and what only some launches do (arg-max, the ranks' exchange) lies out of the way.  From
+// a CTA's start to its first copy 1.1 us instead of 1.8-2.2, and decoding 21.4 instead of 23.2 ms per 16 tokens of an 8B model, 13.1 instead of
+// 14.4 ms per 32 of a 1B model.
 // Every wait on an mbarrier is bounded; a wait that gives up raises the context's error word and carries on.
 #include "gemv_stream.cuh"
 
@@ -28,13 +33,16 @@ namespace ib {
 
 
 struct StreamGeom {
+    ShareGeom share;       // the pipelines' byte-balanced ranges
+    uint32_t nseg;         // 1 where gate and up rows travel together
     uint32_t stages, stage_bytes, act_off, part_off, bar_off;
     // the launch's tiles in hand-out order: per segment the pairs, the pairs per tile and the bytes per pair
     uint32_t seg_pairs[3], seg_pt[3], seg_cost[3], meta_off;
     uint32_t NB, CG, RG, mode;   // see Split
     uint32_t P;            // pipelines
     uint32_t ahead;        // stages: how far the first round of copies runs ahead of their arrival
-    uint32_t slices;       // lanes of the epilogue warp that share the addition of a pair's partial sums
+    uint32_t width_log2;   // lanes of the epilogue warp: groups of so many (log2) pairs share the addition of the pairs' partial sums
+    uint32_t cg_inv;       // 2^16 / CG, rounded up
     uint32_t unit;   // tiles are claimed from a counter, so many at a time; 0: every CTA streams its own byte-balanced range of pairs
     uint32_t head;   // counter hand-out: so many tiles of every pipeline are its own by position
 };
@@ -97,7 +105,8 @@ __device__ __forceinline__ void consume_tiles(const GemvParams &p, const Consume
         });
     };
     uint32_t cur_type = ONE_TYPE ? QT : p.seg[0].qtype, cur_s = 0, stride = (uint32_t)p.seg[0].row_bytes;
-    enter(cur_type, stride);
+    if (ONE_TYPE) enter(cur_type, stride);   // (rows of one format and width are equally long in every segment)
+    bool fresh = !ONE_TYPE;
     const uint32_t together = FOUR ? 4 : 8, half = together / 2;   // rows at a time; gate/up: gate rows, then their up rows
     const uint32_t add = swiglu ? half : together, row_of = g & (add - 1), b_off = swiglu && (g & half) ? c.pt * stride : 0;   // the up rows follow a full tile's gate rows
     const uint32_t part0 = c.part + 4 * (swiglu ? 2 * row_of + ((g & half) ? 1 : 0) : row_of), out_step = 4 * together;
@@ -106,6 +115,10 @@ __device__ __forceinline__ void consume_tiles(const GemvParams &p, const Consume
     uint32_t st = c.stream, par = 0, ring = c.ring;   // ring: address of stage st
 #pragma unroll 1
     for (;;) {
+        if (!ONE_TYPE && fresh) {
+            enter(cur_type, stride);
+            fresh = false;
+        }
         if (!mbar_wait(c.bar0 + 8 * st, par, p.err, 1, p.wait_ns)) return;   // the error word is raised; give up on this CTA's rows
         const uint4 tm = lds128(c.meta + 16 * st);
         const uint32_t n = tm.z;
@@ -113,13 +126,13 @@ __device__ __forceinline__ void consume_tiles(const GemvParams &p, const Consume
             if (c.lane == 0) mbar_arrive(c.bar0 + 8 * (2 * c.S + st));
             break;
         }
-        if (tm.x != cur_s) {
+        if (!ONE_TYPE && tm.x != cur_s) {
             cur_s = tm.x;
-            const uint32_t qtype = ONE_TYPE ? QT : (cur_s == 1 ? p.seg[1].qtype : p.seg[2].qtype);
-            const uint32_t rb = (uint32_t)(cur_s == 1 ? p.seg[1].row_bytes : p.seg[2].row_bytes);
-            if (qtype != cur_type || rb != stride) enter(qtype, rb);
+            const uint32_t qtype = cur_s == 1 ? p.seg[1].qtype : p.seg[2].qtype;
+            fresh = qtype != cur_type;
             cur_type = qtype;
-            stride = rb;
+            stride = (uint32_t)(cur_s == 1 ? p.seg[1].row_bytes : p.seg[2].row_bytes);
+            if (fresh) continue;   // (the tile is still there for the second wait)
         }
         const uint32_t base = ring + b_off, rows = swiglu ? n : 2 * n;
         uint32_t out = part0 + st * (4 * PART_STAGE_FLOATS);
@@ -179,8 +192,8 @@ __device__ __forceinline__ void consume_tiles(const GemvParams &p, const Consume
 // row pairs, one pair per lane.
 __device__ __forceinline__ void finish_tiles(const GemvParams &p, const StreamGeom &geo, uint32_t part, uint32_t meta, uint32_t bar0, uint32_t pipe,
                                              uint32_t lane, const float *red, unsigned long long &best) {
-    const uint32_t S = geo.stages, CG = geo.CG, slices = geo.slices, width = 32 / slices;   // lanes: `slices` groups of `width` pairs
-    const uint32_t pr = lane % width, slice = lane / width;
+    const uint32_t S = geo.stages, CG = geo.CG, width = 1u << geo.width_log2, slices = 32u >> geo.width_log2;   // lanes: `slices` groups of `width` pairs
+    const uint32_t pr = lane & (width - 1), slice = lane >> geo.width_log2;
     uint32_t st = pipe, par = 0;
     float rms = 1.0f;
     if (p.norm_w) {
@@ -233,6 +246,71 @@ __device__ __forceinline__ void finish_tiles(const GemvParams &p, const StreamGe
     }
 }
 
+// Tensor parallel: the previous row-split GEMV of every rank leaves its partial sums in this rank's slots.  The sum (x + the partials
+// in rank order, so every rank gets the same bits) is formed once per rank: an epilogue warp adds up the groups of 32 columns that
+// fall to its CTA and stores them as the new residual stream; the consumer warps of all CTAs wait until every group is there.  (Each
+// CTA adding up the whole vector for itself was N x 16 KiB of L2 reads per CTA: at 8 ranks more than its share of the weights.)
+__device__ __noinline__ void reduce_partials(const GemvParams &p, uint32_t lane) {
+    const uint32_t tag = (*p.epoch_ptr) * p.xchg_per_epoch + p.reduce_use;
+    uint32_t cnt = 0;
+#pragma unroll 1
+    for (uint32_t grp = blockIdx.x; grp < p.cols / 32; grp += gridDim.x) {
+        const uint32_t col = grp * 32 + lane;
+        float v = __ldcg(p.x + col);
+        // on a time-out the error word is raised and the launch runs to its end on whatever is there
+#pragma unroll 1
+        for (uint32_t rk = 0; rk < p.tp; rk++) v += wait_tagged(p.reduce_src + (size_t)rk * p.cols + col, tag, p.err, p.wait_ns);
+        p.x_out[col] = v;
+        cnt++;
+    }
+    __threadfence();
+    __syncwarp();
+    if (lane == 0 && cnt) asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p.reduce_done), "r"(cnt) : "memory");
+}
+
+// EPI_ARGMAX: `best` of an epilogue warp's lanes becomes its pipeline's candidate; the last of the launch's `slots` pipelines to arrive
+// folds all of them (none waits for another).
+__device__ __noinline__ void finish_argmax(const GemvParams &p, unsigned long long best, uint32_t slot, uint32_t slots, uint32_t lane) {
+#pragma unroll 1
+    for (int o = 16; o; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
+    uint32_t last = 0;
+    if (lane == 0) {
+        p.argmax_slots[slot] = best;
+        __threadfence();
+        last = (atomicAdd(p.argmax_counter, 1u) == slots - 1) ? 1u : 0u;
+    }
+    last = __shfl_sync(0xffffffffu, last, 0);
+    if (!last) return;
+    __threadfence();
+    unsigned long long b = 0ull;
+    for (uint32_t i = lane; i < slots; i += 32) b = max(b, __ldcg(p.argmax_slots + i));
+#pragma unroll 1
+    for (int o = 16; o; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
+    if (lane == 0) {
+        *p.argmax_out = 0xFFFFFFFFu - (uint32_t)(b & 0xFFFFFFFFull);
+        *p.argmax_counter = 0u;
+        if (p.tp > 1) {
+            // sharded vocabulary: every rank gets this rank's candidate; the end-of-token kernel folds them
+#pragma unroll 1
+            for (uint32_t rk = 0; rk < p.tp; rk++) *p.amax_dst[rk] = b;
+            __threadfence_system();
+#pragma unroll 1
+            for (uint32_t rk = 0; rk < p.tp; rk++) atomicAdd_system(p.amax_flag[rk], 1u);
+        }
+    }
+}
+
+// One 4-byte word of every 64 bytes of the launch's parameters, each by another warp: a launch's parameters are in no cache when it
+// starts, and a warp that comes to them one after the other waits for every line.
+__device__ __forceinline__ void touch_parameters(const GemvParams &p, const StreamGeom &geo, uint32_t warp) {
+    constexpr uint32_t LP = (sizeof(GemvParams) + 63) / 64, LG = (sizeof(StreamGeom) + 63) / 64;
+    static_assert(LP + LG <= STREAM_THREADS / 32, "a warp per line");
+    uint32_t v = 0;
+    if (warp < LP) v = reinterpret_cast<const uint32_t *>(&p)[16 * warp];
+    else if (warp < LP + LG) v = reinterpret_cast<const uint32_t *>(&geo)[16 * (warp - LP)];
+    asm volatile("" ::"r"(v));
+}
+
 // ---- the kernel ----
 // Shared-memory barriers: full[S] (the producer's expect_tx arrival + the copy's bytes), empty[S] (one arrival: the
 // epilogue warp has read the stage's partials, which implies that every consumer warp is done with its weights),
@@ -240,29 +318,30 @@ __device__ __forceinline__ void finish_tiles(const GemvParams &p, const StreamGe
 // One instance per weight format (or format pair); what the launch does with the row sums is a run-time switch in the
 // epilogue warp, so that the launches of a token graph share their code.
 template <uint32_t QT, uint32_t MODE>
-__global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const GemvParams p, const StreamGeom geo) {
+__global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const __grid_constant__ GemvParams p, const __grid_constant__ StreamGeom geo) {
     extern __shared__ __align__(128) uint8_t smem[];
     __shared__ float red[PACK_THREADS / 32 + 1];
     __shared__ uint4 zeros;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) zeros = make_uint4(0, 0, 0, 0);
+    constexpr int BAR_START = 2;   // named barrier: the mbarriers are ready
 
     uint8_t *act_sm = smem + geo.act_off;
     const uint32_t part = smem_u32(smem + geo.part_off);                        // [stages][CW][2 * PT_MAX] floats
     const uint32_t bar0 = smem_u32(smem + geo.bar_off);                         // full[stages], empty[stages], done[stages]
     const uint32_t S = geo.stages;
-
     const uint32_t CG = geo.CG, RG = geo.RG, active = CG * RG;   // consumer warps with work
 
-    if (threadIdx.x <= 3 * S) {
-        const uint32_t which = threadIdx.x / S;
-        mbar_init(bar0 + 8 * threadIdx.x, which == 2 ? CG : (which == 3 ? (uint32_t)CW : 1u));
-        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    }
-    __syncthreads();
-    if (p.pdl) asm volatile("griddepcontrol.launch_dependents;");
-
     if (warp >= W_PRODUCER && warp < W_EPILOGUE) {
+        // A pipeline's producer makes its stages' barriers ready and goes on to its first copies; the other warps wait for both producers.
+        if ((uint32_t)lane < S && (lane & (geo.P - 1)) == warp - W_PRODUCER) {
+            mbar_init(bar0 + 8 * lane, 1);
+            mbar_init(bar0 + 8 * (S + lane), 1);
+            mbar_init(bar0 + 8 * (2 * S + lane), CG);
+        }
+        if (lane == 31 && warp == W_PRODUCER) mbar_init(bar0 + 8 * (3 * S), CW);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        __syncwarp();
+        asm volatile("bar.arrive %0, %1;" ::"r"(BAR_START), "r"(STREAM_THREADS) : "memory");
         // ================= producer warp: picks tiles and streams them =================
         // With many tiles per CTA they are handed out through a counter in global memory, so that a CTA which starts late
         // (its SM was the last to be freed by the previous kernel) or runs slowly takes fewer of them.  With few tiles per
@@ -285,7 +364,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const Ge
             held = geo.head;
             t = me * held;
         } else {
-            make_share(p, geo.seg_pt, pipes, me, sh);
+            make_share(geo.share, geo.seg_pairs, geo.seg_pt, geo.nseg, me, sh);
             tc.init(sh);
         }
         uint32_t cost = swiglu ? (uint32_t)p.seg[0].row_bytes : geo.seg_cost[0], cost_b = (uint32_t)p.seg[1].row_bytes, cur = 0;
@@ -324,7 +403,7 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const Ge
                     cost = cur == 1 ? geo.seg_cost[1] : geo.seg_cost[2];
                     w = cur == 1 ? p.seg[1].w : p.seg[2].w;
                 }
-                asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the consumers' reads of the slot come first
+                if (!first_round) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");   // the consumers' reads of the slot come first
                 const uint32_t ba = n * cost, bb = swiglu ? n * cost_b : 0u, dst = ring + st * geo.stage_bytes;
                 mbar_expect_tx(full, ba + bb);
                 bulk_g2s(dst, w + (size_t)tm.y * cost, ba, full, policy);
@@ -353,70 +432,27 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const Ge
         return;
     }
 
+    touch_parameters(p, geo, warp);
+    if (threadIdx.x == 0) zeros = make_uint4(0, 0, 0, 0);
+    named_barrier(BAR_START, STREAM_THREADS);
+
     if (warp >= W_EPILOGUE) {
         // ================= epilogue warp =================
+        if (p.pdl) asm volatile("griddepcontrol.launch_dependents;");
         const uint32_t pipe = warp - W_EPILOGUE;
         if (pipe >= geo.P) return;
         // outputs (and the residual it reads) are touched by the previous kernels of the stream: wait for them like the consumers do
         if (p.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
-        if (p.reduce_src && pipe == 0) {
-            // Tensor parallel: the previous row-split GEMV of every rank leaves its partial sums in this rank's slots.  The sum
-            // (x + the partials in rank order, so every rank gets the same bits) is formed once per rank: this warp adds up
-            // the groups of 32 columns that fall to its CTA and stores them as the new residual stream; the consumer warps of
-            // all CTAs wait until every group is there.  (Each CTA adding up the whole vector for itself was N x 16 KiB of L2
-            // reads per CTA: at 8 ranks more than its share of the weights.)
-            const uint32_t tag = (*p.epoch_ptr) * p.xchg_per_epoch + p.reduce_use;
-            uint32_t cnt = 0;
-            for (uint32_t grp = blockIdx.x; grp < p.cols / 32; grp += gridDim.x) {
-                const uint32_t col = grp * 32 + lane;
-                float v = __ldcg(p.x + col);
-                // on a time-out the error word is raised and the launch runs to its end on whatever is there
-                for (uint32_t rk = 0; rk < p.tp; rk++) v += wait_tagged(p.reduce_src + (size_t)rk * p.cols + col, tag, p.err, p.wait_ns);
-                p.x_out[col] = v;
-                cnt++;
-            }
-            __threadfence();
-            __syncwarp();
-            if (lane == 0 && cnt) asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(p.reduce_done), "r"(cnt) : "memory");
-        }
-        const uint32_t epis = geo.P;   // epilogue warps at work
+        if (p.reduce_src && pipe == 0) reduce_partials(p, lane);
         unsigned long long best = 0ull;
         finish_tiles(p, geo, part, smem_u32(smem + geo.meta_off), bar0, pipe, lane, red, best);
-        if (p.epi == EPI_ARGMAX) {
-#pragma unroll
-            for (int o = 16; o; o >>= 1) best = max(best, __shfl_xor_sync(0xffffffffu, best, o));
-            uint32_t last = 0;
-            if (lane == 0) {
-                p.argmax_slots[blockIdx.x * epis + pipe] = best;
-                __threadfence();
-                last = (atomicAdd(p.argmax_counter, 1u) == gridDim.x * epis - 1) ? 1u : 0u;
-            }
-            last = __shfl_sync(0xffffffffu, last, 0);
-            if (last) {
-                // the last pipeline to arrive folds all candidates; no CTA waits for another
-                __threadfence();
-                unsigned long long b = 0ull;
-                for (uint32_t i = lane; i < gridDim.x * epis; i += 32) b = max(b, __ldcg(p.argmax_slots + i));
-#pragma unroll
-                for (int o = 16; o; o >>= 1) b = max(b, __shfl_xor_sync(0xffffffffu, b, o));
-                if (lane == 0) {
-                    *p.argmax_out = 0xFFFFFFFFu - (uint32_t)(b & 0xFFFFFFFFull);
-                    *p.argmax_counter = 0u;
-                    if (p.tp > 1) {
-                        // sharded vocabulary: every rank gets this rank's candidate; the end-of-token kernel folds them
-                        for (uint32_t rk = 0; rk < p.tp; rk++) *p.amax_dst[rk] = b;
-                        __threadfence_system();
-                        for (uint32_t rk = 0; rk < p.tp; rk++) atomicAdd_system(p.amax_flag[rk], 1u);
-                    }
-                }
-            }
-        }
+        if (p.epi == EPI_ARGMAX) finish_argmax(p, best, blockIdx.x * geo.P + pipe, gridDim.x * geo.P, lane);
         return;
     }
 
     // ================= consumer warps =================
     Consumer c;
-    const uint32_t cg = warp % CG, stream = warp / CG, blocks = p.cols / 256;
+    const uint32_t stream = (warp * geo.cg_inv) >> 16, cg = warp - stream * CG, blocks = p.cols / 256;
     c.zeros = smem_u32(&zeros); c.meta = smem_u32(smem + geo.meta_off); c.bar0 = bar0; c.S = S; c.lane = lane;
     c.part = part + 4 * (cg * 2 * PT_MAX);
     c.stream = stream; c.RG = RG; c.pt = geo.seg_pt[0];
@@ -427,20 +463,13 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const Ge
     const Act A{act_sm, p.cols};
     float4 norm_g[2];
     pack_prefetch_norm8(p.norm_w, p.cols, norm_g);   // weights: fetched while the previous kernel is still running
-    {
-        // The launch parameters the tile loop reads, touched while the previous kernel is still running: their first read
-        // misses the constant cache, and that round trip would otherwise sit between the activations and the first tile.
-        const uint32_t touch = (uint32_t)p.seg[0].row_bytes ^ (uint32_t)p.seg[1].row_bytes ^ (uint32_t)p.seg[2].row_bytes ^ p.seg[0].qtype ^
-                               p.seg[1].qtype ^ p.seg[2].qtype ^ p.epi ^ (uint32_t)p.wait_ns ^ (uint32_t)(uintptr_t)p.err;
-        asm volatile("" ::"r"(touch));
-    }
     if (p.pdl) asm volatile("griddepcontrol.wait;" ::: "memory");
     if (p.reduce_src) {
         // tensor parallel: the reduced residual stream is complete once the epilogue warps of all CTAs have stored their groups
         if (threadIdx.x == 0) wait_counter_gpu(p.reduce_done, ((*p.epoch_ptr) * p.xchg_per_epoch + p.reduce_use) * (p.cols / 32), p.err, 7, p.wait_ns);
         named_barrier(1, PACK_THREADS);
     }
-    pack_stream(act_sm, p.cols, p.reduce_src ? p.x_out : p.x, p.norm_w, red, bar0 + 8 * (3 * S), norm_g);
+    pack_stream<MODE == ROWS8 ? 1 : 4>(act_sm, p.cols, p.reduce_src ? p.x_out : p.x, p.norm_w, red, bar0 + 8 * (3 * S), norm_g);
     if ((uint32_t)warp < active) consume_tiles<QT, MODE>(p, c, A);
 }
 
@@ -561,6 +590,14 @@ int32_t launch_gemv_stream(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p
         tiles += (geo.seg_pairs[s] + pt - 1) / pt;
         if (pt * cost > stage_data) stage_data = pt * cost;
     }
+    uint32_t total16 = 0;
+    for (uint32_t s = 0; s < 3; s++) {
+        geo.share.start[s] = total16;
+        geo.share.cost16[s] = geo.seg_cost[s] / 16;
+        geo.share.inv[s] = (uint32_t)(0xFFFFFFFFull / geo.share.cost16[s] + 1);
+        total16 += geo.seg_pairs[s] * geo.share.cost16[s];
+    }
+    geo.nseg = p.epi == EPI_SWIGLU ? 1u : p.nseg;
     geo.stage_bytes = (stage_data + 127) & ~127u;
     uint32_t S = (uint32_t)(room / (geo.stage_bytes + per_stage));
     if (S > MAX_STAGES) S = MAX_STAGES;
@@ -575,7 +612,11 @@ int32_t launch_gemv_stream(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p
     uint32_t most = geo.seg_pt[0] > geo.seg_pt[1] ? geo.seg_pt[0] : geo.seg_pt[1], width = 1;
     most = geo.seg_pt[2] > most ? geo.seg_pt[2] : most;
     while (width < most) width *= 2;
-    geo.slices = 32 / width;
+    geo.width_log2 = 0;
+    while ((1u << geo.width_log2) < width) geo.width_log2++;
+    geo.cg_inv = (65536 + split.CG - 1) / split.CG;
+    const uint32_t pipes = (uint32_t)grid * geo.P;
+    geo.share.scale = (((uint64_t)total16 << 32) + pipes - 1) / pipes;
     geo.ahead = (AHEAD_BYTES / geo.stage_bytes) / geo.P * geo.P;
     if (geo.ahead < geo.P) geo.ahead = geo.P;
     geo.stages = S;

@@ -55,28 +55,6 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
         if (mbar_try_wait(bar, parity)) return true;
     return mbar_wait_long(bar, parity, err, code, limit_ns);
 }
-// ---- waits on words that another GPU (or another CTA) writes.  Counters only grow; a reader waits until the counter has
-// reached the value that the current use implies.  Bounded like every other wait here. ----
-__device__ __forceinline__ uint32_t ld_acquire_sys(const uint32_t *p) {
-    uint32_t v;
-    asm volatile("ld.acquire.sys.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-    return v;
-}
-__device__ __forceinline__ bool wait_counter(const uint32_t *flag, uint32_t target, uint32_t *err, uint32_t code, unsigned long long limit_ns) {
-    if ((int32_t)(ld_acquire_sys(flag) - target) >= 0) return true;
-    const unsigned long long t0 = global_ns();
-    for (;;) {
-        for (int i = 0; i < 64; i++)
-            if ((int32_t)(ld_acquire_sys(flag) - target) >= 0) return true;
-        if (global_ns() - t0 > limit_ns) break;
-    }
-    if (err) {
-        *(volatile uint32_t *)err = code;
-        __threadfence_system();
-    }
-    return false;
-}
-
 // A tagged word of the tensor-parallel exchange: waits (bounded) until the word carries `tag`, returns its value.
 __device__ __forceinline__ float wait_tagged(const uint2 *w, uint32_t tag, uint32_t *err, unsigned long long limit_ns) {
     uint2 v;
@@ -84,6 +62,7 @@ __device__ __forceinline__ float wait_tagged(const uint2 *w, uint32_t tag, uint3
     if (v.y != tag) {
         const unsigned long long t0 = global_ns();
         for (;;) {
+#pragma unroll 1
             for (int i = 0; i < 64 && v.y != tag; i++) asm volatile("ld.relaxed.sys.global.v2.u32 {%0,%1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(w) : "memory");
             if (v.y == tag) break;
             if (global_ns() - t0 > limit_ns) {
@@ -108,6 +87,7 @@ __device__ __forceinline__ bool wait_counter_gpu(const uint32_t *flag, uint32_t 
     if ((int32_t)(ld_acquire_gpu(flag) - target) >= 0) return true;
     const unsigned long long t0 = global_ns();
     for (;;) {
+#pragma unroll 1
         for (int i = 0; i < 64; i++)
             if ((int32_t)(ld_acquire_gpu(flag) - target) >= 0) return true;
         if (global_ns() - t0 > limit_ns) break;
@@ -158,7 +138,6 @@ __device__ __forceinline__ uint32_t lds16(uint32_t a) {
 // (three scalar sets instead of arrays: indexing them with a run-time segment number would put them in local memory)
 struct Share {
     uint32_t a0, a1, a2, b0, b1, b2;   // pair range per segment
-    uint32_t c0, c1, c2;               // bytes per pair
     uint32_t t0, t1, t2;               // pairs per tile
     uint32_t nseg;
     __device__ __forceinline__ uint32_t a(uint32_t s) const { return s == 0 ? a0 : (s == 1 ? a1 : a2); }
@@ -166,42 +145,34 @@ struct Share {
     __device__ __forceinline__ uint32_t pt(uint32_t s) const { return s == 0 ? t0 : (s == 1 ? t1 : t2); }
 };
 
-// all byte counts in units of 16 bytes so that the arithmetic stays in 32 bits (64-bit divisions cost ~0.2 us each)
-__device__ __forceinline__ void share_range(uint32_t lo, uint32_t hi, uint32_t start, uint32_t cost16, uint32_t pairs, uint32_t &a, uint32_t &b) {
-    const uint32_t x = lo > start ? (lo - start + cost16 - 1) / cost16 : 0;
-    const uint32_t y = hi > start ? (hi - start + cost16 - 1) / cost16 : 0;
-    a = x > pairs ? pairs : x;
-    b = y > pairs ? pairs : y;
+// What the split needs, from the host: nothing here divides (a handful of 32-bit divisions at its start cost every launch a microsecond
+// before its first copy).  All byte counts are in units of 16 bytes.
+struct ShareGeom {
+    uint64_t scale;        // total / pipelines in units of 2^-32, rounded up
+    uint32_t start[3];     // where a segment begins in the launch's bytes
+    uint32_t cost16[3];    // bytes per pair
+    uint32_t inv[3];       // 2^32 / cost16, rounded up
+};
+// The first pair that belongs to the part of the launch behind byte `at`.  Neighbours call it with the same `at`, so their ranges meet
+// whatever the product's rounding does; it never decreases, gives 0 at the segment's start and all pairs at its end.
+__host__ __device__ __forceinline__ uint32_t share_pair(uint32_t at, uint32_t start, uint32_t cost16, uint32_t inv, uint32_t pairs) {
+    if (at <= start) return 0;
+    const uint32_t n = (uint32_t)(((uint64_t)(at - start + cost16 - 1) * inv) >> 32);
+    return n < pairs ? n : pairs;
 }
-
-// `swiglu`: gate and up rows travel together (one "pair" = gate row r + up row r).  `sources`/`me`: the CTAs sharing the
-// work and this CTA's index among them.
-__device__ __forceinline__ void make_share_rt(bool swiglu, uint32_t nseg, uint32_t rows0, uint32_t rows1, uint32_t rows2, uint32_t rb0, uint32_t rb1,
-                                              uint32_t rb2, const uint32_t (&pt)[3], uint32_t G, uint32_t me, Share &sh) {
-    uint32_t n0, n1 = 0, n2 = 0;
-    sh.nseg = swiglu ? 1u : nseg;
-    sh.c1 = sh.c2 = 16;
-    if (swiglu) { n0 = rows0; sh.c0 = rb0 + rb1; }
-    else {
-        n0 = rows0 / 2; sh.c0 = 2 * rb0;
-        if (sh.nseg > 1) { n1 = rows1 / 2; sh.c1 = 2 * rb1; }
-        if (sh.nseg > 2) { n2 = rows2 / 2; sh.c2 = 2 * rb2; }
-    }
-    const uint32_t k0 = sh.c0 / 16, k1 = sh.c1 / 16, k2 = sh.c2 / 16;
-    const uint32_t s1 = n0 * k0, s2 = s1 + n1 * k1, total = s2 + n2 * k2;
-    const uint32_t q = total / G, r = total % G;
-    const uint32_t lo = q * me + r * me / G, hi = q * (me + 1) + r * (me + 1) / G;
-    share_range(lo, hi, 0, k0, n0, sh.a0, sh.b0);
-    share_range(lo, hi, s1, k1, n1, sh.a1, sh.b1);
-    share_range(lo, hi, s2, k2, n2, sh.a2, sh.b2);
+__host__ __device__ __forceinline__ uint32_t share_byte(uint64_t scale, uint32_t me) { return (uint32_t)((me * scale) >> 32); }
+__device__ __forceinline__ void make_share(const ShareGeom &g, const uint32_t (&pairs)[3], const uint32_t (&pt)[3], uint32_t nseg, uint32_t me, Share &sh) {
+    const uint32_t lo = share_byte(g.scale, me), hi = share_byte(g.scale, me + 1);
+    sh.nseg = nseg;
+    sh.a0 = share_pair(lo, g.start[0], g.cost16[0], g.inv[0], pairs[0]);
+    sh.b0 = share_pair(hi, g.start[0], g.cost16[0], g.inv[0], pairs[0]);
+    sh.a1 = share_pair(lo, g.start[1], g.cost16[1], g.inv[1], pairs[1]);
+    sh.b1 = share_pair(hi, g.start[1], g.cost16[1], g.inv[1], pairs[1]);
+    sh.a2 = share_pair(lo, g.start[2], g.cost16[2], g.inv[2], pairs[2]);
+    sh.b2 = share_pair(hi, g.start[2], g.cost16[2], g.inv[2], pairs[2]);
     sh.t0 = pt[0];
     sh.t1 = pt[1];
     sh.t2 = pt[2];
-}
-
-__device__ __forceinline__ void make_share(const GemvParams &p, const uint32_t (&pt)[3], uint32_t G, uint32_t me, Share &sh) {
-    make_share_rt(p.epi == EPI_SWIGLU, p.nseg, p.seg[0].rows, p.seg[1].rows, p.seg[2].rows, (uint32_t)p.seg[0].row_bytes, (uint32_t)p.seg[1].row_bytes,
-                  (uint32_t)p.seg[2].row_bytes, pt, G, me, sh);
 }
 
 struct TileCursor {
@@ -581,7 +552,6 @@ inline Split split_of(uint32_t cols, bool long8) {
 // A thread converts 8 consecutive columns at a time (a 32-column group is four lanes, a 16-column sum two): with 4096 columns
 // all 512 threads take part - with 16 columns per thread half of them did, for twice as long.  `g`: the norm weights of
 // the thread's first group, fetched ahead of the wait for the previous kernel.
-constexpr uint32_t PACK_GROUPS = 4;   // groups in flight per thread: 16384 columns
 __device__ __forceinline__ void pack_prefetch_norm8(const float *__restrict__ norm_w, uint32_t cols, float4 (&g)[2]) {
     const uint32_t grp = threadIdx.x;
     if (norm_w && grp < cols / 8) {
@@ -602,15 +572,17 @@ __device__ __forceinline__ void load_8(const float4 *p, bool whole, float4 &a, f
         b = __ldcg(p + 1);
     }
 }
+// GROUPS: groups of 8 columns per thread, all in flight at once: 4096 columns each.
+template <uint32_t GROUPS>
 __device__ __forceinline__ void pack_stream(uint8_t *smem, uint32_t cols, const float *__restrict__ x, const float *__restrict__ norm_w, float *red,
                                             uint32_t ss_bar, const float4 (&g)[2]) {
     constexpr uint32_t NT = PACK_THREADS;
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, groups = cols / 8;   // cols is a multiple of 256: whole warps
     const float4 *x4 = reinterpret_cast<const float4 *>(x), *w4 = reinterpret_cast<const float4 *>(norm_w);
     const bool whole = ((uintptr_t)x & 31) == 0;
-    float4 r[PACK_GROUPS][2];
+    float4 r[GROUPS][2];
 #pragma unroll
-    for (uint32_t i = 0; i < PACK_GROUPS; i++) {
+    for (uint32_t i = 0; i < GROUPS; i++) {
         const uint32_t grp = tid + NT * i;
         r[i][0] = r[i][1] = make_float4(0.f, 0.f, 0.f, 0.f);
         if (grp < groups) load_8(x4 + 2 * grp, whole, r[i][0], r[i][1]);
@@ -619,7 +591,7 @@ __device__ __forceinline__ void pack_stream(uint8_t *smem, uint32_t cols, const 
         // crates/inferi-shaders/src/rms_norm.rs:112-120: the sum of squares; the factor itself is applied by the epilogue warp
         float ss = 0.f;
 #pragma unroll
-        for (uint32_t i = 0; i < PACK_GROUPS; i++)
+        for (uint32_t i = 0; i < GROUPS; i++)
 #pragma unroll
             for (int j = 0; j < 2; j++) ss += (r[i][j].x * r[i][j].x + r[i][j].y * r[i][j].y) + (r[i][j].z * r[i][j].z + r[i][j].w * r[i][j].w);
 #pragma unroll
@@ -631,7 +603,7 @@ __device__ __forceinline__ void pack_stream(uint8_t *smem, uint32_t cols, const 
     }
     float *sc = reinterpret_cast<float *>(smem + ACT_LIMBS * cols), *sx16 = sc + cols / 32;
 #pragma unroll
-    for (uint32_t i = 0; i < PACK_GROUPS; i++) {
+    for (uint32_t i = 0; i < GROUPS; i++) {
         const uint32_t grp = tid + NT * i;
         if (warp * 32 + NT * i >= groups) continue;   // warp-uniform
         const bool ok = grp < groups;
@@ -675,6 +647,16 @@ __device__ __forceinline__ float2 epilogue_prefetch(const GemvParams &p, uint32_
     return make_float2(0.f, 0.f);
 }
 
+// EPI_PUSH, out of line (as what else only some launches do: a launch fetches its code from L2, and what lies between the parts that it
+// runs is fetched with them): row-split matrix of a tensor-parallel model, this rank's partial goes straight into every rank's memory
+// ({value, tag} words: see GemvParams).
+__device__ __noinline__ void push_pair(const GemvParams &p, uint32_t r0, float a, float b) {
+    const uint32_t tag = (*p.epoch_ptr) * p.xchg_per_epoch + p.push_use;
+    const uint4 w = make_uint4(__float_as_uint(a), tag, __float_as_uint(b), tag);
+#pragma unroll 1
+    for (uint32_t rk = 0; rk < p.tp; rk++) *reinterpret_cast<uint4 *>(p.push_dst[rk] + r0) = w;
+}
+
 // ---- epilogue of one row pair (run by an epilogue warp only, so the kind of epilogue is a run-time switch: one kernel
 // instance per weight format serves every role in the token graph and stays in the instruction cache) ----
 // `pre`: from epilogue_prefetch;  `pos`: the token's position (EPI_QKV).
@@ -711,11 +693,7 @@ __device__ __forceinline__ void epilogue(const GemvParams &p, uint32_t s, uint32
             else reinterpret_cast<float2 *>(cache)[off >> 1] = make_float2(a, b);
         }
     } else if (epi == EPI_PUSH) {
-        // row-split matrix of a tensor-parallel model: this rank's partial goes straight into every rank's memory
-        // ({value, tag} words: see GemvParams)
-        const uint32_t tag = (*p.epoch_ptr) * p.xchg_per_epoch + p.push_use;
-        const uint4 w = make_uint4(__float_as_uint(a), tag, __float_as_uint(b), tag);
-        for (uint32_t rk = 0; rk < p.tp; rk++) *reinterpret_cast<uint4 *>(p.push_dst[rk] + r0) = w;
+        push_pair(p, r0, a, b);
     } else if (epi == EPI_ARGMAX) {
         if (p.seg[0].out) *reinterpret_cast<float2 *>(p.seg[0].out + r0) = make_float2(a, b);
         best = max(best, max(argmax_key(a, p.row_offset + r0), argmax_key(b, p.row_offset + r0 + 1)));

@@ -46,6 +46,14 @@ def test_reference_test_shapes_and_edges(backend, qt, rows, cols):
     _shape_case(backend, qt, rows, cols)
 
 
+# the byte-balanced split of the rows over the pipelines (two per SM): fewer row pairs than pipelines, as many, one more, and a last
+# range that ends inside a tile; rows of one block and of the streaming kernel's most
+@pytest.mark.parametrize("rows", [4, 292, 588, 592, 596, 1180, 1188])
+@pytest.mark.parametrize("qt,cols", [(quant.Q4_K, 256), (quant.Q5_K, 2048), (quant.Q8_0, 16384)])
+def test_row_split(backend, qt, cols, rows):
+    _shape_case(backend, qt, rows, cols)
+
+
 # the legacy formats at the shape of the reference's tests (gemv_quant.rs:502-816: 64 x 256; Q8_K blocks span 256 columns)
 # and at a layer-sized one
 @pytest.mark.parametrize("qt,rows,cols", [(q, 64, 256) for q in LEGACY + [quant.Q8_K]] + [(q, 512, 4096) for q in LEGACY + [quant.Q8_K]])
