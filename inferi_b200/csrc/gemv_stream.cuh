@@ -236,7 +236,7 @@ IB_MMA(mma_s8, "s8")
 // Everything that depends only on the lane and the warp's first block: byte offsets inside a row, shifts, masks.
 struct LaneConst {
     uint32_t o0, o1, o2, o3;   // byte offsets inside a row
-    uint32_t sh, ma, mb, mc;   // scale extraction
+    uint32_t sh, ma, mb, mc;   // scale extraction: byte selector, masks
     uint32_t h0, h1;           // Q5_K: shifts of the fifth bits
     uint32_t sc, sx;           // shared addresses of the unit's activation scales and 16-column sums
     bool first;                // this lane's unit is in accumulator rows 0-7
@@ -246,22 +246,28 @@ struct LaneConst {
 // registers (8 rows at a time); longer rows read them from shared memory for every dot product.
 struct UnitAct { float s[4], x[4]; };
 
-// 6-bit (scale, min) pairs of sub-blocks 2t and 2t+1 of a Q4_K / Q5_K header without a branch on t (the lanes of a warp
-// differ in t): lanes with t < 2 carry masks (0x3F3F, 0, 0), the others (0, 0x3030, 0x0F0F), and both read the same three
-// half-words (crates/inferi/src/quantization.rs:394-402).
-__device__ __forceinline__ void kquant_scales_lane(const uint4 &hdr, const LaneConst &lc, uint32_t &sc2, uint32_t &m2) {
-    const uint32_t y2 = hdr.y >> lc.sh, z2 = hdr.z >> lc.sh, w2 = hdr.w >> lc.sh;   // sh = 16 * (t & 1); the masks drop the upper half
-    sc2 = (y2 & lc.ma) | ((y2 >> 2) & lc.mb) | (w2 & lc.mc);
-    m2 = (z2 & lc.ma) | ((z2 >> 2) & lc.mb) | ((w2 >> 4) & lc.mc);
+// A byte of `w` (the `sel`-th, see byte_selector) as a float: behind the exponent of 2^23 its value is the float's low bits.  A byte
+// permute and an addition on the floating-point pipe; extracting and converting it are two instructions of the integer pipe, which is
+// what the dot products are short of (it takes a warp instruction every other clock).
+constexpr uint32_t BYTE_SELECTOR = 0x7440u;   // + the byte's number
+__device__ __forceinline__ float byte_to_float(uint32_t w, uint32_t sel, float bias = 8388608.0f) {
+    return __uint_as_float(__byte_perm(w, 0x4B000000u, sel)) - bias;
+}
+
+// 6-bit (scale, min) pairs of sub-blocks 2t and 2t+1 of a Q4_K / Q5_K header, as bytes scale 2t, scale 2t+1, min 2t, min 2t+1, without a
+// branch on t (the lanes of a warp differ in t): lanes with t < 2 carry masks (0x3F.., 0, 0), the others (0, 0x30.., 0x0F..), and both
+// read the same half of the header's words (crates/inferi/src/quantization.rs:394-402).
+__device__ __forceinline__ uint32_t kquant_scales_lane(const uint4 &hdr, const LaneConst &lc) {
+    const uint32_t p = __byte_perm(hdr.y, hdr.z, lc.sh), q = __byte_perm(hdr.w, hdr.w >> 4, lc.sh);
+    return (p & lc.ma) | ((p >> 2) & lc.mb) | (q & lc.mc);
 }
 // d * (sc_lo * lo + sc_hi * hi) - dmin * (m_lo * x_lo + m_hi * x_hi) for the 64 columns of a unit of a Q4_K / Q5_K block;
 // `lo`, `hi`: the integer dot products, a.s their units, a.x the sums of the columns
 __device__ __forceinline__ float kquant_finish(const uint4 &hdr, const LaneConst &lc, float lo, float hi, const float s0, const float s1, const float x0, const float x1) {
-    uint32_t sc2, m2;
-    kquant_scales_lane(hdr, lc, sc2, m2);
+    const uint32_t k = kquant_scales_lane(hdr, lc);
     const float2 dm = __half22float2(*reinterpret_cast<const __half2 *>(&hdr.x));
-    const float a = (float)(sc2 & 0xFFu) * (s0 * lo) + (float)(sc2 >> 8) * (s1 * hi);
-    const float b = (float)(m2 & 0xFFu) * x0 + (float)(m2 >> 8) * x1;
+    const float a = byte_to_float(k, BYTE_SELECTOR) * (s0 * lo) + byte_to_float(k, BYTE_SELECTOR + 1) * (s1 * hi);
+    const float b = byte_to_float(k, BYTE_SELECTOR + 2) * x0 + byte_to_float(k, BYTE_SELECTOR + 3) * x1;
     return dm.x * a - dm.y * b;
 }
 // scales of columns 64u .. +31 and +32 .. +63 of the block and the sums of the same columns; `hi_unit`: what a high dot product counts
@@ -313,10 +319,10 @@ __device__ __forceinline__ void kquant_init(uint32_t g, uint32_t t, uint32_t str
     lc.o1 = at + quants_at + 16 * t + 64 * l.sx;
     lc.o2 = FOUR ? lc.o1 + block_bytes : at + quants_at + 16 * t + 64 * (1 - l.sx);
     lc.first = l.own;
-    lc.sh = 16 * (l.u & 1);
-    lc.ma = l.u < 2 ? 0x3F3Fu : 0u;
-    lc.mb = l.u < 2 ? 0u : 0x3030u;
-    lc.mc = l.u < 2 ? 0u : 0x0F0Fu;
+    lc.sh = l.u & 1 ? 0x7632u : 0x5410u;   // bytes 2 and 3, or 0 and 1, of either operand
+    lc.ma = l.u < 2 ? 0x3F3F3F3Fu : 0u;
+    lc.mb = l.u < 2 ? 0u : 0x30303030u;
+    lc.mc = l.u < 2 ? 0u : 0x0F0F0F0Fu;
     lc.o3 = at + 16 + 16 * (t & 1);   // Q5_K: the fifth bits of this lane's 16 columns, bit 2u / 2u+1 of a byte for unit u
     lc.h0 = 2 * (t >> 1) + 4 * l.sx;
     lc.h1 = FOUR ? lc.h0 : 2 * (t >> 1) + 4 * (1 - l.sx);
@@ -407,7 +413,7 @@ template <> struct Frag<IB_Q6_K> {
         lc.o1 = grp + 1024 + 64 * bb + 8 * t + (FOUR ? 32 * l.sx : 0);
         lc.o2 = grp + 1536 + 16 * (bb + l.next) + 8 * (l.u >> 1);
         lc.o3 = grp + 1664 + 2 * (bb + l.next);
-        lc.sh = 8 * (l.u & 1);
+        lc.sh = BYTE_SELECTOR + (l.u & 1);
         lc.ma = lc.mb = lc.mc = lc.h0 = lc.h1 = 0;
         lc.first = l.own;
         lc.sc += 4 * (8 * (blk + l.next) + 4 * (l.u >> 1));
@@ -455,9 +461,9 @@ template <> struct Frag<IB_Q6_K> {
         }
         const uint2 scw = lds64(row + lc.o2 + 16 * K * i);   // scales[8 half .. +7]: stretch s is byte 2s + h
         const float d = h2f(lds16(row + lc.o3 + 2 * K * i));
-        const uint32_t sa = scw.x >> lc.sh, sb = scw.y >> lc.sh;
-        const float w[4] = {(float)(int)(int8_t)(sa & 0xFF), (float)(int)(int8_t)((sa >> 16) & 0xFF), (float)(int)(int8_t)(sb & 0xFF),
-                            (float)(int)(int8_t)((sb >> 16) & 0xFF)};
+        const uint32_t sa = scw.x ^ 0x80808080u, sb = scw.y ^ 0x80808080u;   // signed bytes, 128 too high
+        constexpr float BIAS = 8388608.0f + 128.0f;
+        const float w[4] = {byte_to_float(sa, lc.sh, BIAS), byte_to_float(sa, lc.sh + 2, BIAS), byte_to_float(sb, lc.sh, BIAS), byte_to_float(sb, lc.sh + 2, BIAS)};
         float v = 0.f;
 #pragma unroll
         for (int k = 0; k < 4; k++) v += w[k] * (a.s[k] * unit_of<FOUR>(D[k], E[k], lc.first) + a.x[k]);
