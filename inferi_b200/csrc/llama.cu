@@ -141,7 +141,7 @@ struct ib_llama {
         uint8_t *arena = nullptr;
         uint32_t chunks = 0, most = PREFILL_MAX_TOKENS / PF_CHUNK;   // most: what the device has had room for
         float *X = nullptr, *q = nullptr, *planes = nullptr;
-        __half *hi = nullptr, *lo = nullptr;
+        __half *xt = nullptr;
         uint32_t *tokens = nullptr;
     } pf;
     // tensors and device vectors the model owns (a model loaded from a GGUF file frees its weights with itself)
@@ -791,7 +791,7 @@ static int32_t prefill_prepare(ib_llama *m, uint32_t n) {
         size_t total = 0;
         auto place = [&](size_t bytes) { const size_t at = total; total += (bytes + 255) & ~(size_t)255; return at; };
         const size_t oX = place(sizeof(float) * N * H), oq = place(sizeof(float) * N * Q);
-        const size_t ohi = place(sizeof(__half) * chunks * pf_x_halves(widest)), olo = place(sizeof(__half) * chunks * pf_x_halves(widest));
+        const size_t oxt = place(sizeof(__half) * chunks * pf_x_halves(widest));
         const size_t opl = place(sizeof(float) * planes), otok = place(sizeof(uint32_t) * N);
         const cudaError_t e = cudaMalloc(&B.arena, total);
         if (e == cudaErrorMemoryAllocation && chunks > 1) {   // a prompt goes through in shorter passes rather than not at all
@@ -806,7 +806,7 @@ static int32_t prefill_prepare(ib_llama *m, uint32_t n) {
             return set_error(e == cudaErrorMemoryAllocation ? IB_ERR_OOM : IB_ERR_CUDA, "ib_llama_prefill: buffers of %llu bytes: %s", (unsigned long long)total, cudaGetErrorString(e));
         }
         B.X = (float *)(B.arena + oX); B.q = (float *)(B.arena + oq);
-        B.hi = (__half *)(B.arena + ohi); B.lo = (__half *)(B.arena + olo); B.planes = (float *)(B.arena + opl); B.tokens = (uint32_t *)(B.arena + otok);
+        B.xt = (__half *)(B.arena + oxt); B.planes = (float *)(B.arena + opl); B.tokens = (uint32_t *)(B.arena + otok);
         B.chunks = chunks;
         return IB_OK;
     }
@@ -846,7 +846,7 @@ int32_t ib_llama_prefill(ib_llama *m, void *stream, const uint32_t *tokens_host,
             const PrefillGroup &p = groups[i];
             const StreamK sk = prefill_streamk(ctx, p.rows, p.cols, nc);
             const PfPlanes pl{at, at + (size_t)nc * p.rows, sk, p.rows, (nc + PF_CHUNK - 1) / PF_CHUNK, nc};
-            const int32_t r = launch_prefill_gemm(ctx, s, p.mats, p.n_mats, B.hi, B.lo, nc, at, at + (size_t)nc * p.rows, sk);
+            const int32_t r = launch_prefill_gemm(ctx, s, p.mats, p.n_mats, B.xt, nc, at, at + (size_t)nc * p.rows, sk);
             if (r) return r;
             for (uint32_t j = 0, row = 0; j < p.n_mats; row += (uint32_t)p.mats[j]->rows, j++, k++) { g[k] = pl; row0[k] = row; }
             at += prefill_plane_floats(ctx, p, nc);
@@ -864,7 +864,7 @@ int32_t ib_llama_prefill(ib_llama *m, void *stream, const uint32_t *tokens_host,
         for (uint32_t l = 0; l < c.num_hidden_layers; l++) {
             const ib_llama_layer_weights &w = m->layers[l];
             // q, k, v: (the previous layer's residual,) RMSNorm, GEMM, bias, RoPE, cache append (transformer.rs:420-445)
-            PF(launch_prefill_norm_split(ctx, s, B.X, l ? &g[0] : nullptr, w.attn_norm_dev, c.rms_norm_eps, nc, H, B.hi, B.lo));
+            PF(launch_prefill_norm_split(ctx, s, B.X, l ? &g[0] : nullptr, w.attn_norm_dev, c.rms_norm_eps, nc, H, B.xt));
             const ib_qtensor *qkv[3] = {w.attn_q, w.attn_k, w.attn_v}, *gu[2] = {w.ffn_gate, w.ffn_up};
             PF(gemm(qkv, 3, nc, g, row0));
             PfQkv e = {};
@@ -874,13 +874,13 @@ int32_t ib_llama_prefill(ib_llama *m, void *stream, const uint32_t *tokens_host,
             e.q = B.q; e.k_cache = m->k_cache[l]; e.v_cache = m->v_cache[l];
             PF(launch_prefill_qkv(ctx, s, e));
             // causal attention: query t over positions 0 .. pos0 + t (transformer.rs:448)
-            PF(launch_prefill_attention(ctx, s, B.q, m->k_cache[l], m->v_cache[l], nc, pos0, m->n_kv_l, m->head_size, B.hi, B.lo));
+            PF(launch_prefill_attention(ctx, s, B.q, m->k_cache[l], m->v_cache[l], nc, pos0, m->n_kv_l, m->head_size, B.xt));
             // o_proj + residual (transformer.rs:450-453); the residual add is part of the next norm kernel
             PF(gemm(&w.attn_output, 1, nc, g, row0));
             // gate, up, SwiGLU (transformer.rs:454-464)
-            PF(launch_prefill_norm_split(ctx, s, B.X, &g[0], w.ffn_norm_dev, c.rms_norm_eps, nc, H, B.hi, B.lo));
+            PF(launch_prefill_norm_split(ctx, s, B.X, &g[0], w.ffn_norm_dev, c.rms_norm_eps, nc, H, B.xt));
             PF(gemm(gu, 2, nc, g, row0));
-            PF(launch_prefill_swiglu(ctx, s, g[0], B.hi, B.lo));
+            PF(launch_prefill_swiglu(ctx, s, g[0], B.xt));
             // down + residual (transformer.rs:465-468)
             PF(gemm(&w.ffn_down, 1, nc, g, row0));
         }

@@ -17,7 +17,7 @@ namespace ib {
 __device__ __forceinline__ F8 pf_sum8(const PfPlanes &g, uint32_t t, uint32_t r) {
     const size_t at = (size_t)t * g.rows + r, plane = (size_t)g.n * g.rows;
     F8 v = pf_load8u(g.plane0 + at);
-    const uint32_t np = g.sk.pieces((r >> 7) * g.chunks + t / PF_CHUNK);
+    const uint32_t np = g.sk.pieces((r / PF_TILE_ROWS) * g.chunks + t / PF_CHUNK);
     for (uint32_t s = 1; s < np; s += 2) {
         const F8 a = pf_load8(g.planes + (s - 1) * plane + at);
         if (s + 1 < np) {
@@ -45,14 +45,14 @@ __global__ void prefill_embed_kernel(QDesc embd, const uint32_t *tokens, uint32_
 // between the two (PF_KEEP * 8 columns per thread).  Rows n .. n rounded up to 16 are zero-filled.
 constexpr int PF_ROW_THREADS = 512, PF_KEEP = 4;
 __global__ void __launch_bounds__(PF_ROW_THREADS) prefill_norm_split_kernel(float *X, const PfPlanes add, uint32_t has_add, const float *w, float eps, uint32_t n, uint32_t cols,
-                                                                            __half *hi, __half *lo) {
+                                                                            __half *xt) {
     __shared__ float red[PF_ROW_THREADS / 32];
     const uint32_t t = blockIdx.x, tid = threadIdx.x;
     constexpr uint32_t STEP = PF_ROW_THREADS * 8;
     pf_enter();
     if (t >= n) {
         const F8 zero = {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}};
-        for (uint32_t c = tid * 8; c < cols; c += STEP) pf_emit8(hi, lo, t, c, cols, zero);   // cols % 256 == 0: whole warps
+        for (uint32_t c = tid * 8; c < cols; c += STEP) pf_emit8(xt, t, c, cols, zero);   // cols % 256 == 0: whole warps
         return;
     }
     float *x = X + (size_t)t * cols;
@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(PF_ROW_THREADS) prefill_norm_split_kernel(floa
 #pragma unroll
             for (int i = 0; i < 8; i++) v.v[i] = (v.v[i] * rms) * g.v[i];
         }
-        pf_emit8(hi, lo, t, c, cols, v);
+        pf_emit8(xt, t, c, cols, v);
     };
 #pragma unroll
     for (int k = 0; k < PF_KEEP; k++) {
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(256) prefill_finish_kernel(float *out, const P
     const uint32_t per = add.rows / 8, i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= add.n * per) return;
     const uint32_t t = i / per, r = (i - t * per) * 8;
-    if (add.sk.pieces((r >> 7) * add.chunks + t / PF_CHUNK) == 1) return;
+    if (add.sk.pieces((r / PF_TILE_ROWS) * add.chunks + t / PF_CHUNK) == 1) return;
     const F8 v = pf_sum8(add, t, r);   // plane 0 is `out`
     float *o = out + (size_t)t * add.rows + r;
     if (((uintptr_t)o & 15) == 0) { pf_store8(o, v); return; }
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(256) prefill_finish_narrow_kernel(float *out, 
     pf_enter();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= add.n * add.rows) return;
-    const uint32_t t = i / add.rows, r = i - t * add.rows, np = add.sk.pieces((r >> 7) * add.chunks + t / PF_CHUNK);
+    const uint32_t t = i / add.rows, r = i - t * add.rows, np = add.sk.pieces((r / PF_TILE_ROWS) * add.chunks + t / PF_CHUNK);
     if (np == 1) return;
     const size_t plane = (size_t)add.n * add.rows;
     const float *p = add.planes + i;
@@ -146,7 +146,7 @@ __global__ void __launch_bounds__(256) prefill_finish_narrow_kernel(float *out, 
     out[i] = v;
 }
 
-__global__ void __launch_bounds__(256) prefill_swiglu_kernel(const PfPlanes gu, __half *hi, __half *lo) {
+__global__ void __launch_bounds__(256) prefill_swiglu_kernel(const PfPlanes gu, __half *xt) {
     pf_enter();
     const uint32_t F = gu.rows / 2, per = F / 8, i = blockIdx.x * blockDim.x + threadIdx.x, t = i / per, c = (i - t * per) * 8;   // whole warps: F % 256 == 0
     if (t >= ((gu.n + 15) & ~15u)) return;
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(256) prefill_swiglu_kernel(const PfPlanes gu, 
 #pragma unroll
         for (int k = 0; k < 8; k++) y.v[k] = b.v[k] * (a.v[k] / (1.0f + expf(-a.v[k])));   // crates/inferi-shaders/src/silu.rs:16-19,46-52
     }
-    pf_emit8(hi, lo, t, c, F, y);
+    pf_emit8(xt, t, c, F, y);
 }
 
 // Eight rows (four rotation pairs) of q, k or v of one token: bias (transformer.rs:434-442), rotation of adjacent pairs
@@ -220,8 +220,8 @@ int32_t launch_prefill_embed(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *embd
     return pf_launch(ctx, s, prefill_embed_kernel, (uint32_t)(((size_t)n * hidden + 255) / 256), 256, e, tokens_dev, n, hidden, vocab, X);
 }
 
-int32_t launch_prefill_norm_split(ib_ctx *ctx, cudaStream_t s, float *X, const PfPlanes *add, const float *w, float eps, uint32_t n, uint32_t cols, __half *hi, __half *lo) {
-    return pf_launch(ctx, s, prefill_norm_split_kernel, (n + 15) & ~15u, PF_ROW_THREADS, X, add ? *add : PfPlanes{}, add ? 1u : 0u, w, eps, n, cols, hi, lo);
+int32_t launch_prefill_norm_split(ib_ctx *ctx, cudaStream_t s, float *X, const PfPlanes *add, const float *w, float eps, uint32_t n, uint32_t cols, __half *xt) {
+    return pf_launch(ctx, s, prefill_norm_split_kernel, (n + 15) & ~15u, PF_ROW_THREADS, X, add ? *add : PfPlanes{}, add ? 1u : 0u, w, eps, n, cols, xt);
 }
 
 static uint32_t pf_grid(size_t threads) { return (uint32_t)((threads + 255) / 256); }
@@ -237,8 +237,8 @@ int32_t launch_prefill_finish(ib_ctx *ctx, cudaStream_t s, float *out, const PfP
     if (prefill_max_pieces(add.sk) > 8 && columns < (size_t)8 * 256 * (uint32_t)ctx->sm_count) return pf_launch(ctx, s, prefill_finish_narrow_kernel, pf_grid(columns), 256, out, add);
     return pf_launch(ctx, s, prefill_finish_kernel, pf_grid(columns / 8), 256, out, add);
 }
-int32_t launch_prefill_swiglu(ib_ctx *ctx, cudaStream_t s, const PfPlanes &gu, __half *hi, __half *lo) {
-    return pf_launch(ctx, s, prefill_swiglu_kernel, pf_grid((size_t)((gu.n + 15) & ~15u) * gu.rows / 16), 256, gu, hi, lo);
+int32_t launch_prefill_swiglu(ib_ctx *ctx, cudaStream_t s, const PfPlanes &gu, __half *xt) {
+    return pf_launch(ctx, s, prefill_swiglu_kernel, pf_grid((size_t)((gu.n + 15) & ~15u) * gu.rows / 16), 256, gu, xt);
 }
 int32_t launch_prefill_qkv(ib_ctx *ctx, cudaStream_t s, const PfQkv &p) {
     return pf_launch(ctx, s, prefill_qkv_kernel, pf_grid((size_t)p.n * (p.q_dim + 2 * p.kv_dim) / 8), 256, p);
@@ -275,7 +275,7 @@ extern "C" int32_t ib_gemm_quant(ib_ctx *ctx, void *stream, float *out_dev, cons
     auto bytes_of = [&](uint32_t nc, size_t &half_bytes) {
         const StreamK sk = prefill_streamk(ctx, rows, cols, nc);
         half_bytes = (nc + PF_CHUNK - 1) / PF_CHUNK * pf_x_halves(cols) * sizeof(__half);
-        return 2 * half_bytes + (((size_t)(prefill_max_pieces(sk) - 1) * nc * rows * sizeof(float) + 255) & ~(size_t)255);
+        return half_bytes + (((size_t)(prefill_max_pieces(sk) - 1) * nc * rows * sizeof(float) + 255) & ~(size_t)255);
     };
     auto shorter = [](uint32_t p) { return (p / 2 + PF_CHUNK - 1) / PF_CHUNK * PF_CHUNK; };
     size_t half_bytes = 0;
@@ -286,7 +286,7 @@ extern "C" int32_t ib_gemm_quant(ib_ctx *ctx, void *stream, float *out_dev, cons
         need = bytes_of(pass, half_bytes);
         if (n % pass) {   // the last, shorter pass may split its tiles further
             size_t hb = 0;
-            const size_t last = bytes_of(n % pass, hb) - 2 * hb + 2 * half_bytes;
+            const size_t last = bytes_of(n % pass, hb) - hb + half_bytes;
             if (last > need) need = last;
         }
         tiled_at = need;
@@ -311,8 +311,8 @@ extern "C" int32_t ib_gemm_quant(ib_ctx *ctx, void *stream, float *out_dev, cons
         rc = set_error(e == cudaErrorMemoryAllocation ? IB_ERR_OOM : IB_ERR_CUDA, "ib_gemm_quant: scratch of %llu bytes: %s", (unsigned long long)need, cudaGetErrorString(e));
         break;
     }
-    __half *hi = reinterpret_cast<__half *>(ctx->tc_scratch), *lo = reinterpret_cast<__half *>((uint8_t *)ctx->tc_scratch + half_bytes);
-    float *planes = reinterpret_cast<float *>((uint8_t *)ctx->tc_scratch + 2 * half_bytes);
+    __half *xt = reinterpret_cast<__half *>(ctx->tc_scratch);
+    float *planes = reinterpret_cast<float *>((uint8_t *)ctx->tc_scratch + half_bytes);
     if (retile && rc == IB_OK) {
         tiled.dev = (uint8_t *)ctx->tc_scratch + tiled_at;
         rc = retile_to_soa(ctx, s, m->qtype, m->dev, tiled.dev, m->rows, m->nb);
@@ -322,8 +322,8 @@ extern "C" int32_t ib_gemm_quant(ib_ctx *ctx, void *stream, float *out_dev, cons
         const uint32_t nc = n - t0 < pass ? n - t0 : pass;
         const StreamK sk = prefill_streamk(ctx, rows, cols, nc);
         float *out = out_dev + (size_t)t0 * rows;   // plane 0 of every tile
-        rc = launch_prefill_norm_split(ctx, s, const_cast<float *>(x_dev) + (size_t)t0 * cols, nullptr, nullptr, 0.f, nc, cols, hi, lo);
-        if (rc == IB_OK) rc = launch_prefill_gemm(ctx, s, &w, 1, hi, lo, nc, out, planes, sk, !retile);
+        rc = launch_prefill_norm_split(ctx, s, const_cast<float *>(x_dev) + (size_t)t0 * cols, nullptr, nullptr, 0.f, nc, cols, xt);
+        if (rc == IB_OK) rc = launch_prefill_gemm(ctx, s, &w, 1, xt, nc, out, planes, sk, !retile);
         if (rc == IB_OK && prefill_max_pieces(sk) > 1) rc = launch_prefill_finish(ctx, s, out, PfPlanes{out, planes, sk, rows, (nc + PF_CHUNK - 1) / PF_CHUNK, nc});
     }
     if (prev >= 0 && prev != ctx->device) cudaSetDevice(prev);

@@ -28,7 +28,7 @@ constexpr int PA_TOK = 16, PA_HEADS = 4, PA_ROWS = PA_TOK * PA_HEADS, PA_KV = 64
 struct PaParams {
     const float *q;          // [n][q_dim], rotated
     const __half *k, *v;     // this layer's cache [max_pos][kv_dim]
-    __half *hi, *lo;         // the next GEMM's inputs: q_dim columns
+    __half *xt;              // the next GEMM's inputs: q_dim columns
     uint32_t n, pos0, q_dim, kv_dim, splits;
 };
 
@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(PA_THREADS) prefill_attention_kernel(const PaP
         const float inv = t < p.n ? 1.0f / sum : 0.f;   // padding rows (up to a multiple of 16 tokens) are zero
 #pragma unroll
         for (int i = 0; i < 8; i++) y.v[i] *= inv;
-        pf_emit8(p.hi, p.lo, t, head * HS + c, p.q_dim, y);
+        pf_emit8(p.xt, t, head * HS + c, p.q_dim, y);
     }
     if (S > 1) cluster.sync();   // nobody leaves while its partials are being read
 }
@@ -253,9 +253,9 @@ static int32_t pa_launch(ib_ctx *ctx, cudaStream_t s, PaParams &p, uint32_t n_kv
 }
 
 int32_t launch_prefill_attention(ib_ctx *ctx, cudaStream_t s, const float *q, const void *k_cache, const void *v_cache, uint32_t n, uint32_t pos0, uint32_t n_kv, uint32_t head_size,
-                                 __half *hi, __half *lo) {
+                                 __half *xt) {
     PaParams p = {};
-    p.q = q; p.k = (const __half *)k_cache; p.v = (const __half *)v_cache; p.hi = hi; p.lo = lo;
+    p.q = q; p.k = (const __half *)k_cache; p.v = (const __half *)v_cache; p.xt = xt;
     p.n = n; p.pos0 = pos0; p.q_dim = n_kv * PA_HEADS * head_size; p.kv_dim = n_kv * head_size;
     switch (head_size) {
     case 128: return pa_launch<128>(ctx, s, p, n_kv);

@@ -34,7 +34,7 @@ __device__ __forceinline__ void pf_add8(F8 &a, const F8 &b) {
 
 // Columns c .. c + 7 (c % 8 == 0) of token t into the split, tiled inputs of the next GEMM, with the sums of the 32-column
 // sub-blocks: four neighbouring lanes hold one sub-block (all 32 lanes of the warp take part).
-__device__ __forceinline__ void pf_emit8(__half *hi, __half *lo, uint32_t t, uint32_t c, uint32_t cols, const F8 &f) {
+__device__ __forceinline__ void pf_emit8(__half *xt, uint32_t t, uint32_t c, uint32_t cols, const F8 &f) {
     const size_t base = (size_t)(t / PF_CHUNK) * pf_x_halves(cols);
     const uint32_t tc = t % PF_CHUNK;
     uint32_t h[4], l[4];
@@ -51,19 +51,19 @@ __device__ __forceinline__ void pf_emit8(__half *hi, __half *lo, uint32_t t, uin
         sum += f.v[2 * i] + f.v[2 * i + 1];
     }
     const size_t at = base + pf_x_index(tc, c);
-    *reinterpret_cast<uint4 *>(hi + at) = make_uint4(h[0], h[1], h[2], h[3]);
-    *reinterpret_cast<uint4 *>(lo + at) = make_uint4(l[0], l[1], l[2], l[3]);
+    *reinterpret_cast<uint4 *>(xt + at) = make_uint4(h[0], h[1], h[2], h[3]);
+    *reinterpret_cast<uint4 *>(xt + at + PF_X_LO) = make_uint4(l[0], l[1], l[2], l[3]);
     sum += __shfl_xor_sync(0xffffffffu, sum, 1);
     sum += __shfl_xor_sync(0xffffffffu, sum, 2);
     const size_t sat = base + pf_s_index(tc, c >> 5, cols);
     if ((c & 31) == 0) {
         const __half sh = __float2half_rn(sum);
-        hi[sat] = sh;
-        lo[sat] = __float2half_rn(sum - __half2float(sh));
+        xt[sat] = sh;
+        xt[sat + PF_S_LO] = __float2half_rn(sum - __half2float(sh));
     }
     if ((c & 255) == 8) {   // the eight zero halves of the block's row of sums
-        *reinterpret_cast<uint4 *>(hi + sat + 64) = make_uint4(0, 0, 0, 0);
-        *reinterpret_cast<uint4 *>(lo + sat + 64) = make_uint4(0, 0, 0, 0);
+        *reinterpret_cast<uint4 *>(xt + sat + 64) = make_uint4(0, 0, 0, 0);
+        *reinterpret_cast<uint4 *>(xt + sat + PF_S_LO + 64) = make_uint4(0, 0, 0, 0);
     }
 }
 

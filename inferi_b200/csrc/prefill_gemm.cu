@@ -1,5 +1,5 @@
-// The GEMM of the prompt prefill: out^T tile = W tile (128 rows of a quantized matrix) x X^T (up to 128 tokens), on the
-// 5th-generation tensor cores (tcgen05.mma, f32 accumulators in tensor memory).
+// The GEMM of the prompt prefill: out^T tile = W tile (256 rows of a quantized matrix) x X^T (up to 128 tokens), on the
+// 5th-generation tensor cores (tcgen05.mma, f32 accumulators in tensor memory) of a pair of SMs.
 //
 // Exact integer weights.  A k-quant weight is w = d * (sc * q) - dmin * m with d, dmin one f16 (pair) per 256 columns and
 // row, sc a 6- or 8-bit integer, q a small integer (crates/inferi/src/quantization.rs:227-402).  sc * q is an integer; per
@@ -15,7 +15,13 @@
 // memory (through shared memory the tile cost a write, a proxy fence that every warp waited for, and 64 bytes a clock of
 // operand reads next to the inputs' 64).
 //
-// Who does what (19 warps, one CTA per SM):
+// Two SMs per tile (cta_group::2).  Each makes the operand of its 128 rows and keeps their sums; the inputs of the 128 tokens are
+// shared, half of them in either's shared memory.  On one SM a 256-column block of 128 rows took 131 KB of inputs from L2 for 2240
+// clocks of MMAs, and L2 delivers 72 bytes a nanosecond to an SM: 9.5 of at most 10.7 TB/s, 4000 clocks a block.  Now 2490 (Q4_K).
+// Measured, one SM / two: Q4_K 14336 x 4096, 900 tokens 218 / 185 us; with Q6_K's conversions (below) 4096 x 14336, 1000 tokens 383 /
+// 288; a prompt of 1021 tokens of the 8B architecture 39.8 / 33.1 ms, of 128 tokens 6.24 / 5.36.
+//
+// Who does what (19 warps, one CTA per SM; the MMAs of both are issued by the first):
 //   warps 0-7    producers: two warpgroups, each two of the block's four 64-column chunks
 //   warps 8-15   fold: when a block's P is complete, Y += d * P into registers (64 accumulators a thread); at the end of the
 //                tile's K range Y -= Z and the store, [token][row]
@@ -41,7 +47,7 @@ constexpr uint32_t PG_DSLOTS = 4;
 constexpr uint32_t PG_XSTAGES_MAX = 16;   // a stage holds the tokens' 64 columns, hi and lo: few tokens, small stages, more of them (launch)
 constexpr uint32_t PG_STILE = PF_CHUNK * 16 * 2;        // ... of 128 tokens x 16 sub-block sums
 constexpr uint32_t PG_SMEM_LIMIT = 227 * 1024;
-constexpr uint32_t PG_LBO = 128, PG_SBO = 1024, PG_SSBO = 256;   // core matrices of the inputs' tiles and of the sums' tiles
+constexpr uint32_t PG_LBO = 128, PG_SBO = 2048, PG_SSBO = 512;   // core matrices of the inputs' tiles and of the sums' tiles
 // tensor memory columns
 constexpr uint32_t PG_P = 0, PG_Z = 256, PG_A4 = 384, PG_M4 = 480, PG_A6 = 256;
 
@@ -159,16 +165,31 @@ __device__ __forceinline__ void pg_wait_ld() { asm volatile("tcgen05.wait::ld.sy
 __device__ __forceinline__ uint64_t pg_desc(uint32_t smem_addr, uint32_t lbo, uint32_t sbo) {
     return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (uint64_t)((lbo >> 4) & 0x3FFFu) << 16 | (uint64_t)((sbo >> 4) & 0x3FFFu) << 32 | (uint64_t)1 << 46;
 }
-// Instruction descriptor of kind::f16: f16 A and B (both K-major), f32 accumulator, 128 x N.
-__device__ __forceinline__ uint32_t pg_idesc(uint32_t N) { return (1u << 4) | ((N >> 3) << 17) | ((128u >> 4) << 24); }
-// D[128 x N] (+)= A (tensor memory, 16 columns of f16 = 8 columns of 32 bits) x B (shared memory)
+// Instruction descriptor of kind::f16: f16 A and B (both K-major), f32 accumulator, 256 x N.
+__device__ __forceinline__ uint32_t pg_idesc(uint32_t N) { return (1u << 4) | ((N >> 3) << 17) | ((256u >> 4) << 24); }
+// D[256 x N] (+)= A (tensor memory, 16 columns of f16 = 8 columns of 32 bits) x B (shared memory), on both SMs of the pair: each has its
+// 128 rows of A and D in its own tensor memory and half of B's N rows in its own shared memory, at the same places.
 __device__ __forceinline__ void pg_mma(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc),
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc),
                  "r"(idesc), "r"(accumulate)
                  : "memory");
 }
+// arrives, when the MMAs issued so far are done, on the barrier at this place in both CTAs
 __device__ __forceinline__ void pg_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+}
+// ---- between the two CTAs ----
+// (Waits keep the default scope also where the other CTA arrives: what the barriers order is tensor memory and bulk copies, and a wait that
+// acquires at cluster scope made every launch 1.2 to 1.4 times as long.)
+__device__ __forceinline__ uint32_t pg_leader(uint32_t addr) {   // the same place in the pair's first CTA
+    uint32_t a;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(addr));
+    return a;
+}
+__device__ __forceinline__ void pg_arrive_cluster(uint32_t addr) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory"); }
+__device__ __forceinline__ void pg_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
 }
 __device__ __forceinline__ void pg_tma2d(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
@@ -262,7 +283,7 @@ __device__ __forceinline__ void pg_scales(const uint4 &hdr, uint32_t c, uint32_t
 
 // The current unit of a role's walk over its CTA's range, carried forward by additions
 struct PgCursor {
-    uint32_t rt, chunk, kb;   // row tile, chunk of 128 tokens, 256-column block
+    uint32_t rt, chunk, kb;   // row tile of the pair, chunk of 128 tokens, 256-column block
     __device__ __forceinline__ void init(const PgParams &p, uint32_t u) {
         const uint32_t tile = u / p.sk.nb;
         kb = u - tile * p.sk.nb;
@@ -300,26 +321,28 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
     const uint32_t b_zdone = take(1), b_zfree = take(1), s_tmem = nb;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const StreamK sk = p.sk;
-    const uint32_t u0 = sk.first_unit(blockIdx.x), nunits = sk.first_unit(blockIdx.x + 1) - u0;
+    const uint32_t pair = blockIdx.x >> 1, rank = blockIdx.x & 1;   // clusters of two CTAs along x
+    const uint32_t u0 = sk.first_unit(pair), nunits = sk.first_unit(pair + 1) - u0;
 
     asm volatile("griddepcontrol.launch_dependents;");
-    if (tid == 0) {
-        for (uint32_t s = 0; s < R; s++) { pg_bar_init(b_rawfull + 8 * s, 1); pg_bar_init(b_rawempty + 8 * s, PG_PRODUCERS); }
-        for (uint32_t s = 0; s < NS; s++) { pg_bar_init(b_afull + 8 * s, PG_PRODUCERS / 2); pg_bar_init(b_aempty + 8 * s, 1); }
-        for (uint32_t s = 0; s < XS; s++) { pg_bar_init(b_xfull + 8 * s, 1); pg_bar_init(b_xempty + 8 * s, 1); }
-        for (uint32_t s = 0; s < 2; s++) {
-            pg_bar_init(b_pdone + 8 * s, 1); pg_bar_init(b_pfree + 8 * s, PG_FOLD);
+    if (warp == 0) {
+        // A lane per barrier.  What the MMA warp waits for counts both CTAs and lives in the first one; the MMAs' completion arrives in both.
+        constexpr uint32_t X0 = 2 * R + 2 * NS, P0 = X0 + 2 * PG_XSTAGES_MAX;
+        for (uint32_t i = lane; i < P0 + 6; i += 32) {
+            uint32_t count = 1;
+            if (i >= R && i < 2 * R + NS) count = PG_PRODUCERS;                                          // rawempty, afull
+            else if (i >= X0 && i < X0 + PG_XSTAGES_MAX) count = rank == 0 ? 2 : 1;                       // xfull: the bytes, and word of the other CTA's
+            else if (i == P0 + 2 || i == P0 + 3 || i == P0 + 5) count = 2 * PG_FOLD;                      // pfree, zfree
+            pg_bar_init(b_rawfull + 8 * i, count);
         }
-        pg_bar_init(b_zdone, 1);
-        pg_bar_init(b_zfree, PG_FOLD);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == PG_W_MMA) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_tmem), "r"(512u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_tmem), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
     }
     pg_fence_before();
-    __syncthreads();
+    pg_cluster_sync();
     pg_fence_after();
     uint32_t tmem;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(s_tmem));
@@ -327,7 +350,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
 
     if (warp < PG_PRODUCERS) {
         // ===== producers: thread = row; warpgroup `wg` makes chunks 2 wg and 2 wg + 1 of every block =====
-        const uint32_t row = tid & 127, wg = warp >> 2, tl = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+        const uint32_t row = tid & 127, wg = warp >> 2, tl = tmem + ((uint32_t)((warp & 3) * 32) << 16), lead_afull = pg_leader(b_afull);
         if (MIN && wg == 0) {   // columns 4..7 of the minimums' operands (sub-blocks 8..15 of a K = 16 MMA) stay zero
             for (uint32_t m = 0; m < 4; m++)
                 for (uint32_t c = 4; c < 8; c++) pg_st1(tl + PG_M4 + 8 * m + c, 0u);
@@ -338,29 +361,23 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
         for (uint32_t j = 0; j < nunits && ok; j++) {
             if (!(ok = pg_wait_warp(b_rawfull + 8 * slot, rpar, p, 8))) break;
             const uint32_t raw = raw0 + slot * RAW;
-            uint4 hdr = make_uint4(0, 0, 0, 0), f0 = hdr, f1 = hdr, f2 = hdr, f3 = hdr, g0 = hdr, g1 = hdr;
+            // The quants are read where they are converted, not all at the unit's start: registers that wait for their turn are
+            // registers that the conversions of other words cannot overlap in (Q6_K 4096 x 14336, 1000 tokens: 291 us against 383).
+            uint4 hdr = make_uint4(0, 0, 0, 0), f0, f1, g0 = hdr, g1 = hdr;
             uint2 sc8 = make_uint2(0, 0);
             float d;
             if constexpr (MIN) {
                 const uint32_t blk = raw + row * (FMT == PG_Q4K ? 144 : 176);
                 hdr = pg_lds128(blk);
                 if (FMT == PG_Q5K) { g0 = pg_lds128(blk + 16); g1 = pg_lds128(blk + 32); }
-                const uint32_t qs = blk + (FMT == PG_Q4K ? 16 : 48) + 64 * wg;
-                f0 = pg_lds128(qs); f1 = pg_lds128(qs + 16); f2 = pg_lds128(qs + 32); f3 = pg_lds128(qs + 48);
                 d = pg_h2f(hdr.x & 0xFFFFu);
             } else if constexpr (FMT == PG_Q6K) {
-                const uint32_t ql = raw + PG_Q6_QL + row * 144 + 64 * wg, qh = raw + PG_Q6_QH + row * 80 + 32 * wg;
-                f0 = pg_lds128(ql); f1 = pg_lds128(ql + 16); f2 = pg_lds128(ql + 32); f3 = pg_lds128(ql + 48);
+                const uint32_t qh = raw + PG_Q6_QH + row * 80 + 32 * wg;
                 g0 = pg_lds128(qh); g1 = pg_lds128(qh + 16);
                 sc8 = pg_lds64(raw + PG_Q6_SC + row * 16 + 8 * wg);
                 d = pg_h2f(pg_lds16(raw + PG_Q6_D + row * 16 + 2 * (cur.kb & 7)));
             } else {
-                const uint32_t blk = raw + row * 272;
-                const uint32_t qs = blk + 128 * wg;
-                f0 = pg_lds128(qs); f1 = pg_lds128(qs + 16); f2 = pg_lds128(qs + 32); f3 = pg_lds128(qs + 48);
-                hdr.x = 0;
-                sc8 = pg_lds64(blk + 256 + 8 * wg);   // f16 scales of the warpgroup's four blocks
-                g0 = pg_lds128(qs + 64); g1 = pg_lds128(qs + 80);
+                sc8 = pg_lds64(raw + row * 272 + 256 + 8 * wg);   // f16 scales of the warpgroup's four blocks
                 d = 1.0f;
             }
 #pragma unroll
@@ -369,7 +386,9 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
                 if constexpr (MIN) {
                     uint32_t sc2, m2, r[32];
                     pg_scales(hdr, c, sc2, m2);
-                    pg_convert_k<FMT == PG_Q5K>(cc ? f2 : f0, cc ? f3 : f1, g0, g1, c, (float)(sc2 & 0xFFu), (float)(sc2 >> 8), r);
+                    const uint32_t qs = raw + row * (FMT == PG_Q4K ? 144 : 176) + (FMT == PG_Q4K ? 16 : 48) + 32 * c;
+                    f0 = pg_lds128(qs); f1 = pg_lds128(qs + 16);
+                    pg_convert_k<FMT == PG_Q5K>(f0, f1, g0, g1, c, (float)(sc2 & 0xFFu), (float)(sc2 >> 8), r);
                     const float dmin = pg_h2f(hdr.x >> 16), m0 = dmin * (float)(m2 & 0xFFu), m1 = dmin * (float)(m2 >> 8);
                     const __half2 mh = __floats2half2_rn(m0, m1);
                     const float2 back = __half22float2(mh);
@@ -390,23 +409,28 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
                     if constexpr (FMT == PG_Q6K) {
                         const uint32_t sw = cc ? sc8.y : sc8.x;
                         auto sc = [&](uint32_t k) { return (float)(int)(int8_t)((sw >> (8 * k)) & 0xFFu); };
+                        const uint32_t ql = raw + PG_Q6_QL + row * 144 + 64 * wg;
+                        f0 = pg_lds128(ql); f1 = pg_lds128(ql + 16);
                         if (cc == 0) pg_convert_q6<0>(f0, f1, g0, g1, sc(0), sc(1), a, b);
                         else pg_convert_q6<2>(f0, f1, g0, g1, sc(0), sc(1), a, b);
                         if (use && !(ok = pg_wait_warp(b_aempty + 8 * as, (use - 1) & 1, p, 8))) break;
                         pg_fence_after();
                         pg_st16(ta, a);
                         pg_st16(ta + 32, b);
-                        if (cc == 0) pg_convert_q6<1>(f2, f3, g0, g1, sc(2), sc(3), a, b);
-                        else pg_convert_q6<3>(f2, f3, g0, g1, sc(2), sc(3), a, b);
+                        f0 = pg_lds128(ql + 32); f1 = pg_lds128(ql + 48);
+                        if (cc == 0) pg_convert_q6<1>(f0, f1, g0, g1, sc(2), sc(3), a, b);
+                        else pg_convert_q6<3>(f0, f1, g0, g1, sc(2), sc(3), a, b);
                     } else {
                         const __half2 dd = pg_h2(cc ? sc8.y : sc8.x);
-                        if (cc == 1) { f0 = g0; f1 = g1; f2 = pg_lds128(raw + row * 272 + 128 * wg + 96); f3 = pg_lds128(raw + row * 272 + 128 * wg + 112); }
+                        const uint32_t qs = raw + row * 272 + 64 * c;
+                        f0 = pg_lds128(qs); f1 = pg_lds128(qs + 16);
                         pg_convert_q8(f0, f1, __low2half2(dd), a, b);
                         if (use && !(ok = pg_wait_warp(b_aempty + 8 * as, (use - 1) & 1, p, 8))) break;
                         pg_fence_after();
                         pg_st16(ta, a);
                         pg_st16(ta + 32, b);
-                        pg_convert_q8(f2, f3, __high2half2(dd), a, b);
+                        f0 = pg_lds128(qs + 32); f1 = pg_lds128(qs + 48);
+                        pg_convert_q8(f0, f1, __high2half2(dd), a, b);
                     }
                     if (cc == 1) {
                         __syncwarp();
@@ -419,7 +443,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
                 pg_wait_st();
                 pg_fence_before();
                 __syncwarp();
-                if (lane == 0) pg_arrive(b_afull + 8 * as);
+                if (lane == 0) pg_arrive_cluster(lead_afull + 8 * as);
             }
             if (++slot == R) { slot = 0; rpar ^= 1u; }
             cur.next(p);
@@ -428,6 +452,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
     } else if (warp < PG_PRODUCERS + PG_FOLD) {
         // ===== fold: thread = row (tensor-memory lane), 64 of the tokens =====
         const uint32_t row = (warp & 3) * 32 + lane, half = (warp - PG_PRODUCERS) >> 2, tl = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 64 * half;
+        const uint32_t lead_pfree = pg_leader(b_pfree), lead_zfree = pg_leader(b_zfree);
         float Y[64];
 #pragma unroll
         for (int i = 0; i < 64; i++) Y[i] = 0.f;
@@ -455,7 +480,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
             fold(PG_P + 128 * pb, d);
             pg_fence_before();
             __syncwarp();
-            if (lane == 0) pg_arrive(b_pfree + 8 * pb);
+            if (lane == 0) pg_arrive_cluster(lead_pfree + 8 * pb);
             if (end) {
                 if (MIN) {
                     if (!(ok = pg_wait_warp(b_zdone, seg & 1, p, 10))) break;
@@ -463,18 +488,40 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
                     fold(PG_Z, -1.0f);
                     pg_fence_before();
                     __syncwarp();
-                    if (lane == 0) pg_arrive(b_zfree);
+                    if (lane == 0) pg_arrive_cluster(lead_zfree);
                 }
                 seg++;
-                const uint32_t piece = blockIdx.x - sk.cta_of(cur.tile(p) * sk.nb), rt = cur.rt;
+                const uint32_t piece = pair - sk.pair_of(cur.tile(p) * sk.nb), rt = 2 * cur.rt + rank;   // (the last tile may lack its second half)
                 float *out = (piece == 0 ? p.plane0 : p.planes + (size_t)(piece - 1) * p.n * p.rows) + (size_t)(chunk * PF_CHUNK + 64 * half) * p.rows + rt * 128 + row;
+                const uint32_t count = rt * 128 < p.rows && nt > 64 * half ? nt - 64 * half : 0;
+                // (straight stores where 16 tokens are there: this code runs once or twice per launch, and its length is what it costs)
 #pragma unroll
-                for (uint32_t t = 0; t < 64; t++) {
-                    if (64 * half + t < nt) out[(size_t)t * p.rows] = Y[t];
-                    Y[t] = 0.f;
+                for (uint32_t g = 0; g < 4; g++) {
+                    if (count >= 16 * g + 16) {
+#pragma unroll
+                        for (uint32_t t = 0; t < 16; t++, out += p.rows) *out = Y[16 * g + t];
+                    } else {
+#pragma unroll
+                        for (uint32_t t = 0; t < 16; t++, out += p.rows)
+                            if (16 * g + t < count) *out = Y[16 * g + t];
+                    }
+                }
+                if (j + 1 < nunits) {
+#pragma unroll
+                    for (uint32_t t = 0; t < 64; t++) Y[t] = 0.f;
                 }
             }
             cur.next(p);
+        }
+    } else if (warp == PG_W_MMA && rank != 0) {
+        // ===== the second CTA issues no MMAs: it tells the first one when its half of a stage's inputs is there =====
+        const uint32_t lead_xfull = pg_leader(b_xfull);
+        uint32_t xs = 0, par = 0;
+        for (uint32_t i = 0; i < 4 * nunits && ok; i++) {
+            if (!(ok = pg_wait_warp(b_xfull + 8 * xs, par, p, 9))) break;
+            if (pg_elect()) pg_arrive_cluster(lead_xfull + 8 * xs);
+            __syncwarp();
+            if (++xs == XS) { xs = 0; par ^= 1u; }
         }
     } else if (warp == PG_W_MMA) {
         // ===== MMA issue: one elected lane; descriptors differ from the first stage's only in the start-address field =====
@@ -486,7 +533,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
         // is asked for ahead of the current stage's MMAs.  A block's sums arrive with its first inputs and its minimums with
         // its weights: the minimums' MMAs at the end of the block wait for nothing of their own.
         const uint32_t id_full = pg_idesc(PF_CHUNK), id_last = pg_idesc(pg_pad(p.n - (p.chunks - 1) * PF_CHUNK));
-        const uint32_t xstep = 2 * XTILE >> 4, sstep = 2 * STILE >> 4, xlo = XTILE >> 4, slo = STILE >> 4;
+        const uint32_t xstep = 2 * XTILE >> 4, sstep = 2 * STILE >> 4, xlo = PF_X_LO * 2 >> 4, slo = PF_S_LO * 2 >> 4;
         const uint32_t bx_end = b_xfull + 8 * XS, sd_end = (uint32_t)sd0 + SS * sstep, x_empty = b_xempty - b_xfull, a_empty = b_aempty - b_afull;
         const uint32_t x_hi32 = (uint32_t)(xd0 >> 32), s_hi32 = (uint32_t)(sd0 >> 32);
         // carried by additions: full barrier, parity and low descriptor word (start address) of the inputs' stage; barrier, parity and column of the weights'
@@ -556,28 +603,23 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
             else { bp = b_pdone; ppar ^= 1u; }
         }
     } else if (warp == PG_W_X) {
-        // ===== the inputs' tiles (two bulk copies per 64 columns) and, per block, the tiles of their sub-block sums =====
+        // ===== this CTA's half of the tokens' inputs (a bulk copy per 64 columns) and, per block, of their sub-block sums =====
         asm volatile("griddepcontrol.wait;" ::: "memory");   // the previous kernel writes them
         PgCursor cur;
         cur.init(p, u0);
         uint32_t xs = 0, use = 0, ss = 0;
         for (uint32_t j = 0; j < nunits && ok; j++) {
-            const uint32_t chunk = cur.chunk, np = pg_pad(cur.tokens(p));
-            const __half *hi = p.x_hi + (size_t)chunk * p.x_chunk, *lo = p.x_lo + (size_t)chunk * p.x_chunk;
+            const uint32_t tokens = pg_pad(cur.tokens(p)) / 2;
+            const __half *x = p.x + (size_t)cur.chunk * p.x_chunk;
             for (uint32_t c = 0; c < 4; c++) {
                 if (use && !(ok = pg_wait_warp(b_xempty + 8 * xs, (use - 1) & 1, p, 8))) break;
-                const uint32_t full = b_xfull + 8 * xs, dst = xst + xs * 2 * XTILE, bytes = np * 128;
-                const size_t at = (size_t)(4 * cur.kb + c) * (PF_CHUNK * 64);
+                const uint32_t full = b_xfull + 8 * xs, dst = xst + xs * 2 * XTILE, bytes = tokens * 256;
+                const size_t at = (size_t)(4 * cur.kb + c) * (PF_CHUNK * 128) + rank * tokens * 128;
                 if (pg_elect()) {
                     const bool sums = MIN && c == 0;   // (their slot's last reader was issued ahead of the stage just waited for)
-                    pg_expect(full, 2 * bytes + (sums ? bytes / 2 : 0));
-                    pg_bulk(dst, hi + at, bytes, full);
-                    pg_bulk(dst + XTILE, lo + at, bytes, full);
-                    if (sums) {
-                        const size_t sat = (size_t)PF_CHUNK * sk.nb * 256 + (size_t)cur.kb * (PF_CHUNK * 16);
-                        pg_bulk(sst + ss * 2 * STILE, hi + sat, bytes / 4, full);
-                        pg_bulk(sst + ss * 2 * STILE + STILE, lo + sat, bytes / 4, full);
-                    }
+                    pg_expect(full, bytes + (sums ? bytes / 4 : 0));
+                    pg_bulk(dst, x + at, bytes, full);
+                    if (sums) pg_bulk(sst + ss * 2 * STILE, x + (size_t)2 * PF_CHUNK * sk.nb * 256 + (size_t)cur.kb * (PF_CHUNK * 32) + rank * tokens * 32, bytes / 4, full);
                 }
                 __syncwarp();
                 if (++xs == XS) { xs = 0; use++; }
@@ -596,7 +638,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
         uint32_t slot = 0, use = 0;
         for (uint32_t j = 0; j < nunits && ok; j++) {
             if (use && !(ok = pg_wait_warp(b_rawempty + 8 * slot, (use - 1) & 1, p, 8))) break;
-            const uint32_t rt = cur.rt, s = rt >= p.tile0[2] ? 2 : (rt >= p.tile0[1] ? 1 : 0), y = (rt - p.tile0[s]) * 128;
+            const uint32_t rt = 2 * cur.rt + rank, s = rt >= p.tile0[2] ? 2 : (rt >= p.tile0[1] ? 1 : 0), y = (rt - p.tile0[s]) * 128;
             const uint32_t full = b_rawfull + 8 * slot, dst = raw0 + slot * RAW;
             const CUtensorMap *m = maps.m[s];
             if (pg_elect()) {
@@ -622,10 +664,16 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
         const unsigned long long t0 = pg_ns();
         while (pg_ns() - t0 < 100000ull) {}
     }
+    if (warp == PG_W_MMA && ok) {
+        // The last MMAs' commits arrive in both CTAs' shared memory: let them, before either CTA can end.
+        const uint32_t last = 4 * nunits - 1;
+        pg_wait_warp(b_aempty + 8 * (last % NS), (last / NS) & 1, p, 9);
+        pg_wait_warp(b_xempty + 8 * (last % XS), (last / XS) & 1, p, 9);
+    }
     __syncwarp();
     pg_fence_before();
-    __syncthreads();
-    if (warp == PG_W_MMA) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    pg_cluster_sync();   // the other CTA's shared and tensor memory are in use until here
+    if (warp == PG_W_MMA) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -634,15 +682,16 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
 StreamK prefill_streamk(const ib_ctx *ctx, uint32_t rows, uint32_t cols, uint32_t n) {
     StreamK sk;
     sk.nb = cols / 256;
-    sk.total = (rows / 128) * ((n + PF_CHUNK - 1) / PF_CHUNK) * sk.nb;
-    sk.ctas = sk.total < (uint32_t)ctx->sm_count ? sk.total : (uint32_t)ctx->sm_count;
+    sk.total = ((rows + PF_TILE_ROWS - 1) / PF_TILE_ROWS) * ((n + PF_CHUNK - 1) / PF_CHUNK) * sk.nb;
+    const uint32_t pairs = ctx->sm_count >= 2 ? (uint32_t)ctx->sm_count / 2 : 1u;
+    sk.pairs = sk.total < pairs ? sk.total : pairs;
     return sk;
 }
-// Most planes a tile needs: a range of `len` units cut into pieces of at least floor(total / ctas) units each
+// Most planes a tile needs: a range of `len` units cut into pieces of at least floor(total / pairs) units each
 uint32_t prefill_max_pieces(const StreamK &sk) {
-    const uint32_t least = sk.total / sk.ctas;
+    const uint32_t least = sk.total / sk.pairs;
     const uint32_t most = (sk.nb - 1) / least + 2;   // nb consecutive units touch at most this many ranges of that length
-    return most < sk.ctas ? most : sk.ctas;
+    return most < sk.pairs ? most : sk.pairs;
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
@@ -691,8 +740,8 @@ template <int FMT>
 static int32_t pg_launch(ib_ctx *ctx, cudaStream_t s, PgParams &p, const PgMaps &maps, bool early) {
     static bool attr_set[16] = {};
     constexpr uint32_t room = PG_SMEM_LIMIT - pg_fixed_smem(FMT);
-    static_assert(room >= 3 * 2 * PF_CHUNK * 128, "shared memory");
-    p.x_tile = ((p.n < PF_CHUNK ? p.n : PF_CHUNK) + 15) / 16 * 16 * 128;   // 64 columns of the (padded) tokens of a chunk
+    static_assert(room >= 3 * PF_CHUNK * 128, "shared memory");
+    p.x_tile = ((p.n < PF_CHUNK ? p.n : PF_CHUNK) + 15) / 16 * 8 * 128;   // 64 columns of a CTA's half of the (padded) tokens of a chunk
     p.x_stages = room / (2 * p.x_tile) < PG_XSTAGES_MAX ? room / (2 * p.x_tile) : PG_XSTAGES_MAX;
     const uint32_t smem = pg_fixed_smem(FMT) + p.x_stages * 2 * p.x_tile;
     if (!attr_set[ctx->device & 15]) {
@@ -700,25 +749,28 @@ static int32_t pg_launch(ib_ctx *ctx, cudaStream_t s, PgParams &p, const PgMaps 
         attr_set[ctx->device & 15] = true;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(p.sk.ctas);
+    cfg.gridDim = dim3(2 * p.sk.pairs);
     cfg.blockDim = dim3(PG_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = early ? 1 : 0;
+    cfg.numAttrs = early ? 2 : 1;
     IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, prefill_gemm_kernel<FMT>, p, maps));
     ctx->launches++;
     return IB_OK;
 }
 
-int32_t launch_prefill_gemm(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *const *mats, uint32_t n_mats, const __half *x_hi, const __half *x_lo, uint32_t n, float *plane0,
+int32_t launch_prefill_gemm(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *const *mats, uint32_t n_mats, const __half *x, uint32_t n, float *plane0,
                             float *planes, const StreamK &sk, bool early) {
     IB_REQUIRE(n_mats >= 1 && n_mats <= PF_MAX_SEGS, "prefill GEMM: %u matrices", n_mats);
     IB_REQUIRE(sk.total < (1u << 24), "prefill GEMM: %u units of work are too many for one launch", sk.total);
-    IB_REQUIRE(((uintptr_t)x_hi % 16) == 0 && ((uintptr_t)x_lo % 16) == 0, "prefill GEMM: the input tiles must be 16-byte aligned for the bulk copies");
+    IB_REQUIRE(((uintptr_t)x % 16) == 0, "prefill GEMM: the input tiles must be 16-byte aligned for the bulk copies");
     const int fmt = pg_format(mats[0]);
     PgParams p = {};
     PgMaps maps;
@@ -733,7 +785,7 @@ int32_t launch_prefill_gemm(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *const
         tiles += (uint32_t)m->rows / 128;
     }
     p.rows = tiles * 128;
-    p.n = n; p.chunks = (n + PF_CHUNK - 1) / PF_CHUNK; p.x_hi = x_hi; p.x_lo = x_lo; p.x_chunk = pf_x_halves((uint32_t)mats[0]->cols);
+    p.n = n; p.chunks = (n + PF_CHUNK - 1) / PF_CHUNK; p.x = x; p.x_chunk = pf_x_halves((uint32_t)mats[0]->cols);
     p.plane0 = plane0; p.planes = planes; p.sk = sk; p.err = ctx->err_dev; p.wait_ns = ctx->wait_limit_ns;
     switch (fmt) {
     case PG_Q4K: return pg_launch<PG_Q4K>(ctx, s, p, maps, early);

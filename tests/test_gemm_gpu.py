@@ -54,6 +54,13 @@ def test_gemm_across_chunks_of_tokens(backend, qt, rows, cols, n):
     m.close()
 
 
+# a pair of SMs shares 256 rows and a chunk's tokens: an odd number of 128-row halves, the fewest tokens per half, halves with a remainder
+@pytest.mark.parametrize("qt", [quant.Q4_K, quant.Q5_K, quant.Q6_K, quant.Q8_0])
+@pytest.mark.parametrize("rows,n", [(128, 1), (384, 16), (384, 33), (640, 145)])
+def test_gemm_halves_of_a_pair(backend, qt, rows, n):
+    test_gemm_across_chunks_of_tokens(backend, qt, rows, 2048, n)
+
+
 @pytest.mark.parametrize("qt,rows,cols,n", [
     (quant.Q6_K, 128, 34816, 2), (quant.Q6_K, 256, 34816, 130), (quant.Q8_0, 128, 33024, 9),
 ])
