@@ -13,10 +13,9 @@
 //    the inner loop touches shared memory for weights and scales only (gemv_stream.cuh).
 //  * Per-warp partial row sums meet in shared memory; the epilogue warp adds them in a fixed order and runs the epilogue
 //    (store / residual add / SwiGLU / RoPE + KV append / arg-max).  No warp ever waits for another one except through the ring.
-// What bounds it: a launch that streams, HBM (gate/up of an 8B model, 66 MB: 12.8 us, 5.2 TB/s with the fixed part; 13.9 with the RMSNorm
-// ahead of it); every launch
-// carries 3-4 us that no byte moves in - the input vector from L2, its packing, the B operands, the first tile's products and the
-// last tile's epilogue, one after the other - which is most of a short one (4096 x 4096 Q4_K, 9.4 MB: 4.7 us).  Byte dot products on
+// What bounds it: a launch that streams, HBM and the dot products alike (gate/up of an 8B model, 66 MB, with the RMSNorm ahead of it: 13.6 us);
+// every launch carries 3 us that no byte moves in - the input vector from L2, its packing, the B operands, the first tile's products and the
+// last tile's epilogue, one after the other - which is most of a short one (4096 x 4096 Q4_K, 9.4 MB: 4.3 us).  Byte dot products on
 // lanes that each own 64 columns, one producer and one epilogue warp: 15.5 and 5.8 us; there a tile took about 0.9 us whatever its size
 // (a producer's or an epilogue's latency per tile), and the dot products as long as HBM.
 // A launch starts with its code and its parameters in no near cache, so what it runs first is kept short: the split is multiplications by
