@@ -97,17 +97,19 @@ static uint32_t gqa4_cluster_ctas(const ib_ctx *ctx, const ib_attn_params &p, ui
 // of kv heads, the long one's does: with few heads it has more CTAs per head.  Measured us per launch, short / middle / long:
 //   head size 64:   4 kv heads  5.3 / 6.2 / 6.5 at 1536 positions, 6.1 / 6.6 / 7.0 at 2048;  8 heads  4.4 / 5.7 / 6.6 at 640, 4.9 / 5.9 / 6.8 at
 //                   1024, 6.7 / 6.3 / 7.6 at 1536;  16 (middle in clusters of 4)  5.0 / 6.0 / 7.0 at 768, 6.8 / 6.8 / 7.9 at 1024.
-//                   Middle against long: 18.9 / 22.4 at 16384 with 4 heads (26.0 / 24.6 at 24576), 20.2 / 21.0 with 8 (27.4 / 25.2), 20.5 / 23.1
-//                   with 12;  16 heads  8.9 / 9.9 at 2048, 12.4 / 12.6 at 4096 (11.7 / 11.1
-//                   from a cache that is still in L2), 16.2 / 15.6 at 6144.
+//                   Middle against long, launches back to back (caches that stay in L2): 8.3 / 7.4 at 5000 with 4 heads (12.3 / 9.2 at 10000),
+//                   7.6 / 7.5 at 4000 with 8 (10.9 / 9.2 at 8000, 17.4 / 12.3 at 16000), 8.4 / 8.3 at 5000 with 12 (14.0 / 12.4 at 12000), 7.6 /
+//                   6.9 at 2000 with 16.  Inside a token graph the middle regime leaves SMs for the next launch's CTAs, which is worth up to 1.3 us
+//                   (1B architecture, a layer of a token, 2000 positions: 26.5 / 27.9 us, 3000: 27.5 / 28.6): the limits lie that much further.
 //   head size 128:  8 kv heads  3.6 / 4.1 / 4.2 at 128, 4.0 / 4.2 / 4.5 at 192, 4.2 / 4.1 / 4.4 at 224, 5.0 / 4.5 / 6.2 at 512.
-//                   Middle against long: 7.9 / 7.9 at 2560 with 2 heads (8.7 / 8.1 at 3072), 9.1 / 9.3 with 4 (10.1 / 9.5), 10.3 / 10.6 at 3072
-//                   with 8 (12.1 / 11.7 at 4096), 10.4 / 11.5 at 3072 with 12;  16 heads  7.9 / 8.1 at 1024, 9.9 / 9.2 at 1536.
+//                   Middle against long: 6.8 / 6.1 at 2000 with 2 heads, 6.9 / 6.2 at 1800 with 4, 7.0 / 7.2 at 1800 with 8 (8.9 / 8.6 at 3000),
+//                   8.0 / 8.9 at 2500 with 12;  16 heads  5.7 / 6.1 at 600, 7.1 / 6.6 at 1000.  In the graph (a layer of the 8B shapes): 45.6 / 46.9
+//                   at 1900, 48.7 / 48.0 at 2700;  4 heads  28.3 / 29.9 at 1600.
 uint32_t attn_regime_positions(const ib_ctx *ctx, const AttnLaunch &a, uint32_t regime) {
     if (!attn_gqa4_eligible(a) || ctx->sm_count == 0) return 0u;
     const uint32_t n_kv = a.p.n_heads / a.p.kv_mul, middle = gqa4_cluster_ctas(ctx, a.p, ATTN_MIDDLE), c = gqa4_cluster_ctas(ctx, a.p, regime);
     const bool wide = a.p.head_size == 128;
-    if (regime == ATTN_MIDDLE) return c * (wide ? (c < 8 ? 256 : (n_kv <= 4 ? 320 : 384)) : (c < 8 ? 512 : 2048));
+    if (regime == ATTN_MIDDLE) return c * (wide ? (c < 8 ? 256 : (n_kv <= 4 ? 320 : (n_kv <= 8 ? 300 : 384))) : (c < 8 ? 512 : (n_kv <= 8 ? 800 : 1400)));
     if (middle == 0 || c < 8) return c * (wide && middle ? 24 : 64);
     return c * (wide ? 24 : (middle < 8 ? 96 : (n_kv <= 4 ? 256 : 128)));
 }

@@ -111,6 +111,7 @@ def test_attention(backend, kv_dtype, hs, n_heads, kv_mul, pos, seq):
     (128, 8, 512), (128, 8, 513), (128, 8, 3072), (128, 8, 3073), (128, 2, 1000), (128, 12, 700),
     (64, 4, 2048), (64, 4, 2049), (64, 12, 1024), (64, 12, 1025), (64, 12, 16385), (64, 16, 768), (64, 16, 769), (64, 16, 2048), (64, 16, 2049), (64, 26, 257),
     (128, 8, 192), (128, 8, 193), (128, 1, 2560), (128, 1, 2561), (128, 12, 3072), (128, 12, 3073), (128, 16, 192), (128, 16, 1024), (128, 16, 1025),
+    (64, 8, 6400), (64, 8, 6401), (64, 4, 6401), (64, 12, 11200), (64, 12, 11201), (128, 8, 2400), (128, 8, 2401),
     (128, 20, 97), (128, 26, 257), (64, 20, 768), (64, 20, 769), (64, 26, 512), (64, 26, 513), (128, 32, 512), (128, 32, 513), (64, 60, 200),
 ])
 def test_attention_slice_shapes(backend, hs, n_kv, total):
