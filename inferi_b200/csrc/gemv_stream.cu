@@ -110,7 +110,6 @@ __device__ __forceinline__ void consume_tiles(const GemvParams &p, const Consume
     const uint32_t add = swiglu ? half : together, row_of = g & (add - 1), b_off = swiglu && (g & half) ? c.pt * stride : 0;   // the up rows follow a full tile's gate rows
     const uint32_t part0 = c.part + 4 * (swiglu ? 2 * row_of + ((g & half) ? 1 : 0) : row_of), out_step = 4 * together;
     const bool writer = t == 0 && g < together;
-    const bool lone = FOUR && !lc.first;   // 4 rows: this lane's units are in the second block of a step, which the last step may lack
     uint32_t st = c.stream, par = 0, ring = c.ring;   // ring: address of stage st
 #pragma unroll 1
     for (;;) {
@@ -141,13 +140,15 @@ __device__ __forceinline__ void consume_tiles(const GemvParams &p, const Consume
             float v = 0.f;
             with_format<QT>(cur_type, [&](auto f) {   // straight-line code: the steps' loads and products overlap
                 if constexpr (FOUR) {
+                    // `lc.first` differs between formats (swap_stretches).  Where it does not hold, the lane's units are in the second
+                    // block of a step, which the last step may lack.
                     f.template unit<true>(lc, 0, ua[0]);
                     v = f.template dot<true>(row, lc, 0, B[0], B[1], ua[0]);
-                    if (c.nb == 1 && lone) v = 0.f;
+                    if (c.nb == 1 && !lc.first) v = 0.f;
                     if (c.nb > 2) {
                         f.template unit<true>(lc, 1, ua[1]);
                         const float y = f.template dot<true>(row, lc, 1, B[2], B[3], ua[1]);
-                        v += c.nb == 3 && lone ? 0.f : y;
+                        v += c.nb == 3 && !lc.first ? 0.f : y;
                     }
                 } else if constexpr (MODE == ROWS8_LONG) {
                     if (c.nb == NB_MAX) {

@@ -67,6 +67,16 @@ def test_tiny_model_all_quant_types(backend, kv_f16):
     check_loop(backend, TINY, w, kv_f16, prompt=[3, 500, 41, 7], n_gen=24)
 
 
+# q, k and v of three formats in rows of 33 and 35 blocks: 4 rows at a time, the last warp of a row has one block or three, and the formats
+# differ in which lanes' units fall to the block that is not there (their rows start at different banks)
+@pytest.mark.parametrize("heads,types", [(66, (quant.Q8_0, quant.Q5_K, quant.Q4_K)), (66, (quant.Q5_K, quant.Q8_0, quant.Q4_K)),
+                                         (70, (quant.Q5_K, quant.Q8_0, quant.Q4_K)), (70, (quant.Q4_K, quant.Q5_K, quant.Q8_0))])
+def test_wide_rows_of_mixed_formats(backend, heads, types):
+    cfg = Llama2Config(128 * heads, 256, 1, heads, heads // 2, 512, 64, 500000.0, 1e-5)
+    recipe = dict(TINY_RECIPE, attn_q=types[0], attn_k=types[1], attn_v=types[2], ffn_down=quant.Q4_K)
+    check_loop(backend, cfg, synth_weights(cfg, seed=3006, device="cuda", recipe=recipe), True, prompt=[3, 500, 41], n_gen=4)
+
+
 def test_token_graph_launch_count_and_oracle_tokens(backend):
     """A token is a graph of 5 kernels per layer + 3 (begin, classifier, end); the launch counter must say so, and the
     greedy tokens must be the oracle's."""
