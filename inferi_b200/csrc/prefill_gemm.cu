@@ -43,7 +43,7 @@ namespace ib {
 
 constexpr int PG_PRODUCERS = 8, PG_FOLD = 8, PG_W_MMA = 16, PG_W_X = 17, PG_W_RAW = 18;
 constexpr int PG_THREADS = 19 * 32;
-constexpr uint32_t PG_DSLOTS = 4;
+constexpr uint32_t PG_DSLOTS = 8;   // slots of the blocks' scales, each taken from the request of the raw block to the fold (more than the raw stages and the fold's delay)
 constexpr uint32_t PG_XSTAGES_MAX = 16;   // a stage holds the tokens' 64 columns, hi and lo: few tokens, small stages, more of them (launch)
 constexpr uint32_t PG_STILE = PF_CHUNK * 16 * 2;        // ... of 128 tokens x 16 sub-block sums
 constexpr uint32_t PG_SMEM_LIMIT = 227 * 1024;
@@ -179,8 +179,9 @@ __device__ __forceinline__ void pg_commit(uint32_t bar) {
     asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
 }
 // ---- between the two CTAs ----
-// (Waits keep the default scope also where the other CTA arrives: what the barriers order is tensor memory and bulk copies, and a wait that
-// acquires at cluster scope made every launch 1.2 to 1.4 times as long.)
+// (Arrivals and waits keep the default scope also across the pair: what those barriers order is tensor memory and bulk copies.  Waits that
+// acquire, or arrivals that release, at cluster scope make every launch 1.1 to 1.5 times as long.  Plain shared memory - the blocks' scales - is
+// ordered inside the CTA that it lies in, by rawempty, pdone and dempty.)
 __device__ __forceinline__ uint32_t pg_leader(uint32_t addr) {   // the same place in the pair's first CTA
     uint32_t a;
     asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(addr));
@@ -303,7 +304,7 @@ __device__ __forceinline__ uint32_t pg_pad(uint32_t n) { return (n + 15) & ~15u;
 
 template <int FMT>
 __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __grid_constant__ PgParams p, const __grid_constant__ PgMaps maps) {
-    constexpr bool MIN = pg_has_min(FMT);
+    constexpr bool MIN = pg_has_min(FMT), SCALED = FMT != PG_Q80;   // (Q8_0's operands carry their scales)
     constexpr uint32_t NS = pg_slots(FMT), R = pg_raw_stages(FMT), RAW = pg_raw_bytes(FMT), A0 = MIN ? PG_A4 : PG_A6, ACOLS = MIN ? 32 : 64;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -312,12 +313,12 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
     const uint32_t SS = (XS + 6) / 4, STILE = XTILE / 4;                            // ... that the ring's XS stages can touch (4 SS >= XS + 3)
     const uint32_t raw0 = (sst + (MIN ? SS * 2 * STILE : 0) + 127) & ~127u;          // raw blocks
     uint8_t *tail = smem + (raw0 - xst) + R * RAW;
-    float *dsm = reinterpret_cast<float *>(tail);                                   // [PG_DSLOTS][128] the block's scale of every row
+    float *dsm = reinterpret_cast<float *>(tail);                                   // [PG_DSLOTS][128] a block's scale of every row
     uint64_t *bars = reinterpret_cast<uint64_t *>(tail + PG_DSLOTS * 512);
     uint32_t nb = pg_smem(bars);
     auto take = [&](uint32_t n) { const uint32_t b = nb; nb += 8 * n; return b; };
     const uint32_t b_rawfull = take(R), b_rawempty = take(R), b_afull = take(NS), b_aempty = take(NS), b_xfull = take(PG_XSTAGES_MAX), b_xempty = take(PG_XSTAGES_MAX);
-    const uint32_t b_pdone = take(2), b_pfree = take(2);
+    const uint32_t b_pdone = take(PG_DSLOTS), b_dempty = take(PG_DSLOTS), b_pfree = take(2);
     const uint32_t b_zdone = take(1), b_zfree = take(1), s_tmem = nb;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const StreamK sk = p.sk;
@@ -328,11 +329,13 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
     if (warp == 0) {
         // A lane per barrier.  What the MMA warp waits for counts both CTAs and lives in the first one; the MMAs' completion arrives in both.
         constexpr uint32_t X0 = 2 * R + 2 * NS, P0 = X0 + 2 * PG_XSTAGES_MAX;
-        for (uint32_t i = lane; i < P0 + 6; i += 32) {
+        for (uint32_t i = lane; i < P0 + 2 * PG_DSLOTS + 4; i += 32) {
             uint32_t count = 1;
             if (i >= R && i < 2 * R + NS) count = PG_PRODUCERS;                                          // rawempty, afull
             else if (i >= X0 && i < X0 + PG_XSTAGES_MAX) count = rank == 0 ? 2 : 1;                       // xfull: the bytes, and word of the other CTA's
-            else if (i == P0 + 2 || i == P0 + 3 || i == P0 + 5) count = 2 * PG_FOLD;                      // pfree, zfree
+            else if (i >= P0 && i < P0 + PG_DSLOTS) count = SCALED ? 2 : 1;                               // pdone: the MMAs, and the scales
+            else if (i >= P0 + PG_DSLOTS && i < P0 + 2 * PG_DSLOTS) count = PG_FOLD;                      // dempty
+            else if (i >= P0 + 2 * PG_DSLOTS && i != P0 + 2 * PG_DSLOTS + 2) count = 2 * PG_FOLD;         // pfree, zfree
             pg_bar_init(b_rawfull + 8 * i, count);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -365,7 +368,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
             // registers that the conversions of other words cannot overlap in (Q6_K 4096 x 14336, 1000 tokens: 291 us against 383).
             uint4 hdr = make_uint4(0, 0, 0, 0), f0, f1, g0 = hdr, g1 = hdr;
             uint2 sc8 = make_uint2(0, 0);
-            float d;
+            float d = 1.0f;
             if constexpr (MIN) {
                 const uint32_t blk = raw + row * (FMT == PG_Q4K ? 144 : 176);
                 hdr = pg_lds128(blk);
@@ -378,7 +381,6 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
                 d = pg_h2f(pg_lds16(raw + PG_Q6_D + row * 16 + 2 * (cur.kb & 7)));
             } else {
                 sc8 = pg_lds64(raw + row * 272 + 256 + 8 * wg);   // f16 scales of the warpgroup's four blocks
-                d = 1.0f;
             }
 #pragma unroll
             for (uint32_t cc = 0; cc < 2; cc++) {
@@ -439,7 +441,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
                     pg_st16(ta + 16, a);
                     pg_st16(ta + 48, b);
                 }
-                if (cc == 0 && wg == 0) dsm[(j & (PG_DSLOTS - 1)) * 128 + row] = d;   // read by the fold warps behind the block's P
+                if (SCALED && cc == 0 && wg == 0) dsm[(j & (PG_DSLOTS - 1)) * 128 + row] = d;   // for the fold warps (the raw block was requested when the slot was free)
                 pg_wait_st();
                 pg_fence_before();
                 __syncwarp();
@@ -472,11 +474,16 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
                         for (int i = 0; i < 16; i++) Y[16 * g + i] = fmaf(f, __uint_as_float(r[i]), Y[16 * g + i]);
                     }
             };
-            const uint32_t pb = j & 1;
+            const uint32_t pb = j & 1, ds = j & (PG_DSLOTS - 1);
             const bool end = cur.kb + 1 == sk.nb || j + 1 == nunits;
-            if (!(ok = pg_wait_warp(b_pdone + 8 * pb, (j >> 1) & 1, p, 10))) break;
+            if (!(ok = pg_wait_warp(b_pdone + 8 * ds, (j / PG_DSLOTS) & 1, p, 10))) break;
             pg_fence_after();
-            const float d = dsm[(j & (PG_DSLOTS - 1)) * 128 + row];
+            float d = 1.0f;
+            if constexpr (SCALED) {
+                d = dsm[ds * 128 + row];
+                __syncwarp();
+                if (lane == 0) pg_arrive(b_dempty + 8 * ds);
+            }
             fold(PG_P + 128 * pb, d);
             pg_fence_before();
             __syncwarp();
@@ -538,7 +545,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
         const uint32_t x_hi32 = (uint32_t)(xd0 >> 32), s_hi32 = (uint32_t)(sd0 >> 32);
         // carried by additions: full barrier, parity and low descriptor word (start address) of the inputs' stage; barrier, parity and column of the weights'
         uint32_t bx = b_xfull, xpar = 0, xd = (uint32_t)xd0, ba = b_afull, apar = 0, a = tmem + A0, sd = (uint32_t)sd0, seg = 0;
-        uint32_t idesc = cur.chunk + 1 == p.chunks ? id_last : id_full, P = tmem + PG_P, bp = b_pdone, ppar = 1;
+        uint32_t idesc = cur.chunk + 1 == p.chunks ? id_last : id_full, P = tmem + PG_P, bp = b_pfree, ppar = 1, bd = b_pdone;
         bool begin = true, end = cur.kb + 1 == sk.nb || nunits == 1, ready = false;
         auto desc = [](uint32_t hi, uint32_t lo) { return ((uint64_t)hi << 32) | lo; };
         for (uint32_t j = 0; j < nunits; j++) {
@@ -548,7 +555,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
             for (uint32_t c = 0; c < 4; c++) {
                 if (!ready) {
                     // (the first two blocks find the P buffers free: waiting for the parity before the first phase succeeds)
-                    if (c == 0 && !(ok = pg_wait_warp(bp + 16, ppar, p, 9))) break;
+                    if (c == 0 && !(ok = pg_wait_warp(bp, ppar, p, 9))) break;
                     if (!(ok = __all_sync(0xffffffffu, pg_wait(bx, xpar, p, 9) && pg_wait(ba, apar, p, 9)))) break;
                 }
                 if (MIN && c == 3 && begin && seg && !(ok = pg_wait_warp(b_zfree, (seg - 1) & 1, p, 9))) break;
@@ -561,7 +568,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
                 ba += 8;
                 if (ba == b_afull + 8 * NS) { ba = b_afull; a = tmem + A0; apar ^= 1u; }
                 bool next = pg_test(bx, xpar) & pg_test(ba, apar);
-                if (c == 3) next &= pg_test((bp ^ (b_pdone ^ (b_pdone + 8))) + 16, bp == b_pdone ? ppar : ppar ^ 1u);
+                if (c == 3) next &= pg_test(bp ^ (b_pfree ^ (b_pfree + 8)), bp == b_pfree ? ppar : ppar ^ 1u);
                 if (c == 2) {
                     cur.next(p);
                     begin_next = cur.kb == 0;
@@ -576,7 +583,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
                         pg_mma(P, col + 8 * kk, desc(x_hi32, xh + xlo + ko), idesc, 1);
                         if (!MIN) pg_mma(P, col + 32 + 8 * kk, desc(x_hi32, xh + ko), idesc, 1);
                     }
-                    if (c == 3) pg_commit(bp);
+                    if (c == 3) pg_commit(bd);
                     if (MIN && c == 3) {
                         // the block's minimums x sums: hi * hi, hi * lo, lo * hi
                         const uint32_t m = tmem + PG_M4 + 16 * (j & 1);
@@ -599,8 +606,9 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
             begin = begin_next;
             end = end_next;
             P ^= (PG_P ^ (PG_P + 128));
-            if (bp == b_pdone) bp = b_pdone + 8;
-            else { bp = b_pdone; ppar ^= 1u; }
+            if (bp == b_pfree) bp = b_pfree + 8;
+            else { bp = b_pfree; ppar ^= 1u; }
+            bd = bd + 8 == b_dempty ? b_pdone : bd + 8;
         }
     } else if (warp == PG_W_X) {
         // ===== this CTA's half of the tokens' inputs (a bulk copy per 64 columns) and, per block, of their sub-block sums =====
@@ -636,8 +644,18 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
         PgCursor cur;
         cur.init(p, u0);
         uint32_t slot = 0, use = 0;
-        for (uint32_t j = 0; j < nunits && ok; j++) {
-            if (use && !(ok = pg_wait_warp(b_rawempty + 8 * slot, (use - 1) & 1, p, 8))) break;
+        for (uint32_t j = 0; j < nunits + (SCALED ? R : 0) && ok; j++) {
+            if (use) {
+                if (!(ok = pg_wait_warp(b_rawempty + 8 * slot, (use - 1) & 1, p, 8))) break;
+                // Block j - R has been read, so its scales are there too: this warp says so on the producers' behalf (they are short of time).
+                if (SCALED && pg_elect()) pg_arrive(b_pdone + 8 * ((j - R) & (PG_DSLOTS - 1)));
+                __syncwarp();
+            }
+            if (SCALED && j >= nunits) {
+                if (++slot == R) { slot = 0; use++; }
+                continue;
+            }
+            if (SCALED && j >= PG_DSLOTS && !(ok = pg_wait_warp(b_dempty + 8 * (j & (PG_DSLOTS - 1)), (j / PG_DSLOTS - 1) & 1, p, 8))) break;   // its scales' slot is free
             const uint32_t rt = 2 * cur.rt + rank, s = rt >= p.tile0[2] ? 2 : (rt >= p.tile0[1] ? 1 : 0), y = (rt - p.tile0[s]) * 128;
             const uint32_t full = b_rawfull + 8 * slot, dst = raw0 + slot * RAW;
             const CUtensorMap *m = maps.m[s];

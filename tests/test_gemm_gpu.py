@@ -61,6 +61,20 @@ def test_gemm_halves_of_a_pair(backend, qt, rows, n):
     test_gemm_across_chunks_of_tokens(backend, qt, rows, 2048, n)
 
 
+# 17 blocks per pair of SMs: the eight slots of the blocks' scales go round twice, and every block has scales of its own.  The same call gives the same bits.
+@pytest.mark.parametrize("qt", [quant.Q4_K, quant.Q5_K, quant.Q6_K, quant.Q8_0])
+def test_gemm_scales_of_long_ranges(backend, qt):
+    rows, cols, n = 2048, 10240, 400
+    test_gemm_across_chunks_of_tokens(backend, qt, rows, cols, n)
+    m = GpuQuantTensor(backend, qt, rows, cols, quant.random_blocks(qt, rows, cols, seed=5, scale=0.05))
+    x = torch.from_numpy(np.random.default_rng(6).standard_normal((n, cols)).astype(np.float32)).cuda()
+    out = [torch.empty(n, rows, device="cuda") for _ in range(4)]
+    for o in out:
+        GemmQuant(backend).launch(o, m, x)
+    assert all(torch.equal(o, out[0]) for o in out)
+    m.close()
+
+
 @pytest.mark.parametrize("qt,rows,cols,n", [
     (quant.Q6_K, 128, 34816, 2), (quant.Q6_K, 256, 34816, 130), (quant.Q8_0, 128, 33024, 9),
 ])
