@@ -781,10 +781,11 @@ static int32_t prefill_prepare(ib_llama *m, uint32_t n) {
             const ib_qtensor *sets[4][3] = {{w.attn_q, w.attn_k, w.attn_v}, {w.attn_output}, {w.ffn_gate, w.ffn_up}, {w.ffn_down}};
             const uint32_t counts[4] = {3, 1, 2, 1};
             for (int k = 0; k < 4; k++)
-                for (uint32_t ch = 1; ch <= chunks; ch++) {
+                for (uint32_t ch = 0; ch <= chunks + 1; ch++) {   // (passes of few tokens have other tiles)
+                    const uint32_t pass = ch == 0 ? PF_SINGLE_ALWAYS : (ch == 1 ? PF_SINGLE_TOKENS : (ch - 1) * PF_CHUNK);
                     PrefillGroup g[3];
                     size_t sum = 0;
-                    for (uint32_t i = 0, ng = prefill_groups(sets[k], counts[k], g); i < ng; i++) sum += prefill_plane_floats(m->ctx, g[i], ch * PF_CHUNK);
+                    for (uint32_t i = 0, ng = prefill_groups(sets[k], counts[k], g); i < ng; i++) sum += prefill_plane_floats(m->ctx, g[i], pass);
                     planes = sum > planes ? sum : planes;
                 }
         }

@@ -17,7 +17,7 @@ namespace ib {
 __device__ __forceinline__ F8 pf_sum8(const PfPlanes &g, uint32_t t, uint32_t r) {
     const size_t at = (size_t)t * g.rows + r, plane = (size_t)g.n * g.rows;
     F8 v = pf_load8u(g.plane0 + at);
-    const uint32_t np = g.sk.pieces((r / PF_TILE_ROWS) * g.chunks + t / PF_CHUNK);
+    const uint32_t np = g.sk.pieces(g.sk.row_tile(r) * g.chunks + t / PF_CHUNK);
     for (uint32_t s = 1; s < np; s += 2) {
         const F8 a = pf_load8(g.planes + (s - 1) * plane + at);
         if (s + 1 < np) {
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(256) prefill_finish_kernel(float *out, const P
     const uint32_t per = add.rows / 8, i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= add.n * per) return;
     const uint32_t t = i / per, r = (i - t * per) * 8;
-    if (add.sk.pieces((r / PF_TILE_ROWS) * add.chunks + t / PF_CHUNK) == 1) return;
+    if (add.sk.pieces(add.sk.row_tile(r) * add.chunks + t / PF_CHUNK) == 1) return;
     const F8 v = pf_sum8(add, t, r);   // plane 0 is `out`
     float *o = out + (size_t)t * add.rows + r;
     if (((uintptr_t)o & 15) == 0) { pf_store8(o, v); return; }
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(256) prefill_finish_narrow_kernel(float *out, 
     pf_enter();
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= add.n * add.rows) return;
-    const uint32_t t = i / add.rows, r = i - t * add.rows, np = add.sk.pieces((r / PF_TILE_ROWS) * add.chunks + t / PF_CHUNK);
+    const uint32_t t = i / add.rows, r = i - t * add.rows, np = add.sk.pieces(add.sk.row_tile(r) * add.chunks + t / PF_CHUNK);
     if (np == 1) return;
     const size_t plane = (size_t)add.n * add.rows;
     const float *p = add.planes + i;

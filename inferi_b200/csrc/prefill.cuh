@@ -12,18 +12,22 @@ constexpr uint32_t PF_CHUNK = 128;             // tokens per GEMM tile (the N of
 constexpr uint32_t PREFILL_MAX_TOKENS = 1024;
 constexpr uint32_t PF_MAX_SEGS = 3;            // matrices of one GEMM launch
 
-// How a prefill GEMM's work is handed out: the units (256-row tile, chunk of 128 tokens, 256-column block), in that order, are
-// cut into `pairs` contiguous, equally long ranges - one per pair of CTAs of a grid that fills the GPU exactly once, whatever the
+// A tile of the prefill GEMM is 256 rows on a pair of SMs that share the tokens' inputs, or 128 rows on one SM: up to 16 tokens, and up to 64
+// where no SM gets more than one unit of work (prefill_streamk).
+constexpr uint32_t PF_SINGLE_ALWAYS = 16, PF_SINGLE_TOKENS = 64;
+
+// How a prefill GEMM's work is handed out: the units (row tile, chunk of 128 tokens, 256-column block), in that order, are
+// cut into contiguous, equally long ranges - one per CTA or pair of CTAs of a grid that fills the GPU exactly once, whatever the
 // matrix's shape (a grid of tiles x K slices was 1.5 waves for the FFN matrices).  The K range of a tile (= row tile and
-// chunk) can then fall to several pairs; each writes its partial sums to the plane numbered by its position among the tile's
-// pairs, and the element-wise kernel behind the GEMM adds a tile's planes in that order.
-constexpr uint32_t PF_TILE_ROWS = 256;         // rows of a pair's tile, half of them per CTA
+// chunk) can then fall to several ranges; each CTA or pair writes its partial sums to the plane numbered by its position among the
+// tile's, and the element-wise kernel behind the GEMM adds a tile's planes in that order.
 struct StreamK {
-    uint32_t pairs, nb, total;   // pairs of CTAs, 256-column blocks per row, units = tiles * nb
+    uint32_t ranges, nb, total, row_log2;   // ranges, 256-column blocks per row, units = tiles * nb, rows of a tile (log2)
     // 32-bit arithmetic: the launcher keeps total below 2^24
-    __host__ __device__ uint32_t first_unit(uint32_t c) const { return c * total / pairs; }
-    __host__ __device__ uint32_t pair_of(uint32_t u) const { return ((u + 1) * pairs - 1) / total; }
-    __host__ __device__ uint32_t pieces(uint32_t tile) const { return pair_of(tile * nb + nb - 1) - pair_of(tile * nb) + 1; }
+    __host__ __device__ uint32_t first_unit(uint32_t c) const { return c * total / ranges; }
+    __host__ __device__ uint32_t range_of(uint32_t u) const { return ((u + 1) * ranges - 1) / total; }
+    __host__ __device__ uint32_t pieces(uint32_t tile) const { return range_of(tile * nb + nb - 1) - range_of(tile * nb) + 1; }
+    __host__ __device__ uint32_t row_tile(uint32_t row) const { return row >> row_log2; }
 };
 StreamK prefill_streamk(const ib_ctx *ctx, uint32_t rows, uint32_t cols, uint32_t n);
 uint32_t prefill_max_pieces(const StreamK &sk);   // bound of the planes that any tile needs
@@ -33,7 +37,7 @@ struct PgParams {
     uint32_t rows, n, chunks;      // rows of all matrices together, tokens, chunks of 128 tokens
     const __half *x;               // the tokens' inputs split into two f16, tiled (pf_x_index); per chunk x_chunk halves
     size_t x_chunk;
-    float *plane0, *planes;        // [n][rows] the first pair's sums of every tile; [piece - 1][n][rows] the others'
+    float *plane0, *planes;        // [n][rows] the first range's sums of every tile; [piece - 1][n][rows] the others'
     uint32_t x_stages, x_tile;     // ring of the inputs: stages, bytes of a stage's hi (= lo) half (set by the launcher)
     StreamK sk;
     uint32_t *err;
@@ -59,7 +63,7 @@ __host__ __device__ inline uint32_t pf_s_index(uint32_t t, uint32_t sb, uint32_t
 __host__ __device__ inline size_t pf_x_halves(uint32_t cols) { return (size_t)2 * (PF_CHUNK + 8) * cols; }   // halves per chunk
 
 bool prefill_gemm_eligible(const ib_qtensor *m);
-// plane0 / planes = partial sums of W x_t over the K ranges of the tile's pairs of CTAs; x: the layout above, token rows n .. (n rounded
+// plane0 / planes = partial sums of W x_t over the tile's K ranges; x: the layout above, token rows n .. (n rounded
 // up to 16) - 1 of the last chunk zero; early: the weights may be read before the stream's previous kernels are done.  The matrices of a launch have the same type and width; their rows follow one another.
 int32_t launch_prefill_gemm(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *const *mats, uint32_t n_mats, const __half *x, uint32_t n, float *plane0,
                             float *planes, const StreamK &sk, bool early = true);

@@ -1,5 +1,5 @@
 // The GEMM of the prompt prefill: out^T tile = W tile (256 rows of a quantized matrix) x X^T (up to 128 tokens), on the
-// 5th-generation tensor cores (tcgen05.mma, f32 accumulators in tensor memory) of a pair of SMs.
+// 5th-generation tensor cores (tcgen05.mma, f32 accumulators in tensor memory) of a pair of SMs; few tokens: 128 rows on one SM.
 //
 // Exact integer weights.  A k-quant weight is w = d * (sc * q) - dmin * m with d, dmin one f16 (pair) per 256 columns and
 // row, sc a 6- or 8-bit integer, q a small integer (crates/inferi/src/quantization.rs:227-402).  sc * q is an integer; per
@@ -19,7 +19,8 @@
 // shared, half of them in either's shared memory.  On one SM a 256-column block of 128 rows took 131 KB of inputs from L2 for 2240
 // clocks of MMAs, and L2 delivers 72 bytes a nanosecond to an SM: 9.5 of at most 10.7 TB/s, 4000 clocks a block.  Now 2490 (Q4_K).
 // Measured, one SM / two: Q4_K 14336 x 4096, 900 tokens 218 / 185 us; with Q6_K's conversions (below) 4096 x 14336, 1000 tokens 383 /
-// 288; a prompt of 1021 tokens of the 8B architecture 39.8 / 33.1 ms, of 128 tokens 6.24 / 5.36.
+// 288; a prompt of 1021 tokens of the 8B architecture 39.8 / 33.1 ms, of 128 tokens 6.24 / 5.36.  With few tokens L2 has little to deliver, and one
+// SM per tile (PAIR = false, cta_group::1) is the faster way: prefill_streamk.
 //
 // Who does what (19 warps, one CTA per SM; the MMAs of both are issued by the first):
 //   warps 0-7    producers: two warpgroups, each two of the block's four 64-column chunks
@@ -165,32 +166,65 @@ __device__ __forceinline__ void pg_wait_ld() { asm volatile("tcgen05.wait::ld.sy
 __device__ __forceinline__ uint64_t pg_desc(uint32_t smem_addr, uint32_t lbo, uint32_t sbo) {
     return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | (uint64_t)((lbo >> 4) & 0x3FFFu) << 16 | (uint64_t)((sbo >> 4) & 0x3FFFu) << 32 | (uint64_t)1 << 46;
 }
-// Instruction descriptor of kind::f16: f16 A and B (both K-major), f32 accumulator, 256 x N.
-__device__ __forceinline__ uint32_t pg_idesc(uint32_t N) { return (1u << 4) | ((N >> 3) << 17) | ((256u >> 4) << 24); }
-// D[256 x N] (+)= A (tensor memory, 16 columns of f16 = 8 columns of 32 bits) x B (shared memory), on both SMs of the pair: each has its
-// 128 rows of A and D in its own tensor memory and half of B's N rows in its own shared memory, at the same places.
+// Instruction descriptor of kind::f16: f16 A and B (both K-major), f32 accumulator, M x N.
+__device__ __forceinline__ uint32_t pg_idesc(uint32_t M, uint32_t N) { return (1u << 4) | ((N >> 3) << 17) | ((M >> 4) << 24); }
+// D[128 x N] (+)= A (tensor memory, 16 columns of f16 = 8 columns of 32 bits) x B (shared memory).  PAIR: D[256 x N] on both SMs of the
+// pair: each has its 128 rows of A and D in its own tensor memory and half of B's N rows in its own shared memory, at the same places.
+template <bool PAIR>
 __device__ __forceinline__ void pg_mma(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc, uint32_t accumulate) {
-    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc),
-                 "r"(idesc), "r"(accumulate)
-                 : "memory");
+    if constexpr (PAIR)
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem), "r"(a_tmem),
+                     "l"(b_desc), "r"(idesc), "r"(accumulate)
+                     : "memory");
+    else
+        asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}" ::"r"(d_tmem), "r"(a_tmem),
+                     "l"(b_desc), "r"(idesc), "r"(accumulate)
+                     : "memory");
 }
-// arrives, when the MMAs issued so far are done, on the barrier at this place in both CTAs
+// arrives, when the MMAs issued so far are done, on the barrier (PAIR: on the barrier at this place in both CTAs)
+template <bool PAIR>
 __device__ __forceinline__ void pg_commit(uint32_t bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+    if constexpr (PAIR)
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar), "h"((uint16_t)3) : "memory");
+    else asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+}
+// the whole tensor memory; its address is left at shared address `at`
+template <bool PAIR>
+__device__ __forceinline__ void pg_alloc(uint32_t at) {
+    if constexpr (PAIR) {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    } else {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(at), "r"(512u) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+}
+template <bool PAIR>
+__device__ __forceinline__ void pg_dealloc(uint32_t tmem) {
+    if constexpr (PAIR) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
 // ---- between the two CTAs ----
 // (Arrivals and waits keep the default scope also across the pair: what those barriers order is tensor memory and bulk copies.  Waits that
 // acquire, or arrivals that release, at cluster scope make every launch 1.1 to 1.5 times as long.  Plain shared memory - the blocks' scales - is
 // ordered inside the CTA that it lies in, by rawempty, pdone and dempty.)
+template <bool PAIR>
 __device__ __forceinline__ uint32_t pg_leader(uint32_t addr) {   // the same place in the pair's first CTA
-    uint32_t a;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(addr));
+    uint32_t a = addr;
+    if constexpr (PAIR) asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(a) : "r"(addr));
     return a;
 }
-__device__ __forceinline__ void pg_arrive_cluster(uint32_t addr) { asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory"); }
-__device__ __forceinline__ void pg_cluster_sync() {
-    asm volatile("barrier.cluster.arrive.release;" ::: "memory");
-    asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+template <bool PAIR>
+__device__ __forceinline__ void pg_arrive_leader(uint32_t addr) {   // addr: from pg_leader
+    if constexpr (PAIR) asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(addr) : "memory");
+    else pg_arrive(addr);
+}
+template <bool PAIR>
+__device__ __forceinline__ void pg_sync() {
+    if constexpr (PAIR) {
+        asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+    } else __syncthreads();
 }
 __device__ __forceinline__ void pg_tma2d(uint32_t dst, const CUtensorMap *map, uint32_t x, uint32_t y, uint32_t bar) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
@@ -284,7 +318,7 @@ __device__ __forceinline__ void pg_scales(const uint4 &hdr, uint32_t c, uint32_t
 
 // The current unit of a role's walk over its CTA's range, carried forward by additions
 struct PgCursor {
-    uint32_t rt, chunk, kb;   // row tile of the pair, chunk of 128 tokens, 256-column block
+    uint32_t rt, chunk, kb;   // row tile (128 rows, of a pair 256), chunk of 128 tokens, 256-column block
     __device__ __forceinline__ void init(const PgParams &p, uint32_t u) {
         const uint32_t tile = u / p.sk.nb;
         kb = u - tile * p.sk.nb;
@@ -302,9 +336,10 @@ struct PgCursor {
 };
 __device__ __forceinline__ uint32_t pg_pad(uint32_t n) { return (n + 15) & ~15u; }
 
-template <int FMT>
+template <int FMT, bool PAIR>
 __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __grid_constant__ PgParams p, const __grid_constant__ PgMaps maps) {
     constexpr bool MIN = pg_has_min(FMT), SCALED = FMT != PG_Q80;   // (Q8_0's operands carry their scales)
+    constexpr uint32_t CTAS = PAIR ? 2 : 1;
     constexpr uint32_t NS = pg_slots(FMT), R = pg_raw_stages(FMT), RAW = pg_raw_bytes(FMT), A0 = MIN ? PG_A4 : PG_A6, ACOLS = MIN ? 32 : 64;
     extern __shared__ __align__(1024) uint8_t smem_raw[];
     uint8_t *smem = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
@@ -322,8 +357,8 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
     const uint32_t b_zdone = take(1), b_zfree = take(1), s_tmem = nb;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const StreamK sk = p.sk;
-    const uint32_t pair = blockIdx.x >> 1, rank = blockIdx.x & 1;   // clusters of two CTAs along x
-    const uint32_t u0 = sk.first_unit(pair), nunits = sk.first_unit(pair + 1) - u0;
+    const uint32_t range = PAIR ? blockIdx.x >> 1 : blockIdx.x, rank = PAIR ? blockIdx.x & 1 : 0;   // pairs: clusters of two CTAs along x
+    const uint32_t u0 = sk.first_unit(range), nunits = sk.first_unit(range + 1) - u0;
 
     asm volatile("griddepcontrol.launch_dependents;");
     if (warp == 0) {
@@ -331,21 +366,19 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
         constexpr uint32_t X0 = 2 * R + 2 * NS, P0 = X0 + 2 * PG_XSTAGES_MAX;
         for (uint32_t i = lane; i < P0 + 2 * PG_DSLOTS + 4; i += 32) {
             uint32_t count = 1;
-            if (i >= R && i < 2 * R + NS) count = PG_PRODUCERS;                                          // rawempty, afull
-            else if (i >= X0 && i < X0 + PG_XSTAGES_MAX) count = rank == 0 ? 2 : 1;                       // xfull: the bytes, and word of the other CTA's
+            if (i >= R && i < 2 * R) count = PG_PRODUCERS;                                                // rawempty
+            else if (i >= 2 * R && i < 2 * R + NS) count = CTAS * PG_PRODUCERS / 2;                       // afull
+            else if (i >= X0 && i < X0 + PG_XSTAGES_MAX) count = rank == 0 ? CTAS : 1;                    // xfull: the bytes, and word of the other CTA's
             else if (i >= P0 && i < P0 + PG_DSLOTS) count = SCALED ? 2 : 1;                               // pdone: the MMAs, and the scales
             else if (i >= P0 + PG_DSLOTS && i < P0 + 2 * PG_DSLOTS) count = PG_FOLD;                      // dempty
-            else if (i >= P0 + 2 * PG_DSLOTS && i != P0 + 2 * PG_DSLOTS + 2) count = 2 * PG_FOLD;         // pfree, zfree
+            else if (i >= P0 + 2 * PG_DSLOTS && i != P0 + 2 * PG_DSLOTS + 2) count = CTAS * PG_FOLD;      // pfree, zfree
             pg_bar_init(b_rawfull + 8 * i, count);
         }
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
-    if (warp == PG_W_MMA) {
-        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(s_tmem), "r"(512u) : "memory");
-        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-    }
+    if (warp == PG_W_MMA) pg_alloc<PAIR>(s_tmem);
     pg_fence_before();
-    pg_cluster_sync();
+    pg_sync<PAIR>();
     pg_fence_after();
     uint32_t tmem;
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(tmem) : "r"(s_tmem));
@@ -353,7 +386,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
 
     if (warp < PG_PRODUCERS) {
         // ===== producers: thread = row; warpgroup `wg` makes chunks 2 wg and 2 wg + 1 of every block =====
-        const uint32_t row = tid & 127, wg = warp >> 2, tl = tmem + ((uint32_t)((warp & 3) * 32) << 16), lead_afull = pg_leader(b_afull);
+        const uint32_t row = tid & 127, wg = warp >> 2, tl = tmem + ((uint32_t)((warp & 3) * 32) << 16), lead_afull = pg_leader<PAIR>(b_afull);
         if (MIN && wg == 0) {   // columns 4..7 of the minimums' operands (sub-blocks 8..15 of a K = 16 MMA) stay zero
             for (uint32_t m = 0; m < 4; m++)
                 for (uint32_t c = 4; c < 8; c++) pg_st1(tl + PG_M4 + 8 * m + c, 0u);
@@ -445,7 +478,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
                 pg_wait_st();
                 pg_fence_before();
                 __syncwarp();
-                if (lane == 0) pg_arrive_cluster(lead_afull + 8 * as);
+                if (lane == 0) pg_arrive_leader<PAIR>(lead_afull + 8 * as);
             }
             if (++slot == R) { slot = 0; rpar ^= 1u; }
             cur.next(p);
@@ -454,7 +487,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
     } else if (warp < PG_PRODUCERS + PG_FOLD) {
         // ===== fold: thread = row (tensor-memory lane), 64 of the tokens =====
         const uint32_t row = (warp & 3) * 32 + lane, half = (warp - PG_PRODUCERS) >> 2, tl = tmem + ((uint32_t)((warp & 3) * 32) << 16) + 64 * half;
-        const uint32_t lead_pfree = pg_leader(b_pfree), lead_zfree = pg_leader(b_zfree);
+        const uint32_t lead_pfree = pg_leader<PAIR>(b_pfree), lead_zfree = pg_leader<PAIR>(b_zfree);
         float Y[64];
 #pragma unroll
         for (int i = 0; i < 64; i++) Y[i] = 0.f;
@@ -487,7 +520,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
             fold(PG_P + 128 * pb, d);
             pg_fence_before();
             __syncwarp();
-            if (lane == 0) pg_arrive_cluster(lead_pfree + 8 * pb);
+            if (lane == 0) pg_arrive_leader<PAIR>(lead_pfree + 8 * pb);
             if (end) {
                 if (MIN) {
                     if (!(ok = pg_wait_warp(b_zdone, seg & 1, p, 10))) break;
@@ -495,10 +528,10 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
                     fold(PG_Z, -1.0f);
                     pg_fence_before();
                     __syncwarp();
-                    if (lane == 0) pg_arrive_cluster(lead_zfree);
+                    if (lane == 0) pg_arrive_leader<PAIR>(lead_zfree);
                 }
                 seg++;
-                const uint32_t piece = pair - sk.pair_of(cur.tile(p) * sk.nb), rt = 2 * cur.rt + rank;   // (the last tile may lack its second half)
+                const uint32_t piece = range - sk.range_of(cur.tile(p) * sk.nb), rt = CTAS * cur.rt + rank;   // (a pair's last tile may lack its second half)
                 float *out = (piece == 0 ? p.plane0 : p.planes + (size_t)(piece - 1) * p.n * p.rows) + (size_t)(chunk * PF_CHUNK + 64 * half) * p.rows + rt * 128 + row;
                 const uint32_t count = rt * 128 < p.rows && nt > 64 * half ? nt - 64 * half : 0;
                 // (straight stores where 16 tokens are there: this code runs once or twice per launch, and its length is what it costs)
@@ -520,13 +553,13 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
             }
             cur.next(p);
         }
-    } else if (warp == PG_W_MMA && rank != 0) {
+    } else if (PAIR && warp == PG_W_MMA && rank != 0) {
         // ===== the second CTA issues no MMAs: it tells the first one when its half of a stage's inputs is there =====
-        const uint32_t lead_xfull = pg_leader(b_xfull);
+        const uint32_t lead_xfull = pg_leader<PAIR>(b_xfull);
         uint32_t xs = 0, par = 0;
         for (uint32_t i = 0; i < 4 * nunits && ok; i++) {
             if (!(ok = pg_wait_warp(b_xfull + 8 * xs, par, p, 9))) break;
-            if (pg_elect()) pg_arrive_cluster(lead_xfull + 8 * xs);
+            if (pg_elect()) pg_arrive_leader<PAIR>(lead_xfull + 8 * xs);
             __syncwarp();
             if (++xs == XS) { xs = 0; par ^= 1u; }
         }
@@ -539,7 +572,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
         // fit in that.  So everything the next stage needs - whether its barriers are complete, the next block's descriptor -
         // is asked for ahead of the current stage's MMAs.  A block's sums arrive with its first inputs and its minimums with
         // its weights: the minimums' MMAs at the end of the block wait for nothing of their own.
-        const uint32_t id_full = pg_idesc(PF_CHUNK), id_last = pg_idesc(pg_pad(p.n - (p.chunks - 1) * PF_CHUNK));
+        const uint32_t id_full = pg_idesc(128 * CTAS, PF_CHUNK), id_last = pg_idesc(128 * CTAS, pg_pad(p.n - (p.chunks - 1) * PF_CHUNK));
         const uint32_t xstep = 2 * XTILE >> 4, sstep = 2 * STILE >> 4, xlo = PF_X_LO * 2 >> 4, slo = PF_S_LO * 2 >> 4;
         const uint32_t bx_end = b_xfull + 8 * XS, sd_end = (uint32_t)sd0 + SS * sstep, x_empty = b_xempty - b_xfull, a_empty = b_aempty - b_afull;
         const uint32_t x_hi32 = (uint32_t)(xd0 >> 32), s_hi32 = (uint32_t)(sd0 >> 32);
@@ -579,21 +612,21 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
 #pragma unroll
                     for (uint32_t kk = 0; kk < 4; kk++) {
                         const uint32_t ko = kk * (2 * PG_LBO >> 4);
-                        pg_mma(P, col + 8 * kk, desc(x_hi32, xh + ko), idesc, !(c == 0 && kk == 0));   // every block starts a new P
-                        pg_mma(P, col + 8 * kk, desc(x_hi32, xh + xlo + ko), idesc, 1);
-                        if (!MIN) pg_mma(P, col + 32 + 8 * kk, desc(x_hi32, xh + ko), idesc, 1);
+                        pg_mma<PAIR>(P, col + 8 * kk, desc(x_hi32, xh + ko), idesc, !(c == 0 && kk == 0));   // every block starts a new P
+                        pg_mma<PAIR>(P, col + 8 * kk, desc(x_hi32, xh + xlo + ko), idesc, 1);
+                        if (!MIN) pg_mma<PAIR>(P, col + 32 + 8 * kk, desc(x_hi32, xh + ko), idesc, 1);
                     }
-                    if (c == 3) pg_commit(bd);
+                    if (c == 3) pg_commit<PAIR>(bd);
                     if (MIN && c == 3) {
                         // the block's minimums x sums: hi * hi, hi * lo, lo * hi
                         const uint32_t m = tmem + PG_M4 + 16 * (j & 1);
-                        pg_mma(tmem + PG_Z, m, desc(s_hi32, sd), idesc, !begin);
-                        pg_mma(tmem + PG_Z, m, desc(s_hi32, sd + slo), idesc, 1);
-                        pg_mma(tmem + PG_Z, m + 8, desc(s_hi32, sd), idesc, 1);
-                        if (end) pg_commit(b_zdone);
+                        pg_mma<PAIR>(tmem + PG_Z, m, desc(s_hi32, sd), idesc, !begin);
+                        pg_mma<PAIR>(tmem + PG_Z, m, desc(s_hi32, sd + slo), idesc, 1);
+                        pg_mma<PAIR>(tmem + PG_Z, m + 8, desc(s_hi32, sd), idesc, 1);
+                        if (end) pg_commit<PAIR>(b_zdone);
                     }
-                    pg_commit(ca);
-                    pg_commit(cx);
+                    pg_commit<PAIR>(ca);
+                    pg_commit<PAIR>(cx);
                 }
                 __syncwarp();
                 ready = __all_sync(0xffffffffu, next);
@@ -611,13 +644,13 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
             bd = bd + 8 == b_dempty ? b_pdone : bd + 8;
         }
     } else if (warp == PG_W_X) {
-        // ===== this CTA's half of the tokens' inputs (a bulk copy per 64 columns) and, per block, of their sub-block sums =====
+        // ===== the tokens' inputs, of a pair this CTA's half of them (a bulk copy per 64 columns) and, per block, of their sub-block sums =====
         asm volatile("griddepcontrol.wait;" ::: "memory");   // the previous kernel writes them
         PgCursor cur;
         cur.init(p, u0);
         uint32_t xs = 0, use = 0, ss = 0;
         for (uint32_t j = 0; j < nunits && ok; j++) {
-            const uint32_t tokens = pg_pad(cur.tokens(p)) / 2;
+            const uint32_t tokens = pg_pad(cur.tokens(p)) / CTAS;
             const __half *x = p.x + (size_t)cur.chunk * p.x_chunk;
             for (uint32_t c = 0; c < 4; c++) {
                 if (use && !(ok = pg_wait_warp(b_xempty + 8 * xs, (use - 1) & 1, p, 8))) break;
@@ -656,7 +689,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
                 continue;
             }
             if (SCALED && j >= PG_DSLOTS && !(ok = pg_wait_warp(b_dempty + 8 * (j & (PG_DSLOTS - 1)), (j / PG_DSLOTS - 1) & 1, p, 8))) break;   // its scales' slot is free
-            const uint32_t rt = 2 * cur.rt + rank, s = rt >= p.tile0[2] ? 2 : (rt >= p.tile0[1] ? 1 : 0), y = (rt - p.tile0[s]) * 128;
+            const uint32_t rt = CTAS * cur.rt + rank, s = rt >= p.tile0[2] ? 2 : (rt >= p.tile0[1] ? 1 : 0), y = (rt - p.tile0[s]) * 128;
             const uint32_t full = b_rawfull + 8 * slot, dst = raw0 + slot * RAW;
             const CUtensorMap *m = maps.m[s];
             if (pg_elect()) {
@@ -683,15 +716,15 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
         while (pg_ns() - t0 < 100000ull) {}
     }
     if (warp == PG_W_MMA && ok) {
-        // The last MMAs' commits arrive in both CTAs' shared memory: let them, before either CTA can end.
+        // The last MMAs' commits arrive in shared memory, a pair's in both CTAs': let them, before a CTA can end.
         const uint32_t last = 4 * nunits - 1;
         pg_wait_warp(b_aempty + 8 * (last % NS), (last / NS) & 1, p, 9);
         pg_wait_warp(b_xempty + 8 * (last % XS), (last / XS) & 1, p, 9);
     }
     __syncwarp();
     pg_fence_before();
-    pg_cluster_sync();   // the other CTA's shared and tensor memory are in use until here
-    if (warp == PG_W_MMA) asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
+    pg_sync<PAIR>();   // the other CTA's shared and tensor memory are in use until here
+    if (warp == PG_W_MMA) pg_dealloc<PAIR>(tmem);
 }
 
 // ---------------------------------------------------------------------------------------------------------------------
@@ -700,16 +733,22 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
 StreamK prefill_streamk(const ib_ctx *ctx, uint32_t rows, uint32_t cols, uint32_t n) {
     StreamK sk;
     sk.nb = cols / 256;
-    sk.total = ((rows + PF_TILE_ROWS - 1) / PF_TILE_ROWS) * ((n + PF_CHUNK - 1) / PF_CHUNK) * sk.nb;
-    const uint32_t pairs = ctx->sm_count >= 2 ? (uint32_t)ctx->sm_count / 2 : 1u;
-    sk.pairs = sk.total < pairs ? sk.total : pairs;
+    // One SM or a pair per tile.  A pair's start and end (its launch, tensor memory, meetings and remote arrivals) cost a launch about a
+    // microsecond more, what it saves is L2 traffic of the inputs: nothing up to 16 tokens (us, one SM / pair: Q4_K 512 x 1024 10.0 / 10.1, 4096 x
+    // 4096 17.2 / 18.6, 28672 x 4096 39.0 / 41.3), little where no CTA has more than a unit (1152 x 4096, 64 tokens 14.8 / 16.6; 256 x 2048 10.3 /
+    // 12.0).  Beyond, pairs are the faster ones or equal (4096 x 4096, 40 tokens 20.4 / 19.3).
+    const bool pair = n > PF_SINGLE_TOKENS || (n > PF_SINGLE_ALWAYS && (rows >> 7) * sk.nb > (uint32_t)ctx->sm_count);
+    sk.row_log2 = pair ? 8 : 7;
+    sk.total = ((rows + (1u << sk.row_log2) - 1) >> sk.row_log2) * ((n + PF_CHUNK - 1) / PF_CHUNK) * sk.nb;
+    const uint32_t most = pair ? (ctx->sm_count >= 2 ? (uint32_t)ctx->sm_count / 2 : 1u) : (uint32_t)ctx->sm_count;
+    sk.ranges = sk.total < most ? sk.total : most;
     return sk;
 }
-// Most planes a tile needs: a range of `len` units cut into pieces of at least floor(total / pairs) units each
+// Most planes a tile needs: a range of `len` units cut into pieces of at least floor(total / ranges) units each
 uint32_t prefill_max_pieces(const StreamK &sk) {
-    const uint32_t least = sk.total / sk.pairs;
+    const uint32_t least = sk.total / sk.ranges;
     const uint32_t most = (sk.nb - 1) / least + 2;   // nb consecutive units touch at most this many ranges of that length
-    return most < sk.pairs ? most : sk.pairs;
+    return most < sk.ranges ? most : sk.ranges;
 }
 
 typedef CUresult (*EncodeTiledFn)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *, const cuuint64_t *, const cuuint32_t *, const cuuint32_t *,
@@ -754,34 +793,44 @@ static int32_t pg_encode(const ib_qtensor *m, int fmt, CUtensorMap *maps) {
     return IB_OK;
 }
 
-template <int FMT>
+template <int FMT, bool PAIR>
 static int32_t pg_launch(ib_ctx *ctx, cudaStream_t s, PgParams &p, const PgMaps &maps, bool early) {
     static bool attr_set[16] = {};
     constexpr uint32_t room = PG_SMEM_LIMIT - pg_fixed_smem(FMT);
-    static_assert(room >= 3 * PF_CHUNK * 128, "shared memory");
-    p.x_tile = ((p.n < PF_CHUNK ? p.n : PF_CHUNK) + 15) / 16 * 8 * 128;   // 64 columns of a CTA's half of the (padded) tokens of a chunk
+    static_assert(room >= 3 * (PAIR ? PF_CHUNK / 2 : PF_SINGLE_TOKENS) * 256, "shared memory");
+    p.x_tile = ((p.n < PF_CHUNK ? p.n : PF_CHUNK) + 15) / 16 * (PAIR ? 8 : 16) * 128;   // 64 columns of a CTA's (padded) tokens of a chunk
     p.x_stages = room / (2 * p.x_tile) < PG_XSTAGES_MAX ? room / (2 * p.x_tile) : PG_XSTAGES_MAX;
     const uint32_t smem = pg_fixed_smem(FMT) + p.x_stages * 2 * p.x_tile;
     if (!attr_set[ctx->device & 15]) {
-        IB_CHECK_CUDA(cudaFuncSetAttribute(prefill_gemm_kernel<FMT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PG_SMEM_LIMIT));
+        IB_CHECK_CUDA(cudaFuncSetAttribute(prefill_gemm_kernel<FMT, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PG_SMEM_LIMIT));
         attr_set[ctx->device & 15] = true;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * p.sk.pairs);
+    cfg.gridDim = dim3((PAIR ? 2 : 1) * p.sk.ranges);
     cfg.blockDim = dim3(PG_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = early ? 2 : 1;
-    IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, prefill_gemm_kernel<FMT>, p, maps));
+    if (PAIR) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attr[cfg.numAttrs].val.clusterDim.x = 2;
+        attr[cfg.numAttrs].val.clusterDim.y = attr[cfg.numAttrs].val.clusterDim.z = 1;
+        cfg.numAttrs++;
+    }
+    if (early) {
+        attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
+        cfg.numAttrs++;
+    }
+    IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, prefill_gemm_kernel<FMT, PAIR>, p, maps));
     ctx->launches++;
     return IB_OK;
+}
+
+template <int FMT>
+static int32_t pg_launch_rows(ib_ctx *ctx, cudaStream_t s, PgParams &p, const PgMaps &maps, bool early) {
+    return p.sk.row_log2 == 8 ? pg_launch<FMT, true>(ctx, s, p, maps, early) : pg_launch<FMT, false>(ctx, s, p, maps, early);
 }
 
 int32_t launch_prefill_gemm(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *const *mats, uint32_t n_mats, const __half *x, uint32_t n, float *plane0,
@@ -806,10 +855,10 @@ int32_t launch_prefill_gemm(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *const
     p.n = n; p.chunks = (n + PF_CHUNK - 1) / PF_CHUNK; p.x = x; p.x_chunk = pf_x_halves((uint32_t)mats[0]->cols);
     p.plane0 = plane0; p.planes = planes; p.sk = sk; p.err = ctx->err_dev; p.wait_ns = ctx->wait_limit_ns;
     switch (fmt) {
-    case PG_Q4K: return pg_launch<PG_Q4K>(ctx, s, p, maps, early);
-    case PG_Q5K: return pg_launch<PG_Q5K>(ctx, s, p, maps, early);
-    case PG_Q6K: return pg_launch<PG_Q6K>(ctx, s, p, maps, early);
-    case PG_Q80: return pg_launch<PG_Q80>(ctx, s, p, maps, early);
+    case PG_Q4K: return pg_launch_rows<PG_Q4K>(ctx, s, p, maps, early);
+    case PG_Q5K: return pg_launch_rows<PG_Q5K>(ctx, s, p, maps, early);
+    case PG_Q6K: return pg_launch_rows<PG_Q6K>(ctx, s, p, maps, early);
+    case PG_Q80: return pg_launch_rows<PG_Q80>(ctx, s, p, maps, early);
     default: return set_error(IB_ERR_UNSUPPORTED, "prefill GEMM: a matrix of type %d", mats[0]->qtype);
     }
 }

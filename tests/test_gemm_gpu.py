@@ -54,7 +54,8 @@ def test_gemm_across_chunks_of_tokens(backend, qt, rows, cols, n):
     m.close()
 
 
-# a pair of SMs shares 256 rows and a chunk's tokens: an odd number of 128-row halves, the fewest tokens per half, halves with a remainder
+# a pair of SMs shares 256 rows and a chunk's tokens: an odd number of 128-row halves, halves with a remainder (up to 64 tokens such small matrices
+# are one SM's work per tile)
 @pytest.mark.parametrize("qt", [quant.Q4_K, quant.Q5_K, quant.Q6_K, quant.Q8_0])
 @pytest.mark.parametrize("rows,n", [(128, 1), (384, 16), (384, 33), (640, 145)])
 def test_gemm_halves_of_a_pair(backend, qt, rows, n):
@@ -73,6 +74,14 @@ def test_gemm_scales_of_long_ranges(backend, qt):
         GemmQuant(backend).launch(o, m, x)
     assert all(torch.equal(o, out[0]) for o in out)
     m.close()
+
+
+# one SM per tile up to 16 tokens, up to 64 where the matrix has no more 128 x 256 units than the GPU has SMs (148), a pair beyond: either side of each
+# limit, and a last pass of a few tokens behind one of 1024
+@pytest.mark.parametrize("qt", [quant.Q4_K, quant.Q5_K, quant.Q6_K, quant.Q8_0])
+@pytest.mark.parametrize("rows,cols,n", [(128, 2048, 16), (2304, 2048, 64), (2304, 2048, 65), (2432, 2048, 16), (2432, 2048, 17), (384, 2048, 63), (256, 2048, 1030)])
+def test_gemm_of_few_tokens(backend, qt, rows, cols, n):
+    test_gemm_across_chunks_of_tokens(backend, qt, rows, cols, n)
 
 
 @pytest.mark.parametrize("qt,rows,cols,n", [
