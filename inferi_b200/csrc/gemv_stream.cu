@@ -300,11 +300,11 @@ __device__ __noinline__ void finish_argmax(const GemvParams &p, unsigned long lo
     }
 }
 
-// One 4-byte word of every 64 bytes of the launch's parameters, each by another warp: a launch's parameters are in no cache when it
+// One 4-byte word of every 64 bytes of the launch's parameters, each by another consumer warp: a launch's parameters are in no cache when it
 // starts, and a warp that comes to them one after the other waits for every line.
 __device__ __forceinline__ void touch_parameters(const GemvParams &p, const StreamGeom &geo, uint32_t warp) {
     constexpr uint32_t LP = (sizeof(GemvParams) + 63) / 64, LG = (sizeof(StreamGeom) + 63) / 64;
-    static_assert(LP + LG <= STREAM_THREADS / 32, "a warp per line");
+    static_assert(LP + LG <= CW, "a consumer warp per line (the producers do not come here)");
     uint32_t v = 0;
     if (warp < LP) v = reinterpret_cast<const uint32_t *>(&p)[16 * warp];
     else if (warp < LP + LG) v = reinterpret_cast<const uint32_t *>(&geo)[16 * (warp - LP)];
