@@ -42,8 +42,8 @@ uint32_t attn_max_splits(const ib_ctx *ctx, const ib_attn_params &p) {
     uint32_t s = (uint32_t)(ctx->sm_count * 3) / (n_kv ? n_kv : 1);   // three CTAs of either kernel fit one SM: one wave
     if (s < 1) s = 1;
     if (s > 256) s = 256;
-    // the merging block stages every slice's (max, sum) in its accumulator area: 2 * splits * kv_mul floats must fit the
-    // 4 * kv_mul * head_size it owns
+    // attn_kernel's merging block stages every slice's (max, sum) in its accumulator area: 2 * splits * kv_mul floats must fit the
+    // 4 * kv_mul * head_size it owns (attn_gqa4_kernel's holds 256 slices at either head size)
     if (s > 2 * p.head_size) s = 2 * p.head_size;
     return s;
 }
@@ -105,6 +105,9 @@ static uint32_t gqa4_cluster_ctas(const ib_ctx *ctx, const ib_attn_params &p, ui
 //                   Middle against long: 6.8 / 6.1 at 2000 with 2 heads, 6.9 / 6.2 at 1800 with 4, 7.0 / 7.2 at 1800 with 8 (8.9 / 8.6 at 3000),
 //                   8.0 / 8.9 at 2500 with 12;  16 heads  5.7 / 6.1 at 600, 7.1 / 6.6 at 1000.  In the graph (a layer of the 8B shapes): 45.6 / 46.9
 //                   at 1900, 48.7 / 48.0 at 2700;  4 heads  28.3 / 29.9 at 1600.
+// The middle regime's ends are those of the token graph (for head size 64 beyond 3000 positions: the crossing back to back, moved by that margin).  Launches outside it, which take the same ones, would cross over earlier by the
+// figures above: up to 0.9 us of 8 between 4000 and 6400 positions of up to 8 heads of 64, 0.7 of 7 below 2560 positions of 2 to 4 heads of 128.
+// (2 to 4 heads of 128 end at 2560, 8 at 2400: the latter was measured in the graph up to its crossing, the former at 1600 only.)
 uint32_t attn_regime_positions(const ib_ctx *ctx, const AttnLaunch &a, uint32_t regime) {
     if (!attn_gqa4_eligible(a) || ctx->sm_count == 0) return 0u;
     const uint32_t n_kv = a.p.n_heads / a.p.kv_mul, middle = gqa4_cluster_ctas(ctx, a.p, ATTN_MIDDLE), c = gqa4_cluster_ctas(ctx, a.p, regime);

@@ -57,8 +57,7 @@ __host__ __device__ constexpr uint32_t attn_block_smem_floats(uint32_t hs, uint3
 
 // The split of `total` positions: number of non-empty slices and positions per slice.
 // With `knee` > 0 the slices stop multiplying at `knee` until each holds `knee_per` positions: the merge reads every
-// slice's partial (eight per L2 round trip), so beyond a dozen slices more of them only pay once they shorten the row loop
-// by more than they lengthen the merge.
+// slice's partial, so more slices have to shorten the row loop by more than they lengthen the merge.
 __host__ __device__ __forceinline__ void attn_split_plan(uint32_t total, uint32_t max_splits, uint32_t &nsplit, uint32_t &per,
                                                          uint32_t min_per_split = ATTN_MIN_PER_SPLIT, uint32_t knee = 0, uint32_t knee_per = 0) {
     nsplit = (total + min_per_split - 1) / min_per_split;

@@ -30,10 +30,12 @@ constexpr uint32_t GQA4_ROWS_PER_WARP_STEP = 8;
 //  * middle: the same with 8 or 16 warps per CTA, which hold the row loop at a few iterations.
 //  * long: many CTAs of 4 warps (one wave of 3 per SM), merged through global memory.  Slices: one warp step of every warp (32
 //    positions) each while there are at most 16 of them, then 16 slices that grow to 128 positions, then slices of 128
-//    positions up to the launch's maximum, then longer ones.
+//    positions up to the launch's maximum, then longer ones.  Measured us per launch at 2500 / 4096 / 8192 / 16384 positions of 8 heads of
+//    128: this plan 8.7 / 9.2 / 12.0 / 17.6, 32 positions each throughout 8.2 / 9.3 / 12.0 / 17.7, at least 256 each 9.8 / 9.9 / 13.0 / 17.7
+//    (the merge fetches sixteen slices per L2 round trip; when it fetched eight, 32 each cost 12.6 at 2048 where the plan cost 9.2).
 // Clusters have at most 8 CTAs: eight clusters of 16 - one per kv head of the Llama-3 models - do not all fit the GPU at once.
 constexpr uint32_t GQA4_CLUSTER_MAX = 8;
-__host__ __device__ constexpr int gqa4_warps(uint32_t hs, uint32_t regime) { return regime != ATTN_MIDDLE ? ATTN_WARPS : (hs == 128 ? 8 : 16); }   // (head size 128 needs 142 registers)
+__host__ __device__ constexpr int gqa4_warps(uint32_t hs, uint32_t regime) { return regime != ATTN_MIDDLE ? ATTN_WARPS : (hs == 128 ? 8 : 16); }   // (head size 128 needs 196 registers a thread)
 constexpr uint32_t GQA4_MIN_PER_SPLIT = ATTN_WARPS * GQA4_ROWS_PER_WARP_STEP, GQA4_KNEE = 16, GQA4_KNEE_PER = 128;
 __host__ __device__ __forceinline__ void gqa4_plan(uint32_t total, uint32_t max_splits, uint32_t cluster, uint32_t warps, uint32_t &nsplit, uint32_t &per) {
     if (cluster) {
