@@ -45,7 +45,7 @@ def test_llama_3_2_1b_architecture_prefill_then_64_tokens(backend):
 
 
 def test_long_prompt_goes_in_chunks_and_matches_the_oracle(backend):
-    """300 prompt tokens = three GEMM passes; a later turn continues from start_pos > 0.  Small model, also against the oracle."""
+    """300 prompt tokens = three chunks of a GEMM pass; a later turn continues from start_pos > 0.  Small model, also against the oracle."""
     cfg = Llama2Config(512, 1024, 2, 8, 2, 512, 512, 500000.0, 1e-5)
     recipe = dict(Q4_K_M, token_embd=quant.Q4_K, attn_v=quant.Q5_K, ffn_down=quant.Q8_0, output=quant.Q4_K)   # 512 columns: no Q6_K rows here
     w = synth_weights(cfg, seed=21, recipe=recipe)
