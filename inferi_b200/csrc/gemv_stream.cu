@@ -62,6 +62,7 @@ struct Consumer {
     uint32_t zeros;            // shared address of 16 zero bytes
     uint32_t stream, RG, pt;   // the stream's stages: stream, stream + RG, ... < S; pairs per tile
     uint32_t blk, nb;          // the warp's first block of 256 columns, blocks
+    uint32_t stride;           // bytes of a row
     int lane;
 };
 
@@ -75,37 +76,30 @@ constexpr uint32_t PART_STAGE_FLOATS = 2 * CW * PT_MAX;
 // column groups and everything that follows is the epilogue warp's work.
 template <uint32_t QT, uint32_t MODE>
 __device__ __forceinline__ void consume_tiles(const GemvParams &p, const Consumer &c, const Act &A) {
-    const uint32_t g = c.lane >> 2, t = c.lane & 3;
+    const uint32_t g = c.lane >> 2, t = c.lane & 3, stride = c.stride;
+    using F = Frag<QT>;
     LaneConst lc;
     constexpr bool FOUR = MODE == ROWS4;
     constexpr uint32_t NB = MODE == ROWS8 ? 2 : NB_MAX;
     uint32_t B[NB][8];
     UnitAct ua[2];
-    constexpr bool ONE_TYPE = (QT != QT_MIXED && QT != QT_Q4_Q6);
     const bool swiglu = p.epi == EPI_SWIGLU;   // a "pair" is gate row r + up row r: 4 gate rows, then their 4 up rows, at a time
     const uint32_t act = smem_u32(A.base), sc0 = act + ACT_LIMBS * A.cols, sx0 = sc0 + A.cols / 8;
-    // The lane's activations go into registers in the order of a format's B operand: for the first segment before the first tile
-    // is waited for (the copy of that tile and this load overlap), again when a segment of another format begins.
-    auto enter = [&](uint32_t qtype, uint32_t stride) {
-        with_format<QT>(qtype, [&](auto f) {
-            lc.sc = sc0;
-            lc.sx = sx0;
-            f.template init<FOUR>(g, t, stride, c.blk, lc);
+    // The lane's activations go into registers in the order of the format's B operand before the first tile is waited for: the copy of that
+    // tile and this load overlap.
+    lc.sc = sc0;
+    lc.sx = sx0;
+    F::template init<FOUR>(g, t, stride, c.blk, lc);
 #pragma unroll
-            for (uint32_t i = 0; i < NB; i++) {
-                if (i < c.nb) f.operand(FOUR && (i & 1) ? g ^ 4 : g, t, act + (g & 1) * A.cols, c.zeros, c.blk + i, B[i]);
-                else
-                    for (int k = 0; k < 8; k++) B[i][k] = 0;
-            }
-            if (MODE == ROWS8) {
-                f.template unit<FOUR>(lc, 0, ua[0]);
-                if (c.nb == 2) f.template unit<FOUR>(lc, 1, ua[1]);
-            }
-        });
-    };
-    uint32_t cur_type = ONE_TYPE ? QT : p.seg[0].qtype, cur_s = 0, stride = (uint32_t)p.seg[0].row_bytes;
-    if (ONE_TYPE) enter(cur_type, stride);   // (rows of one format and width are equally long in every segment)
-    bool fresh = !ONE_TYPE;
+    for (uint32_t i = 0; i < NB; i++) {
+        if (i < c.nb) F::operand(FOUR && (i & 1) ? g ^ 4 : g, t, act + (g & 1) * A.cols, c.zeros, c.blk + i, B[i]);
+        else
+            for (int k = 0; k < 8; k++) B[i][k] = 0;
+    }
+    if (MODE == ROWS8) {
+        F::template unit<FOUR>(lc, 0, ua[0]);
+        if (c.nb == 2) F::template unit<FOUR>(lc, 1, ua[1]);
+    }
     const uint32_t together = FOUR ? 4 : 8, half = together / 2;   // rows at a time; gate/up: gate rows, then their up rows
     const uint32_t add = swiglu ? half : together, row_of = g & (add - 1), b_off = swiglu && (g & half) ? c.pt * stride : 0;   // the up rows follow a full tile's gate rows
     const uint32_t part0 = c.part + 4 * (swiglu ? 2 * row_of + ((g & half) ? 1 : 0) : row_of), out_step = 4 * together;
@@ -113,10 +107,6 @@ __device__ __forceinline__ void consume_tiles(const GemvParams &p, const Consume
     uint32_t st = c.stream, par = 0, ring = c.ring;   // ring: address of stage st
 #pragma unroll 1
     for (;;) {
-        if (!ONE_TYPE && fresh) {
-            enter(cur_type, stride);
-            fresh = false;
-        }
         if (!mbar_wait(c.bar0 + 8 * st, par, p.err, 1, p.wait_ns)) return;   // the error word is raised; give up on this CTA's rows
         const uint4 tm = lds128(c.meta + 16 * st);
         const uint32_t n = tm.z;
@@ -124,52 +114,43 @@ __device__ __forceinline__ void consume_tiles(const GemvParams &p, const Consume
             if (c.lane == 0) mbar_arrive(c.bar0 + 8 * (2 * c.S + st));
             break;
         }
-        if (!ONE_TYPE && tm.x != cur_s) {
-            cur_s = tm.x;
-            const uint32_t qtype = cur_s == 1 ? p.seg[1].qtype : p.seg[2].qtype;
-            fresh = qtype != cur_type;
-            cur_type = qtype;
-            stride = (uint32_t)(cur_s == 1 ? p.seg[1].row_bytes : p.seg[2].row_bytes);
-            if (fresh) continue;   // (the tile is still there for the second wait)
-        }
         const uint32_t base = ring + b_off, rows = swiglu ? n : 2 * n;
         uint32_t out = part0 + st * (4 * PART_STAGE_FLOATS);
         for (uint32_t r = row_of, first = 0; first < rows; first += add, r += add, out += out_step) {
             // rows past the tile's last one repeat it: what they give is not used
             const uint32_t row = base + (r < rows ? r : rows - 1) * stride;
             float v = 0.f;
-            with_format<QT>(cur_type, [&](auto f) {   // straight-line code: the steps' loads and products overlap
-                if constexpr (FOUR) {
-                    // `lc.first` differs between formats (swap_stretches).  Where it does not hold, the lane's units are in the second
-                    // block of a step, which the last step may lack.
-                    f.template unit<true>(lc, 0, ua[0]);
-                    v = f.template dot<true>(row, lc, 0, B[0], B[1], ua[0]);
-                    if (c.nb == 1 && !lc.first) v = 0.f;
-                    if (c.nb > 2) {
-                        f.template unit<true>(lc, 1, ua[1]);
-                        const float y = f.template dot<true>(row, lc, 1, B[2], B[3], ua[1]);
-                        v += c.nb == 3 && !lc.first ? 0.f : y;
-                    }
-                } else if constexpr (MODE == ROWS8_LONG) {
-                    if (c.nb == NB_MAX) {
+            // straight-line code: the steps' loads and products overlap
+            if constexpr (FOUR) {
+                // `lc.first` differs between formats (swap_stretches).  Where it does not hold, the lane's units are in the second
+                // block of a step, which the last step may lack.
+                F::template unit<true>(lc, 0, ua[0]);
+                v = F::template dot<true>(row, lc, 0, B[0], B[1], ua[0]);
+                if (c.nb == 1 && !lc.first) v = 0.f;
+                if (c.nb > 2) {
+                    F::template unit<true>(lc, 1, ua[1]);
+                    const float y = F::template dot<true>(row, lc, 1, B[2], B[3], ua[1]);
+                    v += c.nb == 3 && !lc.first ? 0.f : y;
+                }
+            } else if constexpr (MODE == ROWS8_LONG) {
+                if (c.nb == NB_MAX) {
 #pragma unroll
-                        for (uint32_t i = 0; i < NB_MAX; i++) {
-                            f.template unit<false>(lc, i, ua[i & 1]);
-                            v += f.template dot<false>(row, lc, i, B[i], B[i], ua[i & 1]);
-                        }
-                    } else {
-#pragma unroll
-                        for (uint32_t i = 0; i < NB_MAX - 1; i++)
-                            if (i < c.nb) {
-                                f.template unit<false>(lc, i, ua[0]);
-                                v += f.template dot<false>(row, lc, i, B[i], B[i], ua[0]);
-                            }
+                    for (uint32_t i = 0; i < NB_MAX; i++) {
+                        F::template unit<false>(lc, i, ua[i & 1]);
+                        v += F::template dot<false>(row, lc, i, B[i], B[i], ua[i & 1]);
                     }
                 } else {
-                    v = f.template dot<false>(row, lc, 0, B[0], B[0], ua[0]);
-                    if (c.nb == 2) v += f.template dot<false>(row, lc, 1, B[1], B[1], ua[1]);
+#pragma unroll
+                    for (uint32_t i = 0; i < NB_MAX - 1; i++)
+                        if (i < c.nb) {
+                            F::template unit<false>(lc, i, ua[0]);
+                            v += F::template dot<false>(row, lc, i, B[i], B[i], ua[0]);
+                        }
                 }
-            });
+            } else {
+                v = F::template dot<false>(row, lc, 0, B[0], B[0], ua[0]);
+                if (c.nb == 2) v += F::template dot<false>(row, lc, 1, B[1], B[1], ua[1]);
+            }
             v += __shfl_xor_sync(0xffffffffu, v, 1);
             v += __shfl_xor_sync(0xffffffffu, v, 2);
             if (FOUR) v += __shfl_xor_sync(0xffffffffu, v, 16);
@@ -315,7 +296,7 @@ __device__ __forceinline__ void touch_parameters(const GemvParams &p, const Stre
 // Shared-memory barriers: full[S] (the producer's expect_tx arrival + the copy's bytes), empty[S] (one arrival: the
 // epilogue warp has read the stage's partials, which implies that every consumer warp is done with its weights),
 // done[S] (one arrival per consumer warp of the tile's stream), ss (one arrival per consumer warp: its part of the input's sum of squares).
-// One instance per weight format (or format pair); what the launch does with the row sums is a run-time switch in the
+// One instance per weight format (and one for launches that mix them); what the launch does with the row sums is a run-time switch in the
 // epilogue warp, so that the launches of a token graph share their code.
 template <uint32_t QT, uint32_t MODE>
 __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const __grid_constant__ GemvParams p, const __grid_constant__ StreamGeom geo) {
@@ -364,7 +345,8 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const __
             held = geo.head;
             t = me * held;
         } else {
-            make_share(geo.share, geo.seg_pairs, geo.seg_pt, geo.nseg, me, sh);
+            const uint32_t group = share_group(geo.share, blockIdx.x);
+            make_share(geo.share, geo.seg_pairs, geo.seg_pt, geo.nseg, group, me - geo.share.cta0[group] * geo.P, sh);
             tc.init(sh);
         }
         uint32_t cost = swiglu ? (uint32_t)p.seg[0].row_bytes : geo.seg_cost[0], cost_b = (uint32_t)p.seg[1].row_bytes, cur = 0;
@@ -460,6 +442,8 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const __
     c.stage_bytes = geo.stage_bytes * RG;   // from one of the stream's stages to the next
     c.blk = cg * geo.NB;
     c.nb = blocks - c.blk < geo.NB ? blocks - c.blk : geo.NB;
+    const uint32_t seg0 = QT == QT_MIXED ? geo.share.seg0[share_group(geo.share, blockIdx.x)] : 0;
+    c.stride = (uint32_t)p.seg[seg0].row_bytes;
     const Act A{act_sm, p.cols};
     float4 norm_g[2];
     pack_prefetch_norm8(p.norm_w, p.cols, norm_g);   // weights: fetched while the previous kernel is still running
@@ -470,7 +454,15 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const __
         named_barrier(1, PACK_THREADS);
     }
     pack_stream<MODE == ROWS8 ? 1 : 4>(act_sm, p.cols, p.reduce_src ? p.x_out : p.x, p.norm_w, red, bar0 + 8 * (3 * S), norm_g);
-    if ((uint32_t)warp < active) consume_tiles<QT, MODE>(p, c, A);
+    if ((uint32_t)warp >= active) return;
+    if constexpr (QT != QT_MIXED) consume_tiles<QT, MODE>(p, c, A);
+    else
+        switch (p.seg[seg0].qtype) {   // of all the CTA's tiles
+        case IB_Q4_K: consume_tiles<IB_Q4_K, MODE>(p, c, A); break;
+        case IB_Q6_K: consume_tiles<IB_Q6_K, MODE>(p, c, A); break;
+        case IB_Q5_K: consume_tiles<IB_Q5_K, MODE>(p, c, A); break;
+        default: consume_tiles<IB_Q8_0, MODE>(p, c, A); break;
+        }
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -524,23 +516,57 @@ static int32_t launch_stream_inst(ib_ctx *ctx, cudaStream_t stream, const GemvPa
     }
 }
 
-// Which instance serves a launch: the one of its format; launches that mix Q4_K and Q6_K segments the two-format one.  (One
-// two-format instance for all launches of a Q4_K_M token keeps one copy of the code in the instruction caches, but each launch then
-// runs through twice the code: 1584 against 1454 us per token of an 8B model.)
+// Which instance serves a launch: the one of its format, or the one whose CTAs each take the path of their own.
 static int32_t launch_stream_format(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p, int grid, const StreamGeom &geo, size_t smem) {
     uint32_t qt = p.seg[0].qtype;
-    bool only_q4_q6 = true;
-    for (uint32_t s = 0; s < p.nseg; s++) {
+    for (uint32_t s = 0; s < p.nseg; s++)
         if (p.seg[s].qtype != qt) qt = QT_MIXED;
-        only_q4_q6 = only_q4_q6 && (p.seg[s].qtype == IB_Q4_K || p.seg[s].qtype == IB_Q6_K);
-    }
-    if (only_q4_q6 && qt == QT_MIXED) return launch_stream_inst<QT_Q4_Q6>(ctx, stream, p, grid, geo, smem);
     switch (qt) {
     case IB_Q4_K: return launch_stream_inst<IB_Q4_K>(ctx, stream, p, grid, geo, smem);
     case IB_Q6_K: return launch_stream_inst<IB_Q6_K>(ctx, stream, p, grid, geo, smem);
     case IB_Q5_K: return launch_stream_inst<IB_Q5_K>(ctx, stream, p, grid, geo, smem);
     case IB_Q8_0: return launch_stream_inst<IB_Q8_0>(ctx, stream, p, grid, geo, smem);
     default: return launch_stream_inst<QT_MIXED>(ctx, stream, p, grid, geo, smem);
+    }
+}
+
+// The CTAs of every group of segments of one format (ShareGeom), in proportion to its bytes; a group has a CTA at least (every segment has
+// two row pairs, so the grid has a CTA for each).
+static void deal_ctas(ShareGeom &g, const GemvParams &p, uint32_t nseg, const uint32_t (&pairs)[3], uint32_t total16, uint32_t grid, uint32_t P) {
+    uint32_t n = 0, bytes[3] = {0, 0, 0}, ctas[3] = {0, 0, 0}, used = 0;
+    for (uint32_t s = 0; s < nseg; s++) {
+        if (s == 0 || p.seg[s].qtype != p.seg[s - 1].qtype) {
+            g.seg0[n] = s;
+            g.base[n++] = g.start[s];
+        }
+        bytes[n - 1] += pairs[s] * g.cost16[s];
+    }
+    for (uint32_t i = 0; i < n; i++) {
+        ctas[i] = (uint32_t)((uint64_t)bytes[i] * grid / total16);
+        if (ctas[i] < 1) ctas[i] = 1;
+        used += ctas[i];
+    }
+    // rounded down: to the group whose CTAs have most; a group that was given its one CTA: from the group that misses it least
+    for (; used != grid; used += used < grid ? 1 : -1) {
+        uint32_t best = 0;
+        for (uint32_t i = 1; i < n; i++) {
+            if (used < grid ? (uint64_t)bytes[i] * ctas[best] > (uint64_t)bytes[best] * ctas[i]
+                            : ctas[best] < 2 || (ctas[i] > 1 && (uint64_t)bytes[i] * (ctas[best] - 1) < (uint64_t)bytes[best] * (ctas[i] - 1)))
+                best = i;
+        }
+        ctas[best] += used < grid ? 1 : -1;
+    }
+    uint32_t at = 0;
+    for (uint32_t i = 0; i < 3; i++) {
+        g.cta0[i] = i < n ? at : 0xFFFFFFFFu;
+        if (i >= n) {
+            g.scale[i] = 0;
+            g.base[i] = g.seg0[i] = 0;
+            continue;
+        }
+        const uint32_t pipes = ctas[i] * P;
+        g.scale[i] = (((uint64_t)bytes[i] << 32) + pipes - 1) / pipes;
+        at += ctas[i];
     }
 }
 
@@ -615,8 +641,7 @@ int32_t launch_gemv_stream(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p
     geo.width_log2 = 0;
     while ((1u << geo.width_log2) < width) geo.width_log2++;
     geo.cg_inv = (65536 + split.CG - 1) / split.CG;
-    const uint32_t pipes = (uint32_t)grid * geo.P;
-    geo.share.scale = (((uint64_t)total16 << 32) + pipes - 1) / pipes;
+    deal_ctas(geo.share, p, geo.nseg, geo.seg_pairs, total16, (uint32_t)grid, geo.P);
     geo.ahead = (AHEAD_BYTES / geo.stage_bytes) / geo.P * geo.P;
     if (geo.ahead < geo.P) geo.ahead = geo.P;
     geo.stages = S;

@@ -147,8 +147,16 @@ struct Share {
 
 // What the split needs, from the host: nothing here divides (a handful of 32-bit divisions at its start cost every launch a microsecond
 // before its first copy).  All byte counts are in units of 16 bytes.
+//
+// A CTA works on one weight format: where a launch mixes formats (q, k, v of most files), the CTAs are dealt out to the runs of segments of one
+// format ("groups") in proportion to their bytes.  Rounded to whole CTAs that is at most 3 % off where a group has 33 of them.  With CTAs that went
+// from one format to the next on the way, through code that switched between them, a 1B-architecture token took 405 instead of 397 us, an 8B one
+// 1323 instead of 1307: a launch fetched twice the code, and loaded its operands a second time behind the first tile.
 struct ShareGeom {
-    uint64_t scale;        // total / pipelines in units of 2^-32, rounded up
+    uint64_t scale[3];     // per group: its bytes / its pipelines in units of 2^-32, rounded up
+    uint32_t base[3];      // where the group begins in the launch's bytes
+    uint32_t cta0[3];      // its first CTA (0xFFFFFFFF: no such group)
+    uint32_t seg0[3];      // its first segment
     uint32_t start[3];     // where a segment begins in the launch's bytes
     uint32_t cost16[3];    // bytes per pair
     uint32_t inv[3];       // 2^32 / cost16, rounded up
@@ -161,8 +169,10 @@ __host__ __device__ __forceinline__ uint32_t share_pair(uint32_t at, uint32_t st
     return n < pairs ? n : pairs;
 }
 __host__ __device__ __forceinline__ uint32_t share_byte(uint64_t scale, uint32_t me) { return (uint32_t)((me * scale) >> 32); }
-__device__ __forceinline__ void make_share(const ShareGeom &g, const uint32_t (&pairs)[3], const uint32_t (&pt)[3], uint32_t nseg, uint32_t me, Share &sh) {
-    const uint32_t lo = share_byte(g.scale, me), hi = share_byte(g.scale, me + 1);
+__device__ __forceinline__ uint32_t share_group(const ShareGeom &g, uint32_t cta) { return cta >= g.cta0[2] ? 2u : (cta >= g.cta0[1] ? 1u : 0u); }
+// `me`: the pipeline's number among its group's
+__device__ __forceinline__ void make_share(const ShareGeom &g, const uint32_t (&pairs)[3], const uint32_t (&pt)[3], uint32_t nseg, uint32_t group, uint32_t me, Share &sh) {
+    const uint32_t lo = g.base[group] + share_byte(g.scale[group], me), hi = g.base[group] + share_byte(g.scale[group], me + 1);
     sh.nseg = nseg;
     sh.a0 = share_pair(lo, g.start[0], g.cost16[0], g.inv[0], pairs[0]);
     sh.b0 = share_pair(hi, g.start[0], g.cost16[0], g.inv[0], pairs[0]);
@@ -513,24 +523,7 @@ template <> struct Frag<IB_Q8_0> {
     }
 };
 
-constexpr uint32_t QT_MIXED = 0xFFu;   // kernel instance for launches whose segments differ in format
-constexpr uint32_t QT_Q4_Q6 = 0xFEu;   // ... and hold only Q4_K and Q6_K (q, k, v of the Q4_K_M recipe): two formats to switch between, not four
-
-// f(Frag<format>) for the format of a launch's instance, or of its segment where the instance serves several
-template <uint32_t QT, class F>
-__device__ __forceinline__ void with_format(uint32_t qtype, F &&f) {
-    if constexpr (QT == QT_Q4_Q6) {
-        if (qtype == IB_Q4_K) f(Frag<IB_Q4_K>{});
-        else f(Frag<IB_Q6_K>{});
-    } else if constexpr (QT == QT_MIXED) {
-        switch (qtype) {
-        case IB_Q4_K: f(Frag<IB_Q4_K>{}); break;
-        case IB_Q6_K: f(Frag<IB_Q6_K>{}); break;
-        case IB_Q5_K: f(Frag<IB_Q5_K>{}); break;
-        default: f(Frag<IB_Q8_0>{}); break;
-        }
-    } else f(Frag<QT>{});
-}
+constexpr uint32_t QT_MIXED = 0xFFu;   // kernel instance for launches whose segments differ in format: every CTA takes the path of its own
 
 // How a launch's rows are split over the consumer warps: NB blocks of 256 columns per warp, CG warps side by side cover a row and
 // form a stream, RG such streams share the tiles.  One or two blocks per warp where half of the warps then cover a row (one stream

@@ -77,6 +77,17 @@ def test_wide_rows_of_mixed_formats(backend, heads, types):
     check_loop(backend, cfg, synth_weights(cfg, seed=3006, device="cuda", recipe=recipe), True, prompt=[3, 500, 41], n_gen=4)
 
 
+# The CTAs of a q/k/v launch are dealt out to the runs of one format: two or three runs, in every order, with fewer rows than the GPU has CTAs
+# (hidden 256), with a run that gets a single CTA (k and v of 64 rows beside q of 1024), and with rows of 5 blocks (an odd share of a row)
+@pytest.mark.parametrize("hidden,heads,kv_heads", [(256, 4, 4), (1024, 16, 2), (1024, 8, 1), (1280, 20, 20)])
+@pytest.mark.parametrize("types", [(quant.Q4_K, quant.Q4_K, quant.Q8_0), (quant.Q8_0, quant.Q5_K, quant.Q5_K), (quant.Q5_K, quant.Q4_K, quant.Q5_K),
+                                   (quant.Q8_0, quant.Q5_K, quant.Q4_K)])
+def test_runs_of_one_format_get_their_ctas(backend, hidden, heads, kv_heads, types):
+    cfg = Llama2Config(hidden, 256, 1, heads, kv_heads, 512, 64, 500000.0, 1e-5)
+    recipe = dict(TINY_RECIPE, attn_q=types[0], attn_k=types[1], attn_v=types[2], ffn_down=quant.Q4_K)
+    check_loop(backend, cfg, synth_weights(cfg, seed=3007, device="cuda", recipe=recipe), True, prompt=[3, 500, 41], n_gen=3)
+
+
 def test_token_graph_launch_count_and_oracle_tokens(backend):
     """A token is a graph of 5 kernels per layer + 3 (begin, classifier, end); the launch counter must say so, and the
     greedy tokens must be the oracle's."""
