@@ -95,6 +95,31 @@ def test_bins_with_more_elements_than_the_list(backend, n, step):
     check_many(backend, logits, 1.0, 0.9, np.float32([0.0, 0.37, 0.999999]))
 
 
+@pytest.mark.parametrize("n", [32768, 32769, 65537, 98305, 131072, 131073, 163841, 330000])
+def test_slices_at_the_edges_of_the_instances(backend, n):
+    """A ranked distribution in which few of a thread's elements are candidates, one token either side of what an instance holds in one round.
+    (No coin next to 1: the oracle's f32 sum of so many tokens ends below it, and it then takes the last token.)"""
+    rng = np.random.default_rng(n)
+    logits = (-1.4 * np.log(rng.permutation(n) + 1.0) + 0.05 * rng.standard_normal(n)).astype(np.float32)
+    for topp in (0.0, 0.95):
+        check_many(backend, logits, 1.0, topp, np.float32([0.0, 0.31, 0.77, 0.98]))
+
+
+@pytest.mark.parametrize("n", [3000, 20000])
+@pytest.mark.parametrize("many,spread", [(31, 0.0), (32, 0.0), (33, 0.0), (33, 1e-4), (200, 0.0), (2048, 1e-3), (2100, 0.0), (2900, 1e-3)])
+def test_the_bin_of_the_crossing(backend, n, many, spread):
+    """`many` tokens of (almost) one probability hold most of the mass, behind a few larger ones: as many as a warp sorts, one more, more than
+    share a finer bin, about what a CTA stages, and more.  Small coins fall to the larger tokens' bins, the others among the many: one bin
+    for both bounds, two bins, or two candidates for the coin's bin."""
+    rng = np.random.default_rng(many)
+    logits = np.full(n, -30.0, dtype=np.float32)
+    at = rng.permutation(n)[:many + 3]
+    logits[at[:3]] = np.float32([2.0, 1.5, 1.6])
+    logits[at[3:]] = np.float32(spread) * rng.standard_normal(many).astype(np.float32)
+    for topp in (0.4, 0.97):
+        check_many(backend, logits, 1.0, topp, np.float32([0.0, 0.004, 0.02, 0.3, 0.6, 0.999]))
+
+
 @pytest.mark.parametrize("n", [2, 100, 40000, 300000])
 @pytest.mark.parametrize("depth", [30.0, 37.0, 85.0])
 def test_a_coin_of_zero_falls_to_the_first_token_that_can_come(backend, n, depth):
