@@ -1,6 +1,7 @@
-"""Builds libinferi_b200.so (sm_100a only) in-tree with nvcc.
+"""Builds libinferi_b200.so (sm_100a only) in-tree with nvcc, and the Python binding of the op launches.
 
-The shared library is the product: a C-ABI (include/inferi_b200.h) with no torch or Python types in it.
+The shared library is the product: a C-ABI (include/inferi_b200.h) with no torch or Python types in it.  `_binding.so` is what `ops.py` calls it
+through where it can (csrc/binding.cpp).
 """
 from __future__ import annotations
 
@@ -8,10 +9,12 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libinferi_b200.so")
+BINDING_PATH = os.path.join(PKG_DIR, "_binding.so")
 SOURCES = ["api.cu", "gemv.cu", "gemv_stream.cu", "ops.cu", "attention.cu", "prefill.cu", "prefill_gemm.cu", "prefill_attention.cu", "llama.cu", "gguf.cu", "sampler.cu", "tokenizer.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -31,7 +34,22 @@ def _stale() -> bool:
         return True
     t = os.path.getmtime(LIB_PATH)
     deps = [os.path.join(CSRC, f) for f in os.listdir(CSRC)] + [os.path.join(PKG_DIR, "..", "include", "inferi_b200.h"), __file__]
-    return any(os.path.getmtime(d) > t for d in deps)
+    return any(os.path.getmtime(d) > t for d in deps) or not os.path.exists(BINDING_PATH)
+
+
+def _binding_command() -> list[str] | None:
+    """How the Python binding of the op launches is compiled (csrc/binding.cpp): against this interpreter and its torch.  None with a torch that has no
+    CUDA: no launch gets as far as the binding there."""
+    import torch
+
+    if torch.version.cuda is None:
+        return None
+    root = os.path.dirname(os.path.abspath(torch.__file__))
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    includes = [f"{root}/include", f"{root}/include/torch/csrc/api/include", f"{cuda}/include", sysconfig.get_paths()["include"]]
+    return [os.environ.get("CXX", "g++"), "-O2", "-std=c++20", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+            *[f"-I{i}" for i in includes], os.path.join(CSRC, "binding.cpp"), "-o", BINDING_PATH, f"-L{root}/lib", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_python",
+            f"-Wl,-rpath,{root}/lib"]
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -50,14 +68,17 @@ def build(force: bool = False, verbose: bool = False) -> str:
         if verbose:
             cmd[1:1] = ["-Xptxas", "-v"]
         procs.append((src, subprocess.Popen(cmd, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
+    binding = _binding_command()
+    if binding:
+        procs.append(("binding.cpp", subprocess.Popen(binding, stdout=subprocess.PIPE, stderr=subprocess.STDOUT, text=True)))
     failed = False
     for src, p in procs:
         out, _ = p.communicate()
         if p.returncode != 0 or verbose:
-            sys.stderr.write(f"--- nvcc {src} ---\n{out}\n")
+            sys.stderr.write(f"--- {src} ---\n{out}\n")
         failed |= p.returncode != 0
     if failed:
-        raise RuntimeError("nvcc failed; see the messages above")
+        raise RuntimeError("the compiler failed; see the messages above")
     link = [nvcc, "-shared", "-o", LIB_PATH, *objs, "-lcudart_static", "-lpthread", "-ldl", "-lrt"]
     subprocess.run(link, check=True)
     return LIB_PATH

@@ -8,6 +8,7 @@
 #include "common.cuh"
 
 #include <math.h>
+#include <string.h>
 
 namespace ib {
 
@@ -73,7 +74,8 @@ int32_t launch_rms_norm(ib_ctx *ctx, cudaStream_t s, float *out, const float *x,
 
 // ---- RoPE: crates/inferi-shaders/src/rope.rs:51-92 (Original), :97-141 (NeoX) ----
 // The per-dimension frequencies theta_j = base^(-2j/head_size) are computed on the host with the C library's
-// powf and passed by value, so that device and host agree on them bit for bit.
+// powf and passed by value, so that device and host agree on them bit for bit.  They are a model's constants: a thread keeps those of the
+// last model it launched for (32 powf are a third of the launch).
 struct RopeTheta { float t[128]; };
 
 __global__ void rope_kernel(int variant, float *q, uint32_t q_len, float *k, uint32_t kv_dim, uint32_t head_size, uint32_t pos,
@@ -99,8 +101,14 @@ __global__ void rope_kernel(int variant, float *q, uint32_t q_len, float *k, uin
 
 int32_t launch_rope(ib_ctx *ctx, cudaStream_t s, int variant, float *q, uint32_t q_len, float *k, uint32_t kv_dim, uint32_t head_size, uint32_t pos,
                     float base_freq) {
-    RopeTheta th;
-    for (uint32_t j = 0; j < head_size / 2; j++) th.t[j] = powf(base_freq, -(float)(2 * j) / (float)head_size);
+    static thread_local RopeTheta th;
+    static thread_local float of_base;
+    static thread_local uint32_t of_size = 0;
+    if (of_size != head_size || memcmp(&of_base, &base_freq, sizeof of_base)) {
+        for (uint32_t j = 0; j < head_size / 2; j++) th.t[j] = powf(base_freq, -(float)(2 * j) / (float)head_size);
+        of_base = base_freq;
+        of_size = head_size;
+    }
     const uint32_t n = q_len / 2;
     return launch_op(ctx, s, rope_kernel, (n + 127) / 128, 128, variant, q, q_len, k, kv_dim, head_size, pos, th);
 }

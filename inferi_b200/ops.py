@@ -36,8 +36,20 @@ def _f32_dev(t: torch.Tensor, name: str) -> int:
     raise InferiError(1, f"{name}: expected a contiguous float32 CUDA tensor")
 
 
-# The launches below take their tensors' addresses first: with a CUDA tensor among them CUDA is initialised, and the stream can be
-# read without asking (these calls are a few microseconds each, most of it the launch itself).
+# A launch goes through the compiled binding (csrc/binding.cpp), which checks what the code behind it checks and answers with the library's status, or
+# with -1 where it has not launched anything: for arguments that it does not know (tensor subclasses), and for those that are refused.  The Python
+# way then does the call or raises the error, and does all of them where there is no binding.
+try:
+    from . import _binding as _fast
+except ImportError:
+    class _fast:
+        gemv = gemm = rms_norm = rope = silu = add = attention = argmax = sample = staticmethod(lambda *a: -1)
+        bind = staticmethod(lambda *a: None)
+_BOUND = ("ib_gemv_quant", "ib_gemm_quant", "ib_rms_norm", "ib_rope", "ib_silu_mul", "ib_add_assign", "ib_attention", "ib_argmax", "ib_sample")
+
+
+# The Python ways take their tensors' addresses first: with a CUDA tensor among them CUDA is initialised, and the stream can be
+# read without asking.
 
 
 class Backend:
@@ -48,7 +60,9 @@ class Backend:
         h = C.c_void_p()
         check(self.lib.ib_ctx_create(device, C.byref(h)))
         self.handle = h
+        self._address = h.value
         self.device = device
+        _fast.bind(*(C.cast(getattr(self.lib, name), C.c_void_p).value for name in _BOUND))
 
     def launch_count(self) -> int:
         n = C.c_uint64()
@@ -66,7 +80,7 @@ class Backend:
     def close(self) -> None:
         if getattr(self, "handle", None):
             self.lib.ib_ctx_destroy(self.handle)
-            self.handle = None
+            self.handle = self._address = None
 
     def __del__(self):
         try:
@@ -92,6 +106,7 @@ class GpuQuantTensor:
             b = np.ascontiguousarray(blocks).view(np.uint8).reshape(-1)
             check(backend.lib.ib_qtensor_upload(backend.handle, qtype, rows, cols, b.ctypes.data_as(C.c_void_p), b.size, 0, C.byref(h)))
         self.handle = h
+        self._address = h.value
 
     @property
     def nbytes(self) -> int:
@@ -100,7 +115,7 @@ class GpuQuantTensor:
     def close(self) -> None:
         if getattr(self, "handle", None):
             self.backend.lib.ib_qtensor_destroy(self.handle)
-            self.handle = None
+            self.handle = self._address = None
 
     def __del__(self):
         try:
@@ -121,6 +136,11 @@ class GemvQuant:
 
     def launch(self, out: torch.Tensor, m: GpuQuantTensor, v: torch.Tensor) -> None:
         """out[rows] = m . v[cols] on the current stream (asynchronous, like recording into a pass)."""
+        rc = _fast.gemv(self.backend and self.backend._address, out, m._address, m.rows, m.cols, v)
+        if rc == 0:
+            return
+        if rc > 0:
+            check(rc)
         if v.numel() != m.cols or out.numel() != m.rows:
             raise InferiError(1, f"gemv: matrix is {m.rows}x{m.cols} but v has {v.numel()} and out {out.numel()} elements")
         b, out_ptr, v_ptr = self.backend, _f32_dev(out, "out"), _f32_dev(v, "v")
@@ -147,6 +167,11 @@ class GemmQuant:
 
     def launch(self, out: torch.Tensor, m: GpuQuantTensor, x: torch.Tensor) -> None:
         """out[n, rows] = x[n, cols] . m^T on the current stream."""
+        rc = _fast.gemm(self.backend and self.backend._address, out, m._address, m.rows, m.cols, x)
+        if rc == 0:
+            return
+        if rc > 0:
+            check(rc)
         n = x.shape[0]
         if x.dim() != 2 or x.shape[1] != m.cols or tuple(out.shape) != (n, m.rows) or not x.is_contiguous() or not out.is_contiguous():
             raise InferiError(1, f"gemm: matrix is {m.rows}x{m.cols}, x {tuple(x.shape)}, out {tuple(out.shape)}")
@@ -182,6 +207,11 @@ class RmsNorm:
     from_backend = classmethod(lambda cls, backend: cls(backend))
 
     def launch(self, config: RmsNormConfig, result: torch.Tensor, value: torch.Tensor, weight: torch.Tensor) -> None:
+        rc = _fast.rms_norm(self.backend and self.backend._address, result, value, weight, config.nudge_factor)
+        if rc == 0:
+            return
+        if rc > 0:
+            check(rc)
         n = value.numel()
         if result.numel() != n or weight.numel() != n:
             raise InferiError(1, "rms_norm: result, value and weight must have the same length")
@@ -209,6 +239,11 @@ class RoPE:
     from_backend = classmethod(lambda cls, backend: cls(backend))
 
     def launch(self, variant: int, config: RoPEConfig, in_out_q: torch.Tensor, in_out_k: torch.Tensor) -> None:
+        rc = _fast.rope(self.backend and self.backend._address, variant, in_out_q, in_out_k, config.kv_dim, config.head_size, config.pos, config.base_freq)
+        if rc == 0:
+            return
+        if rc > 0:
+            check(rc)
         if in_out_k.numel() < config.kv_dim:
             raise InferiError(1, "rope: k is shorter than kv_dim")
         b, q, k = self.backend, _f32_dev(in_out_q, "q"), _f32_dev(in_out_k, "k")
@@ -226,6 +261,11 @@ class Silu:
     from_backend = classmethod(lambda cls, backend: cls(backend))
 
     def launch(self, in_out_h1: torch.Tensor, in_h2: torch.Tensor) -> None:
+        rc = _fast.silu(self.backend and self.backend._address, in_out_h1, in_h2)
+        if rc == 0:
+            return
+        if rc > 0:
+            check(rc)
         n = in_out_h1.numel()
         if n != in_h2.numel():
             raise InferiError(1, "silu: h1 and h2 must have the same length")
@@ -245,6 +285,11 @@ class FusedAttention:
 
     def launch(self, params: AttnParams, q: torch.Tensor, key_cache: torch.Tensor, value_cache: torch.Tensor, xb: torch.Tensor) -> None:
         """key_cache / value_cache: [seq_len, kv_dim] float32 or float16 CUDA tensors."""
+        rc = _fast.attention(self.backend and self.backend._address, params, q, key_cache, value_cache, xb) if type(params) is AttnParams else -1
+        if rc == 0:
+            return
+        if rc > 0:
+            check(rc)
         dtype = key_cache.dtype
         if dtype is not value_cache.dtype or (dtype is not _f16 and dtype is not _f32):
             raise InferiError(1, "attention: the caches must both be float16 or both float32")
@@ -264,6 +309,11 @@ class FusedAttention:
 
 def add_assign(backend: Backend, a: torch.Tensor, b: torch.Tensor) -> None:
     """≙ `LlmContext::add_assign` (crates/inferi/src/context.rs:516-530): a += b."""
+    rc = _fast.add(backend and backend._address, a, b)
+    if rc == 0:
+        return
+    if rc > 0:
+        check(rc)
     n = a.numel()
     if n != b.numel():
         raise InferiError(1, "add_assign: length mismatch")
@@ -275,6 +325,11 @@ def add_assign(backend: Backend, a: torch.Tensor, b: torch.Tensor) -> None:
 
 def argmax(backend: Backend, logits: torch.Tensor, out: torch.Tensor) -> None:
     """≙ greedy `Sampler::sample` (crates/inferi/src/models/sampler.rs:32-36, 54-56); out: int32/uint32[1] on the device."""
+    rc = _fast.argmax(backend and backend._address, logits, out)
+    if rc == 0:
+        return
+    if rc > 0:
+        check(rc)
     if not (out.is_cuda and out.element_size() == 4):
         raise InferiError(1, "argmax: out must be a 4-byte CUDA tensor")
     check(backend.lib.ib_argmax(backend.handle, _stream_ptr(), _f32_dev(logits, "logits"), logits.numel(), out.data_ptr()))
@@ -291,6 +346,11 @@ class Sampler:
         if logits.numel() != self.vocab_size:
             raise ValueError(f"expected {self.vocab_size} logits, got {logits.numel()}")
         out = out if out is not None else torch.empty(1, dtype=torch.int32, device=logits.device)
+        rc = _fast.sample(self.backend and self.backend._address, logits, self.vocab_size, self.temperature, self.topp, coin, out)
+        if rc == 0:
+            return out
+        if rc > 0:
+            check(rc)
         check(self.backend.lib.ib_sample(self.backend.handle, _stream_ptr(), _f32_dev(logits, "logits"), self.vocab_size, self.temperature, self.topp,
                                          float(coin), out.data_ptr()))
         return out
