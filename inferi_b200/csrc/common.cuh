@@ -5,6 +5,7 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 #include <stdio.h>
+#include <mutex>
 #include <string>
 
 #include "../../include/inferi_b200.h"
@@ -90,6 +91,9 @@ struct ib_ctx {
     void *tc_scratch = nullptr;
     size_t tc_scratch_bytes = 0;
     uint32_t tc_pass = 0xFFFFFFFFu;   // the longest pass (tokens) that the device has had room for
+    // pinned staging of copies to the host (read_back), made by the first one
+    void *stage_host = nullptr;
+    std::mutex stage_lock;
     // limit of every wait inside a kernel (on a shared-memory barrier, on another rank's arrival); ib_ctx_set_wait_limit
     uint64_t wait_limit_ns = 2000000000ull;
 };
@@ -178,6 +182,10 @@ bool gemv_stream_eligible(const GemvParams &p);
 int32_t launch_gemv_stream(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p);
 // IB_OK, or IB_ERR_TIMEOUT when a kernel raised the context's error word (call after a synchronisation)
 int32_t check_device_error(ib_ctx *ctx);
+// Device -> host.  Into ordinary host memory: complete when the call returns, as CUDA's own copy is.
+int32_t read_back(ib_ctx *ctx, cudaStream_t s, void *dst, const void *src, size_t nbytes);
+bool host_pageable(const void *p);
+void host_populate(void *p, size_t nbytes);
 int32_t launch_gemv_generic(ib_ctx *ctx, cudaStream_t stream, const ib_qtensor *m, const float *v, float *out);
 int32_t retile_to_soa(ib_ctx *ctx, cudaStream_t stream, int qtype, const uint8_t *src, uint8_t *dst, uint64_t rows, uint32_t nb);
 bool gemv_fast_eligible(int qtype, uint64_t rows, uint64_t cols);

@@ -122,6 +122,7 @@ struct ib_llama {
     uint32_t *reduce_done = nullptr;     // groups of the reduced residual stream stored so far (only ever grows)
     uint32_t *epoch = nullptr;
     uint32_t *h_pinned = nullptr;  // [4 + seq_cap] staging for control block and token ids
+    float *h_logits = nullptr;     // pinned [vocab_l] + the token's word: where ib_llama_forward's results arrive
     cudaEvent_t staged = nullptr;  // the last copy out of h_pinned has been issued and finished
     // [ATTN_LONG], and for the contexts where the attention nodes have another shape [ATTN_SHORT], [ATTN_MIDDLE]: the positions that
     // `regime_positions` says (0: no such graph)
@@ -409,6 +410,7 @@ int32_t ib_llama_destroy(ib_llama *m) {
     for (void *b : m->v_cache)
         if (b) cudaFree(b);
     if (m->h_pinned) cudaFreeHost(m->h_pinned);
+    if (m->h_logits) cudaFreeHost(m->h_logits);
     for (ib_qtensor *t : m->owned_tensors) ib_qtensor_destroy(t);
     for (void *b : m->owned_device) cudaFree(b);
     delete m;
@@ -542,6 +544,7 @@ int32_t ib_llama_create(ib_ctx *ctx, const ib_llama_config *config, const ib_lla
     CU(cudaMalloc(&m->seq, sizeof(uint32_t) * m->seq_cap));
     CU(cudaMemset(m->seq, 0, sizeof(uint32_t) * m->seq_cap));
     CU(cudaMallocHost(&m->h_pinned, sizeof(uint32_t) * (4 + (size_t)m->seq_cap)));
+    CU(cudaMallocHost(&m->h_logits, sizeof(float) * ((size_t)m->vocab_l + 1)));
     CU(cudaEventCreateWithFlags(&m->staged, cudaEventDisableTiming));
     ib_attn_params ap{c.max_position_embeddings, m->kv_dim_l, c.num_attention_heads / c.num_key_value_heads, m->n_heads_l, m->head_size, 0};
     m->attn_splits = attn_max_splits(ctx, ap);
@@ -730,13 +733,17 @@ int32_t ib_llama_forward(ib_llama *m, void *stream, uint32_t token, uint32_t pos
     cudaStream_t s = (cudaStream_t)stream;
     int32_t rc = run_tokens(m, s, &token, 1, pos, 1);
     if (rc) return rc;
-    if (logits_host) IB_CHECK_CUDA(cudaMemcpyAsync(logits_host, m->logits, sizeof(float) * m->vocab_l, cudaMemcpyDeviceToHost, s));
-    if (next_token_host) IB_CHECK_CUDA(cudaMemcpyAsync(next_token_host, &m->ctl->next, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
-    if (logits_host || next_token_host) {
-        IB_CHECK_CUDA(cudaStreamSynchronize(s));
-        return check_device_error(m->ctx);
-    }
-    return IB_OK;
+    if (!logits_host && !next_token_host) return IB_OK;
+    // The results arrive in pinned memory; what the caller's buffer takes (its pages, where it is a fresh one: read_back) is done while the GPU works.
+    const size_t bytes = sizeof(float) * m->vocab_l;
+    const bool staged = logits_host && host_pageable(logits_host);
+    if (logits_host) IB_CHECK_CUDA(cudaMemcpyAsync(staged ? m->h_logits : logits_host, m->logits, bytes, cudaMemcpyDeviceToHost, s));
+    IB_CHECK_CUDA(cudaMemcpyAsync(m->h_logits + m->vocab_l, &m->ctl->next, sizeof(uint32_t), cudaMemcpyDeviceToHost, s));
+    if (staged) host_populate(logits_host, bytes);
+    IB_CHECK_CUDA(cudaStreamSynchronize(s));
+    if (staged) memcpy(logits_host, m->h_logits, bytes);
+    if (next_token_host) memcpy(next_token_host, m->h_logits + m->vocab_l, sizeof(uint32_t));
+    return check_device_error(m->ctx);
 }
 
 // ---- prompt prefill on the tensor cores ----
