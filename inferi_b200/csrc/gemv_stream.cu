@@ -100,11 +100,40 @@ __device__ __forceinline__ void consume_tiles(const GemvParams &p, const Consume
         F::template unit<FOUR>(lc, 0, ua[0]);
         if (c.nb == 2) F::template unit<FOUR>(lc, 1, ua[1]);
     }
-    const uint32_t together = FOUR ? 4 : 8, half = together / 2;   // rows at a time; gate/up: gate rows, then their up rows
+    constexpr bool PAIR = MODE == ROWS8_PAIR;
+    constexpr uint32_t together = FOUR || PAIR ? 4 : 8, half = together / 2;   // rows of a tile at a time; gate/up: gate rows, then their up rows
     const uint32_t add = swiglu ? half : together, row_of = g & (add - 1), b_off = swiglu && (g & half) ? c.pt * stride : 0;   // the up rows follow a full tile's gate rows
     const uint32_t part0 = c.part + 4 * (swiglu ? 2 * row_of + ((g & half) ? 1 : 0) : row_of), out_step = 4 * together;
-    const bool writer = t == 0 && g < together;
+    const bool writer = t == 0 && (PAIR || g < together);
     uint32_t st = c.stream, par = 0, ring = c.ring;   // ring: address of stage st
+    // a row's up to four blocks: straight-line code where they are four, so that the blocks' loads and products overlap
+    auto long_dot = [&](uint32_t row) {
+        float v = 0.f;
+        if (c.nb == NB_MAX) {
+#pragma unroll
+            for (uint32_t i = 0; i < NB_MAX; i++) {
+                F::template unit<false>(lc, i, ua[i & 1]);
+                v += F::template dot<false>(row, lc, i, B[i & (NB - 1)], B[i & (NB - 1)], ua[i & 1]);
+            }
+        } else {
+#pragma unroll
+            for (uint32_t i = 0; i < NB_MAX - 1; i++)
+                if (i < c.nb) {
+                    F::template unit<false>(lc, i, ua[0]);
+                    v += F::template dot<false>(row, lc, i, B[i & (NB - 1)], B[i & (NB - 1)], ua[0]);
+                }
+        }
+        return v;
+    };
+    auto next_stage = [&]() {
+        st += c.RG;
+        ring += c.stage_bytes;
+        if (st >= c.S) {
+            st = c.stream;
+            ring = c.ring;
+            par ^= 1u;
+        }
+    };
 #pragma unroll 1
     for (;;) {
         if (!mbar_wait(c.bar0 + 8 * st, par, p.err, 1, p.wait_ns)) return;   // the error word is raised; give up on this CTA's rows
@@ -113,6 +142,25 @@ __device__ __forceinline__ void consume_tiles(const GemvParams &p, const Consume
         if (n == 0) {   // no tiles left
             if (c.lane == 0) mbar_arrive(c.bar0 + 8 * (2 * c.S + st));
             break;
+        }
+        if constexpr (PAIR) {
+            // Two tiles of 4 rows as 8 rows: the lower lanes' rows are this tile's, the upper ones' the next one's, which may be the end.  The ring
+            // keeps its four stages (and HBM its pace: with two tiles of 8 rows both land together).
+            const uint32_t st_a = st, ring_a = ring;
+            next_stage();
+            if (!mbar_wait(c.bar0 + 8 * st, par, p.err, 1, p.wait_ns)) return;
+            const uint32_t n_b = lds128(c.meta + 16 * st).z;
+            const bool b = (g & 4) && n_b;
+            const uint32_t rows = swiglu ? (b ? n_b : n) : 2 * (b ? n_b : n), row = (b ? ring : ring_a) + b_off + (row_of < rows ? row_of : rows - 1) * stride;
+            float v = long_dot(row);
+            v += __shfl_xor_sync(0xffffffffu, v, 1);
+            v += __shfl_xor_sync(0xffffffffu, v, 2);
+            if (writer) asm volatile("st.shared.f32 [%0], %1;" ::"r"(part0 + (g & 4 ? st : st_a) * (4 * PART_STAGE_FLOATS)), "f"(v) : "memory");
+            __syncwarp();
+            if (c.lane < 2) mbar_arrive(c.bar0 + 8 * (2 * c.S + (c.lane ? st : st_a)));
+            if (n_b == 0) break;
+            next_stage();
+            continue;
         }
         const uint32_t base = ring + b_off, rows = swiglu ? n : 2 * n;
         uint32_t out = part0 + st * (4 * PART_STAGE_FLOATS);
@@ -133,20 +181,7 @@ __device__ __forceinline__ void consume_tiles(const GemvParams &p, const Consume
                     v += c.nb == 3 && !lc.first ? 0.f : y;
                 }
             } else if constexpr (MODE == ROWS8_LONG) {
-                if (c.nb == NB_MAX) {
-#pragma unroll
-                    for (uint32_t i = 0; i < NB_MAX; i++) {
-                        F::template unit<false>(lc, i, ua[i & 1]);
-                        v += F::template dot<false>(row, lc, i, B[i], B[i], ua[i & 1]);
-                    }
-                } else {
-#pragma unroll
-                    for (uint32_t i = 0; i < NB_MAX - 1; i++)
-                        if (i < c.nb) {
-                            F::template unit<false>(lc, i, ua[0]);
-                            v += F::template dot<false>(row, lc, i, B[i], B[i], ua[0]);
-                        }
-                }
+                v = long_dot(row);
             } else {
                 v = F::template dot<false>(row, lc, 0, B[0], B[0], ua[0]);
                 if (c.nb == 2) v += F::template dot<false>(row, lc, 1, B[1], B[1], ua[1]);
@@ -158,13 +193,7 @@ __device__ __forceinline__ void consume_tiles(const GemvParams &p, const Consume
         }
         __syncwarp();   // the lanes' partials are ordered before lane 0's arrival (a release)
         if (c.lane == 0) mbar_arrive(c.bar0 + 8 * (2 * c.S + st));   // this warp is done with the stage: weights read, partials left
-        st += c.RG;
-        ring += c.stage_bytes;
-        if (st >= c.S) {
-            st = c.stream;
-            ring = c.ring;
-            par ^= 1u;
-        }
+        next_stage();
     }
 }
 
@@ -511,6 +540,7 @@ template <uint32_t QT>
 static int32_t launch_stream_inst(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p, int grid, const StreamGeom &geo, size_t smem) {
     switch (geo.mode) {
     case ROWS4: return launch_stream_rows<QT, ROWS4>(ctx, stream, p, grid, geo, smem);
+    case ROWS8_PAIR: return launch_stream_rows<QT, ROWS8_PAIR>(ctx, stream, p, grid, geo, smem);
     case ROWS8_LONG: return launch_stream_rows<QT, ROWS8_LONG>(ctx, stream, p, grid, geo, smem);
     default: return launch_stream_rows<QT, ROWS8>(ctx, stream, p, grid, geo, smem);
     }
@@ -601,7 +631,7 @@ int32_t launch_gemv_stream(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p
         return pt;
     };
     StreamGeom geo;
-    uint32_t stage_data = 0, tiles = 0;
+    uint32_t stage_data = 0, tiles = 0, most_pt = 0;
     for (uint32_t s = 0; s < 3; s++) {
         geo.seg_pairs[s] = 0;
         geo.seg_pt[s] = 1;
@@ -615,6 +645,7 @@ int32_t launch_gemv_stream(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p
         geo.seg_pairs[s] = swiglu ? p.seg[0].rows : p.seg[s].rows / 2;
         tiles += (geo.seg_pairs[s] + pt - 1) / pt;
         if (pt * cost > stage_data) stage_data = pt * cost;
+        if (pt > most_pt) most_pt = pt;
     }
     uint32_t total16 = 0;
     for (uint32_t s = 0; s < 3; s++) {
@@ -630,6 +661,10 @@ int32_t launch_gemv_stream(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p
     // A stage always serves the same stream: the barriers' parities only order uses that one and the same warp waits for.
     while (split.RG > S) split.RG /= 2;
     S -= S % split.RG;
+    if (split.mode == ROWS4 && most_pt == 2 && S >= 5 * split.RG) {
+        split.mode = ROWS8_PAIR;
+        geo.stage_bytes = stage_data;   // the rows of two tiles follow one another: eight rows then start at different banks where their stride lets them
+    }
     geo.NB = split.NB;
     geo.mode = split.mode;
     geo.CG = split.CG;
