@@ -377,8 +377,8 @@ int32_t ib_attention(ib_ctx *ctx, void *stream, const ib_attn_params *params, co
         ctx->attn_scratch_bytes = need;
     }
     if (!ctx->attn_counters) {
-        IB_CHECK_CUDA(cudaMalloc(&ctx->attn_counters, 1024 * sizeof(unsigned int)));
-        IB_CHECK_CUDA(cudaMemset(ctx->attn_counters, 0, 1024 * sizeof(unsigned int)));
+        IB_CHECK_CUDA(cudaMalloc(&ctx->attn_counters, 2048 * sizeof(unsigned int)));
+        IB_CHECK_CUDA(cudaMemset(ctx->attn_counters, 0, 2048 * sizeof(unsigned int)));
     }
     IB_REQUIRE(params->n_heads / params->kv_mul <= 1024, "ib_attention: too many kv heads");
     a.q = q_dev; a.k_cache = k_cache_dev; a.v_cache = v_cache_dev; a.kv_dtype = kv_dtype; a.out = out_dev;

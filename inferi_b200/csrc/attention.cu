@@ -10,27 +10,9 @@
 // un-normalised partial (max, sum, accumulator); the last CTA of a kv head to arrive merges the partials — no CTA
 // ever waits for another.  The split count is derived from the position on the device, so the same launch (and
 // the same CUDA graph node) serves every context length.
-#include "attention.cuh"
-#include "attention_gqa4.cuh"
+#include "attention_group.cuh"
 
 namespace ib {
-
-constexpr int ATTN_STEPS = 8;              // row steps per tile kept in registers
-
-template <int HS, int KVM, typename T>
-__global__ void __launch_bounds__(ATTN_THREADS) attn_kernel(const AttnArgs a) {
-    __shared__ float sm[attn_block_smem_floats(HS, KVM)];
-    if (a.pdl == 1) asm volatile("griddepcontrol.launch_dependents;");   // (2: with the last rows, attn_block)
-    if (a.pdl == 2) asm volatile("griddepcontrol.wait;" ::: "memory");
-    // The position was written by the end of the previous token, many kernels ago, and not by the predecessor (which
-    // only waits for its own predecessor after it has let this kernel start): it can be read before the wait.
-    const uint32_t kvh = blockIdx.x, split = blockIdx.y;
-    const uint32_t pos = a.pos_ptr ? *a.pos_ptr : a.p.pos;
-    uint32_t nsplit, per;
-    attn_split_plan(pos + 1, a.max_splits, nsplit, per);
-    if (split >= nsplit) return;
-    attn_block<HS, KVM, T, ATTN_STEPS>(a, a.kc, a.vc, kvh, split, nsplit, per, pos + 1, (int)threadIdx.x, 1, sm, a.pdl == 1);
-}
 
 size_t attn_scratch_bytes(const ib_attn_params &p, uint32_t max_splits) {
     const size_t n_kv = p.n_heads / p.kv_mul;
@@ -38,47 +20,12 @@ size_t attn_scratch_bytes(const ib_attn_params &p, uint32_t max_splits) {
 }
 
 uint32_t attn_max_splits(const ib_ctx *ctx, const ib_attn_params &p) {
-    const uint32_t n_kv = p.n_heads / p.kv_mul;
-    uint32_t s = (uint32_t)(ctx->sm_count * 3) / (n_kv ? n_kv : 1);   // three CTAs of either kernel fit one SM: one wave
+    const uint32_t groups = attn_groups(p);
+    uint32_t s = (uint32_t)(ctx->sm_count * 3) / (groups ? groups : 1);   // three CTAs fit one SM: one wave
     if (s < 1) s = 1;
-    if (s > 256) s = 256;
-    // attn_kernel's merging block stages every slice's (max, sum) in its accumulator area: 2 * splits * kv_mul floats must fit the
-    // 4 * kv_mul * head_size it owns (attn_gqa4_kernel's holds 256 slices at either head size)
+    if (s > 256) s = 256;             // (the merging CTA keeps so many weights)
     if (s > 2 * p.head_size) s = 2 * p.head_size;
     return s;
-}
-
-template <int HS, int KVM, typename T>
-static int32_t launch_t(ib_ctx *ctx, cudaStream_t s, const AttnArgs &args, dim3 grid) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid;
-    cfg.blockDim = dim3(ATTN_THREADS);
-    cfg.stream = s;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = args.pdl ? 1 : 0;
-    IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, attn_kernel<HS, KVM, T>, args));
-    ctx->launches++;
-    return IB_OK;
-}
-
-template <int HS, typename T>
-static int32_t launch_kvm(ib_ctx *ctx, cudaStream_t s, const AttnArgs &args, dim3 grid) {
-    switch (args.p.kv_mul) {
-    case 1: return launch_t<HS, 1, T>(ctx, s, args, grid);
-    case 2: return launch_t<HS, 2, T>(ctx, s, args, grid);
-    case 4: return launch_t<HS, 4, T>(ctx, s, args, grid);
-    case 8: return launch_t<HS, 8, T>(ctx, s, args, grid);
-    default: return set_error(IB_ERR_UNSUPPORTED, "attention: kv_mul=%u (supported: 1, 2, 4, 8)", args.p.kv_mul);
-    }
-}
-
-// the Llama-3 shape (f16 cache, 4 query heads per kv head, head size 64 or 128, 16-byte aligned buffers) has a kernel of its own
-bool attn_gqa4_eligible(const AttnLaunch &a) {
-    return a.kv_dtype == IB_KV_F16 && a.p.kv_mul == 4 && (a.p.head_size == 64 || a.p.head_size == 128) && ((uintptr_t)a.q % 16) == 0 &&
-           ((uintptr_t)a.k_cache % 16) == 0 && ((uintptr_t)a.v_cache % 16) == 0 && ((uintptr_t)a.out % 16) == 0 && ((uintptr_t)a.scratch % 16) == 0;
 }
 
 // CTAs per cluster, one cluster per kv head.  Short: 8 while that is three (head size 128: two) on every SM, and from there on as many as fit
@@ -86,7 +33,7 @@ bool attn_gqa4_eligible(const AttnLaunch &a) {
 // Middle: its CTAs need an SM each and their clusters a GPC with so many free ones; on more than two thirds of the SMs some clusters wait
 // for others (12 kv heads x 8 CTAs fit; 16 x 8 take twice the time: 13.4 us against 8.9 as 16 x 4 at 2048 positions).  Fewer than 4 CTAs per kv head: no middle regime.
 static uint32_t gqa4_cluster_ctas(const ib_ctx *ctx, const ib_attn_params &p, uint32_t regime) {
-    const uint32_t n_kv = p.n_heads / p.kv_mul, room = (uint32_t)ctx->sm_count * 2 / (regime == ATTN_MIDDLE ? 3 : 2);
+    const uint32_t n_kv = attn_groups(p), room = (uint32_t)ctx->sm_count * 2 / (regime == ATTN_MIDDLE ? 3 : 2);
     uint32_t c = GQA4_CLUSTER_MAX;
     if (regime == ATTN_SHORT && c * n_kv <= (p.head_size == 128 ? 2 : 3) * (uint32_t)ctx->sm_count) return c;
     while (c > 1 && c * n_kv > room) c /= 2;
@@ -107,20 +54,28 @@ static uint32_t gqa4_cluster_ctas(const ib_ctx *ctx, const ib_attn_params &p, ui
 //                   at 1900, 48.7 / 48.0 at 2700;  4 heads  28.3 / 29.9 at 1600.
 // The middle regime's ends are those of the token graph (for head size 64 beyond 3000 positions: the crossing back to back, moved by that margin).  Launches outside it, which take the same ones, would cross over earlier by the
 // figures above: up to 0.9 us of 8 between 4000 and 6400 positions of up to 8 heads of 64, 0.7 of 7 below 2560 positions of 2 to 4 heads of 128.
+// Groups of one or two heads and the f32 cache have no middle regime; short / long, us: f16, head size 128, 8 x 2 heads 2.9 / 3.7 at 200 positions, 4.3 / 4.1 at
+// 450, 16 x 1 4.3 / 4.5 at 450 (6.1 / 5.6 at 900); head size 64, 8 x 2 3.2 / 3.4 at 450 (5.6 / 4.7 at 900).  f32, head size 128, 8 x 4 4.6 / 5.0 at 200,
+// 6.4 / 5.1 at 450, 8 x 8 3.7 / 4.1 at 60, 6.0 / 5.0 at 200, 16 x 1 4.0 / 4.7 at 200, 5.7 / 5.4 at 450; head size 64, 8 x 4 2.9 / 3.5 at 200, 4.2 / 4.0 at 450.
 // (2 to 4 heads of 128 end at 2560, 8 at 2400: the latter was measured in the graph up to its crossing, the former at 1600 only.)
 uint32_t attn_regime_positions(const ib_ctx *ctx, const AttnLaunch &a, uint32_t regime) {
-    if (!attn_gqa4_eligible(a) || ctx->sm_count == 0) return 0u;
-    const uint32_t n_kv = a.p.n_heads / a.p.kv_mul, middle = gqa4_cluster_ctas(ctx, a.p, ATTN_MIDDLE), c = gqa4_cluster_ctas(ctx, a.p, regime);
+    if (ctx->sm_count == 0) return 0u;
+    const bool has_middle = a.kv_dtype == IB_KV_F16 && a.p.kv_mul >= ATTN_GROUP;
+    const uint32_t n_kv = attn_groups(a.p), middle = has_middle ? gqa4_cluster_ctas(ctx, a.p, ATTN_MIDDLE) : 0u;
+    const uint32_t c = regime == ATTN_MIDDLE ? middle : gqa4_cluster_ctas(ctx, a.p, regime);
     const bool wide = a.p.head_size == 128;
     if (regime == ATTN_MIDDLE) return c * (wide ? (c < 8 ? 256 : (n_kv <= 4 ? 320 : (n_kv <= 8 ? 300 : 384))) : (c < 8 ? 512 : (n_kv <= 8 ? 800 : 1400)));
+    if (!has_middle) return c * (wide ? (a.kv_dtype == IB_KV_F16 ? 48 : (a.p.kv_mul > ATTN_GROUP ? 16 : 32)) : (a.kv_dtype == IB_KV_F16 ? 64 : 48));
     if (middle == 0 || c < 8) return c * (wide && middle ? 24 : 64);
     return c * (wide ? 24 : (middle < 8 ? 96 : (n_kv <= 4 ? 256 : 128)));
 }
 
-template <int HS, uint32_t REGIME>
-static int32_t launch_gqa4(ib_ctx *ctx, cudaStream_t s, const AttnArgs &args, dim3 grid) {
-    const uint32_t smem = gqa4_smem_floats(HS, REGIME) * sizeof(float);   // at most 48 KB: no attribute needed
-    static_assert(gqa4_smem_floats(HS, REGIME) * sizeof(float) + 4096 <= 49152, "dynamic and static shared memory without opting in");
+static bool attn_aligned(const float *q, const float *out) { return ((uintptr_t)q % 16) == 0 && ((uintptr_t)out % 16) == 0; }
+
+template <int HS, int KVM, typename T, uint32_t REGIME, bool ALIGNED = true>
+static int32_t launch_group(ib_ctx *ctx, cudaStream_t s, const AttnArgs &args, dim3 grid) {
+    constexpr uint32_t smem = gqa4_smem_floats(HS, KVM, REGIME) * sizeof(float);
+    static_assert(smem + 4096 <= 49152, "dynamic and static shared memory without opting in");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = dim3(gqa4_warps(HS, REGIME) * 32);
@@ -135,9 +90,27 @@ static int32_t launch_gqa4(ib_ctx *ctx, cudaStream_t s, const AttnArgs &args, di
     attr[1].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = args.pdl ? 2 : 1;
-    IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, attn_gqa4_kernel<HS, REGIME>, args));
+    IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, attn_group_kernel<HS, KVM, T, REGIME, ALIGNED>, args));
     ctx->launches++;
     return IB_OK;
+}
+
+template <int HS, int KVM, typename T>
+static int32_t launch_regime(ib_ctx *ctx, cudaStream_t s, const AttnArgs &args, dim3 grid, uint32_t regime) {
+    if (!attn_aligned(args.q, args.out)) return launch_group<HS, KVM, T, ATTN_LONG, false>(ctx, s, args, grid);
+    if constexpr (KVM == (int)ATTN_GROUP && sizeof(T) == 2)
+        if (regime == ATTN_MIDDLE) return launch_group<HS, KVM, T, ATTN_MIDDLE>(ctx, s, args, grid);
+    return regime == ATTN_SHORT ? launch_group<HS, KVM, T, ATTN_SHORT>(ctx, s, args, grid) : launch_group<HS, KVM, T, ATTN_LONG>(ctx, s, args, grid);
+}
+
+template <int HS, typename T>
+static int32_t launch_heads(ib_ctx *ctx, cudaStream_t s, const AttnArgs &args, dim3 grid, uint32_t regime) {
+    switch (args.p.kv_mul) {
+    case 1: return launch_regime<HS, 1, T>(ctx, s, args, grid, regime);
+    case 2: return launch_regime<HS, 2, T>(ctx, s, args, grid, regime);
+    case 4: case 8: return launch_regime<HS, 4, T>(ctx, s, args, grid, regime);
+    default: return set_error(IB_ERR_UNSUPPORTED, "attention: kv_mul=%u (supported: 1, 2, 4, 8)", args.p.kv_mul);
+    }
 }
 
 int32_t launch_attention(ib_ctx *ctx, cudaStream_t s, const AttnLaunch &a) {
@@ -149,41 +122,28 @@ int32_t launch_attention(ib_ctx *ctx, cudaStream_t s, const AttnLaunch &a) {
     IB_REQUIRE(a.max_splits >= 1 && a.max_splits <= 2 * p.head_size && a.max_splits <= 256, "attention: %u position slices exceed what the merge step holds (%u)",
                a.max_splits, 2 * p.head_size < 256 ? 2 * p.head_size : 256);
     IB_REQUIRE(((uintptr_t)a.k_cache % 16) == 0 && ((uintptr_t)a.v_cache % 16) == 0, "attention: the caches must be 16-byte aligned");
+    if (p.head_size != 64 && p.head_size != 128) return set_error(IB_ERR_UNSUPPORTED, "attention: head_size=%u (supported: 64, 128)", p.head_size);
+    if (p.kv_mul != 1 && p.kv_mul != 2 && p.kv_mul != 4 && p.kv_mul != 8) return set_error(IB_ERR_UNSUPPORTED, "attention: kv_mul=%u (supported: 1, 2, 4, 8)", p.kv_mul);
     AttnArgs args{p, a.pos_ptr, a.q, a.k_cache, a.v_cache, a.out, a.scratch, a.counters, a.max_splits, a.pdl, 0u};
+    // A launch that serves many positions (a graph node) is told the regime they are in.  A caller's q or output off the 16-byte boundaries: the long
+    // one, whatever the position.
+    const bool aligned = attn_aligned(a.q, a.out);
+    uint32_t regime = aligned ? a.regime : ATTN_LONG;
+    if (!a.pos_ptr && aligned) {
+        regime = ATTN_LONG;
+        for (uint32_t r : {ATTN_MIDDLE, ATTN_SHORT})
+            if (p.pos < attn_regime_positions(ctx, a, r)) regime = r;
+    }
+    uint32_t splits = a.max_splits, per;
+    if (regime != ATTN_LONG) args.cluster = splits = gqa4_cluster_ctas(ctx, p, regime);
+    if (!a.pos_ptr) {   // with a host-known position only the slices that will do work are launched
+        gqa4_plan(p.pos + 1, a.max_splits, args.cluster, gqa4_warps(p.head_size, regime), p.kv_mul, splits, per);
+        if (regime != ATTN_LONG) args.cluster = splits;
+    }
+    const dim3 grid(attn_groups(p), splits);
     const bool f16 = a.kv_dtype == IB_KV_F16;
-    const bool gqa4 = attn_gqa4_eligible(a);
-    if (gqa4) {
-        // a launch that serves many positions (a graph node) is told the regime they are in
-        uint32_t regime = a.regime;
-        if (!a.pos_ptr) {
-            regime = ATTN_LONG;
-            for (uint32_t r : {ATTN_MIDDLE, ATTN_SHORT})
-                if (p.pos < attn_regime_positions(ctx, a, r)) regime = r;
-        }
-        uint32_t splits = a.max_splits, per;
-        if (regime != ATTN_LONG) args.cluster = splits = gqa4_cluster_ctas(ctx, p, regime);
-        if (!a.pos_ptr) {   // with a host-known position only the slices that will do work are launched
-            gqa4_plan(p.pos + 1, a.max_splits, args.cluster, gqa4_warps(p.head_size, regime), splits, per);
-            if (regime != ATTN_LONG) args.cluster = splits;
-        }
-        const dim3 grid(n_kv, splits);
-        const bool wide = p.head_size == 128;
-        switch (regime) {
-        case ATTN_SHORT: return wide ? launch_gqa4<128, ATTN_SHORT>(ctx, s, args, grid) : launch_gqa4<64, ATTN_SHORT>(ctx, s, args, grid);
-        case ATTN_MIDDLE: return wide ? launch_gqa4<128, ATTN_MIDDLE>(ctx, s, args, grid) : launch_gqa4<64, ATTN_MIDDLE>(ctx, s, args, grid);
-        default: return wide ? launch_gqa4<128, ATTN_LONG>(ctx, s, args, grid) : launch_gqa4<64, ATTN_LONG>(ctx, s, args, grid);
-        }
-    }
-    uint32_t splits = a.max_splits;
-    if (!a.pos_ptr) {
-        uint32_t need, per;
-        attn_split_plan(p.pos + 1, a.max_splits, need, per);
-        if (need < splits) splits = need;
-    }
-    const dim3 grid(n_kv, splits);
-    if (p.head_size == 128) return f16 ? launch_kvm<128, __half>(ctx, s, args, grid) : launch_kvm<128, float>(ctx, s, args, grid);
-    if (p.head_size == 64) return f16 ? launch_kvm<64, __half>(ctx, s, args, grid) : launch_kvm<64, float>(ctx, s, args, grid);
-    return set_error(IB_ERR_UNSUPPORTED, "attention: head_size=%u (supported: 64, 128)", p.head_size);
+    if (p.head_size == 128) return f16 ? launch_heads<128, __half>(ctx, s, args, grid, regime) : launch_heads<128, float>(ctx, s, args, grid, regime);
+    return f16 ? launch_heads<64, __half>(ctx, s, args, grid, regime) : launch_heads<64, float>(ctx, s, args, grid, regime);
 }
 
 }  // namespace ib
@@ -200,13 +160,13 @@ int32_t launch_attention(ib_ctx *ctx, cudaStream_t s, const AttnLaunch &a) {
 // -------------------------------------------------------------------------------------------------------------------
 namespace ib {
 constexpr uint32_t STATIC_ATTN_FLOATS = 262144;    // 1 MiB of partials: bounds n_heads * (head_size + 2) * splits
-constexpr uint32_t STATIC_ATTN_KV_HEADS = 256;     // arrival counters, one per kv head
+constexpr uint32_t STATIC_ATTN_KV_HEADS = 256;     // arrival counters: two per kv head at most (attn_groups)
 constexpr uint32_t STATIC_ATTN_MAX_SPLITS = 32;
 constexpr int STATIC_ATTN_MAX_DEVICES = 64;
 }  // namespace ib
 
 static __device__ __align__(256) float g_static_attn_scratch[ib::STATIC_ATTN_FLOATS];
-static __device__ __align__(256) unsigned int g_static_attn_counters[ib::STATIC_ATTN_KV_HEADS];
+static __device__ __align__(256) unsigned int g_static_attn_counters[2 * ib::STATIC_ATTN_KV_HEADS];
 
 // Device addresses of the two arrays, looked up once per device.  In host code the array names above are only
 // host-side stand-ins for the symbols; the addresses a kernel can use come from cudaGetSymbolAddress, called with the

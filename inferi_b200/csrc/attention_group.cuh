@@ -1,14 +1,12 @@
-// Decode attention for the shape the Llama-3 family uses: f16 cache, 4 query heads per kv head, head size 64 or 128.
-//
-// Same semantics and the same split-K scheme as attention.cuh (one CTA per (kv head, position slice), un-normalised
-// partials, the last CTA of a kv head to arrive merges them; crates/inferi-shaders/src/fused_attention.rs:63-241 and
-// :374-617 are what it replaces), but built for a short critical path at small contexts and for few instructions per
-// cache row at long ones:
-//  * a warp step covers 8 cache rows (HS 128: 4 steps of 2 rows, 16 lanes per row; HS 64: 2 steps of 4 rows, 8 lanes per
-//    row); a lane holds 8 elements of a row and the matching 8 elements of the 4 query vectors;
-//  * the 16 (or 8) per-lane partial scores of the step go through a halving exchange (each shuffle moves one value and
+// Decode attention: one launch's device side.  One CTA per (group of query heads, position slice), un-normalised partials, the last CTA of a group to
+// arrive merges them; crates/inferi-shaders/src/fused_attention.rs:63-241 and :374-617 are what it replaces.  A group is up to four query heads
+// of one kv head (eight are two groups, which read the same rows: the second time from L2), head size 64 or 128, an f16 or f32 cache.
+// Built for a short critical path at small contexts and for few instructions per cache row at long ones:
+//  * a lane holds 8 elements of a cache row and the matching 8 elements of the group's query vectors: 16 lanes a row of 128, 8 lanes a row of 64;
+//    a warp step covers 8 rows (4 of f32 at head size 128: their registers);
+//  * the per-lane partial scores of the step go through a halving exchange (each shuffle moves one value and
 //    leaves half as many to reduce) instead of a butterfly per score: afterwards every lane owns exactly one
-//    (row, head) score, so exp() is evaluated once per score, not once per lane;
+//    (row, head) score - two or four lanes the same one where a step has fewer scores than lanes - so exp() is evaluated once per score;
 //  * the probabilities travel back to the lanes through 128 bytes of shared memory per warp;
 //  * multiply-adds are issued as packed pairs (fma.rn.f32x2);
 //  * the loop body is small (no 8-step unrolling): at short contexts the kernel runs its code once, and the time goes
@@ -20,6 +18,9 @@
 #include <cooperative_groups.h>
 
 namespace ib {
+
+constexpr uint32_t ATTN_GROUP = 4;   // query heads of a group, at most
+__host__ __device__ constexpr uint32_t attn_groups(const ib_attn_params &p) { return p.n_heads / (p.kv_mul < ATTN_GROUP ? p.kv_mul : ATTN_GROUP); }
 
 constexpr uint32_t GQA4_ROWS_PER_WARP_STEP = 8;
 // Three ways to split a kv head's positions, by context length:
@@ -37,10 +38,12 @@ constexpr uint32_t GQA4_ROWS_PER_WARP_STEP = 8;
 constexpr uint32_t GQA4_CLUSTER_MAX = 8;
 __host__ __device__ constexpr int gqa4_warps(uint32_t hs, uint32_t regime) { return regime != ATTN_MIDDLE ? ATTN_WARPS : (hs == 128 ? 8 : 16); }   // (head size 128 needs 196 registers a thread)
 constexpr uint32_t GQA4_MIN_PER_SPLIT = ATTN_WARPS * GQA4_ROWS_PER_WARP_STEP, GQA4_KNEE = 16, GQA4_KNEE_PER = 128;
-__host__ __device__ __forceinline__ void gqa4_plan(uint32_t total, uint32_t max_splits, uint32_t cluster, uint32_t warps, uint32_t &nsplit, uint32_t &per) {
+constexpr uint32_t GQA4_ALONE = 64;   // rows of one or two heads that one CTA is as fast with as two that merge (60 rows, 16 x 1 heads of 128: 2.4 us, 2.7 as two)
+__host__ __device__ __forceinline__ void gqa4_plan(uint32_t total, uint32_t max_splits, uint32_t cluster, uint32_t warps, uint32_t heads, uint32_t &nsplit, uint32_t &per) {
     if (cluster) {
         nsplit = (total + warps * GQA4_ROWS_PER_WARP_STEP - 1) / (warps * GQA4_ROWS_PER_WARP_STEP);
         if (nsplit > cluster) nsplit = cluster;
+        if (heads <= 2 && total <= GQA4_ALONE) nsplit = 1;
         per = (total + nsplit - 1) / nsplit;
         nsplit = (total + per - 1) / per;
     } else {
@@ -73,6 +76,18 @@ __device__ __forceinline__ void halve_exchange(float (&v)[N], int lane, int o) {
     }
 }
 
+// N consecutive floats of shared memory (aligned to all of them)
+template <int N>
+__device__ __forceinline__ void load_few(float (&f)[N], const float *p) {
+    if constexpr (N == 4) {
+        const float4 v = *reinterpret_cast<const float4 *>(p);
+        f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+    } else if constexpr (N == 2) {
+        const float2 v = *reinterpret_cast<const float2 *>(p);
+        f[0] = v.x; f[1] = v.y;
+    } else f[0] = p[0];
+}
+
 // o += w * p[0 .. N-1];  p[0 .. N-1] = w * o: in pairs where there are any (p is 8-byte aligned then)
 template <int N>
 __device__ __forceinline__ void add_scaled(float (&o)[N], float w, const float *p) {
@@ -103,20 +118,61 @@ __device__ __forceinline__ void store_scaled(float *p, const float (&o)[N], floa
 // first is 64 instructions per round that every launch fetches and runs once.  (Many warps: they are added up first.)
 __host__ __device__ constexpr uint32_t gqa4_groups(uint32_t hs, uint32_t regime) { return regime == ATTN_MIDDLE ? 1 : 256 / hs; }
 // floats of dynamic shared memory: the warps' accumulators, and with clusters the slices' partials (in the first CTA)
-__host__ __device__ constexpr uint32_t gqa4_smem_floats(uint32_t hs, uint32_t regime) {
-    return gqa4_warps(hs, regime) * gqa4_groups(hs, regime) * 4 * hs + (regime != ATTN_LONG ? GQA4_CLUSTER_MAX * 4 * (hs + 2) : 0);
+__host__ __device__ constexpr uint32_t gqa4_smem_floats(uint32_t hs, uint32_t kvm, uint32_t regime) {
+    return gqa4_warps(hs, regime) * gqa4_groups(hs, regime) * kvm * hs + (regime != ATTN_LONG ? GQA4_CLUSTER_MAX * kvm * (hs + 2) : 0);
+}
+// The caller's output: in pairs, or one by one where it is aligned to 4 bytes only
+template <int N>
+__device__ __forceinline__ void store_out(float *p, const float (&o)[N], float w, bool pairs) {
+    if (pairs) store_scaled(p, o, w);
+    else {
+#pragma unroll
+        for (int e = 0; e < N; e++) p[e] = o[e] * w;
+    }
 }
 
-template <int HS, uint32_t REGIME>
-__global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MIDDLE ? 1 : 3) attn_gqa4_kernel(const AttnArgs a) {
-    constexpr int KVM = 4, EPL = 8;
+// A lane's 8 elements of a cache row: one 16-byte load of f16, two of f32 (each of them 16 bytes of every lane side by side).  FIRST, SECOND: where its
+// elements 0-3 and 4-7 are in the row.
+template <typename T, int HS> struct LaneRow;
+template <int HS> struct LaneRow<__half, HS> {
+    uint4 r;
+    static __device__ __forceinline__ uint32_t first(int li) { return 8 * li; }
+    static __device__ __forceinline__ uint32_t second(int li) { return 8 * li + 4; }
+    __device__ __forceinline__ void load(const __half *row, int li) { r = __ldcg(reinterpret_cast<const uint4 *>(row + 8 * li)); }
+    __device__ __forceinline__ void get(float2 (&f)[4]) const {
+        const __half2 *h = reinterpret_cast<const __half2 *>(&r);
+#pragma unroll
+        for (int j = 0; j < 4; j++) f[j] = __half22float2(h[j]);
+    }
+};
+template <int HS> struct LaneRow<float, HS> {
+    float4 a, b;
+    static __device__ __forceinline__ uint32_t first(int li) { return 4 * li; }
+    static __device__ __forceinline__ uint32_t second(int li) { return HS / 2 + 4 * li; }
+    __device__ __forceinline__ void load(const float *row, int li) {
+        a = __ldcg(reinterpret_cast<const float4 *>(row + first(li)));
+        b = __ldcg(reinterpret_cast<const float4 *>(row + second(li)));
+    }
+    __device__ __forceinline__ void get(float2 (&f)[4]) const {
+        f[0] = make_float2(a.x, a.y); f[1] = make_float2(a.z, a.w);
+        f[2] = make_float2(b.x, b.y); f[3] = make_float2(b.z, b.w);
+    }
+};
+constexpr int attn_log2(int n) { return n <= 1 ? 0 : 1 + attn_log2(n / 2); }
+
+// ALIGNED: q and out are on 16-byte boundaries.  (A run-time choice made launches of 200 to 250 positions of 8 x 4 heads of 128 0.2 of 3.7 us slower: code.)
+template <int HS, int KVM, typename T, uint32_t REGIME, bool ALIGNED>
+__global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MIDDLE ? 1 : 3) attn_group_kernel(const AttnArgs a) {
+    constexpr int EPL = 8;
     constexpr bool CLUSTER = REGIME != ATTN_LONG;
-    constexpr int W = gqa4_warps(HS, REGIME), T = W * 32;
+    constexpr int W = gqa4_warps(HS, REGIME), THREADS = W * 32;
     constexpr int L = HS / EPL;          // lanes per cache row
     constexpr int RPW = 32 / L;          // rows per warp step
-    constexpr int STEPS = L / KVM;       // steps per warp iteration: STEPS * KVM partial scores per lane = L
-    constexpr int ROWS = STEPS * RPW;    // = 8
-    static_assert(ROWS == (int)GQA4_ROWS_PER_WARP_STEP && STEPS * KVM == L, "lane layout");
+    constexpr int STEPS = sizeof(T) == 2 ? HS / 32 : 2;   // steps per warp iteration
+    constexpr int ROWS = STEPS * RPW;
+    constexpr int N = STEPS * KVM;       // partial scores per lane and iteration; L / N lanes end up with the same complete one
+    static_assert(N <= L && (N & (N - 1)) == 0, "lane layout");
+    constexpr int DUP = attn_log2(L / N), FROM_S = 1 << (DUP + attn_log2(KVM));   // the lane's bits: [row group][step][head][copy]
     constexpr int G = gqa4_groups(HS, REGIME);
     static_assert(G == 1 || G == RPW, "row groups of a warp");
     extern __shared__ __align__(16) float sm_acc[];   // [W][G][KVM][HS]
@@ -139,10 +195,10 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
     const bool early = a.pdl == 1;   // rows may be requested ahead of the wait
     if (a.pdl == 2) asm volatile("griddepcontrol.wait;" ::: "memory");
     // The position was written at the end of the previous token, not by the predecessor: it can be read before the wait.
-    const uint32_t kvh = blockIdx.x, split = blockIdx.y;
+    const uint32_t kvh = blockIdx.x, split = blockIdx.y;   // (kvh: the group's number)
     const uint32_t total = (a.pos_ptr ? *a.pos_ptr : a.p.pos) + 1;
     uint32_t nsplit, per;
-    gqa4_plan(total, a.max_splits, CLUSTER ? a.cluster : 0u, W, nsplit, per);
+    gqa4_plan(total, a.max_splits, CLUSTER ? a.cluster : 0u, W, KVM, nsplit, per);
     if (split >= nsplit) {
         if constexpr (CLUSTER) {
             cluster.barrier_wait();
@@ -154,22 +210,24 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane / L, li = lane % L;
     const uint32_t kv_dim = a.p.kv_dim;
-    const __half *kc = reinterpret_cast<const __half *>(a.kc) + (size_t)kvh * HS + li * EPL;
-    const __half *vc = reinterpret_cast<const __half *>(a.vc) + (size_t)kvh * HS + li * EPL;
+    const uint32_t cache_head = KVM == (int)ATTN_GROUP ? kvh >> (a.p.kv_mul > ATTN_GROUP ? 1 : 0) : kvh;   // (eight heads: two groups)
+    const T *kc = reinterpret_cast<const T *>(a.kc) + (size_t)cache_head * HS;
+    const T *vc = reinterpret_cast<const T *>(a.vc) + (size_t)cache_head * HS;
+    const uint32_t at0 = LaneRow<T, HS>::first(li), at1 = LaneRow<T, HS>::second(li);
     const float scale = 1.0f / sqrtf((float)HS);
 
     // First iteration: the predecessor (the q/k/v kernel) writes this token's q and the newest cache row (position
     // total - 1); every older row is from earlier tokens.  So the older rows are requested before the wait for the
     // predecessor, q and the newest row after it: the cache round trip overlaps the predecessor's tail.
-    uint4 kraw[STEPS], vraw[STEPS];
+    LaneRow<T, HS> kraw[STEPS], vraw[STEPS];
     const uint32_t base0 = t0 + warp * ROWS;
     if (base0 < t1) {
 #pragma unroll
         for (int s = 0; s < STEPS; s++) {
             const uint32_t t = base0 + s * RPW + g, tc = t < t1 ? t : t1 - 1;
             if (tc + 1 != total || !early) {
-                kraw[s] = __ldcg(reinterpret_cast<const uint4 *>(kc + (size_t)tc * kv_dim));
-                vraw[s] = __ldcg(reinterpret_cast<const uint4 *>(vc + (size_t)tc * kv_dim));
+                kraw[s].load(kc + (size_t)tc * kv_dim, li);
+                vraw[s].load(vc + (size_t)tc * kv_dim, li);
             }
         }
     }
@@ -180,8 +238,8 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
             for (int s = 0; s < STEPS; s++) {
                 const uint32_t t = base0 + s * RPW + g, tc = t < t1 ? t : t1 - 1;
                 if (tc + 1 == total) {
-                    kraw[s] = __ldcg(reinterpret_cast<const uint4 *>(kc + (size_t)tc * kv_dim));
-                    vraw[s] = __ldcg(reinterpret_cast<const uint4 *>(vc + (size_t)tc * kv_dim));
+                    kraw[s].load(kc + (size_t)tc * kv_dim, li);
+                    vraw[s].load(vc + (size_t)tc * kv_dim, li);
                 }
             }
         }
@@ -189,14 +247,22 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
     float2 q2[KVM][EPL / 2];
 #pragma unroll
     for (int m = 0; m < KVM; m++) {
-        const float4 *qp = reinterpret_cast<const float4 *>(a.q + (size_t)(kvh * KVM + m) * HS + li * EPL);
-        const float4 x = __ldcg(qp), y = __ldcg(qp + 1);
+        const float *qp = a.q + (size_t)(kvh * KVM + m) * HS;
+        float4 x, y;
+        if constexpr (ALIGNED) {
+            x = __ldcg(reinterpret_cast<const float4 *>(qp + at0));
+            y = __ldcg(reinterpret_cast<const float4 *>(qp + at1));
+        } else {
+            x = make_float4(__ldcg(qp + at0), __ldcg(qp + at0 + 1), __ldcg(qp + at0 + 2), __ldcg(qp + at0 + 3));
+            y = make_float4(__ldcg(qp + at1), __ldcg(qp + at1 + 1), __ldcg(qp + at1 + 2), __ldcg(qp + at1 + 3));
+        }
         q2[m][0] = make_float2(x.x, x.y); q2[m][1] = make_float2(x.z, x.w);
         q2[m][2] = make_float2(y.x, y.y); q2[m][3] = make_float2(y.z, y.w);
     }
 
     // running maximum and sum of the head this lane scores (m_own); accumulators of all four heads for the lane's 8 elements
-    const int s_own = li / KVM;   // (and head li % KVM)
+    const int s_own = (li >> DUP) / KVM;   // (and head (li >> DUP) % KVM)
+    const bool owner = (li & ((1 << DUP) - 1)) == 0;
     float M = -INFINITY, l = 0.f;
     float2 acc[KVM][EPL / 2];
 #pragma unroll
@@ -206,7 +272,7 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
 
     // The rows of the next iteration are requested before the current ones are used: a slice is then one cache round
     // trip plus arithmetic, however many iterations it has, and twice the bytes are in flight per warp.
-    uint4 knext[STEPS], vnext[STEPS];
+    LaneRow<T, HS> knext[STEPS], vnext[STEPS];
 #pragma unroll 1
     for (uint32_t base = base0; base < t1; base += W * ROWS) {
         const uint32_t nbase = base + W * ROWS;
@@ -215,18 +281,16 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
 #pragma unroll
             for (int s = 0; s < STEPS; s++) {
                 const uint32_t t = nbase + s * RPW + g, tc = t < t1 ? t : t1 - 1;
-                knext[s] = __ldcg(reinterpret_cast<const uint4 *>(kc + (size_t)tc * kv_dim));
-                vnext[s] = __ldcg(reinterpret_cast<const uint4 *>(vc + (size_t)tc * kv_dim));
+                knext[s].load(kc + (size_t)tc * kv_dim, li);
+                vnext[s].load(vc + (size_t)tc * kv_dim, li);
             }
         }
         // partial scores of the lane's 8 elements: v[s * KVM + m]
-        float v[L];
+        float v[N];
 #pragma unroll
         for (int s = 0; s < STEPS; s++) {
-            const __half2 *h = reinterpret_cast<const __half2 *>(&kraw[s]);
             float2 k2[EPL / 2];
-#pragma unroll
-            for (int j = 0; j < EPL / 2; j++) k2[j] = __half22float2(h[j]);
+            kraw[s].get(k2);
 #pragma unroll
             for (int m = 0; m < KVM; m++) {
                 float2 d = make_float2(0.f, 0.f);
@@ -235,42 +299,51 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
                 v[s * KVM + m] = d.x + d.y;
             }
         }
-        // complete sums: lane li of the row ends up with score number li = s_own * KVM + m_own
-        if constexpr (L == 16) {
-            halve_exchange<16>(v, lane, 8);
-        }
-        halve_exchange<8>(reinterpret_cast<float (&)[8]>(v), lane, 4);
-        halve_exchange<4>(reinterpret_cast<float (&)[4]>(v), lane, 2);
-        halve_exchange<2>(reinterpret_cast<float (&)[2]>(v), lane, 1);
+        // complete sums: lane li of the row ends up with score number li >> DUP = s_own * KVM + m_own
+        constexpr int H = L / 2;   // the first round's distance
+        if constexpr (N == 16) {
+            halve_exchange<16>(v, lane, H);
+            halve_exchange<8>(reinterpret_cast<float (&)[8]>(v), lane, H / 2);
+            halve_exchange<4>(reinterpret_cast<float (&)[4]>(v), lane, H / 4);
+            halve_exchange<2>(reinterpret_cast<float (&)[2]>(v), lane, H / 8);
+        } else if constexpr (N == 8) {
+            halve_exchange<8>(v, lane, H);
+            halve_exchange<4>(reinterpret_cast<float (&)[4]>(v), lane, H / 2);
+            halve_exchange<2>(reinterpret_cast<float (&)[2]>(v), lane, H / 4);
+        } else if constexpr (N == 4) {
+            halve_exchange<4>(v, lane, H);
+            halve_exchange<2>(reinterpret_cast<float (&)[2]>(v), lane, H / 2);
+        } else halve_exchange<2>(v, lane, H);
+#pragma unroll
+        for (int o = (1 << DUP) / 2; o; o >>= 1) v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
         const bool valid = (base + s_own * RPW + g) < t1;
         const float sc = valid ? v[0] * scale : -INFINITY;
-        // block maximum of the head over the warp's 8 rows: the lanes that share m_own differ in bits 2..4
+        // block maximum of the head over the warp's rows
         float bm = sc;
-        bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 4));
-        bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 8));
-        bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, 16));
+#pragma unroll
+        for (int o = FROM_S; o < 32; o <<= 1) bm = fmaxf(bm, __shfl_xor_sync(0xffffffffu, bm, o));
         const float Mn = fmaxf(M, bm);   // finite: row `base` (step 0, group 0) is valid
         const float alpha = expf(M - Mn), pe = expf(sc - Mn);
         M = Mn;
         l = l * alpha + pe;
         __syncwarp();   // the previous iteration's reads of sm_p are done
-        sm_p[warp][lane] = pe;   // index g * L + s * KVM + m
-        if (lane < KVM) sm_alpha[warp][lane] = alpha;   // lanes 0..3: group 0, step 0, m_own = lane
+        if (owner) {
+            sm_p[warp][g * N + (li >> DUP)] = pe;   // index g * N + s * KVM + m
+            if (lane < FROM_S) sm_alpha[warp][lane >> DUP] = alpha;   // group 0, step 0: m_own
+        }
         __syncwarp();
-        const float4 al = *reinterpret_cast<const float4 *>(sm_alpha[warp]);
-        const float alv[KVM] = {al.x, al.y, al.z, al.w};
+        float alv[KVM];
+        load_few<KVM>(alv, sm_alpha[warp]);
 #pragma unroll
         for (int m = 0; m < KVM; m++)
 #pragma unroll
             for (int j = 0; j < EPL / 2; j++) { acc[m][j].x *= alv[m]; acc[m][j].y *= alv[m]; }
 #pragma unroll
         for (int s = 0; s < STEPS; s++) {
-            const __half2 *h = reinterpret_cast<const __half2 *>(&vraw[s]);
-            const float4 p4 = *reinterpret_cast<const float4 *>(&sm_p[warp][g * L + s * KVM]);
-            const float pv[KVM] = {p4.x, p4.y, p4.z, p4.w};
+            float pv[KVM];
+            load_few<KVM>(pv, &sm_p[warp][g * N + s * KVM]);
             float2 v2[EPL / 2];
-#pragma unroll
-            for (int j = 0; j < EPL / 2; j++) v2[j] = __half22float2(h[j]);
+            vraw[s].get(v2);
 #pragma unroll
             for (int m = 0; m < KVM; m++)
 #pragma unroll
@@ -295,23 +368,22 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
                 }
         }
     }
-    l += __shfl_xor_sync(0xffffffffu, l, 4);    // the lanes that score the same head: bits 2..4
-    l += __shfl_xor_sync(0xffffffffu, l, 8);
-    l += __shfl_xor_sync(0xffffffffu, l, 16);
+#pragma unroll
+    for (int o = FROM_S; o < 32; o <<= 1) l += __shfl_xor_sync(0xffffffffu, l, o);   // the lanes that score the same head
     if (G > 1 || g == 0) {
-        float4 *dst = reinterpret_cast<float4 *>(&sm_acc[(warp * G + (G > 1 ? g : 0)) * KVM * HS + li * EPL]);
+        float *dst = &sm_acc[(warp * G + (G > 1 ? g : 0)) * KVM * HS];
 #pragma unroll
         for (int m = 0; m < KVM; m++) {
-            dst[m * (HS / 4)] = make_float4(acc[m][0].x, acc[m][0].y, acc[m][1].x, acc[m][1].y);
-            dst[m * (HS / 4) + 1] = make_float4(acc[m][2].x, acc[m][2].y, acc[m][3].x, acc[m][3].y);
+            *reinterpret_cast<float4 *>(dst + m * HS + at0) = make_float4(acc[m][0].x, acc[m][0].y, acc[m][1].x, acc[m][1].y);
+            *reinterpret_cast<float4 *>(dst + m * HS + at1) = make_float4(acc[m][2].x, acc[m][2].y, acc[m][3].x, acc[m][3].y);
         }
     }
-    if (lane < KVM) { sm_m[warp * KVM + lane] = M; sm_l[warp * KVM + lane] = l; }
+    if (owner && lane < FROM_S) { sm_m[warp * KVM + (lane >> DUP)] = M; sm_l[warp * KVM + (lane >> DUP)] = l; }
     __syncthreads();
 
     // every thread owns PER consecutive outputs of one head (16 warps at head size 64: half of the threads one each)
     constexpr uint32_t slot = HS + 2;
-    constexpr int PER = KVM * HS >= T ? KVM * HS / T : 1;
+    constexpr int PER = KVM * HS >= THREADS ? KVM * HS / THREADS : 1;
     const bool has = tid * PER < KVM * HS;
     const int at = has ? tid * PER : 0, m_out = at / HS, d_out = at % HS;
     // partials in global memory: the accumulators [kv head][slice][KVM][HS], behind them all (max, sum) pairs [kv head][slice][KVM]
@@ -345,7 +417,7 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
             for (int e = 0; e < PER; e++) o[e] += ww * a[e];
         }
         if (nsplit == 1) {
-            if (has) store_scaled(out, o, 1.0f / ls);
+            if (has) store_out(out, o, 1.0f / ls, ALIGNED);
             if constexpr (CLUSTER) cluster.barrier_wait();
             return;
         }
@@ -372,11 +444,11 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
 #pragma unroll
             for (int e = 0; e < PER; e++) acc[e] = 0.f;
             for (uint32_t s = 0; s < nsplit; s++) add_scaled(acc, __shfl_sync(0xffffffffu, ws, s), sm_cl + (s * KVM + m_out) * slot + d_out);
-            store_scaled(out, acc, 1.0f / lsum);
+            store_out(out, acc, 1.0f / lsum, ALIGNED);
             return;
         } else {
-            store_scaled(part + m_out * HS + d_out, o, 1.0f);
-            if (d_out == 0) part_ml[split * KVM + m_out] = make_float2(mx, ls);
+            if (has) store_scaled(part + m_out * HS + d_out, o, 1.0f);
+            if (has && d_out == 0) part_ml[split * KVM + m_out] = make_float2(mx, ls);
         }
     }
     if constexpr (!CLUSTER) {
@@ -397,19 +469,21 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
     // L2 round trip, the first of them requested ahead of the weights.  Eight slices at a time with their pairs and a running maximum:
     // 21.4 us instead of 17.9 at 16384 positions of 8 heads of 128, 18.9 instead of 13.9 at 20000 of 64.
     constexpr uint32_t MAX_SLICES = 256, AT_ONCE = 16;   // (the launcher's limit of slices)
-    static_assert(W * MAX_SLICES * 4 <= gqa4_smem_floats(HS, REGIME) * 4, "the weights fit the accumulators' place");
+    static_assert(W * MAX_SLICES <= gqa4_smem_floats(HS, KVM, REGIME), "the weights fit the accumulators' place");
     float *sm_w = sm_acc + warp * MAX_SLICES;
     const float *mine = a.scratch + (size_t)kvh * a.max_splits * KVM * HS + m_out * HS + d_out;
-    float2 dat[AT_ONCE][PER / 2];
+    float dat[AT_ONCE][PER];
     auto fetch = [&](uint32_t s0) {
 #pragma unroll
         for (uint32_t j = 0; j < AT_ONCE; j++) {
             const float *ps = mine + (size_t)min(s0 + j, nsplit - 1) * (KVM * HS);   // (slices past the last one have weight 0)
             if constexpr (PER == 4) {
                 const float4 v = __ldcg(reinterpret_cast<const float4 *>(ps));
-                dat[j][0] = make_float2(v.x, v.y);
-                dat[j][1] = make_float2(v.z, v.w);
-            } else dat[j][0] = __ldcg(reinterpret_cast<const float2 *>(ps));
+                dat[j][0] = v.x; dat[j][1] = v.y; dat[j][2] = v.z; dat[j][3] = v.w;
+            } else if constexpr (PER == 2) {
+                const float2 v = __ldcg(reinterpret_cast<const float2 *>(ps));
+                dat[j][0] = v.x; dat[j][1] = v.y;
+            } else dat[j][0] = __ldcg(ps);
         }
     };
     fetch(0);
@@ -444,16 +518,13 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
         for (uint32_t j = 0; j < AT_ONCE; j++) {
             const float wt = sm_w[s0 + j];
 #pragma unroll
-            for (int e = 0; e < PER / 2; e++) {
-                o[2 * e] += wt * dat[j][e].x;
-                o[2 * e + 1] += wt * dat[j][e].y;
-            }
+            for (int e = 0; e < PER; e++) o[e] += wt * dat[j][e];
         }
         s0 += AT_ONCE;
         if (s0 >= nsplit) break;
         fetch(s0);
     }
-    store_scaled(a.out + (size_t)(kvh * KVM + m_out) * HS + d_out, o, 1.0f / ls);
+    if (has) store_out(out, o, 1.0f / ls, ALIGNED);
     if (tid == 0) a.counters[kvh] = 0u;
     }
 }

@@ -212,8 +212,8 @@ struct AttnLaunch {
     const void *k_cache, *v_cache;
     int kv_dtype;
     float *out;
-    float *scratch;            // [n_kv_heads][max_splits][kv_mul][head_size + 2]
-    unsigned int *counters;    // [n_kv_heads], zero before the first launch; the kernel re-zeroes them
+    float *scratch;            // n_kv_heads * max_splits * kv_mul * (head_size + 2) floats
+    unsigned int *counters;    // [2 * n_kv_heads], zero before the first launch; the kernel re-zeroes them
     uint32_t max_splits;
     uint32_t pdl;              // 0: plain launch; 1: programmatic dependent launch inside the token graph, where the predecessor writes only q and the
                                // newest cache row; 2: programmatic dependent launch behind any kernel
@@ -223,7 +223,6 @@ struct AttnLaunch {
     uint32_t regime;
 };
 constexpr uint32_t ATTN_LONG = 0, ATTN_SHORT = 1, ATTN_MIDDLE = 2;
-bool attn_gqa4_eligible(const AttnLaunch &a);
 size_t attn_scratch_bytes(const ib_attn_params &p, uint32_t max_splits);
 uint32_t attn_max_splits(const ib_ctx *ctx, const ib_attn_params &p);
 int32_t launch_attention(ib_ctx *ctx, cudaStream_t s, const AttnLaunch &a);

@@ -549,8 +549,8 @@ int32_t ib_llama_create(ib_ctx *ctx, const ib_llama_config *config, const ib_lla
     ib_attn_params ap{c.max_position_embeddings, m->kv_dim_l, c.num_attention_heads / c.num_key_value_heads, m->n_heads_l, m->head_size, 0};
     m->attn_splits = attn_max_splits(ctx, ap);
     CU(cudaMalloc(&m->attn_scratch, attn_scratch_bytes(ap, m->attn_splits)));
-    CU(cudaMalloc(&m->attn_counters, sizeof(unsigned int) * m->n_kv_l));
-    CU(cudaMemset(m->attn_counters, 0, sizeof(unsigned int) * m->n_kv_l));
+    CU(cudaMalloc(&m->attn_counters, sizeof(unsigned int) * 2 * m->n_kv_l));
+    CU(cudaMemset(m->attn_counters, 0, sizeof(unsigned int) * 2 * m->n_kv_l));
     CU(cudaMalloc(&m->argmax_slots, sizeof(unsigned long long) * (size_t)ctx->sm_count * 2));
     CU(cudaMalloc(&m->argmax_counter, sizeof(unsigned int)));
     CU(cudaMemset(m->argmax_counter, 0, sizeof(unsigned int)));

@@ -118,6 +118,36 @@ def test_attention_slice_shapes(backend, hs, n_kv, total):
     test_attention(backend, np.float16, hs, 4 * n_kv, 4, total - 1, total + 3)
 
 
+# the other groups of heads and the f32 cache: a warp step's rows and one more, both sides of the end of the cluster regime, many heads (smaller clusters,
+# or none that pay), long contexts
+@pytest.mark.parametrize("kv_dtype", [np.float16, np.float32])
+@pytest.mark.parametrize("hs", [64, 128])
+@pytest.mark.parametrize("mul,n_heads,total", [(1, 1, 1), (1, 8, 32), (1, 8, 33), (1, 16, 512), (1, 16, 513), (1, 40, 300), (1, 64, 129), (2, 2, 5), (2, 16, 511), (2, 16, 1025), (2, 8, 5000),
+                                               (8, 8, 9), (8, 32, 260), (8, 64, 512), (8, 64, 513), (8, 64, 2401), (8, 32, 6401), (4, 32, 512), (4, 32, 514), (4, 4, 7000)])
+def test_attention_groups_of_heads(backend, kv_dtype, hs, mul, n_heads, total):
+    test_attention(backend, kv_dtype, hs, n_heads, mul, total - 1, total + 3)
+
+
+@pytest.mark.parametrize("kv_dtype", [torch.float16, torch.float32])
+@pytest.mark.parametrize("mul,total", [(4, 40), (4, 900), (4, 6000), (1, 700), (2, 90), (8, 3000)])
+def test_attention_vectors_off_the_16_byte_boundary(backend, kv_dtype, mul, total):
+    """q and the output of a caller may start at any float.  (Other slices than from aligned ones: sums in another order, a few 2^-24 of values near 1.)"""
+    hs, n_kv = 64, 2
+    g = torch.Generator(device="cuda").manual_seed(total)
+    kc, vc = (torch.randn(total, n_kv * hs, device="cuda", generator=g).to(kv_dtype) for _ in range(2))
+    q = torch.randn(mul * n_kv * hs, device="cuda", generator=g)
+    p, op = AttnParams(total, n_kv * hs, mul, mul * n_kv, hs, total - 1), FusedAttention(backend)
+    out = [torch.zeros_like(q)]
+    op.launch(p, q, kc, vc, out[0])
+    for dq, do in ((1, 0), (0, 1), (3, 2)):
+        odd_q, odd_o = torch.zeros(q.numel() + 4, device="cuda")[dq:dq + q.numel()], torch.zeros(q.numel() + 4, device="cuda")[do:do + q.numel()]
+        odd_q.copy_(q)
+        op.launch(p, odd_q, kc, vc, odd_o)
+        out.append(odd_o)
+    for o in out[1:]:
+        assert_close(o.cpu().numpy(), out[0].cpu().numpy(), rtol=1e-5, what=f"off the boundary, {total} positions")
+
+
 @pytest.mark.parametrize("dtype,mul", [(torch.float16, 4), (torch.float16, 2), (torch.float32, 4)])
 def test_caches_off_the_vector_boundary_are_refused(backend, dtype, mul):
     p, op = AttnParams(8, 128, mul, 2 * mul, 64, 5), FusedAttention(backend)
@@ -197,7 +227,8 @@ def test_attention_contract(backend):
         FusedAttention(backend).launch(AttnParams(16, 64, 1, 1, 64, 3), z, kc, kc.half(), torch.zeros(64, device="cuda"))
 
 
-@pytest.mark.parametrize("qt,rows,cols,norm", [(quant.Q4_K, 1024, 2048, True), (quant.Q4_K, 14336, 4096, True), (quant.Q6_K, 512, 4096, False), (quant.Q8_0, 256, 1024, True)])
+@pytest.mark.parametrize("qt,rows,cols,norm", [(quant.Q4_K, 1024, 2048, True), (quant.Q4_K, 14336, 4096, True), (quant.Q6_K, 512, 4096, False), (quant.Q8_0, 256, 1024, True),
+                                              (quant.Q4_K, 444, 14336, True), (quant.Q6_K, 64, 10240, False)])
 def test_ffn_gate_up_is_norm_two_gemvs_and_silu(backend, qt, rows, cols, norm):
     """`ib_ffn_gate_up` against the op sequence it replaces (transformer.rs:454-464): rms_norm, two quantized GEMVs, silu."""
     from inferi_b200.ops import FfnGateUp, GpuQuantTensor
