@@ -3,6 +3,7 @@
 // The token loop runs on the streaming kernel (gemv_stream.cu).  This file holds
 //  * gemv_wide_kernel: direct 128-bit global loads, one warp per row pair, activations in shared memory; used for
 //    matrices too wide for the streaming kernel's register-resident activations (16384 < cols <= 32768);
+//  * gemv_legacy_kernel: Q4_0, Q4_1, Q5_0, Q5_1;
 //  * gemv_generic_kernel: any shape the contracts allow, straight from the GGUF byte stream with scalar loads; used
 //    where the alignment rules of the 128-bit kernels fail (for instance Q6_K with cols % 2048 != 0);
 //  * the upload-time re-tiling of Q8_0 / Q6_K rows into groups of 8 blocks, and the launch dispatch.
@@ -413,19 +414,6 @@ __device__ float generic_block_dot(int qtype, const uint8_t *b, const float *__r
                 acc += (d2 * (float)hi - m2) * v[64 * c + 32 + l];
             }
         }
-    } else if (qtype == IB_Q4_0 || qtype == IB_Q4_1 || qtype == IB_Q5_0 || qtype == IB_Q5_1) {
-        // crates/inferi/src/quantization.rs:68-82, 96-111, 125-142, 157-175: 32 elements, low nibbles first, optional
-        // minimum (the _1 types) and fifth bit (the Q5 types)
-        const bool has_m = qtype == IB_Q4_1 || qtype == IB_Q5_1, five = qtype == IB_Q5_0 || qtype == IB_Q5_1;
-        const float d = ld_h(b), m = has_m ? ld_h(b + 2) : 0.f;
-        const uint8_t *qhp = b + (has_m ? 4 : 2), *qs = qhp + (five ? 4 : 0);
-        const uint32_t qh = five ? ((uint32_t)qhp[0] | ((uint32_t)qhp[1] << 8) | ((uint32_t)qhp[2] << 16) | ((uint32_t)qhp[3] << 24)) : 0u;
-        const int off = has_m ? 0 : (five ? 16 : 8);
-        for (int j = 0; j < 16; j++) {
-            const uint32_t x0 = (qs[j] & 0x0Fu) | (((qh >> j) << 4) & 0x10u), x1 = (uint32_t)(qs[j] >> 4) | ((qh >> (j + 12)) & 0x10u);
-            acc += ((float)((int)x0 - off) * d + m) * v[j];
-            acc += ((float)((int)x1 - off) * d + m) * v[j + 16];
-        }
     } else if (qtype == IB_Q8_K) {
         // crates/inferi/src/quantization.rs:205-211: f32 scale, 256 int8 quants (the block sums are not used by the GEMV)
         float d;
@@ -469,6 +457,156 @@ __global__ void __launch_bounds__(256) gemv_generic_kernel(const uint8_t *__rest
 #pragma unroll
     for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
     if (lane == 0) out[r] = acc;
+}
+
+// -------------------------------------------------------------------------------------------------
+// The 32-element formats that the token loop does not take (Q4_0, Q4_1, Q5_0, Q5_1), straight from the GGUF byte stream, in f32.
+//
+// A warp works on 4 rows x 8 blocks at a time: four lanes per block, each with 4 bytes of its quants (8 weights: elements 4t .. 4t + 3 and 16 on), so
+// that a row's 8 blocks are read side by side and the input vector's 256 floats, two float4 per lane, serve four rows.  Blocks start at
+// any multiple of 2 bytes: 16-bit loads, through L1.  A nibble becomes a float by a byte permute (behind the exponent of 2^23 it is the float's low
+// bits) and a subtraction, both exact; the scale is applied once per lane and block.
+// What bounds it: 160 instructions per 1024 weights and the latency of the loads (issue slots 43 % busy; requesting a step ahead, or more warps: no
+// faster).  Where there are too few groups of 4 rows to fill the GPU, 2, 4 or 8 warps of a CTA share a group's columns and their sums are added in
+// order (4096 x 14336 at 8 / 16 / 32 warps per SM: 30.9 / 19.6 / 18.8 us; 4096 x 4096 10.1 / 7.4 / 7.5); and where a row has 16 steps for each of
+// them (12464 x 8448, a warp a group / four: 37.1 / 31.4 us; a row of 8 steps is better off alone, 64000 x 2048: 34.0 / 39.2).
+// Q4_0 12464 x 8448 (59 MB): 31 us; one warp per row, one block per lane and byte loads: 406.  4096 x 4096 7.2 us, 73.
+// -------------------------------------------------------------------------------------------------
+template <int QT>
+struct Legacy {
+    static constexpr bool MIN = QT == IB_Q4_1 || QT == IB_Q5_1, FIVE = QT == IB_Q5_0 || QT == IB_Q5_1;
+    static constexpr uint32_t BYTES = 18 + (MIN ? 2 : 0) + (FIVE ? 4 : 0), HIGH = MIN ? 4 : 2, QUANTS = HIGH + (FIVE ? 4 : 0);
+    static constexpr float OFFSET = MIN ? 0.f : (FIVE ? 16.f : 8.f);
+};
+constexpr uint32_t LEGACY_ROWS = 4, LEGACY_WARPS = 8, LEGACY_FILL = 16;   // warps per SM that fill it
+
+// What a lane reads of a step: of each row the two halves of its 4 bytes of quants, the scale, the minimum, and the halves of the fifth bits (elements
+// 0-15 and 16-31)
+template <int QT>
+struct LegacyStep {
+    uint32_t q[LEGACY_ROWS][2], d[LEGACY_ROWS], m[LEGACY_ROWS], h[LEGACY_ROWS][2];
+    // (no asm: the compiler then orders the loads of unrolled steps as it likes)
+    static __device__ __forceinline__ uint32_t u16_at(const uint8_t *p) { return __ldg(reinterpret_cast<const unsigned short *>(p)); }
+    __device__ __forceinline__ void load(const uint8_t *row, uint64_t row_bytes, uint32_t b, uint32_t nb, uint32_t t) {
+        using F = Legacy<QT>;
+        const uint8_t *p = row + (size_t)(b < nb ? b : nb - 1) * F::BYTES;
+#pragma unroll
+        for (uint32_t r = 0; r < LEGACY_ROWS; r++, p += row_bytes) {
+            q[r][0] = u16_at(p + F::QUANTS + 4 * t);
+            q[r][1] = u16_at(p + F::QUANTS + 4 * t + 2);
+            d[r] = u16_at(p);
+            if constexpr (F::MIN) m[r] = u16_at(p + 2);
+            if constexpr (F::FIVE) {
+                h[r][0] = u16_at(p + F::HIGH);
+                h[r][1] = u16_at(p + F::HIGH + 2);
+            }
+        }
+    }
+};
+
+// Pairs of floats, for the packed instructions
+__device__ __forceinline__ unsigned long long pair_of(float a, float b) { return (unsigned long long)__float_as_uint(a) | ((unsigned long long)__float_as_uint(b) << 32); }
+__device__ __forceinline__ float pair_sum(unsigned long long p) { return __uint_as_float((uint32_t)p) + __uint_as_float((uint32_t)(p >> 32)); }
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+// bytes 2k and 2k + 1 of w, minus `bias` - 2^23
+__device__ __forceinline__ unsigned long long byte_pair(uint32_t w, uint32_t k, float bias) {
+    const unsigned long long p = pair_of(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u + 2 * k)), __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7441u + 2 * k)));
+    unsigned long long d;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(p), "l"(pair_of(-bias, -bias)));
+    return d;
+}
+
+// ALIGNED: the vector is on a 16-byte boundary
+template <int QT, bool ALIGNED>
+__global__ void __launch_bounds__(LEGACY_WARPS * 32) gemv_legacy_kernel(const uint8_t *__restrict__ w, uint32_t rows, uint32_t nb, uint64_t row_bytes, uint32_t share,
+                                                                        const float *__restrict__ v, float *__restrict__ out) {
+    using F = Legacy<QT>;
+    __shared__ float part[LEGACY_WARPS][LEGACY_ROWS];
+    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane >> 2, t = lane & 3;
+    const uint32_t group = (blockIdx.x * LEGACY_WARPS + warp) / share, mine = warp % share, r0 = group * LEGACY_ROWS;
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+    float acc[LEGACY_ROWS] = {};
+    if (r0 < rows) {
+        const uint8_t *row = w + (size_t)r0 * row_bytes;
+#pragma unroll 2
+        for (uint32_t b = 8 * mine + j; b - j < nb; b += 8 * share) {
+            LegacyStep<QT> now;
+            now.load(row, row_bytes, b, nb, t);
+            const bool in = b < nb;   // (the last step of a row: what lies past its end counts 0)
+            const float *x = v + 32 * (in ? b : nb - 1) + 4 * t;
+            float4 a, c;
+            if constexpr (ALIGNED) {
+                a = __ldg(reinterpret_cast<const float4 *>(x));
+                c = __ldg(reinterpret_cast<const float4 *>(x + 16));
+            } else {
+                a = make_float4(__ldg(x), __ldg(x + 1), __ldg(x + 2), __ldg(x + 3));
+                c = make_float4(__ldg(x + 16), __ldg(x + 17), __ldg(x + 18), __ldg(x + 19));
+            }
+            if (!in) {
+                a = c = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (uint32_t k = 0; k < LEGACY_ROWS; k++) now.d[k] = now.m[k] = 0u;
+            }
+            const unsigned long long xl[2] = {pair_of(a.x, a.y), pair_of(a.z, a.w)}, xh[2] = {pair_of(c.x, c.y), pair_of(c.z, c.w)};
+            float sx = 0.f;
+            if constexpr (F::MIN) sx = ((a.x + a.y) + (a.z + a.w)) + ((c.x + c.y) + (c.z + c.w));
+#pragma unroll
+            for (uint32_t r = 0; r < LEGACY_ROWS; r++) {
+                const uint32_t q = __byte_perm(now.q[r][0], now.q[r][1], 0x5410u);
+                uint32_t lo = q & 0x0F0F0F0Fu, hi = (q >> 4) & 0x0F0F0F0Fu;
+                if constexpr (F::FIVE) {   // four bits into bit 4 of four bytes
+                    lo |= (((((uint32_t)now.h[r][0] >> (4 * (t & 3))) & 15u) * 0x00204081u) & 0x01010101u) << 4;
+                    hi |= (((((uint32_t)now.h[r][1] >> (4 * (t & 3))) & 15u) * 0x00204081u) & 0x01010101u) << 4;
+                }
+                unsigned long long s = 0ull;   // a pair of sums
+#pragma unroll
+                for (uint32_t k = 0; k < 2; k++) {
+                    s = fma2(byte_pair(lo, k, 8388608.0f + F::OFFSET), xl[k], s);
+                    s = fma2(byte_pair(hi, k, 8388608.0f + F::OFFSET), xh[k], s);
+                }
+                acc[r] = fmaf(h2f(now.d[r]), pair_sum(s), acc[r]);
+                if constexpr (F::MIN) acc[r] = fmaf(h2f(now.m[r]), sx, acc[r]);
+            }
+        }
+    }
+#pragma unroll
+    for (uint32_t r = 0; r < LEGACY_ROWS; r++)
+#pragma unroll
+        for (int o = 16; o; o >>= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
+    if (share > 1) {
+        if (lane < LEGACY_ROWS) part[warp][lane] = lane == 0 ? acc[0] : (lane == 1 ? acc[1] : (lane == 2 ? acc[2] : acc[3]));
+        __syncthreads();
+        if (mine != 0 || r0 >= rows || lane >= LEGACY_ROWS) return;
+        float s = 0.f;
+        for (uint32_t k = 0; k < share; k++) s += part[warp + k][lane];
+        out[r0 + lane] = s;
+    } else if (r0 < rows && lane < LEGACY_ROWS) out[r0 + lane] = lane == 0 ? acc[0] : (lane == 1 ? acc[1] : (lane == 2 ? acc[2] : acc[3]));
+}
+
+template <int QT>
+static int32_t launch_legacy(ib_ctx *ctx, cudaStream_t stream, const ib_qtensor *m, const float *v, float *out) {
+    const uint32_t groups = (uint32_t)(m->rows / LEGACY_ROWS);   // (uploads have whole groups of 4 rows)
+    const uint32_t steps = (uint32_t)((m->cols / 32 + 7) / 8);
+    uint32_t share = 1;
+    while (share < LEGACY_WARPS && (groups * share < LEGACY_FILL * (uint32_t)ctx->sm_count || steps >= 16 * share)) share *= 2;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((groups * share + LEGACY_WARPS - 1) / LEGACY_WARPS);
+    cfg.blockDim = dim3(LEGACY_WARPS * 32);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    const bool aligned = ((uintptr_t)v % 16) == 0;
+    IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, aligned ? gemv_legacy_kernel<QT, true> : gemv_legacy_kernel<QT, false>, (const uint8_t *)m->dev, (uint32_t)m->rows,
+                                     (uint32_t)(m->cols / 32), m->row_bytes, share, v, out));
+    ctx->launches++;
+    return IB_OK;
 }
 
 // -------------------------------------------------------------------------------------------------
@@ -585,6 +723,13 @@ int32_t launch_gemv(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p_in) {
 }
 
 int32_t launch_gemv_generic(ib_ctx *ctx, cudaStream_t stream, const ib_qtensor *m, const float *v, float *out) {
+    switch (m->qtype) {
+    case IB_Q4_0: return launch_legacy<IB_Q4_0>(ctx, stream, m, v, out);
+    case IB_Q4_1: return launch_legacy<IB_Q4_1>(ctx, stream, m, v, out);
+    case IB_Q5_0: return launch_legacy<IB_Q5_0>(ctx, stream, m, v, out);
+    case IB_Q5_1: return launch_legacy<IB_Q5_1>(ctx, stream, m, v, out);
+    default: break;
+    }
     const int warps = 8;
     const int grid = (int)((m->rows + warps - 1) / warps);
     gemv_generic_kernel<<<grid, warps * 32, 0, stream>>>(m->dev, m->qtype, (uint32_t)m->rows, (uint32_t)m->cols, m->row_bytes, v, out);

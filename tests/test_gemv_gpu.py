@@ -69,6 +69,20 @@ def test_legacy_formats(backend, qt, rows, cols):
     _shape_case(backend, qt, rows, cols)
 
 
+# groups of 4 rows: one warp each, and 2, 4 or 8 warps that share the columns; rows of fewer blocks than a step, of whole steps and of a part more
+# (their blocks then start at every multiple of 2 bytes); vectors off the 16-byte boundary
+@pytest.mark.parametrize("qt", LEGACY)
+@pytest.mark.parametrize("rows,cols", [(4, 32), (12, 96), (36, 224), (68, 4128), (2364, 288), (4740, 352), (9476, 64), (9480, 512)])
+def test_legacy_splits(backend, qt, rows, cols):
+    _shape_case(backend, qt, rows, cols)
+    blocks = quant.random_blocks(qt, rows, cols, seed=rows)
+    v = torch.randn(cols + 1, generator=torch.Generator().manual_seed(cols)).cuda()[1:]
+    m = GpuQuantTensor(backend, qt, rows, cols, blocks)
+    out = torch.full((rows,), float("nan"), device="cuda")
+    GemvQuant(backend).launch(out, m, v)
+    assert_close(out.cpu().numpy(), oracle.gemv_ref(qt, rows, cols, blocks, v.cpu().numpy()), what=f"{quant.NAMES[qt]} {rows}x{cols}")
+
+
 def _shape_case(backend, qt, rows, cols):
     blocks = quant.random_blocks(qt, rows, cols, seed=rows * 31 + cols + qt, scale=1.0, subnormal_frac=0.25)
     v = np.random.default_rng(cols).standard_normal(cols).astype(np.float32)
