@@ -849,15 +849,23 @@ int32_t ib_llama_prefill(ib_llama *m, void *stream, const uint32_t *tokens_host,
     auto gemm = [&](const ib_qtensor *const *mats, uint32_t count, uint32_t nc, PfPlanes *g, uint32_t *row0) -> int32_t {
         PrefillGroup groups[3];
         const uint32_t ng = prefill_groups(mats, count, groups);
+        const bool mixed = ng == 2 && prefill_mixable(groups[0].mats[0], groups[1].mats[0], nc);
+        StreamK sk[3];
+        for (uint32_t i = 0; i < ng; i++) sk[i] = prefill_streamk(ctx, groups[i].rows, groups[i].cols, nc);
+        if (mixed) prefill_streamk_mixed(ctx, groups[0].rows, groups[1].rows, groups[0].cols, nc, sk[0], sk[1]);
+        PrefillPart parts[3];
         float *at = B.planes;
         for (uint32_t i = 0, k = 0; i < ng; i++) {
             const PrefillGroup &p = groups[i];
-            const StreamK sk = prefill_streamk(ctx, p.rows, p.cols, nc);
-            const PfPlanes pl{at, at + (size_t)nc * p.rows, sk, p.rows, (nc + PF_CHUNK - 1) / PF_CHUNK, nc};
-            const int32_t r = launch_prefill_gemm(ctx, s, p.mats, p.n_mats, B.xt, nc, at, at + (size_t)nc * p.rows, sk);
-            if (r) return r;
+            const PfPlanes pl{at, at + (size_t)nc * p.rows, sk[i], p.rows, (nc + PF_CHUNK - 1) / PF_CHUNK, nc};
+            parts[i] = PrefillPart{p.mats, p.n_mats, at, at + (size_t)nc * p.rows, sk[i]};
             for (uint32_t j = 0, row = 0; j < p.n_mats; row += (uint32_t)p.mats[j]->rows, j++, k++) { g[k] = pl; row0[k] = row; }
             at += prefill_plane_floats(ctx, p, nc);
+        }
+        if (mixed) return launch_prefill_gemm_mixed(ctx, s, parts[0], parts[1], B.xt, nc);
+        for (uint32_t i = 0; i < ng; i++) {
+            const int32_t r = launch_prefill_gemm(ctx, s, parts[i], B.xt, nc);
+            if (r) return r;
         }
         return IB_OK;
     };

@@ -323,7 +323,7 @@ extern "C" int32_t ib_gemm_quant(ib_ctx *ctx, void *stream, float *out_dev, cons
         const StreamK sk = prefill_streamk(ctx, rows, cols, nc);
         float *out = out_dev + (size_t)t0 * rows;   // plane 0 of every tile
         rc = launch_prefill_norm_split(ctx, s, const_cast<float *>(x_dev) + (size_t)t0 * cols, nullptr, nullptr, 0.f, nc, cols, xt);
-        if (rc == IB_OK) rc = launch_prefill_gemm(ctx, s, &w, 1, xt, nc, out, planes, sk, !retile);
+        if (rc == IB_OK) rc = launch_prefill_gemm(ctx, s, PrefillPart{&w, 1, out, planes, sk}, xt, nc, !retile);
         if (rc == IB_OK && prefill_max_pieces(sk) > 1) rc = launch_prefill_finish(ctx, s, out, PfPlanes{out, planes, sk, rows, (nc + PF_CHUNK - 1) / PF_CHUNK, nc});
     }
     if (prev >= 0 && prev != ctx->device) cudaSetDevice(prev);

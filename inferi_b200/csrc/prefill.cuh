@@ -30,6 +30,8 @@ struct StreamK {
     __host__ __device__ uint32_t row_tile(uint32_t row) const { return row >> row_log2; }
 };
 StreamK prefill_streamk(const ib_ctx *ctx, uint32_t rows, uint32_t cols, uint32_t n);
+// a launch that two groups of rows of different formats share: the split of each.  (Never more pieces per tile than as launches of their own.)
+void prefill_streamk_mixed(const ib_ctx *ctx, uint32_t rows_a, uint32_t rows_b, uint32_t cols, uint32_t n, StreamK &a, StreamK &b);
 uint32_t prefill_max_pieces(const StreamK &sk);   // bound of the planes that any tile needs
 
 struct PgParams {
@@ -63,10 +65,20 @@ __host__ __device__ inline uint32_t pf_s_index(uint32_t t, uint32_t sb, uint32_t
 __host__ __device__ inline size_t pf_x_halves(uint32_t cols) { return (size_t)2 * (PF_CHUNK + 8) * cols; }   // halves per chunk
 
 bool prefill_gemm_eligible(const ib_qtensor *m);
-// plane0 / planes = partial sums of W x_t over the tile's K ranges; x: the layout above, token rows n .. (n rounded
-// up to 16) - 1 of the last chunk zero; early: the weights may be read before the stream's previous kernels are done.  The matrices of a launch have the same type and width; their rows follow one another.
-int32_t launch_prefill_gemm(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *const *mats, uint32_t n_mats, const __half *x, uint32_t n, float *plane0,
-                            float *planes, const StreamK &sk, bool early = true);
+// What one format's matrices of a GEMM launch are and give: plane0 / planes = partial sums of W x_t over the tile's K ranges.  The matrices have the
+// same type and width; their rows follow one another.
+struct PrefillPart {
+    const ib_qtensor *const *mats;
+    uint32_t n_mats;
+    float *plane0, *planes;
+    StreamK sk;
+};
+// x: the layout above, token rows n .. (n rounded up to 16) - 1 of the last chunk zero; early: the weights may be read before the stream's previous
+// kernels are done
+int32_t launch_prefill_gemm(ib_ctx *ctx, cudaStream_t s, const PrefillPart &w, const __half *x, uint32_t n, bool early = true);
+// two formats with the same inputs in one launch: Q4_K or Q5_K, and Q6_K, where that is the faster way for n tokens
+bool prefill_mixable(const ib_qtensor *a, const ib_qtensor *b, uint32_t n);
+int32_t launch_prefill_gemm_mixed(ib_ctx *ctx, cudaStream_t s, const PrefillPart &a, const PrefillPart &b, const __half *x, uint32_t n);
 
 // One GEMM launch's result, as the element-wise kernels read it
 struct PfPlanes {

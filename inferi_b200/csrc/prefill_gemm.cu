@@ -336,8 +336,9 @@ struct PgCursor {
 };
 __device__ __forceinline__ uint32_t pg_pad(uint32_t n) { return (n + 15) & ~15u; }
 
+// One CTA's work, number `cta` of the launch's CTAs of this format
 template <int FMT, bool PAIR>
-__global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __grid_constant__ PgParams p, const __grid_constant__ PgMaps maps) {
+__device__ __forceinline__ void pg_gemm(const PgParams &p, const PgMaps &maps, const uint32_t cta) {
     constexpr bool MIN = pg_has_min(FMT), SCALED = FMT != PG_Q80;   // (Q8_0's operands carry their scales)
     constexpr uint32_t CTAS = PAIR ? 2 : 1;
     constexpr uint32_t NS = pg_slots(FMT), R = pg_raw_stages(FMT), RAW = pg_raw_bytes(FMT), A0 = MIN ? PG_A4 : PG_A6, ACOLS = MIN ? 32 : 64;
@@ -357,7 +358,7 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
     const uint32_t b_zdone = take(1), b_zfree = take(1), s_tmem = nb;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const StreamK sk = p.sk;
-    const uint32_t range = PAIR ? blockIdx.x >> 1 : blockIdx.x, rank = PAIR ? blockIdx.x & 1 : 0;   // pairs: clusters of two CTAs along x
+    const uint32_t range = PAIR ? cta >> 1 : cta, rank = PAIR ? cta & 1 : 0;   // pairs: clusters of two CTAs along x
     const uint32_t u0 = sk.first_unit(range), nunits = sk.first_unit(range + 1) - u0;
 
     asm volatile("griddepcontrol.launch_dependents;");
@@ -727,9 +728,30 @@ __global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __gri
     if (warp == PG_W_MMA) pg_dealloc<PAIR>(tmem);
 }
 
+template <int FMT, bool PAIR>
+__global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_kernel(const __grid_constant__ PgParams p, const __grid_constant__ PgMaps maps) {
+    pg_gemm<FMT, PAIR>(p, maps, blockIdx.x);
+}
+// Matrices of two formats with the same inputs (q and k beside v in most files): the first CTAs take the one, the others the other, each its
+// format's path.  As a launch of its own v's few tiles took a start and an end of a GEMM, and were cut into so many pieces that adding them up was
+// most of the kernel behind it.
+template <int A, int B, bool PAIR>
+__global__ void __launch_bounds__(PG_THREADS, 1) prefill_gemm_mixed_kernel(const __grid_constant__ PgParams pa, const __grid_constant__ PgMaps ma,
+                                                                           const __grid_constant__ PgParams pb, const __grid_constant__ PgMaps mb) {
+    const uint32_t first = (PAIR ? 2 : 1) * pa.sk.ranges;
+    if (blockIdx.x < first) pg_gemm<A, PAIR>(pa, ma, blockIdx.x);
+    else pg_gemm<B, PAIR>(pb, mb, blockIdx.x - first);
+}
+
 // ---------------------------------------------------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------------------------------------------------
+static uint32_t pg_units(uint32_t rows, uint32_t nb, uint32_t n, bool pair) {
+    const uint32_t tile = pair ? 256 : 128;
+    return (rows + tile - 1) / tile * ((n + PF_CHUNK - 1) / PF_CHUNK) * nb;
+}
+static uint32_t pg_most(const ib_ctx *ctx, bool pair) { return pair ? (ctx->sm_count >= 2 ? (uint32_t)ctx->sm_count / 2 : 1u) : (uint32_t)ctx->sm_count; }
+
 StreamK prefill_streamk(const ib_ctx *ctx, uint32_t rows, uint32_t cols, uint32_t n) {
     StreamK sk;
     sk.nb = cols / 256;
@@ -739,10 +761,30 @@ StreamK prefill_streamk(const ib_ctx *ctx, uint32_t rows, uint32_t cols, uint32_
     // 12.0).  Beyond, pairs are the faster ones or equal (4096 x 4096, 40 tokens 20.4 / 19.3).
     const bool pair = n > PF_SINGLE_TOKENS || (n > PF_SINGLE_ALWAYS && (rows >> 7) * sk.nb > (uint32_t)ctx->sm_count);
     sk.row_log2 = pair ? 8 : 7;
-    sk.total = ((rows + (1u << sk.row_log2) - 1) >> sk.row_log2) * ((n + PF_CHUNK - 1) / PF_CHUNK) * sk.nb;
-    const uint32_t most = pair ? (ctx->sm_count >= 2 ? (uint32_t)ctx->sm_count / 2 : 1u) : (uint32_t)ctx->sm_count;
+    sk.total = pg_units(rows, sk.nb, n, pair);
+    const uint32_t most = pg_most(ctx, pair);
     sk.ranges = sk.total < most ? sk.total : most;
     return sk;
+}
+// The same for a launch of two groups of rows of different formats: the ranges are dealt out so that the slower group ends as early as it can.  A
+// unit of Q6_K (three products a weight) takes 3100 clocks, of Q4_K or Q5_K 2490.
+void prefill_streamk_mixed(const ib_ctx *ctx, uint32_t rows_a, uint32_t rows_b, uint32_t cols, uint32_t n, StreamK &a, StreamK &b) {
+    const StreamK all = prefill_streamk(ctx, rows_a + rows_b, cols, n);   // (one SM or two per tile)
+    const bool pair = all.row_log2 == 8;
+    a = b = all;
+    a.total = pg_units(rows_a, all.nb, n, pair);
+    b.total = pg_units(rows_b, all.nb, n, pair);
+    const uint32_t most = pg_most(ctx, pair);
+    uint32_t best = 0xFFFFFFFFu;
+    for (uint32_t r = 1; r < most; r++) {
+        const uint32_t ra = r < a.total ? r : a.total, rb = most - r < b.total ? most - r : b.total;
+        const uint32_t ta = (a.total + ra - 1) / ra * 249, tb = (b.total + rb - 1) / rb * 310, t = ta > tb ? ta : tb;
+        if (t < best) {
+            best = t;
+            a.ranges = ra;
+            b.ranges = rb;
+        }
+    }
 }
 // Most planes a tile needs: a range of `len` units cut into pieces of at least floor(total / ranges) units each
 uint32_t prefill_max_pieces(const StreamK &sk) {
@@ -793,20 +835,24 @@ static int32_t pg_encode(const ib_qtensor *m, int fmt, CUtensorMap *maps) {
     return IB_OK;
 }
 
+// The inputs' ring of a launch; returns the shared memory that it takes
 template <int FMT, bool PAIR>
-static int32_t pg_launch(ib_ctx *ctx, cudaStream_t s, PgParams &p, const PgMaps &maps, bool early) {
-    static bool attr_set[16] = {};
+static uint32_t pg_ring(PgParams &p) {
     constexpr uint32_t room = PG_SMEM_LIMIT - pg_fixed_smem(FMT);
     static_assert(room >= 3 * (PAIR ? PF_CHUNK / 2 : PF_SINGLE_TOKENS) * 256, "shared memory");
     p.x_tile = ((p.n < PF_CHUNK ? p.n : PF_CHUNK) + 15) / 16 * (PAIR ? 8 : 16) * 128;   // 64 columns of a CTA's (padded) tokens of a chunk
     p.x_stages = room / (2 * p.x_tile) < PG_XSTAGES_MAX ? room / (2 * p.x_tile) : PG_XSTAGES_MAX;
-    const uint32_t smem = pg_fixed_smem(FMT) + p.x_stages * 2 * p.x_tile;
-    if (!attr_set[ctx->device & 15]) {
-        IB_CHECK_CUDA(cudaFuncSetAttribute(prefill_gemm_kernel<FMT, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PG_SMEM_LIMIT));
-        attr_set[ctx->device & 15] = true;
+    return pg_fixed_smem(FMT) + p.x_stages * 2 * p.x_tile;
+}
+
+template <bool PAIR, typename... KArgs, typename... Args>
+static int32_t pg_launch_kernel(ib_ctx *ctx, cudaStream_t s, void (*kernel)(KArgs...), bool &attr_set, uint32_t ranges, uint32_t smem, bool early, const Args &...args) {
+    if (!attr_set) {
+        IB_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PG_SMEM_LIMIT));
+        attr_set = true;
     }
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((PAIR ? 2 : 1) * p.sk.ranges);
+    cfg.gridDim = dim3((PAIR ? 2 : 1) * ranges);
     cfg.blockDim = dim3(PG_THREADS);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
@@ -823,9 +869,16 @@ static int32_t pg_launch(ib_ctx *ctx, cudaStream_t s, PgParams &p, const PgMaps 
         attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
         cfg.numAttrs++;
     }
-    IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, prefill_gemm_kernel<FMT, PAIR>, p, maps));
+    IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
     ctx->launches++;
     return IB_OK;
+}
+
+template <int FMT, bool PAIR>
+static int32_t pg_launch(ib_ctx *ctx, cudaStream_t s, PgParams &p, const PgMaps &maps, bool early) {
+    static bool attr_set[16] = {};
+    const uint32_t smem = pg_ring<FMT, PAIR>(p);
+    return pg_launch_kernel<PAIR>(ctx, s, prefill_gemm_kernel<FMT, PAIR>, attr_set[ctx->device & 15], p.sk.ranges, smem, early, p, maps);
 }
 
 template <int FMT>
@@ -833,34 +886,67 @@ static int32_t pg_launch_rows(ib_ctx *ctx, cudaStream_t s, PgParams &p, const Pg
     return p.sk.row_log2 == 8 ? pg_launch<FMT, true>(ctx, s, p, maps, early) : pg_launch<FMT, false>(ctx, s, p, maps, early);
 }
 
-int32_t launch_prefill_gemm(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *const *mats, uint32_t n_mats, const __half *x, uint32_t n, float *plane0,
-                            float *planes, const StreamK &sk, bool early) {
-    IB_REQUIRE(n_mats >= 1 && n_mats <= PF_MAX_SEGS, "prefill GEMM: %u matrices", n_mats);
-    IB_REQUIRE(sk.total < (1u << 24), "prefill GEMM: %u units of work are too many for one launch", sk.total);
+template <int A, bool PAIR>
+static int32_t pg_launch_mixed(ib_ctx *ctx, cudaStream_t s, PgParams &pa, const PgMaps &ma, PgParams &pb, const PgMaps &mb) {
+    static bool attr_set[16] = {};
+    const uint32_t sa = pg_ring<A, PAIR>(pa), sb = pg_ring<PG_Q6K, PAIR>(pb);
+    return pg_launch_kernel<PAIR>(ctx, s, prefill_gemm_mixed_kernel<A, PG_Q6K, PAIR>, attr_set[ctx->device & 15], pa.sk.ranges + pb.sk.ranges, sa > sb ? sa : sb, true, pa, ma, pb, mb);
+}
+
+// What a launch (or its part of one format) is told
+static int32_t pg_describe(const ib_ctx *ctx, const PrefillPart &w, const __half *x, uint32_t n, PgParams &p, PgMaps &maps) {
+    IB_REQUIRE(w.n_mats >= 1 && w.n_mats <= PF_MAX_SEGS, "prefill GEMM: %u matrices", w.n_mats);
+    IB_REQUIRE(w.sk.total < (1u << 24), "prefill GEMM: %u units of work are too many for one launch", w.sk.total);
     IB_REQUIRE(((uintptr_t)x % 16) == 0, "prefill GEMM: the input tiles must be 16-byte aligned for the bulk copies");
-    const int fmt = pg_format(mats[0]);
-    PgParams p = {};
-    PgMaps maps;
+    const int fmt = pg_format(w.mats[0]);
+    p = PgParams{};
     uint32_t tiles = 0;
     for (uint32_t i = 0; i < PF_MAX_SEGS; i++) {
-        p.tile0[i] = i < n_mats ? tiles : 0xFFFFFFFFu;
-        if (i >= n_mats) continue;
-        const ib_qtensor *m = mats[i];
-        IB_REQUIRE(pg_format(m) == fmt && m->cols == mats[0]->cols, "prefill GEMM: the matrices of a launch differ in type or width");
+        p.tile0[i] = i < w.n_mats ? tiles : 0xFFFFFFFFu;
+        if (i >= w.n_mats) continue;
+        const ib_qtensor *m = w.mats[i];
+        IB_REQUIRE(pg_format(m) == fmt && m->cols == w.mats[0]->cols, "prefill GEMM: the matrices of a launch differ in type or width");
         const int32_t rc = pg_encode(m, fmt, maps.m[i]);
         if (rc) return rc;
         tiles += (uint32_t)m->rows / 128;
     }
     p.rows = tiles * 128;
-    p.n = n; p.chunks = (n + PF_CHUNK - 1) / PF_CHUNK; p.x = x; p.x_chunk = pf_x_halves((uint32_t)mats[0]->cols);
-    p.plane0 = plane0; p.planes = planes; p.sk = sk; p.err = ctx->err_dev; p.wait_ns = ctx->wait_limit_ns;
-    switch (fmt) {
+    p.n = n; p.chunks = (n + PF_CHUNK - 1) / PF_CHUNK; p.x = x; p.x_chunk = pf_x_halves((uint32_t)w.mats[0]->cols);
+    p.plane0 = w.plane0; p.planes = w.planes; p.sk = w.sk; p.err = ctx->err_dev; p.wait_ns = ctx->wait_limit_ns;
+    return IB_OK;
+}
+
+int32_t launch_prefill_gemm(ib_ctx *ctx, cudaStream_t s, const PrefillPart &w, const __half *x, uint32_t n, bool early) {
+    PgParams p;
+    PgMaps maps;
+    const int32_t rc = pg_describe(ctx, w, x, n, p, maps);
+    if (rc) return rc;
+    switch (pg_format(w.mats[0])) {
     case PG_Q4K: return pg_launch_rows<PG_Q4K>(ctx, s, p, maps, early);
     case PG_Q5K: return pg_launch_rows<PG_Q5K>(ctx, s, p, maps, early);
     case PG_Q6K: return pg_launch_rows<PG_Q6K>(ctx, s, p, maps, early);
     case PG_Q80: return pg_launch_rows<PG_Q80>(ctx, s, p, maps, early);
-    default: return set_error(IB_ERR_UNSUPPORTED, "prefill GEMM: a matrix of type %d", mats[0]->qtype);
+    default: return set_error(IB_ERR_UNSUPPORTED, "prefill GEMM: a matrix of type %d", w.mats[0]->qtype);
     }
+}
+
+// Longer passes have v enough to do by itself.  A layer, us, two launches / one: 2048 hidden (q4_k and q6_k), 30 tokens 84.2 / 78.4, 128 99.7 / 96.4, 256
+// 132.6 / 128.8, 300 152.1 / 152.9, 384 162.9 / 163.5; 4096 hidden 30 tokens 139.7 / 129.9, 128 168.2 / 166.8, 300 334.5 / 326.2, 384 369.2 / 365.7, 500
+// 471.0 / 470.4.
+bool prefill_mixable(const ib_qtensor *a, const ib_qtensor *b, uint32_t n) {
+    const int fa = pg_format(a);
+    return (fa == PG_Q4K || fa == PG_Q5K) && pg_format(b) == PG_Q6K && a->cols == b->cols && n <= (a->cols >= 4096 ? 3 : 2) * PF_CHUNK;
+}
+int32_t launch_prefill_gemm_mixed(ib_ctx *ctx, cudaStream_t s, const PrefillPart &a, const PrefillPart &b, const __half *x, uint32_t n) {
+    IB_REQUIRE(prefill_mixable(a.mats[0], b.mats[0], n) && a.sk.row_log2 == b.sk.row_log2, "prefill GEMM: these matrices cannot share a launch");
+    PgParams pa, pb;
+    PgMaps ma, mb;
+    int32_t rc = pg_describe(ctx, a, x, n, pa, ma);
+    if (rc == IB_OK) rc = pg_describe(ctx, b, x, n, pb, mb);
+    if (rc) return rc;
+    const bool pair = a.sk.row_log2 == 8;
+    if (pg_format(a.mats[0]) == PG_Q4K) return pair ? pg_launch_mixed<PG_Q4K, true>(ctx, s, pa, ma, pb, mb) : pg_launch_mixed<PG_Q4K, false>(ctx, s, pa, ma, pb, mb);
+    return pair ? pg_launch_mixed<PG_Q5K, true>(ctx, s, pa, ma, pb, mb) : pg_launch_mixed<PG_Q5K, false>(ctx, s, pa, ma, pb, mb);
 }
 
 }  // namespace ib

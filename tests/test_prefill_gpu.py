@@ -74,6 +74,17 @@ def test_long_prompt_goes_in_chunks_and_matches_the_oracle(backend):
     dev_w.close()
 
 
+# q, k (Q4_K or Q5_K) and v (Q6_K) in one GEMM launch, and beyond two chunks of tokens in two: one SM per tile and pairs, a partial and a second chunk
+@pytest.mark.parametrize("qk,heads", [(quant.Q4_K, 32), (quant.Q5_K, 16)])
+def test_formats_that_share_a_launch(backend, qk, heads):
+    cfg = Llama2Config(2048, 2048, 2, heads, heads // 4, 512, 512, 500000.0, 1e-5)
+    w = synth_weights(cfg, seed=31, device="cuda", recipe=dict(Q4_K_M, attn_q=qk, attn_k=qk, token_embd=quant.Q4_K))
+    dev_w = Llama2Weights(backend, cfg, w)
+    for n in (1, 9, 16, 17, 64, 65, 128, 129, 256, 257, 400):
+        loop_vs_prefill(backend, cfg, dev_w, np.random.default_rng(n).integers(0, cfg.vocab_size, n).tolist(), 3)
+    dev_w.close()
+
+
 @pytest.mark.parametrize("hidden,heads,n,start", [(512, 8, 17, 0), (512, 8, 1, 300), (512, 4, 65, 0), (512, 4, 15, 470), (512, 8, 200, 130)])
 def test_prompt_attention_at_the_edges_of_its_tiles(backend, hidden, heads, n, start):
     """16-token and 64-position tiles with remainders, positions divided between the CTAs of a cluster (few tokens far into the
