@@ -40,29 +40,32 @@ __global__ void prefill_embed_kernel(QDesc embd, const uint32_t *tokens, uint32_
     }
 }
 
-// One CTA per token row: X += the planes of the GEMM before (where there is one), then y = (X * rsqrt(mean(X^2) + eps)) * w
-// (crates/inferi-shaders/src/rms_norm.rs:112-120; `w` null: y = X) as the next GEMM's inputs.  The row stays in registers
+// X += the planes of the GEMM before (where there is one), then y = (X * rsqrt(mean(X^2) + eps)) * w
+// (crates/inferi-shaders/src/rms_norm.rs:112-120; `w` null: y = X) as the next GEMM's inputs.  TOK tokens per CTA, a warp's lanes shared out to them: the
+// inputs' layout holds 8 tokens' 8 columns side by side, and a warp of one token writes 16 bytes of every 128.  The row stays in registers
 // between the two (PF_KEEP * 8 columns per thread).  Rows n .. n rounded up to 16 are zero-filled.
 constexpr int PF_ROW_THREADS = 512, PF_KEEP = 4;
+constexpr uint32_t PF_FOUR_TOKENS = 512;   // tokens from which four share a CTA
+template <int TOK>
 __global__ void __launch_bounds__(PF_ROW_THREADS) prefill_norm_split_kernel(float *X, const PfPlanes add, uint32_t has_add, const float *w, float eps, uint32_t n, uint32_t cols,
                                                                             __half *xt) {
-    __shared__ float red[PF_ROW_THREADS / 32];
-    const uint32_t t = blockIdx.x, tid = threadIdx.x;
-    constexpr uint32_t STEP = PF_ROW_THREADS * 8;
+    constexpr uint32_t LANES = 32 / TOK, STEP = PF_ROW_THREADS / TOK * 8, WARPS = PF_ROW_THREADS / 32;
+    __shared__ float red[WARPS][TOK];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, which = lane / LANES, t = blockIdx.x * TOK + which;
+    const uint32_t c0 = (warp * LANES + lane % LANES) * 8;   // cols % 256 == 0: whole warps
+    const bool there = t < n;
     pf_enter();
-    if (t >= n) {
-        const F8 zero = {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}};
-        for (uint32_t c = tid * 8; c < cols; c += STEP) pf_emit8(xt, t, c, cols, zero);   // cols % 256 == 0: whole warps
-        return;
-    }
     float *x = X + (size_t)t * cols;
     F8 keep[PF_KEEP];
     float ss = 0.f;
     auto fetch = [&](uint32_t c) {
-        F8 v = pf_load8u(x + c);
-        if (has_add) {
-            pf_add8(v, pf_sum8(add, t, c));
-            pf_store8(x + c, v);
+        F8 v = {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}};
+        if (there) {
+            v = pf_load8u(x + c);
+            if (has_add) {
+                pf_add8(v, pf_sum8(add, t, c));
+                pf_store8(x + c, v);
+            }
         }
 #pragma unroll
         for (int i = 0; i < 8; i++) ss += v.v[i] * v.v[i];
@@ -70,19 +73,19 @@ __global__ void __launch_bounds__(PF_ROW_THREADS) prefill_norm_split_kernel(floa
     };
 #pragma unroll
     for (int k = 0; k < PF_KEEP; k++) {
-        const uint32_t c = tid * 8 + k * STEP;
+        const uint32_t c = c0 + k * STEP;
         if (c < cols) keep[k] = fetch(c);
     }
-    for (uint32_t c = tid * 8 + PF_KEEP * STEP; c < cols; c += STEP) fetch(c);
+    for (uint32_t c = c0 + PF_KEEP * STEP; c < cols; c += STEP) fetch(c);
     float rms = 1.0f;
     if (w) {
 #pragma unroll
-        for (int o = 16; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if ((tid & 31) == 0) red[tid >> 5] = ss;
+        for (uint32_t o = LANES / 2; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+        if (lane % LANES == 0) red[warp][which] = ss;
         __syncthreads();
         float tot = 0.f;
 #pragma unroll
-        for (int i = 0; i < PF_ROW_THREADS / 32; i++) tot += red[i];
+        for (uint32_t i = 0; i < WARPS; i++) tot += red[i][which];
         rms = 1.0f / sqrtf(tot / (float)cols + eps);
     }
     auto emit = [&](uint32_t c, F8 v) {
@@ -95,10 +98,11 @@ __global__ void __launch_bounds__(PF_ROW_THREADS) prefill_norm_split_kernel(floa
     };
 #pragma unroll
     for (int k = 0; k < PF_KEEP; k++) {
-        const uint32_t c = tid * 8 + k * STEP;
+        const uint32_t c = c0 + k * STEP;
         if (c < cols) emit(c, keep[k]);
     }
-    for (uint32_t c = tid * 8 + PF_KEEP * STEP; c < cols; c += STEP) emit(c, pf_load8u(x + c));
+    const F8 zero = {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}};
+    for (uint32_t c = c0 + PF_KEEP * STEP; c < cols; c += STEP) emit(c, there ? pf_load8u(x + c) : zero);
 }
 
 __global__ void __launch_bounds__(256) prefill_residual_kernel(float *X, const PfPlanes add) {
@@ -146,10 +150,11 @@ __global__ void __launch_bounds__(256) prefill_finish_narrow_kernel(float *out, 
     out[i] = v;
 }
 
+// A warp: 8 tokens x 32 columns, which are whole lines of the next GEMM's inputs (a warp of one token's 256 columns writes 16 bytes of each of 32 lines)
 __global__ void __launch_bounds__(256) prefill_swiglu_kernel(const PfPlanes gu, __half *xt) {
     pf_enter();
-    const uint32_t F = gu.rows / 2, per = F / 8, i = blockIdx.x * blockDim.x + threadIdx.x, t = i / per, c = (i - t * per) * 8;   // whole warps: F % 256 == 0
-    if (t >= ((gu.n + 15) & ~15u)) return;
+    const uint32_t F = gu.rows / 2, per = F / 256, lane = threadIdx.x & 31, group = blockIdx.x / per;   // F % 256 == 0
+    const uint32_t t = group * 8 + (lane >> 2), c = (blockIdx.x - group * per) * 256 + (threadIdx.x >> 5) * 32 + (lane & 3) * 8;
     F8 y = {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}};
     if (t < gu.n) {
         const F8 a = pf_sum8(gu, t, c), b = pf_sum8(gu, t, F + c);
@@ -221,7 +226,10 @@ int32_t launch_prefill_embed(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *embd
 }
 
 int32_t launch_prefill_norm_split(ib_ctx *ctx, cudaStream_t s, float *X, const PfPlanes *add, const float *w, float eps, uint32_t n, uint32_t cols, __half *xt) {
-    return pf_launch(ctx, s, prefill_norm_split_kernel, (n + 15) & ~15u, PF_ROW_THREADS, X, add ? *add : PfPlanes{}, add ? 1u : 0u, w, eps, n, cols, xt);
+    const uint32_t rows = (n + 15) & ~15u;
+    const PfPlanes planes = add ? *add : PfPlanes{};
+    if (n >= PF_FOUR_TOKENS) return pf_launch(ctx, s, prefill_norm_split_kernel<4>, rows / 4, PF_ROW_THREADS, X, planes, add ? 1u : 0u, w, eps, n, cols, xt);
+    return pf_launch(ctx, s, prefill_norm_split_kernel<1>, rows, PF_ROW_THREADS, X, planes, add ? 1u : 0u, w, eps, n, cols, xt);
 }
 
 static uint32_t pf_grid(size_t threads) { return (uint32_t)((threads + 255) / 256); }
@@ -238,7 +246,7 @@ int32_t launch_prefill_finish(ib_ctx *ctx, cudaStream_t s, float *out, const PfP
     return pf_launch(ctx, s, prefill_finish_kernel, pf_grid(columns / 8), 256, out, add);
 }
 int32_t launch_prefill_swiglu(ib_ctx *ctx, cudaStream_t s, const PfPlanes &gu, __half *xt) {
-    return pf_launch(ctx, s, prefill_swiglu_kernel, pf_grid((size_t)((gu.n + 15) & ~15u) * gu.rows / 16), 256, gu, xt);
+    return pf_launch(ctx, s, prefill_swiglu_kernel, ((gu.n + 15) & ~15u) / 8 * (gu.rows / 512), 256, gu, xt);
 }
 int32_t launch_prefill_qkv(ib_ctx *ctx, cudaStream_t s, const PfQkv &p) {
     return pf_launch(ctx, s, prefill_qkv_kernel, pf_grid((size_t)p.n * (p.q_dim + 2 * p.kv_dim) / 8), 256, p);
