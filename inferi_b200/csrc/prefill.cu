@@ -13,18 +13,20 @@
 
 namespace ib {
 
-// Rows r .. r + 7 of token t, added up over the tile's planes in plane order (deterministic); the loads are independent.
+// Rows r .. r + 7 of token t, added up over the tile's planes in plane order (deterministic); DEPTH planes are requested at a time.
+template <int DEPTH = 2>
 __device__ __forceinline__ F8 pf_sum8(const PfPlanes &g, uint32_t t, uint32_t r) {
     const size_t at = (size_t)t * g.rows + r, plane = (size_t)g.n * g.rows;
     F8 v = pf_load8u(g.plane0 + at);
     const uint32_t np = g.sk.pieces(g.sk.row_tile(r) * g.chunks + t / PF_CHUNK);
-    for (uint32_t s = 1; s < np; s += 2) {
-        const F8 a = pf_load8(g.planes + (s - 1) * plane + at);
-        if (s + 1 < np) {
-            const F8 b = pf_load8(g.planes + s * plane + at);
-            pf_add8(v, a);
-            pf_add8(v, b);
-        } else pf_add8(v, a);
+    for (uint32_t s = 1; s < np; s += DEPTH) {
+        F8 a[DEPTH];
+#pragma unroll
+        for (int k = 0; k < DEPTH; k++)
+            if (s + k < np) a[k] = pf_load8(g.planes + (s - 1 + k) * plane + at);
+#pragma unroll
+        for (int k = 0; k < DEPTH; k++)
+            if (s + k < np) pf_add8(v, a[k]);
     }
     return v;
 }
@@ -46,7 +48,7 @@ __global__ void prefill_embed_kernel(QDesc embd, const uint32_t *tokens, uint32_
 // between the two (PF_KEEP * 8 columns per thread).  Rows n .. n rounded up to 16 are zero-filled.
 constexpr int PF_ROW_THREADS = 512, PF_KEEP = 4;
 constexpr uint32_t PF_FOUR_TOKENS = 512;   // tokens from which four share a CTA
-template <int TOK>
+template <int TOK, int DEPTH>
 __global__ void __launch_bounds__(PF_ROW_THREADS) prefill_norm_split_kernel(float *X, const PfPlanes add, uint32_t has_add, const float *w, float eps, uint32_t n, uint32_t cols,
                                                                             __half *xt) {
     constexpr uint32_t LANES = 32 / TOK, STEP = PF_ROW_THREADS / TOK * 8, WARPS = PF_ROW_THREADS / 32;
@@ -63,7 +65,7 @@ __global__ void __launch_bounds__(PF_ROW_THREADS) prefill_norm_split_kernel(floa
         if (there) {
             v = pf_load8u(x + c);
             if (has_add) {
-                pf_add8(v, pf_sum8(add, t, c));
+                pf_add8(v, pf_sum8<DEPTH>(add, t, c));
                 pf_store8(x + c, v);
             }
         }
@@ -166,6 +168,7 @@ __global__ void __launch_bounds__(256) prefill_swiglu_kernel(const PfPlanes gu, 
 
 // Eight rows (four rotation pairs) of q, k or v of one token: bias (transformer.rs:434-442), rotation of adjacent pairs
 // (crates/inferi-shaders/src/rope.rs:75-91, the angle as the decode path forms it), q out or cache append.
+template <int DEPTH>
 __global__ void __launch_bounds__(256) prefill_qkv_kernel(const PfQkv p) {
     pf_enter();
     const uint32_t per = (p.q_dim + 2 * p.kv_dim) / 8, i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -173,7 +176,7 @@ __global__ void __launch_bounds__(256) prefill_qkv_kernel(const PfQkv p) {
     const uint32_t t = i / per;
     uint32_t r = (i - t * per) * 8, which = 0;
     if (r >= p.q_dim) { r -= p.q_dim; which = 1; if (r >= p.kv_dim) { r -= p.kv_dim; which = 2; } }
-    F8 v = which == 0 ? pf_sum8(p.g[0], t, p.row0[0] + r) : (which == 1 ? pf_sum8(p.g[1], t, p.row0[1] + r) : pf_sum8(p.g[2], t, p.row0[2] + r));
+    F8 v = pf_sum8<DEPTH>(which == 0 ? p.g[0] : (which == 1 ? p.g[1] : p.g[2]), t, (which == 0 ? p.row0[0] : (which == 1 ? p.row0[1] : p.row0[2])) + r);
     const float *bias = which == 0 ? p.bias[0] : (which == 1 ? p.bias[1] : p.bias[2]);
     if (bias) pf_add8(v, F8{{bias[r], bias[r + 1], bias[r + 2], bias[r + 3], bias[r + 4], bias[r + 5], bias[r + 6], bias[r + 7]}});
     if (which < 2) {
@@ -225,11 +228,18 @@ int32_t launch_prefill_embed(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *embd
     return pf_launch(ctx, s, prefill_embed_kernel, (uint32_t)(((size_t)n * hidden + 255) / 256), 256, e, tokens_dev, n, hidden, vocab, X);
 }
 
+// Where tiles are cut into many pieces (few tokens: a tile has few units of work, and they are dealt out), four of their planes are requested at a time.
+// A layer, us, two / four / eight: 2048 hidden, 9 tokens 73.5 / 70.7 / 71.0, 45 80.8 / 78.7 / 80.6, 100 91.8 / 87.0 / 88.1, 300 151.0 / 148.4 / 152.2; 4096 hidden, 9
+// 126.7 / 124.7 / 127.1, 128 164.4 / 162.0 / 159.8.  (In every kernel alike, also where a tile has a plane or two, four were slower.)
+constexpr int PF_DEEP = 4;
+static bool pf_deep(const StreamK &sk) { return prefill_max_pieces(sk) > 3; }
+
 int32_t launch_prefill_norm_split(ib_ctx *ctx, cudaStream_t s, float *X, const PfPlanes *add, const float *w, float eps, uint32_t n, uint32_t cols, __half *xt) {
     const uint32_t rows = (n + 15) & ~15u;
     const PfPlanes planes = add ? *add : PfPlanes{};
-    if (n >= PF_FOUR_TOKENS) return pf_launch(ctx, s, prefill_norm_split_kernel<4>, rows / 4, PF_ROW_THREADS, X, planes, add ? 1u : 0u, w, eps, n, cols, xt);
-    return pf_launch(ctx, s, prefill_norm_split_kernel<1>, rows, PF_ROW_THREADS, X, planes, add ? 1u : 0u, w, eps, n, cols, xt);
+    if (n >= PF_FOUR_TOKENS) return pf_launch(ctx, s, prefill_norm_split_kernel<4, 2>, rows / 4, PF_ROW_THREADS, X, planes, add ? 1u : 0u, w, eps, n, cols, xt);
+    if (add && pf_deep(add->sk)) return pf_launch(ctx, s, prefill_norm_split_kernel<1, PF_DEEP>, rows, PF_ROW_THREADS, X, planes, 1u, w, eps, n, cols, xt);
+    return pf_launch(ctx, s, prefill_norm_split_kernel<1, 2>, rows, PF_ROW_THREADS, X, planes, add ? 1u : 0u, w, eps, n, cols, xt);
 }
 
 static uint32_t pf_grid(size_t threads) { return (uint32_t)((threads + 255) / 256); }
@@ -249,7 +259,8 @@ int32_t launch_prefill_swiglu(ib_ctx *ctx, cudaStream_t s, const PfPlanes &gu, _
     return pf_launch(ctx, s, prefill_swiglu_kernel, ((gu.n + 15) & ~15u) / 8 * (gu.rows / 512), 256, gu, xt);
 }
 int32_t launch_prefill_qkv(ib_ctx *ctx, cudaStream_t s, const PfQkv &p) {
-    return pf_launch(ctx, s, prefill_qkv_kernel, pf_grid((size_t)p.n * (p.q_dim + 2 * p.kv_dim) / 8), 256, p);
+    const bool deep = pf_deep(p.g[0].sk) || pf_deep(p.g[1].sk) || pf_deep(p.g[2].sk);
+    return pf_launch(ctx, s, deep ? prefill_qkv_kernel<PF_DEEP> : prefill_qkv_kernel<2>, pf_grid((size_t)p.n * (p.q_dim + 2 * p.kv_dim) / 8), 256, p);
 }
 
 }  // namespace ib
