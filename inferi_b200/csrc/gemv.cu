@@ -464,8 +464,9 @@ __global__ void __launch_bounds__(256) gemv_generic_kernel(const uint8_t *__rest
 //
 // A warp works on 4 rows x 8 blocks at a time: four lanes per block, each with 4 bytes of its quants (8 weights: elements 4t .. 4t + 3 and 16 on), so
 // that a row's 8 blocks are read side by side and the input vector's 256 floats, two float4 per lane, serve four rows.  Blocks start at
-// any multiple of 2 bytes: 16-bit loads, through L1.  A nibble becomes a float by a byte permute (behind the exponent of 2^23 it is the float's low
-// bits) and a subtraction, both exact; the scale is applied once per lane and block.
+// any multiple of 2 bytes: 16-bit loads, through L1.  A nibble becomes a float, divided by 256, by a byte permute (behind the exponent of 2^15 it is the
+// float's low bits) and a subtraction, both exact; the scale is applied once per lane and block, the 256 to a row's sum: without it the eight products
+// that a lane adds up before the scale could exceed the largest float where the result does not.
 // What bounds it: 160 instructions per 1024 weights and the latency of the loads (issue slots 43 % busy; requesting a step ahead, or more warps: no
 // faster).  Where there are too few groups of 4 rows to fill the GPU, 2, 4 or 8 warps of a CTA share a group's columns and their sums are added in
 // order (4096 x 14336 at 8 / 16 / 32 warps per SM: 30.9 / 19.6 / 18.8 us; 4096 x 4096 10.1 / 7.4 / 7.5); and where a row has 16 steps for each of
@@ -512,9 +513,9 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
     asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
     return d;
 }
-// bytes 2k and 2k + 1 of w, minus `bias` - 2^23
+// bytes 2k and 2k + 1 of w, divided by 256, minus `bias` - 2^15
 __device__ __forceinline__ unsigned long long byte_pair(uint32_t w, uint32_t k, float bias) {
-    const unsigned long long p = pair_of(__uint_as_float(__byte_perm(w, 0x4B000000u, 0x7440u + 2 * k)), __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7441u + 2 * k)));
+    const unsigned long long p = pair_of(__uint_as_float(__byte_perm(w, 0x47000000u, 0x7440u + 2 * k)), __uint_as_float(__byte_perm(w, 0x47000000u, 0x7441u + 2 * k)));
     unsigned long long d;
     asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(p), "l"(pair_of(-bias, -bias)));
     return d;
@@ -553,7 +554,11 @@ __global__ void __launch_bounds__(LEGACY_WARPS * 32) gemv_legacy_kernel(const ui
             }
             const unsigned long long xl[2] = {pair_of(a.x, a.y), pair_of(a.z, a.w)}, xh[2] = {pair_of(c.x, c.y), pair_of(c.z, c.w)};
             float sx = 0.f;
-            if constexpr (F::MIN) sx = ((a.x + a.y) + (a.z + a.w)) + ((c.x + c.y) + (c.z + c.w));
+            if constexpr (F::MIN) {   // / 256, as the products
+                constexpr float K = 0.00390625f;
+                const float lo4 = fmaf(a.x, K, a.y * K) + fmaf(a.z, K, a.w * K), hi4 = fmaf(c.x, K, c.y * K) + fmaf(c.z, K, c.w * K);
+                sx = lo4 + hi4;
+            }
 #pragma unroll
             for (uint32_t r = 0; r < LEGACY_ROWS; r++) {
                 const uint32_t q = __byte_perm(now.q[r][0], now.q[r][1], 0x5410u);
@@ -565,8 +570,8 @@ __global__ void __launch_bounds__(LEGACY_WARPS * 32) gemv_legacy_kernel(const ui
                 unsigned long long s = 0ull;   // a pair of sums
 #pragma unroll
                 for (uint32_t k = 0; k < 2; k++) {
-                    s = fma2(byte_pair(lo, k, 8388608.0f + F::OFFSET), xl[k], s);
-                    s = fma2(byte_pair(hi, k, 8388608.0f + F::OFFSET), xh[k], s);
+                    s = fma2(byte_pair(lo, k, 32768.0f + F::OFFSET / 256.0f), xl[k], s);
+                    s = fma2(byte_pair(hi, k, 32768.0f + F::OFFSET / 256.0f), xh[k], s);
                 }
                 acc[r] = fmaf(h2f(now.d[r]), pair_sum(s), acc[r]);
                 if constexpr (F::MIN) acc[r] = fmaf(h2f(now.m[r]), sx, acc[r]);
@@ -577,14 +582,15 @@ __global__ void __launch_bounds__(LEGACY_WARPS * 32) gemv_legacy_kernel(const ui
     for (uint32_t r = 0; r < LEGACY_ROWS; r++)
 #pragma unroll
         for (int o = 16; o; o >>= 1) acc[r] += __shfl_xor_sync(0xffffffffu, acc[r], o);
+    // times 256: where the sum is complete
     if (share > 1) {
         if (lane < LEGACY_ROWS) part[warp][lane] = lane == 0 ? acc[0] : (lane == 1 ? acc[1] : (lane == 2 ? acc[2] : acc[3]));
         __syncthreads();
         if (mine != 0 || r0 >= rows || lane >= LEGACY_ROWS) return;
         float s = 0.f;
         for (uint32_t k = 0; k < share; k++) s += part[warp + k][lane];
-        out[r0 + lane] = s;
-    } else if (r0 < rows && lane < LEGACY_ROWS) out[r0 + lane] = lane == 0 ? acc[0] : (lane == 1 ? acc[1] : (lane == 2 ? acc[2] : acc[3]));
+        out[r0 + lane] = 256.0f * s;
+    } else if (r0 < rows && lane < LEGACY_ROWS) out[r0 + lane] = 256.0f * (lane == 0 ? acc[0] : (lane == 1 ? acc[1] : (lane == 2 ? acc[2] : acc[3])));
 }
 
 template <int QT>

@@ -83,6 +83,19 @@ def test_legacy_splits(backend, qt, rows, cols):
     assert_close(out.cpu().numpy(), oracle.gemv_ref(qt, rows, cols, blocks, v.cpu().numpy()), what=f"{quant.NAMES[qt]} {rows}x{cols}")
 
 
+# A power of two in front of the vector goes through to the result bit by bit (every operation is exact in it), up to elements or results near the
+# largest float: no sum on the way exceeds it earlier.
+@pytest.mark.parametrize("qt", LEGACY)
+@pytest.mark.parametrize("rows,cols", [(12, 96), (9480, 512)])
+def test_legacy_large_vectors(backend, qt, rows, cols):
+    blocks = quant.random_blocks(qt, rows, cols, seed=rows)
+    v = np.clip(np.random.default_rng(cols).standard_normal(cols), -4, 4).astype(np.float32)
+    small = run_gemv(backend, qt, rows, cols, blocks, v)
+    k = 126 - int(np.floor(np.log2(max(np.abs(small).max(), np.abs(v).max()))))   # the largest result or element is then at least 2^126
+    big = run_gemv(backend, qt, rows, cols, blocks, np.ldexp(v, k))
+    assert np.array_equal(big, np.ldexp(small, k))
+
+
 def _shape_case(backend, qt, rows, cols):
     blocks = quant.random_blocks(qt, rows, cols, seed=rows * 31 + cols + qt, scale=1.0, subnormal_frac=0.25)
     v = np.random.default_rng(cols).standard_normal(cols).astype(np.float32)
