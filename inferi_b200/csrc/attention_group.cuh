@@ -131,14 +131,13 @@ __device__ __forceinline__ void store_out(float *p, const float (&o)[N], float w
     }
 }
 
-// A lane's 8 elements of a cache row: one 16-byte load of f16, two of f32 (each of them 16 bytes of every lane side by side).  FIRST, SECOND: where its
-// elements 0-3 and 4-7 are in the row.
+// A lane's 8 elements of a cache row: one 16-byte load of f16, two of f32 (each of them 16 bytes of every lane side by side).  FIRST * li: where its
+// elements 0-3 are in the row; SECOND: how far behind them 4-7 are.  (load: from the lane's elements on)
 template <typename T, int HS> struct LaneRow;
 template <int HS> struct LaneRow<__half, HS> {
+    static constexpr uint32_t FIRST = 8, SECOND = 4;
     uint4 r;
-    static __device__ __forceinline__ uint32_t first(int li) { return 8 * li; }
-    static __device__ __forceinline__ uint32_t second(int li) { return 8 * li + 4; }
-    __device__ __forceinline__ void load(const __half *row, int li) { r = __ldcg(reinterpret_cast<const uint4 *>(row + 8 * li)); }
+    __device__ __forceinline__ void load(const __half *p) { r = __ldcg(reinterpret_cast<const uint4 *>(p)); }
     __device__ __forceinline__ void get(float2 (&f)[4]) const {
         const __half2 *h = reinterpret_cast<const __half2 *>(&r);
 #pragma unroll
@@ -146,12 +145,11 @@ template <int HS> struct LaneRow<__half, HS> {
     }
 };
 template <int HS> struct LaneRow<float, HS> {
+    static constexpr uint32_t FIRST = 4, SECOND = HS / 2;
     float4 a, b;
-    static __device__ __forceinline__ uint32_t first(int li) { return 4 * li; }
-    static __device__ __forceinline__ uint32_t second(int li) { return HS / 2 + 4 * li; }
-    __device__ __forceinline__ void load(const float *row, int li) {
-        a = __ldcg(reinterpret_cast<const float4 *>(row + first(li)));
-        b = __ldcg(reinterpret_cast<const float4 *>(row + second(li)));
+    __device__ __forceinline__ void load(const float *p) {
+        a = __ldcg(reinterpret_cast<const float4 *>(p));
+        b = __ldcg(reinterpret_cast<const float4 *>(p + SECOND));
     }
     __device__ __forceinline__ void get(float2 (&f)[4]) const {
         f[0] = make_float2(a.x, a.y); f[1] = make_float2(a.z, a.w);
@@ -211,9 +209,13 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
     const int g = lane / L, li = lane % L;
     const uint32_t kv_dim = a.p.kv_dim;
     const uint32_t cache_head = KVM == (int)ATTN_GROUP ? kvh >> (a.p.kv_mul > ATTN_GROUP ? 1 : 0) : kvh;   // (eight heads: two groups)
-    const T *kc = reinterpret_cast<const T *>(a.kc) + (size_t)cache_head * HS;
-    const T *vc = reinterpret_cast<const T *>(a.vc) + (size_t)cache_head * HS;
-    const uint32_t at0 = LaneRow<T, HS>::first(li), at1 = LaneRow<T, HS>::second(li);
+    const uint32_t at0 = LaneRow<T, HS>::FIRST * li, at1 = at0 + LaneRow<T, HS>::SECOND;
+    // The lane's offset: part of the pointers that the loop starts from (f16, 19000 positions of 16 heads of 64: 27.3 us, 27.6 if added per load), but not in the
+    // long regime of head size 128, which has no registers left (10000 positions of 8 heads: 13.87 us, 14.00 if it is).
+    constexpr bool FOLDED = HS != 128 || REGIME != ATTN_LONG;
+    const uint32_t in_base = FOLDED ? at0 : 0u, in_load = FOLDED ? 0u : at0;
+    const T *kc = reinterpret_cast<const T *>(a.kc) + (size_t)cache_head * HS + in_base;
+    const T *vc = reinterpret_cast<const T *>(a.vc) + (size_t)cache_head * HS + in_base;
     const float scale = 1.0f / sqrtf((float)HS);
 
     // First iteration: the predecessor (the q/k/v kernel) writes this token's q and the newest cache row (position
@@ -226,8 +228,8 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
         for (int s = 0; s < STEPS; s++) {
             const uint32_t t = base0 + s * RPW + g, tc = t < t1 ? t : t1 - 1;
             if (tc + 1 != total || !early) {
-                kraw[s].load(kc + (size_t)tc * kv_dim, li);
-                vraw[s].load(vc + (size_t)tc * kv_dim, li);
+                kraw[s].load(kc + (size_t)tc * kv_dim + in_load);
+                vraw[s].load(vc + (size_t)tc * kv_dim + in_load);
             }
         }
     }
@@ -238,8 +240,8 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
             for (int s = 0; s < STEPS; s++) {
                 const uint32_t t = base0 + s * RPW + g, tc = t < t1 ? t : t1 - 1;
                 if (tc + 1 == total) {
-                    kraw[s].load(kc + (size_t)tc * kv_dim, li);
-                    vraw[s].load(vc + (size_t)tc * kv_dim, li);
+                    kraw[s].load(kc + (size_t)tc * kv_dim + in_load);
+                    vraw[s].load(vc + (size_t)tc * kv_dim + in_load);
                 }
             }
         }
@@ -281,8 +283,8 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
 #pragma unroll
             for (int s = 0; s < STEPS; s++) {
                 const uint32_t t = nbase + s * RPW + g, tc = t < t1 ? t : t1 - 1;
-                knext[s].load(kc + (size_t)tc * kv_dim, li);
-                vnext[s].load(vc + (size_t)tc * kv_dim, li);
+                knext[s].load(kc + (size_t)tc * kv_dim + in_load);
+                vnext[s].load(vc + (size_t)tc * kv_dim + in_load);
             }
         }
         // partial scores of the lane's 8 elements: v[s * KVM + m]
@@ -384,7 +386,7 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
     // every thread owns PER consecutive outputs of one head (16 warps at head size 64: half of the threads one each)
     constexpr uint32_t slot = HS + 2;
     constexpr int PER = KVM * HS >= THREADS ? KVM * HS / THREADS : 1;
-    const bool has = tid * PER < KVM * HS;
+    const bool has = KVM * HS >= THREADS || tid * PER < KVM * HS;
     const int at = has ? tid * PER : 0, m_out = at / HS, d_out = at % HS;
     // partials in global memory: the accumulators [kv head][slice][KVM][HS], behind them all (max, sum) pairs [kv head][slice][KVM]
     float *part = a.scratch + ((size_t)kvh * a.max_splits + split) * KVM * HS;
