@@ -661,7 +661,17 @@ int32_t launch_gemv_stream(ib_ctx *ctx, cudaStream_t stream, const GemvParams &p
     // A stage always serves the same stream: the barriers' parities only order uses that one and the same warp waits for.
     while (split.RG > S) split.RG /= 2;
     S -= S % split.RG;
-    if (split.mode == ROWS4 && most_pt == 2 && S >= 5 * split.RG) {
+    // Two tiles at a time: where CTAs have more of them than that takes to pay.  us, one / two at a time: Q4_K of 14336 columns, 592 rows (a tile per CTA)
+    // 4.84 / 4.99, 800 5.68 / 5.60, 2000 7.82 / 7.15; Q5_K of 12288, 592 rows 4.52 / 5.09, 1500 6.67 / 6.77, 2000 (3.4 tiles per CTA) 7.77 / 7.45; Q6_K of
+    // 10240, 1180 5.28 / 5.49, 2000 7.07 / 6.94.  Q8_0, which has the fewest instructions per byte, waits for a second tile in vain: 8704 columns, 800 rows
+    // 4.57 / 5.17, 2960 7.75 / 8.64.
+    bool q4_k = true, q8_0 = false;
+    for (uint32_t s = 0; s < p.nseg; s++) {
+        q4_k = q4_k && p.seg[s].qtype == IB_Q4_K;
+        q8_0 = q8_0 || p.seg[s].qtype == IB_Q8_0;
+    }
+    const bool pays = !q8_0 && tiles > (q4_k ? 1 : 3) * (uint32_t)grid;
+    if (split.mode == ROWS4 && most_pt == 2 && S >= 5 * split.RG && pays) {
         split.mode = ROWS8_PAIR;
         geo.stage_bytes = stage_data;   // the rows of two tiles follow one another: eight rows then start at different banks where their stride lets them
     }

@@ -56,7 +56,7 @@ def test_row_split(backend, qt, cols, rows):
 
 # Rows so long that tiles hold 4 of them, two tiles at a time: CTAs with one tile, an odd and an even number of them, and none; the last warp of a row
 # with one to four blocks
-@pytest.mark.parametrize("rows", [4, 8, 588, 600, 1188, 1776, 4100])
+@pytest.mark.parametrize("rows", [4, 8, 588, 600, 1188, 1776, 1780, 2400, 4100])
 @pytest.mark.parametrize("qt,cols", [(quant.Q4_K, 14336), (quant.Q4_K, 15104), (quant.Q5_K, 12800), (quant.Q6_K, 10240), (quant.Q8_0, 8704)])
 def test_long_rows_two_tiles_at_a_time(backend, qt, cols, rows):
     _shape_case(backend, qt, rows, cols)
