@@ -1,7 +1,7 @@
 """Builds libinferi_b200.so (sm_100a only) in-tree with nvcc, and the Python binding of the op launches.
 
 The shared library is the product: a C-ABI (include/inferi_b200.h) with no torch or Python types in it, which needs neither to be built.  The binding
-(csrc/binding.cpp) is what `ops.py` calls it through where there is one; without it calls go through ctypes.
+(csrc/binding.cpp) is what `ops.py` calls it through where there is one for the running interpreter and torch; without it calls go through ctypes.
 """
 from __future__ import annotations
 
@@ -14,7 +14,7 @@ import sysconfig
 PKG_DIR = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG_DIR, "csrc")
 LIB_PATH = os.path.join(PKG_DIR, "libinferi_b200.so")
-BINDING_PATH = os.path.join(PKG_DIR, "_binding.so")
+BINDING_PATH = os.path.join(PKG_DIR, "_binding" + (sysconfig.get_config_var("EXT_SUFFIX") or ".so"))   # (another interpreter does not find it)
 BINDING_SOURCES = [os.path.join(CSRC, "binding.cpp"), os.path.join(PKG_DIR, "..", "include", "inferi_b200.h"), os.path.abspath(__file__)]
 SOURCES = ["api.cu", "gemv.cu", "gemv_stream.cu", "ops.cu", "attention.cu", "prefill.cu", "prefill_gemm.cu", "prefill_attention.cu", "llama.cu", "gguf.cu", "sampler.cu", "tokenizer.cu"]
 NVCC_FLAGS = [
@@ -38,6 +38,13 @@ def _stale() -> bool:
     return _older(LIB_PATH, [os.path.join(CSRC, f) for f in os.listdir(CSRC) if f != "binding.cpp"] + BINDING_SOURCES[1:])
 
 
+def binding_stamp() -> str:
+    """The torch that a binding is for: it reads tensors through inline accessors, which another torch may lay out otherwise."""
+    import torch
+
+    return f"torch {torch.__version__} {torch.version.git_version}"
+
+
 def _binding_command() -> list[str] | None:
     """How the binding is compiled: against this interpreter and its torch.  None without a torch, and with one that has no CUDA: no launch gets as far
     as the binding there."""
@@ -51,8 +58,15 @@ def _binding_command() -> list[str] | None:
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     includes = [f"{root}/include", f"{root}/include/torch/csrc/api/include", f"{cuda}/include", sysconfig.get_paths()["include"]]
     return [os.environ.get("CXX", "g++"), "-O2", "-std=c++20", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
-            *[f"-I{i}" for i in includes], BINDING_SOURCES[0], "-o", BINDING_PATH, f"-L{root}/lib", "-lc10", "-lc10_cuda",
+            f'-DIB_BINDING_STAMP="{binding_stamp()}"', *[f"-I{i}" for i in includes], BINDING_SOURCES[0], "-o", BINDING_PATH, f"-L{root}/lib", "-lc10", "-lc10_cuda",
             "-ltorch_cpu", "-ltorch_python", f"-Wl,-rpath,{root}/lib"]
+
+
+def _binding_stale() -> bool:
+    if _older(BINDING_PATH, BINDING_SOURCES):
+        return True
+    with open(BINDING_PATH, "rb") as f:
+        return binding_stamp().encode() not in f.read()
 
 
 def _start(cmd: list[str]) -> subprocess.Popen | None:
@@ -78,7 +92,7 @@ def _finish_binding(p: subprocess.Popen | None, verbose: bool) -> None:
 def build(force: bool = False, verbose: bool = False) -> str:
     """Compile every .cu of the package into libinferi_b200.so; returns its path.  And the binding, where there is a torch to compile it against."""
     command = _binding_command()
-    wanted = command is not None and (force or _older(BINDING_PATH, BINDING_SOURCES))
+    wanted = command is not None and (force or _binding_stale())
     binding = _start(command) if wanted else None
     try:
         if force or _stale():

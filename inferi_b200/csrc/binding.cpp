@@ -211,4 +211,12 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_binding", nullptr, -1, methods, n
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__binding() { return PyModule_Create(&module); }
+// `stamp`: the torch that this was compiled against.  Tensors are read through its headers' inline code, so it serves no other one.
+PyMODINIT_FUNC PyInit__binding() {
+    PyObject *m = PyModule_Create(&module);
+    if (m && PyModule_AddStringConstant(m, "stamp", IB_BINDING_STAMP)) {
+        Py_DECREF(m);
+        return nullptr;
+    }
+    return m;
+}

@@ -8,6 +8,7 @@ Device buffers are torch CUDA tensors (torch is only the allocator and the strea
 from __future__ import annotations
 
 import ctypes as C
+import importlib
 from dataclasses import dataclass
 
 import numpy as np
@@ -15,6 +16,7 @@ import torch
 
 from . import _lib
 from ._lib import AttnParams, InferiError, KV_F16, KV_F32, ROPE_NEOX, ROPE_ORIGINAL, check  # noqa: F401
+from .build import binding_stamp
 from .quant import BLOCK_BYTES, BLOCK_ELEMS, F32, NAMES, Q4_K, Q5_K, Q6_K, Q8_0, row_bytes  # noqa: F401
 
 
@@ -38,13 +40,21 @@ def _f32_dev(t: torch.Tensor, name: str) -> int:
 
 # A launch goes through the compiled binding (csrc/binding.cpp), which checks what the code behind it checks and answers with the library's status, or
 # with -1 where it has not launched anything: for arguments that it does not know (tensor subclasses), and for those that are refused.  The Python
-# way then does the call or raises the error, and does all of them where there is no binding.
-try:
-    from . import _binding as _fast
-except ImportError:
-    class _fast:
-        gemv = gemm = rms_norm = rope = silu = add = attention = argmax = sample = staticmethod(lambda *a: -1)
-        bind = staticmethod(lambda *a: None)
+# way then does the call or raises the error, and does all of them where there is no binding, or one of another torch.
+class _NoBinding:
+    gemv = gemm = rms_norm = rope = silu = add = attention = argmax = sample = staticmethod(lambda *a: -1)
+    bind = staticmethod(lambda *a: None)
+
+
+def _load_binding():
+    try:
+        m = importlib.import_module("._binding", __package__)
+    except ImportError:
+        return _NoBinding
+    return m if getattr(m, "stamp", None) == binding_stamp() else _NoBinding
+
+
+_fast = _load_binding()
 _BOUND = ("ib_gemv_quant", "ib_gemm_quant", "ib_rms_norm", "ib_rope", "ib_silu_mul", "ib_add_assign", "ib_attention", "ib_argmax", "ib_sample")
 
 

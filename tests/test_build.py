@@ -6,7 +6,7 @@ import types
 import pytest
 import torch
 
-from inferi_b200 import build
+from inferi_b200 import build, ops
 
 COMPILER = """#!/bin/sh
 echo {name} >> {log}
@@ -46,7 +46,7 @@ def tree(tmp_path, monkeypatch):
     monkeypatch.setattr(build, "BINDING_SOURCES", [str(csrc / "binding.cpp"), build.__file__])
     monkeypatch.setattr(build, "SOURCES", ["one.cu"])
     monkeypatch.setattr(build, "_nvcc", lambda: compiler("nvcc"))
-    monkeypatch.setenv("CXX", compiler("cxx"))
+    monkeypatch.setenv("CXX", compiler("cxx", f'echo "{build.binding_stamp()}" > $out'))
     return types.SimpleNamespace(path=tmp_path, csrc=csrc, compiler=compiler, calls=calls)
 
 
@@ -98,3 +98,21 @@ def test_a_torch_that_has_no_binding(tree, monkeypatch, kind):
     assert tree.calls() == LIBRARY
     build.build()
     assert tree.calls() == []
+
+
+@with_cuda
+def test_a_binding_of_another_torch_is_built_again(tree, monkeypatch):
+    build.build()
+    tree.calls()
+    monkeypatch.setattr(build, "binding_stamp", lambda: "torch of tomorrow")
+    build.build()
+    assert tree.calls() == ["cxx"]
+
+
+@pytest.mark.parametrize("stamp", [None, "torch of yesterday"])
+def test_a_binding_of_another_torch_is_not_used(monkeypatch, stamp):
+    other = types.SimpleNamespace(**({"stamp": stamp} if stamp else {}))
+    monkeypatch.setitem(sys.modules, "inferi_b200._binding", other)
+    assert ops._load_binding() is ops._NoBinding
+    other.stamp = build.binding_stamp()
+    assert ops._load_binding() is other
