@@ -43,25 +43,23 @@ __global__ void prefill_embed_kernel(QDesc embd, const uint32_t *tokens, uint32_
 }
 
 // X += the planes of the GEMM before (where there is one), then y = (X * rsqrt(mean(X^2) + eps)) * w
-// (crates/inferi-shaders/src/rms_norm.rs:112-120; `w` null: y = X) as the next GEMM's inputs.  TOK tokens per CTA, a warp's lanes shared out to them: the
-// inputs' layout holds 8 tokens' 8 columns side by side, and a warp of one token writes 16 bytes of every 128.  The row stays in registers
-// between the two (PF_KEEP * 8 columns per thread).  Rows n .. n rounded up to 16 are zero-filled.
+// (crates/inferi-shaders/src/rms_norm.rs:112-120) as the next GEMM's inputs; without NORM y = X.  TOK tokens per CTA, a warp's lanes shared out to them: the
+// inputs' layout holds 8 tokens' 8 columns side by side, and a warp of one token writes 16 bytes of every 128.  With NORM the row stays in registers
+// between the two (PF_KEEP * 8 columns per thread; what is longer is read again).  Rows n .. n rounded up to 16 are zero-filled.
 constexpr int PF_ROW_THREADS = 512, PF_KEEP = 4;
-constexpr uint32_t PF_FOUR_TOKENS = 512;   // tokens from which four share a CTA
-template <int TOK, int DEPTH>
+template <int TOK, int DEPTH, bool NORM>
 __global__ void __launch_bounds__(PF_ROW_THREADS) prefill_norm_split_kernel(float *X, const PfPlanes add, uint32_t has_add, const float *w, float eps, uint32_t n, uint32_t cols,
                                                                             __half *xt) {
     constexpr uint32_t LANES = 32 / TOK, STEP = PF_ROW_THREADS / TOK * 8, WARPS = PF_ROW_THREADS / 32;
-    __shared__ float red[WARPS][TOK];
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, which = lane / LANES, t = blockIdx.x * TOK + which;
     const uint32_t c0 = (warp * LANES + lane % LANES) * 8;   // cols % 256 == 0: whole warps
     const bool there = t < n;
     pf_enter();
     float *x = X + (size_t)t * cols;
+    const F8 zero = {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}};
     F8 keep[PF_KEEP];
-    float ss = 0.f;
     auto fetch = [&](uint32_t c) {
-        F8 v = {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}};
+        F8 v = zero;
         if (there) {
             v = pf_load8u(x + c);
             if (has_add) {
@@ -69,18 +67,32 @@ __global__ void __launch_bounds__(PF_ROW_THREADS) prefill_norm_split_kernel(floa
                 pf_store8(x + c, v);
             }
         }
-#pragma unroll
-        for (int i = 0; i < 8; i++) ss += v.v[i] * v.v[i];
         return v;
     };
+    if constexpr (!NORM) {   // (blockIdx.y: so many of the columns)
+        const uint32_t c1 = c0 + blockIdx.y * PF_KEEP * STEP;
 #pragma unroll
-    for (int k = 0; k < PF_KEEP; k++) {
-        const uint32_t c = c0 + k * STEP;
-        if (c < cols) keep[k] = fetch(c);
-    }
-    for (uint32_t c = c0 + PF_KEEP * STEP; c < cols; c += STEP) fetch(c);
-    float rms = 1.0f;
-    if (w) {
+        for (int k = 0; k < PF_KEEP; k++)
+            if (c1 + k * STEP < cols) keep[k] = fetch(c1 + k * STEP);
+#pragma unroll
+        for (int k = 0; k < PF_KEEP; k++)
+            if (c1 + k * STEP < cols) pf_emit8(xt, t, c1 + k * STEP, cols, keep[k]);
+    } else {
+        __shared__ float red[WARPS][TOK];
+        float ss = 0.f;
+        auto square = [&](const F8 &v) {
+#pragma unroll
+            for (int i = 0; i < 8; i++) ss += v.v[i] * v.v[i];
+        };
+#pragma unroll
+        for (int k = 0; k < PF_KEEP; k++) {
+            const uint32_t c = c0 + k * STEP;
+            if (c < cols) {
+                keep[k] = fetch(c);
+                square(keep[k]);
+            }
+        }
+        for (uint32_t c = c0 + PF_KEEP * STEP; c < cols; c += STEP) square(fetch(c));
 #pragma unroll
         for (uint32_t o = LANES / 2; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
         if (lane % LANES == 0) red[warp][which] = ss;
@@ -88,23 +100,20 @@ __global__ void __launch_bounds__(PF_ROW_THREADS) prefill_norm_split_kernel(floa
         float tot = 0.f;
 #pragma unroll
         for (uint32_t i = 0; i < WARPS; i++) tot += red[i][which];
-        rms = 1.0f / sqrtf(tot / (float)cols + eps);
-    }
-    auto emit = [&](uint32_t c, F8 v) {
-        if (w) {
+        const float rms = 1.0f / sqrtf(tot / (float)cols + eps);
+        auto emit = [&](uint32_t c, F8 v) {
             const F8 g = pf_load8(w + c);
 #pragma unroll
             for (int i = 0; i < 8; i++) v.v[i] = (v.v[i] * rms) * g.v[i];
-        }
-        pf_emit8(xt, t, c, cols, v);
-    };
+            pf_emit8(xt, t, c, cols, v);
+        };
 #pragma unroll
-    for (int k = 0; k < PF_KEEP; k++) {
-        const uint32_t c = c0 + k * STEP;
-        if (c < cols) emit(c, keep[k]);
+        for (int k = 0; k < PF_KEEP; k++) {
+            const uint32_t c = c0 + k * STEP;
+            if (c < cols) emit(c, keep[k]);
+        }
+        for (uint32_t c = c0 + PF_KEEP * STEP; c < cols; c += STEP) emit(c, there ? pf_load8u(x + c) : zero);
     }
-    const F8 zero = {{0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f}};
-    for (uint32_t c = c0 + PF_KEEP * STEP; c < cols; c += STEP) emit(c, there ? pf_load8u(x + c) : zero);
 }
 
 __global__ void __launch_bounds__(256) prefill_residual_kernel(float *X, const PfPlanes add) {
@@ -207,9 +216,9 @@ __global__ void __launch_bounds__(256) prefill_qkv_kernel(const PfQkv p) {
 // host side
 // ---------------------------------------------------------------------------------------------------------------------
 template <typename... KArgs, typename... Args>
-static int32_t pf_launch(ib_ctx *ctx, cudaStream_t s, void (*kernel)(KArgs...), uint32_t grid, uint32_t block, const Args &...args) {
+static int32_t pf_launch(ib_ctx *ctx, cudaStream_t s, void (*kernel)(KArgs...), dim3 grid, uint32_t block, const Args &...args) {
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
+    cfg.gridDim = grid;
     cfg.blockDim = dim3(block);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
@@ -234,12 +243,22 @@ int32_t launch_prefill_embed(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *embd
 constexpr int PF_DEEP = 4;
 static bool pf_deep(const StreamK &sk) { return prefill_max_pieces(sk) > 3; }
 
+// Tokens from which four share a CTA: with a norm as long as the CTA holds four rows in its registers.  Longer rows, read twice, took 64.1 us instead of 58.5
+// (2048 x 8192 Q4_K, 700 tokens, the GEMM with its inputs), a layer of 8192 hidden at 600 tokens 706 instead of 687; two tokens per CTA there 691.  Without a norm nothing
+// is held, and rows are shared out to CTAs of 4096 columns: 2048 x 1024, 1000 tokens 21.0 us (one token per CTA 25.6), x 8192, 700 55.5 (58.4), x 14336, 700
+// 91.0 (94.6; with four whole rows per CTA 102.5: 176 CTAs of 148 at a time).
+constexpr uint32_t PF_MANY_TOKENS = 512;
 int32_t launch_prefill_norm_split(ib_ctx *ctx, cudaStream_t s, float *X, const PfPlanes *add, const float *w, float eps, uint32_t n, uint32_t cols, __half *xt) {
-    const uint32_t rows = (n + 15) & ~15u;
+    constexpr uint32_t held = PF_KEEP * PF_ROW_THREADS * 8;   // columns that a CTA holds in its registers
     const PfPlanes planes = add ? *add : PfPlanes{};
-    if (n >= PF_FOUR_TOKENS) return pf_launch(ctx, s, prefill_norm_split_kernel<4, 2>, rows / 4, PF_ROW_THREADS, X, planes, add ? 1u : 0u, w, eps, n, cols, xt);
-    if (add && pf_deep(add->sk)) return pf_launch(ctx, s, prefill_norm_split_kernel<1, PF_DEEP>, rows, PF_ROW_THREADS, X, planes, 1u, w, eps, n, cols, xt);
-    return pf_launch(ctx, s, prefill_norm_split_kernel<1, 2>, rows, PF_ROW_THREADS, X, planes, add ? 1u : 0u, w, eps, n, cols, xt);
+    auto launch = [&](auto kernel, uint32_t tokens) {
+        const dim3 grid(((n + 15) & ~15u) / tokens, w ? 1 : (cols + held / tokens - 1) / (held / tokens));
+        return pf_launch(ctx, s, kernel, grid, PF_ROW_THREADS, X, planes, add ? 1u : 0u, w, eps, n, cols, xt);
+    };
+    const bool many = n >= PF_MANY_TOKENS;
+    if (!w) return many ? launch(prefill_norm_split_kernel<4, 2, false>, 4) : launch(prefill_norm_split_kernel<1, 2, false>, 1);
+    if (many && cols <= held / 4) return launch(prefill_norm_split_kernel<4, 2, true>, 4);
+    return add && pf_deep(add->sk) ? launch(prefill_norm_split_kernel<1, PF_DEEP, true>, 1) : launch(prefill_norm_split_kernel<1, 2, true>, 1);
 }
 
 static uint32_t pf_grid(size_t threads) { return (uint32_t)((threads + 255) / 256); }

@@ -54,6 +54,14 @@ def test_gemm_across_chunks_of_tokens(backend, qt, rows, cols, n):
     m.close()
 
 
+# from 512 tokens on several of them share a CTA of the kernel that splits the inputs: either side of the limit, rows of up to 4096 columns, of a few
+# more, and of a part of the next 4096
+@pytest.mark.parametrize("cols", [4096, 4352, 14336])
+@pytest.mark.parametrize("n", [511, 513, 1030])
+def test_gemm_inputs_of_many_tokens(backend, cols, n):
+    test_gemm_across_chunks_of_tokens(backend, quant.Q4_K, 128, cols, n)
+
+
 # a pair of SMs shares 256 rows and a chunk's tokens: an odd number of 128-row halves, halves with a remainder (up to 64 tokens such small matrices
 # are one SM's work per tile)
 @pytest.mark.parametrize("qt", [quant.Q4_K, quant.Q5_K, quant.Q6_K, quant.Q8_0])

@@ -85,6 +85,17 @@ def test_formats_that_share_a_launch(backend, qk, heads):
     dev_w.close()
 
 
+# The norm holds four tokens' rows of up to 4096 columns per CTA from 512 tokens on, one token's of up to 16384 else; a token count that leaves padding rows
+@pytest.mark.parametrize("hidden", [2048, 4096, 4608, 8704])
+@pytest.mark.parametrize("n", [9, 517])
+def test_norms_of_many_tokens(backend, hidden, n):
+    cfg = Llama2Config(hidden, 512, 1, hidden // 128, hidden // 512, 512, 640, 500000.0, 1e-5)
+    w = synth_weights(cfg, seed=hidden, device="cuda", recipe={**{k: quant.Q4_K for k in Q4_K_M}, "token_embd": quant.Q4_K})
+    dev_w = Llama2Weights(backend, cfg, w)
+    loop_vs_prefill(backend, cfg, dev_w, np.random.default_rng(n).integers(0, cfg.vocab_size, n).tolist(), 2)
+    dev_w.close()
+
+
 @pytest.mark.parametrize("hidden,heads,n,start", [(512, 8, 17, 0), (512, 8, 1, 300), (512, 4, 65, 0), (512, 4, 15, 470), (512, 8, 200, 130)])
 def test_prompt_attention_at_the_edges_of_its_tiles(backend, hidden, heads, n, start):
     """16-token and 64-position tiles with remainders, positions divided between the CTAs of a cluster (few tokens far into the
