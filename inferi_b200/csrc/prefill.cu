@@ -104,7 +104,7 @@ __global__ void __launch_bounds__(PF_ROW_THREADS) prefill_norm_split_kernel(floa
         auto emit = [&](uint32_t c, F8 v) {
             const F8 g = pf_load8(w + c);
 #pragma unroll
-            for (int i = 0; i < 8; i++) v.v[i] = (v.v[i] * rms) * g.v[i];
+            for (int i = 0; i < 8; i++) v.v[i] = there ? (v.v[i] * rms) * g.v[i] : 0.f;
             pf_emit8(xt, t, c, cols, v);
         };
 #pragma unroll
