@@ -467,11 +467,14 @@ __global__ void __launch_bounds__(256) gemv_generic_kernel(const uint8_t *__rest
 // any multiple of 2 bytes: 16-bit loads, through L1.  A nibble becomes a float, divided by 256, by a byte permute (behind the exponent of 2^15 it is the
 // float's low bits) and a subtraction, both exact; the scale is applied once per lane and block, the 256 to a row's sum: without it the eight products
 // that a lane adds up before the scale could exceed the largest float where the result does not.
+// With a minimum (Q4_1, Q5_1) q goes to the top of the mantissa behind the exponent of 16 or 32, and one multiply-add makes the weight of it, (16 + q) d + (m - 16 d),
+// rounded once (m - 16 d is exact but where the two lie more than 13 powers of two apart).  The sums of q's and of the minimum's products apart nearly
+// cancel: 1.3 to 3.3 times the error of a sum over the weights, for 30.4 instead of 34.7 us at Q4_1 12464 x 8448, 36.1 instead of 39.5 at Q5_1.
 // What bounds it: 160 instructions per 1024 weights and the latency of the loads (issue slots 43 % busy; requesting a step ahead, or more warps: no
 // faster).  Where there are too few groups of 4 rows to fill the GPU, 2, 4 or 8 warps of a CTA share a group's columns and their sums are added in
 // order (4096 x 14336 at 8 / 16 / 32 warps per SM: 30.9 / 19.6 / 18.8 us; 4096 x 4096 10.1 / 7.4 / 7.5); and where a row has 16 steps for each of
 // them (12464 x 8448, a warp a group / four: 37.1 / 31.4 us; a row of 8 steps is better off alone, 64000 x 2048: 34.0 / 39.2).
-// Q4_0 12464 x 8448 (59 MB): 31 us; one warp per row, one block per lane and byte loads: 406.  4096 x 4096 7.2 us, 73.
+// Q4_0 12464 x 8448 (59 MB) 31.6 us, Q5_0 32.7; one warp per row, one block per lane and byte loads: 406.  4096 x 4096 7.0 us, 73.
 // -------------------------------------------------------------------------------------------------
 template <int QT>
 struct Legacy {
@@ -521,6 +524,13 @@ __device__ __forceinline__ unsigned long long byte_pair(uint32_t w, uint32_t k, 
     return d;
 }
 
+// 16 + q, or 32 + q with a fifth bit, of bytes 2k and 2k + 1 of w, which hold q at the top of a float's mantissa
+template <bool FIVE>
+__device__ __forceinline__ unsigned long long mantissa_pair(uint32_t w, uint32_t k) {
+    constexpr uint32_t TOP = FIVE ? 0x42000000u : 0x41000000u;
+    return pair_of(__uint_as_float(__byte_perm(w, TOP, 0x7044u + 0x200u * k)), __uint_as_float(__byte_perm(w, TOP, 0x7144u + 0x200u * k)));
+}
+
 // ALIGNED: the vector is on a 16-byte boundary
 template <int QT, bool ALIGNED>
 __global__ void __launch_bounds__(LEGACY_WARPS * 32) gemv_legacy_kernel(const uint8_t *__restrict__ w, uint32_t rows, uint32_t nb, uint64_t row_bytes, uint32_t share,
@@ -553,28 +563,34 @@ __global__ void __launch_bounds__(LEGACY_WARPS * 32) gemv_legacy_kernel(const ui
                 for (uint32_t k = 0; k < LEGACY_ROWS; k++) now.d[k] = now.m[k] = 0u;
             }
             const unsigned long long xl[2] = {pair_of(a.x, a.y), pair_of(a.z, a.w)}, xh[2] = {pair_of(c.x, c.y), pair_of(c.z, c.w)};
-            float sx = 0.f;
-            if constexpr (F::MIN) {   // / 256, as the products
-                constexpr float K = 0.00390625f;
-                const float lo4 = fmaf(a.x, K, a.y * K) + fmaf(a.z, K, a.w * K), hi4 = fmaf(c.x, K, c.y * K) + fmaf(c.z, K, c.w * K);
-                sx = lo4 + hi4;
-            }
 #pragma unroll
             for (uint32_t r = 0; r < LEGACY_ROWS; r++) {
                 const uint32_t q = __byte_perm(now.q[r][0], now.q[r][1], 0x5410u);
-                uint32_t lo = q & 0x0F0F0F0Fu, hi = (q >> 4) & 0x0F0F0F0Fu;
-                if constexpr (F::FIVE) {   // four bits into bit 4 of four bytes
-                    lo |= (((((uint32_t)now.h[r][0] >> (4 * (t & 3))) & 15u) * 0x00204081u) & 0x01010101u) << 4;
-                    hi |= (((((uint32_t)now.h[r][1] >> (4 * (t & 3))) & 15u) * 0x00204081u) & 0x01010101u) << 4;
+                uint32_t lo_five = 0u, hi_five = 0u;   // four fifth bits, one in front of each byte's
+                if constexpr (F::FIVE) {
+                    lo_five = ((((uint32_t)now.h[r][0] >> (4 * (t & 3))) & 15u) * 0x00204081u) & 0x01010101u;
+                    hi_five = ((((uint32_t)now.h[r][1] >> (4 * (t & 3))) & 15u) * 0x00204081u) & 0x01010101u;
                 }
                 unsigned long long s = 0ull;   // a pair of sums
+                if constexpr (F::MIN) {
+                    constexpr uint32_t UP = F::FIVE ? 2 : 3, MASK = 0x0F0F0F0Fu << UP, ONE = F::FIVE ? 0u : 0x80808080u;
+                    const float d = h2f(now.d[r]) * 0.00390625f, m = fmaf(F::FIVE ? -32.0f : -16.0f, d, h2f(now.m[r]) * 0.00390625f);
+                    const uint32_t lo = ((q << UP) & MASK) | (lo_five << 6) | ONE, hi = ((q >> (4 - UP)) & MASK) | (hi_five << 6) | ONE;
 #pragma unroll
-                for (uint32_t k = 0; k < 2; k++) {
-                    s = fma2(byte_pair(lo, k, 32768.0f + F::OFFSET / 256.0f), xl[k], s);
-                    s = fma2(byte_pair(hi, k, 32768.0f + F::OFFSET / 256.0f), xh[k], s);
+                    for (uint32_t k = 0; k < 2; k++) {
+                        s = fma2(fma2(mantissa_pair<F::FIVE>(lo, k), pair_of(d, d), pair_of(m, m)), xl[k], s);
+                        s = fma2(fma2(mantissa_pair<F::FIVE>(hi, k), pair_of(d, d), pair_of(m, m)), xh[k], s);
+                    }
+                    acc[r] += pair_sum(s);
+                } else {
+                    const uint32_t lo = (q & 0x0F0F0F0Fu) | (lo_five << 4), hi = ((q >> 4) & 0x0F0F0F0Fu) | (hi_five << 4);
+#pragma unroll
+                    for (uint32_t k = 0; k < 2; k++) {
+                        s = fma2(byte_pair(lo, k, 32768.0f + F::OFFSET / 256.0f), xl[k], s);
+                        s = fma2(byte_pair(hi, k, 32768.0f + F::OFFSET / 256.0f), xh[k], s);
+                    }
+                    acc[r] = fmaf(h2f(now.d[r]), pair_sum(s), acc[r]);
                 }
-                acc[r] = fmaf(h2f(now.d[r]), pair_sum(s), acc[r]);
-                if constexpr (F::MIN) acc[r] = fmaf(h2f(now.m[r]), sx, acc[r]);
             }
         }
     }

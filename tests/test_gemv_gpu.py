@@ -13,7 +13,7 @@ from inferi_b200.ops import FfnGateUp, GemvQuant, GpuQuantTensor, InferiError
 pytestmark = pytest.mark.gpu
 GOLDEN = np.load(os.path.join(os.path.dirname(__file__), "golden", "blocks.npz"))
 QTYPES = [quant.Q8_0, quant.Q4_K, quant.Q5_K, quant.Q6_K]
-LEGACY = [quant.Q4_0, quant.Q4_1, quant.Q5_0, quant.Q5_1]   # the reference's other GpuQuantTensor variants (op level, generic kernel)
+LEGACY = [quant.Q4_0, quant.Q4_1, quant.Q5_0, quant.Q5_1]   # the reference's other GpuQuantTensor variants (op level, a kernel of their own)
 
 
 def run_gemv(backend, qt, rows, cols, blocks, v):
@@ -94,6 +94,28 @@ def test_legacy_large_vectors(backend, qt, rows, cols):
     k = 126 - int(np.floor(np.log2(max(np.abs(small).max(), np.abs(v).max()))))   # the largest result or element is then at least 2^126
     big = run_gemv(backend, qt, rows, cols, blocks, np.ldexp(v, k))
     assert np.array_equal(big, np.ldexp(small, k))
+
+
+# Q4_1, Q5_1: a weight is d q + m, and m is about -d times half of q's range.  Every weight is formed (rounded once, 2^-24) before it meets the vector; its
+# products and their sums round as in the other formats: 1.0e-7 of the result's norm in all.  Adding up q's and the minimum's products apart,
+# which nearly cancel, cost 3.4e-7 where the vector's mean is far from 0.
+@pytest.mark.parametrize("qt", [quant.Q4_1, quant.Q5_1])
+@pytest.mark.parametrize("mean", [0.0, 30.0])
+def test_legacy_minimums_do_not_cost_accuracy(backend, qt, mean):
+    rows, cols, five = 512, 4096, qt == quant.Q5_1
+    rng = np.random.default_rng(qt)
+    w = 0.02 * rng.standard_normal((rows, cols // 32, 32))
+    d, m = ((w.max(-1) - w.min(-1)) / (31 if five else 15)).astype(np.float16), w.min(-1).astype(np.float16)
+    q = np.clip(np.rint((w - m[..., None]) / d[..., None]), 0, 31 if five else 15).astype(np.uint8)
+    parts = [d[..., None].view(np.uint8), m[..., None].view(np.uint8)]
+    if five:
+        parts.append(np.packbits(q >> 4, axis=-1, bitorder="little"))
+    parts.append((q[..., :16] & 15) | ((q[..., 16:] & 15) << 4))
+    blocks = np.concatenate(parts, -1).reshape(rows, -1)
+    v = (rng.standard_normal(cols) + mean).astype(np.float32)
+    want = (d.astype(np.float64)[..., None] * q + m.astype(np.float64)[..., None]).reshape(rows, cols) @ v.astype(np.float64)
+    got = run_gemv(backend, qt, rows, cols, blocks, v)
+    assert np.linalg.norm(got - want) <= 2e-7 * np.linalg.norm(want)
 
 
 def _shape_case(backend, qt, rows, cols):
