@@ -534,7 +534,7 @@ __device__ __forceinline__ unsigned long long mantissa_pair(uint32_t w, uint32_t
 // ALIGNED: the vector is on a 16-byte boundary
 template <int QT, bool ALIGNED>
 __global__ void __launch_bounds__(LEGACY_WARPS * 32) gemv_legacy_kernel(const uint8_t *__restrict__ w, uint32_t rows, uint32_t nb, uint64_t row_bytes, uint32_t share,
-                                                                        const float *__restrict__ v, float *__restrict__ out) {
+                                                                        const float *v, float *out) {
     using F = Legacy<QT>;
     __shared__ float part[LEGACY_WARPS][LEGACY_ROWS];
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, j = lane >> 2, t = lane & 3;
@@ -549,13 +549,13 @@ __global__ void __launch_bounds__(LEGACY_WARPS * 32) gemv_legacy_kernel(const ui
             now.load(row, row_bytes, b, nb, t);
             const bool in = b < nb;   // (the last step of a row: what lies past its end counts 0)
             const float *x = v + 32 * (in ? b : nb - 1) + 4 * t;
-            float4 a, c;
+            float4 a, c;   // (not through the read-only path: the kernel before may have been writing them while this one started)
             if constexpr (ALIGNED) {
-                a = __ldg(reinterpret_cast<const float4 *>(x));
-                c = __ldg(reinterpret_cast<const float4 *>(x + 16));
+                a = __ldca(reinterpret_cast<const float4 *>(x));
+                c = __ldca(reinterpret_cast<const float4 *>(x + 16));
             } else {
-                a = make_float4(__ldg(x), __ldg(x + 1), __ldg(x + 2), __ldg(x + 3));
-                c = make_float4(__ldg(x + 16), __ldg(x + 17), __ldg(x + 18), __ldg(x + 19));
+                a = make_float4(__ldca(x), __ldca(x + 1), __ldca(x + 2), __ldca(x + 3));
+                c = make_float4(__ldca(x + 16), __ldca(x + 17), __ldca(x + 18), __ldca(x + 19));
             }
             if (!in) {
                 a = c = make_float4(0.f, 0.f, 0.f, 0.f);

@@ -8,7 +8,7 @@ import torch
 import oracle
 from helpers import OP_RTOL, assert_close
 from inferi_b200 import quant
-from inferi_b200.ops import FfnGateUp, GemvQuant, GpuQuantTensor, InferiError
+from inferi_b200.ops import FfnGateUp, GemvQuant, GpuQuantTensor, InferiError, add_assign
 
 pytestmark = pytest.mark.gpu
 GOLDEN = np.load(os.path.join(os.path.dirname(__file__), "golden", "blocks.npz"))
@@ -116,6 +116,25 @@ def test_legacy_minimums_do_not_cost_accuracy(backend, qt, mean):
     want = (d.astype(np.float64)[..., None] * q + m.astype(np.float64)[..., None]).reshape(rows, cols) @ v.astype(np.float64)
     got = run_gemv(backend, qt, rows, cols, blocks, v)
     assert np.linalg.norm(got - want) <= 2e-7 * np.linalg.norm(want)
+
+
+# A launch starts while the kernel before it still runs: the vector is read as that one leaves it, also where it was read before
+@pytest.mark.parametrize("qt,rows,cols", [(quant.Q4_0, 512, 4096), (quant.Q5_1, 12464, 1024)])
+def test_legacy_follows_the_kernel_that_writes_its_vector(backend, qt, rows, cols):
+    m = GpuQuantTensor(backend, qt, rows, cols, quant.random_blocks(qt, rows, cols, seed=3))
+    x, y = (torch.randn(cols, device="cuda", generator=torch.Generator(device="cuda").manual_seed(i)) for i in (1, 2))
+    out, op = torch.zeros(60, rows, device="cuda"), GemvQuant(backend)
+    z = x.clone()
+    for i in range(60):
+        add_assign(backend, x, y)
+        op.launch(out[i], m, x)
+    for i in range(60):
+        z += y
+        want = torch.zeros(rows, device="cuda")
+        torch.cuda.synchronize()
+        op.launch(want, m, z)
+        torch.cuda.synchronize()
+        assert torch.equal(out[i], want), i
 
 
 def _shape_case(backend, qt, rows, cols):
