@@ -374,8 +374,15 @@ __global__ void __launch_bounds__(STREAM_THREADS, 1) gemv_stream_kernel(const __
             held = geo.head;
             t = me * held;
         } else {
-            const uint32_t group = share_group(geo.share, blockIdx.x);
-            make_share(geo.share, geo.seg_pairs, geo.seg_pt, geo.nseg, group, me - geo.share.cta0[group] * geo.P, sh);
+            uint64_t scale = geo.share.scale[0];
+            uint32_t base = 0, number = me;
+            if constexpr (QT == QT_MIXED) {   // (one format, one group)
+                const uint32_t group = share_group(geo.share, blockIdx.x);
+                scale = geo.share.scale[group];
+                base = geo.share.base[group];
+                number -= geo.share.cta0[group] * geo.P;
+            }
+            make_share(geo.share, geo.seg_pairs, geo.seg_pt, geo.nseg, scale, base, number, sh);
             tc.init(sh);
         }
         uint32_t cost = swiglu ? (uint32_t)p.seg[0].row_bytes : geo.seg_cost[0], cost_b = (uint32_t)p.seg[1].row_bytes, cur = 0;

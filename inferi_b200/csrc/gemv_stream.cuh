@@ -170,9 +170,9 @@ __host__ __device__ __forceinline__ uint32_t share_pair(uint32_t at, uint32_t st
 }
 __host__ __device__ __forceinline__ uint32_t share_byte(uint64_t scale, uint32_t me) { return (uint32_t)((me * scale) >> 32); }
 __device__ __forceinline__ uint32_t share_group(const ShareGeom &g, uint32_t cta) { return cta >= g.cta0[2] ? 2u : (cta >= g.cta0[1] ? 1u : 0u); }
-// `me`: the pipeline's number among its group's
-__device__ __forceinline__ void make_share(const ShareGeom &g, const uint32_t (&pairs)[3], const uint32_t (&pt)[3], uint32_t nseg, uint32_t group, uint32_t me, Share &sh) {
-    const uint32_t lo = g.base[group] + share_byte(g.scale[group], me), hi = g.base[group] + share_byte(g.scale[group], me + 1);
+// `scale`, `base`: the group's; `me`: the pipeline's number among its group's
+__device__ __forceinline__ void make_share(const ShareGeom &g, const uint32_t (&pairs)[3], const uint32_t (&pt)[3], uint32_t nseg, uint64_t scale, uint32_t base, uint32_t me, Share &sh) {
+    const uint32_t lo = base + share_byte(scale, me), hi = base + share_byte(scale, me + 1);
     sh.nseg = nseg;
     sh.a0 = share_pair(lo, g.start[0], g.cost16[0], g.inv[0], pairs[0]);
     sh.b0 = share_pair(hi, g.start[0], g.cost16[0], g.inv[0], pairs[0]);
