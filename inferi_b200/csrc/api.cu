@@ -65,11 +65,20 @@ void host_populate(void *p, size_t nbytes) {
     constexpr int POPULATE_WRITE = 23;   // MADV_POPULATE_WRITE
     madvise((void *)a, (uintptr_t)p + nbytes - a, POPULATE_WRITE);
 }
+// What the calling thread does between these is not held against a capture that another stream of the process is in (its capture mode would refuse it, and end the
+// capture).
+struct BesideCaptures {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
 int32_t read_back(ib_ctx *ctx, cudaStream_t s, void *dst, const void *src, size_t nbytes) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (nbytes >= STAGE_LEAST && nbytes <= STAGE_BYTES && host_pageable(dst) && cudaStreamIsCapturing(s, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+    if (ctx->stage_host && nbytes >= STAGE_LEAST && nbytes <= STAGE_BYTES && host_pageable(dst) && cudaStreamIsCapturing(s, &capture) == cudaSuccess &&
+        capture == cudaStreamCaptureStatusNone) {
         std::unique_lock<std::mutex> mine(ctx->stage_lock, std::try_to_lock);   // another thread has it: CUDA's way
-        if (mine && (ctx->stage_host || cudaMallocHost(&ctx->stage_host, STAGE_BYTES) == cudaSuccess)) {
+        if (mine) {
+            BesideCaptures beside;
             IB_CHECK_CUDA(cudaMemcpyAsync(ctx->stage_host, src, nbytes, cudaMemcpyDeviceToHost, s));
             host_populate(dst, nbytes);
             IB_CHECK_CUDA(cudaStreamSynchronize(s));
@@ -130,6 +139,10 @@ int32_t ib_ctx_create(int32_t device, ib_ctx **out) {
         cudaFreeHost(ctx->err_host);
         delete ctx;
         return set_error(IB_ERR_CUDA, "allocating the tile counters failed: %s", cudaGetErrorString(ce));
+    }
+    if (cudaMallocHost(&ctx->stage_host, STAGE_BYTES) != cudaSuccess) {   // (copies then go CUDA's way)
+        ctx->stage_host = nullptr;
+        cudaGetLastError();
     }
     *out = ctx;
     return IB_OK;

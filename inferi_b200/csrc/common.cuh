@@ -91,7 +91,7 @@ struct ib_ctx {
     void *tc_scratch = nullptr;
     size_t tc_scratch_bytes = 0;
     uint32_t tc_pass = 0xFFFFFFFFu;   // the longest pass (tokens) that the device has had room for
-    // pinned staging of copies to the host (read_back), made by the first one
+    // pinned staging of copies to the host (read_back); null: no room for it
     void *stage_host = nullptr;
     std::mutex stage_lock;
     // limit of every wait inside a kernel (on a shared-memory barrier, on another rank's arrival); ib_ctx_set_wait_limit

@@ -63,3 +63,30 @@ def test_threads_share_one_context():
         t.join()
     b.close()
     assert not wrong
+
+
+@pytest.mark.parametrize("threaded", [False, True])
+def test_a_copy_beside_a_capture(threaded):
+    """A context's first copy, while another stream of the process is being captured: it arrives, and the capture goes on."""
+    b = Backend(0)
+    src, x = torch.arange(130000, dtype=torch.float32, device="cuda"), torch.zeros(8, device="cuda")
+    out, other, graph = np.zeros(130000, np.float32), torch.cuda.Stream(), torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+
+    def copy():
+        d2h(b, out.ctypes.data, src, out.nbytes, other.cuda_stream)
+
+    with torch.cuda.graph(graph, stream=torch.cuda.Stream(), capture_error_mode="global"):
+        x += 1
+        if threaded:
+            t = threading.Thread(target=copy)
+            t.start()
+            t.join()
+        else:
+            copy()
+        x += 1
+    assert np.array_equal(out, src.cpu().numpy())
+    graph.replay()
+    torch.cuda.synchronize()
+    assert (x == 2).all()
+    b.close()
