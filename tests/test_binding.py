@@ -1,4 +1,6 @@
 """The compiled way to the op launches (csrc/binding.cpp) against the Python way behind it: the same results, the same refusals."""
+import importlib
+
 import numpy as np
 import pytest
 import torch
@@ -10,6 +12,24 @@ from inferi_b200.ops import AttnParams, FusedAttention, GemmQuant, GemvQuant, Gp
 class PythonOnly:
     """Takes no call"""
     gemv = gemm = rms_norm = rope = silu = add = attention = argmax = sample = staticmethod(lambda *a: -1)
+
+
+class Recorded:
+    """The compiled binding, and what its entries answered: name -> statuses"""
+    def __init__(self):
+        self.binding, self.answers = importlib.import_module("inferi_b200._binding"), {}
+
+    def __getattr__(self, name):
+        entry = getattr(self.binding, name)
+
+        def call(*args):
+            rc = entry(*args)
+            self.answers.setdefault(name, []).append(rc)
+            return rc
+        return call
+
+
+ENTRIES = {"gemv", "gemm", "rms_norm", "rope", "silu", "add", "attention", "argmax", "sample"}
 
 
 class Tagged(torch.Tensor):
@@ -81,14 +101,21 @@ def calls(b, dev, wrap=lambda t: t):
 
 @pytest.mark.gpu
 def test_both_ways_launch_the_same(backend, monkeypatch):
-    """Bit for bit, on the default stream and on another one, with plain tensors and with a subclass (which takes the Python way)"""
+    """Bit for bit, on the default stream and on another one, with plain tensors (which the binding takes: every entry launches) and with a subclass
+    (which takes the Python way)"""
+    recorded = Recorded()
+    assert ops._fast is recorded.binding
+    monkeypatch.setattr(ops, "_fast", recorded)
     fast = {n: f().cpu() for n, f in calls(backend, "cuda").items()}
     side = torch.cuda.Stream()
     side.wait_stream(torch.cuda.current_stream())
     with torch.cuda.stream(side):
         aside = {n: f() for n, f in calls(backend, "cuda").items()}
     side.synchronize()
+    assert {n: set(rc) for n, rc in recorded.answers.items()} == {n: {0} for n in ENTRIES}
+    recorded.answers.clear()
     tagged = {n: f().cpu().as_subclass(torch.Tensor) for n, f in calls(backend, "cuda", lambda t: t.as_subclass(Tagged)).items()}
+    assert {n: set(rc) for n, rc in recorded.answers.items()} == {n: {-1} for n in ENTRIES}
     monkeypatch.setattr(ops, "_fast", PythonOnly)
     slow = {n: f().cpu() for n, f in calls(backend, "cuda").items()}
     for n in fast:
@@ -122,6 +149,7 @@ def test_both_ways_refuse_the_same(backend, monkeypatch):
             out.append((type(e.value), str(e.value)))
         return out
 
+    assert ops._fast is importlib.import_module("inferi_b200._binding")
     fast = answers()
     monkeypatch.setattr(ops, "_fast", PythonOnly)
     assert answers() == fast
