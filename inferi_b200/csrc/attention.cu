@@ -5,11 +5,11 @@
 // Semantics follow `run_cpu` (:191-245): score = q.k / sqrt(head_size), softmax over positions 0..=pos, weighted
 // sum of V.  Cache rows are [position, kv_dim] (fused_attention.rs:107-108), f32 as in the reference or f16.
 //
-// One CTA per (kv head, position slice): the slice's K and V rows are read once and used for all kv_mul query
-// heads of the group (the reference reads them kv_mul times, one workgroup per query head).  Every CTA leaves an
-// un-normalised partial (max, sum, accumulator); the last CTA of a kv head to arrive merges the partials — no CTA
-// ever waits for another.  The split count is derived from the position on the device, so the same launch (and
-// the same CUDA graph node) serves every context length.
+// A group of up to four query heads of one kv head shares the slices' K and V rows (the reference reads them once per query head, one workgroup each);
+// eight heads are two groups, which read the same rows.  One CTA per (group, position slice) leaves an un-normalised partial (max, sum,
+// accumulator): many slices in global memory, where the last CTA of a group to arrive merges them and none waits for another; few slices
+// in the shared memory of the first CTA of their cluster, whose barrier they meet at (attention_group.cuh).  The split follows from the
+// position on the device, so the same launch (and the same CUDA graph node) serves every context length of its regime.
 #include "attention_group.cuh"
 
 namespace ib {
@@ -19,22 +19,25 @@ size_t attn_scratch_bytes(const ib_attn_params &p, uint32_t max_splits) {
     return n_kv * max_splits * p.kv_mul * (p.head_size + 2) * sizeof(float);
 }
 
+// The merging CTA keeps the weights of ATTN_MAX_SLICES slices.  (Head size 64: half as many.  Only one to three groups of heads could use more; whether
+// they gain by it has not been measured.)
+static uint32_t attn_slice_limit(const ib_attn_params &p) { return 2 * p.head_size < ATTN_MAX_SLICES ? 2 * p.head_size : ATTN_MAX_SLICES; }
+
 uint32_t attn_max_splits(const ib_ctx *ctx, const ib_attn_params &p) {
     const uint32_t groups = attn_groups(p);
     uint32_t s = (uint32_t)(ctx->sm_count * 3) / (groups ? groups : 1);   // three CTAs fit one SM: one wave
     if (s < 1) s = 1;
-    if (s > 256) s = 256;             // (the merging CTA keeps so many weights)
-    if (s > 2 * p.head_size) s = 2 * p.head_size;
-    return s;
+    const uint32_t most = attn_slice_limit(p);
+    return s < most ? s : most;
 }
 
 // CTAs per cluster, one cluster per kv head.  Short: 8 while that is three (head size 128: two) on every SM, and from there on as many as fit
 // with one per SM (head size 64, 400 positions: 26 kv heads 4.8 us in clusters of 8, 6.6 in clusters of 4; 64 heads 8.1 and 6.8).
 // Middle: its CTAs need an SM each and their clusters a GPC with so many free ones; on more than two thirds of the SMs some clusters wait
 // for others (12 kv heads x 8 CTAs fit; 16 x 8 take twice the time: 13.4 us against 8.9 as 16 x 4 at 2048 positions).  Fewer than 4 CTAs per kv head: no middle regime.
-static uint32_t gqa4_cluster_ctas(const ib_ctx *ctx, const ib_attn_params &p, uint32_t regime) {
+static uint32_t attn_cluster_ctas(const ib_ctx *ctx, const ib_attn_params &p, uint32_t regime) {
     const uint32_t n_kv = attn_groups(p), room = (uint32_t)ctx->sm_count * 2 / (regime == ATTN_MIDDLE ? 3 : 2);
-    uint32_t c = GQA4_CLUSTER_MAX;
+    uint32_t c = ATTN_CLUSTER_MAX;
     if (regime == ATTN_SHORT && c * n_kv <= (p.head_size == 128 ? 2 : 3) * (uint32_t)ctx->sm_count) return c;
     while (c > 1 && c * n_kv > room) c /= 2;
     return regime == ATTN_MIDDLE && (c < 4 || c * n_kv > room) ? 0u : c;
@@ -61,8 +64,8 @@ static uint32_t gqa4_cluster_ctas(const ib_ctx *ctx, const ib_attn_params &p, ui
 uint32_t attn_regime_positions(const ib_ctx *ctx, const AttnLaunch &a, uint32_t regime) {
     if (ctx->sm_count == 0) return 0u;
     const bool has_middle = a.kv_dtype == IB_KV_F16 && a.p.kv_mul >= ATTN_GROUP;
-    const uint32_t n_kv = attn_groups(a.p), middle = has_middle ? gqa4_cluster_ctas(ctx, a.p, ATTN_MIDDLE) : 0u;
-    const uint32_t c = regime == ATTN_MIDDLE ? middle : gqa4_cluster_ctas(ctx, a.p, regime);
+    const uint32_t n_kv = attn_groups(a.p), middle = has_middle ? attn_cluster_ctas(ctx, a.p, ATTN_MIDDLE) : 0u;
+    const uint32_t c = regime == ATTN_MIDDLE ? middle : attn_cluster_ctas(ctx, a.p, regime);
     const bool wide = a.p.head_size == 128;
     if (regime == ATTN_MIDDLE) return c * (wide ? (c < 8 ? 256 : (n_kv <= 4 ? 320 : (n_kv <= 8 ? 300 : 384))) : (c < 8 ? 512 : (n_kv <= 8 ? 800 : 1400)));
     if (!has_middle) return c * (wide ? (a.kv_dtype == IB_KV_F16 ? 48 : (a.p.kv_mul > ATTN_GROUP ? 16 : 32)) : (a.kv_dtype == IB_KV_F16 ? 64 : 48));
@@ -74,11 +77,11 @@ static bool attn_aligned(const float *q, const float *out) { return ((uintptr_t)
 
 template <int HS, int KVM, typename T, uint32_t REGIME, bool ALIGNED = true>
 static int32_t launch_group(ib_ctx *ctx, cudaStream_t s, const AttnArgs &args, dim3 grid) {
-    constexpr uint32_t smem = gqa4_smem_floats(HS, KVM, REGIME) * sizeof(float);
+    constexpr uint32_t smem = attn_smem_floats(HS, KVM, REGIME) * sizeof(float);
     static_assert(smem + 4096 <= 49152, "dynamic and static shared memory without opting in");
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
-    cfg.blockDim = dim3(gqa4_warps(HS, REGIME) * 32);
+    cfg.blockDim = dim3(attn_warps(HS, REGIME) * 32);
     cfg.dynamicSmemBytes = smem;
     cfg.stream = s;
     cudaLaunchAttribute attr[2];
@@ -119,8 +122,7 @@ int32_t launch_attention(ib_ctx *ctx, cudaStream_t s, const AttnLaunch &a) {
     const uint32_t n_kv = p.n_heads / p.kv_mul;
     IB_REQUIRE(p.kv_dim == n_kv * p.head_size, "attention: kv_dim=%u != n_kv_heads*head_size=%u", p.kv_dim, n_kv * p.head_size);
     IB_REQUIRE(a.pos_ptr || p.pos < p.seq_len, "attention: pos=%u outside the cache of %u rows", p.pos, p.seq_len);
-    IB_REQUIRE(a.max_splits >= 1 && a.max_splits <= 2 * p.head_size && a.max_splits <= 256, "attention: %u position slices exceed what the merge step holds (%u)",
-               a.max_splits, 2 * p.head_size < 256 ? 2 * p.head_size : 256);
+    IB_REQUIRE(a.max_splits >= 1 && a.max_splits <= attn_slice_limit(p), "attention: %u position slices (1 to %u)", a.max_splits, attn_slice_limit(p));
     IB_REQUIRE(((uintptr_t)a.k_cache % 16) == 0 && ((uintptr_t)a.v_cache % 16) == 0, "attention: the caches must be 16-byte aligned");
     if (p.head_size != 64 && p.head_size != 128) return set_error(IB_ERR_UNSUPPORTED, "attention: head_size=%u (supported: 64, 128)", p.head_size);
     if (p.kv_mul != 1 && p.kv_mul != 2 && p.kv_mul != 4 && p.kv_mul != 8) return set_error(IB_ERR_UNSUPPORTED, "attention: kv_mul=%u (supported: 1, 2, 4, 8)", p.kv_mul);
@@ -135,9 +137,9 @@ int32_t launch_attention(ib_ctx *ctx, cudaStream_t s, const AttnLaunch &a) {
             if (p.pos < attn_regime_positions(ctx, a, r)) regime = r;
     }
     uint32_t splits = a.max_splits, per;
-    if (regime != ATTN_LONG) args.cluster = splits = gqa4_cluster_ctas(ctx, p, regime);
+    if (regime != ATTN_LONG) args.cluster = splits = attn_cluster_ctas(ctx, p, regime);
     if (!a.pos_ptr) {   // with a host-known position only the slices that will do work are launched
-        gqa4_plan(p.pos + 1, a.max_splits, args.cluster, gqa4_warps(p.head_size, regime), p.kv_mul, splits, per);
+        attn_plan(p.pos + 1, a.max_splits, args.cluster, attn_warps(p.head_size, regime), p.kv_mul, splits, per);
         if (regime != ATTN_LONG) args.cluster = splits;
     }
     const dim3 grid(attn_groups(p), splits);

@@ -22,7 +22,7 @@ namespace ib {
 constexpr uint32_t ATTN_GROUP = 4;   // query heads of a group, at most
 __host__ __device__ constexpr uint32_t attn_groups(const ib_attn_params &p) { return p.n_heads / (p.kv_mul < ATTN_GROUP ? p.kv_mul : ATTN_GROUP); }
 
-constexpr uint32_t GQA4_ROWS_PER_WARP_STEP = 8;
+constexpr uint32_t ATTN_ROWS_PER_WARP_STEP = 8;
 // Three ways to split a kv head's positions, by context length:
 //  * short: the slices are the CTAs of one thread-block cluster, 4 warps each.  They leave their partials in the shared memory of the
 //    cluster's first CTA (distributed shared memory) and meet at the cluster barrier; the first CTA merges from its own shared
@@ -35,19 +35,19 @@ constexpr uint32_t GQA4_ROWS_PER_WARP_STEP = 8;
 //    128: this plan 8.7 / 9.2 / 12.0 / 17.6, 32 positions each throughout 8.2 / 9.3 / 12.0 / 17.7, at least 256 each 9.8 / 9.9 / 13.0 / 17.7
 //    (the merge fetches sixteen slices per L2 round trip; when it fetched eight, 32 each cost 12.6 at 2048 where the plan cost 9.2).
 // Clusters have at most 8 CTAs: eight clusters of 16 - one per kv head of the Llama-3 models - do not all fit the GPU at once.
-constexpr uint32_t GQA4_CLUSTER_MAX = 8;
-__host__ __device__ constexpr int gqa4_warps(uint32_t hs, uint32_t regime) { return regime != ATTN_MIDDLE ? ATTN_WARPS : (hs == 128 ? 8 : 16); }   // (head size 128 needs 196 registers a thread)
-constexpr uint32_t GQA4_MIN_PER_SPLIT = ATTN_WARPS * GQA4_ROWS_PER_WARP_STEP, GQA4_KNEE = 16, GQA4_KNEE_PER = 128;
-constexpr uint32_t GQA4_ALONE = 64;   // rows of one or two heads that one CTA is as fast with as two that merge (60 rows, 16 x 1 heads of 128: 2.4 us, 2.7 as two)
-__host__ __device__ __forceinline__ void gqa4_plan(uint32_t total, uint32_t max_splits, uint32_t cluster, uint32_t warps, uint32_t heads, uint32_t &nsplit, uint32_t &per) {
+constexpr uint32_t ATTN_CLUSTER_MAX = 8, ATTN_MAX_SLICES = 256;
+__host__ __device__ constexpr int attn_warps(uint32_t hs, uint32_t regime) { return regime != ATTN_MIDDLE ? ATTN_WARPS : (hs == 128 ? 8 : 16); }   // (head size 128 needs 196 registers a thread)
+constexpr uint32_t ATTN_MIN_PER_SPLIT = ATTN_WARPS * ATTN_ROWS_PER_WARP_STEP, ATTN_KNEE = 16, ATTN_KNEE_PER = 128;
+constexpr uint32_t ATTN_ALONE = 64;   // rows of one or two heads that one CTA is as fast with as two that merge (60 rows, 16 x 1 heads of 128: 2.4 us, 2.7 as two)
+__host__ __device__ __forceinline__ void attn_plan(uint32_t total, uint32_t max_splits, uint32_t cluster, uint32_t warps, uint32_t heads, uint32_t &nsplit, uint32_t &per) {
     if (cluster) {
-        nsplit = (total + warps * GQA4_ROWS_PER_WARP_STEP - 1) / (warps * GQA4_ROWS_PER_WARP_STEP);
+        nsplit = (total + warps * ATTN_ROWS_PER_WARP_STEP - 1) / (warps * ATTN_ROWS_PER_WARP_STEP);
         if (nsplit > cluster) nsplit = cluster;
-        if (heads <= 2 && total <= GQA4_ALONE) nsplit = 1;
+        if (heads <= 2 && total <= ATTN_ALONE) nsplit = 1;
         per = (total + nsplit - 1) / nsplit;
         nsplit = (total + per - 1) / per;
     } else {
-        attn_split_plan(total, max_splits, nsplit, per, GQA4_MIN_PER_SPLIT, GQA4_KNEE, GQA4_KNEE_PER);
+        attn_split_plan(total, max_splits, nsplit, per, ATTN_MIN_PER_SPLIT, ATTN_KNEE, ATTN_KNEE_PER);
     }
 }
 
@@ -116,10 +116,10 @@ __device__ __forceinline__ void store_scaled(float *p, const float (&o)[N], floa
 
 // A warp's accumulators meet in shared memory, by row groups (lanes of one cache row) where there is room: adding the groups up with shuffles
 // first is 64 instructions per round that every launch fetches and runs once.  (Many warps: they are added up first.)
-__host__ __device__ constexpr uint32_t gqa4_groups(uint32_t hs, uint32_t regime) { return regime == ATTN_MIDDLE ? 1 : 256 / hs; }
+__host__ __device__ constexpr uint32_t attn_row_groups(uint32_t hs, uint32_t regime) { return regime == ATTN_MIDDLE ? 1 : 256 / hs; }
 // floats of dynamic shared memory: the warps' accumulators, and with clusters the slices' partials (in the first CTA)
-__host__ __device__ constexpr uint32_t gqa4_smem_floats(uint32_t hs, uint32_t kvm, uint32_t regime) {
-    return gqa4_warps(hs, regime) * gqa4_groups(hs, regime) * kvm * hs + (regime != ATTN_LONG ? GQA4_CLUSTER_MAX * kvm * (hs + 2) : 0);
+__host__ __device__ constexpr uint32_t attn_smem_floats(uint32_t hs, uint32_t kvm, uint32_t regime) {
+    return attn_warps(hs, regime) * attn_row_groups(hs, regime) * kvm * hs + (regime != ATTN_LONG ? ATTN_CLUSTER_MAX * kvm * (hs + 2) : 0);
 }
 // The caller's output: in pairs, or one by one where it is aligned to 4 bytes only
 template <int N>
@@ -160,10 +160,10 @@ constexpr int attn_log2(int n) { return n <= 1 ? 0 : 1 + attn_log2(n / 2); }
 
 // ALIGNED: q and out are on 16-byte boundaries.  (A run-time choice made launches of 200 to 250 positions of 8 x 4 heads of 128 0.2 of 3.7 us slower: code.)
 template <int HS, int KVM, typename T, uint32_t REGIME, bool ALIGNED>
-__global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MIDDLE ? 1 : 3) attn_group_kernel(const AttnArgs a) {
+__global__ void __launch_bounds__(attn_warps(HS, REGIME) * 32, REGIME == ATTN_MIDDLE ? 1 : 3) attn_group_kernel(const AttnArgs a) {
     constexpr int EPL = 8;
     constexpr bool CLUSTER = REGIME != ATTN_LONG;
-    constexpr int W = gqa4_warps(HS, REGIME), THREADS = W * 32;
+    constexpr int W = attn_warps(HS, REGIME), THREADS = W * 32;
     constexpr int L = HS / EPL;          // lanes per cache row
     constexpr int RPW = 32 / L;          // rows per warp step
     constexpr int STEPS = sizeof(T) == 2 ? HS / 32 : 2;   // steps per warp iteration
@@ -171,7 +171,7 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
     constexpr int N = STEPS * KVM;       // partial scores per lane and iteration; L / N lanes end up with the same complete one
     static_assert(N <= L && (N & (N - 1)) == 0, "lane layout");
     constexpr int DUP = attn_log2(L / N), FROM_S = 1 << (DUP + attn_log2(KVM));   // the lane's bits: [row group][step][head][copy]
-    constexpr int G = gqa4_groups(HS, REGIME);
+    constexpr int G = attn_row_groups(HS, REGIME);
     static_assert(G == 1 || G == RPW, "row groups of a warp");
     extern __shared__ __align__(16) float sm_acc[];   // [W][G][KVM][HS]
     float *sm_cl = sm_acc + W * G * KVM * HS;         // clusters: [slices][KVM][HS + 2]
@@ -196,7 +196,7 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
     const uint32_t kvh = blockIdx.x, split = blockIdx.y;   // (kvh: the group's number)
     const uint32_t total = (a.pos_ptr ? *a.pos_ptr : a.p.pos) + 1;
     uint32_t nsplit, per;
-    gqa4_plan(total, a.max_splits, CLUSTER ? a.cluster : 0u, W, KVM, nsplit, per);
+    attn_plan(total, a.max_splits, CLUSTER ? a.cluster : 0u, W, KVM, nsplit, per);
     if (split >= nsplit) {
         if constexpr (CLUSTER) {
             cluster.barrier_wait();
@@ -434,15 +434,15 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
             cluster.sync();
             if (split != 0 || !has) return;   // (whole warps: a warp has outputs or none)
             // (the lanes share out the slices' weights like the warps' above)
-            const uint32_t sl = lane & (GQA4_CLUSTER_MAX - 1);
+            const uint32_t sl = lane & (ATTN_CLUSTER_MAX - 1);
             const float2 ml = sl < nsplit ? *reinterpret_cast<const float2 *>(&sm_cl[(sl * KVM + m_out) * slot + HS]) : make_float2(-INFINITY, 0.f);
             float cm = ml.x;
 #pragma unroll
-            for (int x = 1; x < (int)GQA4_CLUSTER_MAX; x <<= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, x));
+            for (int x = 1; x < (int)ATTN_CLUSTER_MAX; x <<= 1) cm = fmaxf(cm, __shfl_xor_sync(0xffffffffu, cm, x));
             const float ws = merge_weight(ml.x, cm);
             float lsum = ws * ml.y, acc[PER];
 #pragma unroll
-            for (int x = 1; x < (int)GQA4_CLUSTER_MAX; x <<= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, x);
+            for (int x = 1; x < (int)ATTN_CLUSTER_MAX; x <<= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, x);
 #pragma unroll
             for (int e = 0; e < PER; e++) acc[e] = 0.f;
             for (uint32_t s = 0; s < nsplit; s++) add_scaled(acc, __shfl_sync(0xffffffffu, ws, s), sm_cl + (s * KVM + m_out) * slot + d_out);
@@ -470,9 +470,9 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
     // the weights, which then lie in shared memory (the accumulators there have been used); the accumulators come sixteen slices per
     // L2 round trip, the first of them requested ahead of the weights.  Eight slices at a time with their pairs and a running maximum:
     // 21.4 us instead of 17.9 at 16384 positions of 8 heads of 128, 18.9 instead of 13.9 at 20000 of 64.
-    constexpr uint32_t MAX_SLICES = 256, AT_ONCE = 16;   // (the launcher's limit of slices)
-    static_assert(W * MAX_SLICES <= gqa4_smem_floats(HS, KVM, REGIME), "the weights fit the accumulators' place");
-    float *sm_w = sm_acc + warp * MAX_SLICES;
+    constexpr uint32_t AT_ONCE = 16;
+    static_assert(W * ATTN_MAX_SLICES <= attn_smem_floats(HS, KVM, REGIME), "the weights fit the accumulators' place");
+    float *sm_w = sm_acc + warp * ATTN_MAX_SLICES;
     const float *mine = a.scratch + (size_t)kvh * a.max_splits * KVM * HS + m_out * HS + d_out;
     float dat[AT_ONCE][PER];
     auto fetch = [&](uint32_t s0) {
@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(gqa4_warps(HS, REGIME) * 32, REGIME == ATTN_MI
         }
     };
     fetch(0);
-    constexpr uint32_t PAIRS = MAX_SLICES / 32;
+    constexpr uint32_t PAIRS = ATTN_MAX_SLICES / 32;
     float2 ml[PAIRS];
     float cm = -INFINITY;
 #pragma unroll
