@@ -58,8 +58,8 @@ static uint32_t attn_cluster_ctas(const ib_ctx *ctx, const ib_attn_params &p, ui
 // The middle regime's ends are those of the token graph (for head size 64 beyond 3000 positions: the crossing back to back, moved by that margin).  Launches outside it, which take the same ones, would cross over earlier by the
 // figures above: up to 0.9 us of 8 between 4000 and 6400 positions of up to 8 heads of 64, 0.7 of 7 below 2560 positions of 2 to 4 heads of 128.
 // Groups of one or two heads and the f32 cache have no middle regime; short / long, us: f16, head size 128, 8 x 2 heads 2.9 / 3.7 at 200 positions, 4.3 / 4.1 at
-// 450, 16 x 1 4.3 / 4.5 at 450 (6.1 / 5.6 at 900); head size 64, 8 x 2 3.2 / 3.4 at 450 (5.6 / 4.7 at 900).  f32, head size 128, 8 x 4 4.6 / 5.0 at 200,
-// 6.4 / 5.1 at 450, 8 x 8 3.7 / 4.1 at 60, 6.0 / 5.0 at 200, 16 x 1 4.0 / 4.7 at 200, 5.7 / 5.4 at 450; head size 64, 8 x 4 2.9 / 3.5 at 200, 4.2 / 4.0 at 450.
+// 450, 16 x 1 4.3 / 4.5 at 450 (6.1 / 5.6 at 900); head size 64, 8 x 2 3.2 / 3.6 at 500 (4.2 / 3.9 at 600).  f32, head size 128, 8 x 4 4.6 / 5.0 at 200,
+// 6.4 / 5.1 at 450, 8 x 8 3.7 / 4.1 at 60, 6.0 / 5.0 at 200, 16 x 1 4.0 / 4.2 at 200, 4.6 / 4.3 at 260; head size 64, 8 x 4 2.9 / 3.5 at 200, 4.2 / 4.0 at 450, 8 x 1 3.8 / 3.8 at 380.
 // (2 to 4 heads of 128 end at 2560, 8 at 2400: the latter was measured in the graph up to its crossing, the former at 1600 only.)
 uint32_t attn_regime_positions(const ib_ctx *ctx, const AttnLaunch &a, uint32_t regime) {
     if (ctx->sm_count == 0) return 0u;

@@ -3,7 +3,7 @@
 // of one kv head (eight are two groups, which read the same rows: the second time from L2), head size 64 or 128, an f16 or f32 cache.
 // Built for a short critical path at small contexts and for few instructions per cache row at long ones:
 //  * a lane holds 8 elements of a cache row and the matching 8 elements of the group's query vectors: 16 lanes a row of 128, 8 lanes a row of 64;
-//    a warp step covers 8 rows (4 of f32 at head size 128: their registers);
+//    a warp iteration covers 8 rows (4 of f32 at head size 128: their registers; more of one or two heads, attn_steps);
 //  * the per-lane partial scores of the step go through a halving exchange (each shuffle moves one value and
 //    leaves half as many to reduce) instead of a butterfly per score: afterwards every lane owns exactly one
 //    (row, head) score - two or four lanes the same one where a step has fewer scores than lanes - so exp() is evaluated once per score;
@@ -37,6 +37,13 @@ constexpr uint32_t ATTN_ROWS_PER_WARP_STEP = 8;
 // Clusters have at most 8 CTAs: eight clusters of 16 - one per kv head of the Llama-3 models - do not all fit the GPU at once.
 constexpr uint32_t ATTN_CLUSTER_MAX = 8, ATTN_MAX_SLICES = 256;
 __host__ __device__ constexpr int attn_warps(uint32_t hs, uint32_t regime) { return regime != ATTN_MIDDLE ? ATTN_WARPS : (hs == 128 ? 8 : 16); }   // (head size 128 needs 196 registers a thread)
+// Steps of a warp iteration: what of a slice is in flight, twice.  Four heads have registers for 8 rows (f32 at head size 128: 4); fewer heads need more rows, or
+// long contexts wait for them (us, with the 8 rows of four heads / so: f16, head size 64, 30000 positions, 16 x 1 heads 36.2 / 26.3, 16 x 2 38.2 / 26.9, 5000 positions
+// 9.8 / 8.3, 10.3 / 8.7; f32, 30000 positions of 16 x 1, head size 64 42.5 / 40.2, 128 78.6 / 73.9).  Eight steps of one f16 head: 25.0, but 11.1 / 10.5 at 8000.
+__host__ __device__ constexpr int attn_steps(int hs, int heads, int bytes, uint32_t regime) {
+    if (regime == ATTN_LONG && (bytes == 2 ? hs == 64 && heads <= 2 : heads == 1)) return 4;
+    return bytes == 2 ? hs / 32 : 2;
+}
 constexpr uint32_t ATTN_MIN_PER_SPLIT = ATTN_WARPS * ATTN_ROWS_PER_WARP_STEP, ATTN_KNEE = 16, ATTN_KNEE_PER = 128;
 constexpr uint32_t ATTN_ALONE = 64;   // rows of one or two heads that one CTA is as fast with as two that merge (60 rows, 16 x 1 heads of 128: 2.4 us, 2.7 as two)
 __host__ __device__ __forceinline__ void attn_plan(uint32_t total, uint32_t max_splits, uint32_t cluster, uint32_t warps, uint32_t heads, uint32_t &nsplit, uint32_t &per) {
@@ -166,7 +173,7 @@ __global__ void __launch_bounds__(attn_warps(HS, REGIME) * 32, REGIME == ATTN_MI
     constexpr int W = attn_warps(HS, REGIME), THREADS = W * 32;
     constexpr int L = HS / EPL;          // lanes per cache row
     constexpr int RPW = 32 / L;          // rows per warp step
-    constexpr int STEPS = sizeof(T) == 2 ? HS / 32 : 2;   // steps per warp iteration
+    constexpr int STEPS = attn_steps(HS, KVM, sizeof(T), REGIME);   // steps per warp iteration
     constexpr int ROWS = STEPS * RPW;
     constexpr int N = STEPS * KVM;       // partial scores per lane and iteration; L / N lanes end up with the same complete one
     static_assert(N <= L && (N & (N - 1)) == 0, "lane layout");
