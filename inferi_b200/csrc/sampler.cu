@@ -43,7 +43,8 @@ namespace cg = cooperative_groups;
 constexpr int SAMPLE_THREADS = 1024, SAMPLE_WARPS = SAMPLE_THREADS / 32;
 constexpr uint32_t SAMPLE_MAX_CLUSTER = 16;
 // Vocabularies up to this size are one CTA's work: its barriers are a third of a cluster's, and a pass over them is four elements a thread.
-// us per call, 1 / 16 CTAs: 512 tokens 12.4 / 20.5 (flat 20.6 / 28.7), 4096 16.4 / 20.5 (39.6 / 43.1), 8192 18.8 / 20.5, 32000 39.0 / 22.6.
+// us per call, 1 / 16 CTAs, top-p: 512 tokens 7.2 / 10.2, 2048 9.9 / 13.3, 4096 9.6 / 10.7, 8192 11.1 / 10.5, 16384 17.2 / 11.2, 32000 27.4 / 11.9; multinomial:
+// 512 3.7 / 6.0, 4096 5.1 / 6.2, 8192 6.4 / 6.2.
 constexpr uint32_t SAMPLE_ONE_CTA = 4096;
 constexpr uint32_t SAMPLE_BINS = 2048, SAMPLE_TOP_SHIFT = 19;   // p <= 1: bits(p) >> 19 <= 0x7F0
 constexpr uint32_t SAMPLE_LIST = 4096;                          // elements of a bin that are ordered in shared memory
@@ -305,9 +306,10 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const float *__r
         // number of them: a warp's reads of one element each then fall to different banks.
         const uint32_t per = ((len + SAMPLE_THREADS - 1) / SAMPLE_THREADS) | 1u, a = min(len, tid * per), b = min(len, a + per);
         unsigned long long mine = 0ull, total, ahead = 0ull;
-        for (uint32_t base = a; base < b; base += AT_ONCE + 1) {
+        constexpr uint32_t TOGETHER = AT_ONCE == 1 ? 1 : AT_ONCE + 1;   // (places and one more: the odd number)
+        for (uint32_t base = a; base < b; base += TOGETHER) {
 #pragma unroll
-            for (uint32_t k = 0; k < AT_ONCE + 1; k++)
+            for (uint32_t k = 0; k < TOGETHER; k++)
                 if (base + k < b) {
                     const float p = __fdiv_rn(P[base + k], sum);
                     P[base + k] = p;
@@ -418,8 +420,16 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const float *__r
             }
         if (tid == 0) S.total = total;
         __syncthreads();
-        // (no candidates, or a bound that two bins may hold: the general way)
-        if (tid < C) cluster.map_shared_rank(&S, tid)->plan = make_uint4(found ? S.prefix : NO_BIN, S.bin_hi, total != 0ull && S.bin_lo == S.bin_hi ? 1u : 0u, 0u);
+        // (no candidates, a bound that two bins may hold, or more elements than the list has room for - at least a bin's mass over its largest p: the general way)
+        if (tid < C) {
+            const uint32_t bin0 = found ? S.prefix : NO_BIN, bin1 = S.bin_hi;
+            bool plain = total != 0ull && S.bin_lo == bin1;
+            if (plain) {
+                auto least = [](unsigned long long mass, uint32_t bin) { return (float)mass / (float)mass_of(__uint_as_float(((bin + 1) << SAMPLE_TOP_SHIFT) - 1)); };
+                plain = least(S.mass1, bin1) + (found && bin0 != bin1 ? least(S.tot[bin0], bin0) : 0.f) <= (float)(C == 1 ? SAMPLE_BINS : SAMPLE_LIST);
+            }
+            cluster.map_shared_rank(&S, tid)->plan = make_uint4(bin0, bin1, plain ? 1u : 0u, 0u);
+        }
     }
     barrier();
     if (S.plan.z) {
@@ -545,7 +555,7 @@ __global__ void __launch_bounds__(SAMPLE_THREADS) sample_kernel(const float *__r
         __syncthreads();
     };
 
-    gather_bins();
+    if (S.plan.z) gather_bins();   // (else the first CTA's sums of before are still those of all candidates)
     unsigned long long X = X0, total = 0ull;
     uint32_t listed = 0xFFFFFFFFu, listed_m = 0;   // the top-level bin whose elements are in the list, ordered, and their number
     // Query 0: where the running sum exceeds topp (only that running sum matters: `cum`); query 1: where it exceeds coin * cum.
@@ -695,7 +705,7 @@ int32_t launch_sample(ib_ctx *ctx, cudaStream_t s, const float *logits, uint32_t
     // The instance that a slice fits with the fewest idle places: places cost instructions, a second round another trip to L2 (us per call, top-p,
     // 5 / 8 / 10 places: 32000 tokens, 2 a thread, 13.0 / 14.3 / 15.3; 128256, 8 a thread, 16.1 / 14.6 / 15.6; 152000, 10 a thread, 15.7 / 18.0 / 15.4).
     using Kernel = void (*)(const float *, uint32_t, uint32_t, float, float, uint64_t, const uint32_t *, float, float *, uint32_t *, uint32_t *, uint32_t);
-    static constexpr Kernel kernels[] = {sample_kernel<2>, sample_kernel<3>, sample_kernel<4>, sample_kernel<5>, sample_kernel<6>, sample_kernel<7>, sample_kernel<8>, sample_kernel<9>, sample_kernel<10>};
+    static constexpr Kernel kernels[] = {sample_kernel<1>, sample_kernel<2>, sample_kernel<3>, sample_kernel<4>, sample_kernel<5>, sample_kernel<6>, sample_kernel<7>, sample_kernel<8>, sample_kernel<9>, sample_kernel<10>};
     constexpr uint32_t INSTANCES = sizeof(kernels) / sizeof(kernels[0]);
     static uint32_t cluster_size[16] = {0};
     const size_t smem_max = sizeof(SampleShared) + SAMPLE_SLICE_MAX * sizeof(float);
@@ -728,7 +738,7 @@ int32_t launch_sample(ib_ctx *ctx, cudaStream_t s, const float *logits, uint32_t
     cfg.gridDim = dim3(ctas);
     cfg.dynamicSmemBytes = sizeof(SampleShared) + (probs ? 0 : slice * sizeof(float));
     cfg.numAttrs = pdl ? 2 : 1;
-    const uint32_t places = (slice + SAMPLE_THREADS - 1) / SAMPLE_THREADS, fits = places < 2 ? 0 : places - 2;
+    const uint32_t places = (slice + SAMPLE_THREADS - 1) / SAMPLE_THREADS, fits = places < 1 ? 0 : places - 1;
     IB_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernels[fits < INSTANCES ? fits : INSTANCES - 1], logits, n, slice, temperature, topp, seed, pos_ptr, coin, probs, out, out2, pdl));
     ctx->launches++;
     return IB_OK;

@@ -120,6 +120,12 @@ def test_the_bin_of_the_crossing(backend, n, many, spread):
         check_many(backend, logits, 1.0, topp, np.float32([0.0, 0.004, 0.02, 0.3, 0.6, 0.999]))
 
 
+@pytest.mark.parametrize("many,spread", [(3990, 1e-2), (4090, 0.0), (4096, 1e-3), (4110, 0.0), (4600, 1e-2)])
+def test_about_as_many_elements_as_the_list_holds(backend, many, spread):
+    """Whether they fit is estimated from the bin's mass: either answer ends at the same token."""
+    test_the_bin_of_the_crossing(backend, 20000, many, spread)
+
+
 @pytest.mark.parametrize("n", [2, 100, 40000, 300000])
 @pytest.mark.parametrize("depth", [30.0, 37.0, 85.0])
 def test_a_coin_of_zero_falls_to_the_first_token_that_can_come(backend, n, depth):
