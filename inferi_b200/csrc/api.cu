@@ -47,9 +47,9 @@ int32_t check_device_error(ib_ctx *ctx) {
 
 // ---- copies to the host ----
 // Into ordinary host memory CUDA copies through a buffer of its own, step by step, and a fresh result - what a caller mostly hands in - is mapped
-// page by page as it is first written, a microsecond each (513 KB of logits: 53 us into pages that are there, 190 into new ones).  So: one transfer into
-// pinned memory, meanwhile the destination's pages are asked for in one call, then a plain copy.
-constexpr size_t STAGE_BYTES = 1u << 20, STAGE_LEAST = 16384;
+// page by page as it is first written, a microsecond each (513 KB of logits: 53 us into pages that are there, 190 into new ones).  So: transfers into
+// pinned memory, meanwhile the destination's pages are asked for in one call, then plain copies, each while the pieces behind it are still on their way.
+constexpr size_t STAGE_BYTES = 640u << 10, STAGE_LEAST = 16384, STAGE_PIECE = 131072;
 
 bool host_pageable(const void *p) {
     cudaPointerAttributes a;
@@ -72,6 +72,14 @@ struct BesideCaptures {
     BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
     ~BesideCaptures() { cudaThreadExchangeStreamCaptureMode(&mode); }
 };
+static void free_staging(ib_ctx *ctx) {
+    if (ctx->stage_host) cudaFreeHost(ctx->stage_host);
+    ctx->stage_host = nullptr;
+    for (cudaEvent_t &e : ctx->stage_event) {
+        if (e) cudaEventDestroy(e);
+        e = nullptr;
+    }
+}
 int32_t read_back(ib_ctx *ctx, cudaStream_t s, void *dst, const void *src, size_t nbytes) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     if (ctx->stage_host && nbytes >= STAGE_LEAST && nbytes <= STAGE_BYTES && host_pageable(dst) && cudaStreamIsCapturing(s, &capture) == cudaSuccess &&
@@ -79,10 +87,19 @@ int32_t read_back(ib_ctx *ctx, cudaStream_t s, void *dst, const void *src, size_
         std::unique_lock<std::mutex> mine(ctx->stage_lock, std::try_to_lock);   // another thread has it: CUDA's way
         if (mine) {
             BesideCaptures beside;
-            IB_CHECK_CUDA(cudaMemcpyAsync(ctx->stage_host, src, nbytes, cudaMemcpyDeviceToHost, s));
+            const uint32_t pieces = nbytes < 2 * STAGE_PIECE ? 1 : (nbytes < STAGE_PIECES * STAGE_PIECE ? (uint32_t)(nbytes / STAGE_PIECE) : STAGE_PIECES);
+            const size_t piece = ((nbytes + pieces - 1) / pieces + 4095) & ~(size_t)4095;
+            for (uint32_t i = 0; i < pieces; i++) {
+                const size_t at = i * piece, n = nbytes - at < piece ? nbytes - at : piece;
+                IB_CHECK_CUDA(cudaMemcpyAsync((char *)ctx->stage_host + at, (const char *)src + at, n, cudaMemcpyDeviceToHost, s));
+                if (i + 1 < pieces) IB_CHECK_CUDA(cudaEventRecord(ctx->stage_event[i], s));
+            }
             host_populate(dst, nbytes);
-            IB_CHECK_CUDA(cudaStreamSynchronize(s));
-            memcpy(dst, ctx->stage_host, nbytes);
+            for (uint32_t i = 0; i < pieces; i++) {
+                const size_t at = i * piece, n = nbytes - at < piece ? nbytes - at : piece;
+                IB_CHECK_CUDA(i + 1 < pieces ? cudaEventSynchronize(ctx->stage_event[i]) : cudaStreamSynchronize(s));
+                memcpy((char *)dst + at, (const char *)ctx->stage_host + at, n);
+            }
             return IB_OK;
         }
     }
@@ -140,8 +157,10 @@ int32_t ib_ctx_create(int32_t device, ib_ctx **out) {
         delete ctx;
         return set_error(IB_ERR_CUDA, "allocating the tile counters failed: %s", cudaGetErrorString(ce));
     }
-    if (cudaMallocHost(&ctx->stage_host, STAGE_BYTES) != cudaSuccess) {   // (copies then go CUDA's way)
-        ctx->stage_host = nullptr;
+    bool staging = cudaMallocHost(&ctx->stage_host, STAGE_BYTES) == cudaSuccess;
+    for (cudaEvent_t &e : ctx->stage_event) staging = staging && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+    if (!staging) {   // copies then go CUDA's way
+        free_staging(ctx);
         cudaGetLastError();
     }
     *out = ctx;
@@ -158,7 +177,7 @@ int32_t ib_ctx_destroy(ib_ctx *ctx) {
     if (ctx->err_host) cudaFreeHost(ctx->err_host);
     if (ctx->stream_counters) cudaFree(ctx->stream_counters);
     if (ctx->tc_scratch) cudaFree(ctx->tc_scratch);
-    if (ctx->stage_host) cudaFreeHost(ctx->stage_host);
+    free_staging(ctx);
     delete ctx;
     return IB_OK;
 }

@@ -66,6 +66,8 @@ __host__ __device__ inline uint32_t block_elems(int qtype) {
     }
 }
 
+constexpr uint32_t STAGE_PIECES = 4;   // of a copy to the host through pinned memory, at most
+
 }  // namespace ib
 
 struct ib_ctx {
@@ -93,6 +95,7 @@ struct ib_ctx {
     uint32_t tc_pass = 0xFFFFFFFFu;   // the longest pass (tokens) that the device has had room for
     // pinned staging of copies to the host (read_back); null: no room for it
     void *stage_host = nullptr;
+    cudaEvent_t stage_event[ib::STAGE_PIECES - 1] = {};   // a piece has arrived
     std::mutex stage_lock;
     // limit of every wait inside a kernel (on a shared-memory barrier, on another rank's arrival); ib_ctx_set_wait_limit
     uint64_t wait_limit_ns = 2000000000ull;
