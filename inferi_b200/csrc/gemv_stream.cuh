@@ -528,8 +528,9 @@ constexpr uint32_t QT_MIXED = 0xFFu;   // kernel instance for launches whose seg
 // How a launch's rows are split over the consumer warps: NB blocks of 256 columns per warp, CG warps side by side cover a row and
 // form a stream, RG such streams share the tiles.  One or two blocks per warp where half of the warps then cover a row (one stream
 // per pipeline; short rows leave room for two), four for longer rows - 8 rows at a time as long as three such tiles fit the ring
-// (`long8`), else tiles of 4 rows: two of them at a time where the ring holds five (so that a step's successor is there when it ends: 4096 x 14336
-// Q4_K 10.6 -> 9.8 us, 4096 x 10240 Q6_K 10.0 -> 9.4; with four, 4096 x 14336 Q6_K 11.5 -> 12.0), one otherwise.
+// (`long8`), else tiles of 4 rows: two of them at a time where the ring holds five, so that a step's successor is there when it ends, and the format
+// and the number of tiles make it pay (4096 x 14336 Q4_K 10.6 -> 9.8 us, 4096 x 10240 Q6_K 10.0 -> 9.4; with a ring of four, 4096 x 14336 Q6_K 11.5 -> 12.0; the
+// rule and its figures are beside the launcher), one otherwise.
 // 8 rows of one or two blocks per warp, of up to four, 4 rows of up to four, 8 rows of up to four out of two tiles of 4
 constexpr uint32_t ROWS8 = 0, ROWS8_LONG = 1, ROWS4 = 2, ROWS8_PAIR = 3;
 struct Split { uint32_t NB, CG, RG, mode; };
