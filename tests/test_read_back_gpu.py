@@ -9,14 +9,14 @@ import torch
 from inferi_b200.ops import Backend
 
 pytestmark = pytest.mark.gpu
-LEAST, MOST = 16384, 1 << 20
+LEAST, MOST, STAGED = 16384, 1 << 20, 640 << 10   # (beyond STAGED bytes a copy goes past the staging buffer)
 
 
 def d2h(b, dst_ptr, src, nbytes, stream=None):
     assert b.lib.ib_memcpy_d2h(b.handle, stream, dst_ptr, src.data_ptr(), nbytes) == 0
 
 
-@pytest.mark.parametrize("nbytes", [4, LEAST - 4, LEAST, LEAST + 4, 513024, MOST - 4, MOST, MOST + 4, 5 * MOST])
+@pytest.mark.parametrize("nbytes", [4, LEAST - 4, LEAST, LEAST + 4, 513024, MOST - 4, MOST, MOST + 4, 5 * MOST, 262140, 262144, 393220, STAGED - 4, STAGED, STAGED + 4])
 @pytest.mark.parametrize("offset", [0, 4, 4092])
 def test_bytes_arrive(backend, nbytes, offset):
     src = torch.randint(-2**31, 2**31 - 1, (nbytes // 4,), dtype=torch.int32, device="cuda")
