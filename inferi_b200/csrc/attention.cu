@@ -63,6 +63,7 @@ static uint32_t attn_cluster_ctas(const ib_ctx *ctx, const ib_attn_params &p, ui
 // (2 to 4 heads of 128 end at 2560, 8 at 2400: the latter was measured in the graph up to its crossing, the former at 1600 only.)
 uint32_t attn_regime_positions(const ib_ctx *ctx, const AttnLaunch &a, uint32_t regime) {
     if (ctx->sm_count == 0) return 0u;
+    if (regime == ATTN_LONG) return a.p.kv_mul <= 2 ? ATTN_ALONE : 0u;
     const bool has_middle = a.kv_dtype == IB_KV_F16 && a.p.kv_mul >= ATTN_GROUP;
     const uint32_t n_kv = attn_groups(a.p), middle = has_middle ? attn_cluster_ctas(ctx, a.p, ATTN_MIDDLE) : 0u;
     const uint32_t c = regime == ATTN_MIDDLE ? middle : attn_cluster_ctas(ctx, a.p, regime);
@@ -132,9 +133,9 @@ int32_t launch_attention(ib_ctx *ctx, cudaStream_t s, const AttnLaunch &a) {
     const bool aligned = attn_aligned(a.q, a.out);
     uint32_t regime = aligned ? a.regime : ATTN_LONG;
     if (!a.pos_ptr && aligned) {
-        regime = ATTN_LONG;
-        for (uint32_t r : {ATTN_MIDDLE, ATTN_SHORT})
-            if (p.pos < attn_regime_positions(ctx, a, r)) regime = r;
+        uint32_t positions[3];
+        for (uint32_t r : {ATTN_LONG, ATTN_SHORT, ATTN_MIDDLE}) positions[r] = attn_regime_positions(ctx, a, r);
+        regime = attn_regime_of(positions, (uint64_t)p.pos + 1);
     }
     uint32_t splits = a.max_splits, per;
     if (regime != ATTN_LONG) args.cluster = splits = attn_cluster_ctas(ctx, p, regime);

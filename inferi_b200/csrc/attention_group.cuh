@@ -45,12 +45,16 @@ __host__ __device__ constexpr int attn_steps(int hs, int heads, int bytes, uint3
     return bytes == 2 ? hs / 32 : 2;
 }
 constexpr uint32_t ATTN_MIN_PER_SPLIT = ATTN_WARPS * ATTN_ROWS_PER_WARP_STEP, ATTN_KNEE = 16, ATTN_KNEE_PER = 128;
-constexpr uint32_t ATTN_ALONE = 64;   // rows of one or two heads that one CTA is as fast with as two that merge (60 rows, 16 x 1 heads of 128: 2.4 us, 2.7 as two)
+// Rows of one or two heads that one CTA is as fast with as two that merge (60 rows, 16 x 1 heads of 128: 2.4 us, 2.7 as two).  It belongs to the long regime: a cluster
+// starts when all of its CTAs find room at one time (a layer of a token, 32 x 1 heads of 64, 20 positions: 24.7 us, 25.2 as the one busy CTA of a cluster).
+constexpr uint32_t ATTN_ALONE = 64;
 __host__ __device__ __forceinline__ void attn_plan(uint32_t total, uint32_t max_splits, uint32_t cluster, uint32_t warps, uint32_t heads, uint32_t &nsplit, uint32_t &per) {
-    if (cluster) {
+    if (heads <= 2 && total <= ATTN_ALONE) {
+        nsplit = 1;
+        per = total;
+    } else if (cluster) {
         nsplit = (total + warps * ATTN_ROWS_PER_WARP_STEP - 1) / (warps * ATTN_ROWS_PER_WARP_STEP);
         if (nsplit > cluster) nsplit = cluster;
-        if (heads <= 2 && total <= ATTN_ALONE) nsplit = 1;
         per = (total + nsplit - 1) / nsplit;
         nsplit = (total + per - 1) / per;
     } else {

@@ -229,6 +229,11 @@ constexpr uint32_t ATTN_LONG = 0, ATTN_SHORT = 1, ATTN_MIDDLE = 2;
 size_t attn_scratch_bytes(const ib_attn_params &p, uint32_t max_splits);
 uint32_t attn_max_splits(const ib_ctx *ctx, const ib_attn_params &p);
 int32_t launch_attention(ib_ctx *ctx, cudaStream_t s, const AttnLaunch &a);
-uint32_t attn_regime_positions(const ib_ctx *ctx, const AttnLaunch &a, uint32_t regime);   // positions (pos + 1) up to which `regime` may be set; 0: never
+// Positions (pos + 1) up to which `regime` may be set; 0: never.  The long one may always be, and up to these comes before the others.
+uint32_t attn_regime_positions(const ib_ctx *ctx, const AttnLaunch &a, uint32_t regime);
+inline uint32_t attn_regime_of(const uint32_t (&limits)[3], uint64_t positions) {
+    if (positions <= limits[ATTN_LONG]) return ATTN_LONG;
+    return positions <= limits[ATTN_SHORT] ? ATTN_SHORT : (positions <= limits[ATTN_MIDDLE] ? ATTN_MIDDLE : ATTN_LONG);
+}
 
 }  // namespace ib

@@ -125,7 +125,7 @@ struct ib_llama {
     float *h_logits = nullptr;     // pinned [vocab_l] + the token's word: where ib_llama_forward's results arrive
     cudaEvent_t staged = nullptr;  // the last copy out of h_pinned has been issued and finished
     // [ATTN_LONG], and for the contexts where the attention nodes have another shape [ATTN_SHORT], [ATTN_MIDDLE]: the positions that
-    // `regime_positions` says (0: no such graph)
+    // `regime_positions` says (attn_regime_positions; 0: no such graph)
     cudaGraphExec_t graph_exec[3] = {}, graph_exec_sample[3] = {};
     uint32_t regime_positions[3] = {};
     uint32_t recording_regime = ATTN_LONG;
@@ -241,7 +241,7 @@ static int32_t record_token(ib_llama *m, cudaStream_t s, uint32_t pdl) {
         a.out = m->xb; a.scratch = m->attn_scratch; a.counters = m->attn_counters; a.max_splits = m->attn_splits; a.pdl = pdl;
         a.regime = m->recording_regime;
         if (l == 0)
-            for (uint32_t r : {ATTN_SHORT, ATTN_MIDDLE}) m->regime_positions[r] = attn_regime_positions(ctx, a, r);
+            for (uint32_t r : {ATTN_LONG, ATTN_SHORT, ATTN_MIDDLE}) m->regime_positions[r] = attn_regime_positions(ctx, a, r);
         if ((rc = emit_attn(a))) return rc;
         // o_proj + residual (transformer.rs:450-453)
         p = GemvParams{};
@@ -717,7 +717,7 @@ static int32_t run_tokens(ib_llama *m, cudaStream_t s, const uint32_t *tokens, u
     for (uint32_t i = 0; i < n_steps; i++) {
         // the graph whose attention nodes have the shape for this many positions
         const uint64_t positions = (uint64_t)start_pos + i + 1;
-        const uint32_t regime = positions <= m->regime_positions[ATTN_SHORT] ? ATTN_SHORT : (positions <= m->regime_positions[ATTN_MIDDLE] ? ATTN_MIDDLE : ATTN_LONG);
+        const uint32_t regime = attn_regime_of(m->regime_positions, positions);
         cudaGraphExec_t exec = sampled ? m->graph_exec_sample[regime] : m->graph_exec[regime];
         IB_CHECK_CUDA(cudaGraphLaunch(exec, s));
         m->ctx->launches += sampled ? m->launches_per_token_sample : m->launches_per_token;

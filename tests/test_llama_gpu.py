@@ -88,6 +88,14 @@ def test_runs_of_one_format_get_their_ctas(backend, hidden, heads, kv_heads, typ
     check_loop(backend, cfg, synth_weights(cfg, seed=3007, device="cuda", recipe=recipe), True, prompt=[3, 500, 41], n_gen=3)
 
 
+# One or two heads per kv head: up to 64 positions one CTA of the long regime's graph, then clusters, then (head size 64: beyond 512) the long regime again
+@pytest.mark.parametrize("hidden,heads,kv_heads,kv_f16", [(256, 4, 4, True), (256, 4, 2, False), (512, 4, 2, True), (512, 4, 4, False)])
+def test_graphs_of_few_heads_at_64_positions(backend, hidden, heads, kv_heads, kv_f16):
+    cfg = Llama2Config(hidden, 256, 2, heads, kv_heads, 512, 96, 500000.0, 1e-5)
+    check_loop(backend, cfg, synth_weights(cfg, seed=3008, device="cuda", recipe=dict(TINY_RECIPE, ffn_down=quant.Q4_K)), kv_f16,
+               prompt=np.random.default_rng(hidden + kv_heads).integers(0, 512, 61).tolist(), n_gen=8)
+
+
 def test_token_graph_launch_count_and_oracle_tokens(backend):
     """A token is a graph of 5 kernels per layer + 3 (begin, classifier, end); the launch counter must say so, and the
     greedy tokens must be the oracle's."""

@@ -123,7 +123,7 @@ def test_attention_slice_shapes(backend, hs, n_kv, total):
 @pytest.mark.parametrize("kv_dtype", [np.float16, np.float32])
 @pytest.mark.parametrize("hs", [64, 128])
 @pytest.mark.parametrize("mul,n_heads,total", [(1, 1, 1), (1, 8, 32), (1, 8, 33), (1, 16, 512), (1, 16, 513), (1, 40, 300), (1, 64, 129), (2, 2, 5), (2, 16, 511), (2, 16, 1025), (2, 8, 5000),
-                                               (1, 8, 1041), (1, 4, 9007), (2, 8, 1050), (2, 4, 9001), (8, 8, 9), (8, 32, 260), (8, 64, 512), (8, 64, 513), (8, 64, 2401), (8, 32, 6401), (4, 32, 512), (4, 32, 514), (4, 4, 7000)])
+                                               (1, 8, 64), (1, 8, 65), (2, 8, 64), (2, 8, 65), (1, 8, 1041), (1, 4, 9007), (2, 8, 1050), (2, 4, 9001), (8, 8, 9), (8, 32, 260), (8, 64, 512), (8, 64, 513), (8, 64, 2401), (8, 32, 6401), (4, 32, 512), (4, 32, 514), (4, 4, 7000)])
 def test_attention_groups_of_heads(backend, kv_dtype, hs, mul, n_heads, total):
     test_attention(backend, kv_dtype, hs, n_heads, mul, total - 1, total + 3)
 
