@@ -244,20 +244,26 @@ constexpr int PF_DEEP = 4;
 static bool pf_deep(const StreamK &sk) { return prefill_max_pieces(sk) > 3; }
 
 // Tokens from which four share a CTA: with a norm as long as the CTA holds four rows in its registers.  Longer rows, read twice, took 64.1 us instead of 58.5
-// (2048 x 8192 Q4_K, 700 tokens, the GEMM with its inputs), a layer of 8192 hidden at 600 tokens 706 instead of 687; two tokens per CTA there 691.  Without a norm nothing
+// (2048 x 8192 Q4_K, 700 tokens, the GEMM with its inputs), a layer of 8192 hidden at 600 tokens 706 instead of 687; two tokens per CTA there 691.  Two where that ends
+// sooner: 152 CTAs of four tokens are two waves (4096 hidden, a layer, one / two / four tokens per CTA: 600 tokens 413.9 / 413.4 / 420.7, 800 549.0 / 544.3 / 549.0, 1021 670.3 /
+// 665.6 / 662.4).  Without a norm nothing
 // is held, and rows are shared out to CTAs of 4096 columns: 2048 x 1024, 1000 tokens 21.0 us (one token per CTA 25.6), x 8192, 700 55.5 (58.4), x 14336, 700
 // 91.0 (94.6; with four whole rows per CTA 102.5: 176 CTAs of 148 at a time).
 constexpr uint32_t PF_MANY_TOKENS = 512;
 int32_t launch_prefill_norm_split(ib_ctx *ctx, cudaStream_t s, float *X, const PfPlanes *add, const float *w, float eps, uint32_t n, uint32_t cols, __half *xt) {
     constexpr uint32_t held = PF_KEEP * PF_ROW_THREADS * 8;   // columns that a CTA holds in its registers
+    const uint32_t rows = (n + 15) & ~15u;
     const PfPlanes planes = add ? *add : PfPlanes{};
     auto launch = [&](auto kernel, uint32_t tokens) {
-        const dim3 grid(((n + 15) & ~15u) / tokens, w ? 1 : (cols + held / tokens - 1) / (held / tokens));
+        const dim3 grid(rows / tokens, w ? 1 : (cols + held / tokens - 1) / (held / tokens));
         return pf_launch(ctx, s, kernel, grid, PF_ROW_THREADS, X, planes, add ? 1u : 0u, w, eps, n, cols, xt);
     };
     const bool many = n >= PF_MANY_TOKENS;
     if (!w) return many ? launch(prefill_norm_split_kernel<4, 2, false>, 4) : launch(prefill_norm_split_kernel<1, 2, false>, 1);
-    if (many && cols <= held / 4) return launch(prefill_norm_split_kernel<4, 2, true>, 4);
+    if (many && cols <= held / 4) {   // four or two: what leaves the shorter last wave of CTAs (one CTA per SM)
+        auto rounds = [&](uint32_t tokens) { return tokens * ((rows + tokens * ctx->sm_count - 1) / (tokens * ctx->sm_count)); };
+        return rounds(2) < rounds(4) ? launch(prefill_norm_split_kernel<2, 2, true>, 2) : launch(prefill_norm_split_kernel<4, 2, true>, 4);
+    }
     return add && pf_deep(add->sk) ? launch(prefill_norm_split_kernel<1, PF_DEEP, true>, 1) : launch(prefill_norm_split_kernel<1, 2, true>, 1);
 }
 
