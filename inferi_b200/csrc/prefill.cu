@@ -47,11 +47,12 @@ __global__ void prefill_embed_kernel(QDesc embd, const uint32_t *tokens, uint32_
 // inputs' layout holds 8 tokens' 8 columns side by side, and a warp of one token writes 16 bytes of every 128.  With NORM the row stays in registers
 // between the two (PF_KEEP * 8 columns per thread; what is longer is read again).  Rows n .. n rounded up to 16 are zero-filled.
 constexpr int PF_ROW_THREADS = 512, PF_KEEP = 4;
+// Two tokens per CTA: a token's lanes are twice those of four, and the second half continues the first one's sums, so that the bits are those of four.
 template <int TOK, int DEPTH, bool NORM>
-__global__ void __launch_bounds__(PF_ROW_THREADS) prefill_norm_split_kernel(float *X, const PfPlanes add, uint32_t has_add, const float *w, float eps, uint32_t n, uint32_t cols,
+__global__ void __launch_bounds__(PF_ROW_THREADS, TOK == 2 ? 2 : 1) prefill_norm_split_kernel(float *X, const PfPlanes add, uint32_t has_add, const float *w, float eps, uint32_t n, uint32_t cols,
                                                                             __half *xt) {
-    constexpr uint32_t LANES = 32 / TOK, STEP = PF_ROW_THREADS / TOK * 8, WARPS = PF_ROW_THREADS / 32;
-    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, which = lane / LANES, t = blockIdx.x * TOK + which;
+    constexpr uint32_t PARTS = TOK == 2 ? 2 : 1, LANES = 32 / (TOK * PARTS), WARPS = PF_ROW_THREADS / 32, STEP = WARPS * LANES * 8, HELD = PF_KEEP / PARTS;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, which = lane / (LANES * PARTS), part = lane / LANES % PARTS, t = blockIdx.x * TOK + which;
     const uint32_t c0 = (warp * LANES + lane % LANES) * 8;   // cols % 256 == 0: whole warps
     const bool there = t < n;
     pf_enter();
@@ -84,18 +85,24 @@ __global__ void __launch_bounds__(PF_ROW_THREADS) prefill_norm_split_kernel(floa
 #pragma unroll
             for (int i = 0; i < 8; i++) ss += v.v[i] * v.v[i];
         };
+        // The lane's pieces: at c0 + (k0 + k) * STEP, k < HELD, up to the row's end or the half's, for all lanes of a warp alike (pf_emit8).  Two halves: cols is
+        // a multiple of 2 STEP.
+        const uint32_t k0 = PARTS == 1 ? 0 : part * (cols / STEP / 2), end = PARTS == 1 ? cols : c0 + (k0 + cols / STEP / 2) * STEP;
 #pragma unroll
-        for (int k = 0; k < PF_KEEP; k++) {
-            const uint32_t c = c0 + k * STEP;
-            if (c < cols) {
-                keep[k] = fetch(c);
-                square(keep[k]);
-            }
+        for (uint32_t k = 0; k < HELD; k++)
+            if (c0 + (k0 + k) * STEP < end) keep[k] = fetch(c0 + (k0 + k) * STEP);
+#pragma unroll
+        for (uint32_t p = 0; p < PARTS; p++) {
+            if (p) ss = __shfl_sync(0xffffffffu, ss, lane - LANES * part);   // (the second half goes on where the first one ended)
+#pragma unroll
+            for (uint32_t k = 0; k < HELD; k++)
+                if (p == part && c0 + (k0 + k) * STEP < end) square(keep[k]);
         }
-        for (uint32_t c = c0 + PF_KEEP * STEP; c < cols; c += STEP) square(fetch(c));
+        if (PARTS == 1)
+            for (uint32_t c = c0 + HELD * STEP; c < cols; c += STEP) square(fetch(c));
 #pragma unroll
         for (uint32_t o = LANES / 2; o; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        if (lane % LANES == 0) red[warp][which] = ss;
+        if (part == PARTS - 1 && lane % LANES == 0) red[warp][which] = ss;
         __syncthreads();
         float tot = 0.f;
 #pragma unroll
@@ -108,11 +115,10 @@ __global__ void __launch_bounds__(PF_ROW_THREADS) prefill_norm_split_kernel(floa
             pf_emit8(xt, t, c, cols, v);
         };
 #pragma unroll
-        for (int k = 0; k < PF_KEEP; k++) {
-            const uint32_t c = c0 + k * STEP;
-            if (c < cols) emit(c, keep[k]);
-        }
-        for (uint32_t c = c0 + PF_KEEP * STEP; c < cols; c += STEP) emit(c, there ? pf_load8u(x + c) : zero);
+        for (uint32_t k = 0; k < HELD; k++)
+            if (c0 + (k0 + k) * STEP < end) emit(c0 + (k0 + k) * STEP, keep[k]);
+        if (PARTS == 1)
+            for (uint32_t c = c0 + HELD * STEP; c < cols; c += STEP) emit(c, there ? pf_load8u(x + c) : zero);
     }
 }
 
@@ -243,12 +249,12 @@ int32_t launch_prefill_embed(ib_ctx *ctx, cudaStream_t s, const ib_qtensor *embd
 constexpr int PF_DEEP = 4;
 static bool pf_deep(const StreamK &sk) { return prefill_max_pieces(sk) > 3; }
 
-// Tokens from which four share a CTA: with a norm as long as the CTA holds four rows in its registers.  Longer rows, read twice, took 64.1 us instead of 58.5
-// (2048 x 8192 Q4_K, 700 tokens, the GEMM with its inputs), a layer of 8192 hidden at 600 tokens 706 instead of 687; two tokens per CTA there 691.  Two where that ends
-// sooner: 152 CTAs of four tokens are two waves (4096 hidden, a layer, one / two / four tokens per CTA: 600 tokens 413.9 / 413.4 / 420.7, 800 549.0 / 544.3 / 549.0, 1021 670.3 /
-// 665.6 / 662.4).  Without a norm nothing
-// is held, and rows are shared out to CTAs of 4096 columns: 2048 x 1024, 1000 tokens 21.0 us (one token per CTA 25.6), x 8192, 700 55.5 (58.4), x 14336, 700
-// 91.0 (94.6; with four whole rows per CTA 102.5: 176 CTAs of 148 at a time).
+// Tokens from which several share a CTA.  With a norm two, of which two CTAs fit an SM: a layer, one / four / two tokens per CTA, us: 4096 hidden, 512 tokens 351.2 / 349.1 /
+// 346.7, 600 (152 CTAs of four: two waves) 410.8 / 416.9 / 407.5, 1021 658.0 / 654.0 / 652.7; 2048 hidden, 512 199.2 / 190.7 / 189.1, 1021 336.6 / 329.4 / 326.9.  Their halves
+// need rows of 2048 or 4096 columns; four for others that a CTA holds in its registers; longer rows, read twice, took 64.1 us instead of 58.5 (2048 x 8192
+// Q4_K, 700 tokens, the GEMM with its inputs), a layer of 8192 hidden at 600 tokens 706 instead of 687.  Without a norm nothing is held, and rows are shared
+// out to CTAs of 4096 columns: 2048 x 1024, 1000 tokens 21.0 us (one token per CTA 25.6), x 8192, 700 55.5 (58.4), x 14336, 700 91.0 (94.6; with four whole rows
+// per CTA 102.5: 176 CTAs of 148 at a time).
 constexpr uint32_t PF_MANY_TOKENS = 512;
 int32_t launch_prefill_norm_split(ib_ctx *ctx, cudaStream_t s, float *X, const PfPlanes *add, const float *w, float eps, uint32_t n, uint32_t cols, __half *xt) {
     constexpr uint32_t held = PF_KEEP * PF_ROW_THREADS * 8;   // columns that a CTA holds in its registers
@@ -260,10 +266,8 @@ int32_t launch_prefill_norm_split(ib_ctx *ctx, cudaStream_t s, float *X, const P
     };
     const bool many = n >= PF_MANY_TOKENS;
     if (!w) return many ? launch(prefill_norm_split_kernel<4, 2, false>, 4) : launch(prefill_norm_split_kernel<1, 2, false>, 1);
-    if (many && cols <= held / 4) {   // four or two: what leaves the shorter last wave of CTAs (one CTA per SM)
-        auto rounds = [&](uint32_t tokens) { return tokens * ((rows + tokens * ctx->sm_count - 1) / (tokens * ctx->sm_count)); };
-        return rounds(2) < rounds(4) ? launch(prefill_norm_split_kernel<2, 2, true>, 2) : launch(prefill_norm_split_kernel<4, 2, true>, 4);
-    }
+    if (many && cols <= held / 4)
+        return cols % (held / 8) == 0 ? launch(prefill_norm_split_kernel<2, 2, true>, 2) : launch(prefill_norm_split_kernel<4, 2, true>, 4);
     return add && pf_deep(add->sk) ? launch(prefill_norm_split_kernel<1, PF_DEEP, true>, 1) : launch(prefill_norm_split_kernel<1, 2, true>, 1);
 }
 

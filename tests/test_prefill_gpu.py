@@ -85,10 +85,10 @@ def test_formats_that_share_a_launch(backend, qk, heads):
     dev_w.close()
 
 
-# The norm holds four tokens' rows of up to 4096 columns per CTA from 512 tokens on, one token's of up to 16384 else; a token count that leaves padding rows.
-# Without a nudge (eps 0) the padding rows' norm is infinite: they stay zero all the same.
-@pytest.mark.parametrize("hidden,eps", [(2048, 0.0), (4096, 1e-5), (4608, 1e-5), (8704, 0.0)])
-@pytest.mark.parametrize("n", [9, 517, 601])   # (601: two tokens per CTA, whose last wave is shorter)
+# From 512 tokens on the norm's CTAs hold rows of 2048 and 4096 columns of two tokens, others of up to 4096 of four, longer ones of one; a token count that leaves
+# padding rows.  Without a nudge (eps 0) the padding rows' norm is infinite: they stay zero all the same.
+@pytest.mark.parametrize("hidden,eps", [(2048, 0.0), (3072, 0.0), (4096, 1e-5), (4608, 1e-5), (8704, 0.0)])
+@pytest.mark.parametrize("n", [9, 517, 601])
 def test_norms_of_many_tokens(backend, hidden, eps, n):
     cfg = Llama2Config(hidden, 512, 1, hidden // 128, hidden // 512, 512, 640, 500000.0, eps)
     w = synth_weights(cfg, seed=hidden, device="cuda", recipe={**{k: quant.Q4_K for k in Q4_K_M}, "token_embd": quant.Q4_K})
